@@ -1,0 +1,73 @@
+"""Products of more than 256 tokens on CTA pairs (csrc/gemm_pair.cu) against 64-bit torch: token counts around the 32-token
+unit and the 256-token tile, weight rows around the 256-row pair tile, every epilogue, and nothing written outside Y."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+PLAIN, PLAIN_F32, SWIGLU, GEGLU, RELU2 = 0, 1, 2, 3, 4   # tgis_k_gemm out modes
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from vllm_tgis_adapter_b200.engine._lib import load_library
+
+    return load_library()
+
+
+def run(lib, x, w, T, mode, rows):
+    N, K = w.shape
+    y = torch.full((T + 1, N), 7.0, device="cuda", dtype=torch.float32 if mode == PLAIN_F32 else torch.bfloat16)
+    ms = C.c_float()
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    assert lib.tgis_k_gemm(p(x), p(w), p(y), T, N, K, rows, 0, 1, C.byref(ms), mode) == 0, lib.tgis_k_last_error()
+    return y
+
+
+@pytest.mark.parametrize("mode", [PLAIN, PLAIN_F32, SWIGLU, GEGLU, RELU2])
+@pytest.mark.parametrize("T,N,K", [(257, 256, 256), (288, 258, 320), (289, 130, 64), (511, 520, 512), (512, 8, 768), (513, 2128, 256), (2050, 3000, 1088)])
+def test_pair_products(lib, T, N, K, mode):
+    gen = torch.Generator(device="cuda").manual_seed(T + N + K)
+    rows = max(T, 256) + 3   # fewer rows than the last token tile covers: the rest is read as zeros
+    x = torch.randn(rows, K, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(N, K, generator=gen, device="cuda") * K ** -0.5).bfloat16()
+    y = run(lib, x, w, T, mode, rows)
+    acc = x[:T].double() @ w.double().T
+    # fp32 sums of K products in steps of 16: every step may lose an ulp of the running sum, which the sum of magnitudes bounds
+    slack = (x[:T].double().abs() @ w.double().abs().T) * (K / 16 + 8) * 2.0 ** -23
+    if mode == SWIGLU:   # gate, up and silu(gate) are rounded to bf16: 2^-8 each, and the result's own rounding
+        g, u = acc[:, 0::2], acc[:, 1::2]
+        sg, su = slack[:, 0::2], slack[:, 1::2]
+        ref = g * torch.sigmoid(g) * u
+        tol = 5 * 2.0 ** -8 * ref.abs() + 1.1 * ((sg + 2.0 ** -8 * g.abs()) * u.abs() + g.abs() * su)   # |silu'| <= 1.1
+    elif mode == GEGLU:
+        g, u = acc[:, 0::2], acc[:, 1::2]
+        ref = torch.nn.functional.gelu(g, approximate="tanh") * u
+        tol = 2.0 ** -8 * ref.abs() + 1.13 * slack[:, 0::2] * u.abs() + g.abs() * slack[:, 1::2] + 1e-6 * g.abs() * u.abs()
+    elif mode == RELU2:
+        ref = acc.clamp(min=0) ** 2
+        tol = 2.0 ** -8 * ref + (2 * acc.abs() + slack) * slack
+    else:
+        ref, tol = acc, slack + (0 if mode == PLAIN_F32 else 2.0 ** -8) * acc.abs()
+    flat = y.reshape(-1)
+    if mode == GEGLU:   # (this hook gives the GeGLU product rows of N elements, half of each written)
+        got, rest = y[:T, : N // 2], torch.cat([y[:T, N // 2:].reshape(-1), y[T]])
+    elif mode == SWIGLU:
+        got, rest = flat[: T * (N // 2)].view(T, N // 2), flat[T * (N // 2):]
+    else:
+        got, rest = y[:T], y[T]
+    over = (got.double() - ref).abs() - tol
+    assert float(over.max()) <= 0, (float(over.max()), float((over > 0).double().mean()))
+    assert bool((rest == 7.0).all())
+    assert torch.equal(run(lib, x, w, T, mode, rows), y)   # an output is one sum in ascending k: the same bits every time
+
+
+def test_pair_product_does_not_depend_on_the_other_tokens(lib):
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(1200, 512, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(640, 512, generator=gen, device="cuda") * 512 ** -0.5).bfloat16()
+    whole = run(lib, x, w, 1200, PLAIN_F32, 1200)
+    part = run(lib, x[700:].contiguous(), w, 300, PLAIN_F32, 500)   # other tiles, other neighbours
+    assert torch.equal(part[:300], whole[700:1000])

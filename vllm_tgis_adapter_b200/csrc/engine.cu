@@ -192,9 +192,9 @@ __global__ void gather_relayout_kernel(const uint4* __restrict__ gathered, uint4
 }
 
 constexpr int N_BT = 5;
-const int BT_VALUES[N_BT] = {16, 32, 64, 128, 256};
+const int BT_VALUES[N_BT] = {16, 32, 64, 128, 256};  // box heights of the activation maps
 int bt_index(int T) {
-  int bt = gemm_pick_bt(T);
+  const int bt = gemm_x_box(T);
   for (int i = 0; i < N_BT; ++i)
     if (BT_VALUES[i] == bt) return i;
   return N_BT - 1;
@@ -3480,6 +3480,10 @@ struct tgis_engine {
 
   // Wait until everything up to ev1 (the step's last operation on the stream) has executed.
   void wait_step_end() {
+    spin_step_end();
+    if (gemm_pair_failed()) throw CudaError("a product's pipeline wait ran out: the step's results are not valid");
+  }
+  void spin_step_end() {
     if (!sync_spin) {
       CK(cudaStreamSynchronize(stream));
       return;

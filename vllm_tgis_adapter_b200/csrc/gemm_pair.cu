@@ -1,0 +1,486 @@
+// Y = X W^T on CTA pairs (tcgen05 cta_group::2): the products of prompts and of expert segments.
+//
+// Two neighbouring SMs work on one tile of 256 weight rows x up to 256 tokens.  Weights are the MMA's A operand (each CTA
+// holds 128 of the 256 rows), tokens its B operand (each CTA holds half of them and the tensor cores read both halves), so a
+// k-block costs an SM 16 KB of weights and at most 16 KB of tokens for 128 x 256 x 64 multiply-adds: two thirds of what the
+// one-CTA tile of gemm_tcgen05.cu (128 x 256) reads.  That traffic out of L2 (about 10 TB/s) is what bounds a product of
+// thousands of tokens; measured on one B200, T x N x K, one-CTA tiles -> pairs:
+//   2048 x 28672 x 4096 (SwiGLU) 742 -> 312 us (1540 TFLOP/s)      512 x 28672 x 4096 (SwiGLU) 335 -> 99 us
+//   2048 x 4096 x 14336          218 -> 165 us (1460)              512 x 4096 x 14336           75 -> 55 us
+//   2048 x 6144 x 4096           142 -> 84 us (1220)               2048 x 2128 x 2048 (fp32 out)  47 -> 17 us
+//   2048 x 4096 x 4096            90 -> 48 us (1440)               257 x 768 x 3072              37 -> 13 us
+//
+// Token tiles have any size that is a multiple of 32 (UMMA_N), which serves two ends:
+//  * dense products: the tokens are cut into the number of equal tiles that fills whole waves of the 74 pairs best
+//    (gemm_pair_plan); no tile is ever split along k, so there is no reduction between CTAs and an output is one sum in
+//    ascending k whatever the launch;
+//  * grouped products (one row segment per expert): a segment is cut into equal tiles of at most 256 rows, a segment of 40
+//    rows costs 64 columns.  The tile list is derived from the segment offsets on the device.
+//
+// Roles per CTA: warp 0 TMA producer, warp 1 MMA issuer (leader CTA only) and TMEM owner, warps 2..5 epilogue on a double
+// buffered accumulator (2 x 256 columns).  The leader's `full` barrier counts both CTAs' bytes; tcgen05.commit releases a
+// ring slot in both CTAs at once.  No wait is unbounded: after about two seconds a role gives up, raises the host-visible
+// error word and leaves; TMEM is freed on every path.
+#include "kernels.h"
+#include "launch.cuh"
+#include "ptx.cuh"
+
+namespace tgis {
+namespace {
+
+constexpr int PAIR_THREADS = 192;
+constexpr int PAIR_BK = 64;
+constexpr int PAIR_STAGES = 6;
+constexpr int PAIR_TILE_BYTES = 128 * PAIR_BK * 2;         // one CTA's half of either operand
+constexpr int PAIR_UNIT = 32;                              // token tiles are multiples of this (UMMA_N step of an M = 256 pair)
+constexpr int X_BOX_BYTES = GEMM_X_BOX_MANY * PAIR_BK * 2;
+constexpr int PAIR_MAX_GROUPS = 2048;
+constexpr int PAIR_BAR_BYTES = 256;
+constexpr size_t pair_smem(bool grouped) {
+  return (size_t)PAIR_STAGES * 2 * PAIR_TILE_BYTES + 1024 + PAIR_BAR_BYTES + (grouped ? (PAIR_MAX_GROUPS + 1) * sizeof(int) : 0);
+}
+
+struct PairArgs {
+  void* Y;
+  int ldy, T, N, K;
+  int n_tiles, x_tiles;     // weight tiles of 256 rows; token tiles (dense)
+  int y_f32, mode;          // mode: PAIR_* (Y in fp32: PAIR_PLAIN only)
+  const int* seg_off;       // grouped: [n_groups + 1]
+  int n_groups;
+  const float* row_scale;   // PAIR_RELU2: scale of the input row gather[p] (null: 1)
+  const int* gather;
+  int* err;                 // host-visible error word
+};
+
+// ---------------------------------------------------------------- cta_group::2 forms
+template <uint32_t kCols>
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_dst) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(smem_dst)), "n"(kCols));
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n");
+}
+template <uint32_t kCols>
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;\n" ::"r"(taddr), "n"(kCols));
+}
+__device__ __forceinline__ void mma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// arrive on the barrier at this offset in both CTAs of the pair once all MMAs issued so far have retired
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(smem_u32(bar)),
+               "h"((uint16_t)3)
+               : "memory");
+}
+// tile into this CTA's shared memory, bytes counted on a barrier of either CTA of the pair (`bar`: shared::cluster address)
+__device__ __forceinline__ void tma_load_pair(const CUtensorMap* m, uint32_t bar, void* dst, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4}], [%2];\n" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, int* err) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (clock64() - t0 > 4000000000ll) {   // about two seconds: no wait of a working pipeline is that long
+      *reinterpret_cast<volatile int*>(err) = 1;
+      __threadfence_system();
+      return false;
+    }
+  }
+  return true;
+}
+
+// silu without the branch of an IEEE division (a quotient within 2 ulp): the epilogue's values interleave, and the result is
+// rounded to bf16
+__device__ __forceinline__ float pair_silu(float g) { return __fdividef(g, 1.f + expf(-g)); }
+template <int MODE>
+__device__ __forceinline__ float pair_glu(float g, float u) {
+  if constexpr (MODE == PAIR_SWIGLU_BF16) {   // the rounding points of a bf16 gate / up product followed by silu and a product
+    return bf16_round(pair_silu(bf16_round(g))) * bf16_round(u);
+  } else if constexpr (MODE == PAIR_SWIGLU) {
+    return pair_silu(g) * u;
+  } else {
+    return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
+  }
+}
+template <int MODE>
+__device__ __forceinline__ float pair_act(float v, float s) {
+  if constexpr (MODE == PAIR_RELU2) {
+    const float z = fmaxf(v * s, 0.f);
+    return z * z;
+  } else if constexpr (MODE == PAIR_GELU) {
+    return 0.5f * v * (1.f + erff(v * 0.7071067811865476f));
+  } else {
+    return v;
+  }
+}
+template <class OT>
+__device__ __forceinline__ OT pair_out(float v) {
+  if constexpr (sizeof(OT) == 4) return v;
+  else return __float2bfloat16_rn(v);
+}
+
+struct PairTile {
+  int w_row;       // first weight row of the tile in the weight map
+  int n0;          // first output column
+  int row0, rows;  // token rows [row0, row0 + rows)
+  int n;           // UMMA_N: rows rounded up to PAIR_UNIT
+};
+
+// Tiles of one pair in launch order: index pair, pair + pairs, ...
+template <bool GROUPED>
+struct PairIter {
+  const PairArgs& a;
+  const int* start;  // grouped: first tile of every segment [n_groups + 1] (shared memory)
+  int i, step, total, g;
+  __device__ PairIter(const PairArgs& a_, const int* start_, int pair, int pairs) : a(a_), start(start_), i(pair), step(pairs), g(0) {
+    total = GROUPED ? start[a.n_groups] : a.n_tiles * a.x_tiles;
+  }
+  __device__ bool next(PairTile& t) {
+    if (i >= total) return false;
+    int n_tile, x_tile, x_tiles, base, rows, units;
+    if (GROUPED) {
+      while (i >= start[g + 1]) ++g;
+      base = a.seg_off[g];
+      rows = a.seg_off[g + 1] - base;
+      units = (rows + PAIR_UNIT - 1) / PAIR_UNIT;
+      x_tiles = (units + 7) / 8;
+      const int k = i - start[g];   // token tile fastest: the pairs that share a weight tile run side by side
+      n_tile = k / x_tiles;
+      x_tile = k - n_tile * x_tiles;
+    } else {
+      // blocks of 8 weight tiles, token tile next, weight tile fastest: a wave of 74 is a compact rectangle
+      constexpr int NB = 8;
+      base = 0;
+      rows = a.T;
+      units = (rows + PAIR_UNIT - 1) / PAIR_UNIT;
+      x_tiles = a.x_tiles;
+      const int full = NB * x_tiles, nb = i / full, rem = i - nb * full, nb_n = min(NB, a.n_tiles - nb * NB);
+      x_tile = rem / nb_n;
+      n_tile = nb * NB + rem - x_tile * nb_n;
+    }
+    const int u0 = x_tile * units / x_tiles, u1 = (x_tile + 1) * units / x_tiles;
+    t.n0 = n_tile * 256;
+    t.w_row = (GROUPED ? g * a.N : 0) + t.n0;
+    t.row0 = base + u0 * PAIR_UNIT;
+    t.rows = min(rows - u0 * PAIR_UNIT, (u1 - u0) * PAIR_UNIT);
+    t.n = (u1 - u0) * PAIR_UNIT;
+    i += step;
+    return true;
+  }
+};
+
+// One accumulator (this warp's 32 weight rows x t.rows tokens) -> Y; lane = weight row, column = token
+template <int MODE, class OT>
+__device__ __forceinline__ void pair_store(const PairArgs& a, const PairTile& t, int n, uint32_t taddr, int lane) {
+  constexpr bool GLU = MODE == PAIR_SWIGLU || MODE == PAIR_SWIGLU_BF16 || MODE == PAIR_GEGLU;
+  const bool n_ok = GLU ? (n | 1) < a.N : n < a.N;
+  OT* y = reinterpret_cast<OT*>(a.Y) + (size_t)t.row0 * a.ldy + (GLU ? n >> 1 : n);
+#pragma unroll 1
+  for (int c0 = 0; c0 < t.rows; c0 += 32, y += (size_t)32 * a.ldy) {
+    uint32_t r[32];
+    tmem_ld_32x32b_x16(taddr + c0, r);
+    tmem_ld_32x32b_x16(taddr + c0 + 16, r + 16);
+    tmem_ld_wait();
+    const int valid = n_ok ? t.rows - c0 : 0;
+    if constexpr (GLU) {
+      // rows (2j, 2j + 1) of W are (gate_j, up_j), in adjacent lanes: the even lane makes token c's value, the odd lane token
+      // c + 1's, with one exchange for both
+      const bool odd = lane & 1;
+      OT* yl = y + (odd ? a.ldy : 0);
+      const int mine_valid = valid - (odd ? 1 : 0);
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) {
+        const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? r[j] : r[j + 1]), 1);
+        const float g = odd ? got : __uint_as_float(r[j]), u = odd ? __uint_as_float(r[j + 1]) : got;
+        const float v = pair_glu<MODE>(g, u);
+        if (j < mine_valid) yl[(size_t)j * a.ldy] = pair_out<OT>(v);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        if (j < valid) {
+          float s = 1.f;
+          if constexpr (MODE == PAIR_RELU2) {
+            if (a.row_scale != nullptr) s = a.row_scale[a.gather != nullptr ? a.gather[t.row0 + c0 + j] : t.row0 + c0 + j];
+          }
+          y[(size_t)j * a.ldy] = pair_out<OT>(pair_act<MODE>(__uint_as_float(r[j]), s));
+        }
+    }
+  }
+}
+
+template <bool GROUPED>
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ PairArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem_w = smem;
+  uint8_t* smem_x = smem + PAIR_STAGES * PAIR_TILE_BYTES;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + 2 * PAIR_STAGES * PAIR_TILE_BYTES);
+  uint64_t* empty_bar = full_bar + PAIR_STAGES;
+  uint64_t* tmem_full = empty_bar + PAIR_STAGES;
+  uint64_t* tmem_empty = tmem_full + 2;
+  uint32_t* tmem_base_smem = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  int* seg_start = reinterpret_cast<int*>(smem + 2 * PAIR_STAGES * PAIR_TILE_BYTES + PAIR_BAR_BYTES);
+
+  const int warp = threadIdx.x >> 5, lane = (int)lane_id();
+  const int rank = (int)cluster_ctarank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int KB = (a.K + PAIR_BK - 1) / PAIR_BK;
+
+  if (warp == 0 && elect_one()) {
+    tma_prefetch_desc(&wmap);
+    tma_prefetch_desc(&xmap);
+  }
+  if (warp == 1) {
+    if (elect_one()) {
+      for (int i = 0; i < PAIR_STAGES; ++i) {
+        mbar_init(&full_bar[i], 1);    // the leader's expect_tx (both CTAs' bytes)
+        mbar_init(&empty_bar[i], 1);   // commit_pair
+      }
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(&tmem_full[i], 1);   // commit_pair
+        mbar_init(&tmem_empty[i], 8);  // four epilogue warps of either CTA (leader's barrier)
+      }
+      fence_barrier_init();
+    }
+    __syncwarp();
+    tmem_alloc_pair<512>(tmem_base_smem);
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();   // the peer's barriers exist
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_base_smem;
+  griddep_launch();
+  if (GROUPED) {   // the segment offsets come from a kernel of this step
+    griddep_wait();
+    if (warp == 0) {   // exclusive prefix sum of the segments' tile counts
+      int run = 0;
+      for (int g0 = 0; g0 < a.n_groups; g0 += 32) {
+        const int g = g0 + lane;
+        int c = 0;
+        if (g < a.n_groups) c = ((a.seg_off[g + 1] - a.seg_off[g] + PAIR_UNIT - 1) / PAIR_UNIT + 7) / 8 * a.n_tiles;
+        int s = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int up = __shfl_up_sync(0xffffffffu, s, o);
+          if (lane >= o) s += up;
+        }
+        if (g < a.n_groups) seg_start[g] = run + s - c;
+        run += __shfl_sync(0xffffffffu, s, 31);
+      }
+      if (lane == 0) seg_start[a.n_groups] = run;
+    }
+    __syncthreads();
+  }
+
+  if (warp == 0) {
+    // ===================== TMA producer (both CTAs) =====================
+    if (elect_one()) {
+      PairIter<GROUPED> it(a, seg_start, pair, pairs);
+      PairTile t;
+      int stage = 0, issued = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      const uint32_t full0 = dsmem_addr(smem_u32(full_bar), 0);   // the leader's barriers
+      int w_row = 0, x_row = 0, boxes = 0;
+      uint32_t bytes = 0;
+      auto set_tile = [&]() {
+        boxes = (t.n / 2 + GEMM_X_BOX_MANY - 1) / GEMM_X_BOX_MANY;
+        bytes = 2u * (uint32_t)(PAIR_TILE_BYTES + boxes * X_BOX_BYTES);
+        w_row = t.w_row + rank * 128;
+        x_row = t.row0 + rank * (t.n / 2);
+      };
+      auto load_w = [&](int s, int kb) {
+        if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], bytes);
+        tma_load_pair(&wmap, full0 + s * 8, smem_w + s * PAIR_TILE_BYTES, kb * PAIR_BK, w_row);
+      };
+      auto load_x = [&](int s, int kb) {
+#pragma unroll
+        for (int b = 0; b < 128 / GEMM_X_BOX_MANY; ++b)
+          if (b < boxes) tma_load_pair(&xmap, full0 + s * 8, smem_x + s * PAIR_TILE_BYTES + b * X_BOX_BYTES, kb * PAIR_BK, x_row + b * GEMM_X_BOX_MANY);
+      };
+      bool have = it.next(t);
+      if (have) set_tile();
+      if (!GROUPED) {
+        // weights are static: the first ring of them is requested before the previous kernel has finished
+        const int pre = have ? min(KB, PAIR_STAGES) : 0;
+        for (int kb = 0; kb < pre; ++kb) load_w(kb, kb);
+        griddep_wait();
+        for (int kb = 0; kb < pre; ++kb) load_x(kb, kb);
+        issued = pre;
+        stage = pre % PAIR_STAGES;
+        phase = pre == PAIR_STAGES ? 1 : 0;
+      }
+      while (have && ok) {
+        for (int kb = issued; kb < KB; ++kb) {
+          if (!(ok = pair_wait(&empty_bar[stage], phase ^ 1, a.err))) break;
+          load_w(stage, kb);
+          load_x(stage, kb);
+          if (++stage == PAIR_STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        issued = 0;
+        have = it.next(t);
+        if (have) set_tile();
+      }
+      if (!ok) __nanosleep(1000000);   // copies in flight land before the CTA leaves
+    }
+  } else if (warp == 1) {
+    // ===================== MMA issuer (leader) =====================
+    if (rank == 0) {
+      PairIter<GROUPED> it(a, seg_start, pair, pairs);
+      PairTile t;
+      int stage = 0, acc = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      bool ok = true;
+      while (ok && it.next(t)) {
+        const uint32_t idesc = make_idesc_bf16(256, (uint32_t)t.n);
+        ok = __all_sync(0xffffffffu, pair_wait(&tmem_empty[acc], acc_phase ^ 1, a.err));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * 256;
+        for (int kb = 0; kb < KB; ++kb) {
+          ok = __all_sync(0xffffffffu, pair_wait(&full_bar[stage], phase, a.err));
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            const uint64_t a_desc = make_smem_desc_sw128(smem_u32(smem_w + stage * PAIR_TILE_BYTES));
+            const uint64_t b_desc = make_smem_desc_sw128(smem_u32(smem_x + stage * PAIR_TILE_BYTES));
+#pragma unroll
+            for (int k = 0; k < PAIR_BK / 16; ++k)
+              mma_pair(d_tmem, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            commit_pair(&empty_bar[stage]);
+            if (kb == KB - 1) commit_pair(&tmem_full[acc]);
+          }
+          __syncwarp();
+          if (++stage == PAIR_STAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (++acc == 2) {
+          acc = 0;
+          acc_phase ^= 1;
+        }
+      }
+    }
+  } else {
+    // ===================== epilogue (both CTAs): lane = weight row, column = token =====================
+    const int sub = warp & 3;
+    PairIter<GROUPED> it(a, seg_start, pair, pairs);
+    PairTile t;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    if (!GROUPED) griddep_wait();   // Y (and the input scales) may still be in use by the previous kernels
+    while (it.next(t)) {
+      if (!__all_sync(0xffffffffu, pair_wait(&tmem_full[acc], acc_phase, a.err))) break;
+      tc_fence_after();
+      const int n = t.n0 + rank * 128 + sub * 32 + lane;
+      const uint32_t taddr = tmem_base + acc * 256 + ((uint32_t)(sub * 32) << 16);
+      using bf = __nv_bfloat16;
+      switch (a.mode) {
+        case PAIR_SWIGLU_BF16: pair_store<PAIR_SWIGLU_BF16, bf>(a, t, n, taddr, lane); break;
+        case PAIR_SWIGLU: pair_store<PAIR_SWIGLU, bf>(a, t, n, taddr, lane); break;
+        case PAIR_GEGLU: pair_store<PAIR_GEGLU, bf>(a, t, n, taddr, lane); break;
+        case PAIR_RELU2: pair_store<PAIR_RELU2, bf>(a, t, n, taddr, lane); break;
+        case PAIR_GELU: pair_store<PAIR_GELU, bf>(a, t, n, taddr, lane); break;
+        default:
+          if (a.y_f32) pair_store<PAIR_PLAIN, float>(a, t, n, taddr, lane);
+          else pair_store<PAIR_PLAIN, bf>(a, t, n, taddr, lane);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(dsmem_addr(smem_u32(&tmem_empty[acc]), 0));
+      if (++acc == 2) {
+        acc = 0;
+        acc_phase ^= 1;
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();   // nobody leaves while the peer may still read its shared memory or signal its barriers
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair<512>(tmem_base);
+  }
+}
+
+// host-visible error word, one for the process (a raised word is an error of the process's device, as a sticky CUDA error is)
+int* pair_error_word() {
+  static int* word = [] {
+    int* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return (int*)nullptr;
+    *p = 0;
+    return p;
+  }();
+  return word;
+}
+
+template <bool GROUPED>
+cudaError_t launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, PairArgs a, int grid, cudaStream_t stream) {
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(gemm_pair_kernel<GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem(GROUPED));
+  if (attr != cudaSuccess) return attr;
+  a.err = pair_error_word();
+  if (a.err == nullptr) return cudaErrorMemoryAllocation;
+  return launch_k_cluster(gemm_pair_kernel<GROUPED>, dim3(grid), dim3(PAIR_THREADS), pair_smem(GROUPED), stream, 2, wmap, xmap, a);
+}
+
+}  // namespace
+
+bool gemm_pair_failed() {
+  const int* w = pair_error_word();
+  return w != nullptr && *reinterpret_cast<const volatile int*>(w) != 0;
+}
+
+// Number of token tiles for a dense product of T tokens and N weight rows on `pairs` CTA pairs.  A k-block of a tile of n
+// tokens takes about 130 + n nanoseconds when all pairs run (2048 x 28672 x 4096: 382 at n = 256, 339 at 224, 284 at 192,
+// 245 at 128; below 64 the weight half alone is what it takes), so the count that makes waves * (130 + largest n) smallest
+// is taken.  Measured at the sizes of an 8B layer and of 768 to 2048 wide ones, 257 to 2048 tokens: within 3 % of the best
+// count but for 2048 x 6144 x 4096 (8 tiles 84 us, 11 tiles 74 us).
+int gemm_pair_plan(int T, int N, int pairs) {
+  const int units = (T + PAIR_UNIT - 1) / PAIR_UNIT, n_tiles = (N + 255) / 256, least = (units + 7) / 8;
+  int best = least;
+  long long best_cost = -1;
+  for (int x = least; x <= units && x <= least + 16; ++x) {
+    const int n = (units + x - 1) / x * PAIR_UNIT;
+    const long long cost = ((long long)n_tiles * x + pairs - 1) / pairs * (130 + (n > 64 ? n : 64));
+    if (best_cost < 0 || cost < best_cost) {
+      best = x;
+      best_cost = cost;
+    }
+  }
+  return best;
+}
+
+cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int y_f32, int mode, int T, int N, int K,
+                             int num_sms, cudaStream_t stream) {
+  if (T <= 0 || N <= 0 || K <= 0 || (y_f32 && mode != PAIR_PLAIN)) return cudaErrorInvalidValue;
+  const int pairs = num_sms / 2;
+  if (pairs < 1) return cudaErrorInvalidValue;
+  PairArgs a{};
+  a.Y = Y; a.ldy = ldy; a.T = T; a.N = N; a.K = K;
+  a.y_f32 = y_f32; a.mode = mode;
+  a.n_tiles = (N + 255) / 256;
+  a.x_tiles = gemm_pair_plan(T, N, pairs);
+  const int tiles = a.n_tiles * a.x_tiles;
+  return launch_pair<false>(wmap, xmap, a, 2 * (tiles < pairs ? tiles : pairs), stream);
+}
+
+}  // namespace tgis

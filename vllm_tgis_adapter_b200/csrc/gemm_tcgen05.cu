@@ -63,49 +63,29 @@ struct GemmCfg {
   static constexpr int SMEM_MAX = (SMEM_BYTES + 16384) < 227 * 1024 ? (SMEM_BYTES + 16384) : 227 * 1024;
 };
 
-// Prefill-shaped launches (more than one token tile): "data-parallel waves + stream-K tail".  Linear tile index i
-// (see tile_decode) -> the first dp_waves * ncta tiles are whole tiles dealt round-robin, wave w = tiles
-// [w * ncta, (w+1) * ncta): at any moment the 148 CTAs work on ONE compact 8 x ~18 rectangle of (weight tile, token
-// tile) pairs, so both operands of a wave stay in L2 (with contiguous per-CTA ranges the CTAs drift apart, the working
-// set is every weight tile + every activation tile, and ncu showed 11 GB of DRAM reads for 0.3 GB of operands).  The
-// remaining < ncta tiles are cut stream-K style as before.  Decode-shaped launches have dp_waves = 0: unchanged.
+// The launch's tiles (128 weight rows x all T <= 256 tokens; more tokens run on CTA pairs, gemm_pair.cu) are cut stream-K
+// style into one contiguous range of k-blocks per CTA.
 //
-// Decode-shaped launches with at least one tile per CTA (gate_up: 224 tiles on 148 CTAs, lm_head: 1002) use the same two
-// regions in the OPPOSITE order ("sk_first"): every CTA first works through its < 1 tile share of the stream-K region --
+// Launches with at least one tile per CTA (gate_up: 224 tiles on 148 CTAs, lm_head: 1002) have two regions ("sk_first"):
+// whole tiles dealt round-robin (wave w = tiles [w * ncta, (w + 1) * ncta)) and the rest, cut stream-K style; every CTA first
+// works through its < 1 tile share of the stream-K region --
 // the shared tiles, whose last-arriver fix-up (atomic + L2 round trip + ordered sum) then runs in the epilogue warps
 // UNDER the main loop of the following whole tile -- and ends on a whole tile with a direct epilogue.  With the pure
 // stream-K cut most CTAs END on a shared tile piece, and the fix-ups (4-6.5 us at 32 tokens, growing with T) are the
 // launch's tail.  Same tiles, same split points inside a shared tile's k-range order, same rank-ordered sums.
 struct GemmSched {
-  int n_tiles, t_tiles, KB, ncta;
+  int KB, ncta;
   int dp_waves;        // whole-tile waves
   int sk_tile0;        // first tile of the stream-K region
   long long sk_total;  // (tile, k-block) units in the stream-K region
   bool sk_first;       // stream-K region before the whole-tile waves
-  __device__ GemmSched(int n_tiles_, int t_tiles_, int KB_, int ncta_, bool sk_first_)
-      : n_tiles(n_tiles_), t_tiles(t_tiles_), KB(KB_), ncta(ncta_) {
-    const int tiles = n_tiles * t_tiles;
-    sk_first = sk_first_ && t_tiles == 1 && tiles >= ncta;
-    dp_waves = (t_tiles > 1 || sk_first) ? tiles / ncta : 0;
+  __device__ GemmSched(int tiles, int KB_, int ncta_, bool sk_first_) : KB(KB_), ncta(ncta_) {
+    sk_first = sk_first_ && tiles >= ncta;
+    dp_waves = sk_first ? tiles / ncta : 0;
     sk_tile0 = dp_waves * ncta;
     sk_total = (long long)(tiles - sk_tile0) * KB;
   }
 };
-// linear tile index -> (weight tile, token tile).  One token tile: identity.  Otherwise blocks of 8 weight tiles, token
-// tile next, weight tile fastest: 148 consecutive indices = 8 weight tiles x ~18 token tiles.
-__device__ __forceinline__ void tile_decode(const GemmSched& sc, int tile, int& n_tile, int& t_tile) {
-  if (sc.t_tiles == 1) {
-    n_tile = tile;
-    t_tile = 0;
-    return;
-  }
-  constexpr int NB = 8;
-  const int full = NB * sc.t_tiles;
-  const int nb = tile / full, rem = tile - nb * full;
-  const int nb_n = min(NB, sc.n_tiles - nb * NB);
-  t_tile = rem / nb_n;
-  n_tile = nb * NB + rem - t_tile * nb_n;
-}
 
 struct UnitIter {
   // whole tiles wave * ncta + cta for wave < dp_waves, then the contiguous range [pos, end) of the stream-K region's
@@ -271,10 +251,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
   STL_SHARE(stl_slot_smem);  // read by the other warps after the set-up barrier
   if (threadIdx.x == 0) TL(0);  // kernel entry
   const int n_tiles = (N + BNW - 1) / BNW;     // units along N
-  const int t_tiles = (T + BT - 1) / BT;
   const int KB = (K + GEMM_BK - 1) / GEMM_BK;
   const int ncta = gridDim.x, cta = blockIdx.x;
-  const GemmSched sched(n_tiles, t_tiles, KB, ncta, (stream_weights & 2) != 0);
+  const GemmSched sched(n_tiles, KB, ncta, (stream_weights & 2) != 0);
   // cluster mode, push variant: every CTA sends its partial rows straight into the OWNER's receive buffer (tokens
   // t = r (mod s) belong to rank r), ONE cluster barrier, then each owner sums its own shared memory in rank order -- no
   // remote read latency and no exit barrier (pull variant: park locally, barrier, read peers, barrier)
@@ -377,15 +356,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
       // (tile, kb) cursors advanced incrementally: no divisions on the per-k-block issue path.  A cursor walks the
       // CTA's whole tiles (wave order) and then its stream-K range; rows are re-derived only when the tile changes.
       struct Cur {
-        int wave, tile, kb, w_row, x_row;
+        int wave, tile, kb, w_row;
         int sk_left;  // sk_first: k-blocks left in the stream-K share (then the whole-tile waves)
       };
       auto cur_set_tile = [&](Cur& c, int tile) {
         c.tile = tile;
-        int n_tile, t_tile;
-        tile_decode(sched, tile, n_tile, t_tile);
-        c.w_row = n_tile * BNW;
-        c.x_row = t_tile * BT;
+        c.w_row = tile * BNW;
       };
       auto cur_init = [&](Cur& c) {
         c.wave = 0;
@@ -462,7 +438,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
           x_bar = &xfull_bar[stage];
           mbar_arrive_expect_tx(x_bar, Cfg::X_BYTES);
         }
-        tma_load_2d_hint(&xmap, x_bar, smem_x + stage * Cfg::X_BYTES, xc.kb * GEMM_BK, xc.x_row, pol_x);
+        tma_load_2d_hint(&xmap, x_bar, smem_x + stage * Cfg::X_BYTES, xc.kb * GEMM_BK, 0, pol_x);
         cur_next(xc);
         if (++stage == STAGES) {
           stage = 0;
@@ -552,10 +528,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
     int acc = 0;
     uint32_t acc_bits = 0;  // per-buffer phase parity
     while (it.next(tile, kb0, kb1, slot)) {
-      int n_tile, t_tile;
-      tile_decode(sched, tile, n_tile, t_tile);
-      const int t_base = t_tile * BT;
-      const int t_valid = min(BT, T - t_base);
+      const int n_tile = tile, t_valid = min(BT, T);
       const bool partial = (kb0 > 0) || (kb1 < KB);
       mbar_wait(&tmem_full[acc], (acc_bits >> acc) & 1);
       tc_fence_after();
@@ -581,13 +554,13 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
               for (int j = 0; j < 16; ++j) {
                 const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(r[j]), 1);
                 if ((row & 1) == 0 && n < N && c0 + j < t_valid)
-                  Y[(size_t)(t_base + c0 + j) * ldy + (n >> 1)] = glu_bf16(out_f32, __uint_as_float(r[j]), other);
+                  Y[(size_t)(c0 + j) * ldy + (n >> 1)] = glu_bf16(out_f32, __uint_as_float(r[j]), other);
               }
             } else if (n < N) {
 #pragma unroll
               for (int j = 0; j < 16; ++j)
                 if (c0 + j < t_valid) {
-                  const size_t o = (size_t)(t_base + c0 + j) * ldy + n;
+                  const size_t o = (size_t)(c0 + j) * ldy + n;
                   if (out_f32 == 1) Yf[o] = __uint_as_float(r[j]);
                   else Y[o] = __float2bfloat16_rn(ep_act(out_f32, __uint_as_float(r[j])));
                 }
@@ -691,12 +664,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
             for (int j = 0; j < FIX_T; ++j) {
               const int t = tb + 4 * j;
               if (t < t_valid) {
-                const size_t o = (size_t)(t_base + t) * ldy + n4;
+                const size_t o = (size_t)t * ldy + n4;
                 const float av[4] = {acc[j].x, acc[j].y, acc[j].z, acc[j].w};
                 if (rope.positions != nullptr) {  // qkv projection: RoPE + KV scatter (warp-uniform t and tile)
-                  qkv_rope_store(rope, nt, t_base + t, r4, av, Y + o);
+                  qkv_rope_store(rope, nt, t, r4, av, Y + o);
                 } else if (ep_glu(out_f32)) {  // fused SwiGLU / GeGLU: rows (n4, n4+1) and (n4+2, n4+3) are (gate, up) pairs
-                  __nv_bfloat16* yo = Y + (size_t)(t_base + t) * ldy + (n4 >> 1);
+                  __nv_bfloat16* yo = Y + (size_t)t * ldy + (n4 >> 1);
                   if (n4 + 1 < N) yo[0] = glu_bf16(out_f32, av[0], av[1]);
                   if (n4 + 3 < N) yo[1] = glu_bf16(out_f32, av[2], av[3]);
                 } else if (n4 + 3 < N && (ldy & 3) == 0) {
@@ -1139,7 +1112,6 @@ static cudaError_t launch_bt(const CUtensorMap& wmap, const CUtensorMap& xmap, v
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  const int t_tiles = (T + BT - 1) / BT;
   const int grid = gemm_grid_size(T, N, K, num_sms);
   // bit 0: weights are read once (evict-first); bit 1: stream-K share before the whole tiles (GemmSched::sk_first;
   // TGIS_GEMM_SK_FIRST=0: pure stream-K as in round 1).  The fused-norm consumer's transform warps assume the pure cut.
@@ -1150,7 +1122,7 @@ static cudaError_t launch_bt(const CUtensorMap& wmap, const CUtensorMap& xmap, v
     const char* e = getenv("TGIS_GEMM_SK_FIRST");
     sk_first_env = (e && e[0] == '0') ? 0 : 1;
   }
-  int stream_weights = (t_tiles == 1) ? (1 | ((sk_first_env && norm.h == nullptr && BT <= 64) ? 2 : 0)) : 0;
+  int stream_weights = 1 | ((sk_first_env && norm.h == nullptr && BT <= 64) ? 2 : 0);
   const int split = cluster_split_bt<BT, NW>(T, N, K, num_sms);
   // bit 2: push variant of the cluster reduction (receive buffer of (BT + 8) x 128 floats behind the ring; token tiles of
   // at most 32 rows, where it fits next to the full ring).  TGIS_GEMM_CLUSTER_PUSH=1 enables it (default: pull variant).
@@ -1172,7 +1144,7 @@ static cudaError_t launch_bt(const CUtensorMap& wmap, const CUtensorMap& xmap, v
     return cudaErrorInvalidValue;
   const size_t smem_bytes = (size_t)Cfg::SMEM_BYTES + (norm.h != nullptr ? (size_t)K * 2 : 0) +
                             (push ? (size_t)(BT + 8) * GEMM_BN * 4 : 0);
-  if (norm.h != nullptr && (t_tiles != 1 || BT > GEMM_NORM_MAX_T || K % GEMM_BK != 0 || NW != 1 || norm.n_parts <= 0 || norm.n_parts > GEMM_NORM_MAX_PARTS ||
+  if (norm.h != nullptr && (BT > GEMM_NORM_MAX_T || K % GEMM_BK != 0 || NW != 1 || norm.n_parts <= 0 || norm.n_parts > GEMM_NORM_MAX_PARTS ||
                             smem_bytes > (size_t)Cfg::SMEM_MAX))
     return cudaErrorInvalidValue;
   const int threads = norm.h != nullptr ? GEMM_THREADS_NORM : GEMM_THREADS;
@@ -1184,7 +1156,7 @@ static cudaError_t launch_bt(const CUtensorMap& wmap, const CUtensorMap& xmap, v
                   ldy, T, N, K, ws, counters, stream_weights, out_f32, next_wmap, nxt, 0, rope, norm);
 }
 
-// xmap must have been built with box_rows == gemm_pick_bt(T)
+// xmap must have been built with box_rows == gemm_x_box(T)
 cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int T, int N, int K,
                              float* ws, int* counters, int num_sms, cudaStream_t stream, int out_f32,
                              const CUtensorMap* next_wmap, const GemmNext* next, const GemmRope* rope, const GemmNorm* norm) {
@@ -1195,6 +1167,12 @@ cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
   GemmNext nx{};
   if (next && next_wmap) nx = *next;
   const CUtensorMap& nm = (next && next_wmap) ? *next_wmap : wmap;
+  // more than one token tile: CTA pairs (gemm_pair.cu; 1.3 to 3 times as fast at every size measured from 257 tokens on)
+  if (T > 256) {
+    if (rope != nullptr || norm != nullptr || out_f32 < 0 || out_f32 > 4) return cudaErrorInvalidValue;
+    static const int modes[5] = {PAIR_PLAIN, PAIR_PLAIN, PAIR_SWIGLU_BF16, PAIR_GEGLU, PAIR_RELU2};
+    return gemm_pair_launch(wmap, xmap, Y, ldy, out_f32 == 1, modes[out_f32], T, N, K, num_sms, stream);
+  }
   const int nw = gemm_nw(T);
 #define TGIS_GEMM_CASE(B)                                                                                              \
   return nw == 2 ? launch_bt<B, 2>(wmap, xmap, Y, ldy, T, N, K, ws, counters, num_sms, out_f32, stream, nm, nx, rp, nr) \

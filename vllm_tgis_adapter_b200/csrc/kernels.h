@@ -13,6 +13,10 @@ namespace tgis {
 int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld_elems,
                       uint32_t box_rows, uint32_t box_cols);
 int gemm_pick_bt(int T);
+constexpr int GEMM_X_BOX_MANY = 32;
+// rows of one box of the activation map: the token tile, or (more tokens than one tile) small boxes, of which the kernels
+// load as many as a tile of their choice takes
+inline int gemm_x_box(int T) { return T > 256 ? GEMM_X_BOX_MANY : gemm_pick_bt(T); }
 int gemm_nw(int T);  // weight tiles (128 rows each) per unit sharing one activation tile: 2 for decode-shaped launches
 size_t gemm_workspace_bytes(int num_sms);
 int gemm_timeline_read(unsigned long long* out64);  // debug builds (-DTGIS_GEMM_TIMELINE) only
@@ -67,6 +71,19 @@ cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
                              float* ws, int* counters, int num_sms, cudaStream_t stream, int out_f32 = 0,
                              const CUtensorMap* next_wmap = nullptr, const GemmNext* next = nullptr,
                              const GemmRope* rope = nullptr, const GemmNorm* norm = nullptr);
+
+// ---- gemm_pair.cu: the same product on CTA pairs (tcgen05 cta_group::2), thousands of tokens or expert segments ----------
+constexpr int PAIR_PLAIN = 0;        // Y[row, n] = acc
+constexpr int PAIR_SWIGLU_BF16 = 1;  // W rows interleaved (gate_j, up_j): Y[row, j] = silu(gate) * up, gate, up and silu(gate) rounded to bf16
+constexpr int PAIR_SWIGLU = 2;       // the same in fp32, rounded once
+constexpr int PAIR_GEGLU = 3;        // tanh form of gelu on the gate, fp32
+constexpr int PAIR_RELU2 = 4;        // max(acc * s, 0)^2
+constexpr int PAIR_GELU = 5;         // exact gelu
+// wmap: boxes of 128 rows x 64; xmap: boxes of GEMM_X_BOX_MANY rows x 64; Y fp32 (y_f32) or bf16
+cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int y_f32, int mode, int T, int N,
+                             int K, int num_sms, cudaStream_t stream);
+int gemm_pair_plan(int T, int N, int pairs);   // token tiles of the dense launch
+bool gemm_pair_failed();                       // a wait inside a launch of this process ran out
 
 // ---- gemm_ref.cu (debug cross-check only; never on the product path) ---------------------------------------------
 cudaError_t gemm_bf16_ref_launch(const __nv_bfloat16* X, int ldx, const __nv_bfloat16* W, void* Y, int ldy, int T,
