@@ -1,4 +1,4 @@
-"""Products of more than 256 tokens on CTA pairs (csrc/gemm_pair.cu) against 64-bit torch: token counts around the 32-token
+"""Products of more than 256 tokens and of expert segments on CTA pairs (csrc/gemm_pair.cu) against 64-bit torch: token counts around the 32-token
 unit and the 256-token tile, weight rows around the 256-row pair tile, every epilogue, and nothing written outside Y."""
 import ctypes as C
 
@@ -71,3 +71,49 @@ def test_pair_product_does_not_depend_on_the_other_tokens(lib):
     whole = run(lib, x, w, 1200, PLAIN_F32, 1200)
     part = run(lib, x[700:].contiguous(), w, 300, PLAIN_F32, 500)   # other tiles, other neighbours
     assert torch.equal(part[:300], whole[700:1000])
+
+
+ANY = dict(plain=0, swiglu=1, geglu=3, relu2=5, gelu=6)   # include/tgis_kernels.h tgis_k_gemm_any modes
+
+
+@pytest.mark.parametrize("mode", list(ANY))
+@pytest.mark.parametrize("counts,N,K,gathered", [
+    ([1], 256, 64, True), ([0, 33, 0, 31, 32], 130, 72, True), ([256, 257, 0, 1], 300, 192, False), ([700, 0, 5], 512, 264, True),
+    ([2, 3] * 40 + [0] * 20, 96, 128, True), ([0, 0, 3], 64, 64, False)])
+def test_pair_expert_segments(lib, counts, N, K, gathered, mode):
+    """One weight matrix per row segment: empty, single-row and ragged segments, rows gathered through an index list (two
+    places per row) or in place; bf16 results, and the plain sums in fp32 too."""
+    gen = torch.Generator(device="cuda").manual_seed(N + K + len(counts))
+    E, rows = len(counts), sum(counts)
+    seg = torch.tensor([0] + counts, device="cuda").cumsum(0).int()
+    expert = torch.repeat_interleave(torch.arange(E, device="cuda"), torch.tensor(counts, device="cuda"))
+    x = torch.randn((rows + 1) // 2 if gathered else rows, K, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(E, N, K, generator=gen, device="cuda") * K ** -0.5).bfloat16()
+    order = torch.randperm(rows, generator=gen, device="cuda").int()
+    scale = torch.rand(rows, generator=gen, device="cuda") + 0.5
+    src = (order.long() // 2) if gathered else torch.arange(rows, device="cuda")
+    acc, mag = (torch.empty(rows, N, dtype=torch.float64, device="cuda") for _ in range(2))
+    for e in range(E):
+        r = expert == e
+        acc[r] = x[src[r]].double() @ w[e].double().T
+        mag[r] = x[src[r]].double().abs() @ w[e].double().abs().T
+    slack = mag * (K / 16 + 8) * 2.0 ** -23
+    if mode in ("swiglu", "geglu"):
+        act = torch.nn.functional.silu if mode == "swiglu" else (lambda v: torch.nn.functional.gelu(v, approximate="tanh"))
+        g, u = acc[:, 0::2], acc[:, 1::2]
+        ref = act(g) * u
+        tol = 1.13 * slack[:, 0::2] * u.abs() + g.abs() * slack[:, 1::2] + 1e-6 * g.abs() * u.abs()   # |act'| <= 1.13
+    elif mode == "relu2":
+        s = (scale[order.long()] if gathered else scale).double()[:, None]
+        ref, tol = (acc * s).clamp(min=0) ** 2, (2 * (acc * s).abs() + slack * s) * slack * s
+    else:
+        ref = torch.nn.functional.gelu(acc) if mode == "gelu" else acc
+        tol = 1.13 * slack + (1e-6 * acc.abs() if mode == "gelu" else 0)
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    for y_dt in ([1, 0] if mode == "plain" else [1]):
+        y = torch.full((rows + 1, ref.shape[1]), 7.0, device="cuda", dtype=torch.bfloat16 if y_dt else torch.float32)
+        assert lib.tgis_k_gemm_any(p(x), p(w), p(y), 1, 1, y_dt, rows, N, K, K, K, y.shape[1], 1, 0, 0, 0, p(seg), E, N * K,
+                                   p(order) if gathered else None, 2, ANY[mode], p(scale) if mode == "relu2" else None, 0) == 0, lib.tgis_k_last_error()
+        over = (y[:rows].double() - ref).abs() - tol - (2.0 ** -8 * ref.abs() if y_dt else 0)
+        assert float(over.max()) <= 0, float(over.max())
+        assert bool((y[rows] == 7.0).all())

@@ -1830,6 +1830,7 @@ struct tgis_engine {
     pnx_yS = pnx_alloc<float>(T * W);
     pnx_actE = pnx_alloc_dt(T * m_top * m_ff, true);
     pnx_yE = pnx_alloc<float>(T * m_top * W);
+    pnx_yE_bytes = (size_t)T * m_top * W * sizeof(float);
     pnx_last = pnx_alloc_dt(std::max<size_t>(logit_rows_cap, T) * W, true);
     flx_f1 = pnx_alloc<float>(T * m_f1);
     flx_f2 = pnx_alloc<float>(T * m_f2);
@@ -2340,6 +2341,7 @@ struct tgis_engine {
   std::unordered_map<const void*, CUtensorMap> pnx_wmaps;
   std::unordered_map<uint64_t, CUtensorMap> pnx_xmaps;
   bool pnx_tc = true;
+  size_t pnx_yE_bytes = 0;
   size_t pnx_rows_alloc = 0;  // rows of every activation buffer (>= 256: a TMA box never leaves the allocation)
   bool pnx_gemm_tc(const void* X, const void* Wt, void* Y, int ldy, int T, int N, int K, int out_mode) {
     auto wit = pnx_wmaps.find(Wt);
@@ -2360,6 +2362,13 @@ struct tgis_engine {
                         on_side_stream ? gemm_counters2.p : gemm_counters.p, num_sms, on_side_stream ? stream2 : stream, out_mode));
     ++n_launches;
     return true;
+  }
+  // the experts' first product; its gathered input rows are laid out in the buffer that the second one writes
+  void experts_up(GemmAny& a) {
+    a.gather_ws = pnx_yE;
+    a.gather_ws_bytes = pnx_yE_bytes;
+    CK(gemm_any_launch(a, stream));
+    if (gemm_pair_takes_groups(a)) ++n_launches;  // (the rows' own launch)
   }
   void pnx_gemm(const void* X, int x_dt, int ldx, const void* Wt, void* Y, int y_dt, int ldy, int T, int N, int K,
                 int mode = GEMM_ANY_PLAIN, bool x_tma_ok = true) {
@@ -2577,7 +2586,7 @@ struct tgis_engine {
         a.T = T * top; a.N = ff; a.K = W; a.ldx = W; a.ldw = W; a.ldy = ff;
         a.batch = 1; a.seg_off = pnx_segoff; a.n_groups = E; a.w_gs = (long long)ff * W;
         a.gather = pnx_order; a.gather_div = top; a.mode = GEMM_ANY_RELU2; a.row_scale = pnx_mixw;
-        CK(gemm_any_launch(a, stream));
+        experts_up(a);
         GemmAny b{};
         b.X = pnx_actE; b.W = l.w_d_e; b.Y = pnx_yE;
         b.x_dtype = A; b.w_dtype = A; b.y_dtype = DT_F32;
@@ -2818,7 +2827,7 @@ struct tgis_engine {
           a.T = T * top; a.N = ff; a.K = W; a.ldx = W; a.ldw = W; a.ldy = ff;
           a.batch = 1; a.seg_off = pnx_segoff; a.n_groups = E; a.w_gs = (long long)ff * W;
           a.gather = pnx_order; a.gather_div = top; a.mode = GEMM_ANY_GELU;
-          CK(gemm_any_launch(a, stream));
+          experts_up(a);
           GemmAny b{};
           b.X = pnx_actE; b.W = l.w_d_e; b.Y = pnx_yE;
           b.x_dtype = A; b.w_dtype = A; b.y_dtype = DT_F32;
@@ -2977,7 +2986,7 @@ struct tgis_engine {
         a.T = T * top; a.N = 2 * ff; a.K = W; a.ldx = W; a.ldw = W; a.ldy = ff;
         a.batch = 1; a.seg_off = l.tab.seg_off; a.n_groups = s.experts; a.w_gs = (long long)2 * ff * W;
         a.gather = l.tab.order; a.gather_div = top; a.mode = GEMM_ANY_SWIGLU;
-        CK(gemm_any_launch(a, stream));
+        experts_up(a);
         GemmAny b{};
         b.X = pnx_actE; b.W = l.w_d_e; b.Y = pnx_yE;
         b.x_dtype = A; b.w_dtype = A; b.y_dtype = DT_F32;
@@ -3116,7 +3125,7 @@ struct tgis_engine {
           a.T = T * top; a.N = 2 * ff; a.K = W; a.ldx = W; a.ldw = W; a.ldy = ff;
           a.batch = 1; a.seg_off = pnx_segoff; a.n_groups = E; a.w_gs = (long long)2 * ff * W;
           a.gather = pnx_order; a.gather_div = top; a.mode = GEMM_ANY_SWIGLU;
-          CK(gemm_any_launch(a, stream));
+          experts_up(a);
           GemmAny b{};
           b.X = pnx_actE; b.W = l.w_d_e; b.Y = pnx_yE;
           b.x_dtype = A; b.w_dtype = A; b.y_dtype = DT_F32;

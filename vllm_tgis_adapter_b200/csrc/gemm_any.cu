@@ -11,7 +11,7 @@
 // Every output element is the sum over k = 0 .. K-1 in ascending order inside one thread, so a row's result depends
 // neither on the other rows of the launch nor on where in a segment it landed.
 //
-// Three kernels: a handful of outputs over long rows (router and gate projections of a decode step) take one warp per
+// Kernels: grouped bf16 products run on CTA pairs where their rows allow it (gemm_pair.cu); a handful of outputs over long rows (router and gate projections of a decode step) take one warp per
 // output (gemm_any_rowdot_kernel); bf16 operands whose rows start on 16-byte boundaries run on the tensor cores
 // (gemm_any_mma_kernel);
 // everything else -- fp32 operands, odd leading dimensions -- runs on the FMA pipe (a [16 TM x 64] tile per 256-thread CTA,
@@ -430,6 +430,9 @@ cudaError_t gemm_any_launch(const GemmAny& a, cudaStream_t stream) {
     }
     return a.w_dtype == DT_BF16 ? launch_rowdot<float, bf>(a, stream) : launch_rowdot<float, float>(a, stream);
   }
+  // expert segments: CTA pairs.  64 experts of 2 x 1408 x 2048 and back, top 6, both products in microseconds, mma.sync -> pairs:
+  // 4 tokens 126 -> 78, 32 tokens 260 -> 165 (6.3 TB/s of weights), 512 tokens 334 -> 195, 2048 tokens 1003 -> 243
+  if (gemm_pair_takes_groups(a)) return gemm_pair_grouped_launch(a, stream);
   if (mma_eligible(a)) return a.y_dtype == DT_BF16 ? launch_mma<bf>(a, stream) : launch_mma<float>(a, stream);
   const int key = a.x_dtype * 4 + a.w_dtype * 2 + a.y_dtype;  // DT_F32 = 0, DT_BF16 = 1
   switch (key) {

@@ -15,7 +15,8 @@
 //    (gemm_pair_plan); no tile is ever split along k, so there is no reduction between CTAs and an output is one sum in
 //    ascending k whatever the launch;
 //  * grouped products (one row segment per expert): a segment is cut into equal tiles of at most 256 rows, a segment of 40
-//    rows costs 64 columns.  The tile list is derived from the segment offsets on the device.
+//    rows costs 64 columns.  The tile list is derived from the segment offsets on the device.  In a decode step (three rows
+//    an expert) the launch streams the experts' weights at HBM rate, with thousands of tokens it is bound like the dense one.
 //
 // Roles per CTA: warp 0 TMA producer, warp 1 MMA issuer (leader CTA only) and TMEM owner, warps 2..5 epilogue on a double
 // buffered accumulator (2 x 256 columns).  The leader's `full` barrier counts both CTAs' bytes; tcgen05.commit releases a
@@ -481,6 +482,63 @@ cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
   a.x_tiles = gemm_pair_plan(T, N, pairs);
   const int tiles = a.n_tiles * a.x_tiles;
   return launch_pair<false>(wmap, xmap, a, 2 * (tiles < pairs ? tiles : pairs), stream);
+}
+
+// X rows of a grouped product in segment order: out[p] = X[gather[p] / div], p < seg_off[n_groups]
+__global__ void __launch_bounds__(256) gather_segment_rows_kernel(const uint4* __restrict__ X, int ldx16, const int* __restrict__ gather, int div,
+                                                                  const int* __restrict__ seg_end, uint4* __restrict__ out, int row16) {
+  griddep_launch();
+  griddep_wait();
+  const int p = blockIdx.x;
+  if (p >= *seg_end) return;
+  const uint4* src = X + (size_t)(gather[p] / div) * ldx16;
+  uint4* dst = out + (size_t)p * row16;
+  for (int c = threadIdx.x; c < row16; c += 256) dst[c] = src[c];
+}
+
+// Whether a grouped product runs here.  The operands' rows start on 16-byte boundaries and the segments' weight matrices lie
+// one behind the other (one tensor map covers them); gathered rows need room to be laid out in segment order first
+// (12288 rows x 2048: 16 us against 660 us for the product that read them one by one).
+bool gemm_pair_takes_groups(const GemmAny& a) {
+  auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  const bool mode_ok = a.mode == GEMM_ANY_PLAIN || (a.y_dtype == DT_BF16 && (a.mode == GEMM_ANY_SWIGLU || a.mode == GEMM_ANY_GEGLU ||
+                                                                            a.mode == GEMM_ANY_RELU2 || a.mode == GEMM_ANY_GELU));
+  return mode_ok && a.seg_off != nullptr && a.batch <= 1 && a.x_dtype == DT_BF16 && a.w_dtype == DT_BF16 && a.n_groups >= 1 &&
+         a.n_groups <= PAIR_MAX_GROUPS && a.w_gs == (long long)a.N * a.ldw && (long long)a.n_groups * a.N < (1ll << 31) && a.K >= PAIR_BK &&
+         a.K % 8 == 0 && a.ldx % 8 == 0 && a.ldw % 8 == 0 && a.ldx >= a.K && a.ldw >= a.K && al16(a.X) && al16(a.W) &&
+         (a.gather == nullptr || (a.gather_div > 0 && al16(a.gather_ws) && a.gather_ws != nullptr && a.gather_ws_bytes >= (size_t)a.T * a.K * 2));
+}
+
+cudaError_t gemm_pair_grouped_launch(const GemmAny& g, cudaStream_t stream) {
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const void* X = g.X;
+  int ldx = g.ldx;
+  if (g.gather != nullptr) {
+    e = launch_k(gather_segment_rows_kernel, dim3(g.T), dim3(256), 0, stream, (const uint4*)g.X, g.ldx / 8, g.gather, g.gather_div,
+                 g.seg_off + g.n_groups, (uint4*)g.gather_ws, g.K / 8);
+    if (e != cudaSuccess) return e;
+    X = g.gather_ws;
+    ldx = g.K;
+  }
+  CUtensorMap wm, xm;
+  if (make_tmap_bf16_2d(&wm, g.W, (uint64_t)g.n_groups * g.N, g.K, g.ldw, 128, PAIR_BK) != 0 ||
+      make_tmap_bf16_2d(&xm, X, g.T, g.K, ldx, GEMM_X_BOX_MANY, PAIR_BK) != 0)
+    return cudaErrorInvalidValue;
+  PairArgs a{};
+  a.Y = g.Y; a.ldy = g.ldy; a.T = g.T; a.N = g.N; a.K = g.K;
+  a.y_f32 = g.y_dtype == DT_F32;
+  a.mode = g.mode == GEMM_ANY_SWIGLU ? PAIR_SWIGLU : g.mode == GEMM_ANY_GEGLU ? PAIR_GEGLU : g.mode == GEMM_ANY_RELU2 ? PAIR_RELU2
+           : g.mode == GEMM_ANY_GELU ? PAIR_GELU : PAIR_PLAIN;
+  a.n_tiles = (g.N + 255) / 256;
+  a.seg_off = g.seg_off; a.n_groups = g.n_groups;
+  a.row_scale = g.row_scale; a.gather = g.gather;
+  const int pairs = sms / 2;
+  // at most one tile per started 256 rows of every segment: fewer tiles than pairs leave the rest without work
+  const long long most = (long long)a.n_tiles * (g.T / 256 + (g.n_groups < g.T ? g.n_groups : g.T));
+  return launch_pair<true>(wm, xm, a, 2 * (int)(most < pairs ? (most < 1 ? 1 : most) : pairs), stream);
 }
 
 }  // namespace tgis

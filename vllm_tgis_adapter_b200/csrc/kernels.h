@@ -275,7 +275,10 @@ struct GemmAny {
   int gather_div;
   int mode;                        // GEMM_ANY_*
   const float* row_scale; int scale_ld;
+  void* gather_ws; size_t gather_ws_bytes;  // room for the gathered rows in segment order (T x K elements), or nullptr
 };
+bool gemm_pair_takes_groups(const GemmAny& a);   // gemm_pair.cu
+cudaError_t gemm_pair_grouped_launch(const GemmAny& a, cudaStream_t stream);
 cudaError_t gemm_any_launch(const GemmAny& a, cudaStream_t stream);
 
 // ---- norms over an fp32 residual stream (elementwise.cu) ------------------------------------------------------------

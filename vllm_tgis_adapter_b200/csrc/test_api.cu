@@ -522,6 +522,11 @@ int tgis_k_gemm_any(const void* x, const void* w, void* y, int32_t x_dt, int32_t
   a.batch = batch; a.x_bs = x_bs; a.w_bs = w_bs; a.y_bs = y_bs;
   a.seg_off = seg_off_dev; a.n_groups = n_groups; a.w_gs = w_gs; a.gather = gather_dev; a.gather_div = gather_div;
   a.mode = mode; a.row_scale = row_scale; a.scale_ld = scale_ld;
+  Tmp<bf16> ws;
+  if (gather_dev != nullptr && x_dt == DT_BF16) {
+    KCK(ws.alloc((size_t)T * K));
+    a.gather_ws = ws.p; a.gather_ws_bytes = (size_t)T * K * sizeof(bf16);
+  }
   KCK(gemm_any_launch(a, 0));
   KCK(cudaDeviceSynchronize());
   return 0;
