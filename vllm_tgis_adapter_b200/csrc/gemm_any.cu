@@ -8,15 +8,14 @@
 // and seven epilogues (plain store, SwiGLU or GeGLU over interleaved gate/up rows, per-(row, batch) scale, tanh, squared ReLU of
 // the row-scaled sum, exact gelu).
 //
-// Every output element is the sum over k = 0 .. K-1 in ascending order inside one thread, so a row's result depends
-// neither on the other rows of the launch nor on where in a segment it landed.
+// Every output element is a sum in an order of k that only K and the kernel fix, so a row's result depends neither on the
+// other rows of the launch nor on where in a segment it landed.
 //
-// Kernels: grouped bf16 products run on CTA pairs where their rows allow it (gemm_pair.cu); a handful of outputs over long rows (router and gate projections of a decode step) take one warp per
-// output (gemm_any_rowdot_kernel); bf16 operands whose rows start on 16-byte boundaries run on the tensor cores
-// (gemm_any_mma_kernel);
-// everything else -- fp32 operands, odd leading dimensions -- runs on the FMA pipe (a [16 TM x 64] tile per 256-thread CTA,
-// TM x 4 outputs per thread, k-blocks of 16 staged through shared memory).  Dense launches that fit the tcgen05 kernel's
-// operand layout are routed there by the engine.
+// Kernels: grouped bf16 products run on CTA pairs where their rows allow it (gemm_pair.cu); a handful of outputs over long
+// rows (router and gate projections of a decode step) take one warp per output (gemm_any_rowdot_kernel); bf16 operands whose
+// rows start on 16-byte boundaries run on the tensor cores (gemm_any_mma_kernel); everything else -- fp32 operands, odd
+// leading dimensions -- runs on the FMA pipe (gemm_any_kernel).  Dense launches that fit the tcgen05 kernels' operand layout
+// are routed there by the engine.
 #include <cstdint>
 #include <cstdlib>
 
@@ -28,8 +27,6 @@ namespace tgis {
 namespace {
 
 constexpr int ANY_THREADS = 256;
-constexpr int ANY_BN = 64;
-constexpr int ANY_BK = 16;
 
 template <class T>
 __device__ __forceinline__ float ld_as_float(const T* p);
@@ -55,11 +52,48 @@ __device__ __forceinline__ float relu2_row_scale(const GemmAny& a, int dst) {
   return a.row_scale == nullptr ? 1.f : a.row_scale[a.gather != nullptr ? a.gather[dst] : dst];
 }
 
-template <class XT, class WT, class OT, int TM>
-__global__ void __launch_bounds__(ANY_THREADS) gemm_any_kernel(GemmAny a) {
-  constexpr int BM = 16 * TM;
-  __shared__ __align__(16) float Xs[ANY_BK][BM + 4];
-  __shared__ __align__(16) float Ws[ANY_BK][ANY_BN + 4];
+// ---- FMA pipe: fp32 operands (true fp32), fp32 activations under bf16 weights, odd leading dimensions -----------------
+// CTA tile BM x 64 of 128 threads (8 x 16), a thread owns rows ty + 8 i and columns tx + 16 j.  Bound by the FMA pipe: operands
+// are kept in shared memory as they lie in memory ([row][k], rows padded to 36 floats so that eight neighbouring rows start
+// in different bank groups), a thread reads four k of a row with one 16-byte load, and both halves of a packed
+// multiply-add take neighbouring k: an output is the sum over even k plus the sum over odd k, each in ascending order, which
+// no other row and no tile height enters.  BM / 8 + 4 loads feed BM packed multiply-adds of two k each.  The next k-block's
+// global loads (16 bytes each where the rows allow it) are in flight while this one is worked on.
+// Measured, fp32, T x N x K (before: scalar staging, one 16-byte and several 4-byte shared loads for 16 multiply-adds, nothing
+// in flight): 389 x 1088 x 1024 149 -> 40 us, 16 experts of 2048 x 1024 under 778 rows 296 -> 130 us, 10 x 32768 x 1024 189 -> 59 us,
+// 16 x 1024 x 1024 93 -> 25 us; 40 TFLOP/s where there are tiles enough (of 74: the shared-memory loads take the rest).
+constexpr int FMA_THREADS = 128;
+constexpr int FMA_BN = 64, FMA_BK = 32, FMA_LD = FMA_BK + 4;
+constexpr int FMA_SMS = 148;
+
+__device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long x, unsigned long long y) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(x), "l"(y));
+}
+__device__ __forceinline__ float sum2(unsigned long long v) {
+  return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32));
+}
+template <bool VEC>
+__device__ __forceinline__ float4 ld4(const float* p, int left) {   // `left` elements of the row from p on
+  if constexpr (VEC) return left > 0 ? *reinterpret_cast<const float4*>(p) : make_float4(0.f, 0.f, 0.f, 0.f);
+  return make_float4(left > 0 ? p[0] : 0.f, left > 1 ? p[1] : 0.f, left > 2 ? p[2] : 0.f, left > 3 ? p[3] : 0.f);
+}
+template <bool VEC>
+__device__ __forceinline__ float4 ld4(const __nv_bfloat16* p, int left) {
+  if constexpr (VEC) {
+    if (left <= 0) return make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+  }
+  return make_float4(left > 0 ? __bfloat162float(p[0]) : 0.f, left > 1 ? __bfloat162float(p[1]) : 0.f, left > 2 ? __bfloat162float(p[2]) : 0.f,
+                     left > 3 ? __bfloat162float(p[3]) : 0.f);
+}
+
+template <class XT, class WT, class OT, int BM, bool VEC>
+__global__ void __launch_bounds__(FMA_THREADS) gemm_any_kernel(GemmAny a) {
+  constexpr int TM = BM / 8, TN = FMA_BN / 16;
+  constexpr int XV = BM * FMA_BK / 4 / FMA_THREADS, WV = FMA_BN * FMA_BK / 4 / FMA_THREADS;   // 4-element pieces a thread stages
+  __shared__ __align__(16) float Xs[2][BM * FMA_LD];
+  __shared__ __align__(16) float Ws[2][FMA_BN * FMA_LD];
   __shared__ int row_src[BM], row_dst[BM];
   griddep_launch();
   griddep_wait();
@@ -93,68 +127,89 @@ __global__ void __launch_bounds__(ANY_THREADS) gemm_any_kernel(GemmAny a) {
   const XT* X = reinterpret_cast<const XT*>(a.X) + (size_t)z * a.x_bs;
   const WT* W = reinterpret_cast<const WT*>(a.W) + (size_t)z * a.w_bs + (size_t)group * a.w_gs;
   OT* Y = reinterpret_cast<OT*>(a.Y) + (size_t)z * a.y_bs;
-  const int n0 = blockIdx.x * ANY_BN;
+  const int n0 = blockIdx.x * FMA_BN;
   const int ty = tid / 16, tx = tid % 16;
-  float acc[TM][4];
+
+  // pieces of four k: piece e -> row e / 8, k 4 (e % 8)
+  const int pk = (tid & 7) * 4, pr = tid >> 3;
+  const XT* xp[XV];
+  const WT* wp[WV];
+#pragma unroll
+  for (int i = 0; i < XV; ++i) {
+    const int src = row_src[pr + i * (FMA_THREADS / 8)];
+    xp[i] = src >= 0 ? X + (size_t)src * a.ldx + pk : nullptr;
+  }
+#pragma unroll
+  for (int i = 0; i < WV; ++i) {
+    const int n = n0 + pr + i * (FMA_THREADS / 8);
+    wp[i] = n < a.N ? W + (size_t)n * a.ldw + pk : nullptr;
+  }
+  float4 xv[XV], wv[WV];
+  auto fetch = [&](int k0) {
+    const int left = a.K - k0 - pk;
+#pragma unroll
+    for (int i = 0; i < XV; ++i) xv[i] = ld4<VEC>(xp[i] + k0, xp[i] != nullptr ? left : 0);
+#pragma unroll
+    for (int i = 0; i < WV; ++i) wv[i] = ld4<VEC>(wp[i] + k0, wp[i] != nullptr ? left : 0);
+  };
+  auto put = [&](int buf) {
+#pragma unroll
+    for (int i = 0; i < XV; ++i) *reinterpret_cast<float4*>(&Xs[buf][(pr + i * (FMA_THREADS / 8)) * FMA_LD + pk]) = xv[i];
+#pragma unroll
+    for (int i = 0; i < WV; ++i) *reinterpret_cast<float4*>(&Ws[buf][(pr + i * (FMA_THREADS / 8)) * FMA_LD + pk]) = wv[i];
+  };
+  unsigned long long acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
 
-  for (int k0 = 0; k0 < a.K; k0 += ANY_BK) {
-    // stage the two operand tiles (k fastest in memory; transposed into [k][row] so the FMA loop reads rows of 4)
-    for (int e = tid; e < BM * ANY_BK; e += ANY_THREADS) {
-      const int r = e / ANY_BK, k = e % ANY_BK;
-      const int src = row_src[r];
-      float v = 0.f;
-      if (src >= 0 && k0 + k < a.K) v = ld_as_float(X + (size_t)src * a.ldx + k0 + k);
-      Xs[k][r] = v;
-    }
-    for (int e = tid; e < ANY_BN * ANY_BK; e += ANY_THREADS) {
-      const int n = e / ANY_BK, k = e % ANY_BK;
-      float v = 0.f;
-      if (n0 + n < a.N && k0 + k < a.K) v = ld_as_float(W + (size_t)(n0 + n) * a.ldw + k0 + k);
-      Ws[k][n] = v;
-    }
-    __syncthreads();
+  fetch(0);
+  put(0);
+  __syncthreads();
+  const int KB = (a.K + FMA_BK - 1) / FMA_BK;
+  for (int kb = 0; kb < KB; ++kb) {
+    const int cur = kb & 1;
+    if (kb + 1 < KB) fetch((kb + 1) * FMA_BK);
+    const float* xs = &Xs[cur][ty * FMA_LD];
+    const float* ws = &Ws[cur][tx * FMA_LD];
 #pragma unroll
-    for (int k = 0; k < ANY_BK; ++k) {
-      float xa[TM];
+    for (int k = 0; k < FMA_BK; k += 4) {
+      ulonglong2 w2[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) xa[i] = Xs[k][ty * TM + i];
-      const float4 wb = *reinterpret_cast<const float4*>(&Ws[k][tx * 4]);
+      for (int j = 0; j < TN; ++j) w2[j] = *reinterpret_cast<const ulonglong2*>(ws + j * 16 * FMA_LD + k);
 #pragma unroll
       for (int i = 0; i < TM; ++i) {
-        acc[i][0] = fmaf(xa[i], wb.x, acc[i][0]);
-        acc[i][1] = fmaf(xa[i], wb.y, acc[i][1]);
-        acc[i][2] = fmaf(xa[i], wb.z, acc[i][2]);
-        acc[i][3] = fmaf(xa[i], wb.w, acc[i][3]);
+        const ulonglong2 x2 = *reinterpret_cast<const ulonglong2*>(xs + i * 8 * FMA_LD + k);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+          fma2(acc[i][j], x2.x, w2[j].x);
+          fma2(acc[i][j], x2.y, w2[j].y);
+        }
       }
     }
-    __syncthreads();
+    if (kb + 1 < KB) {
+      put(cur ^ 1);   // (last read two k-blocks ago, before the barrier below)
+      __syncthreads();
+    }
   }
-  // ---- epilogue
+  // ---- epilogue: a thread's columns are 16 apart; gate and up of a pair sit in neighbouring threads
+  const bool glu = a.mode == GEMM_ANY_SWIGLU || a.mode == GEMM_ANY_GEGLU;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
-    const int dst = row_dst[ty * TM + i];
-    if (dst < 0) continue;
-    const int n = n0 + tx * 4;
-    if (a.mode == GEMM_ANY_SWIGLU || a.mode == GEMM_ANY_GEGLU) {
-      // columns (2j, 2j + 1) = (gate_j, up_j): out[j] = act(gate) * up
+    const int dst = row_dst[ty + 8 * i];
+    const float s = dst < 0 ? 1.f : a.mode == GEMM_ANY_ROWSCALE ? a.row_scale[(size_t)dst * a.scale_ld + z] : a.mode == GEMM_ANY_RELU2 ? relu2_row_scale(a, dst) : 1.f;
 #pragma unroll
-      for (int j = 0; j < 4; j += 2) {
-        if (n + j + 1 < a.N) st_from_float(Y + (size_t)dst * a.ldy + (n + j) / 2, glu_pair(a.mode, acc[i][j], acc[i][j + 1]));
+    for (int j = 0; j < TN; ++j) {
+      const int n = n0 + tx + 16 * j;
+      const float v = sum2(acc[i][j]);
+      if (glu) {   // columns (2c, 2c + 1) = (gate_c, up_c): out[c] = act(gate) * up
+        const float up = __shfl_down_sync(0xffffffffu, v, 1);
+        if ((tx & 1) == 0 && dst >= 0 && n + 1 < a.N) st_from_float(Y + (size_t)dst * a.ldy + n / 2, glu_pair(a.mode, v, up));
+      } else if (dst >= 0 && n < a.N) {
+        const float o = a.mode == GEMM_ANY_RELU2 ? relu2_scaled(v, s) : a.mode == GEMM_ANY_TANH ? tanhf(v) : a.mode == GEMM_ANY_GELU ? gelu_erf(v) : v * s;
+        st_from_float(Y + (size_t)dst * a.ldy + n, o);
       }
-    } else if (a.mode == GEMM_ANY_RELU2) {
-      const float s = relu2_row_scale(a, dst);
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (n + j < a.N) st_from_float(Y + (size_t)dst * a.ldy + n + j, relu2_scaled(acc[i][j], s));
-    } else {
-      const float s = a.mode == GEMM_ANY_ROWSCALE ? a.row_scale[(size_t)dst * a.scale_ld + z] : 1.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (n + j < a.N) st_from_float(Y + (size_t)dst * a.ldy + n + j, a.mode == GEMM_ANY_TANH ? tanhf(acc[i][j]) : a.mode == GEMM_ANY_GELU ? gelu_erf(acc[i][j]) : acc[i][j] * s);
     }
   }
 }
@@ -401,17 +456,28 @@ cudaError_t launch_rowdot(const GemmAny& a, cudaStream_t stream) {
                   dim3(ANY_THREADS), 0, stream, a);
 }
 
-template <class XT, class WT, class OT>
-cudaError_t launch_tm(const GemmAny& a, cudaStream_t stream) {
-  // rows per tile: 16 for skinny problems (decode steps, small expert segments), 64 otherwise
-  const int rows = a.seg_off != nullptr ? (a.T + a.n_groups - 1) / (a.n_groups > 0 ? a.n_groups : 1) : a.T;
-  const bool small = rows <= 24;
-  const int BM = small ? 16 : 64;
+template <class XT, class WT, class OT, int BM>
+cudaError_t launch_fma_bm(const GemmAny& a, bool vec, cudaStream_t stream) {
   const int row_tiles = a.seg_off != nullptr ? (a.T + BM - 1) / BM + a.n_groups : (a.T + BM - 1) / BM;
-  const dim3 grid((a.N + ANY_BN - 1) / ANY_BN, row_tiles, a.batch > 0 ? a.batch : 1);
+  const dim3 grid((a.N + FMA_BN - 1) / FMA_BN, row_tiles, a.batch > 0 ? a.batch : 1);
   if (grid.y > 65535 || grid.z > 65535) return cudaErrorInvalidValue;
-  if (small) return launch_k(gemm_any_kernel<XT, WT, OT, 1>, grid, dim3(ANY_THREADS), 0, stream, a);
-  return launch_k(gemm_any_kernel<XT, WT, OT, 4>, grid, dim3(ANY_THREADS), 0, stream, a);
+  return vec ? launch_k(gemm_any_kernel<XT, WT, OT, BM, true>, grid, dim3(FMA_THREADS), 0, stream, a)
+             : launch_k(gemm_any_kernel<XT, WT, OT, BM, false>, grid, dim3(FMA_THREADS), 0, stream, a);
+}
+template <class XT, class WT, class OT>
+cudaError_t launch_fma(const GemmAny& a, cudaStream_t stream) {
+  // four elements per load: rows, problems and segments start on a multiple of four elements' bytes, K is a multiple of four
+  auto al = [](const void* p, size_t esz) { return (reinterpret_cast<uintptr_t>(p) & (4 * esz - 1)) == 0; };
+  const bool vec = a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && a.x_bs % 4 == 0 && a.w_bs % 4 == 0 && a.w_gs % 4 == 0 &&
+                   al(a.X, sizeof(XT)) && al(a.W, sizeof(WT));
+  // rows per tile: 16 for skinny problems (decode steps, small segments); 64 where that makes three tiles for every SM, else 32
+  // (K = 1024: 389 x 2048 57 us with 32 rows, 66 with 64; 2048 x 4096 478 and 431)
+  const int rows = a.seg_off != nullptr ? (a.T + a.n_groups - 1) / (a.n_groups > 0 ? a.n_groups : 1) : a.T;
+  const long long tiles64 = (long long)((a.N + FMA_BN - 1) / FMA_BN) * (a.batch > 0 ? a.batch : 1) *
+                            (a.seg_off != nullptr ? (long long)a.n_groups * ((rows + 63) / 64) : (a.T + 63) / 64);
+  if (rows <= 20) return launch_fma_bm<XT, WT, OT, 16>(a, vec, stream);
+  if (rows <= 36 || tiles64 < 3 * FMA_SMS || a.K <= 256) return launch_fma_bm<XT, WT, OT, 32>(a, vec, stream);
+  return launch_fma_bm<XT, WT, OT, 64>(a, vec, stream);
 }
 
 }  // namespace
@@ -436,11 +502,11 @@ cudaError_t gemm_any_launch(const GemmAny& a, cudaStream_t stream) {
   if (mma_eligible(a)) return a.y_dtype == DT_BF16 ? launch_mma<bf>(a, stream) : launch_mma<float>(a, stream);
   const int key = a.x_dtype * 4 + a.w_dtype * 2 + a.y_dtype;  // DT_F32 = 0, DT_BF16 = 1
   switch (key) {
-    case 0: return launch_tm<float, float, float>(a, stream);
-    case 2: return launch_tm<float, bf, float>(a, stream);
-    case 3: return launch_tm<float, bf, bf>(a, stream);
-    case 6: return launch_tm<bf, bf, float>(a, stream);
-    case 7: return launch_tm<bf, bf, bf>(a, stream);
+    case 0: return launch_fma<float, float, float>(a, stream);
+    case 2: return launch_fma<float, bf, float>(a, stream);
+    case 3: return launch_fma<float, bf, bf>(a, stream);
+    case 6: return launch_fma<bf, bf, float>(a, stream);
+    case 7: return launch_fma<bf, bf, bf>(a, stream);
     default: return cudaErrorInvalidValue;  // (fp32 weights under bf16 activations are not a combination any model uses)
   }
 }
