@@ -2359,7 +2359,7 @@ struct tgis_engine {
       xit = pnx_xmaps.emplace(xkey, m).first;
     }
     CK(gemm_bf16_launch(wit->second, xit->second, Y, ldy, T, N, K, on_side_stream ? gemm_ws2.p : gemm_ws.p,
-                        on_side_stream ? gemm_counters2.p : gemm_counters.p, num_sms, on_side_stream ? stream2 : stream, out_mode));
+                        on_side_stream ? gemm_counters2.p : gemm_counters.p, num_sms, on_side_stream ? stream2 : stream, out_mode, nullptr, nullptr, nullptr, nullptr, X, Wt));
     ++n_launches;
     return true;
   }
@@ -3173,7 +3173,7 @@ struct tgis_engine {
       GemmNext nx{};
       if (next_wm && l2_prefetch_kb > 0) nx = gemm_next_desc(nT, nN, nK, num_sms, l2_prefetch_kb);
       CK(gemm_bf16_launch(wm, xmaps[bt_index(T)], Y, ldy, T, N, K, gemm_ws.p, gemm_counters.p, num_sms, stream, out_f32,
-                          nx.kb_prefetch > 0 ? next_wm : nullptr, nx.kb_prefetch > 0 ? &nx : nullptr, rope, norm));
+                          nx.kb_prefetch > 0 ? next_wm : nullptr, nx.kb_prefetch > 0 ? &nx : nullptr, rope, norm, X, W));
     }
     if (pe1) CK(cudaEventRecord(pe1, stream));
     ++n_launches;

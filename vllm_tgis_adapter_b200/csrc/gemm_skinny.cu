@@ -1,0 +1,226 @@
+// Y[T, N] = X[T, K] W[N, K]^T for the few tokens of a decode step (T <= 32, bf16, K a multiple of 64).
+//
+// Such a product is bound by its weight bytes, and below some 30 MB by what a launch takes beside them: the tcgen05 kernel
+// (gemm_tcgen05.cu) sets up tensor memory and barriers, waits for TMA and reduces its k-splits across a cluster, 7 us before
+// the first 4 MB.  Here a warp loads weights straight into the A fragments of mma.sync (16-byte loads; a lane's eight
+// neighbouring k feed two MMAs, the k order inside a chunk of 64 being permuted alike in both operands), the warps of a CTA
+// split K, and one pass through shared memory adds their sums in warp order.  Weights of the first chunk are requested before
+// the previous kernel has ended, all of the CTA's weights are asked into L2.  With many weight bytes or many tokens the
+// activations, which every CTA reads again, cost more than that saves; gemm_skinny_takes draws the line.
+//
+// Measured, microseconds with cold weights, N x K, tcgen05 -> here: 1 token 768 x 768 7.0 -> 2.7, 2048 x 2048 8.7 -> 4.0,
+// 4096 x 4096 12.6 -> 8.6; 32 tokens 768 x 768 8.1 -> 3.6, 2048 x 2048 9.8 -> 5.4 (6144 x 4096 17.7 -> 20.1).
+#include "kernels.h"
+#include "launch.cuh"
+#include "ptx.cuh"
+
+namespace tgis {
+namespace {
+
+struct SkinnyArgs {
+  const __nv_bfloat16* X; const __nv_bfloat16* W; void* Y;
+  int ldy, T, N, K, mode;   // mode: the out modes of gemm_bf16_launch
+  GemmRope rope;            // positions == nullptr: none
+};
+
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint4 ldg_stream(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float skinny_glu(int mode, float g, float u) {
+  if (mode == 2) {   // rounding points of the unfused path
+    g = bf16_round(g);
+    return bf16_round(g / (1.f + expf(-g))) * bf16_round(u);
+  }
+  return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
+}
+
+// MT: 16-row weight tiles per CTA, NT: 8-token tiles, WARPS: k-splits (warp w takes the chunks w, w + WARPS, ...).
+// ROPE (MT = 2): the CTA's two tiles are the dims [16 q, 16 q + 16) of one head and their rotary partners, 64 dims on.
+template <int MT, int NT, int WARPS, bool ROPE>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_kernel(const SkinnyArgs a) {
+  constexpr int R = 16 * MT, TT = 8 * NT, LD = R + 1;
+  extern __shared__ __align__(16) float part[];   // [WARPS][TT][LD]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = ROPE ? (blockIdx.x >> 2) * HEAD_DIM + (blockIdx.x & 3) * 16 : blockIdx.x * R;
+  constexpr int M_STEP = ROPE ? 64 : 16;
+  if (threadIdx.x < MT) {   // weights are static: the CTA's rows (one run of bytes per tile) start on their way to L2
+    const int row = n0 + (int)threadIdx.x * M_STEP, bytes = min(16, a.N - row) * a.K * 2;
+    const char* from = reinterpret_cast<const char*>(a.W + (size_t)row * a.K);
+    for (int off = 0; off < bytes; off += 65536)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(from + off), "r"(min(bytes - off, 65536)) : "memory");
+  }
+  griddep_launch();
+  const int chunks = a.K / 64;
+  const __nv_bfloat16* wr[MT][2];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) wr[m][h] = a.W + (size_t)min(n0 + m * M_STEP + h * 8 + g, a.N - 1) * a.K + t * 8;
+  const __nv_bfloat16* xr[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) xr[n] = a.X + (size_t)min(n * 8 + g, a.T - 1) * a.K + t * 8;
+  float acc[MT][NT][4];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+  uint4 wv[MT][2][2];   // the next chunk
+  auto load_w = [&](int c) {
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int s = 0; s < 2; ++s) wv[m][h][s] = ldg_stream(wr[m][h] + c * 64 + s * 32);
+  };
+  if (warp < chunks) load_w(warp);   // (weights are static)
+  griddep_wait();
+  for (int c = warp; c < chunks; c += WARPS) {
+    uint4 xv[NT][2], wc[MT][2][2];
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int s = 0; s < 2; ++s) xv[n][s] = *reinterpret_cast<const uint4*>(xr[n] + c * 64 + s * 32);
+#pragma unroll
+    for (int m = 0; m < MT; ++m)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int s = 0; s < 2; ++s) wc[m][h][s] = wv[m][h][s];
+    if (c + WARPS < chunks) load_w(c + WARPS);
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          mma_16816(acc[m][n], wc[m][0][s].x, wc[m][1][s].x, wc[m][0][s].y, wc[m][1][s].y, xv[n][s].x, xv[n][s].y);
+          mma_16816(acc[m][n], wc[m][0][s].z, wc[m][1][s].z, wc[m][0][s].w, wc[m][1][s].w, xv[n][s].z, xv[n][s].w);
+        }
+  }
+  // acc[m][n]: rows g, g + 8 of weight tile m, tokens 2t, 2t + 1 of token tile n
+  float* mine = part + (size_t)warp * TT * LD;
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) mine[(n * 8 + 2 * t + (e & 1)) * LD + m * 16 + g + (e >> 1) * 8] = acc[m][n][e];
+  __syncthreads();
+  auto sum = [&](int tok, int j) {
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) v += part[((size_t)w * TT + tok) * LD + j];
+    return v;
+  };
+  __nv_bfloat16* __restrict__ Y = reinterpret_cast<__nv_bfloat16*>(a.Y);
+  if constexpr (ROPE) {
+    // rotary embedding and the scatter into the paged cache (arithmetic and rounding points of rope_kvwrite_kernel)
+    const int head = n0 / HEAD_DIM, d0 = n0 % HEAD_DIM;
+    for (int i = threadIdx.x; i < a.T * 16; i += WARPS * 32) {
+      const int tok = i >> 4, j = i & 15, d = d0 + j;
+      float lo = bf16_round(sum(tok, j)), hi = bf16_round(sum(tok, 16 + j));
+      if (head < a.rope.n_q + a.rope.n_kv) {
+        const __nv_bfloat16* cs = a.rope.cos_sin + (size_t)a.rope.positions[tok] * HEAD_DIM + d;
+        const float c = __bfloat162float(cs[0]), s = __bfloat162float(cs[64]), l = lo, h = hi;
+        lo = bf16_round(l * c) - bf16_round(h * s);
+        hi = bf16_round(h * c) + bf16_round(l * s);
+      }
+      const __nv_bfloat16 out[2] = {__float2bfloat16_rn(lo), __float2bfloat16_rn(hi)};
+      __nv_bfloat16* y = Y + (size_t)tok * a.ldy + n0 + j;
+      y[0] = out[0];
+      y[64] = out[1];
+      const int slot = head >= a.rope.n_q ? a.rope.slot_mapping[tok] : -1;
+      if (slot >= 0) {
+        const int blk = slot / KV_BLOCK, off = slot % KV_BLOCK;
+        const bool key = head < a.rope.n_q + a.rope.n_kv;
+        __nv_bfloat16* base = (key ? a.rope.k_cache : a.rope.v_cache) +
+                              ((size_t)blk * a.rope.n_kv + (head - a.rope.n_q - (key ? 0 : a.rope.n_kv))) * (KV_BLOCK * HEAD_DIM);
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const int dim = d + 64 * p, chunk = dim >> 3, sub = dim & 7;
+          base[key ? (chunk * KV_BLOCK + off) * 8 + sub : off * HEAD_DIM + ((chunk ^ (off & 7)) * 8) + sub] = out[p];
+        }
+      }
+    }
+  } else if (a.mode == 2 || a.mode == 3) {   // rows (2j, 2j + 1) of W are (gate_j, up_j)
+    for (int i = threadIdx.x; i < a.T * (R / 2); i += WARPS * 32) {
+      const int tok = i / (R / 2), j = i % (R / 2);
+      if (n0 + 2 * j + 1 < a.N) Y[(size_t)tok * a.ldy + n0 / 2 + j] = __float2bfloat16_rn(skinny_glu(a.mode, sum(tok, 2 * j), sum(tok, 2 * j + 1)));
+    }
+  } else {
+    for (int i = threadIdx.x; i < a.T * R; i += WARPS * 32) {
+      const int tok = i / R, j = i % R;
+      if (n0 + j >= a.N) continue;
+      float v = sum(tok, j);
+      const size_t o = (size_t)tok * a.ldy + n0 + j;
+      if (a.mode == 1) {
+        reinterpret_cast<float*>(a.Y)[o] = v;
+      } else {
+        if (a.mode == 4) {
+          v = fmaxf(v, 0.f);
+          v *= v;
+        }
+        Y[o] = __float2bfloat16_rn(v);
+      }
+    }
+  }
+}
+
+template <int MT, int NT, int WARPS, bool ROPE>
+cudaError_t launch(const SkinnyArgs& a, cudaStream_t s) {
+  constexpr size_t smem = (size_t)WARPS * 8 * NT * (16 * MT + 1) * sizeof(float);
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(gemm_skinny_kernel<MT, NT, WARPS, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (attr != cudaSuccess) return attr;
+  return launch_k(gemm_skinny_kernel<MT, NT, WARPS, ROPE>, dim3((a.N + 16 * MT - 1) / (16 * MT)), dim3(WARPS * 32), smem, s, a);
+}
+template <int MT, int WARPS, bool ROPE>
+cudaError_t launch_nt(const SkinnyArgs& a, cudaStream_t s) {
+  switch ((a.T + 7) / 8) {
+    case 1: return launch<MT, 1, WARPS, ROPE>(a, s);
+    case 2: return launch<MT, 2, WARPS, ROPE>(a, s);
+    case 3: return launch<MT, 3, WARPS, ROPE>(a, s);
+    default: return launch<MT, 4, WARPS, ROPE>(a, s);
+  }
+}
+
+constexpr int SKINNY_ONE_WAVE = 148 * 16;   // weight rows that 16-row CTAs cover with one CTA per SM
+
+}  // namespace
+
+// Where the line lies was measured inside decode steps, where the tcgen05 kernel's ring (19 MB over all SMs) fills while the
+// kernel before it still runs.  Up to eight tokens: weights of up to 34 MB (steps of an 8B layer: o projection of 34 MB 1.5 %
+// faster, qkv of 50 MB and more slower; steps of a 2048-wide expert model 8 to 11 % faster).  Up to 32 tokens: 9 MB (steps of
+// a 2048-wide recurrent model 6 % faster at 32 tokens; an expert model with products of 9.4 MB 1 % slower).
+bool gemm_skinny_takes(int T, int N, int K) {
+  return T >= 1 && T <= 32 && K >= 64 && K % 64 == 0 && N <= 24576 && (long long)N * K <= (T <= 8 ? 17000000 : 4500000);
+}
+
+cudaError_t gemm_skinny_launch(const void* X, const void* W, void* Y, int ldy, int T, int N, int K, int out_mode, const GemmRope* rope,
+                               cudaStream_t stream) {
+  SkinnyArgs a{(const __nv_bfloat16*)X, (const __nv_bfloat16*)W, Y, ldy, T, N, K, out_mode, {}};
+  // k-splits depend on N and on T <= 8 alone, so that a product has the same bits with every epilogue.  Sixteen warps where an
+  // SM holds one CTA; 32-row CTAs for few tokens (more loads in flight), 16-row ones beyond eight (fewer activation bytes in
+  // flight per register).
+  const bool few = T <= 8, wide = few ? N > 2 * SKINNY_ONE_WAVE : N > SKINNY_ONE_WAVE;
+  if (rope != nullptr) {
+    a.rope = *rope;
+    return wide ? launch_nt<2, 8, true>(a, stream) : launch_nt<2, 16, true>(a, stream);
+  }
+  if (few && wide) return launch<2, 1, 8, false>(a, stream);
+  if (wide) return launch_nt<1, 8, false>(a, stream);
+  if (few && N > SKINNY_ONE_WAVE) return launch<2, 1, 16, false>(a, stream);
+  return launch_nt<1, 16, false>(a, stream);
+}
+
+}  // namespace tgis

@@ -1159,7 +1159,12 @@ static cudaError_t launch_bt(const CUtensorMap& wmap, const CUtensorMap& xmap, v
 // xmap must have been built with box_rows == gemm_x_box(T)
 cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int T, int N, int K,
                              float* ws, int* counters, int num_sms, cudaStream_t stream, int out_f32,
-                             const CUtensorMap* next_wmap, const GemmNext* next, const GemmRope* rope, const GemmNorm* norm) {
+                             const CUtensorMap* next_wmap, const GemmNext* next, const GemmRope* rope, const GemmNorm* norm,
+                             const void* X, const void* W) {
+  if (X != nullptr && W != nullptr && norm == nullptr && gemm_skinny_takes(T, N, K) &&
+      ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) == 0 &&
+      (rope == nullptr || (out_f32 == 0 && N == (rope->n_q + 2 * rope->n_kv) * HEAD_DIM)))
+    return gemm_skinny_launch(X, W, Y, ldy, T, N, K, out_f32, rope, stream);
   GemmRope rp{};
   if (rope) rp = *rope;
   GemmNorm nr{};

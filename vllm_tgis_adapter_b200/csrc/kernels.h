@@ -70,7 +70,8 @@ int gemm_cluster_split(int T, int N, int K, int num_sms);
 cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int T, int N, int K,
                              float* ws, int* counters, int num_sms, cudaStream_t stream, int out_f32 = 0,
                              const CUtensorMap* next_wmap = nullptr, const GemmNext* next = nullptr,
-                             const GemmRope* rope = nullptr, const GemmNorm* norm = nullptr);
+                             const GemmRope* rope = nullptr, const GemmNorm* norm = nullptr, const void* X = nullptr,
+                             const void* W = nullptr);  // X, W: the operands behind the maps ([T, K], [N, K]), if contiguous
 
 // ---- gemm_pair.cu: the same product on CTA pairs (tcgen05 cta_group::2), thousands of tokens or expert segments ----------
 constexpr int PAIR_PLAIN = 0;        // Y[row, n] = acc
@@ -84,6 +85,12 @@ cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
                              int K, int num_sms, cudaStream_t stream);
 int gemm_pair_plan(int T, int N, int pairs);   // token tiles of the dense launch
 bool gemm_pair_failed();                       // a wait inside a launch of this process ran out
+
+// ---- gemm_skinny.cu: the same product for up to 32 tokens; X [T, K], W [N, K] contiguous, rows on 16-byte boundaries; rope: as in
+// gemm_bf16_launch (out mode 0, N a multiple of 128)
+bool gemm_skinny_takes(int T, int N, int K);
+cudaError_t gemm_skinny_launch(const void* X, const void* W, void* Y, int ldy, int T, int N, int K, int out_mode, const GemmRope* rope,
+                               cudaStream_t stream);
 
 // ---- gemm_ref.cu (debug cross-check only; never on the product path) ---------------------------------------------
 cudaError_t gemm_bf16_ref_launch(const __nv_bfloat16* X, int ldx, const __nv_bfloat16* W, void* Y, int ldy, int T,

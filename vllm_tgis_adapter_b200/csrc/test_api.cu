@@ -108,7 +108,8 @@ int tgis_k_gemm(const void* x_dev, const void* w_dev, void* y_dev, int32_t T, in
     KCK(cudaMemset(ctr.p, 0, sizeof(int) << 16));
     KCK(cudaEventRecord(e0, st));
     for (int i = 0; i < iters; ++i)
-      KCK(gemm_bf16_launch(wm, xm, y_dev, out_f32 == 2 ? N / 2 : N, T, N, K, ws.p, ctr.p, sms, st, out_f32));
+      KCK(gemm_bf16_launch(wm, xm, y_dev, out_f32 == 2 ? N / 2 : N, T, N, K, ws.p, ctr.p, sms, st, out_f32, nullptr, nullptr,
+                           nullptr, nullptr, x_dev, w_dev));
     KCK(cudaEventRecord(e1, st));
     KCK(cudaStreamSynchronize(st));
   }
@@ -192,7 +193,7 @@ int tgis_k_gemm_rope(const void* x_dev, const void* w_dev, void* y_dev, int32_t 
   KCK(pos.upload(positions_host, T));
   KCK(sm.upload(slot_mapping_host, T));
   const GemmRope rp{pos.p, sm.p, (const bf16*)cos_sin_dev, (bf16*)k_cache_dev, (bf16*)v_cache_dev, n_q, n_kv};
-  KCK(gemm_bf16_launch(wm, xm, y_dev, N, T, N, K, ws.p, ctr.p, sms, 0, 0, nullptr, nullptr, &rp));
+  KCK(gemm_bf16_launch(wm, xm, y_dev, N, T, N, K, ws.p, ctr.p, sms, 0, 0, nullptr, nullptr, &rp, nullptr, x_dev, w_dev));
   KCK(cudaDeviceSynchronize());
   return 0;
 }
