@@ -101,14 +101,11 @@ __device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, int* e
   return true;
 }
 
-// silu without the branch of an IEEE division (a quotient within 2 ulp): the epilogue's values interleave, and the result is
-// rounded to bf16
+// (a quotient within 2 ulp and without the branch of an IEEE division; the result is rounded to bf16)
 __device__ __forceinline__ float pair_silu(float g) { return __fdividef(g, 1.f + expf(-g)); }
 template <int MODE>
 __device__ __forceinline__ float pair_glu(float g, float u) {
-  if constexpr (MODE == PAIR_SWIGLU_BF16) {   // the rounding points of a bf16 gate / up product followed by silu and a product
-    return bf16_round(pair_silu(bf16_round(g))) * bf16_round(u);
-  } else if constexpr (MODE == PAIR_SWIGLU) {
+  if constexpr (MODE == PAIR_SWIGLU) {
     return pair_silu(g) * u;
   } else {
     return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
@@ -200,13 +197,26 @@ __device__ __forceinline__ void pair_store(const PairArgs& a, const PairTile& t,
       const bool odd = lane & 1;
       OT* yl = y + (odd ? a.ldy : 0);
       const int mine_valid = valid - (odd ? 1 : 0);
+      float g[16], u[16], v[16];
 #pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? r[j] : r[j + 1]), 1);
-        const float g = odd ? got : __uint_as_float(r[j]), u = odd ? __uint_as_float(r[j + 1]) : got;
-        const float v = pair_glu<MODE>(g, u);
-        if (j < mine_valid) yl[(size_t)j * a.ldy] = pair_out<OT>(v);
+      for (int j = 0; j < 16; ++j) {
+        const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? r[2 * j] : r[2 * j + 1]), 1);
+        g[j] = odd ? got : __uint_as_float(r[2 * j]);
+        u[j] = odd ? __uint_as_float(r[2 * j + 1]) : got;
       }
+      if constexpr (MODE == PAIR_SWIGLU_BF16) {   // the rounding points of a bf16 gate / up product followed by silu and a product
+#pragma unroll
+        for (int j = 0; j < 16; ++j) g[j] = bf16_round(g[j]);
+        silu_bf16_n(g, v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] *= bf16_round(u[j]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = pair_glu<MODE>(g[j], u[j]);
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (2 * j < mine_valid) yl[(size_t)(2 * j) * a.ldy] = pair_out<OT>(v[j]);
     } else {
 #pragma unroll
       for (int j = 0; j < 32; ++j)

@@ -151,10 +151,11 @@ __device__ __forceinline__ __nv_bfloat16 swiglu_bf16(float gate_acc, float up_ac
 }
 // The gated pair of out mode 2 (SwiGLU, above) or 3: tanh-form GELU on the gate, evaluated on the fp32 accumulators and
 // rounded once
+__device__ __forceinline__ float geglu(float g, float u) {
+  return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
+}
 __device__ __forceinline__ __nv_bfloat16 glu_bf16(int out_mode, float gate_acc, float up_acc) {
-  if (out_mode == 2) return swiglu_bf16(gate_acc, up_acc);
-  const float g = gate_acc;
-  return __float2bfloat16_rn(0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * up_acc);
+  return out_mode == 2 ? swiglu_bf16(gate_acc, up_acc) : __float2bfloat16_rn(geglu(gate_acc, up_acc));
 }
 
 // Out mode 4: squared ReLU of the accumulator (bf16 out), evaluated in fp32 and rounded once
@@ -549,13 +550,30 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
           if (!partial) {
             if (ep_glu(out_f32)) {
               // fused SwiGLU / GeGLU: weight rows are interleaved (2j = gate_j, 2j+1 = up_j) so the pair sits in adjacent
-              // lanes; even lanes produce act[t, n/2]
+              // lanes; the even lane makes act[t, n/2], the odd lane act[t + 1, n/2], with one exchange for both
+              const bool odd = row & 1;
+              float g[8], u[8], v[8];
 #pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(r[j]), 1);
-                if ((row & 1) == 0 && n < N && c0 + j < t_valid)
-                  Y[(size_t)(c0 + j) * ldy + (n >> 1)] = glu_bf16(out_f32, __uint_as_float(r[j]), other);
+              for (int j = 0; j < 8; ++j) {
+                const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? r[2 * j] : r[2 * j + 1]), 1);
+                g[j] = odd ? got : __uint_as_float(r[2 * j]);
+                u[j] = odd ? __uint_as_float(r[2 * j + 1]) : got;
               }
+              if (out_f32 == 2) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) g[j] = bf16_round(g[j]);
+                silu_bf16_n(g, v);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] *= bf16_round(u[j]);
+              } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = geglu(g[j], u[j]);
+              }
+              const int tok = c0 + (odd ? 1 : 0);
+              __nv_bfloat16* yo = Y + (size_t)tok * ldy + (n >> 1);
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if ((n | 1) < N && tok + 2 * j < t_valid) yo[(size_t)(2 * j) * ldy] = __float2bfloat16_rn(v[j]);
             } else if (n < N) {
 #pragma unroll
               for (int j = 0; j < 16; ++j)

@@ -219,6 +219,32 @@ __device__ __forceinline__ float4 ld_dsmem_f4(uint32_t addr) {
 __device__ __forceinline__ float bf16_bits_to_f32(uint16_t b) { return __uint_as_float(((uint32_t)b) << 16); }
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
+// s[i] = bf16(g[i] / (1 + exp(-g[i]))) for N values at once.  An IEEE division branches for every value and keeps the values of
+// an epilogue from overlapping, so the quotients come from the approximate one (within 2 ulp) and are divided again only where
+// one of them lies within 3 ulp of the middle of two bf16 numbers (or g is so low that the approximation flushes): same bits.
+template <int N>
+__device__ __forceinline__ void silu_bf16_n(const float (&g)[N], float (&s)[N]) {
+  bool close = false;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const float q = __fdividef(g[i], 1.0f + expf(-g[i]));
+    const int below = (int)(__float_as_uint(q) & 0xffffu) - 0x8000;
+    close |= (below >= -3 && below <= 3) || g[i] < -80.f;
+    s[i] = bf16_round(q);
+  }
+  if (close) {
+#pragma unroll 1
+    for (int i = 0; i < N; ++i) {
+      float gi = g[0];
+#pragma unroll
+      for (int j = 1; j < N; ++j) gi = i == j ? g[j] : gi;
+      const float q = bf16_round(gi / (1.0f + expf(-gi)));
+#pragma unroll
+      for (int j = 0; j < N; ++j) s[j] = i == j ? q : s[j];
+    }
+  }
+}
+
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
