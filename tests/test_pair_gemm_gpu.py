@@ -1,4 +1,4 @@
-"""Products of more than 256 tokens and of expert segments on CTA pairs (csrc/gemm_pair.cu) against 64-bit torch: token counts around the 32-token
+"""Products of more than 256 tokens (64 where there are many weight rows) and of expert segments on CTA pairs (csrc/gemm_pair.cu) against 64-bit torch: token counts around the 32-token
 unit and the 256-token tile, weight rows around the 256-row pair tile, every epilogue, and nothing written outside Y."""
 import ctypes as C
 
@@ -27,7 +27,7 @@ def run(lib, x, w, T, mode, rows):
 
 
 @pytest.mark.parametrize("mode", [PLAIN, PLAIN_F32, SWIGLU, GEGLU, RELU2])
-@pytest.mark.parametrize("T,N,K", [(257, 256, 256), (288, 258, 320), (289, 130, 64), (511, 520, 512), (512, 8, 768), (513, 2128, 256), (2050, 3000, 1088)])
+@pytest.mark.parametrize("T,N,K", [(257, 256, 256), (288, 258, 320), (289, 130, 64), (511, 520, 512), (512, 8, 768), (513, 2128, 256), (2050, 3000, 1088), (65, 9474, 192), (256, 9600, 320)])
 def test_pair_products(lib, T, N, K, mode):
     gen = torch.Generator(device="cuda").manual_seed(T + N + K)
     rows = max(T, 256) + 3   # fewer rows than the last token tile covers: the rest is read as zeros

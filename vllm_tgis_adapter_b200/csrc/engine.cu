@@ -193,8 +193,8 @@ __global__ void gather_relayout_kernel(const uint4* __restrict__ gathered, uint4
 
 constexpr int N_BT = 5;
 const int BT_VALUES[N_BT] = {16, 32, 64, 128, 256};  // box heights of the activation maps
-int bt_index(int T) {
-  const int bt = gemm_x_box(T);
+int bt_index(int T, int N, int num_sms) {
+  const int bt = gemm_x_box(T, N, num_sms);
   for (int i = 0; i < N_BT; ++i)
     if (BT_VALUES[i] == bt) return i;
   return N_BT - 1;
@@ -2350,7 +2350,7 @@ struct tgis_engine {
       if (make_tmap_bf16_2d(&m, Wt, (uint64_t)N, (uint64_t)K, (uint64_t)K, 128, 64) != 0) return false;
       wit = pnx_wmaps.emplace(Wt, m).first;
     }
-    const int bi = bt_index(T);
+    const int bi = bt_index(T, N, num_sms);
     const uint64_t xkey = (reinterpret_cast<uint64_t>(X) << 3) ^ ((uint64_t)K << 44) ^ (uint64_t)bi;
     auto xit = pnx_xmaps.find(xkey);
     if (xit == pnx_xmaps.end()) {
@@ -3172,7 +3172,7 @@ struct tgis_engine {
     } else {
       GemmNext nx{};
       if (next_wm && l2_prefetch_kb > 0) nx = gemm_next_desc(nT, nN, nK, num_sms, l2_prefetch_kb);
-      CK(gemm_bf16_launch(wm, xmaps[bt_index(T)], Y, ldy, T, N, K, gemm_ws.p, gemm_counters.p, num_sms, stream, out_f32,
+      CK(gemm_bf16_launch(wm, xmaps[bt_index(T, N, num_sms)], Y, ldy, T, N, K, gemm_ws.p, gemm_counters.p, num_sms, stream, out_f32,
                           nx.kb_prefetch > 0 ? next_wm : nullptr, nx.kb_prefetch > 0 ? &nx : nullptr, rope, norm, X, W));
     }
     if (pe1) CK(cudaEventRecord(pe1, stream));

@@ -1174,7 +1174,7 @@ static cudaError_t launch_bt(const CUtensorMap& wmap, const CUtensorMap& xmap, v
                   ldy, T, N, K, ws, counters, stream_weights, out_f32, next_wmap, nxt, 0, rope, norm);
 }
 
-// xmap must have been built with box_rows == gemm_x_box(T)
+// xmap must have been built with box_rows == gemm_x_box(T, N, num_sms)
 cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int T, int N, int K,
                              float* ws, int* counters, int num_sms, cudaStream_t stream, int out_f32,
                              const CUtensorMap* next_wmap, const GemmNext* next, const GemmRope* rope, const GemmNorm* norm,
@@ -1190,8 +1190,7 @@ cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
   GemmNext nx{};
   if (next && next_wmap) nx = *next;
   const CUtensorMap& nm = (next && next_wmap) ? *next_wmap : wmap;
-  // more than one token tile: CTA pairs (gemm_pair.cu; 1.3 to 3 times as fast at every size measured from 257 tokens on)
-  if (T > 256) {
+  if (gemm_takes_pairs(T, N, num_sms)) {
     if (rope != nullptr || norm != nullptr || out_f32 < 0 || out_f32 > 4) return cudaErrorInvalidValue;
     static const int modes[5] = {PAIR_PLAIN, PAIR_PLAIN, PAIR_SWIGLU_BF16, PAIR_GEGLU, PAIR_RELU2};
     return gemm_pair_launch(wmap, xmap, Y, ldy, out_f32 == 1, modes[out_f32], T, N, K, num_sms, stream);

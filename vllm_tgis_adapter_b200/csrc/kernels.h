@@ -14,9 +14,13 @@ int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_
                       uint32_t box_rows, uint32_t box_cols);
 int gemm_pick_bt(int T);
 constexpr int GEMM_X_BOX_MANY = 32;
-// rows of one box of the activation map: the token tile, or (more tokens than one tile) small boxes, of which the kernels
-// load as many as a tile of their choice takes
-inline int gemm_x_box(int T) { return T > 256 ? GEMM_X_BOX_MANY : gemm_pick_bt(T); }
+// Whether a dense product runs on CTA pairs (gemm_pair.cu): more than 256 tokens always, more than 64 when the weights have more
+// 128-row tiles than half the SMs (fewer are cut along k by the one-CTA kernel, which can also fuse the rotary embedding).
+// Microseconds with cold weights, one CTA -> pairs, at 64, 128 and 256 tokens: 28672 x 4096 (SwiGLU) 59 -> 61, 69 -> 63, 100 -> 69;
+// 128256 x 4096 183 -> 185, 196 -> 189, 257 -> 206; 10248 x 2048 21 -> 14, 28 -> 15, 43 -> 19.
+inline bool gemm_takes_pairs(int T, int N, int num_sms) { return T > 256 || (T > 64 && (N + 127) / 128 > num_sms / 2); }
+// rows of one box of the activation map: the token tile, or (pairs) small boxes, of which a tile takes as many as it has rows
+inline int gemm_x_box(int T, int N, int num_sms) { return gemm_takes_pairs(T, N, num_sms) ? GEMM_X_BOX_MANY : gemm_pick_bt(T); }
 int gemm_nw(int T);  // weight tiles (128 rows each) per unit sharing one activation tile: 2 for decode-shaped launches
 size_t gemm_workspace_bytes(int num_sms);
 int gemm_timeline_read(unsigned long long* out64);  // debug builds (-DTGIS_GEMM_TIMELINE) only

@@ -100,7 +100,7 @@ int tgis_k_gemm(const void* x_dev, const void* w_dev, void* y_dev, int32_t T, in
     const int bt = gemm_pick_bt(T);
     if (x_rows_alloc < bt) return kfail("x must have at least one TMA box of rows allocated");
     if (make_tmap_bf16_2d(&wm, w_dev, N, K, K, 128, 64) != 0) return kfail("weight tensor map failed");
-    if (make_tmap_bf16_2d(&xm, x_dev, x_rows_alloc, K, K, gemm_x_box(T), 64) != 0) return kfail("activation tensor map failed");
+    if (make_tmap_bf16_2d(&xm, x_dev, x_rows_alloc, K, K, gemm_x_box(T, N, sms), 64) != 0) return kfail("activation tensor map failed");
     Tmp<float> ws;
     Tmp<int> ctr;
     KCK(ws.alloc(gemm_workspace_bytes(sms) / sizeof(float)));
@@ -183,7 +183,7 @@ int tgis_k_gemm_rope(const void* x_dev, const void* w_dev, void* y_dev, int32_t 
   const int bt = gemm_pick_bt(T);
   if (x_rows_alloc < bt) return kfail("x must have at least one TMA box of rows allocated");
   if (make_tmap_bf16_2d(&wm, w_dev, N, K, K, 128, 64) != 0) return kfail("weight tensor map failed");
-  if (make_tmap_bf16_2d(&xm, x_dev, x_rows_alloc, K, K, gemm_x_box(T), 64) != 0) return kfail("activation tensor map failed");
+  if (make_tmap_bf16_2d(&xm, x_dev, x_rows_alloc, K, K, gemm_x_box(T, N, sms), 64) != 0) return kfail("activation tensor map failed");
   Tmp<float> ws;
   Tmp<int> ctr;
   Tmp<int32_t> pos, sm;
@@ -222,10 +222,10 @@ int tgis_k_gemm_norm_chain(const void* a_dev, int32_t a_rows_alloc, const void* 
   KCK(cudaMemset(ctr.p, 0, sizeof(int) << 16));
   CUtensorMap wm1, am, wm2, xm;
   if (make_tmap_bf16_2d(&wm1, w1_dev, H, K1, K1, 128, 64) != 0) return kfail("w1 tensor map failed");
-  if (make_tmap_bf16_2d(&am, a_dev, a_rows_alloc, K1, K1, gemm_x_box(T), 64) != 0) return kfail("a tensor map failed");
+  if (make_tmap_bf16_2d(&am, a_dev, a_rows_alloc, K1, K1, gemm_x_box(T, H, sms), 64) != 0) return kfail("a tensor map failed");
   if (make_tmap_bf16_2d(&wm2, w2_dev, N2, H, H, 128, 64) != 0) return kfail("w2 tensor map failed");
   // the fused consumer stages the raw residual stream by TMA and normalises it in shared memory
-  if (make_tmap_bf16_2d(&xm, fused ? residual_dev : (void*)xn.p, fused ? a_rows_alloc : rows, H, H, gemm_x_box(T), 64) != 0)
+  if (make_tmap_bf16_2d(&xm, fused ? residual_dev : (void*)xn.p, fused ? a_rows_alloc : rows, H, H, gemm_x_box(T, N2, sms), 64) != 0)
     return kfail("xn tensor map failed");
   const int ldy2 = out_mode2 == 2 ? N2 / 2 : N2;
   cudaEvent_t e0, e1;
