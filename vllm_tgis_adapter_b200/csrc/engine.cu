@@ -3236,10 +3236,20 @@ struct tgis_engine {
     const bool lora = (samp_complex & 4) != 0 && max_loras > 0;
     const int32_t* d_toklora = ds<int32_t>(off_toklora);
     const int LR = lora_R, kvd = nkv * HEAD_DIM;
-    auto lora_apply = [&](const LoraGroup& g, const bf16* x, int ldx, bf16* y, int ldy) {
+    auto lora_shrink = [&](const LoraGroup& g, const bf16* x, int ldx) {   // (before the projection it corrects)
       CK(lora_shrink_launch(x, ldx, d_toklora, g, lora_v.p, T, stream));
-      CK(lora_expand_launch(lora_v.p, d_toklora, g, y, ldy, T, stream));
-      n_launches += 2;
+      ++n_launches;
+    };
+    auto lora_expand = [&](const LoraGroup& g, bf16* y, int ldy, bf16* act_out = nullptr) {
+      CK(lora_expand_launch(lora_v.p, d_toklora, g, y, ldy, T, stream, act_out));
+      ++n_launches;
+    };
+    auto lora_one = [&](const bf16* A, const bf16* B, int K, int N, int Rm) {
+      LoraGroup g{};
+      g.n_mods = 1;
+      g.v_ld = 3 * LR;
+      g.mod[0] = LoraModule{A, B, K, N, Rm, 0, 0};
+      return g;
     };
     if (lora) ++lora_steps;
     const bool rope_fused = !pnx_on && !lora && fuse_rope && !cfg.debug_gemm_ref && gemm_even_split(T, qkv_dim, H, num_sms) >= 2 &&
@@ -3272,18 +3282,19 @@ struct tgis_engine {
         }
         const GemmRope rp{ds<int32_t>(off_pos), ds<int32_t>(off_slotmap), cos_sin,
                           k_cache.p + (size_t)li * kv_layer_elems, v_cache.p + (size_t)li * kv_layer_elems, nq, nkv};
-        gemm(qkv_norm_in ? xm_resid : xm_xn, l.m_qkv, xn.p, l.wqkv, qkv.p, T, qkv_dim, H, 0, &l.m_o, T, H, q_dim, 0,
-             rope_fused ? &rp : nullptr, qkv_norm_in ? &cons_qkv : nullptr);
+        LoraGroup g{};
         if (lora) {
           const LoraLayerW& ll = lora_layers[li];
-          LoraGroup g{};
           g.n_mods = 3;
           g.v_ld = 3 * LR;
           g.mod[0] = LoraModule{ll.A_q, ll.B_q, H, q_dim, LR, 0, 0};
           g.mod[1] = LoraModule{ll.A_k, ll.B_k, H, kvd, LR, q_dim, LR};
           g.mod[2] = LoraModule{ll.A_v, ll.B_v, H, kvd, LR, q_dim + kvd, 2 * LR};
-          lora_apply(g, xn.p, H, qkv.p, qkv_dim);
+          lora_shrink(g, xn.p, H);
         }
+        gemm(qkv_norm_in ? xm_resid : xm_xn, l.m_qkv, xn.p, l.wqkv, qkv.p, T, qkv_dim, H, 0, &l.m_o, T, H, q_dim, 0,
+             rope_fused ? &rp : nullptr, qkv_norm_in ? &cons_qkv : nullptr);
+        if (lora) lora_expand(g, qkv.p, qkv_dim);
       }
       bf16* kc = k_cache.p + (size_t)li * kv_layer_elems;
       bf16* vc = v_cache.p + (size_t)li * kv_layer_elems;
@@ -3304,15 +3315,10 @@ struct tgis_engine {
                                n_tiles, d_bt, bt_stride, attn_out.p, q_dim, nq, nkv, scale, stream));
         ++n_launches;
       }
+      if (lora) lora_shrink(lora_one(lora_layers[li].A_o, lora_layers[li].B_o, q_dim, H, LR), attn_out.p, q_dim);
       gemm(xm_attn, l.m_o, attn_out.p, l.wo, ar_fused ? ar_buf(0) : tmp.p, T, H, q_dim, 0, &l.m_gu, T, 2 * F, H, 0, nullptr,
            norm_fused ? &prod_attn : nullptr);
-      if (lora) {
-        LoraGroup g{};
-        g.n_mods = 1;
-        g.v_ld = 3 * LR;
-        g.mod[0] = LoraModule{lora_layers[li].A_o, lora_layers[li].B_o, q_dim, H, LR, 0, 0};
-        lora_apply(g, attn_out.p, q_dim, tmp.p, H);
-      }
+      if (lora) lora_expand(lora_one(lora_layers[li].A_o, lora_layers[li].B_o, q_dim, H, LR), tmp.p, H);
       if (norm_fused) {
       } else if (ar_fused) {
         fused_ar_norm(0, l.ln2, T);
@@ -3324,29 +3330,20 @@ struct tgis_engine {
       // gate_up GEMM with SwiGLU fused into its epilogue: writes act[T, F] directly (no gate_up round trip)
       if (lora) {
         // raw interleaved gate_up -> + adapter deltas (gate and up as one module of capacity 2R) -> SwiGLU
+        const LoraGroup g = lora_one(lora_layers[li].A_gu, lora_layers[li].B_gu, H, 2 * F, 2 * LR);
+        lora_shrink(g, xn.p, H);
         gemm(xm_xn, l.m_gu, xn.p, l.wgu, gu_buf.p, T, 2 * F, H, /*out_mode=*/0, &l.m_d, T, H, F, /*ldy=*/2 * F);
-        LoraGroup g{};
-        g.n_mods = 1;
-        g.v_ld = 3 * LR;
-        g.mod[0] = LoraModule{lora_layers[li].A_gu, lora_layers[li].B_gu, H, 2 * F, 2 * LR, 0, 0};
-        lora_apply(g, xn.p, H, gu_buf.p, 2 * F);
-        CK(silu_mul_interleaved_launch(gu_buf.p, act.p, T, F, stream));
-        ++n_launches;
+        lora_expand(g, gu_buf.p, 2 * F, act.p);
       } else
       gemm(norm_fused ? xm_resid : xm_xn, l.m_gu, xn.p, l.wgu, act.p, T, 2 * F, H, /*out_mode=*/2, &l.m_d, T, H, F,
            /*ldy=*/F, nullptr, norm_fused ? &cons_gu : nullptr);
       bf16* down_out = ar_fused ? ar_buf(1) : tmp.p;
+      if (lora) lora_shrink(lora_one(lora_layers[li].A_d, lora_layers[li].B_d, F, H, LR), act.p, F);
       if (li + 1 < c.n_layers)
         gemm(xm_act, l.m_d, act.p, l.wd, down_out, T, H, F, 0, &layers[li + 1].m_qkv, T, qkv_dim, H, 0, nullptr,
              norm_fused ? &prod_mlp : nullptr);
       else gemm(xm_act, l.m_d, act.p, l.wd, down_out, T, H, F, 0, R > 0 ? &m_lm : nullptr, R, Vl, H);
-      if (lora) {
-        LoraGroup g{};
-        g.n_mods = 1;
-        g.v_ld = 3 * LR;
-        g.mod[0] = LoraModule{lora_layers[li].A_d, lora_layers[li].B_d, F, H, LR, 0, 0};
-        lora_apply(g, act.p, F, down_out, H);
-      }
+      if (lora) lora_expand(lora_one(lora_layers[li].A_d, lora_layers[li].B_d, F, H, LR), down_out, H);
       if (!ar_fused) all_reduce_tmp(T);
     }
     // The last down-proj exchange is run even when no row is sampled this step (R == 0): it is what guarantees that

@@ -14,11 +14,12 @@
 // Shape of the problem: HBM/L2-bound skinny products (rank 8..64 against K, N of 1k..14k), integer slot look-ups per
 // token; no tensor-core shape worth having.  Two kernels per adapted projection group:
 //   shrink : CTA = (tile of 8 tokens, 4 rank rows of one module), its 8 warps split K; the A rows are streamed once per
-//            tile with 16-byte loads and used for all 8 tokens when they share the adapter (prefill chunks and
-//            same-adapter decode batches); mixed tiles fall back to one row stream per token.
+//            tile and adapter with 16-byte loads and used for all of the tile's tokens of that adapter.
 //   expand : CTA = (tile of 8 tokens, 1024 output columns), thread = 4 consecutive columns; the 4 B rows of a thread are
-//            one contiguous run (a warp reads 32 consecutive runs -- fully coalesced) and are read ONCE for the 8 tokens of
-//            a same-adapter tile; the tile's rank vectors are staged in shared memory (broadcast reads).
+//            one contiguous run (a warp reads 32 consecutive runs -- fully coalesced) and are read ONCE for the tile's tokens
+//            of one adapter; the tile's rank vectors are staged in shared memory (broadcast reads).
+// Both are launches of a few microseconds of dependent loads.  The engine runs shrink BEFORE the base projection, which it
+// does not depend on: the projection's first weights are on their way while it runs.
 // Adapter storage (engine.cu): per layer and module  A [slots][Rm][K] and B [slots][N][Rm] bf16, zero padded to the module's
 // rank capacity Rm, so no kernel needs the adapter's true rank.  gate_proj / up_proj are stored as ONE module of capacity
 // 2R over the interleaved gate_up projection (row 2j = gate_j, row 2j+1 = up_j: block-sparse B), see engine.cu.
@@ -56,6 +57,29 @@ __device__ __forceinline__ float dot8(const F8& a, const F8& b) {
 constexpr int LORA_TT = 8;  // tokens per tile
 constexpr int LORA_MAX_RM = 128;
 
+// The adapter slots of a tile's tokens (-1 behind the last token).  A tile is worked through once per distinct slot -- the
+// scheduler sorts a step's tokens by adapter, so most tiles have one or two --, by different CTAs in small launches.
+struct TileSlots {
+  int s[LORA_TT];
+  __device__ __forceinline__ TileSlots(const int32_t* tok_slot, int t0, int T) {
+#pragma unroll
+    for (int j = 0; j < LORA_TT; ++j) s[j] = t0 + j < T ? tok_slot[t0 + j] : -1;
+  }
+  // the p-th distinct slot from `least` on, in the order of first tokens; -1: there are fewer
+  __device__ __forceinline__ int distinct(int p, int least) const {
+    int found = -1, n = 0;
+#pragma unroll
+    for (int j = 0; j < LORA_TT; ++j) {
+      bool first = s[j] >= least;
+#pragma unroll
+      for (int i = 0; i < j; ++i) first &= s[i] != s[j];
+      if (first && n++ == p) found = s[j];
+    }
+    return found;
+  }
+};
+inline int lora_passes_apart(int T) { return T <= 1 ? 1 : T <= 256 ? 4 : 1; }   // CTAs that share a tile's distinct slots
+
 __device__ __forceinline__ F8 cvt8(const uint4& r) {
   const uint32_t w[4] = {r.x, r.y, r.z, r.w};
   F8 o;
@@ -87,33 +111,25 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* 
   const LoraModule md = g.mod[m];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t0 = (int)blockIdx.x * LORA_TT;
-  const int nt = min(LORA_TT, T - t0);
-  int slot0 = 0;
-  bool any = false, uniform = true;
-#pragma unroll
-  for (int j = 0; j < LORA_TT; ++j) {
-    const int sj = (j < nt) ? tok_slot[t0 + j] : 0;
-    if (j == 0) slot0 = sj;
-    any |= sj > 0;
-    uniform &= (j >= nt) || sj == slot0;
-  }
-  if (!any) return;
-  float acc[LORA_RPC][LORA_TT];
-#pragma unroll
-  for (int q = 0; q < LORA_RPC; ++q)
-#pragma unroll
-    for (int j = 0; j < LORA_TT; ++j) acc[q][j] = 0.f;
+  const TileSlots tile(tok_slot, t0, T);
   const int nvec = md.K / 8;
   const uint4* xq = reinterpret_cast<const uint4*>(x);
   const size_t ldq = (size_t)ldx / 8;
-  if (uniform) {
-    const uint4* a0 = reinterpret_cast<const uint4*>(md.A + ((size_t)(slot0 - 1) * md.Rm + r0) * md.K);
+  for (int p = blockIdx.z;; p += gridDim.z) {
+    const int slot = tile.distinct(p, 1);
+    if (slot < 0) return;
+    float acc[LORA_RPC][LORA_TT];
+#pragma unroll
+    for (int q = 0; q < LORA_RPC; ++q)
+#pragma unroll
+      for (int j = 0; j < LORA_TT; ++j) acc[q][j] = 0.f;
+    const uint4* a0 = reinterpret_cast<const uint4*>(md.A + ((size_t)(slot - 1) * md.Rm + r0) * md.K);
     for (int kv = warp * 32 + lane; kv < nvec; kv += 256) {
       uint4 ar[LORA_RPC], xr[LORA_TT];
 #pragma unroll
       for (int q = 0; q < LORA_RPC; ++q) ar[q] = a0[(size_t)q * nvec + kv];
 #pragma unroll
-      for (int j = 0; j < LORA_TT; ++j) xr[j] = xq[(size_t)(t0 + (j < nt ? j : 0)) * ldq + kv];
+      for (int j = 0; j < LORA_TT; ++j) xr[j] = tile.s[j] == slot ? xq[(size_t)(t0 + j) * ldq + kv] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
       for (int j = 0; j < LORA_TT; ++j) {
         const F8 xf = cvt8(xr[j]);
@@ -121,38 +137,26 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* 
         for (int q = 0; q < LORA_RPC; ++q) acc[q][j] += dot8(cvt8(ar[q]), xf);
       }
     }
-  } else {
 #pragma unroll
-    for (int j = 0; j < LORA_TT; ++j) {
-      const int sj = (j < nt) ? tok_slot[t0 + j] : 0;
-      if (sj <= 0) continue;
-      const uint4* a0 = reinterpret_cast<const uint4*>(md.A + ((size_t)(sj - 1) * md.Rm + r0) * md.K);
-      const uint4* xrow = xq + (size_t)(t0 + j) * ldq;
-      for (int kv = warp * 32 + lane; kv < nvec; kv += 256) {
-        const F8 xf = cvt8(xrow[kv]);
+    for (int q = 0; q < LORA_RPC; ++q)
 #pragma unroll
-        for (int q = 0; q < LORA_RPC; ++q) acc[q][j] += dot8(cvt8(a0[(size_t)q * nvec + kv]), xf);
+      for (int j = 0; j < LORA_TT; ++j) {
+        float s = acc[q][j];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) part[warp][q][j] = s;
+      }
+    __syncthreads();
+    if (threadIdx.x < LORA_RPC * LORA_TT) {
+      const int q = threadIdx.x / LORA_TT, j = threadIdx.x % LORA_TT;
+      if (t0 + j < T && tok_slot[t0 + j] == slot) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += part[w][q][j];
+        v[(size_t)(t0 + j) * g.v_ld + md.v_off + r0 + q] = s;
       }
     }
-  }
-#pragma unroll
-  for (int q = 0; q < LORA_RPC; ++q)
-#pragma unroll
-    for (int j = 0; j < LORA_TT; ++j) {
-      float s = acc[q][j];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) part[warp][q][j] = s;
-    }
-  __syncthreads();
-  if (threadIdx.x < LORA_RPC * LORA_TT) {
-    const int q = threadIdx.x / LORA_TT, j = threadIdx.x % LORA_TT;
-    if (j < nt && tok_slot[t0 + j] > 0) {
-      float s = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) s += part[w][q][j];
-      v[(size_t)(t0 + j) * g.v_ld + md.v_off + r0 + q] = s;
-    }
+    __syncthreads();   // part is used again
   }
 }
 
@@ -177,104 +181,98 @@ __device__ __forceinline__ void st4f(__nv_bfloat16* p, const float (&f)[4]) {
   r.y = *reinterpret_cast<const uint32_t*>(&hi);
   *reinterpret_cast<uint2*>(p) = r;
 }
+// ACT: the columns are interleaved (gate_j, up_j) pairs; act[t, j] = bf16(silu(gate)) * up of the corrected projection is
+// written (for tokens without an adapter too) and y is only read: the projection's own kernel after it drops out.
+template <bool ACT>
 __global__ void __launch_bounds__(256)
 lora_expand_kernel(const float* __restrict__ v, const int32_t* __restrict__ tok_slot, LoraGroup g,
-                   __nv_bfloat16* __restrict__ y, int ldy, int T) {
+                   __nv_bfloat16* __restrict__ y, int ldy, __nv_bfloat16* __restrict__ act, int T) {
   __shared__ __align__(16) float vsT[LORA_MAX_RM][LORA_TT];  // [rank index][token of the tile]
   griddep_launch();
   griddep_wait();
   const int t0 = (int)blockIdx.y * LORA_TT;
-  const LoraModule md = g.mod[blockIdx.z];
+  const LoraModule md = g.mod[blockIdx.z % g.n_mods];
   if ((int)blockIdx.x * LORA_ECOLS >= md.N) return;
-  int slot0 = 0;
-  bool any = false, uniform = true;
-#pragma unroll
-  for (int j = 0; j < LORA_TT; ++j) {
-    const int sj = (t0 + j < T) ? tok_slot[t0 + j] : 0;
-    if (j == 0) slot0 = sj;
-    any |= sj > 0;
-    uniform &= (t0 + j >= T) || sj == slot0;
-  }
-  if (!any) return;
+  const TileSlots tile(tok_slot, t0, T);
   const int n0 = ((int)blockIdx.x * 256 + (int)threadIdx.x) * LORA_EC;
   const bool col_ok = n0 < md.N;
-  // same-adapter tile: the thread's y values and its first block of B do not depend on the rank vectors -- request them
-  // before the staging barrier so that their latency runs under it (a CTA is only a few microseconds of work)
-  uint2 yraw[LORA_TT];
-  uint4 nxt[LORA_EC];
-  const __nv_bfloat16* brow = md.B + ((size_t)(max(slot0, 1) - 1) * md.N + (col_ok ? n0 : 0)) * md.Rm;
-  if (uniform && col_ok) {
+  for (int p = blockIdx.z / g.n_mods;; p += gridDim.z / g.n_mods) {
+    const int slot = tile.distinct(p, ACT ? 0 : 1);
+    if (slot < 0) return;
+    // the thread's y values and its first block of B do not depend on the rank vectors -- request them before the staging
+    // barrier so that their latency runs under it (a CTA is only a few microseconds of work)
+    uint2 yraw[LORA_TT];
+    uint4 nxt[LORA_EC];
+    const __nv_bfloat16* brow = md.B + ((size_t)(slot > 0 ? slot - 1 : 0) * md.N + (col_ok ? n0 : 0)) * md.Rm;
+    if (col_ok) {
+      if (slot > 0) {
 #pragma unroll
-    for (int e = 0; e < LORA_EC; ++e) nxt[e] = *reinterpret_cast<const uint4*>(brow + (size_t)e * md.Rm);
+        for (int e = 0; e < LORA_EC; ++e) nxt[e] = *reinterpret_cast<const uint4*>(brow + (size_t)e * md.Rm);
+      }
 #pragma unroll
-    for (int j = 0; j < LORA_TT; ++j)
-      yraw[j] = *reinterpret_cast<const uint2*>(y + (size_t)(t0 + (t0 + j < T ? j : 0)) * ldy + md.col0 + n0);
-  }
-  // the fp32 shrink sums enter the second product as bf16 (lora_expand_op.py casts the buffer to the weight dtype)
-  for (int i = threadIdx.x; i < LORA_TT * md.Rm; i += 256) {
-    const int j = i / md.Rm, r = i - j * md.Rm;
-    const bool live = t0 + j < T && tok_slot[t0 + j] > 0;
-    vsT[r][j] = live ? bf16_round(v[(size_t)(t0 + j) * g.v_ld + md.v_off + r]) : 0.f;
-  }
-  __syncthreads();
-  if (!col_ok) return;
-  if (uniform) {
+      for (int j = 0; j < LORA_TT; ++j)
+        if (tile.s[j] == slot) yraw[j] = *reinterpret_cast<const uint2*>(y + (size_t)(t0 + j) * ldy + md.col0 + n0);
+    }
     float acc[LORA_TT][LORA_EC];
 #pragma unroll
     for (int j = 0; j < LORA_TT; ++j)
 #pragma unroll
       for (int e = 0; e < LORA_EC; ++e) acc[j][e] = 0.f;
-    const int nrv = md.Rm / 8;
-    for (int rv = 0; rv < nrv; ++rv) {
-      F8 bb[LORA_EC];
-#pragma unroll
-      for (int e = 0; e < LORA_EC; ++e) bb[e] = cvt8(nxt[e]);
-      if (rv + 1 < nrv) {
-#pragma unroll
-        for (int e = 0; e < LORA_EC; ++e) nxt[e] = *reinterpret_cast<const uint4*>(brow + (size_t)e * md.Rm + 8 * (rv + 1));
+    if (slot > 0) {
+      // the fp32 shrink sums enter the second product as bf16 (lora_expand_op.py casts the buffer to the weight dtype)
+      for (int i = threadIdx.x; i < LORA_TT * md.Rm; i += 256) {
+        const int j = i / md.Rm, r = i - j * md.Rm;
+        const bool live = t0 + j < T && tok_slot[t0 + j] == slot;
+        vsT[r][j] = live ? bf16_round(v[(size_t)(t0 + j) * g.v_ld + md.v_off + r]) : 0.f;
       }
+      __syncthreads();
+      if (col_ok) {
+        const int nrv = md.Rm / 8;
+        for (int rv = 0; rv < nrv; ++rv) {
+          F8 bb[LORA_EC];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 va = *reinterpret_cast<const float4*>(&vsT[rv * 8 + q][0]);
-        const float4 vb = *reinterpret_cast<const float4*>(&vsT[rv * 8 + q][4]);
-        const float vv[LORA_TT] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+          for (int e = 0; e < LORA_EC; ++e) bb[e] = cvt8(nxt[e]);
+          if (rv + 1 < nrv) {
 #pragma unroll
-        for (int e = 0; e < LORA_EC; ++e)
+            for (int e = 0; e < LORA_EC; ++e) nxt[e] = *reinterpret_cast<const uint4*>(brow + (size_t)e * md.Rm + 8 * (rv + 1));
+          }
 #pragma unroll
-          for (int j = 0; j < LORA_TT; ++j) acc[j][e] = fmaf(vv[j], bb[e].v[q], acc[j][e]);
-      }
-    }
+          for (int q = 0; q < 8; ++q) {
+            const float4 va = *reinterpret_cast<const float4*>(&vsT[rv * 8 + q][0]);
+            const float4 vb = *reinterpret_cast<const float4*>(&vsT[rv * 8 + q][4]);
+            const float vv[LORA_TT] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
-    for (int j = 0; j < LORA_TT; ++j) {
-      if (t0 + j >= T) break;
-      __nv_bfloat16* yp = y + (size_t)(t0 + j) * ldy + md.col0 + n0;
-      float yv[LORA_EC] = {__uint_as_float(yraw[j].x << 16), __uint_as_float(yraw[j].x & 0xffff0000u),
-                           __uint_as_float(yraw[j].y << 16), __uint_as_float(yraw[j].y & 0xffff0000u)};
+            for (int e = 0; e < LORA_EC; ++e)
 #pragma unroll
-      for (int e = 0; e < LORA_EC; ++e) yv[e] += bf16_round(acc[j][e]);
-      st4f(yp, yv);
-    }
-  } else {
-    for (int j = 0; j < LORA_TT && t0 + j < T; ++j) {
-      const int sj = tok_slot[t0 + j];
-      if (sj <= 0) continue;
-      const __nv_bfloat16* brow_j = md.B + ((size_t)(sj - 1) * md.N + n0) * md.Rm;
-      __nv_bfloat16* yp = y + (size_t)(t0 + j) * ldy + md.col0 + n0;
-      float yv[LORA_EC];
-      ld4f(yp, yv);
-#pragma unroll
-      for (int e = 0; e < LORA_EC; ++e) {
-        float s = 0.f;
-        const __nv_bfloat16* b = brow_j + (size_t)e * md.Rm;
-        for (int rv = 0; rv < md.Rm / 8; ++rv) {
-          const F8 bb = ld8(b + 8 * rv);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) s = fmaf(vsT[rv * 8 + q][j], bb.v[q], s);
+              for (int j = 0; j < LORA_TT; ++j) acc[j][e] = fmaf(vv[j], bb[e].v[q], acc[j][e]);
+          }
         }
-        yv[e] += bf16_round(s);
       }
-      st4f(yp, yv);
     }
+    if (col_ok) {
+#pragma unroll
+      for (int j = 0; j < LORA_TT; ++j) {
+        if (tile.s[j] != slot) continue;   // (another adapter's token: its sums here are not used)
+        float yv[LORA_EC] = {__uint_as_float(yraw[j].x << 16), __uint_as_float(yraw[j].x & 0xffff0000u),
+                             __uint_as_float(yraw[j].y << 16), __uint_as_float(yraw[j].y & 0xffff0000u)};
+        if (slot > 0) {
+#pragma unroll
+          for (int e = 0; e < LORA_EC; ++e) yv[e] += bf16_round(acc[j][e]);
+        }
+        if constexpr (ACT) {
+          float o[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float gx = bf16_round(yv[2 * h]);
+            o[h] = bf16_round(gx / (1.0f + expf(-gx))) * bf16_round(yv[2 * h + 1]);
+          }
+          *reinterpret_cast<__nv_bfloat162*>(act + (size_t)(t0 + j) * (md.N / 2) + n0 / 2) = __floats2bfloat162_rn(o[0], o[1]);
+        } else {
+          st4f(y + (size_t)(t0 + j) * ldy + md.col0 + n0, yv);
+        }
+      }
+    }
+    __syncthreads();   // vsT is used again
   }
 }
 
@@ -324,17 +322,19 @@ cudaError_t lora_shrink_launch(const __nv_bfloat16* x, int ldx, const int32_t* t
   if (!lora_group_ok(g) || ldx % 8 != 0) return cudaErrorInvalidValue;
   int groups = 0;
   for (int m = 0; m < g.n_mods; ++m) groups += g.mod[m].Rm / LORA_RPC;
-  return launch_k(lora_shrink_kernel, dim3((T + LORA_TT - 1) / LORA_TT, groups), dim3(256), 0, stream, x, ldx, tok_slot, g, v, T);
+  return launch_k(lora_shrink_kernel, dim3((T + LORA_TT - 1) / LORA_TT, groups, lora_passes_apart(T)), dim3(256), 0, stream, x, ldx, tok_slot,
+                  g, v, T);
 }
 
 cudaError_t lora_expand_launch(const float* v, const int32_t* tok_slot, const LoraGroup& g, __nv_bfloat16* y, int ldy, int T,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, __nv_bfloat16* act) {
   if (T <= 0) return cudaSuccess;
-  if (!lora_group_ok(g) || ldy % 8 != 0) return cudaErrorInvalidValue;
+  if (!lora_group_ok(g) || ldy % 8 != 0 || (act != nullptr && (g.n_mods != 1 || g.mod[0].col0 != 0))) return cudaErrorInvalidValue;
   int max_n = 0;
   for (int m = 0; m < g.n_mods; ++m) max_n = g.mod[m].N > max_n ? g.mod[m].N : max_n;
-  return launch_k(lora_expand_kernel, dim3((max_n + LORA_ECOLS - 1) / LORA_ECOLS, (T + LORA_TT - 1) / LORA_TT, g.n_mods),
-                  dim3(256), 0, stream, v, tok_slot, g, y, ldy, T);
+  const dim3 grid((max_n + LORA_ECOLS - 1) / LORA_ECOLS, (T + LORA_TT - 1) / LORA_TT, g.n_mods * lora_passes_apart(T));
+  return act != nullptr ? launch_k(lora_expand_kernel<true>, grid, dim3(256), 0, stream, v, tok_slot, g, y, ldy, act, T)
+                        : launch_k(lora_expand_kernel<false>, grid, dim3(256), 0, stream, v, tok_slot, g, y, ldy, act, T);
 }
 
 cudaError_t silu_mul_interleaved_launch(const __nv_bfloat16* gate_up, __nv_bfloat16* act, int T, int ffn,
