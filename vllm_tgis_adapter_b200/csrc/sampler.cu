@@ -14,7 +14,10 @@
 // CLUSTER of 8 CTAs x 1024 threads on 8 SMs: each CTA scans one eighth of the vocabulary, block results are exchanged
 // through distributed shared memory and combined in rank order (deterministic).  The fp32 row (512 KiB) is read from
 // HBM once and stays in the 126 MB L2 for the selection passes (radix-select thresholds instead of the reference's
-// full sorts).  Loads are 16-byte vectorised and coalesced.
+// full sorts).  Every sweep takes eight entries per thread and 16-byte load; a row's sweeps: the first (max, sum, greedy argmax),
+// entropy and four radix rounds behind typical-p, processed maximum, race, and one for rank and top-n together.
+// Measured, 128256 bf16 logits, microseconds, scalar sweeps with one sweep per top-n entry -> here: greedy with top-5 36 -> 22 (32
+// rows), 97 -> 38 (96 rows); typical-p with penalties 88 -> 62, 350 -> 160 (flat rows 679 -> 287); top-k and top-p 101 -> 86, 442 -> 246.
 #include <cooperative_groups.h>
 
 #include "kernels.h"
@@ -30,6 +33,7 @@ TGIS_STL_DEFINE(sampler)
 constexpr int SAMP_MAX_CL = 8;  // CTAs (SMs) per row: 1, 2, 4 or 8, chosen per launch (sampler_launch)
 constexpr int SAMP_THREADS = 1024;
 constexpr int SAMP_WARPS = SAMP_THREADS / 32;
+constexpr int SAMP_LIST = SAMP_THREADS;
 constexpr float SAMP_FIX = 1073741824.0f;  // 2^30: probabilities are accumulated as fixed-point integers (see below)
 
 // LT = logits element type: __nv_bfloat16 on the product path (vLLM's lm_head emits model-dtype logits and the sampler
@@ -98,26 +102,45 @@ __device__ __forceinline__ void load_x8(const __nv_bfloat16* x, int i0, float (&
   }
 }
 
+// eight bits of a token bitmap from entry i0 on (i0 % 8 == 0)
+__device__ __forceinline__ uint32_t bits8(const uint32_t* map, int i0) { return (map[i0 >> 5] >> (i0 & 31)) & 0xffu; }
+// eight entries of this CTA's slice (i0 % 8 == 0, i0 + 8 <= hi), masked
 template <class LT>
-__device__ __forceinline__ bool is_seen(const RowCtx<LT>& c, int i) {
-  return c.seen != nullptr && ((c.seen[i >> 5] >> (i & 31)) & 1u);
+__device__ __forceinline__ void load_slice8(const RowCtx<LT>& c, int i0, float (&o)[8]) {
+  if (c.xc != nullptr) {
+    load_x8(c.xc, i0 - c.lo, o);
+    return;
+  }
+  load_x8(c.x, i0, o);
+  if (c.allow != nullptr) {
+    const uint32_t bits = bits8(c.allow, i0);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (!((bits >> e) & 1u)) o[e] = -INFINITY;
+  }
 }
 
-// processed logit (before temperature) of vocabulary entry i with raw value x
+// processed logits (before temperature) of the entries i0 .. i0 + 7, in place of their raw values
 template <class LT>
-__device__ __forceinline__ float process(const RowCtx<LT>& c, int i, float x) {
-  float y = x;
-  if (c.typical) {
-    const float lp = (x - c.raw_max) - c.raw_logz;
-    const float s = fabsf((-lp) - c.ent);
-    if (s > c.typ_thr) y = -INFINITY;
+__device__ __forceinline__ void process8(const RowCtx<LT>& c, int i0, float (&v)[8]) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    if (c.typical) {
+      const float lp = (v[e] - c.raw_max) - c.raw_logz;
+      const float s = fabsf((-lp) - c.ent);
+      if (s > c.typ_thr) v[e] = -INFINITY;
+    }
+    if (i0 + e == c.p.eos_id) {
+      if (c.lenfac_m1 != 0.f && isfinite(v[e])) v[e] = __fadd_rn(v[e], __fmul_rn(fabsf(v[e]), c.lenfac_m1));
+      if (c.mask_eos) v[e] = -INFINITY;
+    }
   }
-  if (i == c.p.eos_id) {
-    if (c.lenfac_m1 != 0.f && isfinite(y)) y = __fadd_rn(y, __fmul_rn(fabsf(y), c.lenfac_m1));
-    if (c.mask_eos) y = -INFINITY;
+  const uint32_t seen = c.seen != nullptr ? bits8(c.seen, i0) : 0u;
+  if (seen != 0) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if ((seen >> e) & 1u) v[e] = (v[e] > 0.f) ? __fdiv_rn(v[e], c.p.rep_penalty) : __fmul_rn(v[e], c.p.rep_penalty);
   }
-  if (c.p.rep_penalty != 1.0f && is_seen(c, i)) y = (y > 0.f) ? __fdiv_rn(y, c.p.rep_penalty) : __fmul_rn(y, c.p.rep_penalty);
-  return y;
 }
 
 // ---------------------------------------------------------------- block reductions (1024 threads, result in every thread)
@@ -367,44 +390,82 @@ __device__ void radix_round_pick(const Cl& c, uint32_t* hist, uint32_t* hsum, ui
   __syncthreads();
 }
 
+// Adds eight (digit, weight) pairs of every lane to the histogram (weight 0: does not count).  Where the whole warp's 256
+// entries share a digit (the leading digits of most rows) one redux and one atomic do; else every entry is a shared-memory
+// atomic of its own, on HIST_COPIES copies of the histogram so that lanes of equal digits meet less often.
+constexpr int HIST_COPIES = 4;
+__device__ __forceinline__ void hist_add8(uint32_t* h, const uint32_t (&digit)[8], const uint32_t (&w)[8]) {
+  uint32_t d = 0xffffffffu, sum = 0;
+  bool same = true;
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if (w[e] > 0) {
+      if (d == 0xffffffffu) d = digit[e];
+      same &= digit[e] == d;
+      sum += w[e];
+    }
+  const uint32_t have = __ballot_sync(0xffffffffu, d != 0xffffffffu);
+  if (have == 0) return;
+  const uint32_t d0 = __shfl_sync(0xffffffffu, d, __ffs(have) - 1);
+  if (__all_sync(0xffffffffu, same && (d == d0 || d == 0xffffffffu))) {
+    const uint32_t all = __reduce_add_sync(0xffffffffu, sum);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&h[d0], all);
+    return;
+  }
+  uint32_t* mine = h + (threadIdx.x & (HIST_COPIES - 1)) * 256;
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if (w[e] > 0) atomicAdd(&mine[digit[e]], w[e]);
+}
+// a round's histogram: all copies to zero / their sum in the first
+__device__ __forceinline__ void hist_clear(uint32_t* h) {
+  if (threadIdx.x < 256 * HIST_COPIES) h[threadIdx.x] = 0u;
+  __syncthreads();
+}
+__device__ __forceinline__ void hist_fold(uint32_t* h) {
+  __syncthreads();
+  if (threadIdx.x < 256) {
+    uint32_t t = h[threadIdx.x];
+#pragma unroll
+    for (int k = 1; k < HIST_COPIES; ++k) t += h[k * 256 + threadIdx.x];
+    h[threadIdx.x] = t;
+  }
+}
+
 // Smallest key K (ascending) such that  sum_{key_i <= K} w_i  >= target  (strict: > target); if never reached, the
-// largest present key.  keyf(i) -> uint32 key, wf(i) -> probability-like weight in [0, 1] (sums to ~1 over the row).
-// Weights are accumulated as 2^-30 fixed-point integers: integer addition is associative, so the histograms -- and with
-// them the selected threshold and every seeded draw -- are bit-reproducible whatever the order in which warps and CTAs
-// arrive (float atomics were not), and no warp-serialised aggregation loop is needed: lanes of a warp that hit the same
-// bin are found with match.any, summed with one redux and added with ONE shared-memory atomic.
+// largest present key.  load(i0, v) -> eight values, keyf(v) -> uint32 key, wf(v) -> probability-like weight in [0, 1] (sums
+// to ~1 over the row).  Weights are accumulated as 2^-30 fixed-point integers: integer addition is associative, so the
+// histograms -- and with them the selected threshold and every seeded draw -- are bit-reproducible whatever the order in
+// which warps and CTAs arrive (float atomics were not).
 // 4 rounds of 8 bits; every CTA histograms its slice, the cluster sums them, every CTA runs the same scan.
-template <class KeyF, class WF>
-__device__ uint32_t select_weighted_asc(Cl& c, int lo, int hi, KeyF keyf, WF wf, float target, bool strict,
-                                        uint32_t (*hist)[256], uint32_t* hsum, uint32_t* bcast) {
+template <class LoadF, class KeyF, class WF>
+__device__ uint32_t select_weighted_asc(Cl& c, int lo, int hi, LoadF load, KeyF keyf, WF wf, float target, bool strict,
+                                        uint32_t (*hist)[256 * HIST_COPIES], uint32_t* hsum, uint32_t* bcast) {
   const uint32_t T = __float2uint_rn(fminf(fmaxf(target, 0.f), 2.f) * SAMP_FIX);
   uint32_t prefix = 0, below = 0;
   for (int round = 0; round < 4; ++round) {
     const int shift = 24 - 8 * round;
     uint32_t* h = hist[c.he & 1];
     ++c.he;
-    if (threadIdx.x < 256) h[threadIdx.x] = 0u;
-    __syncthreads();
-    for (int i0 = lo; i0 < hi; i0 += SAMP_THREADS) {
-      const int i = i0 + threadIdx.x;
-      uint32_t w = 0, digit = 0xffffffffu;  // not counted
-      if (i < hi) {
-        // after the first round only ~1/256 of the entries still carry the selected prefix: test the (cheap) key first
-        // and evaluate the weight (an expf) for those only
-        const uint32_t k = keyf(i);
-        if (round == 0 || (k >> (shift + 8)) == (prefix >> (shift + 8))) {
-          w = __float2uint_rn(wf(i) * SAMP_FIX);
-          if (w > 0) digit = (k >> shift) & 255;
+    hist_clear(h);
+    for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
+      const int i0 = base + threadIdx.x * 8;
+      uint32_t digit[8], w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (i0 < hi) {
+        float v[8];
+        load(i0, v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          // after the first round only ~1/256 of the entries still carry the selected prefix: test the (cheap) key first
+          // and evaluate the weight (an expf) for those only
+          const uint32_t k = keyf(v[e]);
+          digit[e] = (k >> shift) & 255;
+          if (round == 0 || (k >> (shift + 8)) == (prefix >> (shift + 8))) w[e] = __float2uint_rn(wf(v[e]) * SAMP_FIX);
         }
       }
-      if (__any_sync(0xffffffffu, digit != 0xffffffffu)) {  // warp-uniform: most warps of rounds 1..3 have nothing to add
-        const uint32_t grp = __match_any_sync(0xffffffffu, digit);
-        if (digit != 0xffffffffu) {
-          const uint32_t sum = __reduce_add_sync(grp, w);
-          if ((int)(threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&h[digit], sum);
-        }
-      }
+      hist_add8(h, digit, w);
     }
+    hist_fold(h);
     radix_round_pick(c, h, hsum, bcast, below, T, strict, /*descending=*/false);
     prefix |= bcast[0] << shift;
     below = bcast[1];
@@ -413,28 +474,31 @@ __device__ uint32_t select_weighted_asc(Cl& c, int lo, int hi, KeyF keyf, WF wf,
 }
 
 // k-th largest key (k >= 1) by count
-template <class KeyF>
-__device__ uint32_t select_kth_largest(Cl& c, int lo, int hi, KeyF keyf, int k, uint32_t (*hist)[256], uint32_t* hsum,
+template <class LoadF, class KeyF>
+__device__ uint32_t select_kth_largest(Cl& c, int lo, int hi, LoadF load, KeyF keyf, int k, uint32_t (*hist)[256 * HIST_COPIES], uint32_t* hsum,
                                        uint32_t* bcast) {
   uint32_t prefix = 0, above = 0;
   for (int round = 0; round < 4; ++round) {
     const int shift = 24 - 8 * round;
     uint32_t* h = hist[c.he & 1];
     ++c.he;
-    if (threadIdx.x < 256) h[threadIdx.x] = 0u;
-    __syncthreads();
-    for (int i0 = lo; i0 < hi; i0 += SAMP_THREADS) {  // warp-aggregated: one atomic per distinct digit per warp
-      const int i = i0 + threadIdx.x;
-      uint32_t digit = 0xffffffffu;  // not counted
-      if (i < hi) {
-        const uint32_t key = keyf(i);
-        if (round == 0 || (key >> (shift + 8)) == (prefix >> (shift + 8))) digit = (key >> shift) & 255;
+    hist_clear(h);
+    for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
+      const int i0 = base + threadIdx.x * 8;
+      uint32_t digit[8], w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (i0 < hi) {
+        float v[8];
+        load(i0, v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const uint32_t key = keyf(v[e]);
+          digit[e] = (key >> shift) & 255;
+          w[e] = round == 0 || (key >> (shift + 8)) == (prefix >> (shift + 8)) ? 1u : 0u;
+        }
       }
-      if (__any_sync(0xffffffffu, digit != 0xffffffffu)) {
-        const uint32_t grp = __match_any_sync(0xffffffffu, digit);
-        if (digit != 0xffffffffu && (int)(threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&h[digit], (uint32_t)__popc(grp));
-      }
+      hist_add8(h, digit, w);
     }
+    hist_fold(h);
     radix_round_pick(c, h, hsum, bcast, above, (uint32_t)k, false, /*descending=*/true);
     prefix |= bcast[0] << shift;
     above = bcast[1];
@@ -471,12 +535,15 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
   extern __shared__ __align__(16) uint8_t dyn_smem[];
   __shared__ float redf[2 * SAMP_WARPS];
   __shared__ int redi[SAMP_WARPS];
-  __shared__ uint32_t hist[2][256];
+  __shared__ uint32_t hist[2][256 * HIST_COPIES];
   __shared__ uint32_t hsum[256];
   __shared__ uint32_t bcast[4];
   __shared__ float xch[2][4];
   __shared__ float cand_v[MAX_TOPN];
   __shared__ int cand_i[MAX_TOPN];
+  __shared__ float list_v[SAMP_LIST];   // thread maxima, then the entries that can be among the slice's top-n
+  __shared__ int list_i[SAMP_LIST];
+  __shared__ int list_n;
   STL_ENTER(6);
   griddep_launch();
   griddep_wait();
@@ -521,7 +588,7 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
   ValIdx best{-INFINITY, -1};
   const bool do_typ = (c.p.flags & SAMPLE_TYPICAL) != 0 && !forced;
   const bool greedy_fast = greedy && !do_typ;  // argmax fused into the first sweep
-  auto consume8 = [&](const float (&xs)[8], int i0) {
+  auto consume8 = [&](float (&xs)[8], int i0) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const float x = xs[e];
@@ -531,10 +598,12 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
       } else if (x != -INFINITY) {
         ms.s += __expf(x - ms.m);
       }
-      if (greedy_fast) {
-        const float yy = process(c, i0 + e, x);
-        if (best.i < 0 || yy > best.v) best = {yy, i0 + e};  // ascending i: strict > keeps the lowest index
-      }
+    }
+    if (greedy_fast) {
+      process8(c, i0, xs);
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (best.i < 0 || xs[e] > best.v) best = {xs[e], i0 + e};  // ascending i: strict > keeps the lowest index
     }
   };
   constexpr int P1_UNROLL = 4;  // 16-byte loads in flight per thread (64 KB per SM)
@@ -561,6 +630,7 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
     }
   }
   if (cache_x) c.xc = xs;  // visible to every thread after the barriers of the reductions below
+  const float thread_max = ms.m;
   int token;
   if (greedy_fast) {
     // one exchange for both reductions: {max, sum-exp, best value, best index}
@@ -587,24 +657,27 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
   // ---- typical-p threshold (R8): entropy, then weighted select over s = |-lp - H| ascending
   if (do_typ) {
     float part = 0.f;
-    for (int i = lo + threadIdx.x; i < hi; i += SAMP_THREADS) {
-      const float lp = (load_x(c, i) - c.raw_max) - c.raw_logz;
-      const float p = expf(lp);
-      const float term = lp * p;
-      if (term == term) part += term;  // nansum
+    for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
+      float x[8];
+      load_slice8(c, i0, x);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float lp = (x[e] - c.raw_max) - c.raw_logz;
+        const float p = expf(lp);
+        const float term = lp * p;
+        if (term == term) part += term;  // nansum
+      }
     }
     c.ent = -cluster_sumf(cl, part, redf, xch);
     const float rm = c.raw_max, lz = c.raw_logz, ent = c.ent;
-    const LT* xx = c.xc != nullptr ? c.xc - lo : c.x;  // indexed xx[i]; the staged copy is already masked
     const RowCtx<LT>& cr = c;
-    const bool mask_here = MASKED && c.allow != nullptr && c.xc == nullptr;
-    auto xval = [=, &cr](int i) { return mask_here ? load_x_any(cr, i) : lt2f(xx[i]); };
-    auto keyf = [=](int i) {
-      const float lp = (xval(i) - rm) - lz;
+    auto load = [&cr](int i0, float (&v)[8]) { load_slice8(cr, i0, v); };
+    auto keyf = [=](float x) {
+      const float lp = (x - rm) - lz;
       return __float_as_uint(fabsf((-lp) - ent));
     };
-    auto wf = [=](int i) { return expf((xval(i) - rm) - lz); };
-    const uint32_t k = select_weighted_asc(cl, lo, hi, keyf, wf, c.p.typical_p, false, hist, hsum, bcast);
+    auto wf = [=](float x) { return expf((x - rm) - lz); };
+    const uint32_t k = select_weighted_asc(cl, lo, hi, load, keyf, wf, c.p.typical_p, false, hist, hsum, bcast);
     c.typ_thr = __uint_as_float(k);
     c.typical = true;
   }
@@ -612,22 +685,37 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
     token = (int)c.p.seed_lo;
   } else if (greedy) {
     if (!greedy_fast) {  // typical-p + greedy (method SAMPLE, temperature 0): argmax after the mask is known
-      for (int i = lo + threadIdx.x; i < hi; i += SAMP_THREADS) {
-        const float yy = process(c, i, load_x(c, i));
-        if (best.i < 0 || yy > best.v) best = {yy, i};
+      for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
+        float x[8];
+        load_slice8(c, i0, x);
+        process8(c, i0, x);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (best.i < 0 || x[e] > best.v) best = {x[e], i0 + e};
       }
       best = cluster_argmax(cl, best, redf, redi, xch);
       token = best.i;
     }
   } else {
-    // ---- processed logits / temperature -> scratch, running max
+    // ---- processed logits / temperature and their maximum; kept in y for what follows, but behind typical-p alone, where few
+    // entries are left, made again
     float mx = -INFINITY;
     const float temp = c.p.temperature;
-    for (int i = lo + threadIdx.x; i < hi; i += SAMP_THREADS) {
-      float v = process(c, i, load_x(c, i));
-      v = __fdiv_rn(v, temp);
-      y[i] = v;
-      mx = fmaxf(mx, v);
+    const bool use_topk = c.p.top_k > 0 && c.p.top_k < V, use_topp = c.p.top_p < 1.0f, keep_y = use_topk || use_topp || !c.typical;
+    auto scaled8 = [&](int i0, float (&v)[8]) {
+      load_slice8(c, i0, v);
+      process8(c, i0, v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (v[e] != -INFINITY) v[e] = __fdiv_rn(v[e], temp);   // (-inf behind typical-p: the quotient is -inf too)
+    };
+    auto load_y = [=](int i0, float (&v)[8]) { load_x8(y, i0, v); };
+    for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
+      float v[8];
+      scaled8(i0, v);
+      if (keep_y) store_x8(y + i0, v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) mx = fmaxf(mx, v[e]);
     }
     {
       MaxSum t = cluster_maxsum(cl, MaxSum{mx, 0.f}, redf, xch);
@@ -635,37 +723,42 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
     }
     // ---- top-k (S6): keep y >= k-th largest value
     float lo_thr = -INFINITY;
-    if (c.p.top_k > 0 && c.p.top_k < V) {
-      auto keyf = [=](int i) { return f2key(y[i]); };
-      lo_thr = key2f(select_kth_largest(cl, lo, hi, keyf, c.p.top_k, hist, hsum, bcast));
+    if (use_topk) {
+      auto keyf = [](float v) { return f2key(v); };
+      lo_thr = key2f(select_kth_largest(cl, lo, hi, load_y, keyf, c.p.top_k, hist, hsum, bcast));
     }
     // ---- top-p (S6): drop the low-probability tail whose cumulative mass <= 1 - p
-    if (c.p.top_p < 1.0f) {
+    if (use_topp) {
       float part = 0.f;
-      for (int i = lo + threadIdx.x; i < hi; i += SAMP_THREADS) {
-        const float v = y[i];
-        if (v >= lo_thr) part += expf(v - mx);
+      for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
+        float v[8];
+        load_y(i0, v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (v[e] >= lo_thr) part += expf(v[e] - mx);
       }
       const float z = cluster_sumf(cl, part, redf, xch);
       const float lt = lo_thr;
-      auto keyf = [=](int i) { return f2key(y[i]); };
-      auto wf = [=](int i) {
-        const float v = y[i];
-        return (v >= lt) ? expf(v - mx) / z : 0.f;
-      };
-      const uint32_t k = select_weighted_asc(cl, lo, hi, keyf, wf, 1.0f - c.p.top_p, true, hist, hsum, bcast);
+      auto keyf = [](float v) { return f2key(v); };
+      auto wf = [=](float v) { return (v >= lt) ? expf(v - mx) / z : 0.f; };
+      const uint32_t k = select_weighted_asc(cl, lo, hi, load_y, keyf, wf, 1.0f - c.p.top_p, true, hist, hsum, bcast);
       lo_thr = fmaxf(lo_thr, key2f(k));
     }
     // ---- exponential race == Gumbel max over the kept set
     const uint2 key = make_uint2(c.p.seed_lo, c.p.seed_hi);
     ValIdx bs{-INFINITY, -1};
-    for (int i = lo + threadIdx.x; i < hi; i += SAMP_THREADS) {
-      const float v = y[i];
-      if (v >= lo_thr && v != -INFINITY) {
-        const uint4 rnd = philox4x32(make_uint4((uint32_t)i, c.p.step, 0u, 0u), key);
-        const float u = ((float)(rnd.x >> 8) + 0.5f) * (1.0f / 16777216.0f);
-        const float score = (v - mx) - logf(-logf(u));
-        if (bs.i < 0 || score > bs.v) bs = {score, i};
+    for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
+      float v[8];
+      if (keep_y) load_y(i0, v);
+      else scaled8(i0, v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        if (v[e] >= lo_thr && v[e] != -INFINITY) {
+          const uint4 rnd = philox4x32(make_uint4((uint32_t)(i0 + e), c.p.step, 0u, 0u), key);
+          const float u = ((float)(rnd.x >> 8) + 0.5f) * (1.0f / 16777216.0f);
+          const float score = (v[e] - mx) - logf(-logf(u));
+          if (bs.i < 0 || score > bs.v) bs = {score, i0 + e};
+        }
       }
     }
     bs = cluster_argmax(cl, bs, redf, redi, xch);
@@ -682,38 +775,101 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
   }
 
   // ---- logprob / rank / top-n on the RAW log-softmax (S1, S8)
+  // The row's top-n is contained in the union of the slices' top-n.  A slice's n-th largest entry is no smaller than the n-th
+  // largest of its threads' maxima (each a different entry, known from the first sweep), so the sweep that counts the token's
+  // rank also lists the entries from that bound on, a few more than n.
   float tok_lp = 0.f;
   int rank = 0;
-  if (want_lp) {
-    tok_lp = (load_x_any(c, token) - c.raw_max) - c.raw_logz;
-    int cnt = 0;
-    for (int i = lo + threadIdx.x; i < hi; i += SAMP_THREADS) {
-      const float lp = (load_x(c, i) - c.raw_max) - c.raw_logz;
-      cnt += (lp >= tok_lp) ? 1 : 0;
-    }
-    rank = cluster_sumi(cl, cnt, redi, xch);
-  }
   SampleOut* o = outs + r;
   const int n_topn = min(c.p.n_topn, MAX_TOPN);
+  float bound = INFINITY;
   if (n_topn > 0) {
-    // The row's top-n is contained in the union of the slices' top-n: every CTA extracts its own n best
-    // (value desc, index asc) with n block reductions, ONE cluster barrier publishes the lists, and warp 0 of the
-    // cluster's rank-0 CTA merges the <= 8 x 12 candidates in registers.
-    float prev_v = INFINITY;
-    int prev_i = -1;
-    for (int n = 0; n < n_topn; ++n) {
-      ValIdx b{-INFINITY, -1};
-      for (int i = lo + threadIdx.x; i < hi; i += SAMP_THREADS) {
-        const float v = load_x(c, i);
-        const bool after = (v < prev_v) || (v == prev_v && i > prev_i);
-        if (after && (b.i < 0 || v > b.v)) b = {v, i};
+    __syncthreads();
+    list_v[threadIdx.x] = thread_max;
+    if (threadIdx.x == 0) list_n = 0;
+    __syncthreads();
+    if (threadIdx.x < 32) {   // the n-th largest of the 1024 maxima, taken out one by one
+      float mine = -INFINITY;
+      int at = 0;
+      auto rescan = [&]() {
+        mine = -INFINITY;
+        for (int j = 0; j < SAMP_THREADS / 32; ++j) {
+          const float v = list_v[j * 32 + threadIdx.x];
+          if (v > mine) { mine = v; at = j; }
+        }
+      };
+      rescan();
+      float m = -INFINITY;
+      for (int n = 0; n < n_topn; ++n) {
+        m = mine;
+#pragma unroll
+        for (int o2 = 16; o2 > 0; o2 >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o2));
+        const uint32_t who = __ballot_sync(0xffffffffu, mine == m);
+        if ((int)threadIdx.x == __ffs(who) - 1) {
+          list_v[at * 32 + threadIdx.x] = -INFINITY;
+          rescan();
+        }
       }
-      b = block_argmax(b, redf, redi);
-      prev_v = b.v;
-      prev_i = b.i;
-      if (threadIdx.x == 0) {
-        cand_v[n] = b.v;
-        cand_i[n] = b.i;
+      if (threadIdx.x == 0) bcast[0] = __float_as_uint(m);
+    }
+    __syncthreads();
+    bound = __uint_as_float(bcast[0]);
+  }
+  const bool listed = n_topn > 0 && bound > -INFINITY;   // (-inf: fewer than n entries are allowed in this slice)
+  if (want_lp || listed) {
+    if (want_lp) tok_lp = (load_x_any(c, token) - c.raw_max) - c.raw_logz;
+    int cnt = 0;
+    for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
+      float x[8];
+      load_slice8(c, i0, x);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float lp = (x[e] - c.raw_max) - c.raw_logz;
+        cnt += (lp >= tok_lp) ? 1 : 0;
+        if (listed && x[e] >= bound) {
+          const int at = atomicAdd(&list_n, 1);
+          if (at < SAMP_LIST) {
+            list_v[at] = x[e];
+            list_i[at] = i0 + e;
+          }
+        }
+      }
+    }
+    if (want_lp) rank = cluster_sumi(cl, cnt, redi, xch);
+  }
+  if (n_topn > 0) {
+    // every CTA extracts its own n best (value desc, index asc), ONE cluster barrier publishes the lists, and warp 0 of the
+    // cluster's rank-0 CTA merges the <= 8 x 12 candidates in registers.
+    __syncthreads();
+    const int found = listed ? list_n : SAMP_LIST + 1;
+    if (found <= SAMP_LIST) {   // (at least n: the maxima that made the bound are among them)
+      if ((int)threadIdx.x < found) {
+        const float v = list_v[threadIdx.x];
+        const int i = list_i[threadIdx.x];
+        int before = 0;
+        for (int j = 0; j < found; ++j) before += (list_v[j] > v || (list_v[j] == v && list_i[j] < i)) ? 1 : 0;
+        if (before < n_topn) {
+          cand_v[before] = v;
+          cand_i[before] = i;
+        }
+      }
+    } else {   // masked to a few tokens, or more ties than the list holds: one sweep per entry
+      float prev_v = INFINITY;
+      int prev_i = -1;
+      for (int n = 0; n < n_topn; ++n) {
+        ValIdx b{-INFINITY, -1};
+        for (int i = lo + threadIdx.x; i < hi; i += SAMP_THREADS) {
+          const float v = load_x(c, i);
+          const bool after = (v < prev_v) || (v == prev_v && i > prev_i);
+          if (after && (b.i < 0 || v > b.v)) b = {v, i};
+        }
+        b = block_argmax(b, redf, redi);
+        prev_v = b.v;
+        prev_i = b.i;
+        if (threadIdx.x == 0) {
+          cand_v[n] = b.v;
+          cand_i[n] = b.i;
+        }
       }
     }
     cl.sync();
