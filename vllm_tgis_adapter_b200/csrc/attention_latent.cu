@@ -461,6 +461,240 @@ latent_attn_mma_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __r
   }
 }
 
+// ---- prompts: four of those tiles of one sequence per CTA ----------------------------------------------------------------
+// With sixteen heads a tile holds one token, and in a prompt neighbouring tokens stream the same cache rows: 16 rows of S for
+// every block staged.  Here a CTA takes up to 64 (token, head) rows, four M tiles against each staged 32-row block:
+//   scores  warp w: M tile w & 3, keys 16 (w >> 2) .. + 15, two interleaved k chains;
+//   softmax fp32, four lanes per row with eight keys each;
+//   output  warp w: columns [8 NTW w, 8 NTW (w + 1)) of all four M tiles (128 fp32 accumulators a thread at kv_rank 512), so that
+//           a fragment of C serves four MMAs.
+// One CTA of eight warps per SM (163 KB at row 576), so what bounds it are the latencies between the three barriers of a
+// block.  Measured: prompts of 937, 767, 68, 220 and 56 tokens, 16 heads, row 576: 360 us a launch before, 235 here.
+constexpr int LATW_ROWS = 4 * LATENT_PAIRS;
+constexpr int LATW_LDS = 36, LATW_LDP = 40;   // padded rows of S (floats) and P (bf16)
+inline size_t lat_wide_smem(int D) {
+  return (size_t)(LATW_ROWS + 2 * KV_BLOCK) * lat_ldq(D) * 2 + (size_t)LATW_ROWS * (LATW_LDS * 4 + LATW_LDP * 2 + 2 * 4);
+}
+template <int NTW>  // NTW * 64 >= kv_rank
+__global__ void __launch_bounds__(LAT_THREADS, 1)
+latent_attn_wide_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __restrict__ cache, const AttnSeq* __restrict__ seqs,
+                        const LatentTile* __restrict__ tiles, int tile_tokens, const int32_t* __restrict__ block_table, int bt_stride,
+                        void* __restrict__ o_lat, int o_dtype, LatentGeom g) {
+  using bf = __nv_bfloat16;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int D = g.row(), R = g.kv_rank, LDQ = lat_ldq(D);
+  bf* Qs = reinterpret_cast<bf*>(smem_raw);                                  // [64][LDQ]
+  bf* Ks = Qs + (size_t)LATW_ROWS * LDQ;                                     // [2][32][LDQ]
+  float* Sp = reinterpret_cast<float*>(Ks + (size_t)2 * KV_BLOCK * LDQ);     // [64][LATW_LDS]
+  bf* Ps = reinterpret_cast<bf*>(Sp + LATW_ROWS * LATW_LDS);                 // [64][LATW_LDP]
+  float* corr_s = reinterpret_cast<float*>(Ps + LATW_ROWS * LATW_LDP);       // [64]
+  float* l_s = corr_s + LATW_ROWS;                                           // [64]
+  griddep_launch();
+  griddep_wait();
+  const LatentTile tile = tiles[blockIdx.x];
+  if (tile.q0 % (4 * tile_tokens) != 0) return;   // the first of its four tiles does the work
+  const AttnSeq sq = seqs[tile.seq];
+  const int h0 = blockIdx.y * LATENT_PAIRS, nh = min(g.heads - h0, LATENT_PAIRS);
+  const int nq = min(4 * tile_tokens, sq.q_len - tile.q0), rows = nq * nh, n_mt = (rows + 15) / 16;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int pos0 = sq.kv_len - sq.q_len + tile.q0, row0 = sq.q_start + tile.q0;
+  {  // zero what no copy fills (unused rows, k padding), then Q, scaled and rounded to bf16 once
+    uint32_t* z = reinterpret_cast<uint32_t*>(smem_raw);
+    for (int i = rows * LDQ / 2 + tid; i < LATW_ROWS * LDQ / 2; i += LAT_THREADS) z[i] = 0u;
+    const int pad = LDQ - D;
+    for (int i = tid; i < rows * pad; i += LAT_THREADS) Qs[(size_t)(i / pad) * LDQ + D + i % pad] = __float2bfloat16_rn(0.f);
+    for (int i = tid; i < 2 * KV_BLOCK * pad; i += LAT_THREADS) Ks[(size_t)(i / pad) * LDQ + D + i % pad] = __float2bfloat16_rn(0.f);
+    const int d4 = D / 4;
+#pragma unroll 4
+    for (int e = tid; e < rows * d4; e += LAT_THREADS) {
+      const int p = e / d4, d = (e - p * d4) * 4, tq = p / nh, h = h0 + p - tq * nh;
+      const float4 v = *reinterpret_cast<const float4*>(q_abs + ((size_t)(row0 + tq) * g.heads + h) * D + d);
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x * g.scale, v.y * g.scale), hi = __floats2bfloat162_rn(v.z * g.scale, v.w * g.scale);
+      uint2 o;
+      o.x = *reinterpret_cast<const uint32_t*>(&lo);
+      o.y = *reinterpret_cast<const uint32_t*>(&hi);
+      *reinterpret_cast<uint2*>(Qs + (size_t)p * LDQ + d) = o;
+    }
+  }
+  const int pos_last = pos0 + nq - 1, kmin = g.window > 0 ? max(0, pos0 - g.window + 1) : 0;
+  const int blk0 = kmin / KV_BLOCK, blk1 = pos_last / KV_BLOCK;
+  const int32_t* bt = block_table + (size_t)sq.block_row * bt_stride;
+  const uint32_t per_row = (uint32_t)D / 8, magic = ((1u << 20) + per_row - 1) / per_row;   // c / per_row for c < 32 per_row <= 2^15
+  auto load_block = [&](int blk, int st) {
+    const bf* src = cache + (size_t)bt[blk] * KV_BLOCK * D;
+    bf* dst = Ks + (size_t)st * KV_BLOCK * LDQ;
+#pragma unroll 4
+    for (uint32_t c = tid; c < KV_BLOCK * per_row; c += LAT_THREADS)
+      lat_cp_async_16(dst + c * 8 + ((c * magic) >> 20) * (uint32_t)(LDQ - D), src + c * 8);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  // softmax: four lanes per row, eight keys each
+  const int sr = tid >> 2, sk = (tid & 3) * 8, sposq = sr < rows ? pos0 + sr / nh : -1;
+  float m_run = -FLT_MAX, l_run = 0.f;
+  float acc[4][NTW][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < NTW; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+  const int KS = (D + 15) / 16, mt = warp & 3, kh = warp >> 2, gq = lane >> 2, t2 = (lane & 3) * 2;
+  const bf* q_frag = Qs + (size_t)(mt * 16 + (lane & 15)) * LDQ + (lane >> 4) * 8;
+  const int k_frag = (kh * 16 + (lane & 7) + ((lane >> 4) & 1) * 8) * LDQ + ((lane >> 3) & 1) * 8;
+
+  load_block(blk0, 0);
+  for (int blk = blk0; blk <= blk1; ++blk) {
+    const int st = (blk - blk0) & 1;
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();  // block `blk` has landed for everyone; everyone is done with the other buffer, P, S and corr
+    if (blk < blk1) load_block(blk + 1, st ^ 1);
+    const bf* Kb = Ks + (size_t)st * KV_BLOCK * LDQ;
+    if (mt < n_mt) {  // ---- scores
+      float c[2][2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) c[i][j][e] = 0.f;
+      const bf* kf = Kb + k_frag;
+#pragma unroll 3
+      for (int ks = 0; ks + 1 < KS; ks += 2) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          uint32_t a[4], b[4];
+          lat_ldsm_x4(a, q_frag + (ks + i) * 16);
+          lat_ldsm_x4(b, kf + (ks + i) * 16);
+          lat_mma(c[i][0], a, b[0], b[1]);
+          lat_mma(c[i][1], a, b[2], b[3]);
+        }
+      }
+      if (KS & 1) {
+        uint32_t a[4], b[4];
+        lat_ldsm_x4(a, q_frag + (KS - 1) * 16);
+        lat_ldsm_x4(b, kf + (KS - 1) * 16);
+        lat_mma(c[0][0], a, b[0], b[1]);
+        lat_mma(c[0][1], a, b[2], b[3]);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float* sp = Sp + (size_t)(mt * 16 + gq) * LATW_LDS + kh * 16 + j * 8 + t2;
+        *reinterpret_cast<float2*>(sp) = make_float2(c[0][j][0] + c[1][j][0], c[0][j][1] + c[1][j][1]);
+        *reinterpret_cast<float2*>(sp + 8 * LATW_LDS) = make_float2(c[0][j][2] + c[1][j][2], c[0][j][3] + c[1][j][3]);
+      }
+    }
+    __syncthreads();
+    {  // ---- softmax
+      float x[8];
+      const float4 xa = *reinterpret_cast<const float4*>(Sp + sr * LATW_LDS + sk), xb = *reinterpret_cast<const float4*>(Sp + sr * LATW_LDS + sk + 4);
+      x[0] = xa.x; x[1] = xa.y; x[2] = xa.z; x[3] = xa.w; x[4] = xb.x; x[5] = xb.y; x[6] = xb.z; x[7] = xb.w;
+      const int last = sposq - (blk * KV_BLOCK + sk), first = g.window > 0 ? last - g.window + 1 : 0;   // visible: first <= e <= last
+      float m_new = -FLT_MAX;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        x[e] = e <= last && e >= first ? x[e] : -FLT_MAX;
+        m_new = fmaxf(m_new, x[e]);
+      }
+      m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 1));
+      m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 2));
+      m_new = fmaxf(m_new, m_run);
+      // nothing visible so far (m_new still the sentinel): all weights 0, state unchanged
+      const float corr = m_new == -FLT_MAX ? 1.f : expf(m_run - m_new);
+      float sum = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        x[e] = x[e] == -FLT_MAX ? 0.f : expf(x[e] - m_new);
+        sum += x[e];
+      }
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      l_run = l_run * corr + sum;
+      m_run = m_new;
+      uint4 pk;
+      uint32_t* w = &pk.x;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const __nv_bfloat162 h2 = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
+        w[e] = *reinterpret_cast<const uint32_t*>(&h2);
+      }
+      *reinterpret_cast<uint4*>(Ps + sr * LATW_LDP + sk) = pk;
+      if (sk == 0) corr_s[sr] = corr;
+    }
+    __syncthreads();
+    {  // ---- output: rescale, then O += P C over this warp's columns
+      const int col0 = warp * 8 * NTW;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (i >= n_mt) break;
+        const float c_lo = corr_s[i * 16 + gq], c_hi = corr_s[i * 16 + gq + 8];
+        if (__any_sync(0xffffffffu, c_lo != 1.f || c_hi != 1.f)) {
+#pragma unroll
+          for (int j = 0; j < NTW; ++j) {
+            acc[i][j][0] *= c_lo; acc[i][j][1] *= c_lo; acc[i][j][2] *= c_hi; acc[i][j][3] *= c_hi;
+          }
+        }
+      }
+      uint32_t a[4][2][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < n_mt) {
+          lat_ldsm_x4(a[i][0], Ps + (size_t)(i * 16 + (lane & 15)) * LATW_LDP + (lane >> 4) * 8);
+          lat_ldsm_x4(a[i][1], Ps + (size_t)(i * 16 + (lane & 15)) * LATW_LDP + 16 + (lane >> 4) * 8);
+        }
+#pragma unroll
+      for (int j = 0; j < NTW; ++j) {
+        const int n0 = col0 + j * 8;
+        if (n0 < R) {
+          uint32_t b[4];
+          lat_ldsm_x4_trans(b, Kb + (size_t)lane * LDQ + n0);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (i < n_mt) {
+              lat_mma(acc[i][j], a[i][0], b[0], b[1]);
+              lat_mma(acc[i][j], a[i][1], b[2], b[3]);
+            }
+        }
+      }
+    }
+  }
+  if (sk == 0 && sr < rows) l_s[sr] = 1.f / (l_run + (g.sink != nullptr ? expf(g.sink[h0 + sr % nh] - m_run) : 0.f));
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {
+      const int p = i * 16 + gq + hf * 8;
+      if (p >= rows) continue;
+      const int tq = p / nh, h = h0 + p - tq * nh;
+      const size_t o = ((size_t)(row0 + tq) * g.heads + h) * R;
+      const float inv = l_s[p];
+#pragma unroll
+      for (int j = 0; j < NTW; ++j) {
+        const int n = warp * 8 * NTW + j * 8 + t2;   // (kv_rank is a multiple of 8)
+        if (n < R) {
+          const float v0 = acc[i][j][hf * 2] * inv, v1 = acc[i][j][hf * 2 + 1] * inv;
+          if (o_dtype == DT_BF16) *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<bf*>(o_lat) + o + n) = __floats2bfloat162_rn(v0, v1);
+          else *reinterpret_cast<float2*>(reinterpret_cast<float*>(o_lat) + o + n) = make_float2(v0, v1);
+        }
+      }
+    }
+}
+
+template <int NTW>
+cudaError_t launch_attn_wide(const float* q_abs, const void* cache, const AttnSeq* seqs, const LatentTile* tiles, int n_tiles,
+                             int tile_tokens, const int32_t* block_table, int bt_stride, void* o_lat, int o_dtype, const LatentGeom& g,
+                             cudaStream_t stream) {
+  const size_t smem = lat_wide_smem(g.row());
+  static size_t attr_bytes = 0;
+  if (smem > attr_bytes) {
+    const cudaError_t e = cudaFuncSetAttribute(latent_attn_wide_kernel<NTW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    attr_bytes = smem;
+  }
+  return launch_k(latent_attn_wide_kernel<NTW>, dim3(n_tiles, (g.heads + LATENT_PAIRS - 1) / LATENT_PAIRS), dim3(LAT_THREADS), smem, stream,
+                  q_abs, reinterpret_cast<const __nv_bfloat16*>(cache), seqs, tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g);
+}
+
 // o_lat[pair] = sum_z e^(m_z - M) acc_z / sum_z e^(m_z - M) l_z over the splits in ascending order, M = max_z m_z.
 // One CTA per (tile, head group, pair); the split weights are worked out once in shared memory.
 constexpr int LATENT_MAX_SPLITS = 64;
@@ -596,7 +830,7 @@ cudaError_t latent_q_rope_launch(const void* q, int q_dtype, const LatentGeom& g
 cudaError_t latent_attn_launch(const float* q_abs, const void* cache, int dtype, const AttnSeq* seqs,
                                const LatentTile* tiles, int n_tiles, const int32_t* block_table, int bt_stride,
                                void* o_lat, int o_dtype, const LatentGeom& g, cudaStream_t stream, float* split_ws,
-                               size_t split_ws_floats, int max_kv_len, int num_sms, int* n_launched) {
+                               size_t split_ws_floats, int max_kv_len, int num_sms, int* n_launched, int n_seqs, int tile_tokens) {
   if (n_launched) *n_launched = n_tiles > 0 ? 1 : 0;
   if (n_tiles <= 0) return cudaSuccess;
   if (latent_mma_eligible(cache, dtype, g)) {
@@ -619,6 +853,13 @@ cudaError_t latent_attn_launch(const float* q_abs, const void* cache, int dtype,
         n_splits = z;
     }
     if (n_launched && n_splits > 1) *n_launched = 2;  // + the merge kernel
+    // prompts (four tiles of a sequence and more on average): the wide kernel.  Below that its CTAs would hold one M tile each.
+    if (n_splits == 1 && n_seqs > 0 && tile_tokens > 0 && tile_tokens <= latent_tile_tokens(g.heads) && n_tiles >= 4 * n_seqs &&
+        lat_wide_smem(g.row()) <= 227 * 1024 && (reinterpret_cast<uintptr_t>(q_abs) & 15) == 0 && (reinterpret_cast<uintptr_t>(o_lat) & 15) == 0) {
+      if (g.kv_rank <= 128) return launch_attn_wide<2>(q_abs, cache, seqs, tiles, n_tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g, stream);
+      if (g.kv_rank <= 256) return launch_attn_wide<4>(q_abs, cache, seqs, tiles, n_tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g, stream);
+      return launch_attn_wide<8>(q_abs, cache, seqs, tiles, n_tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g, stream);
+    }
     if (g.kv_rank <= 128) return launch_attn_mma<2>(q_abs, cache, seqs, tiles, n_tiles, block_table, bt_stride, o_lat, o_dtype, g, stream, split_ws, n_splits);
     if (g.kv_rank <= 256) return launch_attn_mma<4>(q_abs, cache, seqs, tiles, n_tiles, block_table, bt_stride, o_lat, o_dtype, g, stream, split_ws, n_splits);
     return launch_attn_mma<8>(q_abs, cache, seqs, tiles, n_tiles, block_table, bt_stride, o_lat, o_dtype, g, stream, split_ws, n_splits);

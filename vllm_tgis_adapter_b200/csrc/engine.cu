@@ -2687,7 +2687,7 @@ struct tgis_engine {
       }
       int attn_launches = 0;
       CK(latent_attn_launch(pnx_qabs, l.cache, A, d_seqs, ds<LatentTile>(off_ltiles), step_n_ltiles, d_bt, bt_stride, pnx_olat, A, g,
-                            stream, pnx_attn_ws, pnx_attn_ws_floats, step_max_kv, num_sms, &attn_launches));
+                            stream, pnx_attn_ws, pnx_attn_ws_floats, step_max_kv, num_sms, &attn_launches, S, pnx_tile_tokens));
       n_launches += attn_launches - 1;
       {  // o_h = W_uv,h o_lat_h  (times the head's gate where the layer has one)
         GemmAny a{};
@@ -3086,7 +3086,7 @@ struct tgis_engine {
       }
       int attn_launches = 0;
       CK(latent_attn_launch(pnx_qabs, l.cache, A, d_seqs, d_tiles, step_n_ltiles, d_bt, bt_stride, pnx_olat, A, g, stream,
-                            pnx_attn_ws, pnx_attn_ws_floats, step_max_kv, num_sms, &attn_launches));
+                            pnx_attn_ws, pnx_attn_ws_floats, step_max_kv, num_sms, &attn_launches, S, pnx_tile_tokens));
       n_launches += attn_launches - 1;  // (one attention launch is part of the count below)
       {  // o_h = gate_h * W_uv,h o_lat_h
         GemmAny a{};

@@ -412,7 +412,8 @@ constexpr int LATENT_SPLIT_BLOCKS = 4;
 cudaError_t latent_attn_launch(const float* q_abs, const void* cache, int dtype, const AttnSeq* seqs,
                                const LatentTile* tiles, int n_tiles, const int32_t* block_table, int bt_stride,
                                void* o_lat, int o_dtype, const LatentGeom& g, cudaStream_t stream, float* split_ws = nullptr,
-                               size_t split_ws_floats = 0, int max_kv_len = 0, int num_sms = 148, int* n_launched = nullptr);
+                               size_t split_ws_floats = 0, int max_kv_len = 0, int num_sms = 148, int* n_launched = nullptr,
+                               int n_seqs = 0, int tile_tokens = 0);  // sequences of the step, tokens of a full tile (0: unknown)
 
 // ---- attention_capped.cu: grouped-query attention with normed queries / keys and a soft cap on the scores ------------
 // No rotation: positions enter through the causal mask and a query temperature.  Per head: q <- rmsnorm(q) * w_q *

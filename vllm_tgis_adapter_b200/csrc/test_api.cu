@@ -605,7 +605,7 @@ int tgis_k_latent_attn(const float* q_abs, const void* cache, int32_t dt, const 
   int max_kv = 0;
   for (const AttnSeq& s : seqs) max_kv = std::max(max_kv, s.kv_len);
   KCK(latent_attn_launch(q_abs, cache, dt, d_seqs.p, d_tiles.p, (int)tiles.size(), d_bt.p, bt_stride, o_lat, o_dt, geom, 0,
-                         ws.p, ws_floats, max_kv, test_num_sms()));
+                         ws.p, ws_floats, max_kv, test_num_sms(), nullptr, n_seqs, qt));
   KCK(cudaDeviceSynchronize());
   return 0;
 }
