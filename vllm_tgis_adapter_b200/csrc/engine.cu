@@ -259,6 +259,7 @@ struct tgis_engine {
     void* w_o2 = nullptr;                          // the matrix memory's output projection
     float *qk_norm = nullptr, *mm_norm = nullptr, *mm_bias = nullptr, *out_l = nullptr, *out_r = nullptr;
     float *st_S = nullptr, *st_n = nullptr, *st_m = nullptr;   // per sequence slot: matrix, normaliser, running maximum
+    int32_t* st_done = nullptr;                                // ... and the column blocks that have read the latter two
     // TGIS_MIXER_SELECTIVE_SCAN
     void *w_x = nullptr, *w_dt = nullptr;
     float *conv_w = nullptr, *conv_b = nullptr, *dt_b = nullptr, *A_log = nullptr, *Dv = nullptr, *st_conv = nullptr;
@@ -1677,6 +1678,7 @@ struct tgis_engine {
           l.st_S = pnx_alloc<float>(slots * mH * s.mm_dim * s.mm_vdim, true);
           l.st_n = pnx_alloc<float>(slots * mH * s.mm_dim, true);
           l.st_m = pnx_alloc<float>(slots * mH, true);
+          l.st_done = pnx_alloc<int32_t>(slots * mH, true);
           pnx_expected_tensors += 19;  // left.{q,k,v,g,o,q.norm,k.norm,out}, right.{q,k,v,g,o,norm,i,i.b,f,f.b,out}
           m_q = std::max<size_t>(m_q, (size_t)H * s.dim);
           m_ov = std::max<size_t>(m_ov, (size_t)H * s.vdim);
@@ -2433,7 +2435,7 @@ struct tgis_engine {
       os.q_scale = 1.f / std::sqrt((float)s.mm_dim);
       os.ig = pnx_y1 + l.c_mi; os.fg = pnx_y1 + l.c_mf; os.ldg = ld; os.ig_b = l.mm_bias; os.fg_b = l.mm_bias + mH;
       os.gate_cap = s.gate_cap;
-      os.S = l.st_S; os.n = l.st_n; os.m = l.st_m;
+      os.S = l.st_S; os.n = l.st_n; os.m = l.st_m; os.done = l.st_done;
       os.out = flx_f1; os.ldo = mH * s.mm_vdim;
       os.heads = mH; os.dim = s.mm_dim; os.vdim = s.mm_vdim;
       CK(outer_scan_launch(os, d_seqs, S, d_tokslot, stream));

@@ -570,6 +570,7 @@ struct OuterScan {
   const float* step_raw; int lds; const float *step_b, *A_log, *D;   // SSD: [T, heads], [heads], [heads], [heads]
   const float* decay;                          // LIGHTNING, RETENTION: [heads]
   float inv_tau;                               // GLA
+  int32_t* done;                               // GATED: [slots][heads], zero between launches
 };
 cudaError_t outer_scan_launch(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot,
                               cudaStream_t stream);

@@ -423,8 +423,18 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
       if (i < D) Sg[(size_t)i * a.vdim] = S[j];
     }
   }
-  if (blockIdx.z == 0) {
-    if (MODE == OUTER_SCAN_GATED) {
+  // The normaliser and the running maximum belong to all column blocks of the head, each of which started from them.  More blocks
+  // than the chip holds at once do not start together, so only the one that gets here last may overwrite them.
+  if (MODE == OUTER_SCAN_GATED) {
+    __shared__ int last_block;
+    __syncthreads();   // every thread's rows of n and m are read
+    if (tid == 0) {
+      int32_t* done = a.done + (size_t)slot * a.heads + h;
+      last_block = gridDim.z == 1 || atomicAdd(done, 1) == (int)gridDim.z - 1;
+      if (last_block && gridDim.z > 1) *done = 0;
+    }
+    __syncthreads();
+    if (last_block) {
       float* ng = a.n + ((size_t)slot * a.heads + h) * D;
       if (lane == 0) {
 #pragma unroll
@@ -435,6 +445,8 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
       }
       if (tid == 0) a.m[(size_t)slot * a.heads + h] = m_run;
     }
+  }
+  if (blockIdx.z == 0) {
     if (a.x_last != nullptr && h == 0) {
       const float* src = a.x + (size_t)(sq.q_start + sq.q_len - 1) * a.width;
       for (int i = tid; i < a.width; i += OS_THREADS) a.x_last[(size_t)slot * a.width + i] = src[i];
@@ -817,6 +829,7 @@ cudaError_t outer_scan_launch(const OuterScan& a, const AttnSeq* seqs, int n_seq
     if (a.decay_raw == nullptr || a.w0 == nullptr || a.u == nullptr) return cudaErrorInvalidValue;
     return outer_scan_mode<OUTER_SCAN_HGRN>(a, seqs, n_seqs, tok_slot, stream);
   }
+  if (a.mode == OUTER_SCAN_GATED && a.done == nullptr) return cudaErrorInvalidValue;
   return a.mode == OUTER_SCAN_GATED ? outer_scan_mode<OUTER_SCAN_GATED>(a, seqs, n_seqs, tok_slot, stream)
                                     : outer_scan_mode<OUTER_SCAN_DECAY>(a, seqs, n_seqs, tok_slot, stream);
 }

@@ -848,6 +848,11 @@ int tgis_k_outer_scan(int32_t mode, const float* q, const float* k, const float*
   a.ig = ig; a.fg = fg; a.ldg = ldg; a.ig_b = ig_b; a.fg_b = fg_b; a.gate_cap = gate_cap;
   a.S = S; a.n = n; a.m = m; a.out = out; a.ldo = ldo; a.heads = heads; a.dim = dim; a.vdim = vdim;
   a.x = x; a.x_last = x_last; a.width = width;
+  Tmp<int32_t> done;
+  if (mode == OUTER_SCAN_GATED) {   // zeros for every slot the launch may name
+    KCK(done.upload(std::vector<int32_t>((size_t)heads * 4096, 0).data(), (size_t)heads * 4096));
+    a.done = done.p;
+  }
   KCK(outer_scan_launch(a, d_seqs.p, n_seqs, tok_slot, 0));
   KCK(cudaDeviceSynchronize());
   return 0;
