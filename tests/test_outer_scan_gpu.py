@@ -68,3 +68,35 @@ def test_gated_memory_carried_on(d, dv, H, slots, T):
         assert (mg[s].cpu().to(F64) - m1).abs().max() <= c * 12
         o = out[s * T:(s + 1) * T].cpu().to(F64).reshape(T, H, dv).transpose(0, 1)
         assert ((o - ref).abs() <= (c + d * 2.0 ** -24) * size).all()
+
+
+@pytest.mark.parametrize("d,H,T", [(64, 3, 37), (128, 1, 16), (256, 1, 17), (62, 2, 5), (3, 1, 20)])
+def test_decayed_memory_carried_on(d, H, T):
+    """A decay per row, keys that fill the row groups and keys that do not: out = q (S + u k v), then S = w S + k v."""
+    from vllm_tgis_adapter_b200.engine._lib import load_library
+
+    lib = load_library()
+    g = torch.Generator().manual_seed(d + T)
+    A = H * d
+    r, k, v, raw = (torch.randn(T, A, generator=g) for _ in range(4))
+    w0, u, S = torch.randn(A, generator=g) - 1.0, torch.randn(A, generator=g), torch.randn(1, H, d, d, generator=g)
+    dev = [t.cuda() for t in (r, k, v, raw, w0, u)]
+    Sg, out = S.cuda(), torch.full((T, A), float("nan"), device="cuda")
+    tok_slot = torch.zeros(T, dtype=torch.int32, device="cuda")
+    rc = lib.tgis_k_outer_scan(0, _p(dev[0]), _p(dev[1]), _p(dev[2]), A, A, A, ctypes.c_float(0.5), _p(dev[3]), A, _p(dev[4]), _p(dev[5]), None, None, 0,
+                               None, None, ctypes.c_float(0.0), _p(Sg), None, None, _p(out), A, H, d, d, None, None, 0,
+                               (ctypes.c_int32 * 4)(0, T, 9 + T, 0), 1, _p(tok_slot))
+    assert rc == 0
+    per_head = lambda t: t.to(F64).reshape(T, H, d)
+    q, kk, vv = per_head(r) * 0.5, per_head(k), per_head(v)
+    w = torch.exp(-torch.exp(per_head(raw) + w0.to(F64).reshape(H, d)))
+    S1, Sa, uu = S[0].to(F64), S[0].to(F64).abs(), u.to(F64).reshape(H, d)
+    # three roundings a step; a decay's inner exponential (up to ~e^3) passes its error of ~4 units on multiplied by its value
+    c = (3 + 4 * 20) * T * 2.0 ** -24
+    for t in range(T):
+        kv = kk[t, :, :, None] * vv[t, :, None, :]
+        o = torch.einsum("hd,hdv->hv", q[t], S1 + uu[:, :, None] * kv)
+        size = torch.einsum("hd,hdv->hv", q[t].abs(), Sa + uu[:, :, None].abs() * kv.abs())
+        assert ((out[t].cpu().to(F64).reshape(H, d) - o).abs() <= (c + (d + 4) * 2.0 ** -24) * size).all()
+        S1, Sa = w[t, :, :, None] * S1 + kv, w[t, :, :, None] * Sa + kv.abs()
+    assert ((Sg[0].cpu().to(F64) - S1).abs() <= c * Sa + 1e-30).all()

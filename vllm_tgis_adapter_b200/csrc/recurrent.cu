@@ -99,41 +99,136 @@ short_conv_silu_kernel(const float* __restrict__ xz, int ld, int inner, const fl
 
 // ------------------------------------------------------------------------------------------------ selective scan
 constexpr int SCAN_THREADS = 64, SCAN_CHUNK = 8, SCAN_REG_STATE = 16, SCAN_LPC = 4, SCAN_RPL = SCAN_REG_STATE / SCAN_LPC;
-// REG (state <= SCAN_REG_STATE): SCAN_LPC lanes share a channel, lane `sub` keeps states sub, sub + 4, ... and their decay rates in
-// registers and the lanes' partial outputs meet through two shuffles; otherwise one thread per channel, state in shared memory.
-// A chunk's B / C rows are staged in shared memory and its per-channel scalars (step size, input, gate) are fetched ahead
-// of the chunk's arithmetic, so the token loop waits for memory once per chunk, not once per token.
-template <bool REG>
+// the convolution's tail: inputs of the last taps - 1 positions (entry e: position end - (taps - 1) + e)
+__device__ __forceinline__ void scan_save_conv(const SelScan& a, const AttnSeq& sq, int slot, int c) {
+  const int K1 = a.taps - 1, first = sq.kv_len - sq.q_len;
+  float* cs = a.conv_state + (size_t)slot * K1 * a.inner + c;
+  for (int e = 0; e < K1; ++e) {   // ascending: entry e + q_len is read before it could be rewritten
+    const int pp = sq.kv_len - K1 + e;
+    float v = 0.f;
+    if (pp >= first) v = a.xz[(size_t)(sq.q_start + pp - first) * a.ld_xz + c];
+    else if (pp >= 0) v = cs[(size_t)(e + sq.q_len) * a.inner];
+    cs[(size_t)e * a.inner] = v;
+  }
+}
+// Up to SCAN_REG_STATE states: grid (sequences, ceil(inner / 16)), SCAN_LPC lanes share a channel; lane `sub` keeps states
+// 4 sub .. + 3 and their decay rates in registers.  A channel's tokens follow one another, so what is bound is the number of
+// instructions a token takes.  What the four lanes would all do is dealt out: of a chunk's eight tokens a lane fetches two (step
+// size, input, gate), takes their softplus, hands step size and input on by shuffle, and after the chunk receives the two tokens'
+// output sums (a transposing reduction: 6 shuffles for 8 tokens and 4 lanes) and gates and writes them.  B and C rows go through two
+// shared-memory buffers, read four states to a load; the next chunk is fetched while this one is worked through.
+__global__ void __launch_bounds__(SCAN_THREADS)
+selective_scan_reg_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t* __restrict__ tok_slot) {
+  constexpr int TPL = SCAN_CHUNK / SCAN_LPC, ROW = 2 * SCAN_REG_STATE, STAGE = SCAN_CHUNK * ROW / SCAN_THREADS;
+  static_assert(SCAN_LPC == 4 && SCAN_RPL == 4 && TPL == 2, "the reduction below deals eight tokens to four lanes");
+  __shared__ __align__(16) float BC[2][SCAN_CHUNK * ROW];   // per token: B | C, zeros behind the last state
+  griddep_launch();
+  griddep_wait();
+  const AttnSeq sq = seqs[blockIdx.x];
+  const int N = a.state, tid = threadIdx.x, lane = tid & 31, sub = tid % SCAN_LPC;
+  const int c = blockIdx.y * (SCAN_THREADS / SCAN_LPC) + tid / SCAN_LPC;
+  const bool live = c < a.inner;
+  const int slot = tok_slot[sq.q_start];
+  float* Sg = a.S + ((size_t)slot * a.inner + (live ? c : 0)) * N;
+  float Sr[SCAN_RPL], Ar[SCAN_RPL];
+#pragma unroll
+  for (int j = 0; j < SCAN_RPL; ++j) {
+    const int n = sub * SCAN_RPL + j;
+    Sr[j] = (live && sq.kv_len > sq.q_len && n < N) ? Sg[n] : 0.f;
+    Ar[j] = (live && n < N) ? -expf(a.A_log[(size_t)c * N + n]) : 0.f;
+  }
+  const float dtb = live ? a.dt_b[c] : 0.f, Dc = live ? a.D[c] : 0.f;
+  float p_bc[STAGE], p_dt[TPL], p_x[TPL], p_z[TPL];
+  auto fetch = [&](int t0) {
+    const int nt = min(SCAN_CHUNK, sq.q_len - t0);
+#pragma unroll
+    for (int k = 0; k < STAGE; ++k) {
+      const int e = tid + k * SCAN_THREADS, tt = e / ROW, which = (e % ROW) / SCAN_REG_STATE, n = e % SCAN_REG_STATE;
+      p_bc[k] = tt < nt && n < N ? a.proj[(size_t)(sq.q_start + t0 + tt) * a.ld_proj + a.dt_rank + which * N + n] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < TPL; ++i) {
+      const size_t row = (size_t)(sq.q_start + t0 + sub * TPL + i);
+      const bool ok = live && sub * TPL + i < nt;
+      p_dt[i] = ok ? a.dt_raw[row * a.inner + c] : 0.f;
+      p_x[i] = ok ? a.x[row * a.inner + c] : 0.f;
+      p_z[i] = ok ? a.xz[row * a.ld_xz + a.inner + c] : 0.f;
+    }
+  };
+  fetch(0);
+  for (int t0 = 0, buf = 0; t0 < sq.q_len; t0 += SCAN_CHUNK, buf ^= 1) {
+    const int nt = min(SCAN_CHUNK, sq.q_len - t0);
+    float dt[TPL], dx[TPL], xv[TPL], zv[TPL], y[SCAN_CHUNK];
+#pragma unroll
+    for (int k = 0; k < STAGE; ++k) BC[buf][tid + k * SCAN_THREADS] = p_bc[k];
+#pragma unroll
+    for (int i = 0; i < TPL; ++i) {
+      dt[i] = softplus_f(p_dt[i] + dtb);
+      xv[i] = p_x[i];
+      zv[i] = p_z[i];
+      dx[i] = dt[i] * xv[i];
+    }
+    __syncthreads();   // (the buffer written two chunks from now is this one: everyone is through with it by the barrier between)
+    if (t0 + SCAN_CHUNK < sq.q_len) fetch(t0 + SCAN_CHUNK);
+#pragma unroll
+    for (int tt = 0; tt < SCAN_CHUNK; ++tt) {
+      y[tt] = 0.f;
+      if (tt < nt) {
+        const int from = (lane & ~(SCAN_LPC - 1)) + tt / TPL;
+        const float dt_t = __shfl_sync(0xffffffffu, dt[tt % TPL], from), dx_t = __shfl_sync(0xffffffffu, dx[tt % TPL], from);
+        const float4 b4 = *reinterpret_cast<const float4*>(&BC[buf][tt * ROW + sub * SCAN_RPL]);
+        const float4 c4 = *reinterpret_cast<const float4*>(&BC[buf][tt * ROW + SCAN_REG_STATE + sub * SCAN_RPL]);
+        const float bn[4] = {b4.x, b4.y, b4.z, b4.w}, cn[4] = {c4.x, c4.y, c4.z, c4.w};
+#pragma unroll
+        for (int j = 0; j < SCAN_RPL; ++j) {
+          if (sub * SCAN_RPL + j < N) {
+            Sr[j] = fmaf(expf(dt_t * Ar[j]), Sr[j], dx_t * bn[j]);
+            y[tt] = fmaf(Sr[j], cn[j], y[tt]);
+          }
+        }
+      }
+    }
+    float half[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float keep = sub & 2 ? y[4 + i] : y[i], give = sub & 2 ? y[i] : y[4 + i];
+      half[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
+    }
+#pragma unroll
+    for (int i = 0; i < TPL; ++i) {
+      const float keep = sub & 1 ? half[2 + i] : half[i], give = sub & 1 ? half[i] : half[2 + i];
+      const float sum = keep + __shfl_xor_sync(0xffffffffu, give, 1);
+      if (live && sub * TPL + i < nt)
+        st_op(a.out, a.out_dtype, (size_t)(sq.q_start + t0 + sub * TPL + i) * a.inner + c, fmaf(Dc, xv[i], sum) * silu_f(zv[i]));
+    }
+  }
+  if (!live) return;
+#pragma unroll
+  for (int j = 0; j < SCAN_RPL; ++j)
+    if (sub * SCAN_RPL + j < N) Sg[sub * SCAN_RPL + j] = Sr[j];
+  if (sub == 0) scan_save_conv(a, sq, slot, c);
+}
+
+// More states: one thread per channel, state in shared memory.  A chunk's B / C rows are staged in shared memory and its per-channel
+// scalars (step size, input, gate) are fetched ahead of the chunk's arithmetic, so the token loop waits for memory once per chunk.
 __global__ void __launch_bounds__(SCAN_THREADS)
 selective_scan_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t* __restrict__ tok_slot) {
   extern __shared__ float scan_smem[];
   const int N = a.state;
   float* BC = scan_smem;                                         // [SCAN_CHUNK][2 N]
-  float* Ss = BC + (size_t)SCAN_CHUNK * 2 * N;                   // !REG: [N][SCAN_THREADS]
-  float* As = Ss + (REG ? 0 : (size_t)N * SCAN_THREADS);         // !REG: [N][SCAN_THREADS]
+  float* Ss = BC + (size_t)SCAN_CHUNK * 2 * N;                   // [N][SCAN_THREADS]
+  float* As = Ss + (size_t)N * SCAN_THREADS;                     // [N][SCAN_THREADS]
   griddep_launch();
   griddep_wait();
   const AttnSeq sq = seqs[blockIdx.x];
-  const int tid = threadIdx.x;
-  const int sub = REG ? tid % SCAN_LPC : 0;
-  const int c = REG ? blockIdx.y * (SCAN_THREADS / SCAN_LPC) + tid / SCAN_LPC : blockIdx.y * SCAN_THREADS + tid;
+  const int tid = threadIdx.x, c = blockIdx.y * SCAN_THREADS + tid;
   const bool live = c < a.inner;
   const int slot = tok_slot[sq.q_start];
   const int first = sq.kv_len - sq.q_len;   // position of the portion's first token
   float* Sg = a.S + ((size_t)slot * a.inner + (live ? c : 0)) * N;
-  float Sr[SCAN_RPL], Ar[SCAN_RPL];
-  if (REG) {
-#pragma unroll
-    for (int j = 0; j < SCAN_RPL; ++j) {
-      const int n = sub + j * SCAN_LPC;
-      Sr[j] = (live && first > 0 && n < N) ? Sg[n] : 0.f;
-      Ar[j] = (live && n < N) ? -expf(a.A_log[(size_t)c * N + n]) : 0.f;
-    }
-  } else {
-    for (int n = 0; n < N; ++n) {
-      Ss[n * SCAN_THREADS + tid] = (live && first > 0) ? Sg[n] : 0.f;
-      As[n * SCAN_THREADS + tid] = live ? -expf(a.A_log[(size_t)c * N + n]) : 0.f;
-    }
+  for (int n = 0; n < N; ++n) {
+    Ss[n * SCAN_THREADS + tid] = (live && first > 0) ? Sg[n] : 0.f;
+    As[n * SCAN_THREADS + tid] = live ? -expf(a.A_log[(size_t)c * N + n]) : 0.f;
   }
   const float dtb = live ? a.dt_b[c] : 0.f, Dc = live ? a.D[c] : 0.f;
   for (int t0 = 0; t0 < sq.q_len; t0 += SCAN_CHUNK) {
@@ -153,7 +248,7 @@ selective_scan_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t
       zv[tt] = ok ? a.xz[row * a.ld_xz + a.inner + c] : 0.f;
     }
     __syncthreads();
-    if (!REG && !live) continue;   // (REG: every lane takes part in the shuffles)
+    if (!live) continue;
 #pragma unroll
     for (int tt = 0; tt < SCAN_CHUNK; ++tt) {
       if (tt < nt) {
@@ -162,24 +257,10 @@ selective_scan_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t
         const float dx = dt * xv[tt];
         const float* Bt = BC + (size_t)tt * 2 * N;
         float y = 0.f;
-        if (REG) {
-#pragma unroll
-          for (int j = 0; j < SCAN_RPL; ++j) {
-            const int n = sub + j * SCAN_LPC;
-            if (n < N) {
-              Sr[j] = fmaf(expf(dt * Ar[j]), Sr[j], dx * Bt[n]);
-              y = fmaf(Sr[j], Bt[N + n], y);
-            }
-          }
-          y += __shfl_xor_sync(0xffffffffu, y, 1);
-          y += __shfl_xor_sync(0xffffffffu, y, 2);
-          if (!live || sub != 0) continue;
-        } else {
-          for (int n = 0; n < N; ++n) {
-            const float sv = fmaf(expf(dt * As[n * SCAN_THREADS + tid]), Ss[n * SCAN_THREADS + tid], dx * Bt[n]);
-            Ss[n * SCAN_THREADS + tid] = sv;
-            y = fmaf(sv, Bt[N + n], y);
-          }
+        for (int n = 0; n < N; ++n) {
+          const float sv = fmaf(expf(dt * As[n * SCAN_THREADS + tid]), Ss[n * SCAN_THREADS + tid], dx * Bt[n]);
+          Ss[n * SCAN_THREADS + tid] = sv;
+          y = fmaf(sv, Bt[N + n], y);
         }
         y = fmaf(Dc, xv[tt], y);
         st_op(a.out, a.out_dtype, row * a.inner + c, y * silu_f(zv[tt]));
@@ -187,44 +268,51 @@ selective_scan_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t
     }
   }
   if (!live) return;
-  if (REG) {
-#pragma unroll
-    for (int j = 0; j < SCAN_RPL; ++j)
-      if (sub + j * SCAN_LPC < N) Sg[sub + j * SCAN_LPC] = Sr[j];
-    if (sub != 0) return;
-  } else {
-    for (int n = 0; n < N; ++n) Sg[n] = Ss[n * SCAN_THREADS + tid];
-  }
-  // the convolution's tail: inputs of the last taps - 1 positions (entry e: position end - (taps - 1) + e)
-  const int K1 = a.taps - 1;
-  float* cs = a.conv_state + (size_t)slot * K1 * a.inner + c;
-  for (int e = 0; e < K1; ++e) {   // ascending: entry e + q_len is read before it could be rewritten
-    const int pp = sq.kv_len - K1 + e;
-    float v = 0.f;
-    if (pp >= first) v = a.xz[(size_t)(sq.q_start + pp - first) * a.ld_xz + c];
-    else if (pp >= 0) v = cs[(size_t)(e + sq.q_len) * a.inner];
-    cs[(size_t)e * a.inner] = v;
-  }
+  for (int n = 0; n < N; ++n) Sg[n] = Ss[n * SCAN_THREADS + tid];
+  scan_save_conv(a, sq, slot, c);
 }
 
 // ------------------------------------------------------------------------------------------------ outer-product memories
 // grid (sequences, heads, ceil(vdim / 32)); 256 threads = 8 row groups (warps) x 32 value columns (lanes).  Thread (g, c)
-// keeps rows g, g + 8, ... of column c in registers.  The tokens' q / k / decay vectors, value columns and gates are staged
-// in shared memory OS_CHUNK tokens at a time (one wait for memory per chunk).  The recurrence itself is private to a thread (its
-// rows of S, and redundantly the running maximum and its rows of n); only a token's OUTPUT sums over the row groups.  So a thread
-// runs through the chunk's tokens without any barrier, leaving its partial sums per token in shared memory, and after ONE barrier
-// warp w sums and writes the outputs of the chunk's token w.
+// keeps rows 4 (g + 8 j) .. + 3 of column c in registers, two to a packed pair.  The tokens' q / k / decay vectors, value columns
+// and gates are staged in shared memory OS_CHUNK tokens at a time (one wait for memory per chunk).  The recurrence itself is private
+// to a thread; only a token's OUTPUT sums over the row groups.  So a thread runs through the chunk's tokens without any barrier,
+// leaving its partial sums per token in shared memory, and after ONE barrier warp w sums and writes the outputs of the chunk's
+// tokens w, w + 8.  What is the same for all columns is not done once per thread: the gated memory's exponentials are one warp's work
+// before the token loop, and its normaliser is kept a row per thread.
+// Bound by instruction issue and by the latency of a token's chain (one head's tokens are worked through one after the other, and a
+// prompt has only heads * vdim / 32 blocks).  Four rows to a shared-memory load and two to an fma.
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+  return d;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long x, unsigned long long y) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long x, unsigned long long y, unsigned long long z) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
+  return d;
+}
 constexpr int OS_GROUPS = 8, OS_COLS = 32, OS_THREADS = OS_GROUPS * OS_COLS, OS_CHUNK = 16;
-template <int RPT, int MODE>
+// FULL: D == RPT * OS_GROUPS, every thread's rows are there (no branch in the token loop, so a token's loads go ahead of its sums).
+template <int RPT, int MODE, bool FULL>
 __global__ void __launch_bounds__(OS_THREADS)
 outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* __restrict__ tok_slot) {
-  extern __shared__ float os_smem[];
-  const int D = a.dim;
-  float* vec = os_smem;                                  // [OS_CHUNK][3][D]: q | k | w
-  float* vcol = vec + (size_t)OS_CHUNK * 3 * D;          // [OS_CHUNK][OS_COLS]
+  extern __shared__ __align__(16) float os_smem[];
+  const int D = FULL ? RPT * OS_GROUPS : a.dim, DP = (D + 3) & ~3;
+  float* vec = os_smem;                                  // [OS_CHUNK][3][DP]: q | k | w (GATED: n q)
+  float* vcol = vec + (size_t)OS_CHUNK * 3 * DP;         // [OS_CHUNK][OS_COLS]
   __shared__ float part[OS_CHUNK][OS_GROUPS][OS_COLS + 1];
-  __shared__ float part_n[OS_CHUNK][OS_GROUPS];
-  __shared__ float gates[OS_CHUNK][2];                   // GATED: capped log input gate, log forget gate
+  __shared__ float gates[OS_CHUNK][2];                   // GATED, SSD: the decay, the factor of the outer product
   __shared__ float floor_m[OS_CHUNK];                    // GATED: e^(-m) after each token
   static_assert(OS_CHUNK % OS_GROUPS == 0, "warp w writes the outputs of the chunk's tokens w, w + OS_GROUPS, ...");
   griddep_launch();
@@ -236,34 +324,32 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
   const bool col_ok = c < a.vdim;
   const int slot = tok_slot[sq.q_start];
   const bool fresh = sq.kv_len - sq.q_len == 0;
-  float S[RPT];
+  constexpr int NG = RPT / 4;          // groups of four rows
+  constexpr bool OWN_DECAY = MODE == OUTER_SCAN_DECAY || MODE == OUTER_SCAN_HGRN || MODE == OUTER_SCAN_GLA;   // a decay per row
+  auto row_of = [&](int j) { return 4 * (g + (j >> 2) * OS_GROUPS) + (j & 3); };
+  unsigned long long S[2 * NG];
   float* Sg = a.S + (((size_t)slot * a.heads + h) * D) * a.vdim + (col_ok ? c : 0);
 #pragma unroll
-  for (int j = 0; j < RPT; ++j) {
-    const int i = g + j * OS_GROUPS;
-    S[j] = (!fresh && col_ok && i < D) ? Sg[(size_t)i * a.vdim] : 0.f;
+  for (int j = 0; j < RPT; j += 2) {
+    const int i = row_of(j);
+    const float s0 = (!fresh && col_ok && i < D) ? Sg[(size_t)i * a.vdim] : 0.f;
+    const float s1 = (!fresh && col_ok && i + 1 < D) ? Sg[(size_t)(i + 1) * a.vdim] : 0.f;
+    S[j / 2] = pack2(s0, s1);
   }
-  float u_r[RPT];   // DECAY: the bonus u of this thread's rows; GATED: the normaliser n of its rows (the same in every lane)
-  float m_run = 0.f;
+  unsigned long long u_r[2 * NG];      // DECAY: the bonus u of this thread's rows
+  float n_row = 0.f, m_run = 0.f;      // GATED: the normaliser's row tid; the running maximum (warp 0)
   const float ssd_rate = MODE == OUTER_SCAN_SSD ? -expf(a.A_log[h]) : 0.f, ssd_skip = MODE == OUTER_SCAN_SSD ? a.D[h] : 0.f;
   const float fixed_decay = (MODE == OUTER_SCAN_LIGHTNING || MODE == OUTER_SCAN_RETENTION) ? a.decay[h] : 0.f;
-  if (MODE == OUTER_SCAN_SSD || MODE == OUTER_SCAN_HGRN || MODE == OUTER_SCAN_LIGHTNING || MODE == OUTER_SCAN_RETENTION || MODE == OUTER_SCAN_GLA) {
+  if (MODE == OUTER_SCAN_DECAY) {
 #pragma unroll
-    for (int j = 0; j < RPT; ++j) u_r[j] = 0.f;
-  } else if (MODE == OUTER_SCAN_DECAY) {
-#pragma unroll
-    for (int j = 0; j < RPT; ++j) {
-      const int i = g + j * OS_GROUPS;
-      u_r[j] = i < D ? a.u[(size_t)h * D + i] : 0.f;
+    for (int j = 0; j < RPT; j += 2) {
+      const int i = row_of(j);
+      u_r[j / 2] = pack2(i < D ? a.u[(size_t)h * D + i] : 0.f, i + 1 < D ? a.u[(size_t)h * D + i + 1] : 0.f);
     }
-  } else {
-    const float* ng = a.n + ((size_t)slot * a.heads + h) * D;
-#pragma unroll
-    for (int j = 0; j < RPT; ++j) {
-      const int i = g + j * OS_GROUPS;
-      u_r[j] = (!fresh && i < D) ? ng[i] : 0.f;
-    }
-    m_run = fresh ? 0.f : a.m[(size_t)slot * a.heads + h];
+  }
+  if (MODE == OUTER_SCAN_GATED && !fresh) {
+    n_row = tid < D ? a.n[((size_t)slot * a.heads + h) * D + tid] : 0.f;
+    m_run = a.m[(size_t)slot * a.heads + h];
   }
   // A chunk's raw values travel global memory -> registers -> shared memory: thread (tt = tid / 16, l = tid % 16) stages entries
   // l, l + 16, ... of token tt's vectors and two of its value columns, all loads of a chunk are issued back to back, and the
@@ -271,7 +357,9 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
   constexpr int EPT = RPT / 2, TPT = OS_THREADS / OS_CHUNK;
   static_assert(TPT == 16 && OS_CHUNK * OS_COLS == 2 * OS_THREADS, "staging map");
   const int st_tt = tid / TPT, st_l = tid % TPT;
-  float pq[EPT], pk[EPT], pd[EPT], pv[2], pg0 = 0.f, pg1 = 0.f;
+  float pq[EPT], pk[EPT], pd[EPT], pw[EPT], pv[2], pg0 = 0.f, pg1 = 0.f;
+#pragma unroll
+  for (int e = 0; e < EPT; ++e) pw[e] = OWN_DECAY && st_l + e * TPT < D ? a.w0[(size_t)h * D + st_l + e * TPT] : 0.f;
   auto fetch = [&](int t0) {
     const int nt = min(OS_CHUNK, sq.q_len - t0);
     const bool tok = st_tt < nt;
@@ -284,8 +372,7 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
       const bool in = tok && i < D;
       pq[e] = in ? qr[i] : 0.f;
       pk[e] = in ? (MODE == OUTER_SCAN_HGRN ? a.u[(size_t)h * D + i] : kr[i]) : 0.f;   // HGRN: the gate's lower bound
-      if (MODE == OUTER_SCAN_DECAY || MODE == OUTER_SCAN_HGRN || MODE == OUTER_SCAN_GLA)
-        pd[e] = in ? a.decay_raw[row * a.ldd + (size_t)h * D + i] + a.w0[(size_t)h * D + i] : 0.f;
+      if (OWN_DECAY) pd[e] = in ? a.decay_raw[row * a.ldd + (size_t)h * D + i] : 0.f;
     }
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
@@ -303,32 +390,50 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
     const int nt = min(OS_CHUNK, sq.q_len - t0);
     __syncthreads();   // the previous chunk's vectors and partial sums are consumed
     if (st_tt < nt) {
-      float* v3 = vec + (size_t)st_tt * 3 * D;
+      float* v3 = vec + (size_t)st_tt * 3 * DP;
 #pragma unroll
       for (int e = 0; e < EPT; ++e) {
         const int i = st_l + e * TPT;
         if (i < D) {
           if (MODE == OUTER_SCAN_HGRN) {   // q = silu(.), f = l + (1 - l) sigmoid(.), and what is written: 1 - f
             v3[i] = silu_f(pq[e]) * a.q_scale;
-            v3[D + i] = (1.f - pk[e]) * sigmoid_f(-pd[e]);                 // 1 - f without the cancellation near f = 1
-            v3[2 * D + i] = pk[e] + (1.f - pk[e]) * sigmoid_f(pd[e]);
+            const float dl = pd[e] + pw[e];
+            v3[DP + i] = (1.f - pk[e]) * sigmoid_f(-dl);                 // 1 - f without the cancellation near f = 1
+            v3[2 * DP + i] = pk[e] + (1.f - pk[e]) * sigmoid_f(dl);
           } else if (MODE == OUTER_SCAN_LIGHTNING) {
             v3[i] = silu_f(pq[e]) * a.q_scale;
-            v3[D + i] = silu_f(pk[e]);
+            v3[DP + i] = silu_f(pk[e]);
           } else {
             v3[i] = pq[e] * a.q_scale;
-            v3[D + i] = pk[e];
-            if (MODE == OUTER_SCAN_DECAY) v3[2 * D + i] = expf(-expf(pd[e]));
-            if (MODE == OUTER_SCAN_GLA) v3[2 * D + i] = expf(logsigmoid_f(pd[e]) * a.inv_tau);
+            v3[DP + i] = pk[e];
+            if (MODE == OUTER_SCAN_DECAY) v3[2 * DP + i] = expf(-expf(pd[e] + pw[e]));
+            if (MODE == OUTER_SCAN_GLA) v3[2 * DP + i] = expf(logsigmoid_f(pd[e] + pw[e]) * a.inv_tau);
           }
         }
       }
     }
     vcol[st_tt * OS_COLS + 2 * st_l] = MODE == OUTER_SCAN_LIGHTNING ? silu_f(pv[0]) : pv[0];
     vcol[st_tt * OS_COLS + 2 * st_l + 1] = MODE == OUTER_SCAN_LIGHTNING ? silu_f(pv[1]) : pv[1];
-    if (MODE == OUTER_SCAN_GATED && tid < nt) {
-      gates[tid][0] = a.gate_cap * tanhf((pg0 + a.ig_b[h]) / a.gate_cap);
-      gates[tid][1] = logsigmoid_f(a.gate_cap * tanhf((pg1 + a.fg_b[h]) / a.gate_cap));
+    if (MODE == OUTER_SCAN_GATED && tid < 32) {   // lane t: token t's gates, and the maximum that runs through them
+      float ig = 0.f, fg = 0.f, m_before = 0.f, m_after = 0.f;
+      if (lane < nt) {
+        ig = a.gate_cap * tanhf((pg0 + a.ig_b[h]) / a.gate_cap);
+        fg = logsigmoid_f(a.gate_cap * tanhf((pg1 + a.fg_b[h]) / a.gate_cap));
+      }
+#pragma unroll
+      for (int t = 0; t < OS_CHUNK; ++t) {
+        const float it = __shfl_sync(0xffffffffu, ig, t), ft = __shfl_sync(0xffffffffu, fg, t);
+        if (t < nt) {
+          const float m_new = fmaxf(ft + m_run, it);
+          if (lane == t) m_before = m_run, m_after = m_new;
+          m_run = m_new;
+        }
+      }
+      if (lane < nt) {
+        gates[lane][0] = expf(fg + m_before - m_after);
+        gates[lane][1] = expf(ig - m_after);
+        floor_m[lane] = expf(-m_after);
+      }
     }
     if (MODE == OUTER_SCAN_SSD && tid < nt) {   // the token's step size and the decay it gives
       const float dt = softplus_f(pg0 + a.step_b[h]);
@@ -337,68 +442,61 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
     }
     __syncthreads();
     if (t0 + OS_CHUNK < sq.q_len) fetch(t0 + OS_CHUNK);   // lands while this chunk's tokens are worked through
-    for (int tt = 0; tt < nt; ++tt) {
-      const float* v3 = vec + (size_t)tt * 3 * D;
-      const float vc = vcol[tt * OS_COLS + lane];
-      float o = 0.f, nq = 0.f;
-      if (MODE == OUTER_SCAN_DECAY) {
+    if (MODE == OUTER_SCAN_GATED && tid < D) {
+      float nk[OS_CHUNK];   // (tokens behind the last one hold what the chunk before left: read, not used)
 #pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-          const int i = g + j * OS_GROUPS;
-          if (i < D) {
-            const float kv = v3[D + i] * vc;
-            o = fmaf(v3[i], fmaf(u_r[j], kv, S[j]), o);
-            S[j] = fmaf(v3[2 * D + i], S[j], kv);
-          }
-        }
-      } else if (MODE == OUTER_SCAN_HGRN || MODE == OUTER_SCAN_GLA) {
+      for (int tt = 0; tt < OS_CHUNK; ++tt) nk[tt] = gates[tt][1] * vec[(size_t)tt * 3 * DP + DP + tid];
 #pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-          const int i = g + j * OS_GROUPS;
-          if (i < D) {
-            S[j] = fmaf(v3[2 * D + i], S[j], v3[D + i] * vc);
-            o = fmaf(v3[i], S[j], o);
-          }
+      for (int tt = 0; tt < OS_CHUNK; ++tt) {
+        if (tt < nt) {
+          float* v3 = vec + (size_t)tt * 3 * DP;
+          n_row = fmaf(gates[tt][0], n_row, nk[tt]);
+          v3[2 * DP + tid] = n_row * v3[tid];
         }
-      } else if (MODE == OUTER_SCAN_LIGHTNING || MODE == OUTER_SCAN_RETENTION) {
-#pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-          const int i = g + j * OS_GROUPS;
-          if (i < D) {
-            S[j] = fmaf(fixed_decay, S[j], v3[D + i] * vc);
-            o = fmaf(v3[i], S[j], o);
-          }
-        }
-      } else if (MODE == OUTER_SCAN_SSD) {
-        const float da = gates[tt][0], dv = gates[tt][1] * vc;
-#pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-          const int i = g + j * OS_GROUPS;
-          if (i < D) {
-            S[j] = fmaf(da, S[j], v3[D + i] * dv);
-            o = fmaf(v3[i], S[j], o);
-          }
-        }
-      } else {
-        const float ig = gates[tt][0], fg = gates[tt][1];
-        const float m_new = fmaxf(fg + m_run, ig);
-        const float da = expf(fg + m_run - m_new), db = expf(ig - m_new);
-        m_run = m_new;
-#pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-          const int i = g + j * OS_GROUPS;
-          if (i < D) {
-            const float kk = v3[D + i], qq = v3[i];
-            S[j] = fmaf(da, S[j], db * kk * vc);
-            o = fmaf(qq, S[j], o);
-            u_r[j] = fmaf(da, u_r[j], db * kk);
-            nq = fmaf(u_r[j], qq, nq);
-          }
-        }
-        if (lane == 0) part_n[tt][g] = nq;
-        if (tid == 0) floor_m[tt] = expf(-m_run);
       }
-      part[tt][g][lane] = o;
+    }
+#pragma unroll (RPT <= 16 ? 2 : 1)
+    for (int tt = 0; tt < nt; ++tt) {
+      const float* v3 = vec + (size_t)tt * 3 * DP;
+      float vc = vcol[tt * OS_COLS + lane], wd = fixed_decay;
+      if (MODE == OUTER_SCAN_SSD || MODE == OUTER_SCAN_GATED) vc *= gates[tt][1], wd = gates[tt][0];
+      const unsigned long long vc2 = pack2(vc, vc), wd2 = pack2(wd, wd);
+      unsigned long long o01 = 0, o23 = 0;   // two packed zeros
+      auto step = [&](unsigned long long& s, unsigned long long& o, unsigned long long q2, unsigned long long k2, unsigned long long w2,
+                      unsigned long long u2) {
+        const unsigned long long kv = mul2(k2, vc2);
+        if (MODE == OUTER_SCAN_DECAY) {
+          o = fma2(q2, fma2(u2, kv, s), o);
+          s = fma2(w2, s, kv);
+        } else {
+          s = fma2(w2, s, kv);
+          o = fma2(q2, s, o);
+        }
+      };
+#pragma unroll
+      for (int j = 0; j < NG; ++j) {
+        const int i = 4 * (g + j * OS_GROUPS);
+        if (FULL || i + 4 <= D) {
+          const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(v3 + i), k4 = *reinterpret_cast<const ulonglong2*>(v3 + DP + i);
+          ulonglong2 w4 = make_ulonglong2(wd2, wd2);
+          if (OWN_DECAY) w4 = *reinterpret_cast<const ulonglong2*>(v3 + 2 * DP + i);
+          step(S[2 * j], o01, q4.x, k4.x, w4.x, u_r[2 * j]);
+          step(S[2 * j + 1], o23, q4.y, k4.y, w4.y, u_r[2 * j + 1]);
+        } else if (i < D) {   // the last one to three rows: what lies behind them takes no part, whatever the values are
+          auto tail = [&](unsigned long long& s, unsigned long long& o, unsigned long long u, int at) {
+            if (at >= D) return;
+            const float2 s_was = unpack2(s), o_was = unpack2(o);
+            const bool two = at + 1 < D;
+            const float w0 = OWN_DECAY ? v3[2 * DP + at] : wd, w1 = OWN_DECAY && two ? v3[2 * DP + at + 1] : wd;
+            step(s, o, pack2(v3[at], two ? v3[at + 1] : 0.f), pack2(v3[DP + at], two ? v3[DP + at + 1] : 0.f), pack2(w0, w1), u);
+            if (!two) s = pack2(unpack2(s).x, s_was.y), o = pack2(unpack2(o).x, o_was.y);
+          };
+          tail(S[2 * j], o01, u_r[2 * j], i);
+          tail(S[2 * j + 1], o23, u_r[2 * j + 1], i + 2);
+        }
+      }
+      const float2 oa = unpack2(o01), ob = unpack2(o23);
+      part[tt][g][lane] = (oa.x + oa.y) + (ob.x + ob.y);
     }
     __syncthreads();   // the chunk's partial sums are complete
     for (int tt = g; tt < nt; tt += OS_GROUPS) {   // this warp's tokens of the chunk
@@ -407,8 +505,8 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
       for (int r = 0; r < OS_GROUPS; ++r) sum += part[tt][r][lane];
       if (MODE == OUTER_SCAN_GATED) {
         float d = 0.f;
-#pragma unroll
-        for (int r = 0; r < OS_GROUPS; ++r) d += part_n[tt][r];
+        for (int i = lane; i < D; i += 32) d += vec[(size_t)tt * 3 * DP + 2 * DP + i];
+        d = warp_sum_f(d);
         sum = sum / (fmaxf(fabsf(d), floor_m[tt]) + 1e-6f);
       }
       if (MODE == OUTER_SCAN_SSD) sum = fmaf(ssd_skip, vcol[tt * OS_COLS + lane], sum);
@@ -418,16 +516,18 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
   // ---- leave the state behind the portion's last token
   if (col_ok) {
 #pragma unroll
-    for (int j = 0; j < RPT; ++j) {
-      const int i = g + j * OS_GROUPS;
-      if (i < D) Sg[(size_t)i * a.vdim] = S[j];
+    for (int j = 0; j < RPT; j += 2) {
+      const int i = row_of(j);
+      const float2 s = unpack2(S[j / 2]);
+      if (i < D) Sg[(size_t)i * a.vdim] = s.x;
+      if (i + 1 < D) Sg[(size_t)(i + 1) * a.vdim] = s.y;
     }
   }
   // The normaliser and the running maximum belong to all column blocks of the head, each of which started from them.  More blocks
   // than the chip holds at once do not start together, so only the one that gets here last may overwrite them.
   if (MODE == OUTER_SCAN_GATED) {
     __shared__ int last_block;
-    __syncthreads();   // every thread's rows of n and m are read
+    __syncthreads();   // every thread's row of n and m are read
     if (tid == 0) {
       int32_t* done = a.done + (size_t)slot * a.heads + h;
       last_block = gridDim.z == 1 || atomicAdd(done, 1) == (int)gridDim.z - 1;
@@ -435,14 +535,7 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
     }
     __syncthreads();
     if (last_block) {
-      float* ng = a.n + ((size_t)slot * a.heads + h) * D;
-      if (lane == 0) {
-#pragma unroll
-        for (int j = 0; j < RPT; ++j) {
-          const int i = g + j * OS_GROUPS;
-          if (i < D) ng[i] = u_r[j];
-        }
-      }
+      if (tid < D) a.n[((size_t)slot * a.heads + h) * D + tid] = n_row;
       if (tid == 0) a.m[(size_t)slot * a.heads + h] = m_run;
     }
   }
@@ -775,34 +868,37 @@ cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_s
   const size_t bc = (size_t)SCAN_CHUNK * 2 * a.state * sizeof(float);
   if (a.state <= SCAN_REG_STATE) {
     constexpr int per_cta = SCAN_THREADS / SCAN_LPC;
-    return launch_k(selective_scan_kernel<true>, dim3(n_seqs, (a.inner + per_cta - 1) / per_cta), dim3(SCAN_THREADS), bc, stream, a,
-                    seqs, tok_slot);
+    return launch_k(selective_scan_reg_kernel, dim3(n_seqs, (a.inner + per_cta - 1) / per_cta), dim3(SCAN_THREADS), 0, stream, a, seqs,
+                    tok_slot);
   }
   const dim3 grid(n_seqs, (a.inner + SCAN_THREADS - 1) / SCAN_THREADS);
   const size_t smem = bc + (size_t)2 * a.state * SCAN_THREADS * sizeof(float);
   static size_t smem_set = 0;
   if (smem > 48 * 1024 && smem > smem_set) {
-    const cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     smem_set = smem;
   }
-  return launch_k(selective_scan_kernel<false>, grid, dim3(SCAN_THREADS), smem, stream, a, seqs, tok_slot);
+  return launch_k(selective_scan_kernel, grid, dim3(SCAN_THREADS), smem, stream, a, seqs, tok_slot);
 }
 
+template <int RPT, int MODE>
+static cudaError_t outer_scan_rows(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot, cudaStream_t stream) {
+  const dim3 grid(n_seqs, a.heads, (a.vdim + OS_COLS - 1) / OS_COLS);
+  const size_t smem = ((size_t)OS_CHUNK * 3 * ((a.dim + 3) & ~3) + OS_CHUNK * OS_COLS) * sizeof(float);   // <= 50 KB (+ 17 KB static)
+  const auto kernel = a.dim == RPT * OS_GROUPS ? outer_scan_kernel<RPT, MODE, true> : outer_scan_kernel<RPT, MODE, false>;
+  if (RPT > 16) {   // keys of more than 128 entries: the staged chunk passes the default 48 KB of shared memory
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_k(kernel, grid, dim3(OS_THREADS), smem, stream, a, seqs, tok_slot);
+}
 template <int MODE>
 static cudaError_t outer_scan_mode(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot,
                                    cudaStream_t stream) {
-  const dim3 grid(n_seqs, a.heads, (a.vdim + OS_COLS - 1) / OS_COLS);
-  const size_t smem = ((size_t)OS_CHUNK * 3 * a.dim + OS_CHUNK * OS_COLS) * sizeof(float);   // <= 50 KB (+ 18 KB static)
-  if (a.dim <= 8 * OS_GROUPS) return launch_k(outer_scan_kernel<8, MODE>, grid, dim3(OS_THREADS), smem, stream, a, seqs, tok_slot);
-  if (a.dim <= 16 * OS_GROUPS) return launch_k(outer_scan_kernel<16, MODE>, grid, dim3(OS_THREADS), smem, stream, a, seqs, tok_slot);
-  static bool attr_set = false;   // keys of more than 128 entries: the staged chunk passes the default 48 KB of shared memory
-  if (!attr_set) {
-    const cudaError_t e = cudaFuncSetAttribute(outer_scan_kernel<32, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
-  return launch_k(outer_scan_kernel<32, MODE>, grid, dim3(OS_THREADS), smem, stream, a, seqs, tok_slot);
+  if (a.dim <= 8 * OS_GROUPS) return outer_scan_rows<8, MODE>(a, seqs, n_seqs, tok_slot, stream);
+  if (a.dim <= 16 * OS_GROUPS) return outer_scan_rows<16, MODE>(a, seqs, n_seqs, tok_slot, stream);
+  return outer_scan_rows<32, MODE>(a, seqs, n_seqs, tok_slot, stream);
 }
 cudaError_t outer_scan_launch(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot,
                               cudaStream_t stream) {
