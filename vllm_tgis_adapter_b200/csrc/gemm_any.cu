@@ -65,7 +65,15 @@ __device__ __forceinline__ float relu2_row_scale(const GemmAny& a, int dst) {
 constexpr int FMA_THREADS = 128;
 constexpr int FMA_BN = 64, FMA_BK = 32, FMA_LD = FMA_BK + 4;
 constexpr int FMA_SMS = 148;
+// Sums of up to 64 terms run as one ascending chain per output, not as an even and an odd one that meet at the end: two k-blocks
+// wait for memory, not for arithmetic, so they keep the order of a plain loop.
+constexpr int FMA_CHAIN_K = 64;
 
+__device__ __forceinline__ void fma_low(unsigned long long& d, float x, float w) {   // the pair's lower half
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(fmaf(x, w, lo)), "f"(hi));
+}
 __device__ __forceinline__ void fma2(unsigned long long& d, unsigned long long x, unsigned long long y) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;\n" : "+l"(d) : "l"(x), "l"(y));
 }
@@ -173,6 +181,18 @@ __global__ void __launch_bounds__(FMA_THREADS) gemm_any_kernel(GemmAny a) {
     if (kb + 1 < KB) fetch((kb + 1) * FMA_BK);
     const float* xs = &Xs[cur][ty * FMA_LD];
     const float* ws = &Ws[cur][tx * FMA_LD];
+    if (a.K <= FMA_CHAIN_K) {
+#pragma unroll 1
+      for (int k = 0; k < FMA_BK; ++k) {
+        float w1[TN];
+#pragma unroll
+        for (int j = 0; j < TN; ++j) w1[j] = ws[j * 16 * FMA_LD + k];
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) fma_low(acc[i][j], xs[i * 8 * FMA_LD + k], w1[j]);
+      }
+    } else
 #pragma unroll
     for (int k = 0; k < FMA_BK; k += 4) {
       ulonglong2 w2[TN];
