@@ -116,7 +116,8 @@ __device__ __forceinline__ void scan_save_conv(const SelScan& a, const AttnSeq& 
 // instructions a token takes.  What the four lanes would all do is dealt out: of a chunk's eight tokens a lane fetches two (step
 // size, input, gate), takes their softplus, hands step size and input on by shuffle, and after the chunk receives the two tokens'
 // output sums (a transposing reduction: 6 shuffles for 8 tokens and 4 lanes) and gates and writes them.  B and C rows go through two
-// shared-memory buffers, read four states to a load; the next chunk is fetched while this one is worked through.
+// shared-memory buffers, read four states to a load; the next chunk is fetched while this one is worked through.  2048 tokens in 7 prompts, 4096 channels of 16
+// states: 747 -> 338 us.
 __global__ void __launch_bounds__(SCAN_THREADS)
 selective_scan_reg_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t* __restrict__ tok_slot) {
   constexpr int TPL = SCAN_CHUNK / SCAN_LPC, ROW = 2 * SCAN_REG_STATE, STAGE = SCAN_CHUNK * ROW / SCAN_THREADS;
@@ -281,7 +282,9 @@ selective_scan_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t
 // tokens w, w + 8.  What is the same for all columns is not done once per thread: the gated memory's exponentials are one warp's work
 // before the token loop, and its normaliser is kept a row per thread.
 // Bound by instruction issue and by the latency of a token's chain (one head's tokens are worked through one after the other, and a
-// prompt has only heads * vdim / 32 blocks).  Four rows to a shared-memory load and two to an fma.
+// prompt has only heads * vdim / 32 blocks).  Four rows to a shared-memory load and two to an fma.  2048 tokens in 7 prompts: gated,
+// 8 heads of 128 x 256, 636 -> 346 us (507 while the token loop still tested every group of rows: hence FULL); decayed, 32 heads of
+// 64 x 64, 342 -> 255 us; a step of 32 single tokens, gated, 42 -> 30 us.  One 1024-token prompt takes 0.24 us a token.
 __device__ __forceinline__ unsigned long long pack2(float x, float y) {
   unsigned long long d;
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
