@@ -544,6 +544,7 @@ struct tgis_engine {
     if (prop.major != 10) throw CudaError("tgis_engine requires an sm_100 (B200) device; found sm_" +
                                           std::to_string(prop.major) + std::to_string(prop.minor));
     num_sms = prop.multiProcessorCount;
+    CK(gemm_pair_prepare());
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CK(cudaEventCreate(&ev0));
     CK(cudaEventCreate(&ev1));

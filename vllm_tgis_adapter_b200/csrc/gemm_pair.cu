@@ -22,6 +22,9 @@
 // buffered accumulator (2 x 256 columns).  The leader's `full` barrier counts both CTAs' bytes; tcgen05.commit releases a
 // ring slot in both CTAs at once.  No wait is unbounded: after about two seconds a role gives up, raises the host-visible
 // error word and leaves; TMEM is freed on every path.
+#include <atomic>
+#include <mutex>
+
 #include "kernels.h"
 #include "launch.cuh"
 #include "ptx.cuh"
@@ -432,15 +435,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   }
 }
 
-// host-visible error word, one for the process (a raised word is an error of the process's device, as a sticky CUDA error is)
-int* pair_error_word() {
-  static int* word = [] {
-    int* p = nullptr;
-    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return (int*)nullptr;
-    *p = 0;
-    return p;
-  }();
-  return word;
+// host-visible error word, one for the process (a raised word is an error of the process's device, as a sticky CUDA error is).
+// Pinned memory cannot be had while a stream is being captured, so an engine has it made before its first step
+// (gemm_pair_prepare); a refusal is not remembered.
+std::atomic<int*> pair_word{nullptr};
+cudaError_t make_pair_word() {
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lk(mu);
+  if (pair_word.load(std::memory_order_acquire) != nullptr) return cudaSuccess;
+  int* p = nullptr;
+  const cudaError_t e = cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+  if (e != cudaSuccess) return e;
+  *p = 0;
+  pair_word.store(p, std::memory_order_release);
+  return cudaSuccess;
 }
 
 template <bool GROUPED>
@@ -448,15 +456,18 @@ cudaError_t launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, PairAr
   static const cudaError_t attr =
       cudaFuncSetAttribute(gemm_pair_kernel<GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem(GROUPED));
   if (attr != cudaSuccess) return attr;
-  a.err = pair_error_word();
-  if (a.err == nullptr) return cudaErrorMemoryAllocation;
+  const cudaError_t word = gemm_pair_prepare();
+  if (word != cudaSuccess) return word;
+  a.err = pair_word.load(std::memory_order_acquire);
   return launch_k_cluster(gemm_pair_kernel<GROUPED>, dim3(grid), dim3(PAIR_THREADS), pair_smem(GROUPED), stream, 2, wmap, xmap, a);
 }
 
 }  // namespace
 
+cudaError_t gemm_pair_prepare() { return pair_word.load(std::memory_order_acquire) != nullptr ? cudaSuccess : make_pair_word(); }
+
 bool gemm_pair_failed() {
-  const int* w = pair_error_word();
+  const int* w = pair_word.load(std::memory_order_acquire);
   return w != nullptr && *reinterpret_cast<const volatile int*>(w) != 0;
 }
 

@@ -88,6 +88,7 @@ constexpr int PAIR_GELU = 5;         // exact gelu
 cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int y_f32, int mode, int T, int N,
                              int K, int num_sms, cudaStream_t stream);
 int gemm_pair_plan(int T, int N, int pairs);   // token tiles of the dense launch
+cudaError_t gemm_pair_prepare();               // host memory of the launches: to be called before any of them is captured
 bool gemm_pair_failed();                       // a wait inside a launch of this process ran out
 
 // ---- gemm_skinny.cu: the same product for up to 32 tokens; X [T, K], W [N, K] contiguous, rows on 16-byte boundaries; rope: as in
