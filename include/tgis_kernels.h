@@ -98,6 +98,9 @@ int tgis_k_lora_bench(const void* x_dev, int32_t ldx, const int32_t* tok_slot_de
 /* act[t, j] = bf16(silu(gate_up[t, 2j])) * gate_up[t, 2j + 1] */
 int tgis_k_silu_mul_interleaved(const void* gate_up_dev, void* act_dev, int32_t T, int32_t ffn);
 const char* tgis_k_last_error(void);
+/* Products on CTA pairs (csrc/gemm_pair.cu): the host raises the launches' error word at the nth launch from now on, as that launch
+ * would if one of its waits ran out (0: at none); a raised word is taken back.  Returns the launches since the last call. */
+int tgis_k_pair_fault(int32_t nth);
 /* debug builds only (-DTGIS_GEMM_TIMELINE): %globaltimer stamps of CTA 0 and CTA grid/2, [4][16] u64; else -2 */
 int tgis_k_gemm_timeline(uint64_t* out64);
 /* debug builds only (-DTGIS_STEP_TIMELINE; else -2): CTA 0 of every kernel launch records {kernel id, %globaltimer at

@@ -3490,7 +3490,16 @@ struct tgis_engine {
   // Wait until everything up to ev1 (the step's last operation on the stream) has executed.
   void wait_step_end() {
     spin_step_end();
+    check_products();
+  }
+  // A product whose wait ran out leaves its output unwritten and says so on the host: to be looked at behind every wait for the
+  // stream whose results are used.
+  void check_products() {
     if (gemm_pair_failed()) throw CudaError("a product's pipeline wait ran out: the step's results are not valid");
+  }
+  void sync_results() {
+    CK(cudaStreamSynchronize(stream));
+    check_products();
   }
   void spin_step_end() {
     if (!sync_spin) {
@@ -3787,7 +3796,7 @@ struct tgis_engine {
         if (tp > 1) publish_plan(ph);
         exec_step(ph);
         need_norm = 0;
-        CK(cudaStreamSynchronize(stream));
+        sync_results();
         for (int i = 0; i < m; ++i) emit_prompt(*prompt_rows[off + i].r, prompt_rows[off + i].pos, h_plp_out[i]);
       }
     }
@@ -3878,7 +3887,7 @@ struct tgis_engine {
       gather_final_rows(m);
       lm_head_logits(m, 1);
       CK(cudaMemcpyAsync(h_trace_logits, logits.p, (size_t)m * logits_ld * lsz, cudaMemcpyDeviceToHost, stream));
-      CK(cudaStreamSynchronize(stream));
+      sync_results();
       d2h_bytes += (long long)m * logits_ld * lsz;
       float* dst = out + off * V;
       if (logits_bf16) {

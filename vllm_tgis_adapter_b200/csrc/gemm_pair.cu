@@ -451,6 +451,8 @@ cudaError_t make_pair_word() {
   return cudaSuccess;
 }
 
+std::atomic<int> pair_launches{0}, pair_fault_in{0};   // gemm_pair_fault
+
 template <bool GROUPED>
 cudaError_t launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, PairArgs a, int grid, cudaStream_t stream) {
   static const cudaError_t attr =
@@ -459,6 +461,8 @@ cudaError_t launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, PairAr
   const cudaError_t word = gemm_pair_prepare();
   if (word != cudaSuccess) return word;
   a.err = pair_word.load(std::memory_order_acquire);
+  pair_launches.fetch_add(1, std::memory_order_relaxed);
+  if (pair_fault_in.load(std::memory_order_relaxed) > 0 && pair_fault_in.fetch_sub(1) == 1) *reinterpret_cast<volatile int*>(a.err) = 1;
   return launch_k_cluster(gemm_pair_kernel<GROUPED>, dim3(grid), dim3(PAIR_THREADS), pair_smem(GROUPED), stream, 2, wmap, xmap, a);
 }
 
@@ -469,6 +473,12 @@ cudaError_t gemm_pair_prepare() { return pair_word.load(std::memory_order_acquir
 bool gemm_pair_failed() {
   const int* w = pair_word.load(std::memory_order_acquire);
   return w != nullptr && *reinterpret_cast<const volatile int*>(w) != 0;
+}
+
+int gemm_pair_fault(int nth) {
+  if (int* w = pair_word.load(std::memory_order_acquire)) *reinterpret_cast<volatile int*>(w) = 0;
+  pair_fault_in.store(nth);
+  return pair_launches.exchange(0);
 }
 
 // Number of token tiles for a dense product of T tokens and N weight rows on `pairs` CTA pairs.  A k-block of a tile of n

@@ -90,6 +90,9 @@ cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
 int gemm_pair_plan(int T, int N, int pairs);   // token tiles of the dense launch
 cudaError_t gemm_pair_prepare();               // host memory of the launches: to be called before any of them is captured
 bool gemm_pair_failed();                       // a wait inside a launch of this process ran out
+// Tests: the host raises the error word at the nth launch from now on (0: at none), as that launch would if a wait of it ran out;
+// a raised word is taken back.  Returns the launches since the last call.
+int gemm_pair_fault(int nth);
 
 // ---- gemm_skinny.cu: the same product for up to 32 tokens; X [T, K], W [N, K] contiguous, rows on 16-byte boundaries; rope: as in
 // gemm_bf16_launch (out mode 0, N a multiple of 128)

@@ -27,6 +27,12 @@ int kfail(const std::string& m) {
     if (_e != cudaSuccess) return kfail(std::string(#expr) + ": " + cudaGetErrorString(_e)); \
   } while (0)
 
+// end of a hook that may have launched products on CTA pairs
+int product_end() {
+  KCK(cudaDeviceSynchronize());
+  return gemm_pair_failed() ? kfail("a product's pipeline wait ran out") : 0;
+}
+
 int test_num_sms() {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -50,6 +56,8 @@ struct Tmp {
 }  // namespace
 
 extern "C" {
+
+int tgis_k_pair_fault(int32_t nth) { return gemm_pair_fault(nth); }
 
 int tgis_k_gemm_timeline(uint64_t* out64) { return gemm_timeline_read((unsigned long long*)out64); }
 
@@ -113,13 +121,13 @@ int tgis_k_gemm(const void* x_dev, const void* w_dev, void* y_dev, int32_t T, in
     KCK(cudaEventRecord(e1, st));
     KCK(cudaStreamSynchronize(st));
   }
-  KCK(cudaDeviceSynchronize());
+  const int rc = product_end();
   float ms = 0.f;
   KCK(cudaEventElapsedTime(&ms, e0, e1));
   if (ms_out) *ms_out = ms / iters;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  return 0;
+  return rc;
 }
 
 int tgis_k_rmsnorm(const void* x_dev, void* residual_dev, const void* w_dev, void* out_dev, int32_t T, int32_t hidden,
@@ -194,8 +202,7 @@ int tgis_k_gemm_rope(const void* x_dev, const void* w_dev, void* y_dev, int32_t 
   KCK(sm.upload(slot_mapping_host, T));
   const GemmRope rp{pos.p, sm.p, (const bf16*)cos_sin_dev, (bf16*)k_cache_dev, (bf16*)v_cache_dev, n_q, n_kv};
   KCK(gemm_bf16_launch(wm, xm, y_dev, N, T, N, K, ws.p, ctr.p, sms, 0, 0, nullptr, nullptr, &rp, nullptr, x_dev, w_dev));
-  KCK(cudaDeviceSynchronize());
-  return 0;
+  return product_end();
 }
 
 // Layer-stack slice  a -> [GEMM W1] -> (+ residual, RMSNorm w_norm) -> [GEMM W2 (out_mode2: 0 bf16, 2 fused SwiGLU)] -> y2
@@ -253,13 +260,13 @@ int tgis_k_gemm_norm_chain(const void* a_dev, int32_t a_rows_alloc, const void* 
     }
   }
   KCK(cudaEventRecord(e1, 0));
-  KCK(cudaDeviceSynchronize());
+  const int rc = product_end();
   float ms = 0.f;
   KCK(cudaEventElapsedTime(&ms, e0, e1));
   if (us_out) *us_out = ms * 1000.f / iters;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  return 0;
+  return rc;
 }
 
 int tgis_k_attention(const void* qkv_dev, const void* k_cache_dev, const void* v_cache_dev, const int32_t* seqs_host,
@@ -529,8 +536,7 @@ int tgis_k_gemm_any(const void* x, const void* w, void* y, int32_t x_dt, int32_t
     a.gather_ws = ws.p; a.gather_ws_bytes = (size_t)T * K * sizeof(bf16);
   }
   KCK(gemm_any_launch(a, 0));
-  KCK(cudaDeviceSynchronize());
-  return 0;
+  return product_end();
 }
 
 int tgis_k_rmsnorm_f32(const float* x, int32_t ldx, const float* w, float w_off, void* out, int32_t out_dt, int32_t ldo,
