@@ -101,6 +101,9 @@ const char* tgis_k_last_error(void);
 /* Products on CTA pairs (csrc/gemm_pair.cu): the host raises the launches' error word at the nth launch from now on, as that launch
  * would if one of its waits ran out (0: at none); a raised word is taken back.  Returns the launches since the last call. */
 int tgis_k_pair_fault(int32_t nth);
+/* Tensor parallelism, host only (csrc/engine.cu wait_workers): rank 0's wait until the counter of every worker 1 .. tp - 1 stands at
+ * `seq`.  0, or -1 with tgis_last_error when a worker has failed, died or not come that far in timeout_s. */
+int tgis_k_tp_wait(const uint64_t* counters, const int32_t* failed, const int32_t* pids, int32_t tp, uint64_t seq, double timeout_s);
 /* debug builds only (-DTGIS_GEMM_TIMELINE): %globaltimer stamps of CTA 0 and CTA grid/2, [4][16] u64; else -2 */
 int tgis_k_gemm_timeline(uint64_t* out64);
 /* debug builds only (-DTGIS_STEP_TIMELINE; else -2): CTA 0 of every kernel launch records {kernel id, %globaltimer at

@@ -168,7 +168,8 @@ struct ShmCtl {
   std::atomic<uint64_t> seq;
   std::atomic<uint32_t> shutdown;
   uint32_t pad;
-  std::atomic<uint64_t> ack[16];
+  std::atomic<uint64_t> ack[16];     // the plan a worker has taken
+  std::atomic<uint64_t> done[16];    // the plan whose results a worker has and holds valid
   std::atomic<int32_t> pid[16];      // liveness: every rank publishes its process id
   std::atomic<int32_t> failed[16];   // a worker that hit an error says so before it leaves
   StepHeader hdr;
@@ -176,6 +177,30 @@ struct ShmCtl {
 };
 static_assert(sizeof(ShmCtl) <= 1024, "ShmCtl must fit below SHM_STAGE_OFF");
 constexpr size_t SHM_STAGE_OFF = 1024;
+
+bool pid_alive(int pid) { return pid > 0 && (kill(pid, 0) == 0 || errno == EPERM); }
+
+// Rank 0: until the counter of every worker 1 .. tp - 1 stands at `seq`.  Throws when one has failed, died or not come that far
+// in `timeout_s`; returns early when `stop` is set.
+void wait_workers(const std::atomic<uint64_t>* at, const std::atomic<int32_t>* failed, const std::atomic<int32_t>* pids, int tp,
+                  uint64_t seq, double timeout_s, const std::atomic<bool>* stop, const char* what) {
+  for (int r = 1; r < tp; ++r) {
+    double t_check = 0;
+    const double t_start = now_s();
+    while (at[r].load(std::memory_order_acquire) != seq) {
+      if (*stop) return;
+      const double t = now_s();
+      if (t - t_start > 0.002 && t - t_check > 0.05) {
+        t_check = t;
+        const std::string who = "tensor-parallel worker rank " + std::to_string(r);
+        if (failed[r].load(std::memory_order_acquire)) throw CudaError(who + " reported a failure");
+        const int pid = pids[r].load(std::memory_order_acquire);
+        if (pid > 0 && !pid_alive(pid)) throw CudaError(who + " (pid " + std::to_string(pid) + ") died");
+        if (t - t_start > timeout_s) throw CudaError(who + " " + what + " for " + std::to_string((int)timeout_s) + " s");
+      }
+    }
+  }
+}
 
 // gathered: [tp][R][Vl] -> out: [R][tp*Vl], elements of `esz` bytes moved as 16-byte vectors (Vl * esz % 16 == 0)
 __global__ void gather_relayout_kernel(const uint4* __restrict__ gathered, uint4* __restrict__ out, int R, int Vl16,
@@ -838,6 +863,7 @@ struct tgis_engine {
       shm->shutdown.store(0);
       for (auto& a : shm->ack) a.store(0);
       for (auto& a : shm->pid) a.store(0);
+      for (auto& a : shm->done) a.store(0);
       for (auto& a : shm->failed) a.store(0);
       shm->pid[0].store((int32_t)getpid(), std::memory_order_release);
     }
@@ -929,31 +955,12 @@ struct tgis_engine {
     ++n_launches;
   }
 
-  static bool pid_alive(int pid) { return pid > 0 && (kill(pid, 0) == 0 || errno == EPERM); }
-
   // rank 0: wait until every worker has taken the previous plan, then publish this one.  The wait is a spin (the
   // common case is microseconds) with a liveness check: a worker that died or reported a failure turns into an
   // exception here -> fail_all -> errored, instead of rank 0 spinning forever behind a healthy-looking /health.
   void publish_plan(const StepHeader& h) {
-    for (int r = 1; r < tp; ++r) {
-      double t_check = 0;
-      const double t_start = now_s();
-      while (shm->ack[r].load(std::memory_order_acquire) != plan_seq) {
-        if (stop_flag) return;
-        const double t = now_s();
-        if (t - t_start > 0.002 && t - t_check > 0.05) {
-          t_check = t;
-          if (shm->failed[r].load(std::memory_order_acquire))
-            throw CudaError("tensor-parallel worker rank " + std::to_string(r) + " reported a failure");
-          const int pid = shm->pid[r].load(std::memory_order_acquire);
-          if (pid > 0 && !pid_alive(pid))
-            throw CudaError("tensor-parallel worker rank " + std::to_string(r) + " (pid " + std::to_string(pid) + ") died");
-          if (t - t_start > tp_timeout_s)
-            throw CudaError("tensor-parallel worker rank " + std::to_string(r) + " did not take a step plan for " +
-                            std::to_string((int)tp_timeout_s) + " s");
-        }
-      }
-    }
+    wait_workers(shm->ack, shm->failed, shm->pid, tp, plan_seq, tp_timeout_s, &stop_flag, "did not take a step plan");
+    if (stop_flag) return;
     memcpy(reinterpret_cast<uint8_t*>(shm) + SHM_STAGE_OFF, h_stage, h.copy_bytes);
     shm->hdr = h;
     shm->seq.store(++plan_seq, std::memory_order_release);
@@ -982,7 +989,8 @@ struct tgis_engine {
         seen = s;
         shm->ack[rank].store(s, std::memory_order_release);
         exec_step(h);
-        CK(cudaStreamSynchronize(stream));
+        sync_results();
+        shm->done[rank].store(s, std::memory_order_release);
         ++n_steps;
       }
     } catch (...) {
@@ -3494,8 +3502,12 @@ struct tgis_engine {
   }
   // A product whose wait ran out leaves its output unwritten and says so on the host: to be looked at behind every wait for the
   // stream whose results are used.
+  // (rank 0 of a tensor-parallel group: a worker's partial sums are in the results too, so it waits for the workers to have
+  // looked; they end their step before rank 0, which samples after them)
   void check_products() {
     if (gemm_pair_failed()) throw CudaError("a product's pipeline wait ran out: the step's results are not valid");
+    if (tp > 1 && rank == 0 && plan_seq > 0)
+      wait_workers(shm->done, shm->failed, shm->pid, tp, plan_seq, tp_timeout_s, &stop_flag, "did not finish a step");
   }
   void sync_results() {
     CK(cudaStreamSynchronize(stream));
@@ -4652,6 +4664,17 @@ void tgis_engine_destroy(tgis_engine* e) {
   tgis_engine_shutdown(e);
   cudaSetDevice(e->cfg.device);
   delete e;
+}
+
+int tgis_k_tp_wait(const uint64_t* counters, const int32_t* failed, const int32_t* pids, int32_t tp, uint64_t seq, double timeout_s) {
+  const std::atomic<bool> stop{false};
+  try {
+    wait_workers(reinterpret_cast<const std::atomic<uint64_t>*>(counters), reinterpret_cast<const std::atomic<int32_t>*>(failed),
+                 reinterpret_cast<const std::atomic<int32_t>*>(pids), tp, seq, timeout_s, &stop, "did not finish a step");
+  } catch (const std::exception& ex) {
+    return fail(ex.what());
+  }
+  return 0;
 }
 
 }  // extern "C"
