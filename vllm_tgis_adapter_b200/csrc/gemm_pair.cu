@@ -21,7 +21,7 @@
 // Roles per CTA: warp 0 TMA producer, warp 1 MMA issuer (leader CTA only) and TMEM owner, warps 2..5 epilogue on a double
 // buffered accumulator (2 x 256 columns).  The leader's `full` barrier counts both CTAs' bytes; tcgen05.commit releases a
 // ring slot in both CTAs at once.  No wait is unbounded: after about two seconds a role gives up, raises the host-visible
-// error word and leaves; TMEM is freed on every path.
+// error word and leaves; copies and MMAs that are still in flight land first, and TMEM is freed on every path.
 #include <atomic>
 #include <mutex>
 
@@ -246,6 +246,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   uint64_t* tmem_full = empty_bar + PAIR_STAGES;
   uint64_t* tmem_empty = tmem_full + 2;
   uint32_t* tmem_base_smem = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_base_smem + 1);   // some role's wait ran out
   int* seg_start = reinterpret_cast<int*>(smem + 2 * PAIR_STAGES * PAIR_TILE_BYTES + PAIR_BAR_BYTES);
 
   const int warp = threadIdx.x >> 5, lane = (int)lane_id();
@@ -267,6 +268,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
         mbar_init(&tmem_full[i], 1);   // commit_pair
         mbar_init(&tmem_empty[i], 8);  // four epilogue warps of either CTA (leader's barrier)
       }
+      *gave_up = 0;
       fence_barrier_init();
     }
     __syncwarp();
@@ -352,7 +354,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
         have = it.next(t);
         if (have) set_tile();
       }
-      if (!ok) __nanosleep(1000000);   // copies in flight land before the CTA leaves
+      if (!ok) *gave_up = 1;
     }
   } else if (warp == 1) {
     // ===================== MMA issuer (leader) =====================
@@ -392,6 +394,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
           acc_phase ^= 1;
         }
       }
+      if (!ok && lane == 0) *gave_up = 1;
     }
   } else {
     // ===================== epilogue (both CTAs): lane = weight row, column = token =====================
@@ -402,7 +405,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
     uint32_t acc_phase = 0;
     if (!GROUPED) griddep_wait();   // Y (and the input scales) may still be in use by the previous kernels
     while (it.next(t)) {
-      if (!__all_sync(0xffffffffu, pair_wait(&tmem_full[acc], acc_phase, a.err))) break;
+      if (!__all_sync(0xffffffffu, pair_wait(&tmem_full[acc], acc_phase, a.err))) {
+        if (lane == 0) *gave_up = 1;
+        break;
+      }
       tc_fence_after();
       const int n = t.n0 + rank * 128 + sub * 32 + lane;
       const uint32_t taddr = tmem_base + acc * 256 + ((uint32_t)(sub * 32) << 16);
@@ -428,6 +434,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   }
   tc_fence_before();
   __syncthreads();
+  // A wait that ran out in any role leaves copies and MMAs of the others behind, all issued by now and done long before this
+  // millisecond is over: neither shared memory nor TMEM is given back while they may still write there.  (Where the leader's MMAs
+  // stop, the other CTA's epilogue gets no accumulator and comes here too.)
+  if (*gave_up)
+    for (const long long t0 = clock64(); clock64() - t0 < 2000000ll;) {}
   cluster_sync_all();   // nobody leaves while the peer may still read its shared memory or signal its barriers
   if (warp == 1) {
     tc_fence_after();
