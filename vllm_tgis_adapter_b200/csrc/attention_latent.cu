@@ -464,12 +464,15 @@ latent_attn_mma_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __r
 // ---- prompts: four of those tiles of one sequence per CTA ----------------------------------------------------------------
 // With sixteen heads a tile holds one token, and in a prompt neighbouring tokens stream the same cache rows: 16 rows of S for
 // every block staged.  Here a CTA takes up to 64 (token, head) rows, four M tiles against each staged 32-row block:
-//   scores  warp w: M tile w & 3, keys 16 (w >> 2) .. + 15, two interleaved k chains;
+//   scores  warp w: M tile w & 3, keys 16 (w >> 2) .. + 15, the two halves of k as interleaved chains;
 //   softmax fp32, four lanes per row with eight keys each;
 //   output  warp w: columns [8 NTW w, 8 NTW (w + 1)) of all four M tiles (128 fp32 accumulators a thread at kv_rank 512), so that
 //           a fragment of C serves four MMAs.
+// Every sum runs in the order in which latent_attn_mma_kernel makes it, so a query has the same bits whichever of the two kernels
+// the rest of its step sends it to.
 // One CTA of eight warps per SM (163 KB at row 576), so what bounds it are the latencies between the three barriers of a
-// block.  Measured: prompts of 937, 767, 68, 220 and 56 tokens, 16 heads, row 576: 360 us a launch before, 235 here.
+// block.  Measured: prompts of 937, 767, 68, 220 and 56 tokens, 16 heads, row 576: 360 us a launch before, 235 here (the same
+// with the sums in the other kernel's order: 279.6 under the profiler, 278.4 with sums of its own).
 constexpr int LATW_ROWS = 4 * LATENT_PAIRS;
 constexpr int LATW_LDS = 36, LATW_LDP = 40;   // padded rows of S (floats) and P (bf16)
 inline size_t lat_wide_smem(int D) {
@@ -492,12 +495,15 @@ latent_attn_wide_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __
   griddep_launch();
   griddep_wait();
   const LatentTile tile = tiles[blockIdx.x];
-  if (tile.q0 % (4 * tile_tokens) != 0) return;   // the first of its four tiles does the work
   const AttnSeq sq = seqs[tile.seq];
-  const int h0 = blockIdx.y * LATENT_PAIRS, nh = min(g.heads - h0, LATENT_PAIRS);
-  const int nq = min(4 * tile_tokens, sq.q_len - tile.q0), rows = nq * nh, n_mt = (rows + 15) / 16;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int pos0 = sq.kv_len - sq.q_len + tile.q0, row0 = sq.q_start + tile.q0;
+  // The first of a group's tiles does the work.  Groups are cut at positions that are multiples of four tiles, so that they end
+  // where a cache block does (one to eight tokens to a tile): the rows of a group see the same last block, as each tile by itself.
+  const int group = 4 * tile_tokens, at = pos0 % group;
+  if (tile.q0 != 0 && at >= tile_tokens) return;
+  const int h0 = blockIdx.y * LATENT_PAIRS, nh = min(g.heads - h0, LATENT_PAIRS);
+  const int nq = min((group - at + tile_tokens - 1) / tile_tokens * tile_tokens, sq.q_len - tile.q0), rows = nq * nh, n_mt = (rows + 15) / 16;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   {  // zero what no copy fills (unused rows, k padding), then Q, scaled and rounded to bf16 once
     uint32_t* z = reinterpret_cast<uint32_t*>(smem_raw);
     for (int i = rows * LDQ / 2 + tid; i < LATW_ROWS * LDQ / 2; i += LAT_THREADS) z[i] = 0u;
@@ -529,7 +535,7 @@ latent_attn_wide_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   // softmax: four lanes per row, eight keys each
-  const int sr = tid >> 2, sk = (tid & 3) * 8, sposq = sr < rows ? pos0 + sr / nh : -1;
+  const int sr = tid >> 2, sk = tid & 3, sposq = sr < rows ? pos0 + sr / nh : -1;
   float m_run = -FLT_MAX, l_run = 0.f;
   float acc[4][NTW][4];
 #pragma unroll
@@ -549,7 +555,7 @@ latent_attn_wide_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __
     __syncthreads();  // block `blk` has landed for everyone; everyone is done with the other buffer, P, S and corr
     if (blk < blk1) load_block(blk + 1, st ^ 1);
     const bf* Kb = Ks + (size_t)st * KV_BLOCK * LDQ;
-    if (mt < n_mt) {  // ---- scores
+    if (mt < n_mt) {  // ---- scores: the two halves of the row length side by side (chain 1 is one step longer when KS is odd)
       float c[2][2][4];
 #pragma unroll
       for (int i = 0; i < 2; ++i)
@@ -558,24 +564,19 @@ latent_attn_wide_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __
 #pragma unroll
           for (int e = 0; e < 4; ++e) c[i][j][e] = 0.f;
       const bf* kf = Kb + k_frag;
-#pragma unroll 3
-      for (int ks = 0; ks + 1 < KS; ks += 2) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          uint32_t a[4], b[4];
-          lat_ldsm_x4(a, q_frag + (ks + i) * 16);
-          lat_ldsm_x4(b, kf + (ks + i) * 16);
-          lat_mma(c[i][0], a, b[0], b[1]);
-          lat_mma(c[i][1], a, b[2], b[3]);
-        }
-      }
-      if (KS & 1) {
+      auto step = [&](int i, int ks) {
         uint32_t a[4], b[4];
-        lat_ldsm_x4(a, q_frag + (KS - 1) * 16);
-        lat_ldsm_x4(b, kf + (KS - 1) * 16);
-        lat_mma(c[0][0], a, b[0], b[1]);
-        lat_mma(c[0][1], a, b[2], b[3]);
+        lat_ldsm_x4(a, q_frag + ks * 16);
+        lat_ldsm_x4(b, kf + ks * 16);
+        lat_mma(c[i][0], a, b[0], b[1]);
+        lat_mma(c[i][1], a, b[2], b[3]);
+      };
+#pragma unroll 3
+      for (int ks = 0; ks < KS / 2; ++ks) {
+        step(0, ks);
+        step(1, KS / 2 + ks);
       }
+      if (KS & 1) step(1, KS - 1);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         float* sp = Sp + (size_t)(mt * 16 + gq) * LATW_LDS + kh * 16 + j * 8 + t2;
@@ -584,15 +585,15 @@ latent_attn_wide_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __
       }
     }
     __syncthreads();
-    {  // ---- softmax
+    {  // ---- softmax: keys sk, sk + 4, ... of row sr; sums in the order of a warp's sixteen-, eight-, ... lane exchanges over 32 keys
       float x[8];
-      const float4 xa = *reinterpret_cast<const float4*>(Sp + sr * LATW_LDS + sk), xb = *reinterpret_cast<const float4*>(Sp + sr * LATW_LDS + sk + 4);
-      x[0] = xa.x; x[1] = xa.y; x[2] = xa.z; x[3] = xa.w; x[4] = xb.x; x[5] = xb.y; x[6] = xb.z; x[7] = xb.w;
-      const int last = sposq - (blk * KV_BLOCK + sk), first = g.window > 0 ? last - g.window + 1 : 0;   // visible: first <= e <= last
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = Sp[sr * LATW_LDS + sk + 4 * e];
+      const int last = sposq - (blk * KV_BLOCK + sk), first = g.window > 0 ? last - g.window + 1 : 0;   // visible: first <= 4 e <= last
       float m_new = -FLT_MAX;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        x[e] = e <= last && e >= first ? x[e] : -FLT_MAX;
+        x[e] = 4 * e <= last && 4 * e >= first ? x[e] : -FLT_MAX;
         m_new = fmaxf(m_new, x[e]);
       }
       m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 1));
@@ -600,24 +601,15 @@ latent_attn_wide_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __
       m_new = fmaxf(m_new, m_run);
       // nothing visible so far (m_new still the sentinel): all weights 0, state unchanged
       const float corr = m_new == -FLT_MAX ? 1.f : expf(m_run - m_new);
-      float sum = 0.f;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        x[e] = x[e] == -FLT_MAX ? 0.f : expf(x[e] - m_new);
-        sum += x[e];
-      }
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      for (int e = 0; e < 8; ++e) x[e] = x[e] == -FLT_MAX ? 0.f : expf(x[e] - m_new);
+      float sum = ((x[0] + x[4]) + (x[2] + x[6])) + ((x[1] + x[5]) + (x[3] + x[7]));
       sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
       l_run = l_run * corr + sum;
       m_run = m_new;
-      uint4 pk;
-      uint32_t* w = &pk.x;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const __nv_bfloat162 h2 = __floats2bfloat162_rn(x[2 * e], x[2 * e + 1]);
-        w[e] = *reinterpret_cast<const uint32_t*>(&h2);
-      }
-      *reinterpret_cast<uint4*>(Ps + sr * LATW_LDP + sk) = pk;
+      for (int e = 0; e < 8; ++e) Ps[sr * LATW_LDP + sk + 4 * e] = __float2bfloat16_rn(x[e]);
       if (sk == 0) corr_s[sr] = corr;
     }
     __syncthreads();
