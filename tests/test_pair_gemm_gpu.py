@@ -117,3 +117,50 @@ def test_pair_expert_segments(lib, counts, N, K, gathered, mode):
         over = (y[:rows].double() - ref).abs() - tol - (2.0 ** -8 * ref.abs() if y_dt else 0)
         assert float(over.max()) <= 0, float(over.max())
         assert bool((y[rows] == 7.0).all())
+
+
+def test_expert_swiglu_divides_as_the_other_kernels_do(lib):
+    """Every bf16 gate (with bits below it, infinities and NaN among them) and ups of every size: the bits of the one-CTA product
+    over the same rows, whose epilogue divides with IEEE rounding."""
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    gate = torch.arange(-32768, 32768, dtype=torch.int32, device="cuda").to(torch.int16).view(torch.bfloat16)
+    low = (gate.double() * (torch.rand(65536, generator=gen, device="cuda").double() - 0.5) * 2.0 ** -8).bfloat16()   # gate + low is one fp32 number
+    low = torch.where(gate.float().abs().isfinite() & (gate.float().abs() > 2.0 ** -100), low, torch.zeros_like(low))
+    T, N, K = 301, 131072, 64
+    w = torch.zeros(N, K, device="cuda", dtype=torch.bfloat16)
+    w[0::2, 0], w[0::2, 1], w[1::2, 2] = gate, low, 1.0
+    x = torch.zeros(T, K, device="cuda", dtype=torch.bfloat16)
+    x[:, 0] = 1.0
+    x[1::2, 1] = 1.0
+    x[:, 2] = (torch.randn(T, generator=gen, device="cuda") * torch.exp2(torch.randint(-30, 30, (T,), generator=gen, device="cuda").float())).bfloat16()
+    x[:6, 2] = torch.tensor([1.0, 1.0, -1.0, 0.0, 3e38, 1e-38], device="cuda").bfloat16()
+    p = lambda t: C.c_void_p(t.data_ptr()) if t is not None else None  # noqa: E731
+
+    def product(seg):
+        y = torch.empty(T, N // 2, device="cuda", dtype=torch.bfloat16)
+        assert lib.tgis_k_gemm_any(p(x), p(w), p(y), 1, 1, 1, T, N, K, K, K, N // 2, 1, 0, 0, 0, p(seg), 1 if seg is not None else 0, N * K, None, 1, ANY["swiglu"],
+                                   None, 0) == 0, lib.tgis_k_last_error()
+        return y
+
+    pairs, one_cta = product(torch.tensor([0, T], device="cuda", dtype=torch.int32)), product(None)
+    assert torch.equal(pairs.isnan(), one_cta.isnan())
+    differ = (pairs.view(torch.int16) != one_cta.view(torch.int16)) & ~pairs.isnan()
+    assert int(differ.sum()) == 0, (int(differ.sum()), gate[differ.any(0)][:8].tolist())
+
+
+def test_dense_swiglu_divides_as_the_register_kernel_does(lib):
+    """Every bf16 gate through the epilogue that skips the IEEE division where it cannot matter, against the kernel of up to 8
+    tokens, which always divides."""
+    gen = torch.Generator(device="cuda").manual_seed(12)
+    gate = torch.arange(-32768, 32768, dtype=torch.int32, device="cuda").to(torch.int16).view(torch.bfloat16)
+    K = 64
+    w = torch.zeros(131072, K, device="cuda", dtype=torch.bfloat16)
+    w[0::2, 0], w[1::2, 1] = gate, 1.0
+    x = torch.zeros(300, K, device="cuda", dtype=torch.bfloat16)
+    x[:, 0] = 1.0
+    x[:, 1] = torch.randn(300, generator=gen, device="cuda").bfloat16()
+    x[:4, 1] = torch.tensor([1.0, -1.0, 0.0, 3e38], device="cuda").bfloat16()
+    many = run(lib, x, w, 300, SWIGLU, 300).reshape(-1)[: 300 * 65536].view(300, 65536)[:8]
+    few = torch.cat([run(lib, x[:256].contiguous(), w[at: at + 16384].contiguous(), 8, SWIGLU, 256).reshape(-1)[: 8 * 8192].view(8, 8192) for at in range(0, 131072, 16384)], 1)
+    assert torch.equal(many.isnan(), few.isnan())
+    assert bool(((many.view(torch.int16) == few.view(torch.int16)) | many.isnan()).all())

@@ -104,15 +104,8 @@ __device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, int* e
   return true;
 }
 
-// (a quotient within 2 ulp and without the branch of an IEEE division; the result is rounded to bf16)
-__device__ __forceinline__ float pair_silu(float g) { return __fdividef(g, 1.f + expf(-g)); }
-template <int MODE>
-__device__ __forceinline__ float pair_glu(float g, float u) {
-  if constexpr (MODE == PAIR_SWIGLU) {
-    return pair_silu(g) * u;
-  } else {
-    return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
-  }
+__device__ __forceinline__ float pair_geglu(float g, float u) {
+  return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
 }
 template <int MODE>
 __device__ __forceinline__ float pair_act(float v, float s) {
@@ -213,9 +206,11 @@ __device__ __forceinline__ void pair_store(const PairArgs& a, const PairTile& t,
         silu_bf16_n(g, v);
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[j] *= bf16_round(u[j]);
+      } else if constexpr (MODE == PAIR_SWIGLU) {
+        silu_mul_bf16_n(g, u, v, mine_valid <= 0 ? 0u : 0xffffu >> (16 - min((mine_valid + 1) / 2, 16)));   // tokens 2 j < mine_valid
       } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = pair_glu<MODE>(g[j], u[j]);
+        for (int j = 0; j < 16; ++j) v[j] = pair_geglu(g[j], u[j]);
       }
 #pragma unroll
       for (int j = 0; j < 16; ++j)
