@@ -82,3 +82,14 @@ def test_skinny_qkv_with_rope_equals_the_two_launches(lib, T, n_q, n_kv):
     assert torch.equal(y[0][:T], y[1][:T])
     for a, b in zip(*caches):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("N,K", [(2368, 1024), (2384, 1024), (4480, 960), (4736, 896), (4864, 896), (768, 3072)])
+@pytest.mark.parametrize("mode", [PLAIN_F32, SWIGLU])
+def test_a_row_is_the_same_beside_7_8_or_31_others(lib, N, K, mode):
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(32, K, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(N, K, generator=gen, device="cuda") * K ** -0.5).bfloat16()
+    n = N // 2 if mode == SWIGLU else N
+    rows = {T: run(lib, x, w, T, mode).reshape(-1)[: T * n].view(T, n) for T in (1, 8, 9, 32)}
+    assert torch.equal(rows[1], rows[32][:1]) and torch.equal(rows[8], rows[32][:8]) and torch.equal(rows[9], rows[32][:9])

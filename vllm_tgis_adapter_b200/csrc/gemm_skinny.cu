@@ -194,7 +194,7 @@ cudaError_t launch_nt(const SkinnyArgs& a, cudaStream_t s) {
   }
 }
 
-constexpr int SKINNY_ONE_WAVE = 148 * 16;   // weight rows that 16-row CTAs cover with one CTA per SM
+constexpr int SKINNY_ONE_WAVE = 148 * 16;   // weight rows that 16-row CTAs cover with one CTA per SM (a constant: bits hang on it)
 
 }  // namespace
 
@@ -209,18 +209,19 @@ bool gemm_skinny_takes(int T, int N, int K) {
 cudaError_t gemm_skinny_launch(const void* X, const void* W, void* Y, int ldy, int T, int N, int K, int out_mode, const GemmRope* rope,
                                cudaStream_t stream) {
   SkinnyArgs a{(const __nv_bfloat16*)X, (const __nv_bfloat16*)W, Y, ldy, T, N, K, out_mode, {}};
-  // k-splits depend on N and on T <= 8 alone, so that a product has the same bits with every epilogue.  Sixteen warps where an
-  // SM holds one CTA; 32-row CTAs for few tokens (more loads in flight), 16-row ones beyond eight (fewer activation bytes in
-  // flight per register).
-  const bool few = T <= 8, wide = few ? N > 2 * SKINNY_ONE_WAVE : N > SKINNY_ONE_WAVE;
+  // The number of warps, and with it the order of k, hangs on N alone: a row has the same bits beside 31 others as alone, and with
+  // every epilogue.  Sixteen warps where an SM holds one CTA, of 16 rows up to one wave, of 32 rows up to two; eight beyond that,
+  // with 32-row CTAs for few tokens (more loads in flight) and 16-row ones beyond eight (fewer activation bytes in flight per
+  // register).  Between one and two waves eight warps were measured too, microseconds at 1, 8, 9, 16, 24 and 32 tokens, warm
+  // weights, eight warps of 16 rows -> sixteen of 32: 2560 x 1024 2.4 2.5 2.8 3.1 3.5 4.0 -> 2.2 2.2 2.5 2.6 3.5 4.4, 4608 x 960
+  // 2.4 2.6 2.9 3.1 3.6 4.1 -> 2.2 2.2 2.8 2.8 3.9 4.7.
+  const bool sixteen = N <= 2 * SKINNY_ONE_WAVE;
   if (rope != nullptr) {
     a.rope = *rope;
-    return wide ? launch_nt<2, 8, true>(a, stream) : launch_nt<2, 16, true>(a, stream);
+    return sixteen ? launch_nt<2, 16, true>(a, stream) : launch_nt<2, 8, true>(a, stream);
   }
-  if (few && wide) return launch<2, 1, 8, false>(a, stream);
-  if (wide) return launch_nt<1, 8, false>(a, stream);
-  if (few && N > SKINNY_ONE_WAVE) return launch<2, 1, 16, false>(a, stream);
-  return launch_nt<1, 16, false>(a, stream);
+  if (!sixteen) return T <= 8 ? launch<2, 1, 8, false>(a, stream) : launch_nt<1, 8, false>(a, stream);
+  return N > SKINNY_ONE_WAVE ? launch_nt<2, 16, false>(a, stream) : launch_nt<1, 16, false>(a, stream);
 }
 
 }  // namespace tgis
