@@ -73,15 +73,28 @@ def test_segments_and_epilogues(lib, counts, mode, K):
     assert bool((y[rows] == 7.0).all())
 
 
-def test_a_row_is_the_same_in_every_tile_height(lib):
+@pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,N,K,ld", [(1537, 1089, 289, 289), (1600, 1152, 300, 300), (1601, 1100, 260, 264)])
+def test_dense_tiles_of_64_rows(lib, T, N, K, ld, wdt):
+    """Launches of three and more 64 x 64 tiles for every SM and more than 256 products per sum."""
+    test_dense(lib, T, N, K, ld, wdt)
+
+
+@pytest.mark.parametrize("mode,K", [(0, 257), (1, 288), (3, 300), (5, 260), (6, 292)])
+def test_segments_and_epilogues_in_tiles_of_64_rows(lib, mode, K):
+    test_segments_and_epilogues(lib, [1000, 0, 63, 64, 65, 1, 2107] * 5, mode, K)   # 3 column tiles, 35 segments of 470 rows on average
+
+
+@pytest.mark.parametrize("K", [64, 100, 300, 301])   # one chain a sum; 16 and 32 rows only; all three heights, wide and single loads
+def test_a_row_is_the_same_in_every_tile_height(lib, K):
     gen = torch.Generator(device="cuda").manual_seed(3)
-    x, w = torch.randn(1500, 100, generator=gen, device="cuda"), torch.randn(1000, 100, generator=gen, device="cuda")
+    x, w = torch.randn(1600, K, generator=gen, device="cuda"), torch.randn(1100, K, generator=gen, device="cuda")
 
     def run(a):
-        y = torch.empty(a.shape[0], 1000, device="cuda")
-        assert lib.tgis_k_gemm_any(p(a), p(w), p(y), 0, 0, 0, a.shape[0], 1000, 100, 100, 100, 1000, 1, 0, 0, 0, None, 0, 0, None, 1, 0, None, 0) == 0
+        y = torch.empty(a.shape[0], 1100, device="cuda")
+        assert lib.tgis_k_gemm_any(p(a), p(w), p(y), 0, 0, 0, a.shape[0], 1100, K, K, K, 1100, 1, 0, 0, 0, None, 0, 0, None, 1, 0, None, 0) == 0
         return y
 
-    whole = run(x)   # 64-row tiles
+    whole = run(x)   # 450 tiles of 64 rows where K > 256
     assert torch.equal(run(x[40:100].contiguous()), whole[40:100])   # 32
     assert torch.equal(run(x[90:99].contiguous()), whole[90:99])     # 16

@@ -64,9 +64,12 @@ __device__ __forceinline__ float relu2_row_scale(const GemmAny& a, int dst) {
 // 16 x 1024 x 1024 93 -> 25 us; 40 TFLOP/s where there are tiles enough (of 74: the shared-memory loads take the rest).
 constexpr int FMA_THREADS = 128;
 constexpr int FMA_BN = 64, FMA_BK = 32, FMA_LD = FMA_BK + 4;
-constexpr int FMA_SMS = 148;
-// Sums of up to 64 terms run as one ascending chain per output, not as an even and an odd one that meet at the end: two k-blocks
-// wait for memory, not for arithmetic, so they keep the order of a plain loop.
+constexpr int FMA_SMS = 148;   // (tile heights only: a sum does not depend on them)
+// Sums of up to 64 terms run as one ascending chain per output, not as an even and an odd one that meet at the end.  The reason is
+// which values they give, not speed: small float32 models are compared with 64-bit arithmetic to within 1e-4, some of them are
+// conditioned so badly that one ulp of the inputs moves their logits by as much, and this is the order in which they were
+// always summed.  Both orders are equally exact (the bound in the tests holds for either).  It costs time: 2048 x 2048 44 us at K = 64
+// against 40 at K = 68 in packed pairs, 512 x 1024 8.3 against 8.1, 93 x 128 7.6 against 6.2.
 constexpr int FMA_CHAIN_K = 64;
 
 __device__ __forceinline__ void fma_low(unsigned long long& d, float x, float w) {   // the pair's lower half
