@@ -95,7 +95,11 @@ int tgis_k_lora(const void* x_dev, int32_t ldx, const int32_t* tok_slot_dev, con
 int tgis_k_lora_bench(const void* x_dev, int32_t ldx, const int32_t* tok_slot_dev, const void* a_dev, const void* b_dev,
                       int32_t K, int32_t N, int32_t Rm, void* y_dev, int32_t ldy, int32_t T, int32_t iters,
                       float* us_shrink, float* us_expand);
-/* act[t, j] = bf16(silu(gate_up[t, 2j])) * gate_up[t, 2j + 1] */
+/* The same over interleaved gate / up columns with SwiGLU behind it: gate_up [T, 2 ffn] is the projection's result and only read,
+ * y = gate_up + delta as above, act[t, j] = bf16(silu(y[t, 2j])) * y[t, 2j + 1] (tokens without an adapter too); B [slots][2 ffn][Rm] */
+int tgis_k_lora_swiglu(const void* x_dev, int32_t ldx, const int32_t* tok_slot_dev, const void* a_dev, const void* b_dev, int32_t K,
+                       int32_t ffn, int32_t Rm, const void* gate_up_dev, void* act_dev, int32_t T);
+/* ... and where no token has one: act[t, j] = bf16(silu(gate_up[t, 2j])) * gate_up[t, 2j + 1] */
 int tgis_k_silu_mul_interleaved(const void* gate_up_dev, void* act_dev, int32_t T, int32_t ffn);
 const char* tgis_k_last_error(void);
 /* Products on CTA pairs (csrc/gemm_pair.cu): the host raises the launches' error word at the nth launch from now on, as that launch

@@ -64,6 +64,38 @@ def test_silu_mul_interleaved_matches_split_layout(g):
     assert torch.equal(act.cpu(), want)
 
 
+@pytest.mark.parametrize("F,K,Rm", [(520, 256, 8), (4, 64, 16), (1028, 512, 64)])   # 2 F: on both sides of a CTA's 1024 columns
+@pytest.mark.parametrize("T", [1, 7, 8, 9, 256, 257])   # up to 256 tokens four CTAs share a tile's adapters, beyond that one has them all
+def test_lora_with_swiglu_on_tiles_of_up_to_eight_adapters(g, T, F, K, Rm):
+    """The expand that applies SwiGLU, on tiles of one to eight adapters, tokens without one among them: exactly silu and the product
+    of the corrected projection, which the oracle checks; the projection is only read and nothing beside act is written."""
+    from oracle.llama_oracle import lora_add
+
+    gen = torch.Generator().manual_seed(T + F)
+    slots = 11
+    x = torch.randn(T, K, generator=gen).to(torch.bfloat16)
+    gate_up = torch.randn(T, 2 * F, generator=gen).to(torch.bfloat16)
+    a = (torch.randn(slots, Rm, K, generator=gen) * 0.05).to(torch.bfloat16)
+    b = (torch.randn(slots, 2 * F, Rm, generator=gen) * 0.2).to(torch.bfloat16)
+    # tile i holds 1 + i % 8 slots, every second tile slot 0 among them
+    tok = torch.cat([torch.tensor([(3 * i + j) % slots + 1 if (j or i % 2) else 0 for j in range(1 + i % 8)] * 8)[:8] for i in range(-(-T // 8))])[:T].int()
+    if T > 8:
+        assert max(len(set(tok[i:i + 8].tolist())) for i in range(0, T, 8)) >= min(T // 8, 8)
+    xd, gu, ad, bd, td = x.cuda(), gate_up.clone().cuda(), a.cuda(), b.cuda(), tok.cuda()
+    act = torch.full((T + 1, F), 7.0, dtype=torch.bfloat16, device="cuda")
+    assert g.lib().tgis_k_lora_swiglu(g.ptr(xd), K, g.ptr(td), g.ptr(ad), g.ptr(bd), K, F, Rm, g.ptr(gu), g.ptr(act), T) == 0, g.kerr()
+    assert torch.equal(gu.cpu(), gate_up) and bool((act[T] == 7.0).all())
+    y = gate_up.clone().cuda()
+    assert g.lib().tgis_k_lora(g.ptr(xd), K, g.ptr(td), g.ptr(ad), g.ptr(bd), K, 2 * F, Rm, 0, g.ptr(y), 2 * F, T) == 0, g.kerr()
+    y = y.cpu()
+    assert torch.equal(act[:T].cpu(), torch.nn.functional.silu(y[:, 0::2]) * y[:, 1::2])
+    want = torch.cat([lora_add(gate_up[t:t + 1], x[t:t + 1], a[s - 1], b[s - 1]) if s > 0 else gate_up[t:t + 1] for t, s in enumerate(tok.tolist())])
+    # two fp32 sums in another order: every shrink sum, the delta and the result may land one bf16 ulp (2^-7) away
+    mag = torch.stack([((a[s - 1].float() @ x[t].float()).abs() * b[s - 1].float().abs()).sum(-1) if s > 0 else torch.zeros(2 * F) for t, s in enumerate(tok.tolist())])
+    assert bool(((y.float() - want.float()).abs() <= 2.0 ** -7 * (want.float().abs() + 2 * mag)).all())
+    assert float((y == want).float().mean()) > 0.97
+
+
 # ---------------------------------------------------------------------------------------------------- engine level
 def _engine(cfg_name, **kw):
     from oracle.llama_oracle import CONFIGS, rope_table, synthetic_weights

@@ -166,9 +166,6 @@ cudaError_t lora_shrink_launch(const __nv_bfloat16* x, int ldx, const int32_t* t
 // act != nullptr (one module over interleaved gate / up columns): act[t, j] = bf16(silu(gate)) * up of the sum instead of y
 cudaError_t lora_expand_launch(const float* v, const int32_t* tok_slot, const LoraGroup& g, __nv_bfloat16* y, int ldy, int T,
                                cudaStream_t stream, __nv_bfloat16* act = nullptr);
-// act[t, j] = bf16(silu(gate_up[t, 2j])) * gate_up[t, 2j + 1]  (the interleaved gate_up layout the fused GEMM epilogue reads)
-cudaError_t silu_mul_interleaved_launch(const __nv_bfloat16* gate_up, __nv_bfloat16* act, int T, int ffn,
-                                        cudaStream_t stream);
 // ---- opt.cu (OPT layer stack: learned positions, biased projections, ReLU, LayerNorm) ------------------------------
 // out[t] = bf16(tok_table[tok[t]] + pos_table[pos[t] + offset])
 cudaError_t opt_embed_launch(const int32_t* token_ids, const int32_t* positions, const __nv_bfloat16* tok_table,

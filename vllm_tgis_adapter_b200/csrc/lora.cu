@@ -36,17 +36,6 @@ namespace {
 struct F8 {
   float v[8];
 };
-__device__ __forceinline__ F8 ld8(const __nv_bfloat16* p) {
-  const uint4 r = *reinterpret_cast<const uint4*>(p);
-  const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-  F8 o;
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    o.v[2 * e] = __uint_as_float(w[e] << 16);
-    o.v[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
-  }
-  return o;
-}
 __device__ __forceinline__ float dot8(const F8& a, const F8& b) {
   float s = 0.f;
 #pragma unroll
@@ -167,13 +156,6 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* 
 // latency per block).
 constexpr int LORA_EC = 4;
 constexpr int LORA_ECOLS = 256 * LORA_EC;  // columns per CTA
-__device__ __forceinline__ void ld4f(const __nv_bfloat16* p, float (&o)[4]) {  // 4 bf16 through one 8-byte load
-  const uint2 r = *reinterpret_cast<const uint2*>(p);
-  o[0] = __uint_as_float(r.x << 16);
-  o[1] = __uint_as_float(r.x & 0xffff0000u);
-  o[2] = __uint_as_float(r.y << 16);
-  o[3] = __uint_as_float(r.y & 0xffff0000u);
-}
 __device__ __forceinline__ void st4f(__nv_bfloat16* p, const float (&f)[4]) {
   const __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
   uint2 r;
@@ -276,35 +258,6 @@ lora_expand_kernel(const float* __restrict__ v, const int32_t* __restrict__ tok_
   }
 }
 
-// gate_up [T, 2F] with interleaved columns (2j = gate_j, 2j+1 = up_j) -> act [T, F]; the rounding points of the GEMM's
-// fused SwiGLU epilogue (gemm_tcgen05.cu swiglu_bf16) and of silu_mul_kernel
-__global__ void silu_mul_interleaved_kernel(const __nv_bfloat16* __restrict__ gate_up, __nv_bfloat16* __restrict__ act,
-                                            int T, int ffn) {
-  griddep_launch();
-  griddep_wait();
-  const int vec_per_row = ffn / 4;  // 4 outputs from one 16-byte load
-  const long long total = (long long)T * vec_per_row;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int t = (int)(i / vec_per_row), c = (int)(i % vec_per_row);
-    const F8 gu = ld8(gate_up + (size_t)t * 2 * ffn + 8 * c);
-    uint2 pk;
-    uint32_t* w = &pk.x;
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      float o2[2];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const float gx = gu.v[4 * e + 2 * h], ux = gu.v[4 * e + 2 * h + 1];
-        o2[h] = bf16_round(gx / (1.0f + expf(-gx))) * ux;
-      }
-      const __nv_bfloat162 hh = __floats2bfloat162_rn(o2[0], o2[1]);
-      w[e] = *reinterpret_cast<const uint32_t*>(&hh);
-    }
-    *reinterpret_cast<uint2*>(act + (size_t)t * ffn + 4 * c) = pk;
-  }
-}
-
 }  // namespace
 
 static bool lora_group_ok(const LoraGroup& g) {
@@ -335,16 +288,6 @@ cudaError_t lora_expand_launch(const float* v, const int32_t* tok_slot, const Lo
   const dim3 grid((max_n + LORA_ECOLS - 1) / LORA_ECOLS, (T + LORA_TT - 1) / LORA_TT, g.n_mods * lora_passes_apart(T));
   return act != nullptr ? launch_k(lora_expand_kernel<true>, grid, dim3(256), 0, stream, v, tok_slot, g, y, ldy, act, T)
                         : launch_k(lora_expand_kernel<false>, grid, dim3(256), 0, stream, v, tok_slot, g, y, ldy, act, T);
-}
-
-cudaError_t silu_mul_interleaved_launch(const __nv_bfloat16* gate_up, __nv_bfloat16* act, int T, int ffn,
-                                        cudaStream_t stream) {
-  if (T <= 0) return cudaSuccess;
-  if (ffn % 4 != 0) return cudaErrorInvalidValue;
-  const long long total = (long long)T * (ffn / 4);
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  return launch_k(silu_mul_interleaved_kernel, dim3((int)blocks), dim3(256), 0, stream, gate_up, act, T, ffn);
 }
 
 }  // namespace tgis

@@ -507,10 +507,25 @@ int tgis_k_lora_bench(const void* x_dev, int32_t ldx, const int32_t* tok_slot_de
   return 0;
 }
 
-int tgis_k_silu_mul_interleaved(const void* gate_up_dev, void* act_dev, int32_t T, int32_t ffn) {
-  KCK(silu_mul_interleaved_launch((const __nv_bfloat16*)gate_up_dev, (__nv_bfloat16*)act_dev, T, ffn, 0));
+int tgis_k_lora_swiglu(const void* x_dev, int32_t ldx, const int32_t* tok_slot_dev, const void* a_dev, const void* b_dev, int32_t K,
+                       int32_t ffn, int32_t Rm, const void* gate_up_dev, void* act_dev, int32_t T) {
+  Tmp<float> v;
+  KCK(v.alloc((size_t)T * Rm));
+  LoraGroup g{};
+  g.n_mods = 1;
+  g.v_ld = Rm;
+  g.mod[0] = LoraModule{(const __nv_bfloat16*)a_dev, (const __nv_bfloat16*)b_dev, K, 2 * ffn, Rm, 0, 0};
+  if (x_dev != nullptr) KCK(lora_shrink_launch((const __nv_bfloat16*)x_dev, ldx, tok_slot_dev, g, v.p, T, 0));
+  KCK(lora_expand_launch(v.p, tok_slot_dev, g, (__nv_bfloat16*)const_cast<void*>(gate_up_dev), 2 * ffn, T, 0, (__nv_bfloat16*)act_dev));
   KCK(cudaDeviceSynchronize());
   return 0;
+}
+
+int tgis_k_silu_mul_interleaved(const void* gate_up_dev, void* act_dev, int32_t T, int32_t ffn) {   // no token names an adapter
+  if (T <= 0) return 0;
+  Tmp<int32_t> slots;
+  KCK(slots.upload(std::vector<int32_t>(T, 0).data(), T));
+  return tgis_k_lora_swiglu(nullptr, 0, slots.p, nullptr, nullptr, 8, ffn, 8, gate_up_dev, act_dev, T);
 }
 
 int tgis_k_sampler(const void* logits_dev, int32_t ld, int32_t vocab, const void* rows_host, int32_t n_rows,
