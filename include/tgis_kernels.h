@@ -120,6 +120,8 @@ int tgis_k_kv_block(void);
 
 /* ---- kernels of the layer-list architectures (fp32 residual stream, latent attention, mixture of experts) ----------
  * dtype codes: 0 = fp32, 1 = bf16.  All pointers are device memory unless marked host. */
+/* Bytes that tgis_k_gemm_any gives, on this thread, for the gathered rows of a grouped bf16 product (-1: as many as it takes) */
+int tgis_k_gemm_any_room(int64_t bytes);
 /* y = x w^T, any shape; batch > 1: one problem per batch index, operands *_bs elements apart; seg_off_dev != NULL: grouped
  * (row segment g multiplies with weight matrix g, w_gs elements apart; x row of position p = gather[p] / gather_div);
  * mode 0 plain, 1 SwiGLU over interleaved (gate, up) rows, 2 y *= row_scale[row * scale_ld + batch index] */

@@ -164,3 +164,52 @@ def test_dense_swiglu_divides_as_the_register_kernel_does(lib):
     few = torch.cat([run(lib, x[:256].contiguous(), w[at: at + 16384].contiguous(), 8, SWIGLU, 256).reshape(-1)[: 8 * 8192].view(8, 8192) for at in range(0, 131072, 16384)], 1)
     assert torch.equal(many.isnan(), few.isnan())
     assert bool(((many.view(torch.int16) == few.view(torch.int16)) | many.isnan()).all())
+
+
+@pytest.mark.parametrize("groups", [2047, 2048, 2049])
+def test_many_segments_of_few_rows(lib, groups):
+    """More segments than rows, up to the number that the launch takes and one more (which goes to the one-CTA kernel)."""
+    gen = torch.Generator(device="cuda").manual_seed(groups)
+    rows, N, K = 45, 72, 64
+    owner = torch.sort(torch.randint(0, groups, (rows,), generator=gen, device="cuda")).values
+    owner[-1] = groups - 1
+    seg = torch.zeros(groups + 1, device="cuda", dtype=torch.int64)
+    seg[1:] = torch.bincount(owner, minlength=groups).cumsum(0)
+    seg = seg.int()
+    x = torch.randn(rows, K, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(groups, N, K, generator=gen, device="cuda") * K ** -0.5).bfloat16()
+    y = torch.full((rows + 1, N), 7.0, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    lib.tgis_k_pair_fault(0)
+    assert lib.tgis_k_gemm_any(p(x), p(w), p(y), 1, 1, 0, rows, N, K, K, K, N, 1, 0, 0, 0, p(seg), groups, N * K, None, 1, 0, None, 0) == 0, lib.tgis_k_last_error()
+    assert lib.tgis_k_pair_fault(0) == (1 if groups <= 2048 else 0)
+    wd = w[owner].double()
+    want, slack = torch.einsum("rk,rnk->rn", x.double(), wd), torch.einsum("rk,rnk->rn", x.double().abs(), wd.abs()) * 12 * 2.0 ** -23
+    assert float(((y[:rows].double() - want).abs() - slack).max()) <= 0
+    assert bool((y[rows] == 7.0).all())
+
+
+def test_gathered_rows_without_room_go_to_the_one_cta_kernel(lib):
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    counts, N, K = [100, 0, 33, 7], 136, 128
+    rows, E = sum(counts), len(counts)
+    seg = torch.tensor([0] + counts, device="cuda").cumsum(0).int()
+    expert = torch.repeat_interleave(torch.arange(E, device="cuda"), torch.tensor(counts, device="cuda"))
+    x = torch.randn(rows // 2, K, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(E, N, K, generator=gen, device="cuda") * K ** -0.5).bfloat16()
+    order = torch.randperm(rows, generator=gen, device="cuda").int()
+    src = x[order.long() // 2].double()
+    want = torch.einsum("rk,rnk->rn", src, w[expert].double())
+    slack = torch.einsum("rk,rnk->rn", src.abs(), w[expert].double().abs()) * (K / 16 + 8) * 2.0 ** -23
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    try:
+        for room, pairs in ((-1, 1), (rows * K * 2, 1), (rows * K * 2 - 2, 0), (0, 0)):
+            lib.tgis_k_gemm_any_room(room)
+            y = torch.full((rows + 1, N), 7.0, device="cuda")
+            lib.tgis_k_pair_fault(0)
+            assert lib.tgis_k_gemm_any(p(x), p(w), p(y), 1, 1, 0, rows, N, K, K, K, N, 1, 0, 0, 0, p(seg), E, N * K, p(order), 2, 0, None, 0) == 0, lib.tgis_k_last_error()
+            assert lib.tgis_k_pair_fault(0) == pairs
+            assert float(((y[:rows].double() - want).abs() - slack).max()) <= 0
+            assert bool((y[rows] == 7.0).all())
+    finally:
+        lib.tgis_k_gemm_any_room(-1)

@@ -534,6 +534,11 @@ int tgis_k_sampler(const void* logits_dev, int32_t ld, int32_t vocab, const void
 }
 
 // ---- layer-list architectures ----------------------------------------------------------------------------------------
+static thread_local int64_t t_gather_room = -1;
+int tgis_k_gemm_any_room(int64_t bytes) {
+  t_gather_room = bytes;
+  return 0;
+}
 int tgis_k_gemm_any(const void* x, const void* w, void* y, int32_t x_dt, int32_t w_dt, int32_t y_dt, int32_t T, int32_t N,
                     int32_t K, int32_t ldx, int32_t ldw, int32_t ldy, int32_t batch, int64_t x_bs, int64_t w_bs, int64_t y_bs,
                     const int32_t* seg_off_dev, int32_t n_groups, int64_t w_gs, const int32_t* gather_dev, int32_t gather_div,
@@ -547,8 +552,9 @@ int tgis_k_gemm_any(const void* x, const void* w, void* y, int32_t x_dt, int32_t
   a.mode = mode; a.row_scale = row_scale; a.scale_ld = scale_ld;
   Tmp<bf16> ws;
   if (gather_dev != nullptr && x_dt == DT_BF16) {
-    KCK(ws.alloc((size_t)T * K));
-    a.gather_ws = ws.p; a.gather_ws_bytes = (size_t)T * K * sizeof(bf16);
+    a.gather_ws_bytes = t_gather_room >= 0 ? (size_t)t_gather_room : (size_t)T * K * sizeof(bf16);
+    KCK(ws.alloc(a.gather_ws_bytes / sizeof(bf16)));
+    a.gather_ws = ws.p;
   }
   KCK(gemm_any_launch(a, 0));
   return product_end();
