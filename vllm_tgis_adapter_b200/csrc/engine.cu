@@ -4081,8 +4081,8 @@ struct tgis_engine {
       return false;
     }
 
-    // LoRA: sequences that share an adapter sit next to each other in the step, so that lora.cu's 8-token tiles are
-    // same-adapter tiles (A / B rows read once per tile) instead of falling back to one pass per token.  Every kernel's
+    // LoRA: sequences that share an adapter sit next to each other in the step, so that most of lora.cu's 8-token tiles hold one
+    // adapter (A / B rows read once per tile) and need one pass, not one per adapter.  Every kernel's
     // result for a token is independent of its neighbours, and post-processing below walks the same order.
     if (max_loras > 0) {
       bool any_lora = false;

@@ -18,6 +18,9 @@ constexpr int GEMM_X_BOX_MANY = 32;
 // 128-row tiles than half the SMs (fewer are cut along k by the one-CTA kernel, which can also fuse the rotary embedding).
 // Microseconds with cold weights, one CTA -> pairs, at 64, 128 and 256 tokens: 28672 x 4096 (SwiGLU) 59 -> 61, 69 -> 63, 100 -> 69;
 // 128256 x 4096 183 -> 185, 196 -> 189, 257 -> 206; 10248 x 2048 21 -> 14, 28 -> 15, 43 -> 19.
+// The line looks at the rows alone, and between 65 and 256 tokens k decides too.  With fewer rows and little k pairs would be ahead
+// (256 tokens: 2048 x 2048 24 -> 12, 3072 x 1536 23 -> 11, 5632 x 2048 31 -> 17, 6144 x 4096 31 -> 21); where k is long they are
+// behind (4096 x 14336 42 -> 56, 2048 x 11264 29 -> 42).
 inline bool gemm_takes_pairs(int T, int N, int num_sms) { return T > 256 || (T > 64 && (N + 127) / 128 > num_sms / 2); }
 // rows of one box of the activation map: the token tile, or (pairs) small boxes, of which a tile takes as many as it has rows
 inline int gemm_x_box(int T, int N, int num_sms) { return gemm_takes_pairs(T, N, num_sms) ? GEMM_X_BOX_MANY : gemm_pick_bt(T); }
