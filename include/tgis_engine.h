@@ -2,7 +2,7 @@
  * tgis_engine.h — C ABI of libtgis_engine.so, the B200-native continuous-batching engine that replaces the
  * vLLM AsyncLLMEngine behind the TGIS gRPC adapter's generation path.
  *
- * Drop-in boundary (SURVEY.md §8b).  The reference has no FFI; its seam is the `EngineClient` object that
+ * Drop-in boundary.  The reference has no FFI; its seam is the `EngineClient` object that
  * `TextGenerationService` holds.  Each entry point below cites the reference call site it serves
  * (paths relative to /root/reference/src/vllm_tgis_adapter):
  *
@@ -48,10 +48,10 @@ typedef struct tgis_engine tgis_engine;
 
 /* Architectures (tgis_config.arch).  The reference names a model by --model-name (tgis_utils/args.py:104,185-186) and lets
  * vLLM pick the architecture from the checkpoint's config.json; the host-side loader does the same and passes it here.
- *   LLAMA: RMSNorm, neox RoPE, GQA, SwiGLU, no biases (BASELINE configs[1..4])
+ *   LLAMA: RMSNorm, neox RoPE, GQA, SwiGLU, no biases
  *   OPT:   learned positions (offset 2), LayerNorm with bias, biased q/k/v/out/fc1/fc2, ReLU, tied lm_head,
  *          do_layer_norm_before = true, word_embed_proj_dim == hidden -- facebook/opt-125m, the reference's own test
- *          model (/root/reference/tests/conftest.py:79-91 (no --model: vLLM's default, facebook/opt-125m) and tests/test_hub.py:17).  64-dim heads (head_dim = 64) run on the
+ *          model (tests/conftest.py:79-91 (no --model: vLLM's default, facebook/opt-125m) and tests/test_hub.py:17).  64-dim heads (head_dim = 64) run on the
  *          128-dim attention tiles: the engine zero-pads every head's q/k/v rows and out_proj columns at load time, which
  *          leaves every dot product unchanged.  Single GPU, no LoRA slots. */
 #define TGIS_ARCH_LLAMA 0

@@ -8,7 +8,7 @@ Sources of truth exercised here:
     apply_top_k_top_p, v1.sample.sampler.Sampler.gather_logprobs / compute_logprobs, v1.core.sched.utils.check_stop
     semantics
   * transformers 5.5.0 LlamaForCausalLM (fp32, eager attention) for the model half
-The fixtures travel to the GPU box (which has no /root/reference); tests/test_oracle_cpu.py pins oracle/ against them.
+The fixtures are committed, so that no test needs the reference; tests/test_oracle_cpu.py pins oracle/ against them.
 """
 from __future__ import annotations
 

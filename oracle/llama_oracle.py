@@ -22,10 +22,9 @@ HF-format Llama checkpoint.  Restated here, with the file:line each step follows
                      the model dtype, i.e. the fp32 accumulator rounded ONCE to bf16; the sampler then casts to fp32
                      (v1/sample/sampler.py:91).  Exact ties between bf16 logits (thousands per 128k-vocab row) are
                      therefore part of the reference's behaviour: they inflate `rank` and decide greedy argmax by
-                     lowest token id.  (Round 1 kept fp32 logits here and in the engine; `logits_fp32=True` restores
-                     that for the experiment switch TGIS_LOGITS_FP32.)
+                     lowest token id.  (`logits_fp32=True` keeps fp32 logits, for the experiment switch TGIS_LOGITS_FP32.)
 
-PARITY PINNING: the reference's own tests hold no numeric golden vector for this path (SURVEY.md §8c: "parity
+PARITY PINNING: the reference's own tests hold no numeric golden vector for this path ("parity
 unpinned" for token ids / logprobs).  This oracle is therefore pinned against the third-party implementation it
 restates: tests/test_oracle_cpu.py checks it against transformers' LlamaForCausalLM (fp32, eager) on seeded weights and
 against the fixtures in tests/golden/ produced by oracle/gen_golden.py.
@@ -61,11 +60,11 @@ class LlamaConfig:
         return self.n_kv_heads * self.head_dim
 
 
-# Named shapes used across tests / bench (real architectures' dims; weights are synthetic, SURVEY.md §0)
+# Named shapes used across tests / bench (real architectures' dims; weights are synthetic)
 CONFIGS = {
     "tiny": LlamaConfig(n_layers=2, hidden=256, n_q_heads=4, n_kv_heads=2, ffn=512, vocab=1024, max_model_len=512),
     "small": LlamaConfig(n_layers=4, hidden=512, n_q_heads=4, n_kv_heads=1, ffn=1536, vocab=4096, max_model_len=1024),
-    # "opt-125m-size" Llama-class stand-in for BASELINE.json configs[0] (12 layers, hidden 768)
+    # "opt-125m-size" Llama-class stand-in (12 layers, hidden 768)
     "125m": LlamaConfig(n_layers=12, hidden=768, n_q_heads=6, n_kv_heads=2, ffn=3072, vocab=50272, max_model_len=2048),
     # small stack whose 8 kv heads / ffn / vocab split evenly over 2, 4 and 8 tensor-parallel ranks (scripts/tp_check.py)
     "tp8": LlamaConfig(n_layers=2, hidden=1024, n_q_heads=8, n_kv_heads=8, ffn=2048, vocab=8192, max_model_len=512),
@@ -78,7 +77,7 @@ CONFIGS = {
 
 def synthetic_weights(cfg: LlamaConfig, seed: int = 0, dtype: torch.dtype = torch.bfloat16, std: float = 0.02,
                       device: str = "cpu") -> dict[str, torch.Tensor]:
-    """HF-style N(0, 0.02) init, norms = 1 (SURVEY.md §7 'hard parts').  HF parameter names."""
+    """HF-style N(0, 0.02) init, norms = 1  HF parameter names."""
     g = torch.Generator(device=device).manual_seed(seed)
 
     def rnd(*shape: int) -> torch.Tensor:
@@ -141,7 +140,7 @@ class LlamaOracle:
     """Flat-batch Llama forward with the model-dtype rounding points of the vLLM/HF path.
 
     `device`: the same plain-torch restatement can be evaluated on a CUDA device (torch ops only) so that the -m gpu
-    parity tests can afford BASELINE shapes (8B dims, 32 x 512-token prompts); the default and every CPU test use "cpu"."""
+    parity tests can afford full shapes (8B dims, 32 x 512-token prompts); the default and every CPU test use "cpu"."""
 
     def __init__(self, cfg: LlamaConfig, weights: dict[str, torch.Tensor], dtype: torch.dtype = torch.bfloat16,
                  logits_fp32: bool = False, device: str = "cpu"):

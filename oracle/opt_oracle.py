@@ -1,5 +1,4 @@
-"""CPU oracle for the OPT model family ("OPT ... to serve the literal facebook/opt-125m of BASELINE
-configs[0]") — TEST INFRASTRUCTURE ONLY.
+"""CPU oracle for the OPT model family (facebook/opt-125m, the model of the reference's own tests) — TEST INFRASTRUCTURE ONLY.
 
 Only tests/, __graft_entry__.smoke() and bench.py's CPU legs may import this module; the product path never does.
 

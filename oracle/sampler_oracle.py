@@ -13,16 +13,16 @@ Restates, per request row and in fp32, what the reference stack does between the
   exponential race          vllm v1/sample/ops/topk_topp_sampler.py:395-416                               (S7)
   logprobs / rank / top-n   vllm v1/sample/sampler.py:79-88,300-351 ; v1/sample/ops/logprobs.py:10-27     (S1,S8)
 
-Processor order is the contract of SURVEY.md Appendix B (V0 ordering the adapter was written for):
+Processor order is the contract (V0 ordering the adapter was written for):
 raw log-softmax -> typical-p -> ExpDecay(EOS, no-op on a non-finite logit) -> min_tokens -> repetition penalty ->
 greedy argmax | temperature -> top-k -> top-p -> sample.
 
-PARITY PINNING: the reference's tests never exercise these processors (SURVEY.md §8c).  tests/golden/sampler_*.json
+PARITY PINNING: the reference's tests never exercise these processors.  tests/golden/sampler_*.json
 are generated by oracle/gen_golden.py by running the reference's OWN logits_processors.py (imported from
 /root/reference in the build container), transformers' TypicalLogitsWarper and vLLM 0.22's CPU sampler ops on seeded
 logits; tests/test_oracle_cpu.py checks this file against them.
 
-The random draw: torch's Philox stream cannot be reproduced by a custom kernel (SURVEY.md §8a S7), so the engine defines
+The random draw: torch's Philox stream cannot be reproduced by a custom kernel, so the engine defines
 its own counter-based generator (Philox4x32-10 keyed by the request seed, counter = (vocab index, output position)).
 `philox_uniform` restates it bit-exactly in numpy so that even sampled tokens can be compared.
 """
@@ -67,7 +67,7 @@ def typical_keep_mask(logits: torch.Tensor, mass: float) -> torch.Tensor:
 
 
 def exp_decay_length_penalty(logits: torch.Tensor, n_out: int, start: int, decay: float, eos: int) -> None:
-    """In place.  logits_processors.py:38-46, plus the no-op-on-non-finite rule of SURVEY.md §7."""
+    """In place.  logits_processors.py:38-46, plus the no-op-on-non-finite rule."""
     tokens_past = max(0, n_out - start)
     p_factor = pow(decay, tokens_past)          # python float (double)
     if p_factor != 1 and bool(torch.isfinite(logits[eos])):

@@ -1,4 +1,4 @@
-// Paged-KV attention for the TGIS hot path (SURVEY.md §2.2 K6/K7; reference call site: grpc_server.py:222 ->
+// Paged-KV attention for the TGIS hot path (reference call site: grpc_server.py:222 ->
 // vllm v1/attention/backends/flashinfer.py:1665,1803).  Causal, GQA, head_dim 128, bf16 in / fp32 softmax.
 //
 // HBM layout of the cache (ours to choose; see kernels.h): per (block, kv_head) one contiguous 8 KiB K tile stored
@@ -513,7 +513,7 @@ static cudaError_t decode_launch_g(const __nv_bfloat16* qkv, int qkv_ld, const _
   const long long max_flat = (long long)max_entries * n_kv;
   const int grid = (int)std::min<long long>((long long)TGIS_DEC_MINB * num_sms, (max_flat + DEC_WARPS - 1) / DEC_WARPS);
   // split merge: the PDL-chained attn_merge_kernel (default), or inside the streaming kernel by the last-arriving warp
-  // (TGIS_ATTN_INKERNEL_MERGE=1, bit-identical).  Measured (profiles/r02_step_timeline_*): folding the merge saves its
+  // (TGIS_ATTN_INKERNEL_MERGE=1, bit-identical).  Measured: folding the merge saves its
   // launch (-100 us per step at batch 32) but the o-proj GEMM that follows then loses the window in which it prefetched
   // its weights next to the small merge kernel (attention CTAs fill the SM's shared memory): +140 us on the GEMM, net
   // -1 % at batch 64.  So the separate kernel stays the default.

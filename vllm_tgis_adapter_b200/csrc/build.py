@@ -1,6 +1,6 @@
 """Build libtgis_engine.so in-tree with nvcc for sm_100a (no torch extension machinery, no JIT cache).
 
-The .so lands in vllm_tgis_adapter_b200/lib/ so it travels to the GPU box with the repo snapshot.
+The .so lands in vllm_tgis_adapter_b200/lib/ so it travels with the source tree.
 """
 from __future__ import annotations
 
@@ -22,7 +22,7 @@ NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-pthread",
-    # bounded mbarrier spins: a pipeline-protocol bug traps (sticky CUDA error) instead of hanging the GPU box
+    # bounded mbarrier spins: a pipeline-protocol bug traps (sticky CUDA error) instead of hanging the GPU
     "-DTGIS_MBAR_TIMEOUT=1",
 ]
 

@@ -2,7 +2,7 @@
 //
 // This is the B200-native replacement for what sits behind `self.engine.generate(...)`
 // (/root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py:222): vLLM's EngineCore busy loop, scheduler,
-// KV block manager, GPUModelRunner and Sampler (SURVEY.md §2.2 K1-K15, §3.2 "THE HOT LOOP").
+// KV block manager, GPUModelRunner and Sampler.
 //
 //   host side (this file, C++): request queues, paged-KV block allocator, continuous-batching scheduler with chunked
 //       prefill + recompute preemption, stop checks (vllm v1/core/sched/utils.py:94-130), output ring.
@@ -390,7 +390,7 @@ struct tgis_engine {
   // lm_head output [rows, V].  bf16 = the model dtype, rounded once from the fp32 accumulator exactly where vLLM's
   // lm_head rounds (vllm model_executor/layers/logits_processor.py:89-104 -> F.linear in bf16; the sampler then casts to
   // fp32, v1/sample/sampler.py:91): exact ties between bf16 logits, and the ranks / lowest-id argmax they cause, are
-  // reproduced.  TGIS_LOGITS_FP32=1 keeps the raw fp32 accumulator (round 1's behaviour; an experiment switch).
+  // reproduced.  TGIS_LOGITS_FP32=1 keeps the raw fp32 accumulator (an experiment switch).
   DevBuf<uint8_t> logits;
   bool logits_bf16 = true;
   size_t lsz = 2;  // bytes per logit
@@ -467,7 +467,7 @@ struct tgis_engine {
   bool tp_fused_ar = true;
   int tp_exchange_force = -1;                 // TGIS_TP_EXCHANGE
   size_t tp_oneshot_max_bytes = 2u << 20;     // TGIS_TP_ONESHOT_MAX_KB
-  bool tp_graphs = true;  // TGIS_TP_GRAPHS=0: tensor-parallel decode steps are launched kernel by kernel (round 1)
+  bool tp_graphs = true;  // TGIS_TP_GRAPHS=0: tensor-parallel decode steps are launched kernel by kernel
   static constexpr int AR_MAX_T = AR_MAX_ROWS;
   uint8_t* ar_mem = nullptr;        // [2 parities] receive areas (ar_recv_bytes each), then the two local partial buffers
   uint8_t* ar_peer[8] = {};         // the same allocation of every rank, mapped here (cudaIpc)

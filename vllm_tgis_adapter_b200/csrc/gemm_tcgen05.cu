@@ -2,7 +2,7 @@
 //
 // Replaces, for the decode/prefill hot path, what the reference reaches through
 //   vllm: model_executor/layers/linear.py (QKVParallelLinear / RowParallelLinear / MergedColumnParallelLinear
-//   -> F.linear -> cuBLAS)  behind grpc_server.py:222 `self.engine.generate(...)`   (SURVEY.md §2.2 K3/K8/K9/K10).
+//   -> F.linear -> cuBLAS)  behind grpc_server.py:222 `self.engine.generate(...)`.
 //
 // Design (B200-first, not a cuBLAS clone):
 //  * swap-AB: the WEIGHT tile [128 rows of N x 64 of K] is the MMA "A" operand (fills the 128 TMEM lanes), the
@@ -929,7 +929,7 @@ int gemm_pick_bt(int T) {
 
 // Weight tiles per unit (GemmCfg).  1 everywhere by default.  TGIS_GEMM_NW=2 makes decode-shaped launches share one
 // activation tile between two weight tiles (half the activation re-reads per weight byte): built, parity-green, and
-// MEASURED SLOWER (profiles/r02_gemm_nw_ab.log: gate_up 46 -> 55 us at T = 32, down 31 -> 50 us at T = 64, decode step
+// MEASURED SLOWER (gate_up 46 -> 55 us at T = 32, down 31 -> 50 us at T = 64, decode step
 // 3.93 -> 5.05 ms at batch 32): halving the tile count doubles the partial size of every split-K reduction and leaves 5
 // ring stages instead of 8, while the activation re-reads it removes were not what bounds these launches.
 int gemm_nw(int T) {
@@ -987,7 +987,7 @@ static int gemm_max_clusters(int s, int num_sms) {
   }
   return cache[s];
 }
-static bool gemm_fit_clusters() {  // TGIS_GEMM_FIT_CLUSTERS=0: round-1 policy (largest split, cluster mode only if it fits)
+static bool gemm_fit_clusters() {  // TGIS_GEMM_FIT_CLUSTERS=0: the plain policy (largest split, cluster mode only if it fits)
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("TGIS_GEMM_FIT_CLUSTERS");
@@ -1020,13 +1020,13 @@ int gemm_grid_size(int T, int N, int K, int num_sms) {
     // partial traffic than the extra SMs bring -- keep at least 16 k-blocks per CTA
     while (BT > 64 && split > 1 && KB / split < 16) --split;
     // Prefer a split whose clusters are all co-resident (qkv of the 8B model: 48 tiles x 3 CTAs -- only 45 clusters of 3
-    // fit, so round 1 reduced it through global memory; 48 clusters of 2 fit): the on-chip reduction spreads the fused
+    // fit, which would send it through global memory; 48 clusters of 2 fit): the on-chip reduction spreads the fused
     // RoPE + KV-scatter epilogue over the cluster's CTAs, which is what lets it replace rope_kvwrite_kernel above 32 tokens
     if (gemm_fit_clusters() && gemm_cluster_enabled() && t_tiles == 1)
       while (split > 2 && tiles > gemm_max_clusters(split, num_sms)) --split;
     grid = (int)(tiles * split);
   }
-  if (const char* e = getenv("TGIS_GEMM_MAX_CTAS")) {  // experiment knob (scripts/gemm_cta_sweep.py)
+  if (const char* e = getenv("TGIS_GEMM_MAX_CTAS")) {  // experiment knob
     const int cap = atoi(e);
     if (cap > 0 && grid > cap) grid = cap;
   }
@@ -1132,7 +1132,7 @@ static cudaError_t launch_bt(const CUtensorMap& wmap, const CUtensorMap& xmap, v
   }
   const int grid = gemm_grid_size(T, N, K, num_sms);
   // bit 0: weights are read once (evict-first); bit 1: stream-K share before the whole tiles (GemmSched::sk_first;
-  // TGIS_GEMM_SK_FIRST=0: pure stream-K as in round 1).  The fused-norm consumer's transform warps assume the pure cut.
+  // TGIS_GEMM_SK_FIRST=0: pure stream-K).  The fused-norm consumer's transform warps assume the pure cut.
   // Token tiles above 64 rows keep the pure cut: there the whole tile's direct epilogue (128+ tokens through the TMEM
   // loads) is a longer tail than the fix-up it replaces (measured: batch 128 +1.2 %, batch 32 / 64 -2.3 / -1.2 %).
   static int sk_first_env = -1;

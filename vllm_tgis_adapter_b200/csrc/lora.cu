@@ -32,7 +32,7 @@ namespace tgis {
 namespace {
 
 // 8 consecutive bf16 values as fp32 through ONE 16-byte load (an aggregate of eight __nv_bfloat16 read element-wise compiles
-// to eight 2-byte loads: the first version of these kernels ran 10x slower for exactly that reason, profiles/r02_ncu_lora.csv)
+// to eight 2-byte loads: the first version of these kernels ran 10x slower for exactly that reason)
 struct F8 {
   float v[8];
 };

@@ -1,4 +1,4 @@
-// Elementwise / row-reduction kernels of the OPT layer stack (SURVEY.md §8 f-4: the reference's own test model is
+// Elementwise / row-reduction kernels of the OPT layer stack (the reference's own test model is
 // facebook/opt-125m, /root/reference/tests/conftest.py:79-91 (no --model: vLLM's default, facebook/opt-125m) and tests/test_hub.py:17).  The GEMMs, the paged attention kernels, the lm_head and
 // the sampler are the Llama path's; what OPT adds is
 //   * learned position embeddings with offset 2                    vllm model_executor/models/opt.py:61-70, :268-290
@@ -32,7 +32,7 @@ __device__ __forceinline__ float wsum(float v) {
 // Row geometry by hidden size: THREADS threads x NVEC 16-byte vectors each.  The per-thread state (row values in fp32, the
 // affine parameters, the projection bias) lives in registers, so NVEC is as small as the row allows: the 8192-wide
 // instantiation needs 117 registers (2 CTAs of 256 threads per SM), the <= 2048-wide ones 40.  Measured on the first version
-// (one 256 x 4 instantiation for every width, profiles/r02_ncu_opt_v1.csv): a 2048-row prefill chunk of opt-125m
+// (one 256 x 4 instantiation for every width): a 2048-row prefill chunk of opt-125m
 // (hidden 768: 96 of 256 threads busy, seven waves of CTAs) took 17.3 us for 15.7 MB.
 template <int THREADS>
 __device__ __forceinline__ float bsum(float v, float* red) {

@@ -6,7 +6,7 @@
 //                       -> hf generation/logits_process.py:836-856
 //   vllm 0.22       : v1/sample/sampler.py:67-144 (raw log-softmax, min_tokens, penalties, greedy/temperature,
 //                     top-k/top-p, exponential-race sampling, gather_logprobs + rank)         (S1-S8)
-// Contract order per row (SURVEY.md Appendix B): raw log-softmax -> typical-p -> ExpDecay(EOS) -> min_tokens(EOS)
+// Contract order per row: raw log-softmax -> typical-p -> ExpDecay(EOS) -> min_tokens(EOS)
 // -> repetition penalty -> greedy argmax | temperature -> top-k -> top-p -> sample -> logprob / rank / top-n (raw).
 //
 // Shape of the problem: a [rows, V=128256] scan with integer-ish selection work; a sampling row needs ~10 passes of
@@ -919,7 +919,7 @@ int sampler_cluster_size(int n_rows, int any_complex, int num_sms) {
     if (v == 1 || v == 2 || v == 4 || v == 8) return v;
   }
   // one wave of clusters over the GPU: the largest power of two with n_rows * ncl <= #SMs.  Measured for sampling rows too
-  // (profiles/r02_sampler_bench.json: 64 configs[2] rows 403 us with 8 CTAs per row = 4 waves of resident clusters, 256 us
+  // (64 rows with typical-p and penalties 403 us with 8 CTAs per row = 4 waves of resident clusters, 256 us
   // with 2; 32 rows 241 vs 137 us with 4), so the rule does not depend on the row type any more.
   (void)any_complex;
   int ncl = 8;

@@ -1,7 +1,7 @@
 """`EngineClient`-shaped façade over the native engine: the object the TGIS gRPC servicer holds where the reference
 holds vLLM's AsyncLLM (/root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py:166-176).
 
-Members implemented = exactly the ones the reference touches (SURVEY.md §8b table): generate / abort / get_tokenizer /
+Members implemented = exactly the ones the reference touches: generate / abort / get_tokenizer /
 is_tracing_enabled / errored / is_running / vllm_config.model_config.max_model_len / get_model_config.
 
 Threading: the C++ engine runs its own step-loop thread; one Python poller thread blocks in `tgis_engine_poll`
@@ -52,7 +52,7 @@ class AsyncTGISEngine:
         # DELTA (GenerateStream) outputs of several engine steps merge into one RequestOutput when the consumer is behind,
         # as vLLM's RequestOutputCollector does (vllm v1/engine/output_processor.py `put`: aggregate when the previous output
         # has not been taken).  The per-message cost of grpc.aio (~60 us) caps the host stack near 14 k streamed messages/s
-        # (scripts/host_stack_bench.py, DESIGN.md section 3.6); merging lifts the cap exactly when it binds.
+        # (scripts/host_stack_bench.py); merging lifts the cap exactly when it binds.
         #   coalesce_streams / TGIS_STREAM_COALESCE = None / "auto" (default): merge only while at least
         #       TGIS_STREAM_COALESCE_MIN_STREAMS (64) requests are in flight -- below that the engine's decode rate is under
         #       the host's ceiling, and a lightly loaded server keeps sending exactly one message per token, which the

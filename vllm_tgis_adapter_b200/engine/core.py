@@ -46,12 +46,12 @@ class ModelConfig:
 LAYER_LIST_ARCHS = ("ponenex", "falerax", "revepel", "sikazen", "bisuzen", "ludelix")   # created with tgis_engine_create_spec; bfloat16 or float32
 
 
-# Named architectures (real dims; this offline build runs them on synthetic weights — SURVEY.md §0)
+# Named architectures (real dims; this offline build runs them on synthetic weights)
 PRESETS: dict[str, ModelConfig] = {
     "tiny": ModelConfig(n_layers=2, hidden=256, n_q_heads=4, n_kv_heads=2, ffn=512, vocab=1024, max_model_len=512),
     "small": ModelConfig(n_layers=4, hidden=512, n_q_heads=4, n_kv_heads=1, ffn=1536, vocab=4096, max_model_len=1024),
     "125m": ModelConfig(n_layers=12, hidden=768, n_q_heads=6, n_kv_heads=2, ffn=3072, vocab=50272, max_model_len=2048),
-    # facebook/opt-125m (the reference's own test model; BASELINE configs[0]) and a CPU-oracle-sized sibling
+    # facebook/opt-125m (the reference's own test model) and a CPU-oracle-sized sibling
     "opt-125m": ModelConfig(n_layers=12, hidden=768, n_q_heads=12, n_kv_heads=12, ffn=3072, vocab=50272, head_dim=64,
                             max_model_len=2048, arch="opt"),
     "opt-tiny": ModelConfig(n_layers=2, hidden=256, n_q_heads=4, n_kv_heads=4, ffn=1024, vocab=1024, head_dim=64,

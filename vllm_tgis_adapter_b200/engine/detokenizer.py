@@ -1,5 +1,4 @@
-"""Incremental detokenisation + stop-string matching, host side (needs the HF tokenizer, so it stays in Python;
-SURVEY.md §8b).  Semantics restated from vLLM 0.22 (what the reference gets behind `engine.generate`):
+"""Incremental detokenisation + stop-string matching, host side (needs the HF tokenizer, so it stays in Python).  Semantics restated from vLLM 0.22 (what the reference gets behind `engine.generate`):
 
   update / get_next_output_text   vllm v1/engine/detokenizer.py:95-165
   check_stop_strings              vllm v1/engine/detokenizer.py:309-344

@@ -2,7 +2,7 @@
 (/root/reference/src/vllm_tgis_adapter/__main__.py:48): read the HF model directory (config.json + *.safetensors),
 stream each tensor into libtgis_engine.so ("PyTorch tensors for weights only"), attach a tokenizer.
 
-Offline builds have no checkpoints (SURVEY.md §0): `--model <preset> --synthetic-weights` creates seeded N(0, 0.02)
+Offline builds have no checkpoints: `--model <preset> --synthetic-weights` creates seeded N(0, 0.02)
 weights of the named architecture on the device instead."""
 from __future__ import annotations
 

@@ -1,9 +1,9 @@
 """Tokenizers for the server: a HF tokenizer directory when one exists, otherwise the synthetic WordLevel tokenizer
-that the offline build uses everywhere (no tokenizer files exist in this environment; SURVEY.md §0/§8c).
+that the offline build uses everywhere (no tokenizer files exist in this environment).
 
 Synthetic vocabulary: id 0 `<unk>`, 1 `<s>`, 2 `</s>`, id n>=3 -> word `t{n}`; whitespace pre-tokenisation, so a prompt
 of 512 whitespace-separated words is exactly 512 ids and `Tokenize` offsets are exact.  truncation_side is "left" like
-vLLM's generate-runner tokenizers (vllm tokenizers/registry.py:143-147; SURVEY Appendix B)."""
+vLLM's generate-runner tokenizers (vllm tokenizers/registry.py:143-147)."""
 from __future__ import annotations
 
 import functools

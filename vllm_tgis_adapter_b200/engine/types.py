@@ -1,4 +1,4 @@
-"""Value types crossing the drop-in boundary (SURVEY.md §8b): the subset of vLLM's SamplingParams / RequestOutput /
+"""Value types crossing the drop-in boundary: the subset of vLLM's SamplingParams / RequestOutput /
 CompletionOutput / Logprob that /root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py actually touches
 (:205-225 generate kwargs, :282-283,298,374,438-456 RequestOutput, :391-392,477-487,670-690 CompletionOutput,
 :727-755 Logprob).  Same attribute names so the adapter code reads identically."""
@@ -38,7 +38,7 @@ class StructuredOutputsParams:
 
 @dataclasses.dataclass
 class SamplingParams:
-    """Field names follow vllm/sampling_params.py; normalisation rules follow :398-440 (SURVEY Appendix B)."""
+    """Field names follow vllm/sampling_params.py; normalisation rules follow :398-440."""
 
     temperature: float = 1.0
     top_k: int = -1

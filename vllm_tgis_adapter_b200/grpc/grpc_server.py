@@ -3,8 +3,8 @@
 Behavioural mirror of /root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py (same RPC surface, same parameter
 mapping, same stop-reason / token-info conversion, same error strings and status codes) with the engine call
 `self.engine.generate(...)` (:222) landing in libtgis_engine.so instead of vLLM.  Each method cites the reference
-lines whose behaviour it reproduces.  Differences, all deliberate and documented in DESIGN.md:
-  * `max_tokens` is computed per request instead of mutating the shared SamplingParams (:792-797; SURVEY §3.2 note);
+lines whose behaviour it reproduces.  Differences, all deliberate:
+  * `max_tokens` is computed per request instead of mutating the shared SamplingParams (:792-797);
   * the two per-request logits processors (:560-578) travel as data (typical_p / length_penalty) into the fused
     sampling kernel instead of Python callables;
   * guided decoding (:580-586, tgis_utils/structured_outputs.py:14-38): the `guided` oneof becomes a
@@ -425,7 +425,7 @@ class TextGenerationService:
         tokenizer = await self.engine.get_tokenizer()
         responses = []
         for req in request.requests:
-            # transformers 5 dropped encode_plus; __call__ is the same code path (SURVEY Appendix B)
+            # transformers 5 dropped encode_plus; __call__ is the same code path
             enc = tokenizer(req.text, return_offsets_mapping=request.return_offsets,
                             add_special_tokens=ADD_SPECIAL_TOKENS)
             token_ids = enc.input_ids

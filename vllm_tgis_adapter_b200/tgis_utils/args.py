@@ -2,7 +2,7 @@
 
 Behavioural mirror of /root/reference/src/vllm_tgis_adapter/tgis_utils/args.py (env fallback :30-98, TGIS flags
 :101-181, legacy->native translation :184-258) on plain argparse: vLLM's FlexibleArgumentParser and its ~200 engine
-flags have no meaning for this engine, so only the flags the serving path needs exist (SURVEY.md §2.1 #10)."""
+flags have no meaning for this engine, so only the flags the serving path needs exist."""
 from __future__ import annotations
 
 import argparse
