@@ -73,7 +73,7 @@ launch_list(SRC / "launches.csv", DST / f"{tag}_launches_decode_step_summary.csv
 ncu_raw(SRC / "prof_gemm.ncu-rep", DST / f"{tag}_ncu_full_gemm_tcgen05.csv")
 ncu_raw(SRC / "prof_attn.ncu-rep", DST / f"{tag}_ncu_full_attn_decode.csv")
 ncu_raw(SRC / "prof_gemm_prefill.ncu-rep", DST / f"{tag}_ncu_full_gemm_prefill.csv")
-for name in ("bench.log", "bench_ref.log", "parity_stats.json", "gemm_bench.json", "gemm_cta_sweep.json", "gemm_timeline.log",
+for name in ("bench.log", "bench_ref.log", "parity_stats.json", "gemm_bench.json", "gemm_timeline.log",
              "gpu_info.txt", "tp2.log", "bench_tp2.log", "bench_tp4.log", "bench_dp2.log", "attn_bench.json", "grpc_bench.log",
              "bench_b64.log", "bench_b128.log", "bench_b256.log", "bench_b64_cfg3.log"):
     p = SRC / name
