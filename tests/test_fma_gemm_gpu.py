@@ -98,3 +98,13 @@ def test_a_row_is_the_same_in_every_tile_height(lib, K):
     whole = run(x)   # 450 tiles of 64 rows where K > 256
     assert torch.equal(run(x[40:100].contiguous()), whole[40:100])   # 32
     assert torch.equal(run(x[90:99].contiguous()), whole[90:99])     # 16
+
+
+def test_rows_beyond_the_tiles_of_32_that_one_launch_holds(lib):
+    T, N, K = 65535 * 32 + 33, 3, 5
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    x, w = torch.randn(T, K, generator=gen, device="cuda"), torch.randn(N, K, generator=gen, device="cuda")
+    y = torch.full((T + 1, N), 7.0, device="cuda")
+    assert lib.tgis_k_gemm_any(p(x), p(w), p(y), 0, 0, 0, T, N, K, K, K, N, 1, 0, 0, 0, None, 0, 0, None, 1, 0, None, 0) == 0
+    assert float(((y[:T].double() - x.double() @ w.double().T).abs() - bound(x, w, K)).max()) <= 0
+    assert bool((y[T] == 7.0).all())

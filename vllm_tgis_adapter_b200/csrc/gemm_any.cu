@@ -499,7 +499,8 @@ cudaError_t launch_fma(const GemmAny& a, cudaStream_t stream) {
   const long long tiles64 = (long long)((a.N + FMA_BN - 1) / FMA_BN) * (a.batch > 0 ? a.batch : 1) *
                             (a.seg_off != nullptr ? (long long)a.n_groups * ((rows + 63) / 64) : (a.T + 63) / 64);
   if (rows <= 20) return launch_fma_bm<XT, WT, OT, 16>(a, vec, stream);
-  if (rows <= 36 || tiles64 < 3 * FMA_SMS || a.K <= 256) return launch_fma_bm<XT, WT, OT, 32>(a, vec, stream);
+  const bool fit32 = (a.T + 31ll) / 32 + (a.seg_off != nullptr ? a.n_groups : 0) <= 65535;   // tiles of one launch (grid.y)
+  if (fit32 && (rows <= 36 || tiles64 < 3 * FMA_SMS || a.K <= 256)) return launch_fma_bm<XT, WT, OT, 32>(a, vec, stream);
   return launch_fma_bm<XT, WT, OT, 64>(a, vec, stream);
 }
 
