@@ -100,3 +100,23 @@ def test_decayed_memory_carried_on(d, H, T):
         assert ((out[t].cpu().to(F64).reshape(H, d) - o).abs() <= (c + (d + 4) * 2.0 ** -24) * size).all()
         S1, Sa = w[t, :, :, None] * S1 + kv, w[t, :, :, None] * Sa + kv.abs()
     assert ((Sg[0].cpu().to(F64) - S1).abs() <= c * Sa + 1e-30).all()
+
+
+def test_gated_memory_in_a_slot_of_any_number():
+    """The hook's own counters reach as far as the slots it is given."""
+    from vllm_tgis_adapter_b200.engine._lib import load_library
+
+    lib, d, dv, slot, T = load_library(), 8, 40, 5000, 19
+    g = torch.Generator().manual_seed(5)
+    width = 2 * d + dv + 2
+    y, bias = torch.randn(T, width, generator=g).cuda(), torch.zeros(1, device="cuda")
+    outs = []
+    for at in (0, slot):
+        S, n, m = (torch.zeros(slot + 1, *shape, device="cuda") for shape in ((d, dv), (d,), ()))
+        out, tok_slot = torch.full((T, dv), float("nan"), device="cuda"), torch.full((T,), at, dtype=torch.int32, device="cuda")
+        assert lib.tgis_k_outer_scan(1, _p(y), _p(y[:, d:]), _p(y[:, 2 * d:]), width, width, width, ctypes.c_float(1.0), None, 0, None, None,
+                                     _p(y[:, width - 2:]), _p(y[:, width - 1:]), width, _p(bias), _p(bias), ctypes.c_float(6.0), _p(S), _p(n), _p(m), _p(out), dv, 1, d, dv,
+                                     None, None, 0, (ctypes.c_int32 * 4)(0, T, T, 0), 1, _p(tok_slot)) == 0
+        outs += [out, S[at].clone(), n[at].clone(), m[at].clone()]
+        assert int(S[at].count_nonzero()) == int(S.count_nonzero()) > 0
+    assert all(torch.equal(a, b) for a, b in zip(outs[:4], outs[4:])) and bool(outs[0].isfinite().all())

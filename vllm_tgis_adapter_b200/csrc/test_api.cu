@@ -876,8 +876,16 @@ int tgis_k_outer_scan(int32_t mode, const float* q, const float* k, const float*
   a.S = S; a.n = n; a.m = m; a.out = out; a.ldo = ldo; a.heads = heads; a.dim = dim; a.vdim = vdim;
   a.x = x; a.x_last = x_last; a.width = width;
   Tmp<int32_t> done;
-  if (mode == OUTER_SCAN_GATED) {   // zeros for every slot the launch may name
-    KCK(done.upload(std::vector<int32_t>((size_t)heads * 4096, 0).data(), (size_t)heads * 4096));
+  if (mode == OUTER_SCAN_GATED) {   // zeros for every slot that the launch names
+    int32_t slots = 0;
+    for (const AttnSeq& s : seqs) {
+      int32_t slot = 0;
+      KCK(cudaMemcpy(&slot, tok_slot + s.q_start, sizeof(slot), cudaMemcpyDeviceToHost));
+      if (slot < 0) return kfail("a sequence without a slot");
+      slots = std::max(slots, slot + 1);
+    }
+    KCK(done.alloc((size_t)heads * slots));
+    KCK(cudaMemset(done.p, 0, (size_t)heads * slots * sizeof(int32_t)));
     a.done = done.p;
   }
   KCK(outer_scan_launch(a, d_seqs.p, n_seqs, tok_slot, 0));
