@@ -1,0 +1,86 @@
+"""Attention of prompts on tcgen05 (csrc/attention_prefill.cu) where its tiles end: query tokens around the rows of one and of two
+accumulators (128 / G and twice that), contexts around the 32-token blocks and the 128-token tiles, every group size -- against a
+softmax in 64 bits over the same bf16 operands; and the bits of a row, which depend on its own keys alone."""
+import ctypes as C
+import math
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def g():
+    from tests import tgis_gpu_utils
+
+    return tgis_gpu_utils
+
+
+class Case:
+    def __init__(self, g, n_q, n_kv, kv_lens, seed, size=1.0):
+        gen = torch.Generator(device="cuda").manual_seed(seed)
+        self.g, self.n_q, self.n_kv, self.kv_lens = g, n_q, n_kv, kv_lens
+        blocks = [-(-n // 32) for n in kv_lens]
+        order = np.random.RandomState(seed).permutation(sum(blocks)).astype(np.int32)   # scattered physical blocks
+        self.bt = np.zeros((len(kv_lens), max(blocks)), dtype=np.int32)
+        rows = sum(blocks) * 32
+        self.k, self.v = ((torch.randn(rows, n_kv, 128, device="cuda", generator=gen)).bfloat16() for _ in range(2))
+        self.q = [(torch.randn(n, n_q, 128, device="cuda", generator=gen) * size).bfloat16() for n in kv_lens]
+        self.slots, at = [], 0
+        for i, (n, b) in enumerate(zip(kv_lens, blocks)):
+            self.bt[i, :b] = order[at: at + b]
+            at += b
+            self.slots.append(torch.tensor(np.concatenate([np.arange(32) + 32 * x for x in self.bt[i, :b]])[:n], device="cuda"))
+        self.kc, self.vc = g.k_cache_from_dense(self.k, sum(blocks)), g.v_cache_from_dense(self.v, sum(blocks))
+
+    def run(self, parts, scale=128 ** -0.5):
+        """parts: (sequence, first query position, one past the last); the outputs of one launch, in order"""
+        seqs, at, rows = [], 0, []
+        for s, a, b in parts:
+            seqs.append((at, b - a, b, s))
+            rows.append(self.q[s][a:b])
+            at += b - a
+        qkv = torch.zeros(at, self.n_q + 2 * self.n_kv, 128, dtype=torch.bfloat16, device="cuda")
+        qkv[:, : self.n_q] = torch.cat(rows)
+        out = torch.full((at, self.n_q, 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+        sq, bt, g = np.array(seqs, dtype=np.int32), self.bt, self.g
+        rc = g.lib().tgis_k_attention(g.ptr(qkv), g.ptr(self.kc), g.ptr(self.vc), g.i32p(sq.reshape(-1)), len(parts), g.i32p(bt.reshape(-1)),
+                                      bt.shape[0], bt.shape[1], g.ptr(out), self.n_q, self.n_kv, C.c_float(scale))
+        assert rc == 0, g.kerr()
+        return list(out.split([b - a for _, a, b in parts]))
+
+    def exact(self, s, a, b, scale=128 ** -0.5):
+        k, v = (t[self.slots[s][:b]].double().repeat_interleave(self.n_q // self.n_kv, 1) for t in (self.k, self.v))
+        x = torch.einsum("qhd,khd->hqk", self.q[s][a:b].double(), k) * scale
+        x = x.masked_fill(torch.arange(b, device="cuda")[None] > torch.arange(a, b, device="cuda")[:, None], -math.inf)
+        return torch.einsum("hqk,khd->qhd", torch.softmax(x, -1), v)
+
+
+@pytest.mark.parametrize("size,scale", [(1.0, 128 ** -0.5), (6.0, 128 ** -0.5), (1.0, -0.05)])
+@pytest.mark.parametrize("n_q,n_kv", [(8, 2), (8, 1), (2, 2), (6, 2), (5, 1), (7, 1), (4, 2)])
+def test_tile_edges_match_a_softmax_in_64_bits(g, n_q, n_kv, size, scale):
+    tm = 128 * n_kv // n_q // 8 * 8   # query tokens of one accumulator
+    parts = [(c, c + q) for c in (0, 31, 97, 128) for q in (2, tm - 1, tm, tm + 1, 2 * tm, 2 * tm + 3)]
+    parts += [(0, 127), (0, 128), (0, 129), (0, 257), (300, 384), (511, 641)]
+    case = Case(g, n_q, n_kv, [b for _, b in parts], seed=n_q * 10 + n_kv, size=size)
+    out = case.run([(s, a, b) for s, (a, b) in enumerate(parts)], scale)
+    for s, (a, b) in enumerate(parts):
+        want = case.exact(s, a, b, scale)
+        # the result's rounding to 8 bits (half a unit in the last place: at most 2^-8 of it); the probabilities' 16 bits (2^-16 of a
+        # sum of |v| <= 5); scores of up to 100, summed in fp32 (128 terms: 2^-19 of them, which e^x hands on)
+        bound = 1.001 * 2 ** -8 * want.abs() + 5 * (2 ** -16 + 100 * 2 ** -19)
+        off = (out[s].double() - want).abs() - bound
+        assert float(off.max()) <= 0.0, (s, a, b, float(off.max()))
+
+
+@pytest.mark.parametrize("n_q,n_kv", [(8, 2), (6, 2), (2, 2)])
+def test_a_row_has_the_same_bits_whole_in_portions_and_beside_others(g, n_q, n_kv):
+    case = Case(g, n_q, n_kv, [700, 45, 333], seed=3, size=4.0)   # large scores: the running maximum moves often
+    whole = case.run([(0, 0, 700)])[0]
+    beside = case.run([(1, 0, 45), (0, 0, 700), (2, 100, 333)])[1]
+    assert torch.equal(whole, beside)
+    cuts = [0, 2, 33, 64, 200, 511, 513, 700]
+    portions = torch.cat([case.run([(2, 0, 9), (0, a, b)])[1] for a, b in zip(cuts, cuts[1:])])
+    assert torch.equal(whole, portions)

@@ -4,15 +4,12 @@
 // HBM layout of the cache (ours to choose; see kernels.h): per (block, kv_head) one contiguous 8 KiB K tile stored
 // "8-dim chunk major" [16][32 tok][8] and one 8 KiB V tile [32 tok][16 chunks ^ (tok&7)][8].  Both tiles are fetched
 // with ONE 1-D TMA bulk copy each (cp.async.bulk -> UBLKCP) completing on an mbarrier, and both are bank-conflict
-// free for the two consumers below without any in-kernel transposition:
-//   decode : QK^T with lane = token (16-B LDS per 8-dim chunk), PV with lane = 4 dims (8-B LDS per token)
-//   prefill: QK^T B-fragments are plain 4-B LDS, PV B-fragments are ldmatrix.trans rows spread over 8 bank groups
+// free here without any in-kernel transposition (and are operands of the tensor cores as they stand: attention_prefill.cu).
 //
 // decode  (q_len = 1): grid (seq x split, kv_head); split-KV in fixed 128-token chunks (batch-invariant numerics);
 //                      one warp per 32-token block; the G = n_q/n_kv query heads of the group share every K/V byte;
 //                      last-arriving split combines partials in split order (deterministic).
-// prefill (q_len >= 1): grid (16-query tile, kv_head); one warp per query head of the group; mma.sync m16n8k16 with
-//                      online softmax; KV blocks double-buffered through smem by TMA bulk copies.
+// Prompts and their portions (q_len > 1): attention_prefill.cu.
 #include <algorithm>
 
 #include "kernels.h"
@@ -550,188 +547,6 @@ cudaError_t attn_decode_launch(const __nv_bfloat16* qkv, int qkv_ld, const __nv_
     default: return cudaErrorInvalidValue;
   }
 #undef TGIS_DEC
-}
-
-// ================================================================================================ prefill
-constexpr int PF_QROWS = 16;  // query tokens per tile
-
-// grid (n_tiles, n_kv); blockDim = 32 * G (warp = query head inside the GQA group)
-__global__ void __launch_bounds__(256)
-attn_prefill_kernel(const __nv_bfloat16* __restrict__ qkv, int qkv_ld, const __nv_bfloat16* __restrict__ k_cache,
-                    const __nv_bfloat16* __restrict__ v_cache, const AttnSeq* __restrict__ seqs,
-                    const int32_t* __restrict__ tile_seq, const int32_t* __restrict__ tile_q0,
-                    const int32_t* __restrict__ block_table, int bt_stride, __nv_bfloat16* __restrict__ out,
-                    int out_ld, int n_kv, int G, float scale) {
-  __shared__ __align__(128) uint8_t kv_s[2 * 2 * TILE_BYTES];  // 2 stages x (K | V)
-  __shared__ uint64_t bars[2];
-  griddep_launch();
-  griddep_wait();
-  const int tile = blockIdx.x, kvh = blockIdx.y;
-  const AttnSeq sq = seqs[tile_seq[tile]];
-  const int q0 = tile_q0[tile];                      // first query (index within this step's q_len)
-  const int n_rows = min(PF_QROWS, sq.q_len - q0);   // valid query rows in the tile
-  const int pos0 = sq.kv_len - sq.q_len + q0;        // absolute position of row 0
-  const int last_pos = pos0 + n_rows - 1;
-  const int n_blk = last_pos / KV_BLOCK + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int g = lane >> 2, t = lane & 3;
-  const int head = kvh * G + warp;
-
-  if (threadIdx.x == 0) {
-    mbar_init(&bars[0], 1);
-    mbar_init(&bars[1], 1);
-    fence_barrier_init();
-  }
-  __syncthreads();
-  const int32_t* bt = block_table + (size_t)sq.block_row * bt_stride;
-  auto issue = [&](int j) {
-    const int st = j & 1;
-    const size_t tl = ((size_t)bt[j] * n_kv + kvh) * (KV_BLOCK * HEAD_DIM);
-    mbar_arrive_expect_tx(&bars[st], 2 * TILE_BYTES);
-    bulk_load_1d(kv_s + st * 2 * TILE_BYTES, k_cache + tl, TILE_BYTES, &bars[st]);
-    bulk_load_1d(kv_s + st * 2 * TILE_BYTES + TILE_BYTES, v_cache + tl, TILE_BYTES, &bars[st]);
-  };
-  if (threadIdx.x == 0) {
-    issue(0);
-    if (n_blk > 1) issue(1);
-  }
-
-  // Q fragments (A operand), rows g and g+8 of the tile; rows past n_rows are clamped (results discarded)
-  uint32_t qa[8][4];
-  {
-    const int r0 = min(g, n_rows - 1), r1 = min(g + 8, n_rows - 1);
-    const __nv_bfloat16* q_r0 = qkv + (size_t)(sq.q_start + q0 + r0) * qkv_ld + (size_t)head * HEAD_DIM;
-    const __nv_bfloat16* q_r1 = qkv + (size_t)(sq.q_start + q0 + r1) * qkv_ld + (size_t)head * HEAD_DIM;
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      qa[ks][0] = *reinterpret_cast<const uint32_t*>(q_r0 + ks * 16 + t * 2);
-      qa[ks][1] = *reinterpret_cast<const uint32_t*>(q_r1 + ks * 16 + t * 2);
-      qa[ks][2] = *reinterpret_cast<const uint32_t*>(q_r0 + ks * 16 + 8 + t * 2);
-      qa[ks][3] = *reinterpret_cast<const uint32_t*>(q_r1 + ks * 16 + 8 + t * 2);
-    }
-  }
-  float o[16][4];
-#pragma unroll
-  for (int i = 0; i < 16; ++i)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
-  float m_r[2] = {-INFINITY, -INFINITY}, l_r[2] = {0.f, 0.f};
-  const float sl2 = scale * 1.4426950408889634f;  // exp2 domain
-  const int row_pos[2] = {pos0 + g, pos0 + g + 8};
-
-  for (int j = 0; j < n_blk; ++j) {
-    const int st = j & 1;
-    mbar_wait(&bars[st], (j >> 1) & 1);
-    const uint8_t* k_t = kv_s + st * 2 * TILE_BYTES;
-    const uint8_t* v_t = k_t + TILE_BYTES;
-    // ---- S = Q K^T : 4 n-tiles (8 tokens each) x 8 k-steps
-    float s[4][4];
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        const int tok = nt * 8 + g;
-        const uint32_t b0 = *reinterpret_cast<const uint32_t*>(k_t + ((2 * ks) * KV_BLOCK + tok) * 16 + t * 4);
-        const uint32_t b1 = *reinterpret_cast<const uint32_t*>(k_t + ((2 * ks + 1) * KV_BLOCK + tok) * 16 + t * 4);
-        mma_bf16_16816(s[nt], qa[ks], b0, b1);
-      }
-    }
-    // ---- causal mask + online softmax (rows g, g+8; cols nt*8 + t*2 + {0,1})
-    float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int kpos = j * KV_BLOCK + nt * 8 + t * 2 + (e & 1);
-        const int r = e >> 1;
-        s[nt][e] = (kpos <= row_pos[r]) ? s[nt][e] * sl2 : -INFINITY;
-        mx[r] = fmaxf(mx[r], s[nt][e]);
-      }
-    float corr[2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-      const float m_new = fmaxf(m_r[r], mx[r]);
-      corr[r] = (m_r[r] == -INFINITY) ? 0.f : exp2f(m_r[r] - m_new);
-      m_r[r] = m_new;
-      l_r[r] *= corr[r];
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      o[i][0] *= corr[0]; o[i][1] *= corr[0]; o[i][2] *= corr[1]; o[i][3] *= corr[1];
-    }
-    // P is fed to the tensor cores as bf16 hi + bf16 lo (two MMAs): ~16 mantissa bits instead of 8, so the result
-    // tracks the fp32-softmax oracle instead of the usual flash-attention bf16-P rounding.
-    uint32_t pa[2][4], pl[2][4];
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      float p[4], q[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int r = e >> 1;
-        p[e] = (m_r[r] == -INFINITY) ? 0.f : exp2f(s[nt][e] - m_r[r]);
-        l_r[r] += p[e];
-        q[e] = p[e] - bf16_round(p[e]);
-      }
-      const int kk = nt >> 1, hi = nt & 1;
-      pa[kk][hi * 2 + 0] = pack_bf16x2(p[0], p[1]);
-      pa[kk][hi * 2 + 1] = pack_bf16x2(p[2], p[3]);
-      pl[kk][hi * 2 + 0] = pack_bf16x2(q[0], q[1]);
-      pl[kk][hi * 2 + 1] = pack_bf16x2(q[2], q[3]);
-    }
-    // ---- O += P V : 2 k-steps (16 tokens) x 16 n-tiles (8 dims), V B-fragments by ldmatrix.trans
-    const uint32_t v_base = smem_u32(v_t);
-#pragma unroll
-    for (int kk = 0; kk < 2; ++kk) {
-#pragma unroll
-      for (int nd = 0; nd < 16; nd += 2) {
-        // lane -> (matrix = lane/8, row = lane%8): matrices (tok lo, nd), (tok hi, nd), (tok lo, nd+1), (tok hi, nd+1)
-        const int mi = lane >> 3, ri = lane & 7;
-        const int tok = kk * 16 + (mi & 1) * 8 + ri;
-        const int chunk = nd + (mi >> 1);
-        uint32_t vb[4];
-        ldmatrix_x4_trans(vb, v_base + tok * (HEAD_DIM * 2) + ((chunk ^ (tok & 7)) * 16));
-        mma_bf16_16816(o[nd], pa[kk], vb[0], vb[1]);
-        mma_bf16_16816(o[nd + 1], pa[kk], vb[2], vb[3]);
-        mma_bf16_16816(o[nd], pl[kk], vb[0], vb[1]);
-        mma_bf16_16816(o[nd + 1], pl[kk], vb[2], vb[3]);
-      }
-    }
-    __syncthreads();  // every warp is done with stage st
-    if (threadIdx.x == 0 && j + 2 < n_blk) issue(j + 2);
-  }
-  // ---- normalise and store
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    l_r[r] += __shfl_xor_sync(0xffffffffu, l_r[r], 1);
-    l_r[r] += __shfl_xor_sync(0xffffffffu, l_r[r], 2);
-  }
-#pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int row = g + r * 8;
-    if (row < n_rows) {
-      const float inv = 1.f / l_r[r];
-      __nv_bfloat16* dst = out + (size_t)(sq.q_start + q0 + row) * out_ld + (size_t)head * HEAD_DIM;
-#pragma unroll
-      for (int nd = 0; nd < 16; ++nd)
-        *reinterpret_cast<uint32_t*>(dst + nd * 8 + t * 2) = pack_bf16x2(o[nd][r * 2] * inv, o[nd][r * 2 + 1] * inv);
-    }
-  }
-}
-
-cudaError_t attn_prefill_launch(const __nv_bfloat16* qkv, int qkv_ld, const __nv_bfloat16* k_cache,
-                                const __nv_bfloat16* v_cache, const AttnSeq* seqs, const int32_t* tile_seq,
-                                const int32_t* tile_q0, int n_tiles, const int32_t* block_table, int bt_stride,
-                                __nv_bfloat16* out, int out_ld, int n_q, int n_kv, float scale, cudaStream_t stream) {
-  if (n_tiles <= 0) return cudaSuccess;
-  if (n_q % n_kv != 0) return cudaErrorInvalidValue;
-  const int G = n_q / n_kv;
-  if (G > 8) return cudaErrorInvalidValue;
-  dim3 grid(n_tiles, n_kv);
-  return launch_k(attn_prefill_kernel, grid, dim3(32 * G), 0, stream, qkv, qkv_ld, k_cache, v_cache, seqs, tile_seq,
-                  tile_q0, block_table, bt_stride, out, out_ld, n_kv, G, scale);
 }
 
 }  // namespace tgis

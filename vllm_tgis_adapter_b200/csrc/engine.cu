@@ -425,8 +425,8 @@ struct tgis_engine {
   // staging
   uint8_t* h_stage = nullptr;
   DevBuf<uint8_t> d_stage;
-  size_t off_tok = 0, off_pos = 0, off_slotmap = 0, off_tokslot = 0, off_seqs = 0, off_decids = 0, off_tileseq = 0,
-         off_tileq0 = 0, off_samplesrc = 0, off_rows = 0, off_epoch = 0, off_bt = 0, off_toklora = 0, stage_bytes = 0;
+  size_t off_tok = 0, off_pos = 0, off_slotmap = 0, off_tokslot = 0, off_seqs = 0, off_decids = 0, off_units = 0,
+         off_samplesrc = 0, off_rows = 0, off_epoch = 0, off_bt = 0, off_toklora = 0, stage_bytes = 0;
 
   // host state
   std::mutex mu;
@@ -749,8 +749,7 @@ struct tgis_engine {
     off_toklora = place(4 * (size_t)T_max);  // adapter slot of every token (0: base model)
     off_seqs = place(sizeof(AttnSeq) * (size_t)S_max);
     off_decids = place(4 * (size_t)S_max);
-    off_tileseq = place(4 * (size_t)tiles_max);
-    off_tileq0 = place(4 * (size_t)tiles_max);
+    off_units = place(sizeof(PrefillUnit) * (size_t)tiles_max);
     off_samplesrc = place(4 * (size_t)std::max(S_max, logit_rows_cap));
     off_rows = place(sizeof(SampleRow) * (size_t)S_max);
     off_epoch = place(4 * sizeof(uint32_t));  // tensor parallelism: exchange epochs before this step ([0], [1]: per
@@ -3322,8 +3321,8 @@ struct tgis_engine {
         n_launches += (max_splits > 1 && !attn_inkernel_merge) ? 2 : 1;
       }
       if (n_tiles > 0) {
-        CK(attn_prefill_launch(qkv.p, qkv_dim, kc, vc, d_seqs, ds<int32_t>(off_tileseq), ds<int32_t>(off_tileq0),
-                               n_tiles, d_bt, bt_stride, attn_out.p, q_dim, nq, nkv, scale, stream));
+        CK(attn_prefill_launch(qkv.p, qkv_dim, kc, vc, num_blocks, ds<PrefillUnit>(off_units), n_tiles,
+                               d_bt, bt_stride, attn_out.p, q_dim, T, nq, nkv, scale, num_sms, stream));
         ++n_launches;
       }
       if (lora) lora_shrink(lora_one(lora_layers[li].A_o, lora_layers[li].B_o, q_dim, H, LR), attn_out.p, q_dim);
@@ -3413,8 +3412,8 @@ struct tgis_engine {
         n_launches += (max_splits > 1 && !attn_inkernel_merge) ? 2 : 1;
       }
       if (n_tiles > 0) {
-        CK(attn_prefill_launch(qkv.p, qkv_dim, kc, vc, d_seqs, ds<int32_t>(off_tileseq), ds<int32_t>(off_tileq0),
-                               n_tiles, d_bt, bt_stride, attn_out.p, q_dim, nq, nkv, attn_scale, stream));
+        CK(attn_prefill_launch(qkv.p, qkv_dim, kc, vc, num_blocks, ds<PrefillUnit>(off_units), n_tiles,
+                               d_bt, bt_stride, attn_out.p, q_dim, T, nq, nkv, attn_scale, num_sms, stream));
         ++n_launches;
       }
       gemm(xm_attn, l.m_o, attn_out.p, l.wo, y32.p, T, H, q_dim, /*out_f32=*/1, &l.m_gu, T, F, H);
@@ -3601,8 +3600,6 @@ struct tgis_engine {
     int32_t* toklora = hs<int32_t>(off_toklora);
     AttnSeq* seqs = hs<AttnSeq>(off_seqs);
     int32_t* decids = hs<int32_t>(off_decids);
-    int32_t* tileseq = hs<int32_t>(off_tileseq);
-    int32_t* tileq0 = hs<int32_t>(off_tileq0);
     int32_t* samplesrc = hs<int32_t>(off_samplesrc);
     SampleRow* rows = hs<SampleRow>(off_rows);
     int32_t* bt = hs<int32_t>(off_bt);
@@ -3650,11 +3647,6 @@ struct tgis_engine {
       if (q_len == 1) {
         decids[n_dec++] = s;
         max_dec_kv = std::max(max_dec_kv, kv_len);
-      } else {
-        for (int q0 = 0; q0 < q_len; q0 += 16) {
-          tileseq[n_tiles] = s;
-          tileq0[n_tiles++] = q0;
-        }
       }
       if (batch[s].sample) {
         const tgis_sampling_params& sp = r.sp;
@@ -3725,6 +3717,7 @@ struct tgis_engine {
     // (S, max_splits) so that its size is a function of the CUDA-graph key
     const int max_splits_step = (max_dec_kv + DECODE_SPLIT - 1) / DECODE_SPLIT;
     decode_items_build(hs<DecItem>(items_off(S)), seqs, decids, n_dec, bt, bt_stride);
+    if (n_dec < S) n_tiles = prefill_units_build(hs<PrefillUnit>(off_units), seqs, S, pnx_on ? 1 : nq / nkv);
     const size_t copy_bytes = items_off(S) + sizeof(DecItem) * (1 + (size_t)n_dec * max_splits_step);
     const double t_ev0 = debug_launch ? now_s() : 0.0;
     CK(cudaEventRecord(ev0, stream));

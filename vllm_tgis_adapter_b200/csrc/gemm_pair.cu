@@ -476,6 +476,12 @@ cudaError_t launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, PairAr
 
 cudaError_t gemm_pair_prepare() { return pair_word.load(std::memory_order_acquire) != nullptr ? cudaSuccess : make_pair_word(); }
 
+cudaError_t gemm_pair_word(int** word) {
+  const cudaError_t e = gemm_pair_prepare();
+  *word = pair_word.load(std::memory_order_acquire);
+  return e;
+}
+
 bool gemm_pair_failed() {
   const int* w = pair_word.load(std::memory_order_acquire);
   return w != nullptr && *reinterpret_cast<const volatile int*>(w) != 0;

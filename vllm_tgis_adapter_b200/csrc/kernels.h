@@ -12,6 +12,8 @@ namespace tgis {
 // ---- gemm_tcgen05.cu --------------------------------------------------------------------------------------------
 int make_tmap_bf16_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld_elems,
                       uint32_t box_rows, uint32_t box_cols);
+int make_tmap_bf16_3d(CUtensorMap* out, const void* base, const uint64_t (&dims)[3], const uint64_t (&stride_bytes)[2],
+                      const uint32_t (&box)[3], bool swizzle128);
 int gemm_pick_bt(int T);
 constexpr int GEMM_X_BOX_MANY = 32;
 // Whether a dense product runs on CTA pairs (gemm_pair.cu): more than 256 tokens always, more than 64 when the weights have more
@@ -93,6 +95,7 @@ cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
 int gemm_pair_plan(int T, int N, int pairs);   // token tiles of the dense launch
 cudaError_t gemm_pair_prepare();               // host memory of the launches: to be called before any of them is captured
 bool gemm_pair_failed();                       // a wait inside a launch of this process ran out
+cudaError_t gemm_pair_word(int** word);        // the word that such a wait raises (for kernels that share it)
 // Tests: the host raises the error word at the nth launch from now on (0: at none), as that launch would if a wait of it ran out;
 // a raised word is taken back.  Returns the launches since the last call.
 int gemm_pair_fault(int nth);
@@ -258,11 +261,20 @@ cudaError_t attn_decode_launch(const __nv_bfloat16* qkv, int qkv_ld, const __nv_
                                int num_sms, cudaStream_t stream, int* arrive = nullptr);
 // arrive: [n_seqs * n_kv] ints, zero before the first launch (re-armed by the kernel): with it, the split merge runs inside
 // the streaming kernel (last-arriving warp per (sequence, kv head)) and attn_merge_kernel is not launched.
-// Prefill / chunked prefill (q_len >= 1), causal over the paged cache.
-cudaError_t attn_prefill_launch(const __nv_bfloat16* qkv, int qkv_ld, const __nv_bfloat16* k_cache,
-                                const __nv_bfloat16* v_cache, const AttnSeq* seqs, const int32_t* tile_seq,
-                                const int32_t* tile_q0, int n_tiles, const int32_t* block_table, int bt_stride,
-                                __nv_bfloat16* out, int out_ld, int n_q, int n_kv, float scale, cudaStream_t stream);
+
+// ---- attention_prefill.cu: prompts and their portions (q_len > 1), causal over the paged cache -------------------------------
+struct PrefillUnit {  // up to 2 * 128 / G query tokens of one sequence, read as one int4
+  int32_t row0, rows;  // first row in the flat token batch, query tokens
+  int32_t pos0;        // position of the first one
+  int32_t block_row;   // row in the block table
+};
+// The units of a step; every prompt is cut into pieces of at least 16 tokens (but for its last).  Returns their number.
+int prefill_units_build(PrefillUnit* units, const AttnSeq* seqs, int n_seqs, int G);
+// n_blocks: blocks of the caches; T: rows of qkv
+cudaError_t attn_prefill_launch(const __nv_bfloat16* qkv, int qkv_ld, const __nv_bfloat16* k_cache, const __nv_bfloat16* v_cache, int n_blocks,
+                                const PrefillUnit* units, int n_units, const int32_t* block_table, int bt_stride,
+                                __nv_bfloat16* out, int out_ld, int T, int n_q, int n_kv,
+                                float scale, int num_sms, cudaStream_t stream);
 
 // ---- element types of the kernels that run more than one (gemm_any.cu, attention_latent.cu, moe.cu, the fp32-residual norms)
 constexpr int DT_F32 = 0, DT_BF16 = 1;

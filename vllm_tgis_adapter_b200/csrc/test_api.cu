@@ -276,27 +276,27 @@ int tgis_k_attention(const void* qkv_dev, const void* k_cache_dev, const void* v
   const int G = n_q / n_kv;
   const int qkv_ld = (n_q + 2 * n_kv) * HEAD_DIM, out_ld = n_q * HEAD_DIM;
   std::vector<AttnSeq> seqs(n_seqs);
-  std::vector<int32_t> dec, tseq, tq0;
-  int max_kv = 1;
+  std::vector<int32_t> dec;
+  int max_kv = 1, T = 0;
   for (int s = 0; s < n_seqs; ++s) {
     seqs[s] = AttnSeq{seqs_host[4 * s], seqs_host[4 * s + 1], seqs_host[4 * s + 2], seqs_host[4 * s + 3]};
     if (seqs[s].q_len == 1) {
       dec.push_back(s);
       max_kv = std::max(max_kv, seqs[s].kv_len);
-    } else {
-      for (int q0 = 0; q0 < seqs[s].q_len; q0 += 16) {
-        tseq.push_back(s);
-        tq0.push_back(q0);
-      }
     }
+    T = std::max(T, seqs[s].q_start + seqs[s].q_len);
   }
+  int n_blocks = 1;
+  for (int i = 0; i < bt_rows * bt_stride; ++i) n_blocks = std::max(n_blocks, block_table_host[i] + 1);
+  std::vector<PrefillUnit> units(T / 16 + n_seqs + 1);
+  const int n_units = prefill_units_build(units.data(), seqs.data(), n_seqs, G);
   Tmp<AttnSeq> d_seqs;
-  Tmp<int32_t> d_dec, d_tseq, d_tq0, d_bt;
+  Tmp<PrefillUnit> d_units;
+  Tmp<int32_t> d_dec, d_bt;
   Tmp<float> po, pml;
   KCK(d_seqs.upload(seqs.data(), n_seqs));
   KCK(d_dec.upload(dec.data(), dec.size()));
-  KCK(d_tseq.upload(tseq.data(), tseq.size()));
-  KCK(d_tq0.upload(tq0.data(), tq0.size()));
+  KCK(d_units.upload(units.data(), units.size()));
   KCK(d_bt.upload(block_table_host, (size_t)bt_rows * bt_stride));
   const int max_splits = (max_kv + DECODE_SPLIT - 1) / DECODE_SPLIT;
   const size_t nd = dec.size() ? dec.size() : 1;
@@ -312,11 +312,10 @@ int tgis_k_attention(const void* qkv_dev, const void* k_cache_dev, const void* v
   KCK(attn_decode_launch((const bf16*)qkv_dev, qkv_ld, (const bf16*)k_cache_dev, (const bf16*)v_cache_dev, d_items.p,
                          (int)dec.size() * max_splits, d_seqs.p, d_dec.p, (int)dec.size(), max_splits, po.p, pml.p,
                          (bf16*)out_dev, out_ld, n_q, n_kv, scale, test_num_sms(), 0, arrive.p));
-  KCK(attn_prefill_launch((const bf16*)qkv_dev, qkv_ld, (const bf16*)k_cache_dev, (const bf16*)v_cache_dev, d_seqs.p,
-                          d_tseq.p, d_tq0.p, (int)tseq.size(), d_bt.p, bt_stride, (bf16*)out_dev, out_ld, n_q, n_kv,
-                          scale, 0));
-  KCK(cudaDeviceSynchronize());
-  return 0;
+  KCK(attn_prefill_launch((const bf16*)qkv_dev, qkv_ld, (const bf16*)k_cache_dev, (const bf16*)v_cache_dev, n_blocks,
+                          d_units.p, n_units, d_bt.p, bt_stride, (bf16*)out_dev, out_ld, T, n_q, n_kv, scale,
+                          test_num_sms(), 0));
+  return product_end();
 }
 
 // decode attention only, timed: `iters` launches rotating over `n_layers` cache copies (layer_stride_bytes apart) so that
