@@ -2382,7 +2382,7 @@ struct tgis_engine {
   }
   void pnx_gemm(const void* X, int x_dt, int ldx, const void* Wt, void* Y, int y_dt, int ldy, int T, int N, int K,
                 int mode = GEMM_ANY_PLAIN, bool x_tma_ok = true) {
-    if (pnx_tc && x_tma_ok && pnx_dt == DT_BF16 && x_dt == DT_BF16 && ldx == K && K % 64 == 0 && K >= 256 && N % 8 == 0 &&
+    if (pnx_tc && x_tma_ok && pnx_dt == DT_BF16 && x_dt == DT_BF16 && ldx == K && K % 64 == 0 && (K >= 256 || gemm_skinny_takes(T, N, K)) && N % 8 == 0 &&
         N >= 128 && !cfg.debug_gemm_ref && (reinterpret_cast<uintptr_t>(Y) & 15) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0) {
       const int out_mode = mode == GEMM_ANY_SWIGLU && y_dt == DT_BF16 ? 2 : mode == GEMM_ANY_GEGLU && y_dt == DT_BF16 ? 3
                            : mode == GEMM_ANY_RELU2 && y_dt == DT_BF16 ? 4
@@ -2407,6 +2407,12 @@ struct tgis_engine {
       fwrite(hbuf.data(), sizeof(float), hbuf.size(), f);
       fclose(f);
     }
+  }
+
+  // a scan over the step's leading sequences, which have one token each
+  static OuterScan single(OuterScan os) {
+    os.single = 1;
+    return os;
   }
 
   // One layer of a post-norm stack (TGIS_STYLE_POST_NORM): x += rmsnorm(mixer(x)) * norm1, x += rmsnorm(ff(x)) * norm2.
@@ -2438,6 +2444,7 @@ struct tgis_engine {
                         bt_stride, pnx_y1 + l.c_g, ld, pnx_oA, A, l.ca, stream));
       pnx_gemm(pnx_oA, A, H * s.vdim, l.w_o, pnx_o, DT_F32, W, T, W, H * s.vdim);
       OuterScan os{};
+      os.single = T == S;
       os.mode = OUTER_SCAN_GATED;
       os.q = pnx_y1 + l.c_mq; os.k = pnx_y1 + l.c_mk; os.v = pnx_y1 + l.c_mv; os.ldq = os.ldk = os.ldv = ld;
       os.q_scale = 1.f / std::sqrt((float)s.mm_dim);
@@ -2461,6 +2468,7 @@ struct tgis_engine {
       pnx_gemm(xc, A, I, l.w_x, flx_f2, DT_F32, R + 2 * N, T, R + 2 * N, I);
       pnx_gemm(flx_f2, DT_F32, R + 2 * N, l.w_dt, flx_f3, DT_F32, I, T, I, R);
       SelScan sc{};
+      sc.single = T == S;
       sc.x = flx_f1; sc.xz = pnx_y1; sc.ld_xz = 2 * I; sc.proj = flx_f2; sc.ld_proj = R + 2 * N; sc.dt_rank = R;
       sc.dt_raw = flx_f3; sc.dt_b = l.dt_b; sc.A_log = l.A_log; sc.D = l.Dv; sc.S = l.st_S; sc.conv_state = l.st_conv;
       sc.out = flx_op2; sc.out_dtype = A; sc.inner = I; sc.state = N; sc.taps = s.conv;
@@ -2479,6 +2487,7 @@ struct tgis_engine {
       pnx_gemm(mix(4), A, W, l.w_w1, pnx_cq, A, R, T, R, W, GEMM_ANY_TANH);
       pnx_gemm(pnx_cq, A, R, l.w_w2, flx_f2, DT_F32, Ad, T, Ad, R);
       OuterScan os{};
+      os.single = T == S;
       os.mode = OUTER_SCAN_DECAY;
       os.q = pnx_y1; os.k = pnx_y1 + Ad; os.v = pnx_y1 + 2 * Ad; os.ldq = os.ldk = os.ldv = 4 * Ad;
       os.q_scale = 1.f;
@@ -2544,6 +2553,7 @@ struct tgis_engine {
       CK(short_conv_silu_launch(pnx_y1 + inner, ld, C, l.conv_w, l.conv_b, s.conv, d_pos, d_tokslot, l.st_conv, flx_f1, nullptr, A, T, stream));
       CK(conv_state_save_launch(pnx_y1 + inner, ld, C, s.conv, d_seqs, S, d_tokslot, l.st_conv, stream));
       OuterScan os{};
+      os.single = T == S;
       os.mode = OUTER_SCAN_SSD;
       os.v = flx_f1; os.k = flx_f1 + inner; os.q = flx_f1 + inner + GN; os.ldq = os.ldk = os.ldv = C;
       os.q_scale = 1.f;
@@ -2667,6 +2677,7 @@ struct tgis_engine {
       const int H = s.heads, hd = H * s.dim, hv = H * s.vdim, ld = l.in_cols;
       pnx_gemm(pnx_hA, A, W, l.w_in, pnx_y1, DT_F32, ld, T, ld, W);
       OuterScan os{};
+      os.single = T == S;
       os.mode = OUTER_SCAN_HGRN;
       os.q = pnx_y1 + l.c_q; os.k = nullptr; os.v = pnx_y1 + l.c_v; os.ldq = os.ldk = os.ldv = ld;
       os.q_scale = 1.f;
@@ -2765,6 +2776,7 @@ struct tgis_engine {
     auto lightning = [&](cudaStream_t st) {   // -> pnx_yS
       const int mH = s.mm_heads, mv = mH * s.mm_vdim;
       OuterScan os{};
+      os.single = T == S;
       os.mode = OUTER_SCAN_LIGHTNING;
       os.q = pnx_y1 + l.c_mq; os.k = pnx_y1 + l.c_mk; os.v = pnx_y1 + l.c_mv; os.ldq = os.ldk = os.ldv = ld;
       os.q_scale = 1.f;
@@ -2779,7 +2791,7 @@ struct tgis_engine {
         CK(silu_cast_launch(pnx_y1 + l.c_mq, ld, flx_mix, qkv, qkv, T, st));
         const LightningChunk lc{flx_mix, qkv, 0, l.c_mk - l.c_mq, l.c_mv - l.c_mq, l.decay, l.st_S, flx_f1, mv, mH, s.mm_dim, s.mm_vdim};
         CK(lightning_chunk_launch(lc, d_seqs + lead, S - lead, d_tokslot, st));
-        if (lead > 0) CK(outer_scan_launch(os, d_seqs, lead, d_tokslot, st));
+        if (lead > 0) CK(outer_scan_launch(single(os), d_seqs, lead, d_tokslot, st));
         n_launches += lead > 0 ? 2 : 1;
       } else {
         CK(outer_scan_launch(os, d_seqs, S, d_tokslot, st));
@@ -2896,6 +2908,7 @@ struct tgis_engine {
         n_launches += 2;
       }
       OuterScan os{};
+      os.single = T == S;
       os.mode = OUTER_SCAN_GLA;
       os.q = pnx_y1 + l.c_q; os.k = pnx_y1 + l.c_k; os.v = pnx_y1 + l.c_v; os.ldq = os.ldk = os.ldv = ld;
       os.q_scale = 1.f / sqrtf((float)s.dim);
@@ -2903,7 +2916,7 @@ struct tgis_engine {
       os.S = l.st_S;
       os.out = flx_f1; os.ldo = hv;
       os.heads = s.heads; os.dim = s.dim; os.vdim = s.vdim;
-      if (n_scan > 0) CK(outer_scan_launch(os, d_seqs, chunked ? lead : S, d_tokslot, stream));
+      if (n_scan > 0) CK(outer_scan_launch(chunked ? single(os) : os, d_seqs, chunked ? lead : S, d_tokslot, stream));
       CK(head_norm_gate_launch(flx_f1, hv, s.heads, s.vdim, l.mm_norm, pnx_y1 + l.c_mg, ld, /*silu*/ 1, eps, pnx_oA, A, T, stream, 0, 1.f,
                                l.o_cols));
       n_launches += n_scan > 0 ? 2 : 1;
@@ -2918,6 +2931,7 @@ struct tgis_engine {
                       l.cos_sin2, d_pos, chunked ? flx_mix : nullptr, qkv, lead};
         CK(rotary_rows_launch(rr, T, st));
         OuterScan os{};
+      os.single = T == S;
         os.mode = OUTER_SCAN_RETENTION;
         os.q = pnx_y1 + l.c_mq; os.k = pnx_y1 + l.c_mk; os.v = pnx_y1 + l.c_mv; os.ldq = os.ldk = os.ldv = ld;
         os.q_scale = 1.f;
@@ -2928,7 +2942,7 @@ struct tgis_engine {
         if (chunked) {
           const LightningChunk lc{flx_mix, qkv, 0, md, 2 * md, l.decay, l.st_S, flx_f1, mv, mH, s.mm_dim, s.mm_vdim};
           CK(lightning_chunk_launch(lc, d_seqs + lead, S - lead, d_tokslot, st));
-          if (lead > 0) CK(outer_scan_launch(os, d_seqs, lead, d_tokslot, st));
+          if (lead > 0) CK(outer_scan_launch(single(os), d_seqs, lead, d_tokslot, st));
           n_launches += lead > 0 ? 1 : 0;
         } else {
           CK(outer_scan_launch(os, d_seqs, S, d_tokslot, st));

@@ -307,6 +307,8 @@ struct GemmAny {
 };
 bool gemm_pair_takes_groups(const GemmAny& a);   // gemm_pair.cu
 cudaError_t gemm_pair_grouped_launch(const GemmAny& a, cudaStream_t stream);
+bool gemm_skinny_takes_batch(const GemmAny& a);  // gemm_skinny.cu
+cudaError_t gemm_skinny_batch_launch(const GemmAny& a, cudaStream_t stream);
 cudaError_t gemm_any_launch(const GemmAny& a, cudaStream_t stream);
 
 // ---- norms over an fp32 residual stream (elementwise.cu) ------------------------------------------------------------
@@ -551,6 +553,7 @@ struct SelScan {
   float* conv_state;     // [slots][taps - 1][inner]
   void* out; int out_dtype;
   int inner, state, taps;
+  int single;            // every portion of the launch is one token
 };
 constexpr int SELSCAN_MAX_STATE = 128;
 cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot,
@@ -587,6 +590,7 @@ struct OuterScan {
   const float* decay;                          // LIGHTNING, RETENTION: [heads]
   float inv_tau;                               // GLA
   int32_t* done;                               // GATED: [slots][heads], zero between launches
+  int single;                                  // every portion of the launch is one token
 };
 cudaError_t outer_scan_launch(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot,
                               cudaStream_t stream);

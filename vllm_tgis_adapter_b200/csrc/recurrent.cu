@@ -25,6 +25,31 @@ __device__ __forceinline__ void st_op(void* out, int dt, size_t i, float v) {
   if (dt == DT_BF16) reinterpret_cast<__nv_bfloat16*>(out)[i] = __float2bfloat16_rn(v);
   else reinterpret_cast<float*>(out)[i] = v;
 }
+template <int VEC>
+__device__ __forceinline__ void ld_vec(const float* p, float (&v)[VEC]) {
+  if constexpr (VEC == 4) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  } else {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) v[e] = p[e];
+  }
+}
+template <int VEC>
+__device__ __forceinline__ void st_op_vec(void* out, int dt, size_t i, const float (&v)[VEC]) {
+  if constexpr (VEC == 4) {
+    if (dt == DT_BF16) {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v[0], v[1]), hi = __floats2bfloat162_rn(v[2], v[3]);
+      *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(out) + i) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    } else {
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + i) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) st_op(out, dt, i + e, v[e]);
+  }
+}
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
@@ -36,6 +61,9 @@ __device__ __forceinline__ float warp_sum_f(float v) {
 }
 
 // ------------------------------------------------------------------------------------------------ token shift
+// VEC = 4: 16-byte loads, 8- or 16-byte stores (needs width and out_bs to be multiples of four and the pointers aligned); one piece of
+// the row per thread, so that a step of a few tokens is not a chain of loads: 32 tokens x 2048 x 5 mixes 28.9 -> 3.9 us
+template <int VEC>
 __global__ void __launch_bounds__(128)
 token_shift_mix_kernel(const float* __restrict__ x, int width, const float* __restrict__ mu, int n_mix,
                        const int32_t* __restrict__ positions, const int32_t* __restrict__ tok_slot,
@@ -46,10 +74,22 @@ token_shift_mix_kernel(const float* __restrict__ x, int width, const float* __re
   const int slot = tok_slot[t];
   const float* prev = nullptr;   // nullptr: zeros
   if (positions[t] > 0) prev = (t > 0 && tok_slot[t - 1] == slot) ? x + (size_t)(t - 1) * width : prev_state + (size_t)slot * width;
-  const float* xr = x + (size_t)t * width;
-  for (int i = threadIdx.x; i < width; i += 128) {
-    const float h = xr[i], d = (prev ? prev[i] : 0.f) - h;
-    for (int s = 0; s < n_mix; ++s) st_op(out, out_dtype, (size_t)s * out_bs + (size_t)t * width + i, fmaf(d, mu[(size_t)s * width + i], h));
+  const int i = (blockIdx.y * 128 + threadIdx.x) * VEC;
+  if (i >= width) return;
+  float h[VEC], d[VEC];
+  ld_vec<VEC>(x + (size_t)t * width + i, h);
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) d[e] = 0.f;
+  if (prev) ld_vec<VEC>(prev + i, d);
+#pragma unroll
+  for (int e = 0; e < VEC; ++e) d[e] -= h[e];
+#pragma unroll 5
+  for (int s = 0; s < n_mix; ++s) {
+    float m[VEC];
+    ld_vec<VEC>(mu + (size_t)s * width + i, m);
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) m[e] = fmaf(d[e], m[e], h[e]);
+    st_op_vec<VEC>(out, out_dtype, (size_t)s * out_bs + (size_t)t * width + i, m);
   }
 }
 
@@ -71,6 +111,22 @@ short_conv_silu_kernel(const float* __restrict__ xz, int ld, int inner, const fl
   float acc[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) acc[e] = b != nullptr ? b[c + e] : 0.f;
+  if (VEC == 4 && taps == 4) {   // the usual length: all of a channel's loads are on their way before the first sum (32 tokens x 4096 7.9 -> 5.1 us)
+    float v[4][4], wt[4][4];
+#pragma unroll
+    for (int j = 3; j >= 0; --j) {
+      const float* src = j <= nb ? xz + (size_t)(t - j) * ld + c : conv_state + ((size_t)slot * 3 + (3 - j + nb)) * inner + c;
+      if (p - j >= 0) ld_vec<4>(src, v[j]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ld_vec<4>(w + (size_t)(c + e) * 4, wt[e]);
+#pragma unroll
+    for (int j = 3; j >= 0; --j)
+      if (p - j >= 0)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[e] = fmaf(wt[e][3 - j], v[j][e], acc[e]);
+    taps = 0;
+  }
   for (int j = taps - 1; j >= 0; --j) {   // oldest input first
     if (p - j < 0) continue;
     const float* src = j <= nb ? xz + (size_t)(t - j) * ld + c
@@ -91,10 +147,7 @@ short_conv_silu_kernel(const float* __restrict__ xz, int ld, int inner, const fl
     if (VEC == 4) *reinterpret_cast<float4*>(out_f32 + (size_t)t * inner + c) = make_float4(acc[0], acc[1 % VEC], acc[2 % VEC], acc[3 % VEC]);
     else out_f32[(size_t)t * inner + c] = acc[0];
   }
-  if (out_op) {
-#pragma unroll
-    for (int e = 0; e < VEC; ++e) st_op(out_op, out_dtype, (size_t)t * inner + c + e, acc[e]);
-  }
+  if (out_op) st_op_vec<VEC>(out_op, out_dtype, (size_t)t * inner + c, acc);
 }
 
 // ------------------------------------------------------------------------------------------------ selective scan
@@ -208,6 +261,57 @@ selective_scan_reg_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int
   for (int j = 0; j < SCAN_RPL; ++j)
     if (sub * SCAN_RPL + j < N) Sg[sub * SCAN_RPL + j] = Sr[j];
   if (sub == 0) scan_save_conv(a, sq, slot, c);
+}
+
+// Steps whose portions are single tokens: grid (sequences, ceil(inner / 64)), four lanes a channel as above and the same sums in the
+// same order, but every load is requested at once (the states' lines while the kernel before still runs) instead of a chunk's staging.
+// Needs SCAN_REG_STATE states and aligned rows.  32 tokens, 4096 channels: 21.5 -> 9.0 us.
+__global__ void __launch_bounds__(256)
+selective_step_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t* __restrict__ tok_slot) {
+  constexpr int N = SCAN_REG_STATE;
+  griddep_launch();
+  const AttnSeq sq = seqs[blockIdx.x];   // (written by the host before the step, as the slots are)
+  const int slot = tok_slot[sq.q_start], sub = threadIdx.x & 3, c = blockIdx.y * 64 + (threadIdx.x >> 2);
+  const bool live = c < a.inner;
+  float* Sg = a.S + ((size_t)slot * a.inner + (live ? c : 0)) * N + sub * 4;
+  if (live && sub == 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(Sg));
+  float rate[4] = {0.f, 0.f, 0.f, 0.f};
+  if (live) ld_vec<4>(a.A_log + (size_t)c * N + sub * 4, rate);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) rate[j] = -expf(rate[j]);
+  const float dtb = live ? a.dt_b[c] : 0.f, Dc = live ? a.D[c] : 0.f;
+  griddep_wait();
+  if (!live) return;   // (a channel's four lanes leave together)
+  const size_t row = (size_t)sq.q_start;
+  float Sr[4] = {0.f, 0.f, 0.f, 0.f}, bn[4], cn[4];
+  if (sq.kv_len > 1) ld_vec<4>(Sg, Sr);
+  const float* pr = a.proj + row * a.ld_proj + a.dt_rank;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) bn[j] = pr[sub * 4 + j], cn[j] = pr[N + sub * 4 + j];
+  const float xv = a.x[row * a.inner + c], zv = a.xz[row * a.ld_xz + a.inner + c];
+  const float dt = softplus_f(a.dt_raw[row * a.inner + c] + dtb), dx = dt * xv;
+  // the convolution's tail: lane `sub` moves entries sub, sub + 4, ..; it reads them before the lanes that overwrite them write
+  const int K1 = a.taps - 1;
+  float* cs = a.conv_state + (size_t)slot * K1 * a.inner + c;
+  float y = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    Sr[j] = fmaf(expf(dt * rate[j]), Sr[j], dx * bn[j]);
+    y = fmaf(Sr[j], cn[j], y);
+  }
+  const uint32_t four = 0xfu << (threadIdx.x & 28);
+  for (int e0 = 0; e0 < K1; e0 += 4) {
+    const int e = e0 + sub, pp = sq.kv_len - K1 + e;
+    float v = 0.f;
+    if (e < K1 && pp >= 0) v = pp == sq.kv_len - 1 ? a.xz[row * a.ld_xz + c] : cs[(size_t)(e + 1) * a.inner];
+    __syncwarp(four);
+    if (e < K1) cs[(size_t)e * a.inner] = v;
+    __syncwarp(four);
+  }
+  y += __shfl_xor_sync(four, y, 2);
+  y += __shfl_xor_sync(four, y, 1);
+  *reinterpret_cast<float4*>(Sg) = make_float4(Sr[0], Sr[1], Sr[2], Sr[3]);
+  if (sub == 0) st_op(a.out, a.out_dtype, row * a.inner + c, fmaf(Dc, xv, y) * silu_f(zv));
 }
 
 // More states: one thread per channel, state in shared memory.  A chunk's B / C rows are staged in shared memory and its per-channel
@@ -550,6 +654,177 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
   }
 }
 
+// Steps whose portions are single tokens: the same update and the same sums in the same order (bit for bit), laid out for the
+// bytes of the state, which are all there is: 256 threads = 8 warps of rows x 32 lanes of CPT neighbouring columns, a whole
+// [dim, 32 CPT] piece of a head requested at once, its lines already while the kernel before still runs.  Needs dim = 8 RPT and
+// whole pieces.  32 tokens: gated, 8 heads of 128 x 256 (67 MB moved), 30.0 -> 16.4 us; decayed, 32 heads of 64 x 64, 15.0 -> 8.5.
+template <int RPT, int MODE, int CPT>
+__global__ void __launch_bounds__(OS_THREADS)
+outer_step_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* __restrict__ tok_slot) {
+  constexpr int D = RPT * OS_GROUPS, COLS = 32 * CPT;
+  __shared__ __align__(16) float vec[3][D];   // q | k | w (GATED: n q)
+  __shared__ float part[OS_GROUPS][COLS];
+  __shared__ float gates[3];                  // the decay, the factor of the outer product, GATED: e^(-m)
+  griddep_launch();
+  const AttnSeq sq = seqs[blockIdx.x];        // (written by the host before the step, as the slots are)
+  const int h = blockIdx.y, tid = threadIdx.x, g = tid >> 5, lane = tid & 31;
+  const int hq = a.qk_heads > 0 ? h / (a.heads / a.qk_heads) : h;
+  const int c0 = blockIdx.z * COLS, slot = tok_slot[sq.q_start];
+  const bool fresh = sq.kv_len == 1;
+  constexpr bool OWN_DECAY = MODE == OUTER_SCAN_DECAY || MODE == OUTER_SCAN_HGRN || MODE == OUTER_SCAN_GLA;
+  auto row_of = [&](int j) { return 4 * (g + (j >> 2) * OS_GROUPS) + (j & 3); };
+  float* Sg = a.S + (((size_t)slot * a.heads + h) * D) * a.vdim + c0 + lane * CPT;
+  if (!fresh && lane * CPT % 32 == 0) {
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) asm volatile("prefetch.global.L2 [%0];" ::"l"(Sg + (size_t)row_of(j) * a.vdim));
+  }
+  griddep_wait();
+  float S[RPT][CPT];
+#pragma unroll
+  for (int j = 0; j < RPT; ++j) {
+#pragma unroll
+    for (int e = 0; e < CPT; ++e) S[j][e] = 0.f;
+    if (!fresh) {
+      const float* from = Sg + (size_t)row_of(j) * a.vdim;
+      if constexpr (CPT == 4) {
+        ld_vec<4>(from, S[j]);
+      } else {
+        const float2 v = *reinterpret_cast<const float2*>(from);
+        S[j][0] = v.x; S[j][1] = v.y;
+      }
+    }
+  }
+  const size_t row = (size_t)sq.q_start;
+  float n_row = 0.f, m_run = 0.f;
+  if (MODE == OUTER_SCAN_GATED && !fresh) {
+    n_row = tid < D ? a.n[((size_t)slot * a.heads + h) * D + tid] : 0.f;
+    m_run = a.m[(size_t)slot * a.heads + h];
+  }
+  if (tid < D) {
+    const float q = a.q[row * a.ldq + (size_t)hq * D + tid];
+    const float k = MODE == OUTER_SCAN_HGRN ? a.u[(size_t)h * D + tid] : a.k[row * a.ldk + (size_t)hq * D + tid];
+    const float d = OWN_DECAY ? a.decay_raw[row * a.ldd + (size_t)h * D + tid] : 0.f, w = OWN_DECAY ? a.w0[(size_t)h * D + tid] : 0.f;
+    if (MODE == OUTER_SCAN_HGRN) {
+      vec[0][tid] = silu_f(q) * a.q_scale;
+      vec[1][tid] = (1.f - k) * sigmoid_f(-(d + w));
+      vec[2][tid] = k + (1.f - k) * sigmoid_f(d + w);
+    } else if (MODE == OUTER_SCAN_LIGHTNING) {
+      vec[0][tid] = silu_f(q) * a.q_scale;
+      vec[1][tid] = silu_f(k);
+    } else {
+      vec[0][tid] = q * a.q_scale;
+      vec[1][tid] = k;
+      if (MODE == OUTER_SCAN_DECAY) vec[2][tid] = expf(-expf(d + w));
+      if (MODE == OUTER_SCAN_GLA) vec[2][tid] = expf(logsigmoid_f(d + w) * a.inv_tau);
+    }
+  }
+  float m_new = 0.f;
+  if (MODE == OUTER_SCAN_GATED && tid == 0) {
+    const float ig = a.gate_cap * tanhf((a.ig[row * a.ldg + h] + a.ig_b[h]) / a.gate_cap);
+    const float fg = logsigmoid_f(a.gate_cap * tanhf((a.fg[row * a.ldg + h] + a.fg_b[h]) / a.gate_cap));
+    m_new = fmaxf(fg + m_run, ig);
+    gates[0] = expf(fg + m_run - m_new);
+    gates[1] = expf(ig - m_new);
+    gates[2] = expf(-m_new);
+  }
+  if (MODE == OUTER_SCAN_SSD && tid == 0) {
+    const float dt = softplus_f(a.step_raw[row * a.lds + h] + a.step_b[h]);
+    gates[0] = expf(-expf(a.A_log[h]) * dt);
+    gates[1] = dt;
+  }
+  float vr[CPT];   // as it is (SSD's skip reads it), and times the gate
+#pragma unroll
+  for (int e = 0; e < CPT; ++e) {
+    vr[e] = a.v[row * a.ldv + (size_t)h * a.vdim + c0 + lane * CPT + e];
+    if (MODE == OUTER_SCAN_LIGHTNING) vr[e] = silu_f(vr[e]);
+  }
+  __syncthreads();
+  if (MODE == OUTER_SCAN_GATED) {
+    if (tid < D) {
+      n_row = fmaf(gates[0], n_row, gates[1] * vec[1][tid]);
+      vec[2][tid] = n_row * vec[0][tid];
+    }
+  }
+  float wd = (MODE == OUTER_SCAN_LIGHTNING || MODE == OUTER_SCAN_RETENTION) ? a.decay[h] : 0.f, vc[CPT];
+#pragma unroll
+  for (int e = 0; e < CPT; ++e) vc[e] = vr[e];
+  if (MODE == OUTER_SCAN_SSD || MODE == OUTER_SCAN_GATED) {
+    wd = gates[0];
+#pragma unroll
+    for (int e = 0; e < CPT; ++e) vc[e] *= gates[1];
+  }
+  float o[CPT][4];
+#pragma unroll
+  for (int e = 0; e < CPT; ++e)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[e][i] = 0.f;
+#pragma unroll
+  for (int j = 0; j < RPT; j += 4) {
+    float q4[4], k4[4], w4[4] = {wd, wd, wd, wd}, u4[4] = {0.f, 0.f, 0.f, 0.f};
+    const int i0 = row_of(j);
+    ld_vec<4>(&vec[0][i0], q4);
+    ld_vec<4>(&vec[1][i0], k4);
+    if (OWN_DECAY) ld_vec<4>(&vec[2][i0], w4);
+    if (MODE == OUTER_SCAN_DECAY) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) u4[i] = a.u[(size_t)h * D + i0 + i];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < CPT; ++e) {
+        float& s = S[j + i][e];
+        const float kv = __fmul_rn(k4[i], vc[e]);   // (rounded before it is added, as the packed product above is)
+        if (MODE == OUTER_SCAN_DECAY) {
+          o[e][i] = fmaf(q4[i], fmaf(u4[i], kv, s), o[e][i]);
+          s = fmaf(w4[i], s, kv);
+        } else {
+          s = fmaf(w4[i], s, kv);
+          o[e][i] = fmaf(q4[i], s, o[e][i]);
+        }
+      }
+  }
+#pragma unroll
+  for (int e = 0; e < CPT; ++e) part[g][lane * CPT + e] = (o[e][0] + o[e][1]) + (o[e][2] + o[e][3]);
+#pragma unroll
+  for (int j = 0; j < RPT; ++j) {
+    float* to = Sg + (size_t)row_of(j) * a.vdim;
+    if constexpr (CPT == 4) *reinterpret_cast<float4*>(to) = make_float4(S[j][0], S[j][1], S[j][2], S[j][3]);
+    else *reinterpret_cast<float2*>(to) = make_float2(S[j][0], S[j][1]);
+  }
+  __syncthreads();
+  if (tid < COLS) {
+    float sum = 0.f;
+#pragma unroll
+    for (int r = 0; r < OS_GROUPS; ++r) sum += part[r][tid];
+    if (MODE == OUTER_SCAN_GATED) {
+      float d = 0.f;
+      for (int i = lane; i < D; i += 32) d += vec[2][i];
+      d = warp_sum_f(d);
+      sum = sum / (fmaxf(fabsf(d), gates[2]) + 1e-6f);
+    }
+    if (MODE == OUTER_SCAN_SSD) sum = fmaf(a.D[h], a.v[row * a.ldv + (size_t)h * a.vdim + c0 + tid], sum);
+    a.out[row * a.ldo + (size_t)h * a.vdim + c0 + tid] = sum;
+  }
+  if (MODE == OUTER_SCAN_GATED) {   // as above: the head's last piece overwrites what all of them started from
+    __shared__ int last_block;
+    if (tid == 0) {
+      int32_t* done = a.done + (size_t)slot * a.heads + h;
+      last_block = gridDim.z == 1 || atomicAdd(done, 1) == (int)gridDim.z - 1;
+      if (last_block && gridDim.z > 1) *done = 0;
+    }
+    __syncthreads();
+    if (last_block) {
+      if (tid < D) a.n[((size_t)slot * a.heads + h) * D + tid] = n_row;
+      if (tid == 0) a.m[(size_t)slot * a.heads + h] = m_new;
+    }
+  }
+  if (blockIdx.z == 0 && h == 0 && a.x_last != nullptr) {
+    const float* src = a.x + row * a.width;
+    for (int i = tid; i < a.width; i += OS_THREADS) a.x_last[(size_t)slot * a.width + i] = src[i];
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ convolution state
 // grid (sequences, ceil(n / 128)): one thread per channel moves the tail of its convolution forward
 __global__ void __launch_bounds__(128)
@@ -847,8 +1122,12 @@ cudaError_t token_shift_mix_launch(const float* x, int width, const float* mu, i
                                    const int32_t* tok_slot, const float* prev_state, void* out, int out_dtype,
                                    long long out_bs, int T, cudaStream_t stream) {
   if (T <= 0) return cudaSuccess;
-  return launch_k(token_shift_mix_kernel, dim3(T), dim3(128), 0, stream, x, width, mu, n_mix, positions, tok_slot, prev_state,
-                  out, out_dtype, out_bs);
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (width % 4 == 0 && out_bs % 4 == 0 && al16(x) && al16(mu) && al16(prev_state) && al16(out))
+    return launch_k(token_shift_mix_kernel<4>, dim3(T, (width / 4 + 127) / 128), dim3(128), 0, stream, x, width, mu, n_mix, positions,
+                    tok_slot, prev_state, out, out_dtype, out_bs);
+  return launch_k(token_shift_mix_kernel<1>, dim3(T, (width + 127) / 128), dim3(128), 0, stream, x, width, mu, n_mix, positions, tok_slot,
+                  prev_state, out, out_dtype, out_bs);
 }
 
 cudaError_t short_conv_silu_launch(const float* xz, int ld, int inner, const float* w, const float* b, int taps,
@@ -857,7 +1136,7 @@ cudaError_t short_conv_silu_launch(const float* xz, int ld, int inner, const flo
   if (T <= 0) return cudaSuccess;
   if (taps < 1) return cudaErrorInvalidValue;
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-  if (ld % 4 == 0 && inner % 4 == 0 && al16(xz) && al16(conv_state) && al16(out_f32))
+  if (ld % 4 == 0 && inner % 4 == 0 && al16(xz) && al16(conv_state) && al16(out_f32) && al16(w) && al16(out_op))
     return launch_k(short_conv_silu_kernel<4>, dim3(T, (inner / 4 + 127) / 128), dim3(128), 0, stream, xz, ld, inner, w, b, taps,
                     positions, tok_slot, conv_state, out_f32, out_op, out_dtype);
   return launch_k(short_conv_silu_kernel<1>, dim3(T, (inner + 127) / 128), dim3(128), 0, stream, xz, ld, inner, w, b, taps,
@@ -869,6 +1148,9 @@ cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_s
   if (n_seqs <= 0) return cudaSuccess;
   if (a.state < 1 || a.state > SELSCAN_MAX_STATE || a.taps < 1) return cudaErrorInvalidValue;
   const size_t bc = (size_t)SCAN_CHUNK * 2 * a.state * sizeof(float);
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (a.single && a.state == SCAN_REG_STATE && al16(a.S) && al16(a.A_log))
+    return launch_k(selective_step_kernel, dim3(n_seqs, (a.inner + 63) / 64), dim3(256), 0, stream, a, seqs, tok_slot);
   if (a.state <= SCAN_REG_STATE) {
     constexpr int per_cta = SCAN_THREADS / SCAN_LPC;
     return launch_k(selective_scan_reg_kernel, dim3(n_seqs, (a.inner + per_cta - 1) / per_cta), dim3(SCAN_THREADS), 0, stream, a, seqs,
@@ -887,6 +1169,12 @@ cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_s
 
 template <int RPT, int MODE>
 static cudaError_t outer_scan_rows(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot, cudaStream_t stream) {
+  if constexpr (RPT <= 16) {   // (more rows, and columns that are no whole pieces, have no step kernel: 32 x 4 state values would spill)
+    if (a.single && a.dim == RPT * OS_GROUPS && (reinterpret_cast<uintptr_t>(a.S) & 15) == 0) {
+      if (a.vdim % 128 == 0) return launch_k(outer_step_kernel<RPT, MODE, 4>, dim3(n_seqs, a.heads, a.vdim / 128), dim3(OS_THREADS), 0, stream, a, seqs, tok_slot);
+      if (a.vdim % 64 == 0) return launch_k(outer_step_kernel<RPT, MODE, 2>, dim3(n_seqs, a.heads, a.vdim / 64), dim3(OS_THREADS), 0, stream, a, seqs, tok_slot);
+    }
+  }
   const dim3 grid(n_seqs, a.heads, (a.vdim + OS_COLS - 1) / OS_COLS);
   const size_t smem = ((size_t)OS_CHUNK * 3 * ((a.dim + 3) & ~3) + OS_CHUNK * OS_COLS) * sizeof(float);   // <= 50 KB (+ 17 KB static)
   const auto kernel = a.dim == RPT * OS_GROUPS ? outer_scan_kernel<RPT, MODE, true> : outer_scan_kernel<RPT, MODE, false>;
