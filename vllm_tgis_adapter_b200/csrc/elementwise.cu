@@ -660,20 +660,41 @@ cudaError_t rmsnorm_f32_launch(const float* x, int ldx, const float* w, float w_
   return launch_k(rmsnorm_f32_kernel, dim3(T), dim3(NORM_THREADS), 0, stream, x, ldx, w, w_off, out, out_dtype, ldo, n, eps);
 }
 
-__global__ void embed_scale_f32_kernel(const int32_t* __restrict__ tok, const void* __restrict__ table, int table_dtype,
+// a piece of a row per thread (one thread a row's sixteenth was a chain of loads: 32 rows of 2048 10.3 -> 2.3 us); VEC = 4: aligned rows
+template <int VEC>
+__global__ void __launch_bounds__(128) embed_scale_f32_kernel(const int32_t* __restrict__ tok, const void* __restrict__ table, int table_dtype,
                                        float scale, float* __restrict__ resid, int hidden, int vocab) {
   griddep_launch();
   griddep_wait();
   int row = tok[blockIdx.x];
   if (row < 0 || row >= vocab) row = 0;
-  for (int i = threadIdx.x; i < hidden; i += blockDim.x)
-    resid[(size_t)blockIdx.x * hidden + i] = ld_dt(table, table_dtype, (size_t)row * hidden + i) * scale;
+  const int i = (blockIdx.y * 128 + threadIdx.x) * VEC;
+  if (i >= hidden) return;
+  float* out = resid + (size_t)blockIdx.x * hidden + i;
+  if constexpr (VEC == 4) {
+    float v[4];
+    if (table_dtype == DT_BF16) {
+      const uint2 r = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(table) + (size_t)row * hidden + i);
+      v[0] = __uint_as_float(r.x << 16); v[1] = __uint_as_float(r.x & 0xffff0000u);
+      v[2] = __uint_as_float(r.y << 16); v[3] = __uint_as_float(r.y & 0xffff0000u);
+    } else {
+      const float4 r = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(table) + (size_t)row * hidden + i);
+      v[0] = r.x; v[1] = r.y; v[2] = r.z; v[3] = r.w;
+    }
+    *reinterpret_cast<float4*>(out) = make_float4(v[0] * scale, v[1] * scale, v[2] * scale, v[3] * scale);
+  } else {
+    *out = ld_dt(table, table_dtype, (size_t)row * hidden + i) * scale;
+  }
 }
 cudaError_t embed_scale_f32_launch(const int32_t* token_ids, const void* table, int table_dtype, float scale, float* resid,
                                    int T, int hidden, int vocab, cudaStream_t stream) {
   if (T <= 0) return cudaSuccess;
-  return launch_k(embed_scale_f32_kernel, dim3(T), dim3(128), 0, stream, token_ids, table, table_dtype, scale, resid, hidden,
-                  vocab);
+  auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (hidden % 4 == 0 && al16(table) && al16(resid))
+    return launch_k(embed_scale_f32_kernel<4>, dim3(T, (hidden / 4 + 127) / 128), dim3(128), 0, stream, token_ids, table, table_dtype, scale,
+                    resid, hidden, vocab);
+  return launch_k(embed_scale_f32_kernel<1>, dim3(T, (hidden + 127) / 128), dim3(128), 0, stream, token_ids, table, table_dtype, scale, resid,
+                  hidden, vocab);
 }
 
 // VEC = 4: hidden % 4 == 0, every row read and written as 16-byte (fp32) / 8-byte (bf16) vectors; VEC = 1: any width
@@ -821,6 +842,167 @@ __global__ void __launch_bounds__(NORM_THREADS) resid_tail_kernel(ResidTail a, i
     if (threadIdx.x == 0) a.dot_out[t] = 1.f / (1.f + expf(-z));
   }
 }
+// The same for aligned rows of up to NV * 1024 entries, bit for bit, with the row in registers: weights are loaded before the kernel in
+// front ends, and the stream, the outputs and the expert rows' addresses in one round behind it, where the loops above wait for
+// memory once per pass and once per expert.  That wait is all there is where an SM has one row (RESID_ROWS): 32 rows of 2048, warm,
+// with six expert rows beside a shared one 6.5 -> 3.7 us, without 3.9 -> 2.7, of 1024 4.4 -> 3.6 and 3.0 -> 2.7; in a decode
+// step, where the expert rows are cold, 9.1 -> 5.1 on average.  Beyond, its registers cost more rows in flight than it saves: 389 rows
+// of 1024 3.4 -> 4.4 and 5.0 -> 6.7, 2048 rows of 2048 12.8 -> 15.3.
+constexpr int RESID_ROWS = 148;
+template <int NV>
+__global__ void __launch_bounds__(NORM_THREADS) resid_tail_row_kernel(ResidTail a, int hidden) {
+  __shared__ float red[NORM_THREADS / 32];
+  constexpr int TOP = 8;   // expert rows requested at a time
+  const int t = blockIdx.x;
+  const size_t base = (size_t)t * hidden;
+  using V = FV<4>;
+  auto at = [&](int n) { return (int)(threadIdx.x + n * NORM_THREADS) * 4; };
+  auto load = [&](const float* from, V (&v)[NV]) {
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+      v[n] = V{{0.f, 0.f, 0.f, 0.f}};
+      if (from != nullptr && at(n) < hidden) v[n] = ld_fv<4>(from + at(n));
+    }
+  };
+  griddep_launch();
+  V w_post[NV], w_pre[NV];
+  load(a.w_post, w_post);
+  load(a.w_pre, w_pre);
+  griddep_wait();
+  V x[NV], y[NV];
+  load(a.resid + base, x);
+  if (a.y_pair != nullptr) {   // two mixers side by side: each output is normed by itself first
+    V ya[NV], yb[NV], wa[NV], wb[NV];
+    load(a.y_main + base, ya);
+    load(a.y_pair + base, yb);
+    load(a.w_main, wa);
+    load(a.w_pair, wb);
+    float sa = 0.f, sb = 0.f;
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+      if (at(n) < hidden)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          sa = fmaf(ya[n].v[e], ya[n].v[e], sa);
+          sb = fmaf(yb[n].v[e], yb[n].v[e], sb);
+        }
+    const float rs_a = 1.f / sqrtf(block_sum<NORM_THREADS>(sa, red) / (float)hidden + a.eps);
+    const float rs_b = 1.f / sqrtf(block_sum<NORM_THREADS>(sb, red) / (float)hidden + a.eps);
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[n].v[e] = 0.5f * (ya[n].v[e] * rs_a * wa[n].v[e] + yb[n].v[e] * rs_b * wb[n].v[e]);
+  } else if (a.y_main != nullptr) {
+    load(a.y_main + base, y);
+  } else {
+    V side[NV];
+    load(a.y_side != nullptr ? a.y_side + base : nullptr, side);
+    const float sw = a.y_side != nullptr && a.side_gate != nullptr ? a.side_gate[t] : 1.f;
+#pragma unroll
+    for (int n = 0; n < NV; ++n) y[n] = V{{0.f, 0.f, 0.f, 0.f}};
+    if (a.y_rows != nullptr)
+      for (int k0 = 0; k0 < a.top; k0 += TOP) {   // fixed k order
+        int row[TOP];
+        float w[TOP];
+#pragma unroll
+        for (int k = 0; k < TOP; ++k) {
+          const bool in = k0 + k < a.top;
+          row[k] = in ? a.inv[(size_t)t * a.top + k0 + k] : 0;
+          w[k] = !in ? 0.f : a.mix_w != nullptr ? a.mix_w[(size_t)t * a.top + k0 + k] : a.mix_const;
+        }
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+          if (at(n) >= hidden) continue;
+          V rv[TOP];
+#pragma unroll
+          for (int k = 0; k < TOP; ++k)
+            if (k0 + k < a.top) rv[k] = ld_fv<4>(a.y_rows + (size_t)row[k] * hidden + at(n));
+#pragma unroll
+          for (int k = 0; k < TOP; ++k)
+            if (k0 + k < a.top)
+#pragma unroll
+              for (int e = 0; e < 4; ++e) y[n].v[e] = fmaf(w[k], rv[k].v[e], y[n].v[e]);
+        }
+      }
+    if (a.y_side != nullptr)
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[n].v[e] = fmaf(sw, side[n].v[e], y[n].v[e]);
+  }
+  V extra[NV];
+  if (a.extra != nullptr) load(a.extra + base, extra);
+  if (a.w_post != nullptr) {
+    float ss = 0.f;
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+      if (at(n) < hidden)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) ss += y[n].v[e] * y[n].v[e];
+    const float rs = 1.f / sqrtf(block_sum<NORM_THREADS>(ss, red) / (float)hidden + a.eps);
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[n].v[e] = x[n].v[e] + a.mult * (y[n].v[e] * rs * (a.w_off + w_post[n].v[e]));
+  } else {
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[n].v[e] = fmaf(a.mult, y[n].v[e], x[n].v[e]);
+  }
+  float ss2 = 0.f;
+#pragma unroll
+  for (int n = 0; n < NV; ++n)
+    if (at(n) < hidden) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (a.extra != nullptr) x[n].v[e] += extra[n].v[e];
+        ss2 += x[n].v[e] * x[n].v[e];
+      }
+      st_fv<4>(a.resid + base + at(n), x[n]);
+    }
+  auto store = [&](void* out, int n, const V& v) {
+    if (a.out_dtype == DT_BF16) {
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v.v[0], v.v[1]), hi = __floats2bfloat162_rn(v.v[2], v.v[3]);
+      *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(out) + base + at(n)) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    } else {
+      st_fv<4>(reinterpret_cast<float*>(out) + base + at(n), v);
+    }
+  };
+  if (a.w_pre == nullptr) {
+    if (a.cast_out != 0 && a.out != nullptr)
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+        if (at(n) < hidden) store(a.out, n, x[n]);
+    return;
+  }
+  const float rs2 = 1.f / sqrtf(block_sum<NORM_THREADS>(ss2, red) / (float)hidden + a.eps);
+  float dot = 0.f;
+#pragma unroll
+  for (int n = 0; n < NV; ++n) {
+    if (at(n) >= hidden) continue;
+    V o;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o.v[e] = x[n].v[e] * rs2 * (a.w_off + w_pre[n].v[e]);
+    if (a.dot_out != nullptr) {
+      const V d = ld_fv<4>(a.w_dot + at(n));
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dot = fmaf(o.v[e], d.v[e], dot);
+    }
+    store(a.out, n, o);
+    if (a.w_pre2 != nullptr) {
+      const V w2 = ld_fv<4>(a.w_pre2 + at(n));
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o.v[e] = x[n].v[e] * rs2 * (a.w_off + w2.v[e]);
+      store(a.out2, n, o);
+    }
+  }
+  if (a.dot_out != nullptr) {
+    const float z = block_sum<NORM_THREADS>(dot, red);
+    if (threadIdx.x == 0) a.dot_out[t] = 1.f / (1.f + expf(-z));
+  }
+}
 cudaError_t resid_tail_launch(const ResidTail& a, int T, int hidden, cudaStream_t stream) {
   if (T <= 0) return cudaSuccess;
   if (a.resid == nullptr || (size_t)hidden * 4 > 48 * 1024) return cudaErrorInvalidValue;
@@ -830,6 +1012,8 @@ cudaError_t resid_tail_launch(const ResidTail& a, int T, int hidden, cudaStream_
   if (a.w_pre2 != nullptr && (a.w_pre == nullptr || a.out2 == nullptr)) return cudaErrorInvalidValue;
   const bool vec = hidden % 4 == 0 && al16(a.extra) && al16(a.w_pre2) && al16(a.out2) && al16(a.y_main) && al16(a.y_rows) && al16(a.y_side) && al16(a.resid) && al16(a.w_post) && al16(a.w_dot) &&
                    al16(a.w_pre) && al16(a.out) && al16(a.y_pair) && al16(a.w_main) && al16(a.w_pair);
+  if (vec && hidden <= 1024 && T <= RESID_ROWS) return launch_k(resid_tail_row_kernel<1>, dim3(T), dim3(NORM_THREADS), 0, stream, a, hidden);
+  if (vec && hidden <= 2048 && T <= RESID_ROWS) return launch_k(resid_tail_row_kernel<2>, dim3(T), dim3(NORM_THREADS), 0, stream, a, hidden);
   if (vec) return launch_k(resid_tail_kernel<4>, dim3(T), dim3(NORM_THREADS), (size_t)hidden * sizeof(float), stream, a, hidden);
   return launch_k(resid_tail_kernel<1>, dim3(T), dim3(NORM_THREADS), (size_t)hidden * sizeof(float), stream, a, hidden);
 }
