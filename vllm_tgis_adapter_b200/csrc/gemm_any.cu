@@ -466,10 +466,15 @@ __global__ void __launch_bounds__(ANY_THREADS) gemm_any_rowdot_kernel(GemmAny a)
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) reinterpret_cast<float*>(a.Y)[(size_t)t * a.ldy + n] = acc;
+  if (lane == 0) {
+    if (a.mode == GEMM_ANY_TANH) acc = tanhf(acc);
+    if (a.y_dtype == DT_BF16) reinterpret_cast<__nv_bfloat16*>(a.Y)[(size_t)t * a.ldy + n] = __float2bfloat16_rn(acc);
+    else reinterpret_cast<float*>(a.Y)[(size_t)t * a.ldy + n] = acc;
+  }
 }
 bool rowdot_eligible(const GemmAny& a) {
-  return a.seg_off == nullptr && a.batch <= 1 && a.mode == GEMM_ANY_PLAIN && a.y_dtype == DT_F32 && a.N < 128 &&
+  // (with a tanh: the low-rank decay map of a step, 32 x 64 x 2048: one tile of the mma.sync kernel takes 38 us, this 3.7)
+  return a.seg_off == nullptr && a.batch <= 1 && (a.mode == GEMM_ANY_TANH || (a.mode == GEMM_ANY_PLAIN && a.y_dtype == DT_F32)) && a.N < 128 &&
          (long long)a.T * a.N <= 8192 && a.K >= 256 && !(a.x_dtype == DT_BF16 && a.w_dtype == DT_F32);
 }
 template <class XT, class WT, bool VEC8 = false>
@@ -498,7 +503,9 @@ cudaError_t launch_fma(const GemmAny& a, cudaStream_t stream) {
   const int rows = a.seg_off != nullptr ? (a.T + a.n_groups - 1) / (a.n_groups > 0 ? a.n_groups : 1) : a.T;
   const long long tiles64 = (long long)((a.N + FMA_BN - 1) / FMA_BN) * (a.batch > 0 ? a.batch : 1) *
                             (a.seg_off != nullptr ? (long long)a.n_groups * ((rows + 63) / 64) : (a.T + 63) / 64);
-  if (rows <= 20) return launch_fma_bm<XT, WT, OT, 16>(a, vec, stream);
+  // (16 rows too where 32 would leave half of the SMs without a tile and K is short: 32 x 4096 x 128 13.6 -> 7.4 us)
+  const long long tiles32 = (long long)((a.N + FMA_BN - 1) / FMA_BN) * (a.batch > 0 ? a.batch : 1) * ((rows + 31) / 32);
+  if (rows <= 20 || (a.seg_off == nullptr && a.K <= 256 && 2 * tiles32 <= FMA_SMS)) return launch_fma_bm<XT, WT, OT, 16>(a, vec, stream);
   const bool fit32 = (a.T + 31ll) / 32 + (a.seg_off != nullptr ? a.n_groups : 0) <= 65535;   // tiles of one launch (grid.y)
   if (fit32 && (rows <= 36 || tiles64 < 3 * FMA_SMS || a.K <= 256)) return launch_fma_bm<XT, WT, OT, 32>(a, vec, stream);
   return launch_fma_bm<XT, WT, OT, 64>(a, vec, stream);
@@ -523,6 +530,7 @@ cudaError_t gemm_any_launch(const GemmAny& a, cudaStream_t stream) {
   // expert segments: CTA pairs.  64 experts of 2 x 1408 x 2048 and back, top 6, both products in microseconds, mma.sync -> pairs:
   // 4 tokens 126 -> 78, 32 tokens 260 -> 165 (6.3 TB/s of weights), 512 tokens 334 -> 195, 2048 tokens 1003 -> 243
   if (gemm_pair_takes_groups(a)) return gemm_pair_grouped_launch(a, stream);
+  if (mma_eligible(a) && gemm_skinny_takes_batch(a)) return gemm_skinny_batch_launch(a, stream);
   if (mma_eligible(a)) return a.y_dtype == DT_BF16 ? launch_mma<bf>(a, stream) : launch_mma<float>(a, stream);
   const int key = a.x_dtype * 4 + a.w_dtype * 2 + a.y_dtype;  // DT_F32 = 0, DT_BF16 = 1
   switch (key) {

@@ -19,8 +19,11 @@ namespace {
 
 struct SkinnyArgs {
   const __nv_bfloat16* X; const __nv_bfloat16* W; void* Y;
-  int ldy, T, N, K, mode;   // mode: the out modes of gemm_bf16_launch
-  GemmRope rope;            // positions == nullptr: none
+  int ldx, ldy, T, N, K, mode;   // mode: the out modes of gemm_bf16_launch
+  GemmRope rope;                 // positions == nullptr: none
+  long long x_bs, w_bs, y_bs;    // elements between the problems of blockIdx.y
+  const float* row_scale;        // modes 0 and 1: result times row_scale[token * scale_ld + problem] (nullptr: 1)
+  int scale_ld;
 };
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -50,9 +53,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_k
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = ROPE ? (blockIdx.x >> 2) * HEAD_DIM + (blockIdx.x & 3) * 16 : blockIdx.x * R;
   constexpr int M_STEP = ROPE ? 64 : 16;
+  const __nv_bfloat16* X = a.X + (size_t)blockIdx.y * a.x_bs;
+  const __nv_bfloat16* W = a.W + (size_t)blockIdx.y * a.w_bs;
   if (threadIdx.x < MT) {   // weights are static: the CTA's rows (one run of bytes per tile) start on their way to L2
     const int row = n0 + (int)threadIdx.x * M_STEP, bytes = min(16, a.N - row) * a.K * 2;
-    const char* from = reinterpret_cast<const char*>(a.W + (size_t)row * a.K);
+    const char* from = reinterpret_cast<const char*>(W + (size_t)row * a.K);
     for (int off = 0; off < bytes; off += 65536)
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(from + off), "r"(min(bytes - off, 65536)) : "memory");
   }
@@ -62,10 +67,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_k
 #pragma unroll
   for (int m = 0; m < MT; ++m)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) wr[m][h] = a.W + (size_t)min(n0 + m * M_STEP + h * 8 + g, a.N - 1) * a.K + t * 8;
+    for (int h = 0; h < 2; ++h) wr[m][h] = W + (size_t)min(n0 + m * M_STEP + h * 8 + g, a.N - 1) * a.K + t * 8;
   const __nv_bfloat16* xr[NT];
 #pragma unroll
-  for (int n = 0; n < NT; ++n) xr[n] = a.X + (size_t)min(n * 8 + g, a.T - 1) * a.K + t * 8;
+  for (int n = 0; n < NT; ++n) xr[n] = X + (size_t)min(n * 8 + g, a.T - 1) * a.ldx + t * 8;
   float acc[MT][NT][4];
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -162,7 +167,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_k
       const int tok = i / R, j = i % R;
       if (n0 + j >= a.N) continue;
       float v = sum(tok, j);
-      const size_t o = (size_t)tok * a.ldy + n0 + j;
+      if (a.row_scale != nullptr) v *= a.row_scale[(size_t)tok * a.scale_ld + blockIdx.y];
+      const size_t o = (size_t)blockIdx.y * a.y_bs + (size_t)tok * a.ldy + n0 + j;
       if (a.mode == 1) {
         reinterpret_cast<float*>(a.Y)[o] = v;
       } else {
@@ -177,20 +183,20 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_k
 }
 
 template <int MT, int NT, int WARPS, bool ROPE>
-cudaError_t launch(const SkinnyArgs& a, cudaStream_t s) {
+cudaError_t launch(const SkinnyArgs& a, cudaStream_t s, int problems = 1) {
   constexpr size_t smem = (size_t)WARPS * 8 * NT * (16 * MT + 1) * sizeof(float);
   static const cudaError_t attr =
       cudaFuncSetAttribute(gemm_skinny_kernel<MT, NT, WARPS, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (attr != cudaSuccess) return attr;
-  return launch_k(gemm_skinny_kernel<MT, NT, WARPS, ROPE>, dim3((a.N + 16 * MT - 1) / (16 * MT)), dim3(WARPS * 32), smem, s, a);
+  return launch_k(gemm_skinny_kernel<MT, NT, WARPS, ROPE>, dim3((a.N + 16 * MT - 1) / (16 * MT), problems), dim3(WARPS * 32), smem, s, a);
 }
 template <int MT, int WARPS, bool ROPE>
-cudaError_t launch_nt(const SkinnyArgs& a, cudaStream_t s) {
+cudaError_t launch_nt(const SkinnyArgs& a, cudaStream_t s, int problems = 1) {
   switch ((a.T + 7) / 8) {
-    case 1: return launch<MT, 1, WARPS, ROPE>(a, s);
-    case 2: return launch<MT, 2, WARPS, ROPE>(a, s);
-    case 3: return launch<MT, 3, WARPS, ROPE>(a, s);
-    default: return launch<MT, 4, WARPS, ROPE>(a, s);
+    case 1: return launch<MT, 1, WARPS, ROPE>(a, s, problems);
+    case 2: return launch<MT, 2, WARPS, ROPE>(a, s, problems);
+    case 3: return launch<MT, 3, WARPS, ROPE>(a, s, problems);
+    default: return launch<MT, 4, WARPS, ROPE>(a, s, problems);
   }
 }
 
@@ -208,7 +214,7 @@ bool gemm_skinny_takes(int T, int N, int K) {
 
 cudaError_t gemm_skinny_launch(const void* X, const void* W, void* Y, int ldy, int T, int N, int K, int out_mode, const GemmRope* rope,
                                cudaStream_t stream) {
-  SkinnyArgs a{(const __nv_bfloat16*)X, (const __nv_bfloat16*)W, Y, ldy, T, N, K, out_mode, {}};
+  SkinnyArgs a{(const __nv_bfloat16*)X, (const __nv_bfloat16*)W, Y, K, ldy, T, N, K, out_mode, {}, 0, 0, 0, nullptr, 0};
   // The number of warps, and with it the order of k, hangs on N alone: a row has the same bits beside 31 others as alone, and with
   // every epilogue.  Sixteen warps where an SM holds one CTA, of 16 rows up to one wave, of 32 rows up to two; eight beyond that,
   // with 32-row CTAs for few tokens (more loads in flight) and 16-row ones beyond eight (fewer activation bytes in flight per
@@ -222,6 +228,22 @@ cudaError_t gemm_skinny_launch(const void* X, const void* W, void* Y, int ldy, i
   }
   if (!sixteen) return T <= 8 ? launch<2, 1, 8, false>(a, stream) : launch_nt<1, 8, false>(a, stream);
   return N > SKINNY_ONE_WAVE ? launch_nt<2, 16, false>(a, stream) : launch_nt<1, 16, false>(a, stream);
+}
+
+// One product per head (the up-projections that latent attention folds into queries and outputs), up to 32 tokens: grid (16 weight
+// rows, problem), four warps up to 256 k, eight beyond.  32 tokens, 16 heads, microseconds, mma.sync tiles of 64 x 128 -> here:
+// 512 x 128 9.4 -> 4.4, 128 x 512 (16 tiles in all) 15.5 -> 3.7.
+bool gemm_skinny_takes_batch(const GemmAny& a) {
+  auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  return a.batch > 1 && a.batch <= 65535 && a.seg_off == nullptr && a.gather == nullptr && a.x_dtype == DT_BF16 && a.w_dtype == DT_BF16 &&
+         (a.mode == GEMM_ANY_PLAIN || a.mode == GEMM_ANY_ROWSCALE) && gemm_skinny_takes(a.T, a.N, a.K) &&
+         (long long)a.batch * a.N * a.K <= (a.T <= 8 ? 17000000 : 4500000) && a.ldw == a.K && a.ldx >= a.K && a.ldx % 8 == 0 &&
+         a.x_bs % 8 == 0 && a.w_bs % 8 == 0 && al16(a.X) && al16(a.W);
+}
+cudaError_t gemm_skinny_batch_launch(const GemmAny& g, cudaStream_t stream) {
+  SkinnyArgs a{(const __nv_bfloat16*)g.X, (const __nv_bfloat16*)g.W, g.Y, g.ldx, g.ldy, g.T, g.N, g.K, g.y_dtype == DT_F32 ? 1 : 0, {},
+               g.x_bs, g.w_bs, g.y_bs, g.mode == GEMM_ANY_ROWSCALE ? g.row_scale : nullptr, g.scale_ld};
+  return g.K <= 256 ? launch_nt<1, 4, false>(a, stream, g.batch) : launch_nt<1, 8, false>(a, stream, g.batch);
 }
 
 }  // namespace tgis
