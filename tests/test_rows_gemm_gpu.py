@@ -1,0 +1,53 @@
+"""Products of 17 to 256 tokens in equal shares of weight rows, and on CTA pairs from 129 (csrc/gemm_pair.cu): rows that no share
+divides, one wave and two, one and two k-blocks to a barrier, token counts around the 32-token unit and the limits of the rules, every
+epilogue, the rotary embedding behind them, and nothing written outside Y."""
+import ctypes as C
+
+import pytest
+import torch
+
+from tests.test_pair_gemm_gpu import GEGLU, PLAIN, PLAIN_F32, RELU2, SWIGLU, test_pair_products as check
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from vllm_tgis_adapter_b200.engine._lib import load_library
+
+    return load_library()
+
+
+@pytest.mark.parametrize("mode", [PLAIN, PLAIN_F32, SWIGLU, GEGLU, RELU2])
+@pytest.mark.parametrize("T,N,K", [(17, 5920, 64), (32, 6144, 128), (33, 10256, 192), (48, 8192, 320), (49, 6002, 2112), (64, 18944, 256), (65, 592, 64),
+                                   (96, 1184, 320), (100, 19000, 128), (128, 4096, 4096), (129, 18946, 192), (130, 520, 512), (200, 40000, 64),
+                                   (255, 8190, 320), (256, 37890, 128), (256, 2048, 1088)])
+def test_products(lib, T, N, K, mode):
+    check(lib, T, N, K, mode)
+
+
+def p(t):
+    return C.c_void_p(t.data_ptr())
+
+
+@pytest.mark.parametrize("T,n_q,n_kv,K", [(17, 32, 8, 512), (32, 8, 32, 768), (100, 32, 8, 512), (160, 32, 8, 512), (256, 32, 8, 512)])
+def test_rotary_embedding_behind_the_product(lib, T, n_q, n_kv, K):
+    """What the product and the rope kernel do one after the other, bit for bit, and the cache written for tokens with a slot only."""
+    N, blocks = (n_q + 2 * n_kv) * 128, -(-T // 32) + 1
+    gen = torch.Generator(device="cuda").manual_seed(T + n_q)
+    x = torch.randn(256, K, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(N, K, generator=gen, device="cuda") * 0.05).bfloat16()
+    cs = torch.randn(64, 128, generator=gen, device="cuda").bfloat16()
+    pos = (C.c_int32 * T)(*[(7 * i) % 64 for i in range(T)])
+    slots = (C.c_int32 * T)(*[-1 if i % 5 == 4 else T + 31 - i for i in range(T)])
+    caches = [[torch.full((blocks, n_kv, 32 * 128), 3.0, device="cuda").bfloat16() for _ in range(2)] for _ in range(2)]
+    y, ms = [torch.empty(256, N, device="cuda", dtype=torch.bfloat16) for _ in range(2)], C.c_float()
+    rc = lib.tgis_k_gemm_rope(p(x), p(w), p(y[0]), T, n_q, n_kv, K, 256, pos, slots, p(cs), p(caches[0][0]), p(caches[0][1]))
+    if rc == 1:
+        pytest.skip("this shape does not fuse")
+    assert rc == 0
+    assert lib.tgis_k_gemm(p(x), p(w), p(y[1]), T, N, K, 256, 0, 1, C.byref(ms), 0) == 0
+    assert lib.tgis_k_rope_kv(p(y[1]), pos, slots, p(cs), p(caches[1][0]), p(caches[1][1]), T, n_q, n_kv) == 0
+    assert torch.equal(y[0][:T], y[1][:T])
+    for a, b in zip(*caches):
+        assert torch.equal(a, b)

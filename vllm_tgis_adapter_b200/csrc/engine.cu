@@ -3276,7 +3276,9 @@ struct tgis_engine {
       return g;
     };
     if (lora) ++lora_steps;
-    const bool rope_fused = !pnx_on && !lora && fuse_rope && !cfg.debug_gemm_ref && gemm_even_split(T, qkv_dim, H, num_sms) >= 2 &&
+    // (the products that are ahead of the one cut along k, by more than the rotary kernel takes, have no fused form)
+    const bool rope_fused = !pnx_on && !lora && fuse_rope && !cfg.debug_gemm_ref && !gemm_rows_takes(T, qkv_dim, H, num_sms) &&
+                            !gemm_small_pairs(T, H) && gemm_even_split(T, qkv_dim, H, num_sms) >= 2 &&
                             T <= (qkv_cluster > 0 ? std::max(rope_fuse_max_t, rope_fuse_cluster_max_t) : rope_fuse_max_t);
     // residual add + RMSNorm inside the GEMMs either side of it (single GPU, small steps, both row-"producers" reduced
     // on chip): o-proj -> [post-attention norm] -> gate_up and down-proj -> [next layer's input norm] -> qkv

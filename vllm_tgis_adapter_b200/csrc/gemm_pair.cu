@@ -22,6 +22,7 @@
 // buffered accumulator (2 x 256 columns).  The leader's `full` barrier counts both CTAs' bytes; tcgen05.commit releases a
 // ring slot in both CTAs at once.  No wait is unbounded: after about two seconds a role gives up, raises the host-visible
 // error word and leaves; copies and MMAs that are still in flight land first, and TMEM is freed on every path.
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -199,6 +200,7 @@ __device__ __forceinline__ void pair_store(const PairArgs& a, const PairTile& t,
         const float got = __shfl_xor_sync(0xffffffffu, __uint_as_float(odd ? r[2 * j] : r[2 * j + 1]), 1);
         g[j] = odd ? got : __uint_as_float(r[2 * j]);
         u[j] = odd ? __uint_as_float(r[2 * j + 1]) : got;
+        if (!n_ok) g[j] = 0.f;   // (whatever such a row holds does not send the warp into a division)
       }
       if constexpr (MODE == PAIR_SWIGLU_BF16) {   // the rounding points of a bf16 gate / up product followed by silu and a product
 #pragma unroll
@@ -353,43 +355,38 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
     }
   } else if (warp == 1) {
     // ===================== MMA issuer (leader) =====================
-    if (rank == 0) {
+    if (rank == 0 && elect_one()) {
       PairIter<GROUPED> it(a, seg_start, pair, pairs);
       PairTile t;
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
-      while (ok && it.next(t)) {
+      while (ok && it.next(t)) {   // (one thread: 257 tokens x 4096 x 14336 56.3 us with a warp's votes at every k-block, 54.1 without)
         const uint32_t idesc = make_idesc_bf16(256, (uint32_t)t.n);
-        ok = __all_sync(0xffffffffu, pair_wait(&tmem_empty[acc], acc_phase ^ 1, a.err));
-        if (!ok) break;
+        if (!(ok = pair_wait(&tmem_empty[acc], acc_phase ^ 1, a.err))) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * 256;
         for (int kb = 0; kb < KB; ++kb) {
-          ok = __all_sync(0xffffffffu, pair_wait(&full_bar[stage], phase, a.err));
-          if (!ok) break;
+          if (!(ok = pair_wait(&full_bar[stage], phase, a.err))) break;
           tc_fence_after();
-          if (elect_one()) {
-            const uint64_t a_desc = make_smem_desc_sw128(smem_u32(smem_w + stage * PAIR_TILE_BYTES));
-            const uint64_t b_desc = make_smem_desc_sw128(smem_u32(smem_x + stage * PAIR_TILE_BYTES));
+          const uint64_t a_desc = make_smem_desc_sw128(smem_u32(smem_w + stage * PAIR_TILE_BYTES));
+          const uint64_t b_desc = make_smem_desc_sw128(smem_u32(smem_x + stage * PAIR_TILE_BYTES));
 #pragma unroll
-            for (int k = 0; k < PAIR_BK / 16; ++k)
-              mma_pair(d_tmem, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-            commit_pair(&empty_bar[stage]);
-            if (kb == KB - 1) commit_pair(&tmem_full[acc]);
-          }
-          __syncwarp();
+          for (int k = 0; k < PAIR_BK / 16; ++k)
+            mma_pair(d_tmem, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          commit_pair(&empty_bar[stage]);
           if (++stage == PAIR_STAGES) {
             stage = 0;
             phase ^= 1;
           }
         }
+        if (ok) commit_pair(&tmem_full[acc]);
         if (++acc == 2) {
           acc = 0;
           acc_phase ^= 1;
         }
       }
-      if (!ok && lane == 0) *gave_up = 1;
+      if (!ok) *gave_up = 1;
     }
   } else {
     // ===================== epilogue (both CTAs): lane = weight row, column = token =====================
@@ -441,6 +438,188 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   }
 }
 
+// ---------------------------------------------------------------- few tokens: equal shares of weight rows
+// A product of up to 256 tokens is bound by its weight bytes, so what counts is that every SM streams the same number of them from
+// the first microsecond to the last.  Here a pair's tile has as many rows as make the tiles fill whole waves of pairs (2 R, R even,
+// up to 128 a CTA): a CTA loads exactly its R rows, the MMA's other rows read what happens to lie behind them in shared memory and
+// go nowhere.  No tile is split along k, so nothing is reduced between CTAs and an output is one sum in ascending k.  Each
+// CTA loads half of the tokens, R + n / 2 rows a k-block; gemm_rows_takes says where that is less than what a split along k costs.
+// One thread issues all MMAs and a barrier covers two k-blocks: with few tokens a k-block takes no longer than a warp's votes and a
+// commit (28672 x 4096 in bf16, 96 tokens, 46 us; 10256 x 2048 15.4 us with a k-block to a barrier, 12.9 with two).  What bounds it
+// now: 22528 x 2048 streams its weights at 4.9 TB/s of a launch's 19 us, of which 4 are its start and its end; shares of fewer
+// than some 56 rows wait for the 0.16 us that a k-block's MMAs take.
+constexpr int ROWS_MAX_STAGES = 24;
+constexpr int ROWS_RING = 200 * 1024;
+constexpr int ROWS_BAR_BYTES = 512;
+constexpr int ROWS_SMEM = ROWS_RING + PAIR_TILE_BYTES + 1024 + ROWS_BAR_BYTES;   // (the last stage's MMA reads 128 rows as well)
+struct RowsArgs {
+  PairArgs p;
+  int R, n, tiles;                  // weight rows of a CTA's share of a tile, UMMA_N, tiles
+  int stages, ksub, w_bytes, x_bytes;   // ring; k-blocks of a stage; bytes of one k-block's operands in it (whole 8-row groups)
+};
+__device__ __forceinline__ void tma_load_pair_hint(const CUtensorMap* m, uint32_t bar, void* dst, int c0, int c1, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes.L2::cache_hint"
+      " [%0], [%1, {%3, %4}], [%2], %5;\n" ::"r"(smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(m)), "r"(bar), "r"(c0), "r"(c1), "l"(policy)
+      : "memory");
+}
+
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
+gemm_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ RowsArgs ra) {
+  extern __shared__ uint8_t smem_raw[];
+  const PairArgs& a = ra.p;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + ROWS_RING + PAIR_TILE_BYTES);
+  uint64_t* empty_bar = full_bar + ROWS_MAX_STAGES;
+  uint64_t* tmem_full = empty_bar + ROWS_MAX_STAGES;
+  uint64_t* tmem_empty = tmem_full + 2;
+  uint32_t* tmem_base_smem = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_base_smem + 1);
+
+  const int warp = threadIdx.x >> 5, lane = (int)lane_id();
+  const int rank = (int)cluster_ctarank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int sub_bytes = ra.w_bytes + ra.x_bytes, stage_bytes = ra.ksub * sub_bytes, KS = a.K / (PAIR_BK * ra.ksub);
+
+  if (warp == 0 && elect_one()) {
+    tma_prefetch_desc(&wmap);
+    tma_prefetch_desc(&xmap);
+  }
+  if (warp == 1) {
+    if (elect_one()) {
+      for (int i = 0; i < ra.stages; ++i) {
+        mbar_init(&full_bar[i], 1);
+        mbar_init(&empty_bar[i], 1);
+      }
+      for (int i = 0; i < 2; ++i) {
+        mbar_init(&tmem_full[i], 1);
+        mbar_init(&tmem_empty[i], 8);
+      }
+      *gave_up = 0;
+      fence_barrier_init();
+    }
+    __syncwarp();
+    tmem_alloc_pair<512>(tmem_base_smem);
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();   // the peer's barriers exist
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_base_smem;
+  griddep_launch();
+
+  if (warp == 0) {
+    // ===================== TMA producer (both CTAs) =====================
+    if (elect_one()) {
+      const uint32_t full0 = dsmem_addr(smem_u32(full_bar), 0);   // the leader's barriers
+      const uint32_t bytes = 2u * (uint32_t)(ra.ksub * (ra.R + ra.n / 2) * PAIR_BK * 2);
+      const uint64_t once = policy_evict_first();
+      const int x_row = rank * (ra.n / 2);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      auto load_w = [&](int s, int ks, int w_row) {
+        if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], bytes);
+        for (int j = 0; j < ra.ksub; ++j)
+          tma_load_pair_hint(&wmap, full0 + s * 8, smem + s * stage_bytes + j * sub_bytes, (ks * ra.ksub + j) * PAIR_BK, w_row, once);
+      };
+      auto load_x = [&](int s, int ks) {
+        for (int j = 0; j < ra.ksub; ++j)
+          tma_load_pair(&xmap, full0 + s * 8, smem + s * stage_bytes + j * sub_bytes + ra.w_bytes, (ks * ra.ksub + j) * PAIR_BK, x_row);
+      };
+      // weights are static: the first ring of them is requested before the previous kernel has finished
+      const int pre = pair < ra.tiles ? min(KS, ra.stages) : 0;
+      for (int ks = 0; ks < pre; ++ks) load_w(ks, ks, (pair * 2 + rank) * ra.R);
+      griddep_wait();
+      for (int ks = 0; ks < pre; ++ks) load_x(ks, ks);
+      stage = pre % ra.stages;
+      phase = pre == ra.stages ? 1 : 0;
+      for (int t = pair, first = pre; t < ra.tiles && ok; t += pairs, first = 0) {
+        const int w_row = (t * 2 + rank) * ra.R;
+        for (int ks = first; ks < KS; ++ks) {
+          if (!(ok = pair_wait(&empty_bar[stage], phase ^ 1, a.err))) break;
+          load_w(stage, ks, w_row);
+          load_x(stage, ks);
+          if (++stage == ra.stages) stage = 0, phase ^= 1;
+        }
+      }
+      if (!ok) *gave_up = 1;
+    }
+  } else if (warp == 1) {
+    // ===================== MMA issuer (leader) =====================
+    if (rank == 0 && elect_one()) {   // (one thread from end to end: with few tokens a stage takes no longer than a warp's votes)
+      int stage = 0, acc = 0;
+      uint32_t phase = 0, acc_phase = 0;
+      bool ok = true;
+      const uint32_t idesc = make_idesc_bf16(256, (uint32_t)ra.n), ring = smem_u32(smem);
+      for (int t = pair; t < ra.tiles && ok; t += pairs) {
+        if (!(ok = pair_wait(&tmem_empty[acc], acc_phase ^ 1, a.err))) break;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * 256;
+        for (int ks = 0; ks < KS; ++ks) {
+          if (!(ok = pair_wait(&full_bar[stage], phase, a.err))) break;
+          tc_fence_after();
+          for (int j = 0; j < ra.ksub; ++j) {
+            const uint32_t at = ring + stage * stage_bytes + j * sub_bytes;
+            const uint64_t a_desc = make_smem_desc_sw128(at), b_desc = make_smem_desc_sw128(at + ra.w_bytes);
+#pragma unroll
+            for (int k = 0; k < PAIR_BK / 16; ++k)
+              mma_pair(d_tmem, a_desc + (uint64_t)(k * 2), b_desc + (uint64_t)(k * 2), idesc, (ks > 0 || j > 0 || k > 0) ? 1u : 0u);
+          }
+          commit_pair(&empty_bar[stage]);
+          if (++stage == ra.stages) stage = 0, phase ^= 1;
+        }
+        if (ok) commit_pair(&tmem_full[acc]);
+        if (++acc == 2) acc = 0, acc_phase ^= 1;
+      }
+      if (!ok) *gave_up = 1;
+    }
+  } else {
+    // ===================== epilogue (both CTAs): lane = weight row, column = token =====================
+    const int sub = warp & 3, row = sub * 32 + lane;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    griddep_wait();   // Y may still be in use by the previous kernels
+    for (int t = pair; t < ra.tiles; t += pairs) {
+      if (!__all_sync(0xffffffffu, pair_wait(&tmem_full[acc], acc_phase, a.err))) {
+        if (lane == 0) *gave_up = 1;
+        break;
+      }
+      tc_fence_after();
+      if (sub * 32 < ra.R) {
+        PairTile pt;
+        pt.n0 = 0; pt.w_row = 0;
+        pt.row0 = 0; pt.rows = a.T; pt.n = ra.n;
+        const int n = row < ra.R ? (t * 2 + rank) * ra.R + row : a.N;
+        const uint32_t taddr = tmem_base + acc * 256 + ((uint32_t)(sub * 32) << 16);
+        using bf = __nv_bfloat16;
+        switch (a.mode) {
+          case PAIR_SWIGLU_BF16: pair_store<PAIR_SWIGLU_BF16, bf>(a, pt, n, taddr, lane); break;
+          case PAIR_GEGLU: pair_store<PAIR_GEGLU, bf>(a, pt, n, taddr, lane); break;
+          case PAIR_RELU2: pair_store<PAIR_RELU2, bf>(a, pt, n, taddr, lane); break;
+          default:
+            if (a.y_f32) pair_store<PAIR_PLAIN, float>(a, pt, n, taddr, lane);
+            else pair_store<PAIR_PLAIN, bf>(a, pt, n, taddr, lane);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(dsmem_addr(smem_u32(&tmem_empty[acc]), 0));
+      if (++acc == 2) acc = 0, acc_phase ^= 1;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (*gave_up)   // as in gemm_pair_kernel
+    for (const long long t0 = clock64(); clock64() - t0 < 2000000ll;) {}
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair<512>(tmem_base);
+  }
+}
+
 // host-visible error word, one for the process (a raised word is an error of the process's device, as a sticky CUDA error is).
 // Pinned memory cannot be had while a stream is being captured, so an engine has it made before its first step
 // (gemm_pair_prepare); a refusal is not remembered.
@@ -459,16 +638,23 @@ cudaError_t make_pair_word() {
 
 std::atomic<int> pair_launches{0}, pair_fault_in{0};   // gemm_pair_fault
 
+// the error word for one launch (and the host's stand-in for a wait of it that runs out, gemm_pair_fault)
+cudaError_t claim_pair_word(int*& err) {
+  const cudaError_t word = gemm_pair_prepare();
+  if (word != cudaSuccess) return word;
+  err = pair_word.load(std::memory_order_acquire);
+  pair_launches.fetch_add(1, std::memory_order_relaxed);
+  if (pair_fault_in.load(std::memory_order_relaxed) > 0 && pair_fault_in.fetch_sub(1) == 1) *reinterpret_cast<volatile int*>(err) = 1;
+  return cudaSuccess;
+}
+
 template <bool GROUPED>
 cudaError_t launch_pair(const CUtensorMap& wmap, const CUtensorMap& xmap, PairArgs a, int grid, cudaStream_t stream) {
   static const cudaError_t attr =
       cudaFuncSetAttribute(gemm_pair_kernel<GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem(GROUPED));
   if (attr != cudaSuccess) return attr;
-  const cudaError_t word = gemm_pair_prepare();
+  const cudaError_t word = claim_pair_word(a.err);
   if (word != cudaSuccess) return word;
-  a.err = pair_word.load(std::memory_order_acquire);
-  pair_launches.fetch_add(1, std::memory_order_relaxed);
-  if (pair_fault_in.load(std::memory_order_relaxed) > 0 && pair_fault_in.fetch_sub(1) == 1) *reinterpret_cast<volatile int*>(a.err) = 1;
   return launch_k_cluster(gemm_pair_kernel<GROUPED>, dim3(grid), dim3(PAIR_THREADS), pair_smem(GROUPED), stream, 2, wmap, xmap, a);
 }
 
@@ -525,6 +711,46 @@ cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
   a.x_tiles = gemm_pair_plan(T, N, pairs);
   const int tiles = a.n_tiles * a.x_tiles;
   return launch_pair<false>(wmap, xmap, a, 2 * (tiles < pairs ? tiles : pairs), stream);
+}
+
+// The share of a product of N weight rows that one CTA of a pair takes: whole waves of pairs, an even number of rows
+static int rows_share(int N, int pairs) {
+  const int waves = (N + 256 * pairs - 1) / (256 * pairs), per = (N + 2 * pairs * waves - 1) / (2 * pairs * waves);
+  return (per + 1) & ~1;
+}
+// At least 40 rows a CTA up to 64 tokens, eight from there (fewer rows: the cut along k or the pairs' token tiles are ahead); beyond 128
+// tokens only where the rows fill more than one wave; a long k only where its bytes take longer than its MMAs.  The measured
+// table stands at gemm_takes_pairs.
+bool gemm_rows_takes(int T, int N, int K, int num_sms) {
+  if (T <= 16 || T > 256 || K % PAIR_BK != 0 || num_sms < 2) return false;
+  const int pairs = num_sms / 2, R = rows_share(N, pairs);
+  if (R < 56 && K > 4096) return false;
+  if (T <= 48 && K > 2048) return false;   // (in a chain of kernels the cut along k is ahead there: its ring is under way sooner)
+  return T <= 128 ? R >= 40 || (T > 64 && N >= 8 * pairs) : N > 256 * pairs;
+}
+cudaError_t gemm_rows_launch(const void* X, const void* W, void* Y, int ldy, int y_f32, int mode, int T, int N, int K, int num_sms,
+                             cudaStream_t stream) {
+  if (!gemm_rows_takes(T, N, K, num_sms) || (y_f32 && mode != PAIR_PLAIN)) return cudaErrorInvalidValue;
+  const int pairs = num_sms / 2;
+  RowsArgs ra{};
+  PairArgs& a = ra.p;
+  a.Y = Y; a.ldy = ldy; a.T = T; a.N = N; a.K = K;
+  a.y_f32 = y_f32; a.mode = mode;
+  ra.R = rows_share(N, pairs);
+  ra.n = (T + PAIR_UNIT - 1) / PAIR_UNIT * PAIR_UNIT;
+  ra.tiles = (N + 2 * ra.R - 1) / (2 * ra.R);
+  ra.w_bytes = (ra.R + 7) / 8 * 1024;
+  ra.x_bytes = ra.n / 2 * PAIR_BK * 2;
+  ra.ksub = K % (2 * PAIR_BK) == 0 ? 2 : 1;   // (a barrier costs the issuing thread as much as two k-blocks of few tokens)
+  ra.stages = std::min(ROWS_RING / (ra.ksub * (ra.w_bytes + ra.x_bytes)), ROWS_MAX_STAGES);
+  CUtensorMap wm, xm;
+  if (make_tmap_bf16_2d(&wm, W, N, K, K, ra.R, PAIR_BK) != 0 || make_tmap_bf16_2d(&xm, X, T, K, K, ra.n / 2, PAIR_BK) != 0)
+    return cudaErrorInvalidValue;
+  static const cudaError_t attr = cudaFuncSetAttribute(gemm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ROWS_SMEM);
+  if (attr != cudaSuccess) return attr;
+  const cudaError_t word = claim_pair_word(a.err);
+  if (word != cudaSuccess) return word;
+  return launch_k_cluster(gemm_rows_kernel, dim3(2 * std::min(ra.tiles, pairs)), dim3(PAIR_THREADS), ROWS_SMEM, stream, 2, wm, xm, ra);
 }
 
 // X rows of a grouped product in segment order: out[p] = X[gather[p] / div], p < seg_off[n_groups]

@@ -1187,6 +1187,10 @@ static cudaError_t launch_bt(const CUtensorMap& wmap, const CUtensorMap& xmap, v
                   ldy, T, N, K, ws, counters, stream_weights, out_f32, next_wmap, nxt, 0, rope, norm);
 }
 
+static int pair_mode(int out_mode) {   // 0 .. 4
+  static const int modes[5] = {PAIR_PLAIN, PAIR_PLAIN, PAIR_SWIGLU_BF16, PAIR_GEGLU, PAIR_RELU2};
+  return modes[out_mode];
+}
 // xmap must have been built with box_rows == gemm_x_box(T, N, num_sms)
 cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int T, int N, int K,
                              float* ws, int* counters, int num_sms, cudaStream_t stream, int out_f32,
@@ -1196,6 +1200,19 @@ cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
       ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) == 0 &&
       (rope == nullptr || (out_f32 == 0 && N == (rope->n_q + 2 * rope->n_kv) * HEAD_DIM)))
     return gemm_skinny_launch(X, W, Y, ldy, T, N, K, out_f32, rope, stream);
+  if (X != nullptr && W != nullptr && norm == nullptr && out_f32 >= 0 && out_f32 <= 4 && K % 64 == 0 && num_sms >= 2 &&
+      ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) == 0 &&
+      (rope == nullptr || (out_f32 == 0 && ldy == N && N == (rope->n_q + 2 * rope->n_kv) * HEAD_DIM))) {
+    cudaError_t e = cudaErrorNotSupported;
+    CUtensorMap xm;
+    if (gemm_rows_takes(T, N, K, num_sms)) e = gemm_rows_launch(X, W, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream);
+    else if (gemm_small_pairs(T, K) && make_tmap_bf16_2d(&xm, X, T, K, K, GEMM_X_BOX_MANY, 64) == 0)
+      e = gemm_pair_launch(wmap, xm, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream);
+    if (e == cudaSuccess && rope != nullptr)   // no fused form of these: the bits of a row are those of the product without it
+      e = rope_kvwrite_launch((__nv_bfloat16*)Y, rope->positions, rope->slot_mapping, rope->cos_sin, rope->k_cache, rope->v_cache, T, rope->n_q,
+                              rope->n_kv, stream);
+    if (e != cudaErrorNotSupported) return e;
+  }
   GemmRope rp{};
   if (rope) rp = *rope;
   GemmNorm nr{};
@@ -1205,8 +1222,7 @@ cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
   const CUtensorMap& nm = (next && next_wmap) ? *next_wmap : wmap;
   if (gemm_takes_pairs(T, N, num_sms)) {
     if (rope != nullptr || norm != nullptr || out_f32 < 0 || out_f32 > 4) return cudaErrorInvalidValue;
-    static const int modes[5] = {PAIR_PLAIN, PAIR_PLAIN, PAIR_SWIGLU_BF16, PAIR_GEGLU, PAIR_RELU2};
-    return gemm_pair_launch(wmap, xmap, Y, ldy, out_f32 == 1, modes[out_f32], T, N, K, num_sms, stream);
+    return gemm_pair_launch(wmap, xmap, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream);
   }
   const int nw = gemm_nw(T);
 #define TGIS_GEMM_CASE(B)                                                                                              \

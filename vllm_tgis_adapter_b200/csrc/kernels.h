@@ -16,13 +16,22 @@ int make_tmap_bf16_3d(CUtensorMap* out, const void* base, const uint64_t (&dims)
                       const uint32_t (&box)[3], bool swizzle128);
 int gemm_pick_bt(int T);
 constexpr int GEMM_X_BOX_MANY = 32;
-// Whether a dense product runs on CTA pairs (gemm_pair.cu): more than 256 tokens always, more than 64 when the weights have more
-// 128-row tiles than half the SMs (fewer are cut along k by the one-CTA kernel, which can also fuse the rotary embedding).
-// Microseconds with cold weights, one CTA -> pairs, at 64, 128 and 256 tokens: 28672 x 4096 (SwiGLU) 59 -> 61, 69 -> 63, 100 -> 69;
-// 128256 x 4096 183 -> 185, 196 -> 189, 257 -> 206; 10248 x 2048 21 -> 14, 28 -> 15, 43 -> 19.
-// The line looks at the rows alone, and between 65 and 256 tokens k decides too.  With fewer rows and little k pairs would be ahead
-// (256 tokens: 2048 x 2048 24 -> 12, 3072 x 1536 23 -> 11, 5632 x 2048 31 -> 17, 6144 x 4096 31 -> 21); where k is long they are
-// behind (4096 x 14336 42 -> 56, 2048 x 11264 29 -> 42).
+// Whether a dense product's maps are those of the CTA pairs (gemm_pair.cu): more than 256 tokens always, more than 64 when the weights
+// have more 128-row tiles than half the SMs (fewer are cut along k by the one-CTA kernel, which can also fuse the rotary embedding).
+// Up to 256 tokens two more forms make maps of their own where the caller names the operands and wants no fused epilogue
+// (gemm_rows_takes, gemm_small_pairs).  Microseconds with cold weights at 32, 64, 96, 128, 192 and 256 tokens, cut along k (from 96
+// tokens on and with many rows: pairs, which went before), pairs, equal shares of rows:
+//   6144 x 4096    17.3 19.7 21.3 22.8 27.9 31.0   18.4 19.0 18.9 19.2 19.4 20.1   15.3 15.7 16.3 18.0 23.5 29.3
+//   4096 x 4096    13.7 15.8 16.8 18.1 21.7 24.1   17.8 18.5 18.2 18.3 18.4 18.5   15.0 15.6 15.8 17.9 23.5 29.2
+//   28672 x 4096   42.0 51.5 52.0 54.4 56.4 63.9   47.8 48.9 50.1 53.9 56.4 62.5   42.4 45.3 46.0 47.8 51.3 61.1
+//   128256 x 4096   164  169  179  181  188  200    168  171  176  178  185  197    159  163  167  170  183  198
+//   10256 x 2048   17.4 21.0 14.4 14.5 15.7 18.4   12.8 13.3 14.1 14.2 15.7 18.3   12.2 12.5 12.9 13.7 16.2 19.5
+//   22528 x 2048   23.1 31.1 26.4 26.9 29.0 32.4   23.3 24.0 25.2 26.1 28.4 31.8   19.1 19.8 20.7 22.4 26.5 32.6
+//   8192 x 2048    13.5 16.0 17.1 18.7 22.8 25.8   12.0 12.4 12.5 12.6 13.2 13.8   11.7 11.8 12.0 12.8 15.6 18.4
+//   2048 x 2048     5.6 11.0 14.9 16.4 20.5 23.5      - 11.3 11.0 11.2 11.2 11.2      - 10.7 10.7 11.7 14.6 17.6
+//   4096 x 14336   26.1 27.9 29.7 31.1 37.6 40.4   49.9 51.0 50.3 51.1 51.4 51.8   37.7 39.8 41.6 45.6 65.2 84.7
+//   2048 x 11264   16.8 18.6 20.5 22.4 26.0 28.4   38.4 39.1 38.3 38.7 38.7 38.6   30.1 31.7 32.8 36.7 51.9 67.1
+// (a k-block takes the tensor cores some 0.16 us however few rows and tokens it has, so long k is for the kernel that cuts it).
 inline bool gemm_takes_pairs(int T, int N, int num_sms) { return T > 256 || (T > 64 && (N + 127) / 128 > num_sms / 2); }
 // rows of one box of the activation map: the token tile, or (pairs) small boxes, of which a tile takes as many as it has rows
 inline int gemm_x_box(int T, int N, int num_sms) { return gemm_takes_pairs(T, N, num_sms) ? GEMM_X_BOX_MANY : gemm_pick_bt(T); }
@@ -92,6 +101,12 @@ constexpr int PAIR_GELU = 5;         // exact gelu
 // wmap: boxes of 128 rows x 64; xmap: boxes of GEMM_X_BOX_MANY rows x 64; Y fp32 (y_f32) or bf16
 cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int y_f32, int mode, int T, int N,
                              int K, int num_sms, cudaStream_t stream);
+// the same for up to 256 tokens in equal shares of weight rows; X [T, K], W [N, K] contiguous
+bool gemm_rows_takes(int T, int N, int K, int num_sms);
+cudaError_t gemm_rows_launch(const void* X, const void* W, void* Y, int ldy, int y_f32, int mode, int T, int N, int K, int num_sms,
+                             cudaStream_t stream);
+// CTA pairs with 129 to 256 tokens where no share of rows is large enough and k is short
+inline bool gemm_small_pairs(int T, int K) { return T > 128 && T <= 256 && K <= 4096; }
 int gemm_pair_plan(int T, int N, int pairs);   // token tiles of the dense launch
 cudaError_t gemm_pair_prepare();               // host memory of the launches: to be called before any of them is captured
 bool gemm_pair_failed();                       // a wait inside a launch of this process ran out
