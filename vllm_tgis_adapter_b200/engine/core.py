@@ -4,6 +4,7 @@ from __future__ import annotations
 import ctypes as C
 import dataclasses
 import importlib
+from array import array
 from typing import Iterable
 
 from . import _lib
@@ -137,6 +138,17 @@ def make_sampling_params(*, greedy: bool = True, temperature: float = 1.0, top_k
     return sp
 
 
+def _int32_array(values):
+    """`values` as a ctypes array.  By way of array(): 2048 entries in 34 us, one by one as ctypes arguments 210."""
+    if type(values) is list and values:
+        try:
+            buf = array("i", values)
+            return (C.c_int32 * len(buf)).from_buffer(buf)
+        except OverflowError:   # (ctypes wraps what does not fit)
+            pass
+    return (C.c_int32 * len(values))(*values)
+
+
 class NativeEngine:
     """Owns one `tgis_engine*`."""
 
@@ -212,7 +224,7 @@ class NativeEngine:
             raise EngineError(_lib.last_error(self.lib))
 
     def add_request(self, request_id: str, prompt_ids: list[int], params: TgisSamplingParams) -> None:
-        arr = (C.c_int32 * len(prompt_ids))(*prompt_ids)
+        arr = _int32_array(prompt_ids)
         if self.lib.tgis_engine_add_request(self._h, request_id.encode(), arr, len(prompt_ids), C.byref(params)) != 0:
             raise EngineError(f"add_request failed: {_lib.last_error(self.lib)}")
 
@@ -267,7 +279,7 @@ class NativeEngine:
         keep = []
         n_want = 0
         for i, (rid, toks, want) in enumerate(entries):
-            t = (C.c_int32 * len(toks))(*toks)
+            t = _int32_array(toks)
             w = (C.c_int32 * max(len(want), 1))(*want)
             keep += [t, w]
             arr[i].request_id = rid.encode()
