@@ -96,6 +96,33 @@ def test_lora_with_swiglu_on_tiles_of_up_to_eight_adapters(g, T, F, K, Rm):
     assert float((y == want).float().mean()) > 0.97
 
 
+@pytest.mark.parametrize("N,Rm,col0", [(504, 8, 0), (512, 24, 8), (520, 16, 64), (1096, 104, 0), (8, 128, 16)])   # around the 512 columns of a CTA; 8 and 24: half a chunk of 16 rank indices
+@pytest.mark.parametrize("T", [1, 15, 16, 17, 33, 300])   # around the 16 tokens of a tile
+def test_lora_on_tiles_of_up_to_sixteen_adapters(g, T, N, Rm, col0):
+    """Every token against its own adapter in 64 bits, tiles of one to sixteen adapters; nothing outside the module's columns changes."""
+    gen = torch.Generator().manual_seed(T + N)
+    slots, K = 16, 128
+    x = torch.randn(T, K, generator=gen).to(torch.bfloat16)
+    ldy = col0 + N + 8
+    y = torch.randn(T, ldy, generator=gen).to(torch.bfloat16)
+    a = (torch.randn(slots, Rm, K, generator=gen) * K ** -0.5).to(torch.bfloat16)
+    b = (torch.randn(slots, N, Rm, generator=gen) * Rm ** -0.5).to(torch.bfloat16)
+    many = torch.tensor([16, 1, 5, 2])[torch.arange(T) // 16 % 4]   # adapters in the tile
+    tok = (torch.arange(T) * 7 % many + (torch.arange(T) // 16 + 1) % 2).int()   # slot 0 (no adapter) in every second tile
+    xd, yd, ad, bd, td = x.cuda(), y.clone().cuda(), a.cuda(), b.cuda(), tok.cuda()
+    assert g.lib().tgis_k_lora(g.ptr(xd), K, g.ptr(td), g.ptr(ad), g.ptr(bd), K, N, Rm, col0, g.ptr(yd), ldy, T) == 0, g.kerr()
+    got = yd.cpu()
+    s = (tok.long() - 1).clamp(min=0)
+    v = torch.einsum("tk,trk->tr", x.double(), a[s].double())
+    delta = torch.einsum("tr,tnr->tn", v.bfloat16().double(), b[s].double()) * (tok > 0)[:, None]
+    mag = torch.einsum("tr,tnr->tn", v.abs(), b[s].double().abs()) * (tok > 0)[:, None]
+    want = y[:, col0:col0 + N].double() + delta
+    # v may round to the other neighbour (2^-8 of it, and one more in doubt); the delta and the sum are rounded once each
+    assert bool(((got[:, col0:col0 + N].double() - want).abs() <= 2.0 ** -8 * (want.abs() + delta.abs()) + 2.0 ** -7 * mag + 1e-6).all())
+    assert torch.equal(got[tok == 0], y[tok == 0])
+    assert torch.equal(got[:, :col0], y[:, :col0]) and torch.equal(got[:, col0 + N:], y[:, col0 + N:])
+
+
 # ---------------------------------------------------------------------------------------------------- engine level
 def _engine(cfg_name, **kw):
     from oracle.llama_oracle import CONFIGS, rope_table, synthetic_weights

@@ -699,7 +699,7 @@ struct tgis_engine {
         ll.A_gu = take(Sl * 2 * R * H); ll.B_gu = take(Sl * (size_t)2 * F * 2 * R);
         ll.A_d = take(Sl * R * F);      ll.B_d = take(Sl * H * R);
       }
-      lora_v.alloc(lora_buffer_rows(T_alloc) * 3 * R);
+      lora_v.alloc(T_alloc * 3 * R);
       gu_buf.alloc(T_alloc * (size_t)2 * F);
     }
     }  // !pnx_on

@@ -182,9 +182,6 @@ struct LoraGroup {
   int n_mods;
   int v_ld;                // floats per token in the shrink buffer (a multiple of four)
 };
-constexpr int LORA_PARTS = 8, LORA_PARTS_TOKENS = 64;   // steps of up to 64 tokens leave the shrink's sums in eight parts
-// rows of v_ld floats that the shrink buffer needs for steps of up to T tokens
-inline size_t lora_buffer_rows(size_t T) { const size_t few = (size_t)LORA_PARTS * (T < LORA_PARTS_TOKENS ? T : LORA_PARTS_TOKENS); return T > few ? T : few; }
 cudaError_t lora_shrink_launch(const __nv_bfloat16* x, int ldx, const int32_t* tok_slot, const LoraGroup& g, float* v, int T,
                                cudaStream_t stream);
 // act != nullptr (one module over interleaved gate / up columns): act[t, j] = bf16(silu(gate)) * up of the sum instead of y

@@ -11,13 +11,14 @@
 //   vllm/lora/lora_weights.py `optimize`               the alpha/r scaling is folded into B once at load time (host side)
 // Rounding points restated here exactly: fp32 shrink sums -> bf16 -> fp32 expand sums -> bf16 delta -> bf16(y + delta).
 //
-// Shape of the problem: HBM/L2-bound skinny products (rank 8..64 against K, N of 1k..14k), integer slot look-ups per
-// token; no tensor-core shape worth having.  Two kernels per adapted projection group:
+// Shape of the problem: skinny products (rank 8..64 against K, N of 1k..14k) of a few kilobytes to a few megabytes with integer slot
+// look-ups per token.  Two kernels per adapted projection group:
 //   shrink : CTA = (tile of 8 tokens, 4 rank rows of one module), its 8 warps split K; the A rows are streamed once per
-//            tile and adapter with 16-byte loads and used for all of the tile's tokens of that adapter.
-//   expand : CTA = (tile of 8 tokens, 1024 output columns), thread = 4 consecutive columns; the 4 B rows of a thread are
-//            one contiguous run (a warp reads 32 consecutive runs -- fully coalesced) and are read ONCE for the tile's tokens
-//            of one adapter; the tile's rank vectors are staged in shared memory (broadcast reads).
+//            tile and adapter with 16-byte loads and used for all of the tile's tokens of that adapter.  (As mma.sync fragments of
+//            16 tokens x 16 ranks in eight parts of K a launch of a small step took 9.8 us instead of 6.6, one of 1300 tokens 74.)
+//   expand : CTA = (tile of 16 tokens, 512 output columns), warp = 64 columns: B rows as fragments of mma.sync straight from global
+//            memory, all requested in one round, each lane 8 neighbouring columns of 2 tokens.  24 tokens, four adapters of rank 16, 8B
+//            widths, microseconds a launch against multiply-adds from shared memory (8 tokens x 1024 columns): 6.3 -> 4.8, with SwiGLU 19.8 -> 11.3.
 // Both are launches of a few microseconds of dependent loads.  The engine runs shrink BEFORE the base projection, which it
 // does not depend on: the projection's first weights are on their way while it runs.
 // Adapter storage (engine.cu): per layer and module  A [slots][Rm][K] and B [slots][N][Rm] bf16, zero padded to the module's
@@ -43,22 +44,41 @@ __device__ __forceinline__ float dot8(const F8& a, const F8& b) {
   return s;
 }
 
-constexpr int LORA_TT = 8;  // tokens per tile
+constexpr int LORA_TT = 16;   // tokens per tile of the expand
+constexpr int LORA_ST = 8;    // of the shrink
 constexpr int LORA_MAX_RM = 128;
 
-// The adapter slots of a tile's tokens (-1 behind the last token).  A tile is worked through once per distinct slot -- the
-// scheduler sorts a step's tokens by adapter, so most tiles have one or two --, by different CTAs in small launches.
+// The adapter slots of a tile's TT tokens, lane i: token i's (-1 behind the last token).  A tile is worked through once per distinct slot --
+// the scheduler sorts a step's tokens by adapter, so most tiles have one or two --, by different CTAs in small launches.
+template <int TT>
 struct TileSlots {
-  int s[LORA_TT];
+  int mine;
   __device__ __forceinline__ TileSlots(const int32_t* tok_slot, int t0, int T) {
+    const int i = threadIdx.x & 31;
+    mine = i < TT && t0 + i < T ? tok_slot[t0 + i] : -1;
+  }
+  // the n-th distinct slot from `least` on, in the order of first tokens; -1: there are fewer
+  __device__ __forceinline__ int distinct(int n, int least) const {
+    const uint32_t same = __match_any_sync(0xffffffffu, mine);
+    uint32_t firsts = __ballot_sync(0xffffffffu, mine >= least && (int)(threadIdx.x & 31) == __ffs(same) - 1);
+    for (int i = 0; i < n; ++i) firsts &= firsts - 1;
+    const int s = __shfl_sync(0xffffffffu, mine, firsts != 0 ? __ffs(firsts) - 1 : 0);
+    return firsts != 0 ? s : -1;
+  }
+  __device__ __forceinline__ int of(int token) const { return __shfl_sync(0xffffffffu, mine, token); }
+};
+// The same for the shrink, in every thread.
+struct ShrinkSlots {
+  int s[LORA_ST];
+  __device__ __forceinline__ ShrinkSlots(const int32_t* tok_slot, int t0, int T) {
 #pragma unroll
-    for (int j = 0; j < LORA_TT; ++j) s[j] = t0 + j < T ? tok_slot[t0 + j] : -1;
+    for (int j = 0; j < LORA_ST; ++j) s[j] = t0 + j < T ? tok_slot[t0 + j] : -1;
   }
   // the p-th distinct slot from `least` on, in the order of first tokens; -1: there are fewer
   __device__ __forceinline__ int distinct(int p, int least) const {
     int found = -1, n = 0;
 #pragma unroll
-    for (int j = 0; j < LORA_TT; ++j) {
+    for (int j = 0; j < LORA_ST; ++j) {
       bool first = s[j] >= least;
 #pragma unroll
       for (int i = 0; i < j; ++i) first &= s[i] != s[j];
@@ -89,7 +109,7 @@ constexpr int LORA_RPC = 4;
 __global__ void __launch_bounds__(256)
 lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* __restrict__ tok_slot, LoraGroup g,
                    float* __restrict__ v, int T) {
-  __shared__ float part[8][LORA_RPC][LORA_TT];
+  __shared__ float part[8][LORA_RPC][LORA_ST];
   griddep_launch();
   griddep_wait();
   int m = 0, r0 = (int)blockIdx.y * LORA_RPC;  // blockIdx.y enumerates (module, group of LORA_RPC rank rows)
@@ -99,28 +119,28 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* 
   }
   const LoraModule md = g.mod[m];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t0 = (int)blockIdx.x * LORA_TT;
-  const TileSlots tile(tok_slot, t0, T);
+  const int t0 = (int)blockIdx.x * LORA_ST;
+  const ShrinkSlots tile(tok_slot, t0, T);
   const int nvec = md.K / 8;
   const uint4* xq = reinterpret_cast<const uint4*>(x);
   const size_t ldq = (size_t)ldx / 8;
   for (int p = blockIdx.z;; p += gridDim.z) {
     const int slot = tile.distinct(p, 1);
     if (slot < 0) return;
-    float acc[LORA_RPC][LORA_TT];
+    float acc[LORA_RPC][LORA_ST];
 #pragma unroll
     for (int q = 0; q < LORA_RPC; ++q)
 #pragma unroll
-      for (int j = 0; j < LORA_TT; ++j) acc[q][j] = 0.f;
+      for (int j = 0; j < LORA_ST; ++j) acc[q][j] = 0.f;
     const uint4* a0 = reinterpret_cast<const uint4*>(md.A + ((size_t)(slot - 1) * md.Rm + r0) * md.K);
     for (int kv = warp * 32 + lane; kv < nvec; kv += 256) {
-      uint4 ar[LORA_RPC], xr[LORA_TT];
+      uint4 ar[LORA_RPC], xr[LORA_ST];
 #pragma unroll
       for (int q = 0; q < LORA_RPC; ++q) ar[q] = a0[(size_t)q * nvec + kv];
 #pragma unroll
-      for (int j = 0; j < LORA_TT; ++j) xr[j] = tile.s[j] == slot ? xq[(size_t)(t0 + j) * ldq + kv] : make_uint4(0u, 0u, 0u, 0u);
+      for (int j = 0; j < LORA_ST; ++j) xr[j] = tile.s[j] == slot ? xq[(size_t)(t0 + j) * ldq + kv] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-      for (int j = 0; j < LORA_TT; ++j) {
+      for (int j = 0; j < LORA_ST; ++j) {
         const F8 xf = cvt8(xr[j]);
 #pragma unroll
         for (int q = 0; q < LORA_RPC; ++q) acc[q][j] += dot8(cvt8(ar[q]), xf);
@@ -129,15 +149,15 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* 
 #pragma unroll
     for (int q = 0; q < LORA_RPC; ++q)
 #pragma unroll
-      for (int j = 0; j < LORA_TT; ++j) {
+      for (int j = 0; j < LORA_ST; ++j) {
         float s = acc[q][j];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (lane == 0) part[warp][q][j] = s;
       }
     __syncthreads();
-    if (threadIdx.x < LORA_RPC * LORA_TT) {
-      const int q = threadIdx.x / LORA_TT, j = threadIdx.x % LORA_TT;
+    if (threadIdx.x < LORA_RPC * LORA_ST) {
+      const int q = threadIdx.x / LORA_ST, j = threadIdx.x % LORA_ST;
       if (t0 + j < T && tok_slot[t0 + j] == slot) {
         float s = 0.f;
 #pragma unroll
@@ -149,112 +169,133 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* 
   }
 }
 
-// expand: CTA = (tile of 8 tokens, 1024 output columns), thread = LORA_EC = 4 consecutive columns (~100 registers: two
-// CTAs per SM).  Same-adapter tile: per 8 rank indices the thread holds its 4 x 8 block of B in registers -- the next
-// block is already in flight while this one is used -- and, per rank index, the tile's 8 rank values arrive as two
-// broadcast 16-byte shared-memory loads (32 FMAs per 2 LDS; the first version paid one LDS per FMA and one exposed memory
-// latency per block).
-constexpr int LORA_EC = 4;
-constexpr int LORA_ECOLS = 256 * LORA_EC;  // columns per CTA
-__device__ __forceinline__ void st4f(__nv_bfloat16* p, const float (&f)[4]) {
-  const __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
-  uint2 r;
-  r.x = *reinterpret_cast<const uint32_t*>(&lo);
-  r.y = *reinterpret_cast<const uint32_t*>(&hi);
-  *reinterpret_cast<uint2*>(p) = r;
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+
+constexpr int LORA_ECOLS = 512;   // columns per CTA of the expand: 8 warps x 64
 // ACT: the columns are interleaved (gate_j, up_j) pairs; act[t, j] = bf16(silu(gate)) * up of the corrected projection is
 // written (for tokens without an adapter too) and y is only read: the projection's own kernel after it drops out.
 template <bool ACT>
-__global__ void __launch_bounds__(256)
-lora_expand_kernel(const float* __restrict__ v, const int32_t* __restrict__ tok_slot, LoraGroup g,
+__global__ void __launch_bounds__(256, 2)
+lora_expand_kernel(const float* __restrict__ v, const int32_t* __restrict__ tok_slot, LoraGroup gr,
                    __nv_bfloat16* __restrict__ y, int ldy, __nv_bfloat16* __restrict__ act, int T) {
-  __shared__ __align__(16) float vsT[LORA_MAX_RM][LORA_TT];  // [rank index][token of the tile]
+  __shared__ __align__(16) __nv_bfloat16 vs[LORA_TT][LORA_MAX_RM + 8];   // the tile's rank vectors
   griddep_launch();
-  griddep_wait();
   const int t0 = (int)blockIdx.y * LORA_TT;
-  const LoraModule md = g.mod[blockIdx.z % g.n_mods];
+  const LoraModule md = gr.mod[blockIdx.z % gr.n_mods];
   if ((int)blockIdx.x * LORA_ECOLS >= md.N) return;
-  const TileSlots tile(tok_slot, t0, T);
-  const int n0 = ((int)blockIdx.x * 256 + (int)threadIdx.x) * LORA_EC;
-  const bool col_ok = n0 < md.N;
-  for (int p = blockIdx.z / g.n_mods;; p += gridDim.z / g.n_mods) {
+  const TileSlots<LORA_TT> tile(tok_slot, t0, T);   // (written by the host before the step)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int n0 = (int)blockIdx.x * LORA_ECOLS + warp * 64;
+  const int kc = (md.Rm + 15) / 16;   // chunks of 16 rank indices
+  const int slot_of[2] = {tile.of(g), tile.of(g + 8)};
+  griddep_wait();
+  for (int p = blockIdx.z / gr.n_mods;; p += gridDim.z / gr.n_mods) {
     const int slot = tile.distinct(p, ACT ? 0 : 1);
     if (slot < 0) return;
-    // the thread's y values and its first block of B do not depend on the rank vectors -- request them before the staging
-    // barrier so that their latency runs under it (a CTA is only a few microseconds of work)
-    uint2 yraw[LORA_TT];
-    uint4 nxt[LORA_EC];
-    const __nv_bfloat16* brow = md.B + ((size_t)(slot > 0 ? slot - 1 : 0) * md.N + (col_ok ? n0 : 0)) * md.Rm;
-    if (col_ok) {
-      if (slot > 0) {
+    // columns n0 + 32 h + 8 t .. + 7 of tokens g and g + 8 are this lane's; of the products' column blocks j = 0 .. 3 (8 wide) lane
+    // group t holds the neighbours 2 j, 2 j + 1, so block j is made of the columns 8 (c / 2) + 2 j + c % 2, c = 0 .. 7
+    uint4 yv[2][2];
 #pragma unroll
-        for (int e = 0; e < LORA_EC; ++e) nxt[e] = *reinterpret_cast<const uint4*>(brow + (size_t)e * md.Rm);
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int n = n0 + 32 * h + 8 * t;
+        yv[h][k] = make_uint4(0u, 0u, 0u, 0u);
+        if (slot_of[k] == slot && n < md.N) {
+          const uint2* from = reinterpret_cast<const uint2*>(y + (size_t)(t0 + g + 8 * k) * ldy + md.col0 + n);
+          const uint2 lo = from[0], hi = from[1];
+          yv[h][k] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        }
       }
-#pragma unroll
-      for (int j = 0; j < LORA_TT; ++j)
-        if (tile.s[j] == slot) yraw[j] = *reinterpret_cast<const uint2*>(y + (size_t)(t0 + j) * ldy + md.col0 + n0);
-    }
-    float acc[LORA_TT][LORA_EC];
-#pragma unroll
-    for (int j = 0; j < LORA_TT; ++j)
-#pragma unroll
-      for (int e = 0; e < LORA_EC; ++e) acc[j][e] = 0.f;
+    float acc[2][4][4] = {};
     if (slot > 0) {
+      const __nv_bfloat16* brow[2][4];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int n = min(n0 + 32 * h + 8 * (g >> 1) + 2 * j + (g & 1), md.N - 1);
+          brow[h][j] = md.B + ((size_t)(slot - 1) * md.N + n) * md.Rm;
+        }
+      uint2 nxt[2][4];
+      auto load = [&](int c) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            nxt[h][j] = c * 16 + t * 4 < md.Rm ? *reinterpret_cast<const uint2*>(brow[h][j] + c * 16 + t * 4) : make_uint2(0u, 0u);
+      };
+      load(0);
       // the fp32 shrink sums enter the second product as bf16 (lora_expand_op.py casts the buffer to the weight dtype)
-      for (int i = threadIdx.x; i < LORA_TT * md.Rm; i += 256) {
-        const int j = i / md.Rm, r = i - j * md.Rm;
-        const bool live = t0 + j < T && tok_slot[t0 + j] == slot;
-        vsT[r][j] = live ? bf16_round(v[(size_t)(t0 + j) * g.v_ld + md.v_off + r]) : 0.f;
+      const int row4 = kc * 4;
+      for (int i = threadIdx.x; i < LORA_TT * row4; i += 256) {
+        const int tok = i / row4, r = i % row4 * 4;
+        float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t0 + tok < T && r < md.Rm && tok_slot[t0 + tok] == slot) {
+          const float* from = v + (size_t)(t0 + tok) * gr.v_ld + md.v_off + r;
+          f = *reinterpret_cast<const float4*>(from);
+        }
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(f.x, f.y), hi = __floats2bfloat162_rn(f.z, f.w);
+        *reinterpret_cast<uint2*>(&vs[tok][r]) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
       }
       __syncthreads();
-      if (col_ok) {
-        const int nrv = md.Rm / 8;
-        for (int rv = 0; rv < nrv; ++rv) {
-          F8 bb[LORA_EC];
+      for (int c = 0; c < kc; ++c) {
+        uint2 bv[2][4];
 #pragma unroll
-          for (int e = 0; e < LORA_EC; ++e) bb[e] = cvt8(nxt[e]);
-          if (rv + 1 < nrv) {
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int e = 0; e < LORA_EC; ++e) nxt[e] = *reinterpret_cast<const uint4*>(brow + (size_t)e * md.Rm + 8 * (rv + 1));
-          }
+          for (int j = 0; j < 4; ++j) bv[h][j] = nxt[h][j];
+        if (c + 1 < kc) load(c + 1);
+        const uint2 a0 = *reinterpret_cast<const uint2*>(&vs[g][c * 16 + t * 4]), a1 = *reinterpret_cast<const uint2*>(&vs[g + 8][c * 16 + t * 4]);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const float4 va = *reinterpret_cast<const float4*>(&vsT[rv * 8 + q][0]);
-            const float4 vb = *reinterpret_cast<const float4*>(&vsT[rv * 8 + q][4]);
-            const float vv[LORA_TT] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int e = 0; e < LORA_EC; ++e)
-#pragma unroll
-              for (int j = 0; j < LORA_TT; ++j) acc[j][e] = fmaf(vv[j], bb[e].v[q], acc[j][e]);
-          }
-        }
+          for (int j = 0; j < 4; ++j) mma_16816(acc[h][j], a0.x, a1.x, a0.y, a1.y, bv[h][j].x, bv[h][j].y);
       }
     }
-    if (col_ok) {
 #pragma unroll
-      for (int j = 0; j < LORA_TT; ++j) {
-        if (tile.s[j] != slot) continue;   // (another adapter's token: its sums here are not used)
-        float yv[LORA_EC] = {__uint_as_float(yraw[j].x << 16), __uint_as_float(yraw[j].x & 0xffff0000u),
-                             __uint_as_float(yraw[j].y << 16), __uint_as_float(yraw[j].y & 0xffff0000u)};
-        if (slot > 0) {
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
-          for (int e = 0; e < LORA_EC; ++e) yv[e] += bf16_round(acc[j][e]);
+      for (int k = 0; k < 2; ++k) {
+        const int n = n0 + 32 * h + 8 * t;
+        if (slot_of[k] != slot || n >= md.N) continue;   // (another adapter's token: its sums here are not used)
+        const uint32_t yw[4] = {yv[h][k].x, yv[h][k].y, yv[h][k].z, yv[h][k].w};
+        float o[8];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          o[2 * j] = __uint_as_float(yw[j] << 16);
+          o[2 * j + 1] = __uint_as_float(yw[j] & 0xffff0000u);
+          if (slot > 0) {
+            o[2 * j] += bf16_round(acc[h][j][2 * k]);
+            o[2 * j + 1] += bf16_round(acc[h][j][2 * k + 1]);
+          }
         }
         if constexpr (ACT) {
-          float o[2];
+          float gate[4], s[4];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const float gx = bf16_round(yv[2 * h]);
-            o[h] = bf16_round(gx / (1.0f + expf(-gx))) * bf16_round(yv[2 * h + 1]);
-          }
-          *reinterpret_cast<__nv_bfloat162*>(act + (size_t)(t0 + j) * (md.N / 2) + n0 / 2) = __floats2bfloat162_rn(o[0], o[1]);
+          for (int j = 0; j < 4; ++j) gate[j] = bf16_round(o[2 * j]);
+          silu_bf16_n(gate, s);
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(s[0] * bf16_round(o[1]), s[1] * bf16_round(o[3]));
+          const __nv_bfloat162 hi = __floats2bfloat162_rn(s[2] * bf16_round(o[5]), s[3] * bf16_round(o[7]));
+          *reinterpret_cast<uint2*>(act + (size_t)(t0 + g + 8 * k) * (md.N / 2) + n / 2) =
+              make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
         } else {
-          st4f(y + (size_t)(t0 + j) * ldy + md.col0 + n0, yv);
+          uint2* to = reinterpret_cast<uint2*>(y + (size_t)(t0 + g + 8 * k) * ldy + md.col0 + n);
+          uint32_t w[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const __nv_bfloat162 q = __floats2bfloat162_rn(o[2 * j], o[2 * j + 1]);
+            w[j] = *reinterpret_cast<const uint32_t*>(&q);
+          }
+          to[0] = make_uint2(w[0], w[1]);
+          to[1] = make_uint2(w[2], w[3]);
         }
       }
-    }
-    __syncthreads();   // vsT is used again
+    __syncthreads();   // vs is used again
   }
 }
 
@@ -275,7 +316,7 @@ cudaError_t lora_shrink_launch(const __nv_bfloat16* x, int ldx, const int32_t* t
   if (!lora_group_ok(g) || ldx % 8 != 0) return cudaErrorInvalidValue;
   int groups = 0;
   for (int m = 0; m < g.n_mods; ++m) groups += g.mod[m].Rm / LORA_RPC;
-  return launch_k(lora_shrink_kernel, dim3((T + LORA_TT - 1) / LORA_TT, groups, lora_passes_apart(T)), dim3(256), 0, stream, x, ldx, tok_slot,
+  return launch_k(lora_shrink_kernel, dim3((T + LORA_ST - 1) / LORA_ST, groups, lora_passes_apart(T)), dim3(256), 0, stream, x, ldx, tok_slot,
                   g, v, T);
 }
 

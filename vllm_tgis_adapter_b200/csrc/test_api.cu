@@ -465,7 +465,7 @@ int tgis_k_sampler_ex(const void* logits_dev, int32_t logits_bf16, int32_t ld, i
 int tgis_k_lora(const void* x_dev, int32_t ldx, const int32_t* tok_slot_dev, const void* a_dev, const void* b_dev, int32_t K,
                 int32_t N, int32_t Rm, int32_t col0, void* y_dev, int32_t ldy, int32_t T) {
   Tmp<float> v;
-  KCK(v.alloc(lora_buffer_rows(T) * Rm));
+  KCK(v.alloc((size_t)T * Rm));
   LoraGroup g{};
   g.n_mods = 1;
   g.v_ld = Rm;
@@ -481,7 +481,7 @@ int tgis_k_lora_bench(const void* x_dev, int32_t ldx, const int32_t* tok_slot_de
                       int32_t K, int32_t N, int32_t Rm, void* y_dev, int32_t ldy, int32_t T, int32_t iters,
                       float* us_shrink, float* us_expand) {
   Tmp<float> v;
-  KCK(v.alloc(lora_buffer_rows(T) * Rm));
+  KCK(v.alloc((size_t)T * Rm));
   LoraGroup g{};
   g.n_mods = 1;
   g.v_ld = Rm;
@@ -513,7 +513,7 @@ int tgis_k_lora_bench(const void* x_dev, int32_t ldx, const int32_t* tok_slot_de
 int tgis_k_lora_swiglu(const void* x_dev, int32_t ldx, const int32_t* tok_slot_dev, const void* a_dev, const void* b_dev, int32_t K,
                        int32_t ffn, int32_t Rm, const void* gate_up_dev, void* act_dev, int32_t T) {
   Tmp<float> v;
-  KCK(v.alloc(lora_buffer_rows(T) * Rm));
+  KCK(v.alloc((size_t)T * Rm));
   LoraGroup g{};
   g.n_mods = 1;
   g.v_ld = Rm;
