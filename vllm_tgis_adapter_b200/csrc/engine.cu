@@ -4090,6 +4090,13 @@ struct tgis_engine {
       (q == 1 ? dec : pre).push_back(s);
     }
     const double t_now = now_s();
+    BitmapSlots fresh{};   // slots of the requests admitted here: no token has been seen yet
+    auto clear_fresh = [&]() {
+      if (fresh.n == 0) return;
+      CK(bitmap_clear_launch(seen_bitmap.p, bitmap_words, fresh, stream));
+      ++n_launches;
+      fresh.n = 0;
+    };
     while (!waiting.empty() && budget > 0 && (int)running.size() < S_max && !free_slots.empty()) {
       Request& r = *waiting.front();
       const int remaining = (int)r.tokens.size() - r.n_computed;
@@ -4099,8 +4106,8 @@ struct tgis_engine {
       r.slot = free_slots.back();
       free_slots.pop_back();
       ensure_blocks(r, r.n_computed + q);
-      CK(bitmap_clear_launch(seen_bitmap.p, bitmap_words, r.slot, stream));
-      ++n_launches;
+      fresh.slot[fresh.n++] = r.slot;
+      if (fresh.n == BITMAP_SLOTS) clear_fresh();
       if (r.ts_first_sched == 0) r.ts_first_sched = t_now;
       budget -= q;
       Sched s{&r, q, r.n_computed + q == (int)r.tokens.size()};
@@ -4108,6 +4115,7 @@ struct tgis_engine {
       running.push_back(std::move(waiting.front()));
       waiting.pop_front();
     }
+    clear_fresh();
     std::vector<Sched> batch;
     batch.reserve(dec.size() + pre.size());
     batch.insert(batch.end(), dec.begin(), dec.end());

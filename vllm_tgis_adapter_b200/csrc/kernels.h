@@ -742,7 +742,11 @@ cudaError_t sampler_launch(const void* logits, int logits_bf16, int ld, int voca
                            const uint32_t* allow_bitmap = nullptr /* [slots][bitmap_words], rows flagged SAMPLE_MASKED */);
 int sampler_cluster_size(int n_rows, int any_complex, int num_sms);
 // seen-token bitmap maintenance
-cudaError_t bitmap_clear_launch(uint32_t* bitmap, int bitmap_words, int slot, cudaStream_t stream);
+constexpr int BITMAP_SLOTS = 64;
+struct BitmapSlots {   // by value: the requests that a step admits, one launch for 64 of them
+  int n, slot[BITMAP_SLOTS];
+};
+cudaError_t bitmap_clear_launch(uint32_t* bitmap, int bitmap_words, const BitmapSlots& slots, cudaStream_t stream);
 cudaError_t bitmap_set_launch(uint32_t* bitmap, int bitmap_words, const int32_t* slots, const int32_t* tokens, int n,
                               cudaStream_t stream);
 size_t sampler_scratch_floats(int vocab);

@@ -980,10 +980,12 @@ cudaError_t sampler_launch(const void* logits, int logits_bf16, int ld, int voca
 size_t sampler_scratch_floats(int vocab) { return (size_t)vocab; }
 
 // ---------------------------------------------------------------- seen-token bitmap maintenance
-__global__ void bitmap_clear_kernel(uint32_t* bm, int words) {
+// grid (8, slots)
+__global__ void bitmap_clear_kernel(uint32_t* bm, int words, BitmapSlots slots) {
   griddep_launch();
   griddep_wait();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x) bm[i] = 0u;
+  uint32_t* row = bm + (size_t)slots.slot[blockIdx.y] * words;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < words; i += gridDim.x * blockDim.x) row[i] = 0u;
 }
 __global__ void bitmap_set_kernel(uint32_t* bm, int words, const int32_t* slots, const int32_t* tokens, int n) {
   griddep_launch();
@@ -994,8 +996,10 @@ __global__ void bitmap_set_kernel(uint32_t* bm, int words, const int32_t* slots,
   if (s < 0 || t < 0 || (t >> 5) >= words) return;
   atomicOr(&bm[(size_t)s * words + (t >> 5)], 1u << (t & 31));
 }
-cudaError_t bitmap_clear_launch(uint32_t* bitmap, int bitmap_words, int slot, cudaStream_t stream) {
-  return launch_k(bitmap_clear_kernel, dim3(8), dim3(256), 0, stream, bitmap + (size_t)slot * bitmap_words, bitmap_words);
+cudaError_t bitmap_clear_launch(uint32_t* bitmap, int bitmap_words, const BitmapSlots& slots, cudaStream_t stream) {
+  if (slots.n <= 0) return cudaSuccess;
+  if (slots.n > BITMAP_SLOTS) return cudaErrorInvalidValue;
+  return launch_k(bitmap_clear_kernel, dim3(8, slots.n), dim3(256), 0, stream, bitmap, bitmap_words, slots);
 }
 cudaError_t bitmap_set_launch(uint32_t* bitmap, int bitmap_words, const int32_t* slots, const int32_t* tokens, int n,
                               cudaStream_t stream) {
