@@ -141,3 +141,24 @@ def test_tanh_of_few_outputs(lib, T, N, K, y_dt):
     assert lib.tgis_k_gemm_any(p(x), p(w), p(y), 1, 1, y_dt, T, N, K, K, K, N, 1, 0, 0, 0, None, 0, 0, None, 1, 4, None, 0) == 0
     want = torch.tanh(x.to(F64) @ w.to(F64).T)
     assert ((y.to(F64) - want).abs() <= 1e-5 + (2 ** -8 * want.abs() if y_dt else 0)).all()
+
+
+@pytest.mark.parametrize("inner", [128, 516])
+def test_short_convolution_of_prompts_has_the_bits_of_single_tokens(lib, inner):
+    """300 tokens in portions of every length around the run of eight, fresh and carried on, against the same tokens in launches of
+    fewer than 256 (the kernel with a token per thread)."""
+    gen = torch.Generator(device="cuda").manual_seed(inner)
+    lens, before = [1, 2, 3, 4, 7, 8, 9, 16, 17, 40, 93, 100], [0, 5, 1, 0, 2, 3, 0, 1, 9, 2, 0, 30]
+    T, n = sum(lens), len(lens)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    xz, w, b, state = rnd(T, 2 * inner), rnd(inner, 4), rnd(inner), rnd(n, 3, inner)
+    slot = torch.tensor([s for s, k in enumerate(lens) for _ in range(k)], dtype=torch.int32, device="cuda")
+    pos = torch.tensor([q + i for k, q in zip(lens, before) for i in range(k)], dtype=torch.int32, device="cuda")
+    res, cut = [], sum(lens[:-1])
+    for parts in ([(0, T)], [(0, cut), (cut, T)]):
+        f32, op = torch.zeros(T, inner, device="cuda"), torch.zeros(T, inner, device="cuda", dtype=torch.bfloat16)
+        for a, e in parts:
+            assert lib.tgis_k_short_conv(p(xz[a:]), 2 * inner, inner, p(w), p(b), 4, p(pos[a:].clone()), p(slot[a:].clone()), p(state), p(f32[a:]), p(op[a:]), 1, e - a) == 0
+        res.append((f32, op))
+    assert T == 300 and cut < 256
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])

@@ -150,6 +150,56 @@ short_conv_silu_kernel(const float* __restrict__ xz, int ld, int inner, const fl
   if (out_op) st_op_vec<VEC>(out_op, out_dtype, (size_t)t * inner + c, acc);
 }
 
+// The same for four taps and aligned rows, eight tokens per thread: a token's three predecessors are the values just used (the batch
+// holds portions one behind the other), so an input is read once and not four times.  2048 tokens x 4096 channels: 80 -> 26 us.
+constexpr int CONV_RUN = 8;
+__global__ void __launch_bounds__(128)
+short_conv_run_kernel(const float* __restrict__ xz, int ld, int inner, const float* __restrict__ w, const float* __restrict__ b,
+                      const int32_t* __restrict__ positions, const int32_t* __restrict__ tok_slot, const float* __restrict__ conv_state,
+                      float* __restrict__ out_f32, void* __restrict__ out_op, int out_dtype, int T) {
+  griddep_launch();
+  const int t0 = blockIdx.x * CONV_RUN, c = (blockIdx.y * 128 + threadIdx.x) * 4;
+  if (c >= inner) return;
+  float wt[4][4], bias[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) ld_vec<4>(w + (size_t)(c + e) * 4, wt[e]);
+  if (b != nullptr)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) bias[e] = b[c + e];
+  griddep_wait();
+  int slot[CONV_RUN + 3];
+  float x[CONV_RUN + 3][4];
+#pragma unroll
+  for (int i = 0; i < CONV_RUN + 3; ++i) {
+    const int t = t0 - 3 + i;
+    slot[i] = t >= 0 && t < T ? tok_slot[t] : -1;
+    if (t >= 0 && t < T) ld_vec<4>(xz + (size_t)t * ld + c, x[i]);
+  }
+#pragma unroll
+  for (int i = 0; i < CONV_RUN; ++i) {
+    const int t = t0 + i;
+    if (t >= T) break;
+    const int p = positions[t], s = slot[i + 3];
+    int nb = 0;   // predecessors of this token inside the batch
+#pragma unroll
+    for (int j = 1; j < 4; ++j)
+      if (nb == j - 1 && slot[i + 3 - j] == s) nb = j;
+    float acc[4] = {bias[0], bias[1], bias[2], bias[3]};
+#pragma unroll
+    for (int j = 3; j >= 0; --j) {   // oldest input first
+      if (p - j < 0) continue;
+      float v[4] = {x[i + 3 - j][0], x[i + 3 - j][1], x[i + 3 - j][2], x[i + 3 - j][3]};
+      if (j > nb) ld_vec<4>(conv_state + ((size_t)s * 3 + (3 - j + nb)) * inner + c, v);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[e] = fmaf(wt[e][3 - j], v[e], acc[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] = silu_f(acc[e]);
+    if (out_f32) *reinterpret_cast<float4*>(out_f32 + (size_t)t * inner + c) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    if (out_op) st_op_vec<4>(out_op, out_dtype, (size_t)t * inner + c, acc);
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ selective scan
 constexpr int SCAN_THREADS = 64, SCAN_CHUNK = 8, SCAN_REG_STATE = 16, SCAN_LPC = 4, SCAN_RPL = SCAN_REG_STATE / SCAN_LPC;
 // the convolution's tail: inputs of the last taps - 1 positions (entry e: position end - (taps - 1) + e)
@@ -1136,9 +1186,13 @@ cudaError_t short_conv_silu_launch(const float* xz, int ld, int inner, const flo
   if (T <= 0) return cudaSuccess;
   if (taps < 1) return cudaErrorInvalidValue;
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
-  if (ld % 4 == 0 && inner % 4 == 0 && al16(xz) && al16(conv_state) && al16(out_f32) && al16(w) && al16(out_op))
+  if (ld % 4 == 0 && inner % 4 == 0 && al16(xz) && al16(conv_state) && al16(out_f32) && al16(w) && al16(out_op)) {
+    if (taps == 4 && T >= 256)   // (blocks enough with eight tokens each)
+      return launch_k(short_conv_run_kernel, dim3((T + CONV_RUN - 1) / CONV_RUN, (inner / 4 + 127) / 128), dim3(128), 0, stream, xz, ld, inner, w, b,
+                      positions, tok_slot, conv_state, out_f32, out_op, out_dtype, T);
     return launch_k(short_conv_silu_kernel<4>, dim3(T, (inner / 4 + 127) / 128), dim3(128), 0, stream, xz, ld, inner, w, b, taps,
                     positions, tok_slot, conv_state, out_f32, out_op, out_dtype);
+  }
   return launch_k(short_conv_silu_kernel<1>, dim3(T, (inner + 127) / 128), dim3(128), 0, stream, xz, ld, inner, w, b, taps,
                   positions, tok_slot, conv_state, out_f32, out_op, out_dtype);
 }
