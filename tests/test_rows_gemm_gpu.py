@@ -51,3 +51,50 @@ def test_rotary_embedding_behind_the_product(lib, T, n_q, n_kv, K):
     assert torch.equal(y[0][:T], y[1][:T])
     for a, b in zip(*caches):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("T", [257, 300, 1030])
+@pytest.mark.parametrize("batch,N,K,mode,y_dt", [(16, 512, 128, 0, 0), (5, 128, 512, 2, 1), (3, 40, 64, 0, 1), (1, 65, 2048, 0, 0), (1, 64, 320, 4, 1), (2, 300, 192, 2, 1)])
+def test_prompts_side_by_side_and_with_few_weight_rows(lib, T, batch, N, K, mode, y_dt):
+    """Products of more than 256 tokens that only the general entry takes: one per head in neighbouring columns, a router's few rows,
+    a tanh, a scale per row and head; columns between the problems and rows behind the last token stay as they are."""
+    gen = torch.Generator(device="cuda").manual_seed(T + N + K)
+    xs, ys = K + 8, N + 3
+    x = torch.randn(T, batch, xs, device="cuda", generator=gen).bfloat16()
+    w = (torch.randn(batch, N, K, device="cuda", generator=gen) * K ** -0.5).bfloat16()
+    s = torch.rand(T, batch, device="cuda", generator=gen)
+    y = torch.full((T + 1, batch, ys), 7.0, device="cuda", dtype=torch.bfloat16 if y_dt else torch.float32)
+    rc = lib.tgis_k_gemm_any(p(x), p(w), p(y), 1, 1, y_dt, T, N, K, batch * xs, K, batch * ys, batch, xs, N * K, ys, None, 0, 0, None, 1, mode, p(s), batch)
+    assert rc == 0
+    a, b = x[:, :, :K].double(), w.double()
+    want = torch.einsum("thk,hnk->thn", a, b)
+    slack = torch.einsum("thk,hnk->thn", a.abs(), b.abs()) * (K / 16 + 8) * 2.0 ** -23   # as in the products above
+    if mode == 2:
+        want, slack = want * s.double()[:, :, None], slack * s.double()[:, :, None]
+    if mode == 4:
+        want, slack = torch.tanh(want), slack + 1e-6
+    got = y[:T, :, :N].double()
+    assert ((got - want).abs() <= slack + (2.0 ** -8 * want.abs() if y_dt else 1e-6 * want.abs())).all()
+    assert bool((y[:T, :, N:] == 7.0).all()) and bool((y[T] == 7.0).all())
+
+
+@pytest.mark.parametrize("N,K", [(40, 64), (300, 192)])
+def test_expert_rows_with_a_scale_ahead_of_the_squared_relu(lib, N, K):
+    """Segments around the 32 tokens that a warp of the epilogue takes at once, each gathered row with the scale of its origin."""
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    lens = [0, 1, 31, 32, 33, 65, 257, 301]
+    R, E = sum(lens), len(lens)
+    x = torch.randn(R, K, device="cuda", generator=gen).bfloat16()
+    w = (torch.randn(E, N, K, device="cuda", generator=gen) * K ** -0.5).bfloat16()
+    s = torch.randn(R, device="cuda", generator=gen)
+    order = torch.randperm(R, device="cuda", generator=gen).int()
+    seg = torch.tensor([0] + lens, device="cuda").cumsum(0).int()
+    y = torch.full((R + 1, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    assert lib.tgis_k_gemm_any(p(x), p(w), p(y), 1, 1, 1, R, N, K, K, K, N, 1, 0, 0, 0, p(seg), E, N * K, p(order), 1, 5, p(s), 0) == 0
+    e = torch.repeat_interleave(torch.arange(E, device="cuda"), torch.tensor(lens, device="cuda"))
+    o = order.long()
+    a = torch.einsum("rk,rnk->rn", x[o].double(), w[e].double()) * s[o].double()[:, None]
+    slack = torch.einsum("rk,rnk->rn", x[o].double().abs(), w[e].double().abs()) * s[o].double().abs()[:, None] * (K / 16 + 8) * 2.0 ** -23
+    want = a.clamp(min=0) ** 2
+    assert ((y[:R].double() - want).abs() <= 2.0 ** -8 * want + 2 * a.abs() * slack + slack ** 2 + 1e-6 * want).all()
+    assert bool((y[R] == 7.0).all())

@@ -530,6 +530,7 @@ cudaError_t gemm_any_launch(const GemmAny& a, cudaStream_t stream) {
   // expert segments: CTA pairs.  64 experts of 2 x 1408 x 2048 and back, top 6, both products in microseconds, mma.sync -> pairs:
   // 4 tokens 126 -> 78, 32 tokens 260 -> 165 (6.3 TB/s of weights), 512 tokens 334 -> 195, 2048 tokens 1003 -> 243
   if (gemm_pair_takes_groups(a)) return gemm_pair_grouped_launch(a, stream);
+  if (mma_eligible(a) && gemm_pair_takes_dense(a)) return gemm_pair_dense_launch(a, stream);
   if (mma_eligible(a) && gemm_skinny_takes_batch(a)) return gemm_skinny_batch_launch(a, stream);
   if (mma_eligible(a)) return a.y_dtype == DT_BF16 ? launch_mma<bf>(a, stream) : launch_mma<float>(a, stream);
   const int key = a.x_dtype * 4 + a.w_dtype * 2 + a.y_dtype;  // DT_F32 = 0, DT_BF16 = 1

@@ -55,6 +55,9 @@ struct PairArgs {
   const float* row_scale;   // PAIR_RELU2: scale of the input row gather[p] (null: 1)
   const int* gather;
   int* err;                 // host-visible error word
+  int batch, x_cs;          // dense: problems side by side (0 or 1: one); columns of X between them (W: N rows, Y: y_bs elements)
+  long long y_bs;
+  int scale_ld;             // PAIR_ROWSCALE: scale of token t and problem z: row_scale[t * scale_ld + z]
 };
 
 // ---------------------------------------------------------------- cta_group::2 forms
@@ -113,6 +116,10 @@ __device__ __forceinline__ float pair_act(float v, float s) {
   if constexpr (MODE == PAIR_RELU2) {
     const float z = fmaxf(v * s, 0.f);
     return z * z;
+  } else if constexpr (MODE == PAIR_TANH) {
+    return tanhf(v);
+  } else if constexpr (MODE == PAIR_ROWSCALE) {
+    return v * s;
   } else if constexpr (MODE == PAIR_GELU) {
     return 0.5f * v * (1.f + erff(v * 0.7071067811865476f));
   } else {
@@ -130,6 +137,7 @@ struct PairTile {
   int n0;          // first output column
   int row0, rows;  // token rows [row0, row0 + rows)
   int n;           // UMMA_N: rows rounded up to PAIR_UNIT
+  int z;           // problem
 };
 
 // Tiles of one pair in launch order: index pair, pair + pairs, ...
@@ -139,7 +147,7 @@ struct PairIter {
   const int* start;  // grouped: first tile of every segment [n_groups + 1] (shared memory)
   int i, step, total, g;
   __device__ PairIter(const PairArgs& a_, const int* start_, int pair, int pairs) : a(a_), start(start_), i(pair), step(pairs), g(0) {
-    total = GROUPED ? start[a.n_groups] : a.n_tiles * a.x_tiles;
+    total = GROUPED ? start[a.n_groups] : a.n_tiles * a.x_tiles * max(a.batch, 1);
   }
   __device__ bool next(PairTile& t) {
     if (i >= total) return false;
@@ -160,13 +168,16 @@ struct PairIter {
       rows = a.T;
       units = (rows + PAIR_UNIT - 1) / PAIR_UNIT;
       x_tiles = a.x_tiles;
-      const int full = NB * x_tiles, nb = i / full, rem = i - nb * full, nb_n = min(NB, a.n_tiles - nb * NB);
+      const int each = a.n_tiles * x_tiles, z = i / each, k = i - z * each;
+      const int full = NB * x_tiles, nb = k / full, rem = k - nb * full, nb_n = min(NB, a.n_tiles - nb * NB);
+      t.z = z;
       x_tile = rem / nb_n;
       n_tile = nb * NB + rem - x_tile * nb_n;
     }
     const int u0 = x_tile * units / x_tiles, u1 = (x_tile + 1) * units / x_tiles;
     t.n0 = n_tile * 256;
-    t.w_row = (GROUPED ? g * a.N : 0) + t.n0;
+    if (GROUPED) t.z = 0;
+    t.w_row = (GROUPED ? g : t.z) * a.N + t.n0;
     t.row0 = base + u0 * PAIR_UNIT;
     t.rows = min(rows - u0 * PAIR_UNIT, (u1 - u0) * PAIR_UNIT);
     t.n = (u1 - u0) * PAIR_UNIT;
@@ -180,10 +191,18 @@ template <int MODE, class OT>
 __device__ __forceinline__ void pair_store(const PairArgs& a, const PairTile& t, int n, uint32_t taddr, int lane) {
   constexpr bool GLU = MODE == PAIR_SWIGLU || MODE == PAIR_SWIGLU_BF16 || MODE == PAIR_GEGLU;
   const bool n_ok = GLU ? (n | 1) < a.N : n < a.N;
-  OT* y = reinterpret_cast<OT*>(a.Y) + (size_t)t.row0 * a.ldy + (GLU ? n >> 1 : n);
+  OT* y = reinterpret_cast<OT*>(a.Y) + (size_t)t.z * a.y_bs + (size_t)t.row0 * a.ldy + (GLU ? n >> 1 : n);
 #pragma unroll 1
   for (int c0 = 0; c0 < t.rows; c0 += 32, y += (size_t)32 * a.ldy) {
     uint32_t r[32];
+    // the scale of token c0 + lane: one load in flight for 32 tokens, not one behind the other per token (4096 rows of 1024 x 2048 in 8
+    // segments 77 -> 22 us; 16 heads of 128 x 512 at 2048 tokens 97 -> 18)
+    float scale = 1.f;
+    if constexpr (MODE == PAIR_RELU2) {
+      if (a.row_scale != nullptr && c0 + lane < t.rows) scale = a.row_scale[a.gather != nullptr ? a.gather[t.row0 + c0 + lane] : t.row0 + c0 + lane];
+    } else if constexpr (MODE == PAIR_ROWSCALE) {
+      if (c0 + lane < t.rows) scale = a.row_scale[(size_t)(t.row0 + c0 + lane) * a.scale_ld + t.z];
+    }
     tmem_ld_32x32b_x16(taddr + c0, r);
     tmem_ld_32x32b_x16(taddr + c0 + 16, r + 16);
     tmem_ld_wait();
@@ -219,14 +238,11 @@ __device__ __forceinline__ void pair_store(const PairArgs& a, const PairTile& t,
         if (2 * j < mine_valid) yl[(size_t)(2 * j) * a.ldy] = pair_out<OT>(v[j]);
     } else {
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (j < valid) {
-          float s = 1.f;
-          if constexpr (MODE == PAIR_RELU2) {
-            if (a.row_scale != nullptr) s = a.row_scale[a.gather != nullptr ? a.gather[t.row0 + c0 + j] : t.row0 + c0 + j];
-          }
-          y[(size_t)j * a.ldy] = pair_out<OT>(pair_act<MODE>(__uint_as_float(r[j]), s));
-        }
+      for (int j = 0; j < 32; ++j) {
+        float s = 1.f;
+        if constexpr (MODE == PAIR_RELU2 || MODE == PAIR_ROWSCALE) s = __shfl_sync(0xffffffffu, scale, j);
+        if (j < valid) y[(size_t)j * a.ldy] = pair_out<OT>(pair_act<MODE>(__uint_as_float(r[j]), s));
+      }
     }
   }
 }
@@ -308,13 +324,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       uint32_t phase = 0;
       bool ok = true;
       const uint32_t full0 = dsmem_addr(smem_u32(full_bar), 0);   // the leader's barriers
-      int w_row = 0, x_row = 0, boxes = 0;
+      int w_row = 0, x_row = 0, x_col = 0, boxes = 0;
       uint32_t bytes = 0;
       auto set_tile = [&]() {
         boxes = (t.n / 2 + GEMM_X_BOX_MANY - 1) / GEMM_X_BOX_MANY;
         bytes = 2u * (uint32_t)(PAIR_TILE_BYTES + boxes * X_BOX_BYTES);
         w_row = t.w_row + rank * 128;
         x_row = t.row0 + rank * (t.n / 2);
+        x_col = t.z * a.x_cs;
       };
       auto load_w = [&](int s, int kb) {
         if (rank == 0) mbar_arrive_expect_tx(&full_bar[s], bytes);
@@ -323,7 +340,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       auto load_x = [&](int s, int kb) {
 #pragma unroll
         for (int b = 0; b < 128 / GEMM_X_BOX_MANY; ++b)
-          if (b < boxes) tma_load_pair(&xmap, full0 + s * 8, smem_x + s * PAIR_TILE_BYTES + b * X_BOX_BYTES, kb * PAIR_BK, x_row + b * GEMM_X_BOX_MANY);
+          if (b < boxes) tma_load_pair(&xmap, full0 + s * 8, smem_x + s * PAIR_TILE_BYTES + b * X_BOX_BYTES, x_col + kb * PAIR_BK, x_row + b * GEMM_X_BOX_MANY);
       };
       bool have = it.next(t);
       if (have) set_tile();
@@ -411,6 +428,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
         case PAIR_GEGLU: pair_store<PAIR_GEGLU, bf>(a, t, n, taddr, lane); break;
         case PAIR_RELU2: pair_store<PAIR_RELU2, bf>(a, t, n, taddr, lane); break;
         case PAIR_GELU: pair_store<PAIR_GELU, bf>(a, t, n, taddr, lane); break;
+        case PAIR_TANH: pair_store<PAIR_TANH, bf>(a, t, n, taddr, lane); break;
+        case PAIR_ROWSCALE: pair_store<PAIR_ROWSCALE, bf>(a, t, n, taddr, lane); break;
         default:
           if (a.y_f32) pair_store<PAIR_PLAIN, float>(a, t, n, taddr, lane);
           else pair_store<PAIR_PLAIN, bf>(a, t, n, taddr, lane);
@@ -589,7 +608,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       tc_fence_after();
       if (sub * 32 < ra.R) {
         PairTile pt;
-        pt.n0 = 0; pt.w_row = 0;
+        pt.n0 = 0; pt.w_row = 0; pt.z = 0;
         pt.row0 = 0; pt.rows = a.T; pt.n = ra.n;
         const int n = row < ra.R ? (t * 2 + rank) * ra.R + row : a.N;
         const uint32_t taddr = tmem_base + acc * 256 + ((uint32_t)(sub * 32) << 16);
@@ -711,6 +730,44 @@ cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
   a.x_tiles = gemm_pair_plan(T, N, pairs);
   const int tiles = a.n_tiles * a.x_tiles;
   return launch_pair<false>(wmap, xmap, a, 2 * (tiles < pairs ? tiles : pairs), stream);
+}
+
+// Dense products of prompts that gemm_bf16_launch's layout does not cover: one per head side by side in the columns of X, few weight
+// rows (a router), a tanh, a scale per row and problem.  mma.sync tiles -> here, microseconds at 300 and 2048 tokens: 16 heads of
+// 512 x 128 14.0 -> 6.7 and 55 -> 20, 16 of 128 x 512 with scales 19.6 -> 7.7 and 28 -> 18, 65 x 2048 48 -> 10 and 48 -> 11, tanh 64 x 2048
+// 53 -> 13 and 53 -> 15, 2048 x 64 11.6 -> 5.2 and 12.9 -> 7.4; the errors against 64 bits are equal to all digits.  Up to 256 tokens the
+// register products and the warp per output have them; fewer than 32 weight rows would fill an eighth of a tile.
+bool gemm_pair_takes_dense(const GemmAny& a) {
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  const int batch = a.batch > 1 ? a.batch : 1;
+  const bool mode_ok = a.mode == GEMM_ANY_PLAIN || (a.y_dtype == DT_BF16 && (a.mode == GEMM_ANY_TANH || a.mode == GEMM_ANY_ROWSCALE));
+  return mode_ok && a.seg_off == nullptr && a.gather == nullptr && a.T > 256 && a.N >= 32 && a.K >= PAIR_BK && a.K % PAIR_BK == 0 &&
+         a.x_dtype == DT_BF16 && a.w_dtype == DT_BF16 && a.ldw == a.K && a.ldx % 8 == 0 && a.ldx >= a.K && al16(a.X) && al16(a.W) &&
+         (batch == 1 || (a.w_bs == (long long)a.N * a.K && a.x_bs % 8 == 0 && a.x_bs >= 0 && (long long)(batch - 1) * a.x_bs + a.K <= a.ldx)) &&
+         (long long)batch * a.N < (1ll << 31);
+}
+cudaError_t gemm_pair_dense_launch(const GemmAny& g, cudaStream_t stream) {
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const int batch = g.batch > 1 ? g.batch : 1, pairs = sms / 2;
+  if (pairs < 1) return cudaErrorInvalidValue;
+  const uint64_t cols = (uint64_t)g.K + (batch > 1 ? (uint64_t)(batch - 1) * g.x_bs : 0);
+  CUtensorMap wm, xm;
+  if (make_tmap_bf16_2d(&wm, g.W, (uint64_t)batch * g.N, g.K, g.K, 128, PAIR_BK) != 0 ||
+      make_tmap_bf16_2d(&xm, g.X, g.T, cols, g.ldx, GEMM_X_BOX_MANY, PAIR_BK) != 0)
+    return cudaErrorInvalidValue;
+  PairArgs a{};
+  a.Y = g.Y; a.ldy = g.ldy; a.T = g.T; a.N = g.N; a.K = g.K;
+  a.y_f32 = g.y_dtype == DT_F32;
+  a.mode = g.mode == GEMM_ANY_TANH ? PAIR_TANH : g.mode == GEMM_ANY_ROWSCALE ? PAIR_ROWSCALE : PAIR_PLAIN;
+  a.n_tiles = (g.N + 255) / 256;
+  a.x_tiles = gemm_pair_plan(g.T, a.n_tiles * 256 * batch, pairs);
+  a.row_scale = g.row_scale; a.scale_ld = g.scale_ld;
+  a.batch = batch; a.x_cs = batch > 1 ? (int)g.x_bs : 0; a.y_bs = batch > 1 ? g.y_bs : 0;
+  const long long tiles = (long long)a.n_tiles * a.x_tiles * batch;
+  return launch_pair<false>(wm, xm, a, 2 * (int)(tiles < pairs ? tiles : pairs), stream);
 }
 
 // The share of a product of N weight rows that one CTA of a pair takes: whole waves of pairs, an even number of rows

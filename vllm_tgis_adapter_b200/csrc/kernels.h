@@ -98,6 +98,8 @@ constexpr int PAIR_SWIGLU = 2;       // the same in fp32, rounded once
 constexpr int PAIR_GEGLU = 3;        // tanh form of gelu on the gate, fp32
 constexpr int PAIR_RELU2 = 4;        // max(acc * s, 0)^2
 constexpr int PAIR_GELU = 5;         // exact gelu
+constexpr int PAIR_TANH = 6;
+constexpr int PAIR_ROWSCALE = 7;     // times a scale per row (and problem)
 // wmap: boxes of 128 rows x 64; xmap: boxes of GEMM_X_BOX_MANY rows x 64; Y fp32 (y_f32) or bf16
 cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int y_f32, int mode, int T, int N,
                              int K, int num_sms, cudaStream_t stream);
@@ -322,6 +324,8 @@ struct GemmAny {
 };
 bool gemm_pair_takes_groups(const GemmAny& a);   // gemm_pair.cu
 cudaError_t gemm_pair_grouped_launch(const GemmAny& a, cudaStream_t stream);
+bool gemm_pair_takes_dense(const GemmAny& a);    // gemm_pair.cu
+cudaError_t gemm_pair_dense_launch(const GemmAny& a, cudaStream_t stream);
 bool gemm_skinny_takes_batch(const GemmAny& a);  // gemm_skinny.cu
 cudaError_t gemm_skinny_batch_launch(const GemmAny& a, cudaStream_t stream);
 cudaError_t gemm_any_launch(const GemmAny& a, cudaStream_t stream);
