@@ -18,7 +18,7 @@
 //            16 tokens x 16 ranks in eight parts of K a launch of a small step took 9.8 us instead of 6.6, one of 1300 tokens 74.)
 //   expand : CTA = (tile of 16 tokens, 512 output columns), warp = 64 columns: B rows as fragments of mma.sync straight from global
 //            memory, all requested in one round, each lane 8 neighbouring columns of 2 tokens.  24 tokens, four adapters of rank 16, 8B
-//            widths, microseconds a launch against multiply-adds from shared memory (8 tokens x 1024 columns): 6.3 -> 4.8, with SwiGLU 19.8 -> 11.3.
+//            widths, microseconds a launch against multiply-adds from shared memory (8 tokens x 1024 columns): 6.3 -> 4.0, with SwiGLU 19.8 -> 10.4.
 // Both are launches of a few microseconds of dependent loads.  The engine runs shrink BEFORE the base projection, which it
 // does not depend on: the projection's first weights are on their way while it runs.
 // Adapter storage (engine.cu): per layer and module  A [slots][Rm][K] and B [slots][N][Rm] bf16, zero padded to the module's
@@ -105,13 +105,15 @@ __device__ __forceinline__ F8 cvt8(const uint4& r) {
 // instead of a handful of warps walking a whole row (the first version: 16 .. 56 serial memory latencies per launch), and
 // the tile's x vectors are loaded once for the four rows (one row per CTA made a prefill chunk L2-bandwidth bound:
 // 16 CTAs re-read the same 64 KB of x).  Partial sums meet in shared memory and are added in warp order: deterministic.
+// A launch is a chain of latencies: rows of A are asked for under the kernel before and a round ahead, 32 sums meet in 31 exchanges
+// instead of 160, the modules' table is read from the parameters instead of a copy in local memory (24 requests with adapters, average
+// launch, microseconds: 8.1 -> 7.3, the expands 4.8 -> 4.0 and 11.3 -> 10.4 by the last of these).
 constexpr int LORA_RPC = 4;
 __global__ void __launch_bounds__(256)
-lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* __restrict__ tok_slot, LoraGroup g,
+lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* __restrict__ tok_slot, const __grid_constant__ LoraGroup g,
                    float* __restrict__ v, int T) {
   __shared__ float part[8][LORA_RPC][LORA_ST];
   griddep_launch();
-  griddep_wait();
   int m = 0, r0 = (int)blockIdx.y * LORA_RPC;  // blockIdx.y enumerates (module, group of LORA_RPC rank rows)
   while (m + 1 < g.n_mods && r0 >= g.mod[m].Rm) {
     r0 -= g.mod[m].Rm;
@@ -124,37 +126,48 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* 
   const int nvec = md.K / 8;
   const uint4* xq = reinterpret_cast<const uint4*>(x);
   const size_t ldq = (size_t)ldx / 8;
-  for (int p = blockIdx.z;; p += gridDim.z) {
-    const int slot = tile.distinct(p, 1);
-    if (slot < 0) return;
-    float acc[LORA_RPC][LORA_ST];
-#pragma unroll
-    for (int q = 0; q < LORA_RPC; ++q)
-#pragma unroll
-      for (int j = 0; j < LORA_ST; ++j) acc[q][j] = 0.f;
+  bool first = true;
+  for (int p = blockIdx.z;; p += gridDim.z, first = false) {
+    const int slot = tile.distinct(p, 1);   // (slots and adapters are written ahead of the step: x alone is waited for)
+    if (slot < 0) {
+      if (first) griddep_wait();
+      return;
+    }
+    static_assert(LORA_RPC * LORA_ST == 32, "one sum per lane");
+    float acc[32] = {};
     const uint4* a0 = reinterpret_cast<const uint4*>(md.A + ((size_t)(slot - 1) * md.Rm + r0) * md.K);
-    for (int kv = warp * 32 + lane; kv < nvec; kv += 256) {
-      uint4 ar[LORA_RPC], xr[LORA_ST];
+    uint4 ar[LORA_RPC];
+    auto load_a = [&](int kv) {
 #pragma unroll
-      for (int q = 0; q < LORA_RPC; ++q) ar[q] = a0[(size_t)q * nvec + kv];
+      for (int q = 0; q < LORA_RPC; ++q) ar[q] = kv < nvec ? a0[(size_t)q * nvec + kv] : make_uint4(0u, 0u, 0u, 0u);
+    };
+    load_a(warp * 32 + lane);
+    if (first) griddep_wait();
+    for (int kv = warp * 32 + lane; kv < nvec; kv += 256) {
+      uint4 xr[LORA_ST];
 #pragma unroll
       for (int j = 0; j < LORA_ST; ++j) xr[j] = tile.s[j] == slot ? xq[(size_t)(t0 + j) * ldq + kv] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
       for (int j = 0; j < LORA_ST; ++j) {
         const F8 xf = cvt8(xr[j]);
 #pragma unroll
-        for (int q = 0; q < LORA_RPC; ++q) acc[q][j] += dot8(cvt8(ar[q]), xf);
+        for (int q = 0; q < LORA_RPC; ++q) acc[q * LORA_ST + j] += dot8(cvt8(ar[q]), xf);
       }
+      if (kv + 256 < nvec) load_a(kv + 256);
     }
+    // 32 sums over 32 lanes, each lane ends with one: 31 exchanges instead of 160, the same pairs added
 #pragma unroll
-    for (int q = 0; q < LORA_RPC; ++q)
+    for (int step = 0; step < 5; ++step) {
+      const int o = 16 >> step;
+      const bool upper = (lane & o) != 0;
 #pragma unroll
-      for (int j = 0; j < LORA_ST; ++j) {
-        float s = acc[q][j];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) part[warp][q][j] = s;
-      }
+      for (int i = 0; i < 16; ++i)
+        if (i < o) {
+          const float keep = upper ? acc[i + o] : acc[i], give = upper ? acc[i] : acc[i + o];
+          acc[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+    }
+    part[warp][lane / LORA_ST][lane % LORA_ST] = acc[0];
     __syncthreads();
     if (threadIdx.x < LORA_RPC * LORA_ST) {
       const int q = threadIdx.x / LORA_ST, j = threadIdx.x % LORA_ST;
@@ -180,7 +193,7 @@ constexpr int LORA_ECOLS = 512;   // columns per CTA of the expand: 8 warps x 64
 // written (for tokens without an adapter too) and y is only read: the projection's own kernel after it drops out.
 template <bool ACT>
 __global__ void __launch_bounds__(256, 2)
-lora_expand_kernel(const float* __restrict__ v, const int32_t* __restrict__ tok_slot, LoraGroup gr,
+lora_expand_kernel(const float* __restrict__ v, const int32_t* __restrict__ tok_slot, const __grid_constant__ LoraGroup gr,
                    __nv_bfloat16* __restrict__ y, int ldy, __nv_bfloat16* __restrict__ act, int T) {
   __shared__ __align__(16) __nv_bfloat16 vs[LORA_TT][LORA_MAX_RM + 8];   // the tile's rank vectors
   griddep_launch();
