@@ -10,6 +10,8 @@
 //
 // Measured, microseconds with cold weights, N x K, tcgen05 -> here: 1 token 768 x 768 7.0 -> 2.7, 2048 x 2048 8.7 -> 4.0,
 // 4096 x 4096 12.6 -> 8.6; 32 tokens 768 x 768 8.1 -> 3.6, 2048 x 2048 9.8 -> 5.4 (6144 x 4096 17.7 -> 20.1).
+#include <type_traits>
+
 #include "kernels.h"
 #include "launch.cuh"
 #include "ptx.cuh"
@@ -19,9 +21,14 @@ namespace {
 
 struct SkinnyArgs {
   const __nv_bfloat16* X; const __nv_bfloat16* W; void* Y;
-  int ldx, ldy, T, N, K, mode;   // mode: the out modes of gemm_bf16_launch
-  GemmRope rope;                 // positions == nullptr: none
-  long long x_bs, w_bs, y_bs;    // elements between the problems of blockIdx.y
+  int ldy, T, N, K, mode;   // mode: the out modes of gemm_bf16_launch
+  GemmRope rope;            // positions == nullptr: none
+};
+// The problems of blockIdx.y side by side.  A type of its own: as members of SkinnyArgs, zero for one problem, these cost every launch of
+// a chain 0.13 us (768 x 768, one token 3.24 -> 3.37; a request on a 12-layer model 4.43 -> 4.53 ms).
+struct SkinnyBatch : SkinnyArgs {
+  int ldx;
+  long long x_bs, w_bs, y_bs;    // elements between the problems
   const float* row_scale;        // modes 0 and 1: result times row_scale[token * scale_ld + problem] (nullptr: 1)
   int scale_ld;
 };
@@ -46,15 +53,21 @@ __device__ __forceinline__ float skinny_glu(int mode, float g, float u) {
 
 // MT: 16-row weight tiles per CTA, NT: 8-token tiles, WARPS: k-splits (warp w takes the chunks w, w + WARPS, ...).
 // ROPE (MT = 2): the CTA's two tiles are the dims [16 q, 16 q + 16) of one head and their rotary partners, 64 dims on.
-template <int MT, int NT, int WARPS, bool ROPE>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_kernel(const SkinnyArgs a) {
+template <int MT, int NT, int WARPS, bool ROPE, class Args>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_kernel(const Args a) {
+  constexpr bool BATCH = std::is_same<Args, SkinnyBatch>::value;
   constexpr int R = 16 * MT, TT = 8 * NT, LD = R + 1;
   extern __shared__ __align__(16) float part[];   // [WARPS][TT][LD]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int n0 = ROPE ? (blockIdx.x >> 2) * HEAD_DIM + (blockIdx.x & 3) * 16 : blockIdx.x * R;
   constexpr int M_STEP = ROPE ? 64 : 16;
-  const __nv_bfloat16* X = a.X + (size_t)blockIdx.y * a.x_bs;
-  const __nv_bfloat16* W = a.W + (size_t)blockIdx.y * a.w_bs;
+  const __nv_bfloat16 *X = a.X, *W = a.W;
+  int ldx = a.K;
+  if constexpr (BATCH) {
+    X += (size_t)blockIdx.y * a.x_bs;
+    W += (size_t)blockIdx.y * a.w_bs;
+    ldx = a.ldx;
+  }
   if (threadIdx.x < MT) {   // weights are static: the CTA's rows (one run of bytes per tile) start on their way to L2
     const int row = n0 + (int)threadIdx.x * M_STEP, bytes = min(16, a.N - row) * a.K * 2;
     const char* from = reinterpret_cast<const char*>(W + (size_t)row * a.K);
@@ -70,7 +83,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_k
     for (int h = 0; h < 2; ++h) wr[m][h] = W + (size_t)min(n0 + m * M_STEP + h * 8 + g, a.N - 1) * a.K + t * 8;
   const __nv_bfloat16* xr[NT];
 #pragma unroll
-  for (int n = 0; n < NT; ++n) xr[n] = X + (size_t)min(n * 8 + g, a.T - 1) * a.ldx + t * 8;
+  for (int n = 0; n < NT; ++n) xr[n] = X + (size_t)min(n * 8 + g, a.T - 1) * ldx + t * 8;
   float acc[MT][NT][4];
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -167,8 +180,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_k
       const int tok = i / R, j = i % R;
       if (n0 + j >= a.N) continue;
       float v = sum(tok, j);
-      if (a.row_scale != nullptr) v *= a.row_scale[(size_t)tok * a.scale_ld + blockIdx.y];
-      const size_t o = (size_t)blockIdx.y * a.y_bs + (size_t)tok * a.ldy + n0 + j;
+      size_t o = (size_t)tok * a.ldy + n0 + j;
+      if constexpr (BATCH) {
+        if (a.row_scale != nullptr) v *= a.row_scale[(size_t)tok * a.scale_ld + blockIdx.y];
+        o += (size_t)blockIdx.y * a.y_bs;
+      }
       if (a.mode == 1) {
         reinterpret_cast<float*>(a.Y)[o] = v;
       } else {
@@ -182,16 +198,16 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_k
   }
 }
 
-template <int MT, int NT, int WARPS, bool ROPE>
-cudaError_t launch(const SkinnyArgs& a, cudaStream_t s, int problems = 1) {
+template <int MT, int NT, int WARPS, bool ROPE, class Args>
+cudaError_t launch(const Args& a, cudaStream_t s, int problems = 1) {
   constexpr size_t smem = (size_t)WARPS * 8 * NT * (16 * MT + 1) * sizeof(float);
   static const cudaError_t attr =
-      cudaFuncSetAttribute(gemm_skinny_kernel<MT, NT, WARPS, ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      cudaFuncSetAttribute(gemm_skinny_kernel<MT, NT, WARPS, ROPE, Args>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (attr != cudaSuccess) return attr;
-  return launch_k(gemm_skinny_kernel<MT, NT, WARPS, ROPE>, dim3((a.N + 16 * MT - 1) / (16 * MT), problems), dim3(WARPS * 32), smem, s, a);
+  return launch_k(gemm_skinny_kernel<MT, NT, WARPS, ROPE, Args>, dim3((a.N + 16 * MT - 1) / (16 * MT), problems), dim3(WARPS * 32), smem, s, a);
 }
-template <int MT, int WARPS, bool ROPE>
-cudaError_t launch_nt(const SkinnyArgs& a, cudaStream_t s, int problems = 1) {
+template <int MT, int WARPS, bool ROPE, class Args>
+cudaError_t launch_nt(const Args& a, cudaStream_t s, int problems = 1) {
   switch ((a.T + 7) / 8) {
     case 1: return launch<MT, 1, WARPS, ROPE>(a, s, problems);
     case 2: return launch<MT, 2, WARPS, ROPE>(a, s, problems);
@@ -214,7 +230,7 @@ bool gemm_skinny_takes(int T, int N, int K) {
 
 cudaError_t gemm_skinny_launch(const void* X, const void* W, void* Y, int ldy, int T, int N, int K, int out_mode, const GemmRope* rope,
                                cudaStream_t stream) {
-  SkinnyArgs a{(const __nv_bfloat16*)X, (const __nv_bfloat16*)W, Y, K, ldy, T, N, K, out_mode, {}, 0, 0, 0, nullptr, 0};
+  SkinnyArgs a{(const __nv_bfloat16*)X, (const __nv_bfloat16*)W, Y, ldy, T, N, K, out_mode, {}};
   // The number of warps, and with it the order of k, hangs on N alone: a row has the same bits beside 31 others as alone, and with
   // every epilogue.  Sixteen warps where an SM holds one CTA, of 16 rows up to one wave, of 32 rows up to two; eight beyond that,
   // with 32-row CTAs for few tokens (more loads in flight) and 16-row ones beyond eight (fewer activation bytes in flight per
@@ -241,8 +257,8 @@ bool gemm_skinny_takes_batch(const GemmAny& a) {
          a.x_bs % 8 == 0 && a.w_bs % 8 == 0 && al16(a.X) && al16(a.W);
 }
 cudaError_t gemm_skinny_batch_launch(const GemmAny& g, cudaStream_t stream) {
-  SkinnyArgs a{(const __nv_bfloat16*)g.X, (const __nv_bfloat16*)g.W, g.Y, g.ldx, g.ldy, g.T, g.N, g.K, g.y_dtype == DT_F32 ? 1 : 0, {},
-               g.x_bs, g.w_bs, g.y_bs, g.mode == GEMM_ANY_ROWSCALE ? g.row_scale : nullptr, g.scale_ld};
+  const SkinnyBatch a{{(const __nv_bfloat16*)g.X, (const __nv_bfloat16*)g.W, g.Y, g.ldy, g.T, g.N, g.K, g.y_dtype == DT_F32 ? 1 : 0, {}},
+                      g.ldx, g.x_bs, g.w_bs, g.y_bs, g.mode == GEMM_ANY_ROWSCALE ? g.row_scale : nullptr, g.scale_ld};
   return g.K <= 256 ? launch_nt<1, 4, false>(a, stream, g.batch) : launch_nt<1, 8, false>(a, stream, g.batch);
 }
 
