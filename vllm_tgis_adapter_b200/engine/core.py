@@ -144,7 +144,7 @@ def _int32_array(values):
         try:
             buf = array("i", values)
             return (C.c_int32 * len(buf)).from_buffer(buf)
-        except OverflowError:   # (ctypes wraps what does not fit)
+        except (OverflowError, TypeError):   # (ctypes wraps what does not fit and takes its own integers)
             pass
     return (C.c_int32 * len(values))(*values)
 
