@@ -84,3 +84,17 @@ def test_a_row_has_the_same_bits_whole_in_portions_and_beside_others(g, n_q, n_k
     cuts = [0, 2, 33, 64, 200, 511, 513, 700]
     portions = torch.cat([case.run([(2, 0, 9), (0, a, b)])[1] for a, b in zip(cuts, cuts[1:])])
     assert torch.equal(whole, portions)
+
+
+def test_keys_that_score_minus_infinity_weigh_nothing(g):
+    """Keys 0 .. 131 score -inf under every query: a whole 128-token tile without a finite score, then part of one."""
+    case = Case(g, 8, 2, [300], seed=11)
+    case.q[0][..., 0] = case.q[0][..., 0].abs() + 0.125
+    case.k[case.slots[0][:132], :, 0] = -math.inf
+    case.kc = g.k_cache_from_dense(case.k, case.bt.shape[1])
+    want = case.exact(0, 0, 300)
+    assert bool(want[:132].isnan().all()) and bool(want[132:].isfinite().all())
+    got = case.run([(0, 0, 300)])[0].double()
+    assert bool(got[:132].isnan().all())
+    bound = 1.001 * 2 ** -8 * want.abs() + 5 * (2 ** -16 + 100 * 2 ** -19)   # as above
+    assert float(((got - want).abs() - bound)[132:].max()) <= 0.0

@@ -402,7 +402,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
             tmem_st_x16(o_t + c * 16, o);
           }
         }
-        const uint64_t neg_m = pack2(-m, -m);
+        const float ref = m == -INFINITY ? 0.f : m;   // (no score above -inf so far: every probability is 0, not the NaN of inf - inf)
+        const uint64_t neg_m = pack2(-ref, -ref);
         uint64_t sum0 = 0, sum1 = 0;
 #pragma unroll
         for (int c = 0; c < 2 * PT_BLOCKS; ++c) {
