@@ -98,3 +98,31 @@ def test_keys_that_score_minus_infinity_weigh_nothing(g):
     assert bool(got[:132].isnan().all())
     bound = 1.001 * 2 ** -8 * want.abs() + 5 * (2 ** -16 + 100 * 2 ** -19)   # as above
     assert float(((got - want).abs() - bound)[132:].max()) <= 0.0
+
+
+@pytest.mark.parametrize("n_q,n_kv,scale", [(8, 2, 128 ** -0.5), (2, 2, 128 ** -0.5), (8, 1, 128 ** -0.5), (6, 2, -0.05)])
+def test_values_that_are_not_finite_reach_only_the_rows_that_see_them(g, n_q, n_kv, scale):
+    """Infinities and a NaN in the values of later tokens, and in the cache behind the sequence: a row in front of them is what it is
+    without them; a row that sees one has numbers that are not finite in that dim, and its own in the others."""
+    case = Case(g, n_q, n_kv, [420], seed=5)
+    blocks = case.bt.shape[1]
+    k, v = case.slots[0], case.v.clone()
+    clean = case.run([(0, 0, 420)], scale)[0]
+    bad = ((70, 3, math.inf), (260, 127, -math.inf), (300, 64, math.nan))   # (position, dim, value) in the last kv head
+    for t, d, x in bad:
+        case.v[k[t], n_kv - 1, d] = x
+    case.vc = g.v_cache_from_dense(case.v, blocks)
+    behind = case.vc.view(blocks, n_kv, 32, 128)[int(case.bt[0, -1])]        # positions 416 .. 447: four are the sequence's
+    behind[:, 4:] = math.inf
+    got = case.run([(0, 0, 420)], scale)[0]
+    case.v = v
+    want = case.exact(0, 0, 420, scale)
+    sees = torch.zeros(420, n_q, 128, dtype=torch.bool, device="cuda")
+    for t, d, _ in bad:
+        sees[t:, n_q - n_q // n_kv:, d] = True
+    assert not bool(got[sees].isfinite().any())
+    bound = 1.001 * 2 ** -8 * want.abs() + 5 * (2 ** -16 + 100 * 2 ** -19)   # as above
+    assert float(((got.double() - want).abs() - bound)[~sees].max()) <= 0.0
+    if n_kv > 1:   # the last block reaches the last unit of the other heads alone: the rows in front keep their bits
+        first = 420 - 2 * (128 // (n_q // n_kv) // 8 * 8) - 1
+        assert torch.equal(got[:first, : n_q // n_kv], clean[:first, : n_q // n_kv])

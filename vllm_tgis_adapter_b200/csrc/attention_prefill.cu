@@ -14,8 +14,11 @@
 // columns) and low parts (64 columns: 16 mantissa bits in all, so that the result tracks an fp32 softmax), and the tensor cores
 // read them from there: O += P_hi V + P_lo V.  The two accumulators alternate, so one's softmax runs under the other's products.
 // The running maximum a row's sums refer to moves only when a score exceeds it by 2^8 (the sums are in fp32, so nothing is
-// lost below it); a warp scales its part of O only then.  A row's bits depend on its own keys alone: tiles are counted from the
-// sequence's first token, and what another row or request does changes neither order nor reference of its sums.
+// lost below it); a warp scales its part of O only then (the conditional rescaling published with FlashAttention-4).  A row's bits
+// depend on its own keys alone: tiles are counted from the sequence's first token, and what another row or request does changes
+// neither order nor reference of its sums.  The one thing that reaches a row from a key it does not see is a value that is not
+// finite: the tensor cores add 0 * V.  A row that comes out with such numbers although its own scores are finite is summed again over
+// its own keys alone (sum_again), without the matrix instructions: its bits are then those of another order, and its numbers right.
 //
 // What bounds it: the tensor pipe, 3 x 128 x 128 x 128 multiply-adds a tile (S once, P V twice) -- two thirds busy on an SM that has
 // work, the rest goes to the way S -> softmax -> P V of one accumulator where it is longer than the other's products -- and whole
@@ -49,11 +52,11 @@ constexpr size_t PT_SMEM = (size_t)(2 + 2 * PT_STAGES) * PT_TILE_BYTES + 1024 + 
 constexpr float PT_SLACK = 8.f;                          // exp2 domain: how far a score may exceed its row's reference
 
 struct PrefillArgs {
-  const __nv_bfloat16* k_cache;
+  const __nv_bfloat16 *qkv, *k_cache, *v_cache;
   const PrefillUnit* units;
   const int32_t* block_table;
   __nv_bfloat16* out;
-  int n_units, bt_stride, out_ld, n_kv, G, TM;
+  int n_units, bt_stride, qkv_ld, out_ld, n_kv, G, TM;
   float sl2;                                             // |scale| * log2(e)
   uint32_t minus;                                        // scale < 0: bit "negate A" of the score products' descriptor
   int* err;
@@ -177,6 +180,77 @@ struct UnitIter {
   }
 };
 
+// dims 4 lane .. 4 lane + 3 of a token of a V block
+__device__ __forceinline__ const __nv_bfloat16* value_of(const __nv_bfloat16* block, int token, int lane) {
+  return block + token * HEAD_DIM + ((lane >> 1) ^ (token & 7)) * 8 + (lane & 1) * 4;
+}
+// One row by a warp, the two passes of a softmax in the order of the keys: lane = token for the scores, lane = four dims for the values.
+__device__ __forceinline__ void attend_row(const PrefillArgs& a, int block_row, int kvh, int head, int row, int pos) {
+  const int lane = (int)lane_id();
+  const float sl2 = a.minus != 0 ? -a.sl2 : a.sl2;
+  const uint4* q = reinterpret_cast<const uint4*>(a.qkv + (size_t)row * a.qkv_ld + (size_t)head * HEAD_DIM);
+  auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
+  auto hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
+  auto tile_of = [&](int b) { return ((size_t)a.block_table[(size_t)block_row * a.bt_stride + b] * a.n_kv + kvh) * (KV_BLOCK * HEAD_DIM); };
+  auto score = [&](int b) {   // of the lane's token of block b
+    if (b * KV_BLOCK + lane > pos) return -INFINITY;
+    const __nv_bfloat16* from = a.k_cache + tile_of(b) + lane * 8;
+    float s = 0.f;
+#pragma unroll 2
+    for (int c = 0; c < HEAD_DIM / 8; ++c) {
+      const uint4 k = *reinterpret_cast<const uint4*>(from + c * (KV_BLOCK * 8)), x = q[c];
+      s = fmaf(lo(x.x), lo(k.x), s); s = fmaf(hi(x.x), hi(k.x), s);
+      s = fmaf(lo(x.y), lo(k.y), s); s = fmaf(hi(x.y), hi(k.y), s);
+      s = fmaf(lo(x.z), lo(k.z), s); s = fmaf(hi(x.z), hi(k.z), s);
+      s = fmaf(lo(x.w), lo(k.w), s); s = fmaf(hi(x.w), hi(k.w), s);
+    }
+    return s * sl2;
+  };
+  float m = -INFINITY, l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+  for (int b = 0; b <= pos / KV_BLOCK; ++b) m = fmaxf(m, score(b));
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, i));
+#pragma unroll 1
+  for (int b = 0; b <= pos / KV_BLOCK; ++b) {
+    const float p = ex2(score(b) - m);
+    l += p;
+    const int n = min(KV_BLOCK, pos - b * KV_BLOCK + 1);   // (hidden keys are not touched)
+#pragma unroll 4
+    for (int t = 0; t < n; ++t) {
+      const float w = __shfl_sync(0xffffffffu, p, t);
+      const uint2 v = *reinterpret_cast<const uint2*>(value_of(a.v_cache + tile_of(b), t, lane));
+      o[0] = fmaf(w, lo(v.x), o[0]); o[1] = fmaf(w, hi(v.x), o[1]);
+      o[2] = fmaf(w, lo(v.y), o[2]); o[3] = fmaf(w, hi(v.y), o[3]);
+    }
+  }
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) l += __shfl_xor_sync(0xffffffffu, l, i);
+  const float inv = 1.f / l;
+  *reinterpret_cast<uint2*>(a.out + (size_t)row * a.out_ld + (size_t)head * HEAD_DIM + lane * 4) =
+      make_uint2(cvt2(o[0] * inv, o[1] * inv), cvt2(o[2] * inv, o[3] * inv));
+}
+
+// The CTA's rows that came out with numbers that are not finite, by its softmax warps, which have stored them all.  Where the value of
+// a row's own token accounts for them (a token that has overflowed in full, and all that follow it in the next layers) they stand.
+__device__ __noinline__ void sum_again(const PrefillArgs& a) {
+  const int lane = (int)lane_id();
+  auto odd = [](const uint2& w) {   // one bit per number of four
+    const uint32_t e = 0x7f80u;
+    return ((w.x & e) == e) | ((w.x >> 16 & e) == e) << 1 | ((w.y & e) == e) << 2 | ((w.y >> 16 & e) == e) << 3;
+  };
+  Unit u;
+  for (UnitIter it(a); it.next(u);)
+    for (int r = threadIdx.x >> 5; r < u.rows * a.G; r += PT_WARP_COPY) {
+      const int t = r / a.G, row = u.row0 + t, head = u.kvh * a.G + r - t * a.G, pos = u.pos0 + t;
+      const int mine = odd(*reinterpret_cast<const uint2*>(a.out + (size_t)row * a.out_ld + (size_t)head * HEAD_DIM + lane * 4));
+      if (!__any_sync(0xffffffffu, mine != 0)) continue;
+      const int block = a.block_table[(size_t)u.block_row * a.bt_stride + pos / KV_BLOCK], slot = pos % KV_BLOCK;
+      const int own = odd(*reinterpret_cast<const uint2*>(value_of(a.v_cache + ((size_t)block * a.n_kv + u.kvh) * (KV_BLOCK * HEAD_DIM), slot, lane)));
+      if (__any_sync(0xffffffffu, (mine & ~own) != 0)) attend_row(a, u.block_row, u.kvh, head, row, pos);
+    }
+}
+
 __global__ void __launch_bounds__(PT_THREADS, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap vmap, const __grid_constant__ PrefillArgs a) {
   extern __shared__ uint8_t smem_raw[];
@@ -195,6 +269,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   uint64_t* o_full = p_full + 2;            // [2]
   uint32_t* tmem_base_smem = reinterpret_cast<uint32_t*>(o_full + 2);
   volatile int* gave_up = reinterpret_cast<volatile int*>(tmem_base_smem + 1);
+  volatile int* redo = gave_up + 1;         // rows of the CTA have to be summed again
 
   const int warp = threadIdx.x >> 5, lane = (int)lane_id();
   if (warp == PT_WARP_MMA) {
@@ -213,6 +288,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         mbar_init(&o_full[i], 1);
       }
       *gave_up = 0;
+      *redo = 0;
       fence_barrier_init();
     }
     __syncwarp();
@@ -444,6 +520,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
       const float inv = 1.f / l;
       const bool wanted = tok < a.TM && g * a.TM + tok < u.rows;
       __nv_bfloat16* dst = a.out + (size_t)(u.row0 + g * a.TM + tok) * a.out_ld + (size_t)(u.kvh * a.G + head) * HEAD_DIM;
+      float odd = 0.f;   // NaN where numbers of the row are not finite (taken eight at a time: all of them at once spill)
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         uint32_t o[32];
@@ -455,16 +532,23 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
             uint32_t w[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) w[k] = cvt2(__uint_as_float(o[i * 8 + 2 * k]) * inv, __uint_as_float(o[i * 8 + 2 * k + 1]) * inv);
+            float z = 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) z += __uint_as_float(o[i * 8 + k]);
+            odd = fmaf(z, 0.f, odd);
             *reinterpret_cast<uint4*>(dst + c * 32 + i * 8) = make_uint4(w[0], w[1], w[2], w[3]);
           }
         }
       }
       tc_fence_before();
+      if (wanted && l - l == 0.f && odd != 0.f) *redo = 1;
     }
   }
   if (!ok && lane == 0) *gave_up = 1;
   tc_fence_before();
   __syncthreads();
+  // rows whose numbers may come from keys that they do not see (registers: only the softmax warps have enough)
+  if (*redo != 0 && *gave_up == 0 && warp < PT_WARP_COPY) sum_again(a);
   // after a wait that ran out copies and MMAs of the other roles may be in flight; they are done long before this millisecond is over
   if (*gave_up)
     for (const long long t0 = clock64(); clock64() - t0 < 2000000ll;) {}
@@ -507,9 +591,9 @@ cudaError_t attn_prefill_launch(const __nv_bfloat16* qkv, int qkv_ld, const __nv
   PrefillArgs a{};
   cudaError_t e = gemm_pair_word(&a.err);
   if (e != cudaSuccess) return e;
-  a.k_cache = k_cache; a.units = units; a.block_table = block_table;
+  a.qkv = qkv; a.k_cache = k_cache; a.v_cache = v_cache; a.units = units; a.block_table = block_table;
   a.out = out;
-  a.n_units = n_units * n_kv; a.bt_stride = bt_stride; a.out_ld = out_ld; a.n_kv = n_kv; a.G = G; a.TM = accumulator_tokens(G);
+  a.n_units = n_units * n_kv; a.bt_stride = bt_stride; a.qkv_ld = qkv_ld; a.out_ld = out_ld; a.n_kv = n_kv; a.G = G; a.TM = accumulator_tokens(G);
   a.sl2 = scale != 0.f ? fabsf(scale) * 1.4426950408889634f : 1e-30f;   // hidden scores are -inf before they are scaled
   a.minus = scale < 0.f ? 1u << 13 : 0u;
   CUtensorMap qm, vm;
