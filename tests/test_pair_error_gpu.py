@@ -88,6 +88,21 @@ def test_a_wait_that_runs_out_inside_the_step_is_reported(lib):
     eng.close()
 
 
+def test_a_step_that_fails_leaves_the_callers_buffer_alone(lib, monkeypatch):
+    eng, made = _engine(), []
+
+    def full(shape, dtype):
+        made.append(np.full(shape, 7.0, dtype))
+        return made[-1]
+
+    monkeypatch.setattr(np, "empty", full)
+    lib.tgis_k_pair_fault(1)
+    with pytest.raises(EngineError, match="wait ran out"):
+        _replay(eng)
+    assert len(made) == 1 and made[0].size > 4096 and bool((made[0] == 7.0).all())
+    eng.close()
+
+
 def test_kernel_hooks_report_it(lib):
     x, w, y = (torch.zeros(512, 512, device="cuda", dtype=torch.bfloat16) for _ in range(3))
     p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731

@@ -3602,8 +3602,18 @@ struct tgis_engine {
     ++n_graph_launches;
   }
 
+  // Memory of the caller's that results of this step go to.  It is usually fresh: its pages are faulted in while the device works
+  // (6 MB of logits: 0.5 ms of page faults that the conversion took before) and hold what they held, for the step may still fail.
+  struct Results {
+    char* at = nullptr;
+    size_t bytes = 0;
+    void fault_in() const {
+      for (size_t i = 0; i < bytes; i += 4096) __atomic_fetch_or(at + i, 0, __ATOMIC_RELAXED);
+      if (bytes > 0) __atomic_fetch_or(at + bytes - 1, 0, __ATOMIC_RELAXED);
+    }
+  };
   // returns number of sampled rows
-  int run_batch(std::vector<Sched>& batch) {
+  int run_batch(std::vector<Sched>& batch, const Results& results) {
     const tgis_config& c = cfg;
     const int H = c.hidden, V = c.vocab;
     int T = 0, n_dec = 0, n_tiles = 0, R = 0, max_dec_kv = 0, samp_complex = 0;
@@ -3759,7 +3769,7 @@ struct tgis_engine {
     exec_step(hdr);
     CK(cudaEventRecord(ev1, stream));
     const double t_launched = debug_launch ? now_s() : 0.0;
-    touch_results();
+    results.fault_in();
     wait_step_end();
     if (debug_launch) {
       t_after_wait = now_s();
@@ -3894,14 +3904,6 @@ struct tgis_engine {
   }
 
   // ------------------------------------------------------------------------------------------------ trace replay
-  // The caller's buffer for the rows wanted of this step, usually fresh memory: its pages are faulted in while the device works
-  // (6 MB of logits: 0.5 ms of page faults that the conversion below took before).
-  char* results_at = nullptr;
-  size_t results_bytes = 0;
-  void touch_results() {
-    for (size_t i = 0; i < results_bytes; i += 4096) reinterpret_cast<volatile char*>(results_at)[i] = 0;
-    results_bytes = 0;
-  }
   // n bf16 values as fp32
   static void widen(const bf16* from, float* to, size_t n) {
     size_t i = 0;
@@ -3997,9 +3999,7 @@ struct tgis_engine {
     if (!batch.empty()) {
       size_t wanted = 0;
       for (int i = 0; i < n_entries; ++i) wanted += (size_t)std::max(entries[i].n_want, 0);
-      results_at = reinterpret_cast<char*>(logits_out);
-      results_bytes = logits_out != nullptr ? wanted * cfg.vocab * sizeof(float) : 0;
-      run_batch(batch);
+      run_batch(batch, Results{reinterpret_cast<char*>(logits_out), logits_out != nullptr ? wanted * cfg.vocab * sizeof(float) : 0});
       ++n_steps;
       for (Sched& s : batch) s.r->n_computed += s.q_len;
       std::vector<int> rows;
@@ -4139,7 +4139,7 @@ struct tgis_engine {
     }
 
     // ---- run
-    run_batch(batch);
+    run_batch(batch, Results{});
     ++n_steps;
 
     // ---- post-process (vllm v1/core/sched/utils.py:94-130 check_stop)
