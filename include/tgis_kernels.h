@@ -41,9 +41,12 @@ int tgis_k_opt_embed(const void* tok_dev, const void* pos_dev, const void* tok_t
                      void* out_dev, int32_t T, int32_t hidden, int32_t vocab, int32_t n_pos_rows, int32_t offset);
 int tgis_k_rope_kv(void* qkv_dev, const int32_t* positions_host, const int32_t* slot_mapping_host,
                    const void* cos_sin_dev, void* k_cache_dev, void* v_cache_dev, int32_t T, int32_t n_q, int32_t n_kv);
-/* qkv projection y[T, (n_q + 2 n_kv) * 128] = x . w^T with RoPE and the KV-cache scatter fused into the GEMM's
- * split-tile reduction (cluster / DSMEM or global fix-up); returns 1 (and computes nothing) when the launch plan does not
- * split every weight tile */
+/* the kernel that a dense product goes to: 0 registers, 1 equal shares of weight rows, 2 / 3 CTA pairs (maps of their own / the
+ * caller's), 4 cut along k, 5 (ask_device != 0 only, needs a GPU) cut along k and reduced inside clusters; -1: bad shape */
+int tgis_k_gemm_route(int32_t T, int32_t N, int32_t K, int32_t num_sms, int32_t ask_device);
+/* qkv projection y[T, (n_q + 2 n_kv) * 128] = x . w^T with RoPE and the KV-cache scatter fused into the register product or into
+ * the split-tile reduction (cluster / DSMEM or global fix-up) of the one cut along k; returns 1 (and computes nothing) when the
+ * kernel that the shape goes to has no such form */
 int tgis_k_gemm_rope(const void* x_dev, const void* w_dev, void* y_dev, int32_t T, int32_t n_q, int32_t n_kv, int32_t K,
                      int32_t x_rows_alloc, const int32_t* positions_host, const int32_t* slot_mapping_host,
                      const void* cos_sin_dev, void* k_cache_dev, void* v_cache_dev);

@@ -223,3 +223,26 @@ def test_fused_rope_epilogue_is_bit_identical(model, monkeypatch):
         runs.append([[(r.new_token, r.logprob, r.rank, tuple(r.topn)) for r in recs if r.new_token is not None]
                      for recs in outs])
     assert runs[0] == runs[1]
+
+
+def test_rope_stays_fused_beside_a_fused_norm(monkeypatch):
+    """With the norms inside the products the qkv product of every layer but the first is the one cut along k, which takes the rotary
+    embedding too, whatever kernel the first layer's goes to: two launches less a decode step in a stack of three, and the same bits."""
+    import dataclasses
+
+    from oracle.llama_oracle import CONFIGS
+    from vllm_tgis_adapter_b200.engine.core import make_sampling_params
+
+    monkeypatch.setitem(CONFIGS, "wide", dataclasses.replace(CONFIGS["tiny"], n_layers=3, hidden=2048, n_q_heads=32, n_kv_heads=8, ffn=1024))
+    rng = np.random.RandomState(17)
+    prompts = [rng.randint(3, 1024, size=3).tolist() for _ in range(32)]
+    sp, runs, launches = make_sampling_params(greedy=True, max_tokens=6, min_tokens=6, num_logprobs=2), [], []
+    monkeypatch.setenv("TGIS_FUSE_NORM", "1")
+    for flag in ("0", "1"):
+        monkeypatch.setenv("TGIS_FUSE_ROPE", flag)
+        _, _, outs, st = _run_engine("wide", prompts, sp, max_num_seqs=32, max_batched_tokens=512, kv_cache_bytes=64 << 20)
+        assert st.errored == 0
+        runs.append([[(r.new_token, r.logprob, r.rank, tuple(r.topn)) for r in recs if r.new_token is not None] for recs in outs])
+        launches.append(st.kernel_launches)
+    assert runs[0] == runs[1] and all(len(r) == 6 for r in runs[0])
+    assert launches[0] - launches[1] == 2 * 5

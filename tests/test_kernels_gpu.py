@@ -178,17 +178,37 @@ def test_rope_and_kv_scatter_bit_exact(g):
     assert torch.equal(v_dense[slots], qkv[:, cfg.n_q_heads + cfg.n_kv_heads:])
 
 
-@pytest.mark.parametrize("heads", [(24, 4), (32, 8)])
-@pytest.mark.parametrize("T", [32, 200])
-def test_qkv_gemm_with_fused_rope_epilogue_is_bit_identical(g, T, heads):
+CUT, CLUSTERS = 4, 5   # tgis_k_gemm_route
+FUSED_ROPE = [(17, (32, 8), 4096), (32, (32, 8), 4096), (64, (32, 8), 8192), (32, (24, 4), 4608), (100, (24, 4), 8192), (200, (24, 4), 8192)]
+
+
+@pytest.mark.parametrize("T,heads,K", FUSED_ROPE)
+def test_qkv_gemm_with_fused_rope_epilogue_is_bit_identical(g, T, heads, K):
+    """Reductions through distributed shared memory, which these shapes are cut for as long as their clusters fit the device."""
+    _fused_rope_is_bit_identical(g, T, heads, K, CLUSTERS)
+
+
+def test_qkv_gemm_with_fused_rope_epilogue_through_global_memory():
+    """The same shapes with the fix-up through global memory, for devices that hold fewer clusters (the choice is made once a process)."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    code = ("import sys; sys.path[:0] = ['tests', '.']; import tgis_gpu_utils as g, test_kernels_gpu as t\n"
+            "for case in t.FUSED_ROPE: t._fused_rope_is_bit_identical(g, *case, t.CUT)\nprint('all equal')")
+    r = subprocess.run([sys.executable, "-c", code], cwd=Path(__file__).resolve().parent.parent, env=dict(os.environ, TGIS_GEMM_CLUSTER="0"),
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "all equal" in r.stdout, r.stdout + r.stderr
+
+
+def _fused_rope_is_bit_identical(g, T, heads, K, route):
     """The qkv projection's split-tile reduction (gemm_tcgen05.cu) followed in the same kernel by RoPE + scatter into the
     paged K / V layouts, against the unfused pair (GEMM -> bf16 qkv, then rope_kvwrite_kernel): qkv rows and both caches
-    must be bit-identical.  32 heads = 32 weight tiles split 4 ways = clusters of 4 (reduction through distributed
-    shared memory); 48 heads (the Llama-3-8B shape) = 48 tiles split 3 ways, whose 48 clusters do not fit a 148-SM part
-    at once, so that shape takes the global-memory fix-up path."""
+    must be bit-identical.  The shapes are among those that the dispatch sends there."""
     import ctypes as C
 
-    (n_q, n_kv), K = heads, 1024
+    n_q, n_kv = heads
     n_heads = n_q + 2 * n_kv
     N = n_heads * 128
     torch.manual_seed(21)
@@ -207,9 +227,9 @@ def test_qkv_gemm_with_fused_rope_epilogue_is_bit_identical(g, T, heads):
     y1 = torch.zeros(T, N, dtype=torch.bfloat16, device="cuda")
     rc = g.lib().tgis_k_gemm_rope(g.ptr(x), g.ptr(w), g.ptr(y1), T, n_q, n_kv, K, rows, g.i32p(positions), g.i32p(slots),
                                   g.ptr(table), g.ptr(kc1), g.ptr(vc1))
-    assert rc in (0, 1), g.kerr()
-    if rc == 1:
-        pytest.skip("the launch plan does not split every tile on this device")
+    assert rc == 0, g.kerr()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert g.lib().tgis_k_gemm_route(T, N, K, sms, 1) == route
     y2 = torch.zeros(T, N, dtype=torch.bfloat16, device="cuda")
     ms = C.c_float(0)
     assert g.lib().tgis_k_gemm(g.ptr(x), g.ptr(w), g.ptr(y2), T, N, K, rows, 0, 1, C.byref(ms), 0) == 0, g.kerr()

@@ -3279,10 +3279,8 @@ struct tgis_engine {
       return g;
     };
     if (lora) ++lora_steps;
-    // (the products that are ahead of the one cut along k, by more than the rotary kernel takes, have no fused form)
-    const bool rope_fused = !pnx_on && !lora && fuse_rope && !cfg.debug_gemm_ref && !gemm_rows_takes(T, qkv_dim, H, num_sms) &&
-                            !gemm_small_pairs(T, H) && gemm_even_split(T, qkv_dim, H, num_sms) >= 2 &&
-                            T <= (qkv_cluster > 0 ? std::max(rope_fuse_max_t, rope_fuse_cluster_max_t) : rope_fuse_max_t);
+    const bool rope_wanted = !pnx_on && !lora && fuse_rope && !cfg.debug_gemm_ref && gemm_even_split(T, qkv_dim, H, num_sms) >= 2 &&
+                             T <= (qkv_cluster > 0 ? std::max(rope_fuse_max_t, rope_fuse_cluster_max_t) : rope_fuse_max_t);
     // residual add + RMSNorm inside the GEMMs either side of it (single GPU, small steps, both row-"producers" reduced
     // on chip): o-proj -> [post-attention norm] -> gate_up and down-proj -> [next layer's input norm] -> qkv
     const bool norm_fused = !pnx_on && !lora && fuse_norm && tp == 1 && !cfg.debug_gemm_ref && T <= GEMM_NORM_MAX_T && H % 128 == 0 && H / 128 <= GEMM_NORM_MAX_PARTS &&
@@ -3297,6 +3295,7 @@ struct tgis_engine {
       const GemmNorm cons_qkv{nullptr, nullptr, resid.p, ssq_mlp, l.ln1, n_parts, c.rms_eps};
       const GemmNorm cons_gu{nullptr, nullptr, resid.p, ssq_attn, l.ln2, n_parts, c.rms_eps};
       const bool qkv_norm_in = norm_fused && li > 0;
+      const bool rope_fused = rope_wanted && gemm_fuses_rope(T, qkv_dim, H, num_sms, !qkv_norm_in);
       {
         if (li == 0) {
           CK(rmsnorm_launch(resid.p, l.ln1, xn.p, T, H, c.rms_eps, stream));

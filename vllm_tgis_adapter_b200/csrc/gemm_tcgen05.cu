@@ -1191,27 +1191,34 @@ static int pair_mode(int out_mode) {   // 0 .. 4
   static const int modes[5] = {PAIR_PLAIN, PAIR_PLAIN, PAIR_SWIGLU_BF16, PAIR_GEGLU, PAIR_RELU2};
   return modes[out_mode];
 }
+GemmRoute gemm_route(int T, int N, int K, int num_sms, bool named) {
+  if (named && gemm_skinny_takes(T, N, K)) return GEMM_REGISTERS;
+  if (named && K % GEMM_BK == 0 && num_sms >= 2) {
+    if (gemm_rows_takes(T, N, K, num_sms)) return GEMM_SHARES;
+    if (gemm_small_pairs(T, K)) return GEMM_SMALL_PAIRS;
+  }
+  return gemm_takes_pairs(T, N, num_sms) ? GEMM_PAIRS : GEMM_CUT;
+}
+bool gemm_fuses_rope(int T, int N, int K, int num_sms, bool named) {
+  const GemmRoute route = gemm_route(T, N, K, num_sms, named);
+  return route == GEMM_REGISTERS || (route == GEMM_CUT && gemm_even_split(T, N, K, num_sms) >= 2);
+}
 // xmap must have been built with box_rows == gemm_x_box(T, N, num_sms)
 cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int T, int N, int K,
                              float* ws, int* counters, int num_sms, cudaStream_t stream, int out_f32,
                              const CUtensorMap* next_wmap, const GemmNext* next, const GemmRope* rope, const GemmNorm* norm,
                              const void* X, const void* W) {
-  if (X != nullptr && W != nullptr && norm == nullptr && gemm_skinny_takes(T, N, K) &&
-      ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) == 0 &&
-      (rope == nullptr || (out_f32 == 0 && N == (rope->n_q + 2 * rope->n_kv) * HEAD_DIM)))
-    return gemm_skinny_launch(X, W, Y, ldy, T, N, K, out_f32, rope, stream);
-  if (X != nullptr && W != nullptr && norm == nullptr && out_f32 >= 0 && out_f32 <= 4 && K % 64 == 0 && num_sms >= 2 &&
-      ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) == 0 &&
-      (rope == nullptr || (out_f32 == 0 && ldy == N && N == (rope->n_q + 2 * rope->n_kv) * HEAD_DIM))) {
-    cudaError_t e = cudaErrorNotSupported;
+  const bool named = X != nullptr && W != nullptr && norm == nullptr && ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
+  const GemmRoute route = gemm_route(T, N, K, num_sms, named);
+  if (rope != nullptr && (out_f32 != 0 || N != (rope->n_q + 2 * rope->n_kv) * HEAD_DIM || !gemm_fuses_rope(T, N, K, num_sms, named)))
+    return cudaErrorInvalidValue;
+  if (route == GEMM_REGISTERS) return gemm_skinny_launch(X, W, Y, ldy, T, N, K, out_f32, rope, stream);
+  if (route != GEMM_CUT) {
+    if (norm != nullptr || out_f32 < 0 || out_f32 > 4) return cudaErrorInvalidValue;
+    if (route == GEMM_SHARES) return gemm_rows_launch(X, W, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream);
     CUtensorMap xm;
-    if (gemm_rows_takes(T, N, K, num_sms)) e = gemm_rows_launch(X, W, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream);
-    else if (gemm_small_pairs(T, K) && make_tmap_bf16_2d(&xm, X, T, K, K, GEMM_X_BOX_MANY, 64) == 0)
-      e = gemm_pair_launch(wmap, xm, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream);
-    if (e == cudaSuccess && rope != nullptr)   // no fused form of these: the bits of a row are those of the product without it
-      e = rope_kvwrite_launch((__nv_bfloat16*)Y, rope->positions, rope->slot_mapping, rope->cos_sin, rope->k_cache, rope->v_cache, T, rope->n_q,
-                              rope->n_kv, stream);
-    if (e != cudaErrorNotSupported) return e;
+    if (route == GEMM_SMALL_PAIRS && make_tmap_bf16_2d(&xm, X, T, K, K, GEMM_X_BOX_MANY, 64) != 0) return cudaErrorInvalidValue;
+    return gemm_pair_launch(wmap, route == GEMM_SMALL_PAIRS ? xm : xmap, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream);
   }
   GemmRope rp{};
   if (rope) rp = *rope;
@@ -1220,10 +1227,6 @@ cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
   GemmNext nx{};
   if (next && next_wmap) nx = *next;
   const CUtensorMap& nm = (next && next_wmap) ? *next_wmap : wmap;
-  if (gemm_takes_pairs(T, N, num_sms)) {
-    if (rope != nullptr || norm != nullptr || out_f32 < 0 || out_f32 > 4) return cudaErrorInvalidValue;
-    return gemm_pair_launch(wmap, xmap, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream);
-  }
   const int nw = gemm_nw(T);
 #define TGIS_GEMM_CASE(B)                                                                                              \
   return nw == 2 ? launch_bt<B, 2>(wmap, xmap, Y, ldy, T, N, K, ws, counters, num_sms, out_f32, stream, nm, nx, rp, nr) \

@@ -85,6 +85,18 @@ struct GemmNorm {
 constexpr int GEMM_NORM_MAX_T = 64;
 constexpr int GEMM_NORM_MAX_PARTS = 64;  // hidden <= 8192
 int gemm_cluster_split(int T, int N, int K, int num_sms);
+// The kernel that gemm_bf16_launch sends a product to.  `named`: the caller gives X and W, on 16-byte boundaries, and fuses no norm.
+enum GemmRoute {
+  GEMM_REGISTERS = 0,    // gemm_skinny.cu
+  GEMM_SHARES = 1,       // gemm_pair.cu, equal shares of weight rows (gemm_rows_takes)
+  GEMM_SMALL_PAIRS = 2,  // gemm_pair.cu, maps made by the launch (gemm_small_pairs)
+  GEMM_PAIRS = 3,        // gemm_pair.cu, the caller's maps (gemm_takes_pairs)
+  GEMM_CUT = 4,          // gemm_tcgen05.cu, cut along k
+};
+GemmRoute gemm_route(int T, int N, int K, int num_sms, bool named);
+// ... and whether that kernel can fuse the rotary embedding (the products on pairs have no such form; what they are ahead by is more
+// than the rotary kernel takes)
+bool gemm_fuses_rope(int T, int N, int K, int num_sms, bool named);
 cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int T, int N, int K,
                              float* ws, int* counters, int num_sms, cudaStream_t stream, int out_f32 = 0,
                              const CUtensorMap* next_wmap = nullptr, const GemmNext* next = nullptr,

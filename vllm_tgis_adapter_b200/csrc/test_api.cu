@@ -183,14 +183,22 @@ int tgis_k_rope_kv(void* qkv_dev, const int32_t* positions_host, const int32_t* 
   return 0;
 }
 
-// qkv projection with the fused RoPE + KV-scatter epilogue (in the cluster or the global split-tile reduction).  Returns 1
-// when the launch plan does not split every tile (nothing computed), 0 on success.
+// The kernel that a dense product of named operands goes to (GemmRoute); ask_device: 5 where the one cut along k reduces inside
+// clusters (which depends on how many of them the device holds).
+int tgis_k_gemm_route(int32_t T, int32_t N, int32_t K, int32_t num_sms, int32_t ask_device) {
+  if (T <= 0 || N <= 0 || K <= 0 || num_sms <= 0) return kfail("bad shape");
+  const GemmRoute r = gemm_route(T, N, K, num_sms, true);
+  return ask_device && r == GEMM_CUT && gemm_cluster_split(T, N, K, num_sms) > 0 ? 5 : r;
+}
+
+// qkv projection with the fused RoPE + KV-scatter epilogue (of the register product, or in the cluster or the global split-tile
+// reduction).  Returns 1 when the kernel that the shape goes to has no such form (nothing computed), 0 on success.
 int tgis_k_gemm_rope(const void* x_dev, const void* w_dev, void* y_dev, int32_t T, int32_t n_q, int32_t n_kv, int32_t K,
                      int32_t x_rows_alloc, const int32_t* positions_host, const int32_t* slot_mapping_host,
                      const void* cos_sin_dev, void* k_cache_dev, void* v_cache_dev) {
   const int N = (n_q + 2 * n_kv) * HEAD_DIM;
   const int sms = test_num_sms();
-  if (gemm_even_split(T, N, K, sms) < 2) return 1;
+  if (!gemm_fuses_rope(T, N, K, sms, true)) return 1;
   CUtensorMap wm, xm;
   const int bt = gemm_pick_bt(T);
   if (x_rows_alloc < bt) return kfail("x must have at least one TMA box of rows allocated");
