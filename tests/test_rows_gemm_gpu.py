@@ -88,3 +88,32 @@ def test_expert_rows_with_a_scale_ahead_of_the_squared_relu(lib, N, K):
     want = a.clamp(min=0) ** 2
     assert ((y[:R].double() - want).abs() <= 2.0 ** -8 * want + 2 * a.abs() * slack + slack ** 2 + 1e-6 * want).all()
     assert bool((y[R] == 7.0).all())
+
+
+@pytest.mark.parametrize("N,K", [(6144, 4096), (28672, 2304), (768, 768), (2048, 2048), (9728, 512)])
+@pytest.mark.parametrize("tokens", [(33, 40, 48, 49, 64), (65, 66, 96, 128), (129, 200, 256)])
+def test_a_row_changes_its_bits_only_where_the_token_tiles_change(lib, N, K, tokens):
+    gen = torch.Generator(device="cuda").manual_seed(N + K)
+    x = torch.randn(256, K, generator=gen, device="cuda").bfloat16()
+    w = (torch.randn(N, K, generator=gen, device="cuda") * K ** -0.5).bfloat16()
+    rows = []
+    for T in tokens:
+        y, ms = torch.empty(T, N, device="cuda", dtype=torch.float32), C.c_float()
+        assert lib.tgis_k_gemm(p(x), p(w), p(y), T, N, K, 256, 0, 1, C.byref(ms), PLAIN_F32) == 0
+        rows.append(y)
+    assert all(torch.equal(r[: tokens[0]], rows[0]) for r in rows)
+
+
+@pytest.mark.parametrize("N,K,dt,tokens", [(64, 2048, 1, (1, 32, 33, 64, 65, 128, 129, 256)), (127, 512, 1, (64, 65, 256)), (96, 1024, 0, (1, 8, 64)), (96, 1024, 0, (65, 86, 128))])
+def test_a_row_of_a_tanh_map_has_the_same_bits_beside_many_others(lib, N, K, dt, tokens):
+    gen = torch.Generator(device="cuda").manual_seed(N + K)
+    to = torch.bfloat16 if dt else torch.float32
+    x, w = torch.randn(256, K, generator=gen, device="cuda").to(to), (torch.randn(N, K, generator=gen, device="cuda") * K ** -0.5).to(to)
+    rows = []
+    for T in tokens:
+        y = torch.empty(T, N, device="cuda")
+        assert lib.tgis_k_gemm_any(p(x), p(w), p(y), dt, dt, 0, T, N, K, K, K, N, 1, 0, 0, 0, None, 0, 0, None, 1, 4, None, 0) == 0
+        rows.append(y)
+    assert all(torch.equal(r[: tokens[0]], rows[0]) for r in rows)
+    want = torch.tanh(x[: len(y)].double() @ w.double().T)
+    assert float((y.double() - want).abs().max()) <= K / 8 * 2.0 ** -24 * float((x.double().abs() @ w.double().abs().T).max()) + 1e-6

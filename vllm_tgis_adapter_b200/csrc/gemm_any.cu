@@ -473,9 +473,12 @@ __global__ void __launch_bounds__(ANY_THREADS) gemm_any_rowdot_kernel(GemmAny a)
   }
 }
 bool rowdot_eligible(const GemmAny& a) {
-  // (with a tanh: the low-rank decay map of a step, 32 x 64 x 2048: one tile of the mma.sync kernel takes 38 us, this 3.7)
-  return a.seg_off == nullptr && a.batch <= 1 && (a.mode == GEMM_ANY_TANH || (a.mode == GEMM_ANY_PLAIN && a.y_dtype == DT_F32)) && a.N < 128 &&
-         (long long)a.T * a.N <= 8192 && a.K >= 256 && !(a.x_dtype == DT_BF16 && a.w_dtype == DT_F32);
+  // With a tanh (the low-rank decay map) the line lies in tokens alone, where other products change their kernel too.  bf16, K = 2048,
+  // microseconds, tiles of the mma.sync kernel -> here, 32, 64, 128 and 256 tokens: 64 outputs 32 35 53 53 -> 2.9 3.9 5.6 9.5, 127 outputs 32 37
+  // 55 55 -> 4.0 5.7 9.5 17.0; K = 4096, 64 outputs: 58 66 92 92 -> 4.0 5.8 8.5 14.9.  (More tokens: gemm_pair_takes_dense.)
+  const bool bf16 = a.x_dtype == DT_BF16 && a.w_dtype == DT_BF16;
+  const bool few = a.mode == GEMM_ANY_TANH ? a.T <= (bf16 ? 256 : 64) : a.mode == GEMM_ANY_PLAIN && a.y_dtype == DT_F32 && (long long)a.T * a.N <= 8192;
+  return a.seg_off == nullptr && a.batch <= 1 && few && a.N < 128 && a.K >= 256 && !(a.x_dtype == DT_BF16 && a.w_dtype == DT_F32);
 }
 template <class XT, class WT, bool VEC8 = false>
 cudaError_t launch_rowdot(const GemmAny& a, cudaStream_t stream) {

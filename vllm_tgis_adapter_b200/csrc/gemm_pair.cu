@@ -775,14 +775,16 @@ static int rows_share(int N, int pairs) {
   const int waves = (N + 256 * pairs - 1) / (256 * pairs), per = (N + 2 * pairs * waves - 1) / (2 * pairs * waves);
   return (per + 1) & ~1;
 }
-// At least 40 rows a CTA up to 64 tokens, eight from there (fewer rows: the cut along k or the pairs' token tiles are ahead); beyond 128
+// At least 40 rows a CTA up to 64 tokens, four from there (fewer rows: the cut along k or the pairs' token tiles are ahead); beyond 128
 // tokens only where the rows fill more than one wave; a long k only where its bytes take longer than its MMAs.  The measured
-// table stands at gemm_takes_pairs.
+// table stands at gemm_takes_pairs.  Every line in T is one at which the token tiles change anyway: a row's bits change nowhere else.
 bool gemm_rows_takes(int T, int N, int K, int num_sms) {
   if (T <= 16 || T > 256 || K % PAIR_BK != 0 || num_sms < 2) return false;
   const int pairs = num_sms / 2, R = rows_share(N, pairs);
   if (R < 56 && K > 4096) return false;
-  if (T <= 48 && K > 2048) return false;   // (in a chain of kernels the cut along k is ahead there: its ring is under way sooner)
+  // (In a chain of kernels the cut along k is ahead up to 32 tokens: its ring is under way sooner.  Eight 8B layers, 24 decode steps, ms, cut
+  // -> shares, at 33, 40 and 48 requests: 34.6 -> 33.7, 36.7 -> 35.8, 39.3 -> 38.3; at 56 and 64 without shares 42.1 and 45.6, with 40.4 and 43.7.)
+  if (T <= 32 && K > 2048) return false;
   return T <= 128 ? R >= 40 || (T > 64 && N >= 8 * pairs) : N > 256 * pairs;
 }
 cudaError_t gemm_rows_launch(const void* X, const void* W, void* Y, int ldy, int y_f32, int mode, int T, int N, int K, int num_sms,
