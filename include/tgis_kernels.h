@@ -275,6 +275,9 @@ int tgis_k_head_norm_gate(const float* o, int32_t ldo, int32_t heads, int32_t vd
                           int32_t act, float eps, void* out, int32_t out_dt, int32_t T);
 /* resid += rmsnorm((rmsnorm(y_main) * w_main + rmsnorm(y_pair) * w_pair) / 2) * w_post; out = rmsnorm(resid) * w_pre, or the
  * stream itself in the operand type (w_pre NULL, cast_out != 0) */
+int tgis_k_resid_tail_two(const float* y_main, const float* extra, const float* w_post, const float* w_pre, const float* w_pre2, const float* w_dot,
+                          float* resid, void* out, void* out2, int32_t out_dt, float* dot_out, float mult, float w_off, float eps, int32_t T,
+                          int32_t hidden);
 int tgis_k_resid_tail_pair(const float* y_main, const float* y_pair, const float* w_main, const float* w_pair,
                            const float* w_post, const float* w_pre, float* resid, void* out, int32_t out_dt, int32_t cast_out,
                            float eps, int32_t T, int32_t hidden);

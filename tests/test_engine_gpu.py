@@ -203,6 +203,48 @@ def test_prompt_logprobs_match_oracle(chunk):
     assert float(diffs.mean()) < 4e-3 and float(diffs.max()) < 3e-2, (float(diffs.mean()), float(diffs.max()))
 
 
+def test_a_step_that_admits_more_requests_than_one_launch_clears():
+    """96 requests with a repetition penalty in one step, then the same again in the same slots: what the first have seen is forgotten."""
+    from oracle.llama_oracle import CONFIGS, rope_table, synthetic_weights
+    from vllm_tgis_adapter_b200.engine.core import ModelConfig, NativeEngine, make_sampling_params
+
+    cfg = CONFIGS["tiny"]
+    mc = ModelConfig(n_layers=cfg.n_layers, hidden=cfg.hidden, n_q_heads=cfg.n_q_heads, n_kv_heads=cfg.n_kv_heads, ffn=cfg.ffn, vocab=cfg.vocab,
+                     rope_theta=cfg.rope_theta, rms_eps=cfg.rms_eps, max_model_len=cfg.max_model_len)
+    eng = NativeEngine(mc, max_num_seqs=96, max_batched_tokens=1024, kv_cache_bytes=32 << 20)
+    eng.load_weights(synthetic_weights(cfg, seed=1))
+    eng.load_weight("tgis.rope_cos_sin", rope_table(cfg))
+    rng = np.random.RandomState(3)
+    prompts = [rng.randint(3, 1024, size=rng.randint(3, 9)).tolist() for _ in range(96)]
+    sp = make_sampling_params(greedy=True, max_tokens=8, min_tokens=8, repetition_penalty=3.0)
+    runs = [[[r.new_token for r in recs if r.new_token is not None] for recs in eng.generate_sync(prompts, sp)] for _ in range(3)]
+    plain = [[r.new_token for r in recs if r.new_token is not None] for recs in eng.generate_sync(prompts, make_sampling_params(greedy=True, max_tokens=8, min_tokens=8))]
+    eng.close()
+    assert runs[0] == runs[1] == runs[2]
+    assert sum(a != b for a, b in zip(runs[0], plain)) > 48   # (the penalty counts: a slot that was not cleared would show)
+
+
+def test_replayed_logits_are_the_rounded_sums(monkeypatch):
+    """Rows wanted of a replay step come as bf16 from the device and are widened on the host: the rounding of the fp32 logits, row by row,
+    with more rows than one pass of the head takes."""
+    from oracle.llama_oracle import CONFIGS, rope_table, synthetic_weights
+    from vllm_tgis_adapter_b200.engine.core import ModelConfig, NativeEngine
+
+    cfg, res = CONFIGS["tiny"], []
+    mc = ModelConfig(n_layers=cfg.n_layers, hidden=cfg.hidden, n_q_heads=cfg.n_q_heads, n_kv_heads=cfg.n_kv_heads, ffn=cfg.ffn, vocab=cfg.vocab,
+                     rope_theta=cfg.rope_theta, rms_eps=cfg.rms_eps, max_model_len=cfg.max_model_len)
+    tokens = np.random.RandomState(5).randint(3, 1024, size=300).tolist()
+    for fp32 in ("0", "1"):
+        monkeypatch.setenv("TGIS_LOGITS_FP32", fp32)
+        eng = NativeEngine(mc, max_num_seqs=4, max_batched_tokens=512, kv_cache_bytes=32 << 20)
+        eng.load_weights(synthetic_weights(cfg, seed=1))
+        eng.load_weight("tgis.rope_cos_sin", rope_table(cfg))
+        res.append(torch.from_numpy(eng.trace_step([("a", tokens, list(range(0, 300, 2))), ("b", tokens[:7], [6, 0])], ["a", "b"])))
+        eng.close()
+    assert res[0].shape == (152, cfg.vocab) and torch.equal(res[0], res[1].bfloat16().float())
+    assert not torch.equal(res[0], res[1])
+
+
 @pytest.mark.parametrize("model", ["tiny", "small"])
 def test_fused_rope_epilogue_is_bit_identical(model, monkeypatch):
     """Decode-shaped steps apply RoPE and scatter K/V into the paged cache inside the qkv GEMM's cluster epilogue

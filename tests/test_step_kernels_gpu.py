@@ -116,6 +116,35 @@ def test_row_tail_with_and_without_experts(lib, hidden, top, side):
     assert ((out - rms(want) * (1 + wq.to(F64))).abs() <= 2e-5 * (1 + want.abs())).all()
 
 
+@pytest.mark.parametrize("hidden", [4, 1020, 1024, 1028, 2048])
+@pytest.mark.parametrize("out_dt", [0, 1])
+@pytest.mark.parametrize("form", ["pair", "pair, cast", "pair, no norm", "extra", "extra, no norm", "two norms and a gate", "mixture and a gate"])
+def test_row_tail_has_the_bits_of_the_general_kernel(lib, hidden, out_dt, form):
+    few, T, top, eps, gen = 5, 150, 3, C.c_float(1e-5), torch.Generator(device="cuda").manual_seed(hidden)   # more rows than SMs: the general one
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    y, z, resid, ws, rows = rnd(T, hidden), rnd(T, hidden), rnd(T, hidden), [rnd(hidden) for _ in range(5)], rnd(T * top, hidden)
+    inv, gate = torch.randperm(T * top, device="cuda", generator=gen).int(), rnd(T)
+    res = []
+    for n in (few, T):
+        r, dot = resid.clone(), torch.zeros(T, device="cuda")
+        o, o2 = (torch.zeros(T, hidden, device="cuda", dtype=torch.bfloat16 if out_dt else torch.float32) for _ in range(2))
+        post, pre = None if "no norm" in form else p(ws[0]), p(ws[1])
+        if form.startswith("pair"):
+            cast = form == "pair, cast"
+            rc = lib.tgis_k_resid_tail_pair(p(y), p(z), p(ws[2]), p(ws[3]), post, None if cast else pre, p(r), p(o), out_dt, int(cast), eps, n, hidden)
+        elif form == "mixture and a gate":
+            rc = lib.tgis_k_resid_tail_plain(None, p(rows), p(inv), C.c_float(0.3), top, p(z), p(gate), pre, p(r), p(o), out_dt, p(ws[4]), p(dot), eps, n, hidden)
+        else:
+            two = form.startswith("two")
+            rc = lib.tgis_k_resid_tail_two(p(y), p(z), post, pre, p(ws[2]) if two else None, p(ws[4]) if two else None, p(r), p(o), p(o2) if two else None,
+                                           out_dt, p(dot) if two else None, C.c_float(0.7), C.c_float(1.0), eps, n, hidden)
+        assert rc == 0
+        res.append([t[:few] for t in (r, o, o2, dot)])
+    assert all(torch.equal(a, b) for a, b in zip(*res))
+    assert not torch.equal(res[0][0], resid[:few]) and bool(res[0][1].any())
+    assert bool(res[0][2].any()) == form.startswith("two") and bool(res[0][3].any()) == ("gate" in form)
+
+
 @pytest.mark.parametrize("T", [1, 8, 9, 32])
 @pytest.mark.parametrize("heads,N,K,scaled,y_dt", [(16, 512, 128, False, 0), (16, 128, 512, True, 1), (3, 40, 64, False, 1), (5, 24, 320, True, 0)])
 def test_products_per_head(lib, T, heads, N, K, scaled, y_dt):

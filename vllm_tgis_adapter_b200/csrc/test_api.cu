@@ -1007,6 +1007,17 @@ int tgis_k_head_norm_gate(const float* o, int32_t ldo, int32_t heads, int32_t vd
   return 0;
 }
 
+// ... with a further term of the stream, a second pre-norm and a gate computed from the normed row (each may be null)
+int tgis_k_resid_tail_two(const float* y_main, const float* extra, const float* w_post, const float* w_pre, const float* w_pre2, const float* w_dot,
+                          float* resid, void* out, void* out2, int32_t out_dt, float* dot_out, float mult, float w_off, float eps, int32_t T,
+                          int32_t hidden) {
+  ResidTail a{};
+  a.y_main = y_main; a.extra = extra; a.w_post = w_post; a.w_pre = w_pre; a.w_pre2 = w_pre2; a.w_dot = w_dot;
+  a.resid = resid; a.out = out; a.out2 = out2; a.out_dtype = out_dt; a.dot_out = dot_out; a.mult = mult; a.w_off = w_off; a.eps = eps;
+  KCK(resid_tail_launch(a, T, hidden, 0));
+  KCK(cudaDeviceSynchronize());
+  return 0;
+}
 int tgis_k_resid_tail_pair(const float* y_main, const float* y_pair, const float* w_main, const float* w_pair,
                            const float* w_post, const float* w_pre, float* resid, void* out, int32_t out_dt, int32_t cast_out,
                            float eps, int32_t T, int32_t hidden) {
