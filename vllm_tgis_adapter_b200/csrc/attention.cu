@@ -35,12 +35,6 @@ __device__ __forceinline__ float warp_add(float v) {
   return v;
 }
 
-__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
@@ -242,7 +236,7 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ qkv, int qkv_ld, const __nv
         for (int mt = 0; mt < 2; ++mt) {
           uint32_t ka[4];
           ldmatrix_x4(ka, k_base + ((2 * ks + (mi >> 1)) * KV_BLOCK + mt * 16 + (mi & 1) * 8 + ri) * 16);
-          mma_bf16_16816(st[mt], ka, qb[ks][0], qb[ks][1]);
+          mma_16816(st[mt], ka, qb[ks][0], qb[ks][1]);
         }
       }
       __syncwarp();
@@ -310,10 +304,10 @@ attn_decode_kernel(const __nv_bfloat16* __restrict__ qkv, int qkv_ld, const __nv
 #pragma unroll
           for (int u = 0; u < 2; ++u)
             ldmatrix_x4_trans(va[u], v_base + tok * (HEAD_DIM * 2) + (((2 * (md + u) + (mi & 1)) ^ (tok & 7)) * 16));
-          mma_bf16_16816(ot[md], va[0], bh[kk][0], bh[kk][1]);
-          mma_bf16_16816(ot[md + 1], va[1], bh[kk][0], bh[kk][1]);
-          mma_bf16_16816(ot[md], va[0], bl[kk][0], bl[kk][1]);
-          mma_bf16_16816(ot[md + 1], va[1], bl[kk][0], bl[kk][1]);
+          mma_16816(ot[md], va[0], bh[kk][0], bh[kk][1]);
+          mma_16816(ot[md + 1], va[1], bh[kk][0], bh[kk][1]);
+          mma_16816(ot[md], va[0], bl[kk][0], bl[kk][1]);
+          mma_16816(ot[md + 1], va[1], bl[kk][0], bl[kk][1]);
         }
       }
       __syncwarp();

@@ -223,11 +223,6 @@ __device__ __forceinline__ void ca_cp_async16(void* smem, const void* gmem) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void ca_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 
 __global__ void __launch_bounds__(CA_THREADS)
 capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
@@ -303,7 +298,7 @@ capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
       if (ks < nks) {
         uint32_t kb[2];
         ca_ldsm_x2(kb, Ks + (size_t)(warp * 8 + (lane & 7)) * LDK + ks * 16 + ((lane >> 3) & 1) * 8);
-        ca_mma(c, qa[ks], kb[0], kb[1]);
+        mma_16816(c, qa[ks], kb[0], kb[1]);
       }
     bool ok[4];
 #pragma unroll
@@ -352,8 +347,8 @@ capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
         acc[j][0] *= al[0]; acc[j][1] *= al[0]; acc[j][2] *= al[1]; acc[j][3] *= al[1];
         uint32_t vb[4];
         ca_ldsm_x4_trans(vb, Vs + (size_t)lane * LDV + n0);
-        ca_mma(acc[j], a0, vb[0], vb[1]);
-        ca_mma(acc[j], a1, vb[2], vb[3]);
+        mma_16816(acc[j], a0, vb[0], vb[1]);
+        mma_16816(acc[j], a1, vb[2], vb[3]);
       }
     }
     __syncthreads();   // this pass's buffers, maxima and weights are consumed
@@ -469,7 +464,7 @@ capattn_mma_group_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat1
         if (ks < nks) {
           uint32_t kb[2];
           ca_ldsm_x2(kb, Ks + (size_t)(nt * 8 + (lane & 7)) * LDK + ks * 16 + ((lane >> 3) & 1) * 8);
-          ca_mma(sc[nt], qa[ks], kb[0], kb[1]);
+          mma_16816(sc[nt], qa[ks], kb[0], kb[1]);
         }
     }
     float mx[2] = {-INFINITY, -INFINITY};
@@ -512,8 +507,8 @@ capattn_mma_group_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat1
         acc[j][0] *= al[0]; acc[j][1] *= al[0]; acc[j][2] *= al[1]; acc[j][3] *= al[1];
         uint32_t vb[4];
         ca_ldsm_x4_trans(vb, Vs + (size_t)lane * LDV + j * 8);
-        ca_mma(acc[j], pa[0], vb[0], vb[1]);
-        ca_mma(acc[j], pa[1], vb[2], vb[3]);
+        mma_16816(acc[j], pa[0], vb[0], vb[1]);
+        mma_16816(acc[j], pa[1], vb[2], vb[3]);
       }
     __syncthreads();   // this pass's buffer is consumed
   }

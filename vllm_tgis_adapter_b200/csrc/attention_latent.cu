@@ -258,11 +258,6 @@ __device__ __forceinline__ void lat_ldsm_x4_trans(uint32_t (&r)[4], const void* 
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s));
 }
-__device__ __forceinline__ void lat_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 inline __host__ __device__ int lat_ldq(int D) { return (D + 15) / 16 * 16 + 8; }  // padded row length (bf16 elements)
 inline size_t lat_mma_smem(int D) {
   return (size_t)(LATENT_PAIRS + 2 * KV_BLOCK) * lat_ldq(D) * 2 + (size_t)2 * LATENT_PAIRS * 33 * 4 + LATENT_PAIRS * 40 * 2 +
@@ -370,7 +365,7 @@ latent_attn_mma_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __r
         uint32_t a[4], b[2];
         lat_ldsm_x4(a, Qs + (size_t)(lane & 15) * LDQ + ks * 16 + (lane >> 4) * 8);
         lat_ldsm_x2(b, Kb + (size_t)(ntk * 8 + (lane & 7)) * LDQ + ks * 16 + ((lane >> 3) & 1) * 8);
-        lat_mma(c, a, b[0], b[1]);
+        mma_16816(c, a, b[0], b[1]);
       }
       float* sp = Sp + (size_t)half * LATENT_PAIRS * 33;
       sp[gq * 33 + ntk * 8 + t2] = c[0];
@@ -408,8 +403,8 @@ latent_attn_mma_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __r
           acc[j][0] *= c_lo; acc[j][1] *= c_lo; acc[j][2] *= c_hi; acc[j][3] *= c_hi;
           uint32_t b[4];
           lat_ldsm_x4_trans(b, Kb + (size_t)lane * LDQ + n0);
-          lat_mma(acc[j], a0, b[0], b[1]);
-          lat_mma(acc[j], a1, b[2], b[3]);
+          mma_16816(acc[j], a0, b[0], b[1]);
+          mma_16816(acc[j], a1, b[2], b[3]);
         }
       }
     }
@@ -568,8 +563,8 @@ latent_attn_wide_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __
         uint32_t a[4], b[4];
         lat_ldsm_x4(a, q_frag + ks * 16);
         lat_ldsm_x4(b, kf + ks * 16);
-        lat_mma(c[i][0], a, b[0], b[1]);
-        lat_mma(c[i][1], a, b[2], b[3]);
+        mma_16816(c[i][0], a, b[0], b[1]);
+        mma_16816(c[i][1], a, b[2], b[3]);
       };
 #pragma unroll 3
       for (int ks = 0; ks < KS / 2; ++ks) {
@@ -642,8 +637,8 @@ latent_attn_wide_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __
 #pragma unroll
           for (int i = 0; i < 4; ++i)
             if (i < n_mt) {
-              lat_mma(acc[i][j], a[i][0], b[0], b[1]);
-              lat_mma(acc[i][j], a[i][1], b[2], b[3]);
+              mma_16816(acc[i][j], a[i][0], b[0], b[1]);
+              mma_16816(acc[i][j], a[i][1], b[2], b[3]);
             }
         }
       }

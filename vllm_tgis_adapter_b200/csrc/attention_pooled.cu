@@ -514,11 +514,6 @@ __device__ __forceinline__ void pa_cp_async16(void* smem, const void* gmem) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void pa_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 
 // 2^x of the special function unit (relative error of a few 2^-23; results below 2^-126 become zero)
 __device__ __forceinline__ float pa_exp2(float x) {
@@ -667,8 +662,8 @@ poolattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
           for (int jj = 0; jj < 2; ++jj) {
             uint32_t kb[4];
             pa_ldsm_x4(kb, Ks + (size_t)(jj * 16 + (lane >> 4) * 8 + (lane & 7)) * LDK + ks * 16 + ((lane >> 3) & 1) * 8);
-            pa_mma(sc[2 * jj], qa[ks], kb[0], kb[1]);
-            pa_mma(sc[2 * jj + 1], qa[ks], kb[2], kb[3]);
+            mma_16816(sc[2 * jj], qa[ks], kb[0], kb[1]);
+            mma_16816(sc[2 * jj + 1], qa[ks], kb[2], kb[3]);
           }
         }
 #pragma unroll
@@ -722,8 +717,8 @@ poolattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __
         if (EXACT || j * 8 < dv) {
           uint32_t vb[4];
           pa_ldsm_x4_trans(vb, Vs + (size_t)lane * LDV + j * 8);
-          pa_mma(acc[j], pa[0], vb[0], vb[1]);
-          pa_mma(acc[j], pa[1], vb[2], vb[3]);
+          mma_16816(acc[j], pa[0], vb[0], vb[1]);
+          mma_16816(acc[j], pa[1], vb[2], vb[3]);
         }
     }
   }

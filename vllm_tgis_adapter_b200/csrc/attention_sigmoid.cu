@@ -190,11 +190,6 @@ __device__ __forceinline__ void sa_cp_async16(void* smem, const void* gmem) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void sa_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 
 __global__ void __launch_bounds__(SA_THREADS)
 sigattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
@@ -268,7 +263,7 @@ sigattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
       if (ks < nks) {
         uint32_t kb[2];
         sa_ldsm_x2(kb, Ks + (size_t)(warp * 8 + (lane & 7)) * LDK + ks * 16 + ((lane >> 3) & 1) * 8);
-        sa_mma(c, qa[ks], kb[0], kb[1]);
+        mma_16816(c, qa[ks], kb[0], kb[1]);
       }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
@@ -293,8 +288,8 @@ sigattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
       if (n0 < dv) {
         uint32_t vb[4];
         sa_ldsm_x4_trans(vb, Vs + (size_t)lane * LDV + n0);
-        sa_mma(acc[j], a0, vb[0], vb[1]);
-        sa_mma(acc[j], a1, vb[2], vb[3]);
+        mma_16816(acc[j], a0, vb[0], vb[1]);
+        mma_16816(acc[j], a1, vb[2], vb[3]);
       }
     }
     __syncthreads();   // this pass's buffers and weights are consumed

@@ -1,7 +1,7 @@
 // libtgis_engine.so — continuous-batching engine + C ABI (include/tgis_engine.h).
 //
 // This is the B200-native replacement for what sits behind `self.engine.generate(...)`
-// (/root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py:222): vLLM's EngineCore busy loop, scheduler,
+// (src/vllm_tgis_adapter/grpc/grpc_server.py:222): vLLM's EngineCore busy loop, scheduler,
 // KV block manager, GPUModelRunner and Sampler.
 //
 //   host side (this file, C++): request queues, paged-KV block allocator, continuous-batching scheduler with chunked
@@ -2934,7 +2934,7 @@ struct tgis_engine {
                       l.cos_sin2, d_pos, chunked ? flx_mix : nullptr, qkv, lead};
         CK(rotary_rows_launch(rr, T, st));
         OuterScan os{};
-      os.single = T == S;
+        os.single = T == S;
         os.mode = OUTER_SCAN_RETENTION;
         os.q = pnx_y1 + l.c_mq; os.k = pnx_y1 + l.c_mk; os.v = pnx_y1 + l.c_mv; os.ldq = os.ldk = os.ldv = ld;
         os.q_scale = 1.f;

@@ -46,11 +46,6 @@ __device__ __forceinline__ void l_ldsm_x4_trans(uint32_t (&r)[4], const void* sm
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
-__device__ __forceinline__ void l_mma(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ void l_cp_async16(void* smem, const void* gmem) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(gmem) : "memory");
@@ -252,8 +247,8 @@ lightning_chunk_kernel(LightningChunk a, const AttnSeq* __restrict__ seqs, const
             if (jj <= warp) {
               uint32_t kf[4];
               l_ldsm_x4(kf, Ks + (size_t)(jj * 16 + (lane >> 4) * 8 + (lane & 7)) * LDQ + ks * 16 + ((lane >> 3) & 1) * 8);
-              l_mma(sc[2 * jj], qf, kf[0], kf[1]);
-              l_mma(sc[2 * jj + 1], qf, kf[2], kf[3]);
+              mma_16816(sc[2 * jj], qf, kf[0], kf[1]);
+              mma_16816(sc[2 * jj + 1], qf, kf[2], kf[3]);
             }
         }
 #pragma unroll
@@ -293,8 +288,8 @@ lightning_chunk_kernel(LightningChunk a, const AttnSeq* __restrict__ seqs, const
               l_ldsm_x4(qf, Qs + (size_t)(mt * 16 + (lane & 15)) * LDQ + ks * 16 + (lane >> 4) * 8);
 #pragma unroll
               for (int n = 0; n < 2; ++n) {
-                l_mma(o[mt][n], qf, bh[n][0], bh[n][1]);
-                l_mma(o[mt][n], qf, bl[n][0], bl[n][1]);
+                mma_16816(o[mt][n], qf, bh[n][0], bh[n][1]);
+                mma_16816(o[mt][n], qf, bl[n][0], bl[n][1]);
               }
             }
         }
@@ -319,8 +314,8 @@ lightning_chunk_kernel(LightningChunk a, const AttnSeq* __restrict__ seqs, const
             l_ldsm_x4(al, Al + (size_t)(mt * 16 + (lane & 15)) * LDA_ + kk * 16 + (lane >> 4) * 8);
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
-              l_mma(o[mt][n], ah, vf[2 * n], vf[2 * n + 1]);
-              l_mma(o[mt][n], al, vf[2 * n], vf[2 * n + 1]);
+              mma_16816(o[mt][n], ah, vf[2 * n], vf[2 * n + 1]);
+              mma_16816(o[mt][n], al, vf[2 * n], vf[2 * n + 1]);
             }
           }
       }
@@ -351,10 +346,10 @@ lightning_chunk_kernel(LightningChunk a, const AttnSeq* __restrict__ seqs, const
           if (ks < nks) {
             uint32_t kf[4];
             l_ldsm_x4_trans(kf, Ks + (size_t)(kk * 16 + (lane & 15)) * LDQ + ks * 16 + (lane >> 4) * 8);
-            l_mma(S[2 * ks], vh, kf[0], kf[1]);
-            l_mma(S[2 * ks + 1], vh, kf[2], kf[3]);
-            l_mma(S[2 * ks], vl, kf[0], kf[1]);
-            l_mma(S[2 * ks + 1], vl, kf[2], kf[3]);
+            mma_16816(S[2 * ks], vh, kf[0], kf[1]);
+            mma_16816(S[2 * ks + 1], vh, kf[2], kf[3]);
+            mma_16816(S[2 * ks], vl, kf[0], kf[1]);
+            mma_16816(S[2 * ks + 1], vl, kf[2], kf[3]);
           }
       }
   }
@@ -612,9 +607,9 @@ gla_prep_kernel(GlaChunk a, const AttnSeq* __restrict__ seqs, const LatentTile* 
       l_ldsm_x4(ql, qll + qa);
       l_ldsm_x4(kh, klh + ka);
       l_ldsm_x4(kl, kll + ka);
-      l_mma(s, qh, kh[2 * warp], kh[2 * warp + 1]);
-      l_mma(s, qh, kl[2 * warp], kl[2 * warp + 1]);
-      l_mma(s, ql, kh[2 * warp], kh[2 * warp + 1]);
+      mma_16816(s, qh, kh[2 * warp], kh[2 * warp + 1]);
+      mma_16816(s, qh, kl[2 * warp], kl[2 * warp + 1]);
+      mma_16816(s, ql, kh[2 * warp], kh[2 * warp + 1]);
     }
     const int g = lane >> 2, t2 = (lane & 3) * 2 + 8 * warp;
     As[(GB + g) * (GC + 1) + t2] = s[0];
@@ -729,9 +724,9 @@ gla_chunk_kernel(GlaChunk a, const AttnSeq* __restrict__ seqs, const int32_t* __
               l_ldsm_x4(ql, Ql + at);
 #pragma unroll
               for (int n = 0; n < 2; ++n) {
-                l_mma(o[mt][n], qh, bh[n][0], bh[n][1]);
-                l_mma(o[mt][n], qh, bl[n][0], bl[n][1]);
-                l_mma(o[mt][n], ql, bh[n][0], bh[n][1]);
+                mma_16816(o[mt][n], qh, bh[n][0], bh[n][1]);
+                mma_16816(o[mt][n], qh, bl[n][0], bl[n][1]);
+                mma_16816(o[mt][n], ql, bh[n][0], bh[n][1]);
               }
             }
         }
@@ -750,8 +745,8 @@ gla_chunk_kernel(GlaChunk a, const AttnSeq* __restrict__ seqs, const int32_t* __
             l_ldsm_x4(al, Al + at);
 #pragma unroll
             for (int n = 0; n < 2; ++n) {
-              l_mma(o[mt][n], ah, vf[2 * n], vf[2 * n + 1]);
-              l_mma(o[mt][n], al, vf[2 * n], vf[2 * n + 1]);
+              mma_16816(o[mt][n], ah, vf[2 * n], vf[2 * n + 1]);
+              mma_16816(o[mt][n], al, vf[2 * n], vf[2 * n + 1]);
             }
           }
       }
@@ -785,10 +780,10 @@ gla_chunk_kernel(GlaChunk a, const AttnSeq* __restrict__ seqs, const int32_t* __
             const size_t at = (size_t)(kk * 16 + (lane & 15)) * LDQ + ks * 16 + (lane >> 4) * 8;
             l_ldsm_x4_trans(kh, Kh + at);
             l_ldsm_x4_trans(kl, Kl + at);
-            l_mma(S[2 * ks], va, kh[0], kh[1]);
-            l_mma(S[2 * ks + 1], va, kh[2], kh[3]);
-            l_mma(S[2 * ks], va, kl[0], kl[1]);
-            l_mma(S[2 * ks + 1], va, kl[2], kl[3]);
+            mma_16816(S[2 * ks], va, kh[0], kh[1]);
+            mma_16816(S[2 * ks + 1], va, kh[2], kh[3]);
+            mma_16816(S[2 * ks], va, kl[0], kl[1]);
+            mma_16816(S[2 * ks + 1], va, kl[2], kl[3]);
           }
       }
   }

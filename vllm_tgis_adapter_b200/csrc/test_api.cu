@@ -957,7 +957,7 @@ int tgis_k_retention_scan(float* x, int32_t ld, int32_t q_off, int32_t k_off, in
     a.q = x + q_off; a.k = x + k_off; a.v = x + v_off; a.ldq = a.ldk = a.ldv = ld; a.q_scale = 1.f;
     a.decay = decay; a.S = S; a.out = out; a.ldo = ldo; a.heads = heads; a.dim = dim; a.vdim = vdim;
     a.single = all_single(seqs);
-  KCK(outer_scan_launch(a, d_seqs.p, n_seqs, tok_slot, 0));
+    KCK(outer_scan_launch(a, d_seqs.p, n_seqs, tok_slot, 0));
   }
   KCK(cudaDeviceSynchronize());
   return 0;
