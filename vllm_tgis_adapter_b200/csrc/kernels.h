@@ -32,6 +32,17 @@ constexpr int GEMM_X_BOX_MANY = 32;
 //   4096 x 14336   26.1 27.9 29.7 31.1 37.6 40.4   49.9 51.0 50.3 51.1 51.4 51.8   37.7 39.8 41.6 45.6 65.2 84.7
 //   2048 x 11264   16.8 18.6 20.5 22.4 26.0 28.4   38.4 39.1 38.3 38.7 38.7 38.6   30.1 31.7 32.8 36.7 51.9 67.1
 // (a k-block takes the tensor cores some 0.16 us however few rows and tokens it has, so long k is for the kernel that cuts it).
+// The same at 65, 96, 128, 129, 192 and 256 tokens for fewer rows (equal shares below 592 rows are not taken; where they are, they are
+// behind the cut by at most 1.2 us, at k = 4096, and ahead by up to 5.3; pairs are behind it by 0.1 us in one case and ahead by up to 15):
+//   2048 x 512    13.8 14.9 17.9 16.9 18.8 21.5  11.5 12.3 11.8 11.6 11.9 11.5  11.3 10.6 13.0 11.9 12.7 13.9
+//   1536 x 4096   18.6 19.3 21.1 21.5 24.1 26.8  22.0 21.5 22.0 21.5 22.0 20.8  18.9 19.3 21.3 23.7 26.9 33.0
+//   1024 x 2048   18.3 19.8 21.1 21.8 25.2 27.8  15.8 16.2 17.3 15.3 15.7 15.5  15.0 17.2 19.5 17.5 19.1 22.0
+//   1024 x 4096   18.2 19.0 21.1 21.8 24.0 26.6  21.6 21.8 22.0 20.9 20.7 20.8  18.9 19.7 21.7 23.9 27.0 33.1
+//   768 x 768     17.0 15.8 17.0 18.2 20.3 23.0  11.7 12.0 11.9 11.8 11.7 12.6  11.7 11.6 12.5 12.7 13.7 14.8
+//   768 x 3072    19.6 19.0 22.0 21.5 23.8 27.1  19.0 20.2 19.0 18.8 18.6 18.0  19.0 18.3 21.2 20.9 22.9 26.9
+//   640 x 4096    17.7 19.2 20.1 21.2 23.8 26.2  21.6 21.9 21.7 21.3 21.7 22.7  18.9 18.9 21.0 23.7 27.1 32.9
+//   384 x 4096    17.6 19.4 19.8 21.2 23.3 25.8  20.9 20.8 21.0 20.7 20.8 20.8  18.9 18.8 20.9 23.1 26.5 32.0
+//   64 x 2048     19.5 19.7 21.7 23.0 25.9 29.8  15.0 15.0 14.7 14.7 14.8 14.8  15.1 14.6 14.8 16.3 17.7 20.0
 inline bool gemm_takes_pairs(int T, int N, int num_sms) { return T > 256 || (T > 64 && (N + 127) / 128 > num_sms / 2); }
 // rows of one box of the activation map: the token tile, or (pairs) small boxes, of which a tile takes as many as it has rows
 inline int gemm_x_box(int T, int N, int num_sms) { return gemm_takes_pairs(T, N, num_sms) ? GEMM_X_BOX_MANY : gemm_pick_bt(T); }
