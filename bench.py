@@ -291,7 +291,7 @@ def cpu_reference_opt(args, steps: int, warmup: int, budget_s: float | None = No
 
 def ncu_traffic_per_launch(n_layers: int):
     """DRAM bytes (read + write) per launch of the dominant kernel from the committed `ncu --set full` capture
-    (profiles/, produced by scripts/gpu_check.sh prof_gemm: the qkv, o, gate_up, down and lm_head launches of one decode
+    (profiles/, the qkv, o, gate_up, down and lm_head launches of one decode
     step at batch 32), weighted like the timed mix: n_layers x the four layer GEMMs + one lm_head."""
     import csv
     import glob
@@ -319,7 +319,7 @@ def ncu_traffic_per_launch(n_layers: int):
 
 def reduce_over_ranks(max_vals: list[float], sum_vals: list[float], device: str) -> tuple[list[float], list[float]]:
     """Whole-job aggregation for the N>1 (data-parallel replicas) path: times -> MAX over ranks, counts -> SUM.
-    Works on any initialised torch.distributed backend (NCCL on the GPU box, gloo in tests/test_multirank_cpu.py)."""
+    Works on any initialised torch.distributed backend (NCCL on GPUs, gloo in tests/test_multirank_cpu.py)."""
     import torch
     import torch.distributed as dist
 
@@ -549,7 +549,7 @@ def _vllm_baseline(model: str, batch: int):
                 return {"decode_tokens_per_s": r["decode_tokens_per_s"], "decode_ms_per_step": r["decode_ms_per_step"],
                         "job_output_tokens_per_s": r["job_output_tokens_per_s"],
                         "prefill_burst_s": r["t_prefill_burst_s"], "vllm": d["meta"]["vllm"], "gpu": d["meta"]["gpu"],
-                        "source": f"profiles/{Path(files[-1]).name} (builder-run on this pool; not timed in this run)"}
+                        "source": f"profiles/{Path(files[-1]).name} (an earlier run; not timed in this run)"}
     except Exception:  # noqa: BLE001
         return None
     return None
@@ -635,7 +635,7 @@ def run_ours(args) -> dict | None:
     # ============================================================ N > 1: secondary legs
     dp_leg = parity = named70 = None
     if tp > 1:
-        # (a) data-parallel replicas of the same workload (weak scaling; what round 1 reported) + the N=1 tokens for the
+        # (a) data-parallel replicas of the same workload (weak scaling) + the N=1 tokens for the
         #     in-run parity check of the tensor-parallel engine
         e1, c1 = _build_engine(args.model, max_seqs=B, max_len=max_len, kv_tokens=B * (P + G + 32),
                                max_batched=args.max_batched_tokens, tp=1, rank=rank, local=local, weight_seed=1234,
@@ -1021,11 +1021,13 @@ def main():
     out = run_ours(args)
     if out is None:
         return
-    try:  # keep the GPU numbers even if the CPU baseline leg is cut short by a timeout
-        (ROOT / "gpurun_out").mkdir(exist_ok=True)
-        (ROOT / "gpurun_out" / "bench_ours_partial.json").write_text(json.dumps(out))
-    except OSError:
-        pass
+    if os.environ.get("TGIS_OUT_DIR"):  # keep the GPU numbers even if the CPU baseline leg is cut short by a timeout
+        try:
+            partial = Path(os.environ["TGIS_OUT_DIR"])
+            partial.mkdir(parents=True, exist_ok=True)
+            (partial / "bench_ours_partial.json").write_text(json.dumps(out))
+        except OSError:
+            pass
     if not args.no_cpu_baseline:   # rank 0, every N
         ref = cpu_reference(args, steps=args.cpu_steps, warmup=3, budget_s=args.cpu_budget_s)
         out["cpu_baseline"] = {k: ref[k] for k in ("value", "unit", "cores", "kind", "sample", "ttft_p50_est_ms")}

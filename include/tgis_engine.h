@@ -4,7 +4,7 @@
  *
  * Drop-in boundary.  The reference has no FFI; its seam is the `EngineClient` object that
  * `TextGenerationService` holds.  Each entry point below cites the reference call site it serves
- * (paths relative to /root/reference/src/vllm_tgis_adapter):
+ * (paths relative to src/vllm_tgis_adapter):
  *
  *   tgis_engine_create / _load_weight / _start   <- __main__.py:48   `build_async_engine_client(args)`
  *   tgis_engine_add_request                      <- grpc/grpc_server.py:205-225 `_make_generator` -> engine.generate(

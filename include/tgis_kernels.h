@@ -5,7 +5,7 @@
  * staged internally.  Every call synchronises before returning; 0 = ok, <0 = error (tgis_last_error()).
  *
  * Reference semantics restated by these kernels (vLLM 0.22 = the arithmetic behind
- * /root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py:222):
+ * src/vllm_tgis_adapter/grpc/grpc_server.py:222):
  *   tgis_k_gemm        vllm model_executor/layers/linear.py (F.linear, bf16 in, fp32 accumulate, bf16 out)
  *   tgis_k_rmsnorm     vllm model_executor/layers/layernorm.py:104,173 (rms_norm / fused_add_rms_norm)
  *   tgis_k_silu_mul    vllm model_executor/layers/activation.py:117-143

@@ -4,7 +4,7 @@ Only tests/, __graft_entry__.smoke() and bench.py's cpu_baseline / --impl refere
 product path (vllm_tgis_adapter_b200) never does and fails loudly without its CUDA library.
 
 It restates, in plain torch CPU ops, the arithmetic that sits behind the reference's single engine call
-`self.engine.generate(...)` (/root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py:222).  That arithmetic is not in
+`self.engine.generate(...)` (src/vllm_tgis_adapter/grpc/grpc_server.py:222).  That arithmetic is not in
 the reference tree: it is the un-vendored dependency vLLM (pyproject.toml:30 `vllm>=0.10.0`; installed 0.22.0) running a
 HF-format Llama checkpoint.  Restated here, with the file:line each step follows:
 

@@ -3,7 +3,7 @@
 Only tests/, __graft_entry__.smoke() and bench.py's CPU legs may import this module; the product path never does.
 
 The reference's own OPT fixture is `facebook/opt-125m` served through `self.engine.generate(...)`
-(/root/reference/tests/conftest.py:79-91 (no --model: vLLM's default, facebook/opt-125m) and tests/test_hub.py:17, tests/test_grpc_server.py:42-49, grpc/grpc_server.py:222); the arithmetic is
+(tests/conftest.py:79-91 (no --model: vLLM's default, facebook/opt-125m) and tests/test_hub.py:17, tests/test_grpc_server.py:42-49, grpc/grpc_server.py:222); the arithmetic is
 the un-vendored dependency vLLM (installed 0.22.0).  Restated here in plain torch ops with the model-dtype rounding
 points of that path, each step citing the file:line it follows:
 

@@ -3,8 +3,8 @@
 Restates, per request row and in fp32, what the reference stack does between the lm_head logits and the
 (token, logprob, rank, top-n) record.  Each function cites what it follows:
 
-  exp_decay_length_penalty  /root/reference/src/vllm_tgis_adapter/tgis_utils/logits_processors.py:33-47   (R7)
-  typical_mask              /root/reference/src/vllm_tgis_adapter/tgis_utils/logits_processors.py:11-21   (R8)
+  exp_decay_length_penalty  src/vllm_tgis_adapter/tgis_utils/logits_processors.py:33-47   (R7)
+  typical_mask              src/vllm_tgis_adapter/tgis_utils/logits_processors.py:11-21   (R8)
                             -> transformers generation/logits_process.py:836-856 (TypicalLogitsWarper.__call__)
   min_tokens                vllm v1/sample/logits_processor/builtin.py:168-240                            (S2)
   repetition_penalty        vllm model_executor/layers/utils.py:51-89, _custom_ops.py:360-408             (S3)
@@ -19,7 +19,7 @@ greedy argmax | temperature -> top-k -> top-p -> sample.
 
 PARITY PINNING: the reference's tests never exercise these processors.  tests/golden/sampler_*.json
 are generated by oracle/gen_golden.py by running the reference's OWN logits_processors.py (imported from
-/root/reference in the build container), transformers' TypicalLogitsWarper and vLLM 0.22's CPU sampler ops on seeded
+its source tree), transformers' TypicalLogitsWarper and vLLM 0.22's CPU sampler ops on seeded
 logits; tests/test_oracle_cpu.py checks this file against them.
 
 The random draw: torch's Philox stream cannot be reproduced by a custom kernel, so the engine defines

@@ -2,6 +2,7 @@
 heads of 128).  The cache is replicated over enough "layers" that every launch streams its KV from HBM, not L2."""
 import ctypes as C
 import json
+import os
 import sys
 from pathlib import Path
 
@@ -41,5 +42,6 @@ for B, kv in cases:
     res.append(r)
     print(json.dumps(r), flush=True)
     del kc, vc
-Path("gpurun_out").mkdir(exist_ok=True)
-Path("gpurun_out/attn_bench.json").write_text(json.dumps(res, indent=1))
+OUT = Path(os.environ.get("TGIS_OUT_DIR", "out"))
+OUT.mkdir(parents=True, exist_ok=True)
+(OUT / "attn_bench.json").write_text(json.dumps(res, indent=1))

@@ -5,7 +5,7 @@
   lora4   : the requests spread over FOUR adapters (mixed-adapter token tiles)
   guided  : every request under a token bitmask (a provider that allows every token: the cost measured is the per-step
             host callback x 32, the 16 KB H2D per row and the masked sampler instantiation -- not a grammar's own cost)
-Writes gpurun_out/feature_decode_bench.json."""
+Writes feature_decode_bench.json under TGIS_OUT_DIR (default: out)."""
 import ctypes as C
 import json
 import os
@@ -82,6 +82,7 @@ def run(tag, slots, guided):
 
 out = [run("base", [0] * B, False), run("lora (1 adapter, rank 16, 7 modules)", [1] * B, False),
        run("lora4 (4 adapters mixed)", [1 + i % 4 for i in range(B)], False), run("guided (allow-all mask)", [0] * B, True)]
-os.makedirs("gpurun_out", exist_ok=True)
-Path("gpurun_out/feature_decode_bench.json").write_text(json.dumps(out, indent=1))
+OUT = Path(os.environ.get("TGIS_OUT_DIR", "out"))
+OUT.mkdir(parents=True, exist_ok=True)
+(OUT / "feature_decode_bench.json").write_text(json.dumps(out, indent=1))
 eng.close()

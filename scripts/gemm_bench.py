@@ -2,6 +2,7 @@
 Weights are rotated over several distinct buffers so every launch streams from HBM, not L2."""
 import ctypes as C
 import json
+import os
 import sys
 from pathlib import Path
 
@@ -51,5 +52,6 @@ for name, N, K in SHAPES:
         print(json.dumps(r), flush=True)
         del ws, x, y
         torch.cuda.empty_cache()
-Path("gpurun_out").mkdir(exist_ok=True)
-Path(f"gpurun_out/gemm_bench_{sys.argv[1]}.json" if len(sys.argv) > 1 else "gpurun_out/gemm_bench.json").write_text(json.dumps(res, indent=1))
+OUT = Path(os.environ.get("TGIS_OUT_DIR", "out"))
+OUT.mkdir(parents=True, exist_ok=True)
+(OUT / (f"gemm_bench_{sys.argv[1]}.json" if len(sys.argv) > 1 else "gemm_bench.json")).write_text(json.dumps(res, indent=1))

@@ -6,6 +6,7 @@ import argparse
 import asyncio
 import dataclasses
 import json
+import os
 import statistics
 import sys
 import threading
@@ -105,7 +106,8 @@ out = {"surface": "fmaas.GenerationService/GenerateStream over grpc.aio (in-proc
        "decode_tokens_per_s_median": statistics.median(r["decode_tokens_per_s"] for r in rounds),
        "ttft_p50_ms_median": statistics.median(r["ttft_p50_ms"] for r in rounds), "best": best}
 print(json.dumps(out), flush=True)
-Path("gpurun_out").mkdir(exist_ok=True)
-Path("gpurun_out/grpc_bench.json").write_text(json.dumps(out, indent=1))
+OUT = Path(os.environ.get("TGIS_OUT_DIR", "out"))
+OUT.mkdir(parents=True, exist_ok=True)
+(OUT / "grpc_bench.json").write_text(json.dumps(out, indent=1))
 srv_loop.call_soon_threadsafe(state["stop"].set)
 time.sleep(1.0)

@@ -4,7 +4,7 @@ launches through the C-ABI test hooks):
     decode-shaped step (T = 32, four adapters mixed) and a prefill chunk (T = 2048, one adapter), against the bytes the
     kernels must move (A and B of the adapters present once, x and y once);
   * the fused sampling kernel with and without a guided-decoding bitmask (V = 128256, bf16 logits, greedy rows).
-Writes gpurun_out/lora_guided_bench.json.  LORA_BENCH_ONLY=1: two launches per case (ncu captures)."""
+Writes lora_guided_bench.json under TGIS_OUT_DIR (default: out).  LORA_BENCH_ONLY=1: two launches per case (ncu captures)."""
 import ctypes as C
 import json
 import os
@@ -74,5 +74,6 @@ for n in ((32,) if os.environ.get("LORA_BENCH_ONLY") else (32, 64, 256)):
                            "hbm_floor_us_one_read_of_the_logits": round(floor_us, 2),
                            "mask_bytes_per_row": words * 4})
     print(res["sampler"][-1], flush=True)
-os.makedirs("gpurun_out", exist_ok=True)
-Path("gpurun_out/lora_guided_bench.json").write_text(json.dumps(res, indent=1))
+OUT = Path(os.environ.get("TGIS_OUT_DIR", "out"))
+OUT.mkdir(parents=True, exist_ok=True)
+(OUT / "lora_guided_bench.json").write_text(json.dumps(res, indent=1))

@@ -1,6 +1,6 @@
 """Micro-benchmark of the fused sampling kernel at V = 128256 on bf16 logits (the product path's dtype): device time per
 launch (CUDA events around `iters` launches, C-ABI hook tgis_k_sampler_ex) for the BASELINE row mixes, against the HBM
-floor of ONE read of the rows' logits.  Writes gpurun_out/sampler_bench.json."""
+floor of ONE read of the rows' logits.  Writes sampler_bench.json under TGIS_OUT_DIR (default: out)."""
 import json
 import os
 import sys
@@ -72,5 +72,6 @@ for n, kind in CASES:
                     "logits_GBps": n * V * 2 / (us * 1e-6) / 1e9})
         print(json.dumps(res[-1]), flush=True)
 os.environ.pop("TGIS_SAMPLER_CLUSTER", None)
-Path("gpurun_out").mkdir(exist_ok=True)
-Path("gpurun_out/sampler_bench.json").write_text(json.dumps(res, indent=1))
+OUT = Path(os.environ.get("TGIS_OUT_DIR", "out"))
+OUT.mkdir(parents=True, exist_ok=True)
+(OUT / "sampler_bench.json").write_text(json.dumps(res, indent=1))

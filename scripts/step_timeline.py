@@ -7,6 +7,7 @@ between the previous kernel's exit and this kernel's dependency-wait return (= e
 import ctypes as C
 import dataclasses
 import json
+import os
 import sys
 from pathlib import Path
 
@@ -124,6 +125,7 @@ print("---- GEMM CTA 0, mean us after its dependency wait returned: first MMA is
 for k, (c, a1, a2, a3, a4) in sorted(gph.items()):
     print(f"{k:>18}  first_mma {a1 / c:6.2f}  last_tma {a2 / c:6.2f}  acc_ready {a3 / c:6.2f}  exit {agg[k][2] / agg[k][0]:6.2f}"
           f"  rstd {a4 / c:5.2f}")
-Path("gpurun_out").mkdir(exist_ok=True)
-Path("gpurun_out/step_timeline.json").write_text(json.dumps({"layers": L, "batch": B, "prompt": P, "rows": out_rows, "agg": agg}))
+OUT = Path(os.environ.get("TGIS_OUT_DIR", "out"))
+OUT.mkdir(parents=True, exist_ok=True)
+(OUT / "step_timeline.json").write_text(json.dumps({"layers": L, "batch": B, "prompt": P, "rows": out_rows, "agg": agg}))
 eng.close()

@@ -1,16 +1,17 @@
-"""Turn the scratch artefacts of a GPU run (gpurun_out/) into the small, tracked summaries under profiles/.
+"""Turn the scratch artefacts of a GPU run (TGIS_OUT_DIR, default: out) into the small, tracked summaries under profiles/.
 Usage: python scripts/summarize_profiles.py r01"""
 import collections
 import csv
 import io
 import json
+import os
 import shutil
 import subprocess
 import sys
 from pathlib import Path
 
 ROOT = Path(__file__).resolve().parent.parent
-SRC, DST = ROOT / "gpurun_out", ROOT / "profiles"
+SRC, DST = ROOT / os.environ.get("TGIS_OUT_DIR", "out"), ROOT / "profiles"
 tag = sys.argv[1] if len(sys.argv) > 1 else "r01"
 DST.mkdir(exist_ok=True)
 

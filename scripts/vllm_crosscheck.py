@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Cross-check of this engine and the CPU oracle against the reference's REAL engine path, and the GPU-vLLM baseline.
 
-The reference adapter's hot path is one call into vLLM (`/root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py:205-225`
+The reference adapter's hot path is one call into vLLM (`src/vllm_tgis_adapter/grpc/grpc_server.py:205-225`
 `engine.generate(prompt=TokensPrompt(prompt_token_ids=...), sampling_params=..., request_id=...)`; parameters built at
 `:560-622`).  vLLM 0.22.0 is installed on the GPU box (not importable with CUDA here), so this script runs THERE:
 
@@ -455,7 +455,7 @@ def compare(cfg_name: str, v: dict, e: dict, o: dict, e_tf: list[list[dict]]) ->
 def cmd_check(args) -> None:
     SCRATCH.mkdir(parents=True, exist_ok=True)
     gold = ROOT / "tests" / "golden"
-    outdir = ROOT / "gpurun_out"
+    outdir = ROOT / os.environ.get("TGIS_OUT_DIR", "out")
     outdir.mkdir(exist_ok=True)
     summary = {}
     for name in args.configs:
@@ -467,7 +467,7 @@ def cmd_check(args) -> None:
                            timeout=args.vllm_timeout)
         (outdir / f"vllm_run_{name}.log").write_text(r.stdout[-20000:] + "\n---- stderr ----\n" + r.stderr[-40000:])
         if r.returncode != 0 or not vpath.exists():
-            print(f"[check] {name}: vLLM run FAILED rc={r.returncode}; see gpurun_out/vllm_run_{name}.log", flush=True)
+            print(f"[check] {name}: vLLM run FAILED rc={r.returncode}; see vllm_run_{name}.log in {outdir}", flush=True)
             summary[name] = {"error": f"vllm run failed rc={r.returncode}", "stderr_tail": r.stderr[-2000:]}
             continue
         v = json.loads(vpath.read_text())
@@ -488,7 +488,7 @@ def cmd_check(args) -> None:
             fx["lenpen"] = v["lenpen"]
         # logprob floats are kept to 6 decimals: 1e-6 is far below every tolerance in play
         (gold / f"vllm_{name}.json").write_text(json.dumps(_round(fx)))
-        # only gpurun_out/ travels back from the GPU box: the fixture is copied from there into tests/golden/ and committed
+        # a fixture worth keeping is copied from there into tests/golden/ and committed
         (outdir / "golden").mkdir(exist_ok=True)
         (outdir / "golden" / f"vllm_{name}.json").write_text(json.dumps(_round(fx)))
         tag = "_opt" if all(is_opt(n) for n in args.configs) else ""
@@ -576,7 +576,7 @@ def cmd_bench_inner(args) -> None:
 
 
 def cmd_bench(args) -> None:
-    outdir = ROOT / "gpurun_out"
+    outdir = ROOT / os.environ.get("TGIS_OUT_DIR", "out")
     outdir.mkdir(exist_ok=True)
     out = outdir / "vllm_baseline.json"
     cmd = [sys.executable, __file__, "bench-inner", "--model", args.model, "--out", str(out), "--prompt-len",
@@ -607,7 +607,7 @@ def main() -> None:
         b.add_argument("--max-batched-tokens", type=int, default=2048)
         b.add_argument("--eager", type=int, default=0)
         b.add_argument("--vllm-timeout", type=int, default=1200)
-        b.add_argument("--out", default=str(ROOT / "gpurun_out" / "vllm_baseline.json"))
+        b.add_argument("--out", default=str(ROOT / os.environ.get("TGIS_OUT_DIR", "out") / "vllm_baseline.json"))
     args = ap.parse_args()
     if args.cmd == "check":
         cmd_check(args)

@@ -1,6 +1,6 @@
 """Host-logic tests (no GPU): the real gRPC servicer + async engine wrapper + detokenizer on a deterministic fake
 native engine, driven over a real grpc channel.  Mirrors what the reference's tests pin at this boundary
-(/root/reference/tests/test_grpc_server.py:42-131: non-empty text, token counts, 11 stream chunks for 10 tokens,
+(tests/test_grpc_server.py:42-131: non-empty text, token counts, 11 stream chunks for 10 tokens,
 batch of 2 -> 2 responses, Tokenize count, correlation id) and adds the numeric/semantic cases the reference never
 tests (stop sequences, stop reasons, logprobs/ranks/top-n, validation errors)."""
 import argparse

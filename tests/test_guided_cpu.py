@@ -1,5 +1,5 @@
 """Guided decoding, host side (no GPU).  What the reference pins at this seam
-(/root/reference/tests/test_grpc_server.py:170-232 `test_guided_decoding_request`): each member of the `guided` oneof
+(tests/test_grpc_server.py:170-232 `test_guided_decoding_request`): each member of the `guided` oneof
 reaches the engine as the matching StructuredOutputsParams field.  Added here: the mask-provider hook the native engine
 calls (include/tgis_engine.h `tgis_mask_fn`), the oracle's restatement of the logits masking pinned to xgrammar's own CPU
 kernel, and the whole host path over a real gRPC channel on the fake engine (the output obeys the constraint)."""

@@ -1,4 +1,4 @@
-"""LoRA adapters, host side (no GPU).  Mirrors /root/reference/tests/test_adapters.py (a LoRA adapter_id becomes a
+"""LoRA adapters, host side (no GPU).  Mirrors tests/test_adapters.py (a LoRA adapter_id becomes a
 `lora_request`, the load happens once, later requests reuse the engine's registry entry) and adds what the reference never
 tests: the error strings of adapters.py, the PEFT checkpoint reader's vLLM rules, slot recycling, and the oracle's LoRA
 arithmetic pinned to vLLM's own reference ops."""

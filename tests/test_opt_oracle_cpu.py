@@ -1,6 +1,6 @@
 """Pin the OPT oracle (oracle/opt_oracle.py) against transformers' OPTForCausalLM run in this container
 (oracle/gen_opt_golden.py -> tests/golden/opt_hf_{fp32,bf16}.json).  The reference's OPT fixture is facebook/opt-125m
-(/root/reference/tests/conftest.py:79-91 (no --model: vLLM's default, facebook/opt-125m) and tests/test_hub.py:17); the fixtures carry seeded random weights of that architecture."""
+(tests/conftest.py:79-91 (no --model: vLLM's default, facebook/opt-125m) and tests/test_hub.py:17); the fixtures carry seeded random weights of that architecture."""
 import dataclasses
 import json
 from pathlib import Path

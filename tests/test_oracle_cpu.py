@@ -1,6 +1,6 @@
 """Pin the CPU oracle against golden vectors produced by the reference's own code (oracle/gen_golden.py):
 the reference's logits_processors.py, transformers' TypicalLogitsWarper / LlamaForCausalLM and vLLM 0.22's sampler ops.
-Runs on the GPU-less box and on the GPU box (no access to /root/reference needed)."""
+Runs without a GPU and without the reference."""
 import json
 from pathlib import Path
 

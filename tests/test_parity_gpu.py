@@ -31,8 +31,9 @@ GOLD = Path(__file__).parent / "golden"
 
 
 def _record_stats(name, stats):
-    os.makedirs("gpurun_out", exist_ok=True)
-    path = "gpurun_out/parity_stats.json"
+    out = os.environ.get("TGIS_OUT_DIR", "out")
+    os.makedirs(out, exist_ok=True)
+    path = os.path.join(out, "parity_stats.json")
     allstats = {}
     if os.path.exists(path):
         with open(path) as f:

@@ -248,7 +248,7 @@ def test_generate_stream_greedy_tokens_match_oracle(live):
 def test_cfg0_125m_single_greedy_generate_matches_oracle():
     """the 125m-class model (12 layers, hidden 768; the Llama-architecture stand-in for
     facebook/opt-125m, whose weights/architecture are not available offline), ONE greedy request through `Generate` --
-    the reference's own fixture path (/root/reference/tests/test_grpc_server.py:42-49: text, token count, stop reason) --
+    the reference's own fixture path (tests/test_grpc_server.py:42-49: text, token count, stop reason) --
     checked token by token against the CPU oracle run in full."""
     from vllm_tgis_adapter_b200.engine.tokenizer import synthetic_prompt
     from vllm_tgis_adapter_b200.grpc.pb import generation_pb2 as pb

@@ -1,4 +1,4 @@
-"""Flag system: env-var fallback matrix (model: /root/reference/tests/test_tgis_utils.py:13-168) + TGIS legacy flags."""
+"""Flag system: env-var fallback matrix (model: tests/test_tgis_utils.py:13-168) + TGIS legacy flags."""
 import argparse
 
 import pytest

@@ -1,5 +1,5 @@
 """-m gpu parity of the OPT model family (the reference's own test model is facebook/opt-125m:
-/root/reference/tests/conftest.py:79-91 leaves --model at vLLM's default, tests/test_hub.py:17 names it).
+tests/conftest.py:79-91 leaves --model at vLLM's default, tests/test_hub.py:17 names it).
 
 Kernel level: csrc/opt.cu against the arithmetic of oracle/opt_oracle.py (torch.nn.LayerNorm / F.linear(x, W, b) / ReLU
 rounding points).  Engine level, through the C ABI: greedy tokens, logprobs, ranks and prompt logprobs against the CPU
@@ -96,8 +96,9 @@ def _record(name, stats):
     import json
     import os
 
-    os.makedirs("gpurun_out", exist_ok=True)
-    path = "gpurun_out/parity_stats_opt.json"
+    out = os.environ.get("TGIS_OUT_DIR", "out")
+    os.makedirs(out, exist_ok=True)
+    path = os.path.join(out, "parity_stats_opt.json")
     allstats = json.load(open(path)) if os.path.exists(path) else {}
     allstats[name] = stats
     with open(path, "w") as f:
@@ -336,7 +337,7 @@ def test_cfg0_opt_125m_single_greedy_generate_matches_oracle():
     """BASELINE.json configs[0] on the architecture it names: facebook/opt-125m's dims (12 layers, hidden 768, 12 x 64-dim
     heads, ffn 3072, vocab 50272, learned positions, biases, LayerNorm, ReLU; seeded random weights -- the hub checkpoint
     is not obtainable offline), ONE greedy request through `Generate` -- the reference's fixture path
-    (/root/reference/tests/test_grpc_server.py:42-49: text, token count, stop reason) -- token by token against the oracle."""
+    (tests/test_grpc_server.py:42-49: text, token count, stop reason) -- token by token against the oracle."""
     from oracle.opt_oracle import OPTOracle
     from test_server_gpu import LiveServer
     from vllm_tgis_adapter_b200.engine.tokenizer import synthetic_prompt

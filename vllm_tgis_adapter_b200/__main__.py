@@ -1,6 +1,6 @@
-"""`python -m vllm_tgis_adapter` entrypoint (shim in /root/repo/vllm_tgis_adapter/__main__.py).
+"""`python -m vllm_tgis_adapter` entrypoint (shim in vllm_tgis_adapter/__main__.py).
 
-Same supervision structure as /root/reference/src/vllm_tgis_adapter/__main__.py:38-131: build the engine, run the
+Same supervision structure as src/vllm_tgis_adapter/__main__.py:38-131: build the engine, run the
 HTTP and gRPC servers as tasks, exit as soon as either stops or the engine dies (:66-97), write the termination log
 (:100-111)."""
 from __future__ import annotations

@@ -1,7 +1,7 @@
 """ctypes binding of libtgis_engine.so (C ABI: include/tgis_engine.h, include/tgis_kernels.h).
 
 This is the reference-side binding a maintainer would add next to `build_async_engine_client`
-(/root/reference/src/vllm_tgis_adapter/__main__.py:48); see INTEGRATION.md.  There is no Python/CPU fallback: if the
+(src/vllm_tgis_adapter/__main__.py:48); see INTEGRATION.md.  There is no Python/CPU fallback: if the
 library is missing it is built with nvcc, and if that is impossible the import fails loudly.
 """
 from __future__ import annotations

@@ -1,5 +1,5 @@
 """`EngineClient`-shaped façade over the native engine: the object the TGIS gRPC servicer holds where the reference
-holds vLLM's AsyncLLM (/root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py:166-176).
+holds vLLM's AsyncLLM (src/vllm_tgis_adapter/grpc/grpc_server.py:166-176).
 
 Members implemented = exactly the ones the reference touches: generate / abort / get_tokenizer /
 is_tracing_enabled / errored / is_running / vllm_config.model_config.max_model_len / get_model_config.

@@ -1,6 +1,6 @@
 """Guided decoding, host side: grammar matchers that feed the engine's mask provider hook.
 
-Reference seam: /root/reference/src/vllm_tgis_adapter/tgis_utils/structured_outputs.py:14-38 turns the request's
+Reference seam: src/vllm_tgis_adapter/tgis_utils/structured_outputs.py:14-38 turns the request's
 `DecodingParameters.guided` oneof into vLLM `StructuredOutputsParams`; vLLM then (v1/structured_output/backend_xgrammar.py)
 compiles the spec with the xgrammar library, keeps one `GrammarMatcher` per request, fills a token bitmask per step
 (v1/structured_output/__init__.py:204-300) and masks the logits before its sampler.  Here the split is the same: xgrammar

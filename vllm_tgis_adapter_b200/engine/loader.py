@@ -1,5 +1,5 @@
 """Build the engine the way `build_async_engine_client(args)` does for the reference
-(/root/reference/src/vllm_tgis_adapter/__main__.py:48): read the HF model directory (config.json + *.safetensors),
+(src/vllm_tgis_adapter/__main__.py:48): read the HF model directory (config.json + *.safetensors),
 stream each tensor into libtgis_engine.so ("PyTorch tensors for weights only"), attach a tokenizer.
 
 Offline builds have no checkpoints: `--model <preset> --synthetic-weights` creates seeded N(0, 0.02)

@@ -1,6 +1,6 @@
 """LoRA adapters, host side: PEFT checkpoint -> engine adapter slot.
 
-Reference seam: /root/reference/src/vllm_tgis_adapter/grpc/adapters.py:63-163 resolves `adapter_id` to a directory under
+Reference seam: src/vllm_tgis_adapter/grpc/adapters.py:63-163 resolves `adapter_id` to a directory under
 the adapter cache, reads `adapter_config.json`, and hands a `LoRARequest` to vLLM, which loads the weights
 (vllm/lora/lora_model.py `from_local_checkpoint` / `from_lora_tensors`, peft_helper.py) and applies them per request.
 What is restated here, with the vLLM lines it follows:

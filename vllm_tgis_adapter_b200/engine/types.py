@@ -1,5 +1,5 @@
 """Value types crossing the drop-in boundary: the subset of vLLM's SamplingParams / RequestOutput /
-CompletionOutput / Logprob that /root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py actually touches
+CompletionOutput / Logprob that src/vllm_tgis_adapter/grpc/grpc_server.py actually touches
 (:205-225 generate kwargs, :282-283,298,374,438-456 RequestOutput, :391-392,477-487,670-690 CompletionOutput,
 :727-755 Logprob).  Same attribute names so the adapter code reads identically."""
 from __future__ import annotations
@@ -17,7 +17,7 @@ class RequestOutputKind(enum.Enum):
 @dataclasses.dataclass
 class StructuredOutputsParams:
     """vllm/sampling_params.py `StructuredOutputsParams`, the members the adapter sets
-    (/root/reference/src/vllm_tgis_adapter/tgis_utils/structured_outputs.py:14-38): exactly one of them."""
+    (src/vllm_tgis_adapter/tgis_utils/structured_outputs.py:14-38): exactly one of them."""
 
     json: str | dict | None = None
     regex: str | None = None

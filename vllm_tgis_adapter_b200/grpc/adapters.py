@@ -1,6 +1,6 @@
 """adapter_id -> `lora_request` kwarg of engine.generate.
 
-Behavioural mirror of /root/reference/src/vllm_tgis_adapter/grpc/adapters.py:63-223 (same entry point name, same error
+Behavioural mirror of src/vllm_tgis_adapter/grpc/adapters.py:63-223 (same entry point name, same error
 strings through TGISValidationError, same caching rule: LoRA adapters are remembered by the ENGINE's registry, other
 adapter types by the store).  The reference asks vLLM's `OpenAIServingModels.load_lora_adapter`; here the engine façade
 (`AsyncTGISEngine.load_lora_adapter` / `.lora_requests`) plays that part."""

@@ -1,6 +1,6 @@
 """`fmaas.GenerationService` servicer on top of the B200-native engine.
 
-Behavioural mirror of /root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py (same RPC surface, same parameter
+Behavioural mirror of src/vllm_tgis_adapter/grpc/grpc_server.py (same RPC surface, same parameter
 mapping, same stop-reason / token-info conversion, same error strings and status codes) with the engine call
 `self.engine.generate(...)` (:222) landing in libtgis_engine.so instead of vLLM.  Each method cites the reference
 lines whose behaviour it reproduces.  Differences, all deliberate:

@@ -1,7 +1,7 @@
 """grpc.health.v1.Health (Check + Watch) without the grpcio-health-checking package (absent in this image).
 
 The reference registers grpc_health's HealthServicer and flips `fmaas.GenerationService` to SERVING in post_init
-(/root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py:195-203,907-908); its tests and the k8s probe CLI
+(src/vllm_tgis_adapter/grpc/grpc_server.py:195-203,907-908); its tests and the k8s probe CLI
 (healthcheck.py:1-96) poll `Check`.  The two messages are tiny, so they are declared at run time like generation_pb2."""
 from __future__ import annotations
 

@@ -2,7 +2,7 @@
 
 `grpc_tools.protoc` (which the reference runs in setup.py:22-36 to generate generation_pb2*.py) is not available in
 this image, so the FileDescriptorProto is written out by hand, field for field, from
-/root/reference/src/vllm_tgis_adapter/grpc/pb/generation.proto:1-279 (package, message names, field NUMBERS, proto3
+src/vllm_tgis_adapter/grpc/pb/generation.proto:1-279 (package, message names, field NUMBERS, proto3
 `optional` presence, the `guided` oneof, enum values).  The resulting classes are byte-compatible with the
 reference's generated module and expose the same names (`BatchedGenerationRequest`, `StopReason`, ...,
 `DESCRIPTOR.services_by_name["GenerationService"]`).

@@ -2,7 +2,7 @@
 (absent in this image).
 
 The reference enables it for `health`, `fmaas.GenerationService` and the reflection service itself
-(/root/reference/src/vllm_tgis_adapter/grpc/grpc_server.py:919-926) so that `grpcurl` (examples/inference.sh) can
+(src/vllm_tgis_adapter/grpc/grpc_server.py:919-926) so that `grpcurl` (examples/inference.sh) can
 discover the API.  The protocol is one bidi stream of small oneof messages; both package versions share the wire
 layout, so one run-time-built descriptor per package serves both.  What is answered: list_services,
 file_containing_symbol, file_by_filename; extension queries return NOT_FOUND / empty (proto3 files, no extensions)."""

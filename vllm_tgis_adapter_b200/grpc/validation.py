@@ -1,6 +1,6 @@
 """TGIS request validation with the error strings of the TGIS API.
 
-Behavioural mirror of /root/reference/src/vllm_tgis_adapter/grpc/validation.py:1-144 (message texts at :18-61 must
+Behavioural mirror of src/vllm_tgis_adapter/grpc/validation.py:1-144 (message texts at :18-61 must
 match the TGIS router byte for byte because clients grep them); re-written, not copied: checks are table driven.
 """
 from __future__ import annotations

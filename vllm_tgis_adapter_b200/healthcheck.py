@@ -1,6 +1,6 @@
 """k8s probe CLI: one unary `grpc.health.v1.Health/Check` against a running server, exit status 0 = SERVING.
 
-Mirrors the reference's probe (/root/reference/src/vllm_tgis_adapter/healthcheck.py:1-96, console script
+Mirrors the reference's probe (src/vllm_tgis_adapter/healthcheck.py:1-96, console script
 `grpc_healthcheck`, pyproject.toml:46): same flags (`--insecure` | `--secure`, `--server-url`, `--timeout`,
 `--service-name`), same defaults (localhost:8033, 1 s, `fmaas.GenerationService`), same two output shapes
 (`health check...status: SERVING` / `health check...Health.Check failed: code=..., details=...`) and exit codes, so a

@@ -1,5 +1,5 @@
 """HTTP side-car: /health and /metrics (Prometheus text), the two endpoints k8s probes and dashboards hit on the
-reference's HTTP port (/root/reference/src/vllm_tgis_adapter/http.py:41-99, tests/test_http_server.py:4-34).  The
+reference's HTTP port (src/vllm_tgis_adapter/http.py:41-99, tests/test_http_server.py:4-34).  The
 OpenAI routes the reference re-exports from vLLM are out of scope."""
 from __future__ import annotations
 

@@ -1,5 +1,5 @@
 """Request-level Prometheus metrics under vLLM's metric names, so dashboards built for the reference's /metrics keep
-working (the reference re-exports vLLM's registry: /root/reference/src/vllm_tgis_adapter/http.py:41-99; names from
+working (the reference re-exports vLLM's registry: src/vllm_tgis_adapter/http.py:41-99; names from
 vllm v1/metrics/loggers.py `PrometheusStatLogger`).  Engine-level gauges are read from `tgis_engine_status` at scrape
 time; the histograms are fed by AsyncTGISEngine when a request finishes, from the engine's own timestamps."""
 from __future__ import annotations

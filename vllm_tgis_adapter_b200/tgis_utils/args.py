@@ -1,6 +1,6 @@
 """Flag system: every `--foo-bar` flag also reads env `FOO_BAR`, plus the TGIS legacy flag names.
 
-Behavioural mirror of /root/reference/src/vllm_tgis_adapter/tgis_utils/args.py (env fallback :30-98, TGIS flags
+Behavioural mirror of src/vllm_tgis_adapter/tgis_utils/args.py (env fallback :30-98, TGIS flags
 :101-181, legacy->native translation :184-258) on plain argparse: vLLM's FlexibleArgumentParser and its ~200 engine
 flags have no meaning for this engine, so only the flags the serving path needs exist."""
 from __future__ import annotations

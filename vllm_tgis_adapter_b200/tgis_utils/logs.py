@@ -1,6 +1,6 @@
 """TGIS-style request / response log lines.
 
-Same two lines, same field layout as /root/reference/src/vllm_tgis_adapter/tgis_utils/logs.py:150-226
+Same two lines, same field layout as src/vllm_tgis_adapter/tgis_utils/logs.py:150-226
 ("Processing request: {...}" / "Finished processing request: {...}. Timing info: {...}. Generated N tokens ..."),
 same correlation-id blackboard (:29-45).  The reference monkey-patches engine.generate (:48-114); here the wrapper is an
 explicit async generator the servicer calls, and the timing fields come from the engine's CLOCK_MONOTONIC stamps."""

@@ -1,4 +1,4 @@
-"""Termination log + task helpers (reference: /root/reference/src/vllm_tgis_adapter/utils.py:1-44)."""
+"""Termination log + task helpers (reference: src/vllm_tgis_adapter/utils.py:1-44)."""
 from __future__ import annotations
 
 import asyncio
