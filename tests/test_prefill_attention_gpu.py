@@ -126,3 +126,32 @@ def test_values_that_are_not_finite_reach_only_the_rows_that_see_them(g, n_q, n_
     if n_kv > 1:   # the last block reaches the last unit of the other heads alone: the rows in front keep their bits
         first = 420 - 2 * (128 // (n_q // n_kv) // 8 * 8) - 1
         assert torch.equal(got[:first, : n_q // n_kv], clean[:first, : n_q // n_kv])
+
+
+@pytest.mark.parametrize("n_q,n_kv,scale", [(8, 2, 128 ** -0.5), (8, 1, 128 ** -0.5), (2, 2, 128 ** -0.5), (6, 2, -0.05), (5, 1, 128 ** -0.5)])
+def test_few_short_prompts_have_the_bits_of_many(g, n_q, n_kv, scale):
+    """Up to 128 keys and no more units than SMs: one accumulator per CTA and rings as long as the longest sequence.  Every length around
+    its blocks and rows, alone and two at a time, against 64 bits and against the launch that a longer prompt beside it asks for."""
+    parts = [(a, b) for b in (2, 17, 32, 33, 63, 64, 65, 96, 97, 127, 128) for a in (0, 1, 30, 31, 32, 95) if b - a > 1]
+    case = Case(g, n_q, n_kv, [b for _, b in parts] + [300], seed=n_q + n_kv, size=3.0)
+    beside = case.run([(len(parts), 0, 300)] + [(s, a, b) for s, (a, b) in enumerate(parts)], scale)[1:]
+    alone = [case.run([(s, a, b)], scale)[0] for s, (a, b) in enumerate(parts)]
+    for s in range(len(parts) - 1):
+        alone[s: s + 2] = case.run([(i, *parts[i]) for i in (s, s + 1)], scale) if s % 3 == 0 else alone[s: s + 2]
+    for s, (a, b) in enumerate(parts):
+        want = case.exact(s, a, b, scale)
+        assert torch.equal(alone[s], beside[s]), (a, b)
+        bound = 1.001 * 2 ** -8 * want.abs() + 5 * (2 ** -16 + 100 * 2 ** -19)   # as above
+        assert float(((alone[s].double() - want).abs() - bound).max()) <= 0.0, (a, b)
+
+
+def test_a_value_that_is_not_finite_in_a_short_prompt(g):
+    case = Case(g, 8, 2, [60], seed=8)
+    want = case.exact(0, 0, 60)
+    case.v[case.slots[0][40], 0, 9] = math.inf
+    case.vc = g.v_cache_from_dense(case.v, case.bt.shape[1])
+    got = case.run([(0, 0, 60)])[0].double()
+    sees = torch.zeros(60, 8, 128, dtype=torch.bool, device="cuda")
+    sees[40:, :4, 9] = True
+    bound = 1.001 * 2 ** -8 * want.abs() + 5 * (2 ** -16 + 100 * 2 ** -19)   # as above
+    assert not bool(got[sees].isfinite().any()) and float(((got - want).abs() - bound)[~sees].max()) <= 0.0

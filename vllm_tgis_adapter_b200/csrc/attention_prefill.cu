@@ -25,9 +25,16 @@
 // units: 2048 tokens are 256 of them, so some SMs work twice and some once.  Microseconds a launch on one B200, 32 query
 // and 8 kv heads, against the mma.sync kernel that went before (16 tokens x one head a warp, 32-token blocks, its pipe 56 %
 // active): 1859 tokens behind 6144: 1289 -> 345 (620 TFLOP/s, counting P V once); 2048 alone 243 -> 61; 2048 in 6 prompts 71 -> 30;
-// 32 prompts of 64 tokens 21.7 -> 16.1; 96 of 9 to 56 33.3 -> 29.3; one of 17 tokens 4.2 -> 6.3, of which a chain hides the
-// first two (the block table is read under the kernel before).  No faster: two threads per row (345 -> 356, short prompts
+// 32 prompts of 64 tokens 21.7 -> 16.1; 96 of 9 to 56 33.3 -> 29.3.  No faster: two threads per row (345 -> 356, short prompts
 // 29 -> 39), tiles of 64 tokens with scores two tiles ahead (404), P handed over in halves (344).
+//
+// One short prompt is a chain of latencies and of CTAs that wait for their SM: with two accumulators a CTA takes all of its registers and
+// shared memory, so neither it nor the product behind it can be resident under the kernel before.  A step of at most 128 keys a sequence
+// and one unit per SM (prefill_units_build) therefore has one accumulator per CTA and rings as long as its longest sequence; and of
+// at most 32 keys 90 registers a thread, which is what fits beside a CTA of the product cut along k.  Microseconds of a whole prompt step,
+// mma.sync kernel -> two accumulators -> this: 8 layers of the 8B model, 17 tokens 839 -> 867 -> 840, 32 tokens 867 -> 897 -> 874, 64 tokens
+// 1019 -> 951 -> 917; 12 layers 768 wide, 17 tokens 364 -> 400 -> 378, 64 tokens 634 -> 686 -> 667 (the mma.sync kernel stays ahead there:
+// its operands need no copy, barrier and commit each; but a row's bits would depend on its step if it took these).
 //
 // No wait is unbounded: after about two seconds a role gives up, raises the word that gemm_pair_failed() looks at and leaves;
 // copies and MMAs in flight land first and TMEM is freed on every path.
@@ -40,15 +47,15 @@
 namespace tgis {
 namespace {
 
-constexpr int PT_THREADS = 384;                          // warps 0..3 softmax of accumulator 0, 4..7 of 1, 8 copies, 9 MMAs, 10 and 11 idle
-constexpr int PT_WARP_COPY = 8, PT_WARP_MMA = 9;
+// ACC accumulators: warps 0..3 softmax of accumulator 0, 4..7 of 1, then one for copies, one for MMAs, (ACC = 2) two idle
+constexpr int PT_THREADS(int acc) { return acc == 2 ? 384 : 192; }
 constexpr int PT_REGS_SOFTMAX = 208, PT_REGS_OTHER = 88; // 256 x 208 + 128 x 88 = 384 x 168, what the launch gives every thread
 constexpr int PT_KV = 128;                               // tokens of a cache tile
 constexpr int PT_BLOCKS = PT_KV / KV_BLOCK;
 constexpr int PT_BLOCK_BYTES = KV_BLOCK * HEAD_DIM * 2;
 constexpr int PT_TILE_BYTES = PT_KV * HEAD_DIM * 2;      // 32 KiB: a K tile, a V tile, one accumulator's Q
-constexpr int PT_STAGES = 2;
-constexpr size_t PT_SMEM = (size_t)(2 + 2 * PT_STAGES) * PT_TILE_BYTES + 1024 + 256;
+// Q, rings of ACC tiles of `blocks` cache blocks for K and V, barriers
+constexpr size_t PT_SMEM(int acc, int blocks) { return (size_t)acc * (PT_TILE_BYTES + 2 * blocks * PT_BLOCK_BYTES) + 1024 + 256; }
 constexpr float PT_SLACK = 8.f;                          // exp2 domain: how far a score may exceed its row's reference
 
 struct PrefillArgs {
@@ -57,6 +64,7 @@ struct PrefillArgs {
   const int32_t* block_table;
   __nv_bfloat16* out;
   int n_units, bt_stride, qkv_ld, out_ld, n_kv, G, TM;
+  int blocks;                                            // ACC = 1: of a tile (all keys of a unit)
   float sl2;                                             // |scale| * log2(e)
   uint32_t minus;                                        // scale < 0: bit "negate A" of the score products' descriptor
   int* err;
@@ -233,6 +241,7 @@ __device__ __forceinline__ void attend_row(const PrefillArgs& a, int block_row, 
 
 // The CTA's rows that came out with numbers that are not finite, by its softmax warps, which have stored them all.  Where the value of
 // a row's own token accounts for them (a token that has overflowed in full, and all that follow it in the next layers) they stand.
+template <int ACC>
 __device__ __noinline__ void sum_again(const PrefillArgs& a) {
   const int lane = (int)lane_id();
   auto odd = [](const uint2& w) {   // one bit per number of four
@@ -241,7 +250,7 @@ __device__ __noinline__ void sum_again(const PrefillArgs& a) {
   };
   Unit u;
   for (UnitIter it(a); it.next(u);)
-    for (int r = threadIdx.x >> 5; r < u.rows * a.G; r += PT_WARP_COPY) {
+    for (int r = threadIdx.x >> 5; r < u.rows * a.G; r += 4 * ACC) {
       const int t = r / a.G, row = u.row0 + t, head = u.kvh * a.G + r - t * a.G, pos = u.pos0 + t;
       const int mine = odd(*reinterpret_cast<const uint2*>(a.out + (size_t)row * a.out_ld + (size_t)head * HEAD_DIM + lane * 4));
       if (!__any_sync(0xffffffffu, mine != 0)) continue;
@@ -251,14 +260,17 @@ __device__ __noinline__ void sum_again(const PrefillArgs& a) {
     }
 }
 
-__global__ void __launch_bounds__(PT_THREADS, 1)
+template <int ACC, int BLOCKS>
+__global__ void __launch_bounds__(PT_THREADS(ACC), BLOCKS == 1 ? 3 : 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap vmap, const __grid_constant__ PrefillArgs a) {
+  constexpr int PT_WARP_COPY = 4 * ACC, PT_WARP_MMA = PT_WARP_COPY + 1, PT_STAGES = ACC;
+  const int tile_blocks = ACC == 2 ? PT_BLOCKS : a.blocks, ring_bytes = tile_blocks * PT_BLOCK_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* q_s = smem;
-  uint8_t* k_s = q_s + 2 * PT_TILE_BYTES;
-  uint8_t* v_s = k_s + PT_STAGES * PT_TILE_BYTES;
-  uint64_t* q_full = reinterpret_cast<uint64_t*>(v_s + PT_STAGES * PT_TILE_BYTES);
+  uint8_t* k_s = q_s + ACC * PT_TILE_BYTES;
+  uint8_t* v_s = k_s + PT_STAGES * ring_bytes;
+  uint64_t* q_full = reinterpret_cast<uint64_t*>(v_s + PT_STAGES * ring_bytes);
   uint64_t* q_empty = q_full + 1;
   uint64_t* k_full = q_empty + 1;
   uint64_t* k_empty = k_full + PT_STAGES;
@@ -272,6 +284,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   volatile int* redo = gave_up + 1;         // rows of the CTA have to be summed again
 
   const int warp = threadIdx.x >> 5, lane = (int)lane_id();
+  // units and block table are written by the host before the step: they are read while the kernel before this one still runs
+  UnitIter it(a);
+  auto tiles = [](const Unit& u) { return ACC == 2 ? u.n_kt : 1; };
   if (warp == PT_WARP_MMA) {
     if (elect_one()) {
       mbar_init(q_full, 1);
@@ -292,7 +307,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
       fence_barrier_init();
     }
     __syncwarp();
-    tmem_alloc<512>(tmem_base_smem);
+    tmem_alloc<256 * ACC>(tmem_base_smem);
   }
   if (warp == PT_WARP_COPY && lane == 0) {
     tma_prefetch_desc(&qmap);
@@ -301,14 +316,12 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_base_smem;   // [S0 | S1 | O0 | O1], 128 columns each
+  const uint32_t tmem_base = *tmem_base_smem;   // [S0 | S1 | O0 | O1] or [S0 | O0], 128 columns each
   griddep_launch();
-  // units and block table are written by the host before the step: they are read while the kernel before this one still runs
-  UnitIter it(a);
   Unit u;
   bool ok = true;
   if (warp >= PT_WARP_COPY) {
-    set_regs<PT_REGS_OTHER, false>();
+    if constexpr (ACC == 2) set_regs<PT_REGS_OTHER, false>();
     if (warp == PT_WARP_COPY) {
       // ===================== copies =====================
       int kst = 0, vst = 0;
@@ -331,17 +344,20 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
             for (int h = 0; h < 2; ++h)
               tma_load_3d(&qmap, q_full, q_s + g * PT_TILE_BYTES + h * (PT_TILE_BYTES / 2), h * 64, u.kvh * a.G, u.row0 + g * a.TM);
         }
-        for (int j = 0; j < u.n_kt; ++j) {
+        for (int j = 0; j < tiles(u); ++j) {
           const int nb = min(PT_BLOCKS, u.n_blk - j * PT_BLOCKS);
           ok = __all_sync(0xffffffffu, bounded_wait(&k_empty[kst], kph, a.err));
           if (!ok) break;
           if (lane == 0) mbar_arrive_expect_tx(&k_full[kst], nb * PT_BLOCK_BYTES);
           __syncwarp();
-          for (int b = lane >> 4; b < PT_BLOCKS; b += 2) {   // lane -> (block, chunk)
+          // a block by itself lies as in the cache (one copy; sixteen take the copy unit half a microsecond)
+          if (nb == 1 && lane == 0)
+            bulk_load_1d(k_s + kst * ring_bytes, a.k_cache + ((size_t)blk * a.n_kv + u.kvh) * (KV_BLOCK * HEAD_DIM), PT_BLOCK_BYTES, &k_full[kst]);
+          for (int b = lane >> 4; nb > 1 && b < PT_BLOCKS; b += 2) {   // lane -> (block, chunk)
             const int pb = __shfl_sync(0xffffffffu, blk, b);
             const int c = lane & 15;
             if (b < nb)
-              bulk_load_1d(k_s + kst * PT_TILE_BYTES + c * (PT_KV * 16) + b * (KV_BLOCK * 16),
+              bulk_load_1d(k_s + kst * ring_bytes + c * (tile_blocks * KV_BLOCK * 16) + b * (KV_BLOCK * 16),
                            a.k_cache + ((size_t)pb * a.n_kv + u.kvh) * (KV_BLOCK * HEAD_DIM) + c * (KV_BLOCK * 8), KV_BLOCK * 16, &k_full[kst]);
           }
           if (++kst == PT_STAGES) kst = 0, kph ^= 1;
@@ -350,7 +366,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
           if (lane == 0) mbar_arrive_expect_tx(&v_full[vst], nb * PT_BLOCK_BYTES);
           __syncwarp();
           if (lane < nb)
-            tma_load_3d(&vmap, &v_full[vst], v_s + vst * PT_TILE_BYTES + lane * PT_BLOCK_BYTES, 0, (blk * a.n_kv + u.kvh) * KV_BLOCK, 0);
+            tma_load_3d(&vmap, &v_full[vst], v_s + vst * ring_bytes + lane * PT_BLOCK_BYTES, 0, (blk * a.n_kv + u.kvh) * KV_BLOCK, 0);
           if (++vst == PT_STAGES) vst = 0, vph ^= 1;
           blk = block_of(j + 1);
         }
@@ -363,23 +379,24 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
       const uint32_t idesc_pv = make_idesc_bf16(128, HEAD_DIM) | (1u << 16);   // B (V) has its dims contiguous
       auto scores = [&](int g, int nb) {
         const uint32_t idesc = make_idesc_bf16(128, nb * KV_BLOCK) | a.minus;
-        const uint32_t q = smem_u32(q_s + g * PT_TILE_BYTES), k = smem_u32(k_s + kst * PT_TILE_BYTES);
+        const uint32_t q = smem_u32(q_s + g * PT_TILE_BYTES), k = smem_u32(k_s + kst * ring_bytes);
+        const uint32_t chunk = (nb == 1 ? 1 : tile_blocks) * KV_BLOCK * 16;
 #pragma unroll
         for (int ks = 0; ks < HEAD_DIM / 16; ++ks)
           tc_mma_f16(tmem_base + g * 128, make_smem_desc_sw128(q + ((7 - ks) >> 2) * (PT_TILE_BYTES / 2) + ((7 - ks) & 3) * 32),
-                     smem_desc(k + (7 - ks) * 2 * (PT_KV * 16), PT_KV * 16, 128, 0), idesc, ks > 0);
+                     smem_desc(k + (7 - ks) * 2 * chunk, chunk, 128, 0), idesc, ks > 0);
         tc_commit(&s_full[g]);
       };
       auto values = [&](int g, int nb, bool first) {
-        const uint32_t v = smem_u32(v_s + vst * PT_TILE_BYTES);
+        const uint32_t v = smem_u32(v_s + vst * ring_bytes);
         for (int ks = 0; ks < 2 * nb; ++ks) {
           const uint64_t vd = smem_desc(v + (ks >> 1) * PT_BLOCK_BYTES + (ks & 1) * 2048, PT_BLOCK_BYTES / 2, 1024, 2);
-          mma_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + ks * 8, vd, idesc_pv, !(first && ks == 0));
-          mma_ts(tmem_base + 256 + g * 128, tmem_base + g * 128 + 64 + ks * 8, vd, idesc_pv, 1);
+          mma_ts(tmem_base + ACC * 128 + g * 128, tmem_base + g * 128 + ks * 8, vd, idesc_pv, !(first && ks == 0));
+          mma_ts(tmem_base + ACC * 128 + g * 128, tmem_base + g * 128 + 64 + ks * 8, vd, idesc_pv, 1);
         }
       };
       while (ok && it.next(u)) {
-        const int groups = u.two ? 2 : 1;
+        const int groups = ACC == 2 && u.two ? 2 : 1;
         auto blocks = [&](int j) { return min(PT_BLOCKS, u.n_blk - j * PT_BLOCKS); };
         ok = __all_sync(0xffffffffu, bounded_wait(q_full, qph, a.err) && bounded_wait(&k_full[kst], kph, a.err));
         if (!ok) break;
@@ -388,12 +405,12 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         if (elect_one()) {
           for (int g = 0; g < groups; ++g) scores(g, blocks(0));
           tc_commit(&k_empty[kst]);
-          if (u.n_kt == 1) tc_commit(q_empty);
+          if (tiles(u) == 1) tc_commit(q_empty);
         }
         __syncwarp();
         if (++kst == PT_STAGES) kst = 0, kph ^= 1;
-        for (int j = 0; j < u.n_kt && ok; ++j) {
-          const bool more = j + 1 < u.n_kt;
+        for (int j = 0; j < tiles(u) && ok; ++j) {
+          const bool more = j + 1 < tiles(u);
           ok = __all_sync(0xffffffffu, bounded_wait(&v_full[vst], vph, a.err));
           for (int g = 0; g < groups && ok; ++g) {
             ok = __all_sync(0xffffffffu, bounded_wait(&p_full[g], pph[g], a.err) && (g > 0 || !more || bounded_wait(&k_full[kst], kph, a.err)));
@@ -407,7 +424,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
               if (last) {
                 tc_commit(&v_empty[vst]);
                 if (more) tc_commit(&k_empty[kst]);
-                if (j + 2 == u.n_kt) tc_commit(q_empty);
+                if (j + 2 == tiles(u)) tc_commit(q_empty);
               }
               if (!more) tc_commit(&o_full[g]);
             }
@@ -420,12 +437,12 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
     }
   } else {
     // ===================== softmax: thread = row =====================
-    set_regs<PT_REGS_SOFTMAX, true>();
+    if constexpr (ACC == 2) set_regs<PT_REGS_SOFTMAX, true>();
     const int g = warp >> 2;
     const int r = (warp & 3) * 32 + lane, tok = r / a.G, head = r - tok * a.G;
     const int tok_lo = (warp & 3) * 32 / a.G;                       // first token of the warp
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t s_t = tmem_base + g * 128 + lanes, o_t = tmem_base + 256 + g * 128 + lanes;
+    const uint32_t s_t = tmem_base + g * 128 + lanes, o_t = tmem_base + ACC * 128 + g * 128 + lanes;
     const uint64_t sl2_2 = pack2(a.sl2, a.sl2), minus1 = pack2(-1.f, -1.f);
     uint32_t sph = 0, oph = 0;
     griddep_wait();   // `out` may still be read
@@ -433,32 +450,37 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
       if (g == 1 && !u.two) continue;
       const int pos = u.pos0 + g * a.TM + tok, pos_lo = u.pos0 + g * a.TM + tok_lo;
       float m = 0.f, l = 0.f;
-      for (int j = 0; j < u.n_kt; ++j) {
-        const int nb = min(PT_BLOCKS, u.n_blk - j * PT_BLOCKS);
+      for (int j = 0; j < tiles(u); ++j) {
+        const int nb = BLOCKS == 1 ? 1 : min(PT_BLOCKS, u.n_blk - j * PT_BLOCKS);
         const int lim = pos - j * PT_KV;   // last column this row sees
         const bool mask = j * PT_KV + nb * KV_BLOCK - 1 > pos_lo;
         ok = __all_sync(0xffffffffu, bounded_wait(&s_full[g], sph, a.err));
         if (!ok) break;
         sph ^= 1;
         tc_fence_after();
-        uint32_t s[PT_KV];
+        uint32_t s[BLOCKS * KV_BLOCK];
+        // (one way out of each loop: a prompt of a block would else run past all of their code, which no cache holds yet)
 #pragma unroll
-        for (int c = 0; c < PT_BLOCKS; ++c)
-          if (c < nb) tmem_ld_x32(s_t + c * 32, s + c * 32);
+        for (int c = 0; c < BLOCKS; ++c) {
+          if (c >= nb) break;
+          tmem_ld_x32(s_t + c * 32, s + c * 32);
+        }
         tmem_ld_wait();
         if (mask) {
 #pragma unroll
-          for (int i = 0; i < PT_KV; ++i)
-            if (i > lim) s[i] = __float_as_uint(-INFINITY);
-        }
-        float mx[PT_BLOCKS];
+          for (int c = 0; c < BLOCKS; ++c) {
+            if (c >= nb) break;
 #pragma unroll
-        for (int c = 0; c < PT_BLOCKS; ++c) {
-          mx[c] = -INFINITY;
-          if (c < nb) {
-#pragma unroll
-            for (int i = 0; i < 32; i += 2) mx[c] = fmaxf(mx[c], fmaxf(__uint_as_float(s[c * 32 + i]), __uint_as_float(s[c * 32 + i + 1])));
+            for (int i = c * 32; i < c * 32 + 32; ++i)
+              if (i > lim) s[i] = __float_as_uint(-INFINITY);
           }
+        }
+        float mx[PT_BLOCKS] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+        for (int c = 0; c < BLOCKS; ++c) {
+          if (c >= nb) break;
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) mx[c] = fmaxf(mx[c], fmaxf(__uint_as_float(s[c * 32 + i]), __uint_as_float(s[c * 32 + i + 1])));
         }
         const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * a.sl2;
         if (j == 0) {
@@ -482,27 +504,26 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
         const uint64_t neg_m = pack2(-ref, -ref);
         uint64_t sum0 = 0, sum1 = 0;
 #pragma unroll
-        for (int c = 0; c < 2 * PT_BLOCKS; ++c) {
-          if (c < 2 * nb) {
-            uint32_t hi[8], lo[8];
+        for (int c = 0; c < 2 * BLOCKS; ++c) {
+          if (c >= 2 * nb) break;
+          uint32_t hi[8], lo[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int col = c * 16 + 2 * i;
-              float x, y;
-              unpack2(fma2(pack2(__uint_as_float(s[col]), __uint_as_float(s[col + 1])), sl2_2, neg_m), x, y);
-              x = ex2(x);
-              y = ex2(y);
-              const uint64_t p = pack2(x, y);
-              if (i & 1) sum1 = add2(sum1, p);
-              else sum0 = add2(sum0, p);
-              hi[i] = cvt2(x, y);
-              const uint64_t back = pack2(__uint_as_float(hi[i] << 16), __uint_as_float(hi[i] & 0xffff0000u));
-              unpack2(fma2(back, minus1, p), x, y);
-              lo[i] = cvt2(x, y);
-            }
-            tmem_st_x8(s_t + c * 8, hi);
-            tmem_st_x8(s_t + 64 + c * 8, lo);
+          for (int i = 0; i < 8; ++i) {
+            const int col = c * 16 + 2 * i;
+            float x, y;
+            unpack2(fma2(pack2(__uint_as_float(s[col]), __uint_as_float(s[col + 1])), sl2_2, neg_m), x, y);
+            x = ex2(x);
+            y = ex2(y);
+            const uint64_t p = pack2(x, y);
+            if (i & 1) sum1 = add2(sum1, p);
+            else sum0 = add2(sum0, p);
+            hi[i] = cvt2(x, y);
+            const uint64_t back = pack2(__uint_as_float(hi[i] << 16), __uint_as_float(hi[i] & 0xffff0000u));
+            unpack2(fma2(back, minus1, p), x, y);
+            lo[i] = cvt2(x, y);
           }
+          tmem_st_x8(s_t + c * 8, hi);
+          tmem_st_x8(s_t + 64 + c * 8, lo);
         }
         tmem_st_wait();
         tc_fence_before();
@@ -548,24 +569,40 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_const
   tc_fence_before();
   __syncthreads();
   // rows whose numbers may come from keys that they do not see (registers: only the softmax warps have enough)
-  if (*redo != 0 && *gave_up == 0 && warp < PT_WARP_COPY) sum_again(a);
+  if (*redo != 0 && *gave_up == 0 && warp < PT_WARP_COPY) sum_again<ACC>(a);
   // after a wait that ran out copies and MMAs of the other roles may be in flight; they are done long before this millisecond is over
   if (*gave_up)
     for (const long long t0 = clock64(); clock64() - t0 < 2000000ll;) {}
   __syncthreads();
   if (warp == PT_WARP_MMA) {
     tc_fence_after();
-    tmem_dealloc<512>(tmem_base);
+    tmem_dealloc<256 * ACC>(tmem_base);
   }
+}
+
+template <int ACC, int BLOCKS>
+cudaError_t launch(const CUtensorMap& qm, const CUtensorMap& vm, const PrefillArgs& a, int num_sms, cudaStream_t stream) {
+  static const cudaError_t attr = cudaFuncSetAttribute(attn_prefill_kernel<ACC, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PT_SMEM(ACC, BLOCKS));
+  if (attr != cudaSuccess) return attr;
+  return launch_k(attn_prefill_kernel<ACC, BLOCKS>, dim3(std::min(a.n_units, num_sms)), dim3(PT_THREADS(ACC)), PT_SMEM(ACC, ACC == 2 ? BLOCKS : a.blocks), stream,
+                  qm, vm, a);
 }
 
 int accumulator_tokens(int G) { return std::max(128 / G & ~7, 8); }
 
 }  // namespace
 
-// Units of the prompts and portions among `seqs` (q_len > 1), those with the most cache tiles first (ties in order).
-int prefill_units_build(PrefillUnit* units, const AttnSeq* seqs, int n_seqs, int G) {
-  const int step = 2 * accumulator_tokens(G);
+// Units of the prompts and portions among `seqs` (q_len > 1), those with the most cache tiles first (ties in order).  Where no sequence
+// has more than one tile of keys and the SMs take all units at once, a unit is one accumulator's rows and the launch the small one:
+// *short_blocks is then the number of cache blocks of the longest sequence, else 0.
+int prefill_units_build(PrefillUnit* units, const AttnSeq* seqs, int n_seqs, int G, int n_kv, int num_sms, int* short_blocks) {
+  const int rows = accumulator_tokens(G);
+  int keys = 0;
+  long long pieces = 0;
+  for (int s = 0; s < n_seqs; ++s)
+    if (seqs[s].q_len > 1) keys = std::max(keys, seqs[s].kv_len), pieces += (seqs[s].q_len + rows - 1) / rows;
+  *short_blocks = keys <= PT_KV && pieces * n_kv <= num_sms ? (keys + KV_BLOCK - 1) / KV_BLOCK : 0;
+  const int step = *short_blocks > 0 ? rows : 2 * rows;
   int n = 0;
   for (int s = 0; s < n_seqs; ++s) {
     const AttnSeq& q = seqs[s];
@@ -580,14 +617,12 @@ int prefill_units_build(PrefillUnit* units, const AttnSeq* seqs, int n_seqs, int
 }
 
 cudaError_t attn_prefill_launch(const __nv_bfloat16* qkv, int qkv_ld, const __nv_bfloat16* k_cache, const __nv_bfloat16* v_cache, int n_blocks,
-                                const PrefillUnit* units, int n_units, const int32_t* block_table, int bt_stride, __nv_bfloat16* out, int out_ld, int T, int n_q, int n_kv,
-                                float scale, int num_sms, cudaStream_t stream) {
+                                const PrefillUnit* units, int n_units, int short_blocks, const int32_t* block_table, int bt_stride,
+                                __nv_bfloat16* out, int out_ld, int T, int n_q, int n_kv, float scale, int num_sms, cudaStream_t stream) {
   if (n_units <= 0) return cudaSuccess;
   if (n_kv <= 0 || n_q % n_kv != 0) return cudaErrorInvalidValue;
   const int G = n_q / n_kv;
   if (G > 8) return cudaErrorInvalidValue;
-  static const cudaError_t attr = cudaFuncSetAttribute(attn_prefill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PT_SMEM);
-  if (attr != cudaSuccess) return attr;
   PrefillArgs a{};
   cudaError_t e = gemm_pair_word(&a.err);
   if (e != cudaSuccess) return e;
@@ -602,7 +637,9 @@ cudaError_t attn_prefill_launch(const __nv_bfloat16* qkv, int qkv_ld, const __nv
                         {64, (uint32_t)G, (uint32_t)a.TM}, true) != 0 ||
       make_tmap_bf16_3d(&vm, v_cache, {64, (uint64_t)n_blocks * n_kv * KV_BLOCK, 2}, {HEAD_DIM * 2ull, 128}, {64, KV_BLOCK, 2}, false) != 0)
     return cudaErrorInvalidValue;
-  return launch_k(attn_prefill_kernel, dim3(std::min(a.n_units, num_sms)), dim3(PT_THREADS), PT_SMEM, stream, qm, vm, a);
+  a.blocks = short_blocks;
+  if (short_blocks == 1) return launch<1, 1>(qm, vm, a, num_sms, stream);
+  return short_blocks > 0 ? launch<1, PT_BLOCKS>(qm, vm, a, num_sms, stream) : launch<2, PT_BLOCKS>(qm, vm, a, num_sms, stream);
 }
 
 }  // namespace tgis

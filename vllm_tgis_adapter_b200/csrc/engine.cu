@@ -165,7 +165,7 @@ struct StepHeader {
   int32_t kind;          // 0: engine step; 1: prompt-logprob pass over R rows of the step just executed (T = its tokens,
   int32_t need_norm;     //    need_norm: the final RMSNorm has not run yet)
   int32_t lg_idx;        // index of this plan's logits gather inside the step (epoch = staged base + lg_idx)
-  int32_t pad;
+  int32_t short_blocks;  // of the prompts' attention (prefill_units_build)
 };
 struct ShmCtl {
   std::atomic<uint64_t> seq;
@@ -3339,7 +3339,7 @@ struct tgis_engine {
         n_launches += (max_splits > 1 && !attn_inkernel_merge) ? 2 : 1;
       }
       if (n_tiles > 0) {
-        CK(attn_prefill_launch(qkv.p, qkv_dim, kc, vc, num_blocks, ds<PrefillUnit>(off_units), n_tiles,
+        CK(attn_prefill_launch(qkv.p, qkv_dim, kc, vc, num_blocks, ds<PrefillUnit>(off_units), n_tiles, step_short_blocks,
                                d_bt, bt_stride, attn_out.p, q_dim, T, nq, nkv, scale, num_sms, stream));
         ++n_launches;
       }
@@ -3430,7 +3430,7 @@ struct tgis_engine {
         n_launches += (max_splits > 1 && !attn_inkernel_merge) ? 2 : 1;
       }
       if (n_tiles > 0) {
-        CK(attn_prefill_launch(qkv.p, qkv_dim, kc, vc, num_blocks, ds<PrefillUnit>(off_units), n_tiles,
+        CK(attn_prefill_launch(qkv.p, qkv_dim, kc, vc, num_blocks, ds<PrefillUnit>(off_units), n_tiles, step_short_blocks,
                                d_bt, bt_stride, attn_out.p, q_dim, T, nq, nkv, attn_scale, num_sms, stream));
         ++n_launches;
       }
@@ -3553,11 +3553,13 @@ struct tgis_engine {
   // graph per (batch size, KV splits), captured on first use; every per-step quantity is read from the staged device
   // buffer, so the captured launch sequence is step-independent -- or the plain launch sequence otherwise.  Rank 0
   // and the tensor-parallel workers run the same function on the same header.
+  int step_short_blocks = 0;
   void exec_step(const StepHeader& h) {
     if (h.kind == 1) {
       plp_pass(h.R, h.need_norm, h.T, h.copy_bytes, h.lg_idx);
       return;
     }
+    step_short_blocks = h.short_blocks;
     if (!h.graphable) {
       launch_step(h.copy_bytes, h.T, h.n_dec, h.n_tiles, h.R, h.max_dec_kv, h.S, h.samp_complex);
       return;
@@ -3615,7 +3617,7 @@ struct tgis_engine {
   int run_batch(std::vector<Sched>& batch, const Results& results) {
     const tgis_config& c = cfg;
     const int H = c.hidden, V = c.vocab;
-    int T = 0, n_dec = 0, n_tiles = 0, R = 0, max_dec_kv = 0, samp_complex = 0;
+    int T = 0, n_dec = 0, n_tiles = 0, R = 0, max_dec_kv = 0, samp_complex = 0, short_blocks = 0;
     struct PromptRow {
       int row, target, pos;
       Request* r;
@@ -3745,12 +3747,13 @@ struct tgis_engine {
     // (S, max_splits) so that its size is a function of the CUDA-graph key
     const int max_splits_step = (max_dec_kv + DECODE_SPLIT - 1) / DECODE_SPLIT;
     decode_items_build(hs<DecItem>(items_off(S)), seqs, decids, n_dec, bt, bt_stride);
-    if (n_dec < S) n_tiles = prefill_units_build(hs<PrefillUnit>(off_units), seqs, S, pnx_on ? 1 : nq / nkv);
+    if (n_dec < S)
+      n_tiles = prefill_units_build(hs<PrefillUnit>(off_units), seqs, S, pnx_on ? 1 : nq / nkv, pnx_on ? 1 : nkv, num_sms, &short_blocks);
     const size_t copy_bytes = items_off(S) + sizeof(DecItem) * (1 + (size_t)n_dec * max_splits_step);
     const double t_ev0 = debug_launch ? now_s() : 0.0;
     CK(cudaEventRecord(ev0, stream));
     const bool graphable = cfg.use_cuda_graphs && (tp == 1 || tp_graphs) && !profiling && n_tiles == 0 && n_dec == S && R == S;
-    StepHeader hdr{T, n_dec, n_tiles, R, max_dec_kv, S, graphable ? 1 : 0, samp_complex, (uint64_t)copy_bytes, 0, 0, 1, 0};
+    StepHeader hdr{T, n_dec, n_tiles, R, max_dec_kv, S, graphable ? 1 : 0, samp_complex, (uint64_t)copy_bytes, 0, 0, 1, short_blocks};
     if (tp > 1) {
       // exchange epochs of this step = staged base + index inside the step (ar_add_rmsnorm_kernel)
       uint32_t* eb = hs<uint32_t>(off_epoch);

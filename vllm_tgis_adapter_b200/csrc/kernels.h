@@ -308,11 +308,12 @@ struct PrefillUnit {  // up to 2 * 128 / G query tokens of one sequence, read as
   int32_t pos0;        // position of the first one
   int32_t block_row;   // row in the block table
 };
-// The units of a step; every prompt is cut into pieces of at least 16 tokens (but for its last).  Returns their number.
-int prefill_units_build(PrefillUnit* units, const AttnSeq* seqs, int n_seqs, int G);
+// The units of a step; every prompt is cut into pieces of at least 16 tokens (but for its last).  Returns their number;
+// *short_blocks: for the launch (0, or the blocks of the longest sequence of a step of few short prompts; the bits are the same).
+int prefill_units_build(PrefillUnit* units, const AttnSeq* seqs, int n_seqs, int G, int n_kv, int num_sms, int* short_blocks);
 // n_blocks: blocks of the caches; T: rows of qkv
 cudaError_t attn_prefill_launch(const __nv_bfloat16* qkv, int qkv_ld, const __nv_bfloat16* k_cache, const __nv_bfloat16* v_cache, int n_blocks,
-                                const PrefillUnit* units, int n_units, const int32_t* block_table, int bt_stride,
+                                const PrefillUnit* units, int n_units, int short_blocks, const int32_t* block_table, int bt_stride,
                                 __nv_bfloat16* out, int out_ld, int T, int n_q, int n_kv,
                                 float scale, int num_sms, cudaStream_t stream);
 

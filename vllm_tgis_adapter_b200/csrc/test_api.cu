@@ -301,7 +301,8 @@ int tgis_k_attention(const void* qkv_dev, const void* k_cache_dev, const void* v
   int n_blocks = 1;
   for (int i = 0; i < bt_rows * bt_stride; ++i) n_blocks = std::max(n_blocks, block_table_host[i] + 1);
   std::vector<PrefillUnit> units(T / 16 + n_seqs + 1);
-  const int n_units = prefill_units_build(units.data(), seqs.data(), n_seqs, G);
+  int short_blocks = 0;
+  const int n_units = prefill_units_build(units.data(), seqs.data(), n_seqs, G, n_kv, test_num_sms(), &short_blocks);
   Tmp<AttnSeq> d_seqs;
   Tmp<PrefillUnit> d_units;
   Tmp<int32_t> d_dec, d_bt;
@@ -325,7 +326,7 @@ int tgis_k_attention(const void* qkv_dev, const void* k_cache_dev, const void* v
                          (int)dec.size() * max_splits, d_seqs.p, d_dec.p, (int)dec.size(), max_splits, po.p, pml.p,
                          (bf16*)out_dev, out_ld, n_q, n_kv, scale, test_num_sms(), 0, arrive.p));
   KCK(attn_prefill_launch((const bf16*)qkv_dev, qkv_ld, (const bf16*)k_cache_dev, (const bf16*)v_cache_dev, n_blocks,
-                          d_units.p, n_units, d_bt.p, bt_stride, (bf16*)out_dev, out_ld, T, n_q, n_kv, scale,
+                          d_units.p, n_units, short_blocks, d_bt.p, bt_stride, (bf16*)out_dev, out_ld, T, n_q, n_kv, scale,
                           test_num_sms(), 0));
   return product_end();
 }
