@@ -20,9 +20,9 @@
 // finite: the tensor cores add 0 * V.  A row that comes out with such numbers although its own scores are finite is summed again over
 // its own keys alone (sum_again), without the matrix instructions: its bits are then those of another order, and its numbers right.
 //
-// What bounds it: the tensor pipe, 3 x 128 x 128 x 128 multiply-adds a tile (S once, P V twice) -- two thirds busy on an SM that has
-// work, the rest goes to the way S -> softmax -> P V of one accumulator where it is longer than the other's products -- and whole
-// units: 2048 tokens are 256 of them, so some SMs work twice and some once.  Microseconds a launch on one B200, 32 query
+// What bounds it: the tensor pipe, 3 x 128 x 128 x 128 multiply-adds a tile (S once, P V twice) -- 56 % active on an SM that has work
+// (1859 tokens behind 6144), the rest goes to the way S -> softmax -> P V of one accumulator where it is longer than the other's
+// products -- and whole units: 2048 tokens are 256 of them, so some SMs work twice and some once.  Microseconds a launch on one B200, 32 query
 // and 8 kv heads, against the mma.sync kernel that went before (16 tokens x one head a warp, 32-token blocks, its pipe 56 %
 // active): 1859 tokens behind 6144: 1289 -> 345 (620 TFLOP/s, counting P V once); 2048 alone 243 -> 61; 2048 in 6 prompts 71 -> 30;
 // 32 prompts of 64 tokens 21.7 -> 16.1; 96 of 9 to 56 33.3 -> 29.3.  No faster: two threads per row (345 -> 356, short prompts
