@@ -155,3 +155,13 @@ def test_a_value_that_is_not_finite_in_a_short_prompt(g):
     sees[40:, :4, 9] = True
     bound = 1.001 * 2 ** -8 * want.abs() + 5 * (2 ** -16 + 100 * 2 ** -19)   # as above
     assert not bool(got[sees].isfinite().any()) and float(((got - want).abs() - bound)[~sees].max()) <= 0.0
+
+
+def test_sums_that_overflow_before_they_are_divided(g):
+    """Values near the largest of their type: a row's sum in front of the division may pass it, its result does not."""
+    case = Case(g, 8, 2, [200], seed=4)
+    case.v = (case.v.sign() * 3e38 * torch.rand(case.v.shape, device="cuda").clamp(min=0.5)).bfloat16()
+    case.vc = g.v_cache_from_dense(case.v, case.bt.shape[1])
+    want, got = case.exact(0, 0, 200), case.run([(0, 0, 200)])[0].double()
+    assert bool(got.isfinite().all())
+    assert float(((got - want).abs() - 1.001 * 2 ** -8 * want.abs()).max()) <= 3e38 * (2 ** -16 + 100 * 2 ** -19)

@@ -192,7 +192,8 @@ struct UnitIter {
 __device__ __forceinline__ const __nv_bfloat16* value_of(const __nv_bfloat16* block, int token, int lane) {
   return block + token * HEAD_DIM + ((lane >> 1) ^ (token & 7)) * 8 + (lane & 1) * 4;
 }
-// One row by a warp, the two passes of a softmax in the order of the keys: lane = token for the scores, lane = four dims for the values.
+// One row by a warp, in the order of the keys: lane = token for the scores (twice), lane = four dims for the values, whose weights sum to
+// one, so that no sum passes the largest value.
 __device__ __forceinline__ void attend_row(const PrefillArgs& a, int block_row, int kvh, int head, int row, int pos) {
   const int lane = (int)lane_id();
   const float sl2 = a.minus != 0 ? -a.sl2 : a.sl2;
@@ -216,13 +217,21 @@ __device__ __forceinline__ void attend_row(const PrefillArgs& a, int block_row, 
   };
   float m = -INFINITY, l = 0.f, o[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-  for (int b = 0; b <= pos / KV_BLOCK; ++b) m = fmaxf(m, score(b));
+  for (int b = 0; b <= pos / KV_BLOCK; ++b) {   // maximum and sum of the lane's tokens
+    const float x = score(b), top = fmaxf(m, x);
+    if (top > -INFINITY) l = l * ex2(m - top) + ex2(x - top);
+    m = top;
+  }
+  float ref = m;
 #pragma unroll
-  for (int i = 16; i > 0; i >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, i));
+  for (int i = 16; i > 0; i >>= 1) ref = fmaxf(ref, __shfl_xor_sync(0xffffffffu, ref, i));
+  l *= ex2(m - ref);
+#pragma unroll
+  for (int i = 16; i > 0; i >>= 1) l += __shfl_xor_sync(0xffffffffu, l, i);
+  const float inv = 1.f / l;
 #pragma unroll 1
   for (int b = 0; b <= pos / KV_BLOCK; ++b) {
-    const float p = ex2(score(b) - m);
-    l += p;
+    const float p = ex2(score(b) - ref) * inv;
     const int n = min(KV_BLOCK, pos - b * KV_BLOCK + 1);   // (hidden keys are not touched)
 #pragma unroll 4
     for (int t = 0; t < n; ++t) {
@@ -232,15 +241,12 @@ __device__ __forceinline__ void attend_row(const PrefillArgs& a, int block_row, 
       o[2] = fmaf(w, lo(v.y), o[2]); o[3] = fmaf(w, hi(v.y), o[3]);
     }
   }
-#pragma unroll
-  for (int i = 16; i > 0; i >>= 1) l += __shfl_xor_sync(0xffffffffu, l, i);
-  const float inv = 1.f / l;
-  *reinterpret_cast<uint2*>(a.out + (size_t)row * a.out_ld + (size_t)head * HEAD_DIM + lane * 4) =
-      make_uint2(cvt2(o[0] * inv, o[1] * inv), cvt2(o[2] * inv, o[3] * inv));
+  *reinterpret_cast<uint2*>(a.out + (size_t)row * a.out_ld + (size_t)head * HEAD_DIM + lane * 4) = make_uint2(cvt2(o[0], o[1]), cvt2(o[2], o[3]));
 }
 
-// The CTA's rows that came out with numbers that are not finite, by its softmax warps, which have stored them all.  Where the value of
-// a row's own token accounts for them (a token that has overflowed in full, and all that follow it in the next layers) they stand.
+// The CTA's rows that came out with numbers that are not finite, by its softmax warps, which have stored them all.  Where a key that the
+// row sees accounts for them they stand: a unit's values are looked through once for the first such key of every dim, so that a
+// sequence which has overflowed costs no more than that (a row summed again reads all of its keys twice, 32 loads in flight at most).
 template <int ACC>
 __device__ __noinline__ void sum_again(const PrefillArgs& a) {
   const int lane = (int)lane_id();
@@ -249,15 +255,35 @@ __device__ __noinline__ void sum_again(const PrefillArgs& a) {
     return ((w.x & e) == e) | ((w.x >> 16 & e) == e) << 1 | ((w.y & e) == e) << 2 | ((w.y >> 16 & e) == e) << 3;
   };
   Unit u;
-  for (UnitIter it(a); it.next(u);)
+  for (UnitIter it(a); it.next(u);) {
+    int first[4] = {-1, -1, -1, -1};   // of the lane's dims: the first key whose value is not finite (none: behind the last key)
     for (int r = threadIdx.x >> 5; r < u.rows * a.G; r += 4 * ACC) {
       const int t = r / a.G, row = u.row0 + t, head = u.kvh * a.G + r - t * a.G, pos = u.pos0 + t;
       const int mine = odd(*reinterpret_cast<const uint2*>(a.out + (size_t)row * a.out_ld + (size_t)head * HEAD_DIM + lane * 4));
       if (!__any_sync(0xffffffffu, mine != 0)) continue;
-      const int block = a.block_table[(size_t)u.block_row * a.bt_stride + pos / KV_BLOCK], slot = pos % KV_BLOCK;
-      const int own = odd(*reinterpret_cast<const uint2*>(value_of(a.v_cache + ((size_t)block * a.n_kv + u.kvh) * (KV_BLOCK * HEAD_DIM), slot, lane)));
-      if (__any_sync(0xffffffffu, (mine & ~own) != 0)) attend_row(a, u.block_row, u.kvh, head, row, pos);
+      if (first[0] < 0) {
+        int seen = 0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) first[e] = u.n_blk * KV_BLOCK;
+        for (int b = 0; b < u.n_blk && !__all_sync(0xffffffffu, seen == 15); ++b) {
+          const int block = a.block_table[(size_t)u.block_row * a.bt_stride + b];
+          const __nv_bfloat16* from = a.v_cache + ((size_t)block * a.n_kv + u.kvh) * (KV_BLOCK * HEAD_DIM);
+#pragma unroll 4
+          for (int k = 0; k < KV_BLOCK; ++k) {
+            const int now = odd(*reinterpret_cast<const uint2*>(value_of(from, k, lane))) & ~seen;
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (now >> e & 1) first[e] = b * KV_BLOCK + k;
+            seen |= now;
+          }
+        }
+      }
+      int hidden = 0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) hidden |= (first[e] > pos) << e;
+      if (__any_sync(0xffffffffu, (mine & hidden) != 0)) attend_row(a, u.block_row, u.kvh, head, row, pos);
     }
+  }
 }
 
 template <int ACC, int BLOCKS>
