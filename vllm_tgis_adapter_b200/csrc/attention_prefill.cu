@@ -17,8 +17,8 @@
 // lost below it); a warp scales its part of O only then (the conditional rescaling published with FlashAttention-4).  A row's bits
 // depend on its own keys alone: tiles are counted from the sequence's first token, and what another row or request does changes
 // neither order nor reference of its sums.  The one thing that reaches a row from a key it does not see is a value that is not
-// finite: the tensor cores add 0 * V.  A row that comes out with such numbers although its own scores are finite is summed again over
-// its own keys alone (sum_again), without the matrix instructions: its bits are then those of another order, and its numbers right.
+// finite: the tensor cores add 0 * V.  A row that comes out with such numbers although no key that it sees has them is summed again
+// over its own keys alone (sum_again), without the matrix instructions: its bits are then those of another order, and its numbers right.
 //
 // What bounds it: the tensor pipe, 3 x 128 x 128 x 128 multiply-adds a tile (S once, P V twice) -- 56 % active on an SM that has work
 // (1859 tokens behind 6144), the rest goes to the way S -> softmax -> P V of one accumulator where it is longer than the other's
