@@ -200,8 +200,24 @@ short_conv_run_kernel(const float* __restrict__ xz, int ld, int inner, const flo
   }
 }
 
+// The sequence of rank `rank` by length, longest first (ties in order), where the block has a thread for every one; else number `rank`.
+// (seqs is written by the host before the step.)
+__device__ __forceinline__ int longest_first(const AttnSeq* __restrict__ seqs, int n_seqs, int rank, int* lens, int* pick) {
+  if (n_seqs <= 1 || n_seqs > (int)blockDim.x) return rank;
+  const int tid = threadIdx.x;
+  if (tid < n_seqs) lens[tid] = seqs[tid].q_len;
+  __syncthreads();
+  if (tid < n_seqs) {
+    int before = 0;
+    for (int j = 0; j < n_seqs; ++j) before += lens[j] > lens[tid] || (lens[j] == lens[tid] && j < tid);
+    if (before == rank) *pick = tid;
+  }
+  __syncthreads();
+  return *pick;
+}
+
 // ------------------------------------------------------------------------------------------------ selective scan
-constexpr int SCAN_THREADS = 64, SCAN_CHUNK = 8, SCAN_REG_STATE = 16, SCAN_LPC = 4, SCAN_RPL = SCAN_REG_STATE / SCAN_LPC;
+constexpr int SCAN_THREADS = 64, SCAN_CHUNK = 8, SCAN_REG_CHUNK = 16, SCAN_REG_STATE = 16, SCAN_LPC = 4, SCAN_RPL = SCAN_REG_STATE / SCAN_LPC;
 // the convolution's tail: inputs of the last taps - 1 positions (entry e: position end - (taps - 1) + e)
 __device__ __forceinline__ void scan_save_conv(const SelScan& a, const AttnSeq& sq, int slot, int c) {
   const int K1 = a.taps - 1, first = sq.kv_len - sq.q_len;
@@ -214,23 +230,30 @@ __device__ __forceinline__ void scan_save_conv(const SelScan& a, const AttnSeq& 
     cs[(size_t)e * a.inner] = v;
   }
 }
-// Up to SCAN_REG_STATE states: grid (sequences, ceil(inner / 16)), SCAN_LPC lanes share a channel; lane `sub` keeps states
+// Up to SCAN_REG_STATE states: grid (sequences * ceil(inner / 16)), SCAN_LPC lanes share a channel; lane `sub` keeps states
 // 4 sub .. + 3 and their decay rates in registers.  A channel's tokens follow one another, so what is bound is the number of
-// instructions a token takes.  What the four lanes would all do is dealt out: of a chunk's eight tokens a lane fetches two (step
-// size, input, gate), takes their softplus, hands step size and input on by shuffle, and after the chunk receives the two tokens'
-// output sums (a transposing reduction: 6 shuffles for 8 tokens and 4 lanes) and gates and writes them.  B and C rows go through two
-// shared-memory buffers, read four states to a load; the next chunk is fetched while this one is worked through.  2048 tokens in 7 prompts, 4096 channels of 16
-// states: 747 -> 338 us.
+// instructions a token takes, and where few channels are left their latency.  What the four lanes would all do is dealt out: of a chunk's
+// sixteen tokens a lane fetches four (step size, input, gate), takes their softplus, hands step size and input on by shuffle, and after the
+// chunk receives the four tokens' output sums (a transposing reduction: 12 shuffles for 16 tokens and 4 lanes) and gates and writes
+// them.  B and C rows go through two shared-memory buffers, read four states to a load; the next chunk's step sizes are worked out
+// beside this chunk's outputs, its loads a chunk before.  Whole chunks of ALL = SCAN_REG_STATE states have no branch in them, so that the
+// tokens' exponentials run beside one another and only the fma of a state waits for the token before; a sequence's last chunk tests
+// its tokens one by one.  Longest sequences first.  4096 channels of 16 states, microseconds without overlap: 2048 tokens in 7 prompts 306 -> 163, 32 prompts of
+// 64 tokens 142 -> 127; with chunks of 8 tokens 206 and 122, of 32 188 and 191.
+template <bool ALL>
 __global__ void __launch_bounds__(SCAN_THREADS)
-selective_scan_reg_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t* __restrict__ tok_slot) {
-  constexpr int TPL = SCAN_CHUNK / SCAN_LPC, ROW = 2 * SCAN_REG_STATE, STAGE = SCAN_CHUNK * ROW / SCAN_THREADS;
-  static_assert(SCAN_LPC == 4 && SCAN_RPL == 4 && TPL == 2, "the reduction below deals eight tokens to four lanes");
-  __shared__ __align__(16) float BC[2][SCAN_CHUNK * ROW];   // per token: B | C, zeros behind the last state
+selective_scan_reg_kernel(SelScan a, const AttnSeq* __restrict__ seqs, int n_seqs, const int32_t* __restrict__ tok_slot) {
+  constexpr int CHUNK = SCAN_REG_CHUNK, TPL = CHUNK / SCAN_LPC, ROW = 2 * SCAN_REG_STATE, STAGE = CHUNK * ROW / SCAN_THREADS;
+  static_assert(SCAN_LPC == 4 && SCAN_RPL == 4, "the reduction below deals a chunk's tokens to four lanes");
+  __shared__ __align__(16) float BC[2][CHUNK * ROW];   // per token: B | C, zeros behind the last state
+  __shared__ int lens[SCAN_THREADS], pick;
   griddep_launch();
+  constexpr int CH = SCAN_THREADS / SCAN_LPC;
+  const int n_blk = (a.inner + CH - 1) / CH, N = ALL ? SCAN_REG_STATE : a.state, tid = threadIdx.x, lane = tid & 31, sub = tid % SCAN_LPC;
+  const int seq = longest_first(seqs, n_seqs, blockIdx.x / n_blk, lens, &pick);
+  const AttnSeq sq = seqs[seq];
   griddep_wait();
-  const AttnSeq sq = seqs[blockIdx.x];
-  const int N = a.state, tid = threadIdx.x, lane = tid & 31, sub = tid % SCAN_LPC;
-  const int c = blockIdx.y * (SCAN_THREADS / SCAN_LPC) + tid / SCAN_LPC;
+  const int c = blockIdx.x % n_blk * CH + tid / SCAN_LPC;
   const bool live = c < a.inner;
   const int slot = tok_slot[sq.q_start];
   float* Sg = a.S + ((size_t)slot * a.inner + (live ? c : 0)) * N;
@@ -244,7 +267,7 @@ selective_scan_reg_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int
   const float dtb = live ? a.dt_b[c] : 0.f, Dc = live ? a.D[c] : 0.f;
   float p_bc[STAGE], p_dt[TPL], p_x[TPL], p_z[TPL];
   auto fetch = [&](int t0) {
-    const int nt = min(SCAN_CHUNK, sq.q_len - t0);
+    const int nt = min(CHUNK, sq.q_len - t0);
 #pragma unroll
     for (int k = 0; k < STAGE; ++k) {
       const int e = tid + k * SCAN_THREADS, tt = e / ROW, which = (e % ROW) / SCAN_REG_STATE, n = e % SCAN_REG_STATE;
@@ -259,10 +282,8 @@ selective_scan_reg_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int
       p_z[i] = ok ? a.xz[row * a.ld_xz + a.inner + c] : 0.f;
     }
   };
-  fetch(0);
-  for (int t0 = 0, buf = 0; t0 < sq.q_len; t0 += SCAN_CHUNK, buf ^= 1) {
-    const int nt = min(SCAN_CHUNK, sq.q_len - t0);
-    float dt[TPL], dx[TPL], xv[TPL], zv[TPL], y[SCAN_CHUNK];
+  float dt[TPL], dx[TPL], xv[TPL], zv[TPL];
+  auto stage = [&](int buf) {   // what was fetched: B and C to a buffer, the tokens' step sizes
 #pragma unroll
     for (int k = 0; k < STAGE; ++k) BC[buf][tid + k * SCAN_THREADS] = p_bc[k];
 #pragma unroll
@@ -272,39 +293,57 @@ selective_scan_reg_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int
       zv[i] = p_z[i];
       dx[i] = dt[i] * xv[i];
     }
-    __syncthreads();   // (the buffer written two chunks from now is this one: everyone is through with it by the barrier between)
-    if (t0 + SCAN_CHUNK < sq.q_len) fetch(t0 + SCAN_CHUNK);
-#pragma unroll
-    for (int tt = 0; tt < SCAN_CHUNK; ++tt) {
+  };
+  fetch(0);
+  stage(0);
+  if (CHUNK < sq.q_len) fetch(CHUNK);
+  for (int t0 = 0, buf = 0; t0 < sq.q_len; t0 += CHUNK, buf ^= 1) {
+    const int nt = min(CHUNK, sq.q_len - t0);
+    __syncthreads();   // (the other buffer is written below: everyone read it before this barrier)
+    float y[CHUNK];
+    auto token = [&](int tt) {
+      const int from = (lane & ~(SCAN_LPC - 1)) + tt / TPL;
+      const float dt_t = __shfl_sync(0xffffffffu, dt[tt % TPL], from), dx_t = __shfl_sync(0xffffffffu, dx[tt % TPL], from);
+      const float4 b4 = *reinterpret_cast<const float4*>(&BC[buf][tt * ROW + sub * SCAN_RPL]);
+      const float4 c4 = *reinterpret_cast<const float4*>(&BC[buf][tt * ROW + SCAN_REG_STATE + sub * SCAN_RPL]);
+      const float bn[4] = {b4.x, b4.y, b4.z, b4.w}, cn[4] = {c4.x, c4.y, c4.z, c4.w};
       y[tt] = 0.f;
-      if (tt < nt) {
-        const int from = (lane & ~(SCAN_LPC - 1)) + tt / TPL;
-        const float dt_t = __shfl_sync(0xffffffffu, dt[tt % TPL], from), dx_t = __shfl_sync(0xffffffffu, dx[tt % TPL], from);
-        const float4 b4 = *reinterpret_cast<const float4*>(&BC[buf][tt * ROW + sub * SCAN_RPL]);
-        const float4 c4 = *reinterpret_cast<const float4*>(&BC[buf][tt * ROW + SCAN_REG_STATE + sub * SCAN_RPL]);
-        const float bn[4] = {b4.x, b4.y, b4.z, b4.w}, cn[4] = {c4.x, c4.y, c4.z, c4.w};
 #pragma unroll
-        for (int j = 0; j < SCAN_RPL; ++j) {
-          if (sub * SCAN_RPL + j < N) {
-            Sr[j] = fmaf(expf(dt_t * Ar[j]), Sr[j], dx_t * bn[j]);
-            y[tt] = fmaf(Sr[j], cn[j], y[tt]);
-          }
+      for (int j = 0; j < SCAN_RPL; ++j) {
+        if (ALL || sub * SCAN_RPL + j < N) {
+          Sr[j] = fmaf(expf(dt_t * Ar[j]), Sr[j], dx_t * bn[j]);
+          y[tt] = fmaf(Sr[j], cn[j], y[tt]);
         }
       }
-    }
-    float half[4];
+    };
+    if (nt == CHUNK) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float keep = sub & 2 ? y[4 + i] : y[i], give = sub & 2 ? y[i] : y[4 + i];
+      for (int tt = 0; tt < CHUNK; ++tt) token(tt);
+    } else {
+#pragma unroll
+      for (int tt = 0; tt < CHUNK; ++tt) {
+        y[tt] = 0.f;
+        if (tt < nt) token(tt);
+      }
+    }
+    float half[2 * TPL], out[TPL];
+#pragma unroll
+    for (int i = 0; i < 2 * TPL; ++i) {
+      const float keep = sub & 2 ? y[2 * TPL + i] : y[i], give = sub & 2 ? y[i] : y[2 * TPL + i];
       half[i] = keep + __shfl_xor_sync(0xffffffffu, give, 2);
     }
 #pragma unroll
     for (int i = 0; i < TPL; ++i) {
-      const float keep = sub & 1 ? half[2 + i] : half[i], give = sub & 1 ? half[i] : half[2 + i];
-      const float sum = keep + __shfl_xor_sync(0xffffffffu, give, 1);
-      if (live && sub * TPL + i < nt)
-        st_op(a.out, a.out_dtype, (size_t)(sq.q_start + t0 + sub * TPL + i) * a.inner + c, fmaf(Dc, xv[i], sum) * silu_f(zv[i]));
+      const float keep = sub & 1 ? half[TPL + i] : half[i], give = sub & 1 ? half[i] : half[TPL + i];
+      out[i] = fmaf(Dc, xv[i], keep + __shfl_xor_sync(0xffffffffu, give, 1)) * silu_f(zv[i]);
     }
+    if (t0 + CHUNK < sq.q_len) {
+      stage(buf ^ 1);
+      if (t0 + 2 * CHUNK < sq.q_len) fetch(t0 + 2 * CHUNK);
+    }
+#pragma unroll
+    for (int i = 0; i < TPL; ++i)
+      if (live && sub * TPL + i < nt) st_op(a.out, a.out_dtype, (size_t)(sq.q_start + t0 + sub * TPL + i) * a.inner + c, out[i]);
   }
   if (!live) return;
 #pragma unroll
@@ -436,9 +475,8 @@ selective_scan_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t
 // tokens w, w + 8.  What is the same for all columns is not done once per thread: the gated memory's exponentials are one warp's work
 // before the token loop, and its normaliser is kept a row per thread.
 // Bound by instruction issue and by the latency of a token's chain (one head's tokens are worked through one after the other, and a
-// prompt has only heads * vdim / 32 blocks).  Four rows to a shared-memory load and two to an fma.  2048 tokens in 7 prompts: gated,
-// 8 heads of 128 x 256, 636 -> 346 us (507 while the token loop still tested every group of rows: hence FULL); decayed, 32 heads of
-// 64 x 64, 342 -> 255 us; a step of 32 single tokens, gated, 42 -> 30 us.  One 1024-token prompt takes 0.24 us a token.
+// prompt has only heads * vdim / 32 blocks).  Four rows to a shared-memory load and two to an fma.  This is the kernel of keys that leave
+// the last row group short, and of rows that 16-byte loads cannot reach; the others' prompts have outer_run_kernel.
 __device__ __forceinline__ unsigned long long pack2(float x, float y) {
   unsigned long long d;
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
@@ -460,12 +498,11 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long x, unsigne
   return d;
 }
 constexpr int OS_GROUPS = 8, OS_COLS = 32, OS_THREADS = OS_GROUPS * OS_COLS, OS_CHUNK = 16;
-// FULL: D == RPT * OS_GROUPS, every thread's rows are there (no branch in the token loop, so a token's loads go ahead of its sums).
-template <int RPT, int MODE, bool FULL>
+template <int RPT, int MODE>
 __global__ void __launch_bounds__(OS_THREADS)
 outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* __restrict__ tok_slot) {
   extern __shared__ __align__(16) float os_smem[];
-  const int D = FULL ? RPT * OS_GROUPS : a.dim, DP = (D + 3) & ~3;
+  const int D = a.dim, DP = (D + 3) & ~3;
   float* vec = os_smem;                                  // [OS_CHUNK][3][DP]: q | k | w (GATED: n q)
   float* vcol = vec + (size_t)OS_CHUNK * 3 * DP;         // [OS_CHUNK][OS_COLS]
   __shared__ float part[OS_CHUNK][OS_GROUPS][OS_COLS + 1];
@@ -633,7 +670,7 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
 #pragma unroll
       for (int j = 0; j < NG; ++j) {
         const int i = 4 * (g + j * OS_GROUPS);
-        if (FULL || i + 4 <= D) {
+        if (i + 4 <= D) {
           const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(v3 + i), k4 = *reinterpret_cast<const ulonglong2*>(v3 + DP + i);
           ulonglong2 w4 = make_ulonglong2(wd2, wd2);
           if (OWN_DECAY) w4 = *reinterpret_cast<const ulonglong2*>(v3 + 2 * DP + i);
@@ -701,6 +738,366 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
       const float* src = a.x + (size_t)(sq.q_start + sq.q_len - 1) * a.width;
       for (int i = tid; i < a.width; i += OS_THREADS) a.x_last[(size_t)slot * a.width + i] = src[i];
     }
+  }
+}
+
+// Portions of several tokens whose keys fill the row groups (dim = 8 RPT): the sums of the kernel above in the same order, bit for bit.
+// There a thread has one column, so that two 16-byte loads feed six packed operations, and everyone waits at a chunk's barriers while a
+// few lanes take exponentials.  Here a row thread has two neighbouring columns of its group's rows, and what is not the recurrence is
+// others' work: four warps fetch and stage the tokens' vectors, four rows to an instruction (the first of them also runs the gates, 32
+// tokens at a time and a block of them ahead), two sum and write the outputs.  Rows, writers and stagers hand a chunk's buffer round by
+// a named barrier each.  Longest sequences first: a piece's tokens follow one another, so the launch ends with the longest.
+// Bound by instruction issue, of which the rows' packed multiply-adds are a third.  2048 tokens in 7 prompts (838 the longest), microseconds
+// without overlap, before -> here: gated, 8 heads of 128 x 256, 302 -> 136; decayed, 32 heads of 64 x 64, 234 -> 106; 32 prompts of 64 tokens 137 ->
+// 119 and 92 -> 90.  Slower: four columns a thread or 64 a piece (gated 184 to 194), chunks of eight tokens in a ring of four (154), one helping
+// group for all of it (174), vectors staged number by number (155).
+template <int MODE>
+constexpr bool OS_OWN_DECAY = MODE == OUTER_SCAN_DECAY || MODE == OUTER_SCAN_HGRN || MODE == OUTER_SCAN_GLA;   // a decay per row
+template <int MODE>
+constexpr int OS_VECS = OS_OWN_DECAY<MODE> || MODE == OUTER_SCAN_GATED ? 3 : 2;   // q | k | w (GATED: n q)
+constexpr int RUN_CHUNK = 16, RUN_RING = 2;
+constexpr int RUN_ROWS = OS_THREADS / 2, RUN_STAGE = 128, RUN_WRITE = 64, RUN_THREADS = RUN_ROWS + RUN_STAGE + RUN_WRITE;
+template <int RPT, int MODE>
+constexpr size_t RUN_SMEM = (size_t)RUN_RING * RUN_CHUNK * (OS_VECS<MODE> * RPT * OS_GROUPS + (MODE == OUTER_SCAN_SSD ? 2 : 1) * OS_COLS + OS_GROUPS * OS_COLS) * sizeof(float);
+// barrier ID + i, i < RUN_RING (ids as constants: one in a register would reserve all sixteen)
+template <int ID>
+__device__ __forceinline__ void bar_sync_at(int i, int threads) {
+  if (i == 0) asm volatile("bar.sync %0, %1;\n" ::"n"(ID), "r"(threads) : "memory");
+  else asm volatile("bar.sync %0, %1;\n" ::"n"(ID + 1), "r"(threads) : "memory");
+}
+template <int ID>
+__device__ __forceinline__ void bar_arrive_at(int i, int threads) {
+  if (i == 0) asm volatile("bar.arrive %0, %1;\n" ::"n"(ID), "r"(threads) : "memory");
+  else asm volatile("bar.arrive %0, %1;\n" ::"n"(ID + 1), "r"(threads) : "memory");
+}
+
+template <int RPT, int MODE>
+__global__ void __launch_bounds__(RUN_THREADS, RPT <= 16 ? 2 : 1)
+outer_run_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, int n_seqs, const int32_t* __restrict__ tok_slot) {
+  constexpr int D = RPT * OS_GROUPS, NV = OS_VECS<MODE>, C = RUN_CHUNK, RING = RUN_RING, CT = 2, NG = RPT / 4, UNROLL = RPT <= 16 ? 2 : 1;
+  constexpr int FULL = 1, DONE = FULL + RUN_RING, EMPTY = DONE + RUN_RING, STAGED = EMPTY + RUN_RING;   // barriers: stagers -> rows -> writers -> stagers
+  static_assert(RING == 2 && 32 % C == 0, "barriers; blocks of gates");
+  constexpr bool GATES = MODE == OUTER_SCAN_GATED || MODE == OUTER_SCAN_SSD;
+  extern __shared__ __align__(16) float os_smem[];
+  float* vec = os_smem;                              // [RING][C][NV][D]
+  float* vcol = vec + RING * C * NV * D;         // [RING][C][OS_COLS], times the token's factor
+  float* part = vcol + RING * C * OS_COLS;       // [RING][C][OS_GROUPS][OS_COLS]
+  float* vraw = part + RING * C * OS_GROUPS * OS_COLS;   // SSD: [RING][C][OS_COLS]
+  __shared__ float gates[3][32][2], floor_m[3][32];  // as above, of three blocks of 32 tokens: one is made while chunks of the two before it are in the ring
+  __shared__ int lens[RUN_THREADS], pick, last_block;
+  griddep_launch();
+  const int tid = threadIdx.x, nz = (a.vdim + OS_COLS - 1) / OS_COLS, piece = blockIdx.x % (a.heads * nz);
+  const int seq = longest_first(seqs, n_seqs, blockIdx.x / (a.heads * nz), lens, &pick);
+  const AttnSeq sq = seqs[seq];
+  const int h = piece / nz, zb = piece % nz, c0 = zb * OS_COLS;
+  const int hq = a.qk_heads > 0 ? h / (a.heads / a.qk_heads) : h;   // the q / k head this head reads
+  const int n_chunks = (sq.q_len + C - 1) / C;
+  griddep_wait();
+  const int slot = tok_slot[sq.q_start];
+  const bool fresh = sq.kv_len - sq.q_len == 0;
+  auto block_of = [](int n) { return n * C / 32 % 3; };   // gates of chunk n: row block_of(n), from n * C % 32 on
+  constexpr int EPT = C * D / 4 / RUN_STAGE, TSTEP = RUN_STAGE * 4 / D, VPT = C * OS_COLS / RUN_STAGE, NR = (D + RUN_STAGE - 1) / RUN_STAGE;
+  const int ht = tid - RUN_ROWS, lane = tid & 31;
+  float n_row[NR], m_run = 0.f;                      // GATED, stagers: the normaliser's rows ht, ht + 128; the running maximum (first warp)
+#pragma unroll
+  for (int r = 0; r < NR; ++r) n_row[r] = 0.f;
+  if (tid < RUN_ROWS) {
+    // ===================== the recurrence: two columns of the rows 4 (g + 8 j) .. + 3 =====================
+    constexpr int LPG = OS_COLS / CT;                   // lanes of a row group
+    const int g = tid / LPG, c = c0 + (tid % LPG) * CT;
+    auto row_of = [&](int j) { return 4 * (g + (j >> 2) * OS_GROUPS) + (j & 3); };
+    float* Sg = a.S + (((size_t)slot * a.heads + h) * D) * a.vdim + c;
+    unsigned long long S[CT][2 * NG];
+#pragma unroll
+    for (int j = 0; j < RPT; j += 2)
+#pragma unroll
+      for (int e = 0; e < CT; ++e) {
+        const bool in = !fresh && c + e < a.vdim;
+        const float s0 = in ? Sg[(size_t)row_of(j) * a.vdim + e] : 0.f, s1 = in ? Sg[(size_t)row_of(j + 1) * a.vdim + e] : 0.f;
+        S[e][j / 2] = pack2(s0, s1);
+      }
+    unsigned long long u_r[2 * NG];                  // DECAY: the bonus u of this thread's rows
+    if (MODE == OUTER_SCAN_DECAY) {
+#pragma unroll
+      for (int j = 0; j < RPT; j += 2) u_r[j / 2] = pack2(a.u[(size_t)h * D + row_of(j)], a.u[(size_t)h * D + row_of(j) + 1]);
+    }
+    const float fixed_decay = (MODE == OUTER_SCAN_LIGHTNING || MODE == OUTER_SCAN_RETENTION) ? a.decay[h] : 0.f;
+    for (int n = 0; n < n_chunks; ++n) {
+      const int buf = n % RING;
+      const float* v3 = vec + (size_t)buf * C * NV * D + 4 * g;
+      const float* vc_from = vcol + buf * C * OS_COLS + (tid % LPG) * CT;
+      const float* gate = &gates[block_of(n)][n * C % 32][0];
+      float* to = part + ((size_t)buf * C * OS_GROUPS + g) * OS_COLS + (tid % LPG) * CT;
+      auto token = [&](int tt) {
+        unsigned long long vc2[CT], o01[CT], o23[CT];
+        const float2 vc = *reinterpret_cast<const float2*>(vc_from + tt * OS_COLS);
+        const float wd = GATES ? gate[2 * tt] : fixed_decay;
+        const unsigned long long wd2 = pack2(wd, wd);
+        vc2[0] = pack2(vc.x, vc.x);
+        vc2[1] = pack2(vc.y, vc.y);
+#pragma unroll
+        for (int e = 0; e < CT; ++e) o01[e] = 0, o23[e] = 0;   // packed zeros
+        auto step = [&](unsigned long long& s, unsigned long long& o, unsigned long long q2, unsigned long long k2, unsigned long long w2,
+                        unsigned long long u2, unsigned long long v2) {
+          const unsigned long long kv = mul2(k2, v2);
+          if (MODE == OUTER_SCAN_DECAY) {
+            o = fma2(q2, fma2(u2, kv, s), o);
+            s = fma2(w2, s, kv);
+          } else {
+            s = fma2(w2, s, kv);
+            o = fma2(q2, s, o);
+          }
+        };
+        const float* vt = v3 + tt * NV * D;
+#pragma unroll
+        for (int j = 0; j < NG; ++j) {
+          const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(vt + 4 * j * OS_GROUPS), k4 = *reinterpret_cast<const ulonglong2*>(vt + D + 4 * j * OS_GROUPS);
+          ulonglong2 w4 = make_ulonglong2(wd2, wd2);
+          if (OS_OWN_DECAY<MODE>) w4 = *reinterpret_cast<const ulonglong2*>(vt + 2 * D + 4 * j * OS_GROUPS);
+#pragma unroll
+          for (int e = 0; e < CT; ++e) {
+            step(S[e][2 * j], o01[e], q4.x, k4.x, w4.x, u_r[2 * j], vc2[e]);
+            step(S[e][2 * j + 1], o23[e], q4.y, k4.y, w4.y, u_r[2 * j + 1], vc2[e]);
+          }
+        }
+        float sum[CT];
+#pragma unroll
+        for (int e = 0; e < CT; ++e) {
+          const float2 oa = unpack2(o01[e]), ob = unpack2(o23[e]);
+          sum[e] = (oa.x + oa.y) + (ob.x + ob.y);
+        }
+        *reinterpret_cast<float2*>(to + tt * OS_GROUPS * OS_COLS) = make_float2(sum[0], sum[1]);
+      };
+      bar_sync_at<FULL>(buf, RUN_ROWS + RUN_STAGE);
+      const int nt = min(C, sq.q_len - n * C);
+      if (nt == C) {
+#pragma unroll UNROLL
+        for (int tt = 0; tt < C; ++tt) token(tt);
+      } else {
+#pragma unroll 1
+        for (int tt = 0; tt < nt; ++tt) token(tt);
+      }
+      bar_arrive_at<DONE>(buf, RUN_ROWS + RUN_WRITE);
+    }
+    // ---- leave the state behind the portion's last token
+#pragma unroll
+    for (int j = 0; j < RPT; j += 2)
+#pragma unroll
+      for (int e = 0; e < CT; ++e)
+        if (c + e < a.vdim) {
+          const float2 s = unpack2(S[e][j / 2]);
+          Sg[(size_t)row_of(j) * a.vdim + e] = s.x;
+          Sg[(size_t)row_of(j + 1) * a.vdim + e] = s.y;
+        }
+  } else if (ht < RUN_STAGE) {
+    // ===================== gates, vectors, normaliser =====================
+    const float ssd_rate = MODE == OUTER_SCAN_SSD ? -expf(a.A_log[h]) : 0.f;
+    // a thread stages rows row4 .. + 3 of the tokens tok, tok + TSTEP, ... of a chunk
+    const int row4 = ht * 4 % D, tok = ht * 4 / D;
+    float4 pq[EPT], pk[EPT], pd[EPT];
+    float pv[VPT], w0[4], low[4], pg0 = 0.f, pg1 = 0.f;   // (HGRN: low is the gate's lower bound)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      w0[k] = OS_OWN_DECAY<MODE> ? a.w0[(size_t)h * D + row4 + k] : 0.f;
+      low[k] = MODE == OUTER_SCAN_HGRN ? a.u[(size_t)h * D + row4 + k] : 0.f;
+    }
+    if (MODE == OUTER_SCAN_GATED && !fresh) {
+      m_run = a.m[(size_t)slot * a.heads + h];
+#pragma unroll
+      for (int r = 0; r < NR; ++r)
+        if (ht + r * RUN_STAGE < D) n_row[r] = a.n[((size_t)slot * a.heads + h) * D + ht + r * RUN_STAGE];
+    }
+    const float* q_at = a.q + (size_t)(sq.q_start + tok) * a.ldq + (size_t)hq * D + row4;
+    const float* k_at = MODE == OUTER_SCAN_HGRN ? nullptr : a.k + (size_t)(sq.q_start + tok) * a.ldk + (size_t)hq * D + row4;
+    const float* d_at = OS_OWN_DECAY<MODE> ? a.decay_raw + (size_t)(sq.q_start + tok) * a.ldd + (size_t)h * D + row4 : nullptr;
+    const float* v_at = a.v + (size_t)(sq.q_start + ht / OS_COLS) * a.ldv + (size_t)h * a.vdim + c0 + lane;
+    const bool v_in = c0 + lane < a.vdim;
+    auto fetch = [&](int n) {
+      const int nt = min(C, sq.q_len - n * C);
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int e = 0; e < EPT; ++e) {
+        const bool in = tok + e * TSTEP < nt;
+        pq[e] = in ? *reinterpret_cast<const float4*>(q_at + (size_t)(e * TSTEP) * a.ldq) : zero;
+        if (MODE != OUTER_SCAN_HGRN) pk[e] = in ? *reinterpret_cast<const float4*>(k_at + (size_t)(e * TSTEP) * a.ldk) : zero;
+        if (OS_OWN_DECAY<MODE>) pd[e] = in ? *reinterpret_cast<const float4*>(d_at + (size_t)(e * TSTEP) * a.ldd) : zero;
+      }
+#pragma unroll
+      for (int e = 0; e < VPT; ++e) pv[e] = v_in && ht / OS_COLS + 4 * e < nt ? v_at[(size_t)(4 * e) * a.ldv] : 0.f;
+      q_at += (size_t)C * a.ldq;
+      if (MODE != OUTER_SCAN_HGRN) k_at += (size_t)C * a.ldk;
+      if (OS_OWN_DECAY<MODE>) d_at += (size_t)C * a.ldd;
+      v_at += (size_t)C * a.ldv;
+    };
+    auto fetch_gates = [&](int blk) {                // first warp, lane: token 32 blk + lane
+      const int t = blk * 32 + lane;
+      if (t >= sq.q_len) return;
+      const size_t row = (size_t)(sq.q_start + t);
+      if (MODE == OUTER_SCAN_GATED) { pg0 = a.ig[row * a.ldg + h]; pg1 = a.fg[row * a.ldg + h]; }
+      if (MODE == OUTER_SCAN_SSD) pg0 = a.step_raw[row * a.lds + h];
+    };
+    auto take_gates = [&](int blk) {                 // ... the token's gates, and the maximum that runs through them
+      const int nt = min(32, sq.q_len - blk * 32), at = blk % 3;
+      if (MODE == OUTER_SCAN_GATED) {
+        float ig = 0.f, fg = 0.f, m_before = 0.f, m_after = 0.f;
+        if (lane < nt) {
+          ig = a.gate_cap * tanhf((pg0 + a.ig_b[h]) / a.gate_cap);
+          fg = logsigmoid_f(a.gate_cap * tanhf((pg1 + a.fg_b[h]) / a.gate_cap));
+        }
+#pragma unroll
+        for (int t = 0; t < 32; ++t) {
+          const float it = __shfl_sync(0xffffffffu, ig, t), ft = __shfl_sync(0xffffffffu, fg, t);
+          if (t < nt) {
+            const float m_new = fmaxf(ft + m_run, it);
+            if (lane == t) m_before = m_run, m_after = m_new;
+            m_run = m_new;
+          }
+        }
+        if (lane < nt) {
+          gates[at][lane][0] = expf(fg + m_before - m_after);
+          gates[at][lane][1] = expf(ig - m_after);
+          floor_m[at][lane] = expf(-m_after);
+        }
+      }
+      if (MODE == OUTER_SCAN_SSD && lane < nt) {     // the token's step size and the decay it gives
+        const float dt = softplus_f(pg0 + a.step_b[h]);
+        gates[at][lane][0] = expf(ssd_rate * dt);
+        gates[at][lane][1] = dt;
+      }
+    };
+    auto stage = [&](int n) {
+      const int buf = n % RING, nt = min(C, sq.q_len - n * C);
+      const float* gate = &gates[block_of(n)][n * C % 32][0];
+#pragma unroll
+      for (int e = 0; e < EPT; ++e) {
+        float* v3 = vec + ((size_t)(buf * C + tok + e * TSTEP) * NV) * D + row4;
+        float q[4] = {pq[e].x, pq[e].y, pq[e].z, pq[e].w}, k[4] = {pk[e].x, pk[e].y, pk[e].z, pk[e].w}, w[4] = {pd[e].x, pd[e].y, pd[e].z, pd[e].w};
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          if (MODE == OUTER_SCAN_HGRN) {             // q = silu(.), f = l + (1 - l) sigmoid(.), and what is written: 1 - f
+            const float dl = w[x] + w0[x];
+            k[x] = (1.f - low[x]) * sigmoid_f(-dl);  // 1 - f without the cancellation near f = 1
+            w[x] = low[x] + (1.f - low[x]) * sigmoid_f(dl);
+          }
+          if (MODE == OUTER_SCAN_LIGHTNING) k[x] = silu_f(k[x]);
+          if (MODE == OUTER_SCAN_DECAY) w[x] = expf(-expf(w[x] + w0[x]));
+          if (MODE == OUTER_SCAN_GLA) w[x] = expf(logsigmoid_f(w[x] + w0[x]) * a.inv_tau);
+          q[x] = (MODE == OUTER_SCAN_HGRN || MODE == OUTER_SCAN_LIGHTNING ? silu_f(q[x]) : q[x]) * a.q_scale;
+        }
+        *reinterpret_cast<float4*>(v3) = make_float4(q[0], q[1], q[2], q[3]);
+        *reinterpret_cast<float4*>(v3 + D) = make_float4(k[0], k[1], k[2], k[3]);
+        if (OS_OWN_DECAY<MODE>) *reinterpret_cast<float4*>(v3 + 2 * D) = make_float4(w[0], w[1], w[2], w[3]);
+      }
+#pragma unroll
+      for (int e = 0; e < VPT; ++e) {
+        const int tt = (ht + e * RUN_STAGE) / OS_COLS, at = buf * C * OS_COLS + ht + e * RUN_STAGE;
+        if (tt < nt) vcol[at] = GATES ? pv[e] * gate[2 * tt + 1] : MODE == OUTER_SCAN_LIGHTNING ? silu_f(pv[e]) : pv[e];
+        if (MODE == OUTER_SCAN_SSD) vraw[at] = pv[e];
+      }
+    };
+    auto normalise = [&](int n) {                    // GATED: n q of the chunk's tokens, a row per thread
+      const int nt = min(C, sq.q_len - n * C);
+      const float* gate = &gates[block_of(n)][n * C % 32][0];
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        const int i = ht + r * RUN_STAGE;
+        if (i >= D) continue;
+        float* v3 = vec + (size_t)(n % RING) * C * NV * D + i;
+        float nk[C], q[C];
+#pragma unroll
+        for (int tt = 0; tt < C; ++tt) nk[tt] = gate[2 * tt + 1] * v3[tt * NV * D + D], q[tt] = v3[tt * NV * D];   // (behind the last token: not used)
+#pragma unroll
+        for (int tt = 0; tt < C; ++tt)
+          if (tt < nt) {
+            n_row[r] = fmaf(gate[2 * tt], n_row[r], nk[tt]);
+            v3[tt * NV * D + 2 * D] = n_row[r] * q[tt];
+          }
+      }
+    };
+    const int n_blocks = (sq.q_len + 31) / 32;
+    const bool first_warp = ht < 32;
+    if (n_chunks > 0) fetch(0);
+    if (GATES && first_warp) {
+      fetch_gates(0);
+      take_gates(0);
+      fetch_gates(1);
+    }
+    for (int n = 0; n < n_chunks; ++n) {
+      if (n >= RING) bar_sync_at<EMPTY>(n % RING, RUN_STAGE + RUN_WRITE);
+      if (GATES) bar_sync_at<STAGED>(0, RUN_STAGE);  // the gates of this chunk's block are there
+      stage(n);
+      if (n + 1 < n_chunks) fetch(n + 1);
+      if (MODE == OUTER_SCAN_GATED) {
+        bar_sync_at<STAGED>(0, RUN_STAGE);           // every key of the chunk is there
+        normalise(n);
+      }
+      bar_arrive_at<FULL>(n % RING, RUN_ROWS + RUN_STAGE);
+      if (GATES && first_warp && n * C % 32 == 0 && n * C / 32 + 1 < n_blocks) {   // (the chunks of the block it replaces are out: EMPTY above)
+        take_gates(n * C / 32 + 1);
+        fetch_gates(n * C / 32 + 2);
+      }
+    }
+  } else {
+    // ===================== outputs: token t of a chunk by writer warp t & 1 =====================
+    constexpr int TPW = C / 2;
+    const int w = (ht - RUN_STAGE) >> 5;
+    const float ssd_skip = MODE == OUTER_SCAN_SSD ? a.D[h] : 0.f;
+    float* o_at = a.out + (size_t)(sq.q_start + w) * a.ldo + (size_t)h * a.vdim + c0 + lane;
+    const bool o_in = c0 + lane < a.vdim;
+    for (int n = 0; n < n_chunks; ++n) {
+      const int buf = n % RING, nt = min(C, sq.q_len - n * C);
+      bar_sync_at<DONE>(buf, RUN_ROWS + RUN_WRITE);
+      float sum[TPW], d[TPW];
+#pragma unroll
+      for (int e = 0; e < TPW; ++e) {
+        const int tt = w + 2 * e;
+        const float* from = part + (size_t)(buf * C + tt) * OS_GROUPS * OS_COLS + lane;
+        sum[e] = 0.f;
+#pragma unroll
+        for (int r = 0; r < OS_GROUPS; ++r) sum[e] += from[r * OS_COLS];
+        d[e] = 0.f;
+        if (MODE == OUTER_SCAN_GATED) {
+#pragma unroll
+          for (int i = 0; i < D; i += 32) d[e] += vec[((size_t)(buf * C + tt) * NV + 2) * D + i + lane];
+        }
+      }
+      if (MODE == OUTER_SCAN_GATED) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+          for (int e = 0; e < TPW; ++e) d[e] += __shfl_xor_sync(0xffffffffu, d[e], o);
+      }
+#pragma unroll
+      for (int e = 0; e < TPW; ++e) {
+        const int tt = w + 2 * e;
+        if (MODE == OUTER_SCAN_GATED) sum[e] = sum[e] / (fmaxf(fabsf(d[e]), floor_m[block_of(n)][n * C % 32 + tt]) + 1e-6f);
+        if (MODE == OUTER_SCAN_SSD) sum[e] = fmaf(ssd_skip, vraw[(buf * C + tt) * OS_COLS + lane], sum[e]);
+      }
+      if (n + RING < n_chunks) bar_arrive_at<EMPTY>(buf, RUN_STAGE + RUN_WRITE);
+#pragma unroll
+      for (int e = 0; e < TPW; ++e)
+        if (o_in && w + 2 * e < nt) o_at[(size_t)(2 * e) * a.ldo] = sum[e];
+      o_at += (size_t)C * a.ldo;
+    }
+  }
+  if (MODE == OUTER_SCAN_GATED) {                    // as above: the head's last piece overwrites what all of them started from
+    __syncthreads();
+    if (tid == 0) {
+      int32_t* done = a.done + (size_t)slot * a.heads + h;
+      last_block = nz == 1 || atomicAdd(done, 1) == nz - 1;
+      if (last_block && nz > 1) *done = 0;
+    }
+    __syncthreads();
+    if (last_block && ht >= 0 && ht < RUN_STAGE) {
+#pragma unroll
+      for (int r = 0; r < NR; ++r)
+        if (ht + r * RUN_STAGE < D) a.n[((size_t)slot * a.heads + h) * D + ht + r * RUN_STAGE] = n_row[r];
+      if (ht == 0) a.m[(size_t)slot * a.heads + h] = m_run;
+    }
+  }
+  if (zb == 0 && h == 0 && a.x_last != nullptr) {
+    const float* src = a.x + (size_t)(sq.q_start + sq.q_len - 1) * a.width;
+    for (int i = tid; i < a.width; i += RUN_THREADS) a.x_last[(size_t)slot * a.width + i] = src[i];
   }
 }
 
@@ -1207,8 +1604,10 @@ cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_s
     return launch_k(selective_step_kernel, dim3(n_seqs, (a.inner + 63) / 64), dim3(256), 0, stream, a, seqs, tok_slot);
   if (a.state <= SCAN_REG_STATE) {
     constexpr int per_cta = SCAN_THREADS / SCAN_LPC;
-    return launch_k(selective_scan_reg_kernel, dim3(n_seqs, (a.inner + per_cta - 1) / per_cta), dim3(SCAN_THREADS), 0, stream, a, seqs,
-                    tok_slot);
+    const long long blocks = (long long)n_seqs * ((a.inner + per_cta - 1) / per_cta);
+    if (blocks >= (1ll << 31)) return cudaErrorInvalidValue;
+    return launch_k(a.state == SCAN_REG_STATE ? selective_scan_reg_kernel<true> : selective_scan_reg_kernel<false>, dim3((unsigned)blocks), dim3(SCAN_THREADS), 0,
+                    stream, a, seqs, n_seqs, tok_slot);
   }
   const dim3 grid(n_seqs, (a.inner + SCAN_THREADS - 1) / SCAN_THREADS);
   const size_t smem = bc + (size_t)2 * a.state * SCAN_THREADS * sizeof(float);
@@ -1222,6 +1621,12 @@ cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_s
 }
 
 template <int RPT, int MODE>
+static cudaError_t outer_run(const OuterScan& a, const AttnSeq* seqs, int n_seqs, int pieces, const int32_t* tok_slot, cudaStream_t stream) {
+  static const cudaError_t attr = cudaFuncSetAttribute(outer_run_kernel<RPT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RUN_SMEM<RPT, MODE>);
+  if (attr != cudaSuccess) return attr;
+  return launch_k(outer_run_kernel<RPT, MODE>, dim3(pieces), dim3(RUN_THREADS), RUN_SMEM<RPT, MODE>, stream, a, seqs, n_seqs, tok_slot);
+}
+template <int RPT, int MODE>
 static cudaError_t outer_scan_rows(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot, cudaStream_t stream) {
   if constexpr (RPT <= 16) {   // (more rows, and columns that are no whole pieces, have no step kernel: 32 x 4 state values would spill)
     if (a.single && a.dim == RPT * OS_GROUPS && (reinterpret_cast<uintptr_t>(a.S) & 15) == 0) {
@@ -1229,14 +1634,18 @@ static cudaError_t outer_scan_rows(const OuterScan& a, const AttnSeq* seqs, int 
       if (a.vdim % 64 == 0) return launch_k(outer_step_kernel<RPT, MODE, 2>, dim3(n_seqs, a.heads, a.vdim / 64), dim3(OS_THREADS), 0, stream, a, seqs, tok_slot);
     }
   }
+  const long long pieces = (long long)n_seqs * a.heads * ((a.vdim + OS_COLS - 1) / OS_COLS);
+  auto al16 = [](const float* p, int ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; };   // (nullptr where the mode has none)
+  if (a.dim == RPT * OS_GROUPS && pieces < (1ll << 31) && al16(a.q, a.ldq) && (MODE == OUTER_SCAN_HGRN || al16(a.k, a.ldk)) &&
+      (!OS_OWN_DECAY<MODE> || al16(a.decay_raw, a.ldd)))
+    return outer_run<RPT, MODE>(a, seqs, n_seqs, (int)pieces, tok_slot, stream);
   const dim3 grid(n_seqs, a.heads, (a.vdim + OS_COLS - 1) / OS_COLS);
   const size_t smem = ((size_t)OS_CHUNK * 3 * ((a.dim + 3) & ~3) + OS_CHUNK * OS_COLS) * sizeof(float);   // <= 50 KB (+ 17 KB static)
-  const auto kernel = a.dim == RPT * OS_GROUPS ? outer_scan_kernel<RPT, MODE, true> : outer_scan_kernel<RPT, MODE, false>;
   if (RPT > 16) {   // keys of more than 128 entries: the staged chunk passes the default 48 KB of shared memory
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(outer_scan_kernel<RPT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
     if (e != cudaSuccess) return e;
   }
-  return launch_k(kernel, grid, dim3(OS_THREADS), smem, stream, a, seqs, tok_slot);
+  return launch_k(outer_scan_kernel<RPT, MODE>, grid, dim3(OS_THREADS), smem, stream, a, seqs, tok_slot);
 }
 template <int MODE>
 static cudaError_t outer_scan_mode(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot,
