@@ -60,8 +60,9 @@ __device__ __forceinline__ float relu2_row_scale(const GemmAny& a, int dst) {
 // no other row and no tile height enters.  BM / 8 + 4 loads feed BM packed multiply-adds of two k each.  The next k-block's
 // global loads (16 bytes each where the rows allow it) are in flight while this one is worked on.
 // Measured, fp32, T x N x K (before: scalar staging, one 16-byte and several 4-byte shared loads for 16 multiply-adds, nothing
-// in flight): 389 x 1088 x 1024 149 -> 40 us, 16 experts of 2048 x 1024 under 778 rows 296 -> 130 us, 10 x 32768 x 1024 189 -> 59 us,
-// 16 x 1024 x 1024 93 -> 25 us; 40 TFLOP/s where there are tiles enough (of 74: the shared-memory loads take the rest).
+// in flight; then with half-warps instead of neighbouring lanes on one weight row): 389 x 1088 x 1024 149 -> 47 -> 41 us, 16 experts of
+// 2048 x 1024 under 778 rows 296 -> 165 (tiles of 64 rows) -> 118 us, 10 x 32768 x 1024 189 -> 57 -> 44 us.  With one or two warps to a
+// scheduler the waits between dependent instructions are what is left; the operands of the next four k in registers ahead: no faster (41).
 constexpr int FMA_THREADS = 128;
 constexpr int FMA_BN = 64, FMA_BK = 32, FMA_LD = FMA_BK + 4;
 constexpr int FMA_SMS = 148;   // (tile heights only: a sum does not depend on them)
@@ -139,7 +140,9 @@ __global__ void __launch_bounds__(FMA_THREADS) gemm_any_kernel(GemmAny a) {
   const WT* W = reinterpret_cast<const WT*>(a.W) + (size_t)z * a.w_bs + (size_t)group * a.w_gs;
   OT* Y = reinterpret_cast<OT*>(a.Y) + (size_t)z * a.y_bs;
   const int n0 = blockIdx.x * FMA_BN;
-  const int ty = tid / 16, tx = tid % 16;
+  // neighbouring lanes share a weight row: a 16-byte load whose lanes agree in pairs takes two passes over the banks, one whose half-warps
+  // agree takes four
+  const int ty = tid / 32 * 2 + (tid & 1), tx = tid % 32 / 2;
 
   // pieces of four k: piece e -> row e / 8, k 4 (e % 8)
   const int pk = (tid & 7) * 4, pr = tid >> 3;
@@ -216,7 +219,7 @@ __global__ void __launch_bounds__(FMA_THREADS) gemm_any_kernel(GemmAny a) {
       __syncthreads();
     }
   }
-  // ---- epilogue: a thread's columns are 16 apart; gate and up of a pair sit in neighbouring threads
+  // ---- epilogue: a thread's columns are 16 apart; gate and up of a pair sit two threads apart
   const bool glu = a.mode == GEMM_ANY_SWIGLU || a.mode == GEMM_ANY_GEGLU;
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -227,7 +230,7 @@ __global__ void __launch_bounds__(FMA_THREADS) gemm_any_kernel(GemmAny a) {
       const int n = n0 + tx + 16 * j;
       const float v = sum2(acc[i][j]);
       if (glu) {   // columns (2c, 2c + 1) = (gate_c, up_c): out[c] = act(gate) * up
-        const float up = __shfl_down_sync(0xffffffffu, v, 1);
+        const float up = __shfl_down_sync(0xffffffffu, v, 2);
         if ((tx & 1) == 0 && dst >= 0 && n + 1 < a.N) st_from_float(Y + (size_t)dst * a.ldy + n / 2, glu_pair(a.mode, v, up));
       } else if (dst >= 0 && n < a.N) {
         const float o = a.mode == GEMM_ANY_RELU2 ? relu2_scaled(v, s) : a.mode == GEMM_ANY_TANH ? tanhf(v) : a.mode == GEMM_ANY_GELU ? gelu_erf(v) : v * s;
@@ -497,15 +500,15 @@ cudaError_t launch_fma(const GemmAny& a, cudaStream_t stream) {
   const bool vec = a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && a.x_bs % 4 == 0 && a.w_bs % 4 == 0 && a.w_gs % 4 == 0 &&
                    al(a.X, sizeof(XT)) && al(a.W, sizeof(WT));
   // rows per tile: 16 for skinny problems (decode steps, small segments); 64 where that makes three tiles for every SM, else 32
-  // (K = 1024: 389 x 2048 57 us with 32 rows, 66 with 64; 2048 x 4096 478 and 431)
+  // (K = 1024: 389 x 2048 57 us with 32 rows, 66 with 64; 2048 x 4096 478 and 431).  Segments take 32: they end inside their last tile
+  // (16 experts of 2048 x 1024, 16 / 32 / 64 rows: 389 rows in all 82 / 74 / 127, 778 129 / 118 / 130, 4096 549 / 472 / 500)
   const int rows = a.seg_off != nullptr ? (a.T + a.n_groups - 1) / (a.n_groups > 0 ? a.n_groups : 1) : a.T;
-  const long long tiles64 = (long long)((a.N + FMA_BN - 1) / FMA_BN) * (a.batch > 0 ? a.batch : 1) *
-                            (a.seg_off != nullptr ? (long long)a.n_groups * ((rows + 63) / 64) : (a.T + 63) / 64);
+  const long long tiles64 = (long long)((a.N + FMA_BN - 1) / FMA_BN) * (a.batch > 0 ? a.batch : 1) * ((a.T + 63) / 64);
   // (16 rows too where 32 would leave half of the SMs without a tile and K is short: 32 x 4096 x 128 13.6 -> 7.4 us)
   const long long tiles32 = (long long)((a.N + FMA_BN - 1) / FMA_BN) * (a.batch > 0 ? a.batch : 1) * ((rows + 31) / 32);
   if (rows <= 20 || (a.seg_off == nullptr && a.K <= 256 && 2 * tiles32 <= FMA_SMS)) return launch_fma_bm<XT, WT, OT, 16>(a, vec, stream);
   const bool fit32 = (a.T + 31ll) / 32 + (a.seg_off != nullptr ? a.n_groups : 0) <= 65535;   // tiles of one launch (grid.y)
-  if (fit32 && (rows <= 36 || tiles64 < 3 * FMA_SMS || a.K <= 256)) return launch_fma_bm<XT, WT, OT, 32>(a, vec, stream);
+  if (fit32 && (a.seg_off != nullptr || rows <= 36 || tiles64 < 3 * FMA_SMS || a.K <= 256)) return launch_fma_bm<XT, WT, OT, 32>(a, vec, stream);
   return launch_fma_bm<XT, WT, OT, 64>(a, vec, stream);
 }
 
