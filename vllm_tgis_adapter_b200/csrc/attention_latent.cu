@@ -230,6 +230,29 @@ latent_attn_kernel(const float* __restrict__ q_abs, const CT* __restrict__ cache
   }
 }
 
+inline __host__ __device__ int lat_ld32(int D) { return D + (D % 8 == 0 ? 4 : 8); }   // padded row (floats): 16-byte pieces of eight rows in 32 banks
+constexpr size_t LAT_ROWS_SMEM = 227 * 1024;
+inline size_t lat_rows_smem(int D, int tiles, int stages) {
+  const size_t rows = (size_t)tiles * LATENT_PAIRS;
+  return ((rows + (size_t)stages * KV_BLOCK) * lat_ld32(D) + rows * 36 + KV_BLOCK * (rows + 4) + 2 * rows) * sizeof(float);
+}
+__device__ __forceinline__ unsigned long long pack2f(float x, float y) {
+  unsigned long long d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ void unpack2f(unsigned long long v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+__device__ __forceinline__ unsigned long long mul2f(unsigned long long x, unsigned long long y) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ unsigned long long fma2f(unsigned long long x, unsigned long long y, unsigned long long z) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(x), "l"(y), "l"(z));
+  return d;
+}
+
 // ---- tensor-core variant (bf16 cache rows of a multiple of 8 entries) ------------------------------------------------
 // Same work split as latent_attn_kernel (a CTA = up to 16 (token, head) pairs of one sequence against the 32-row cache
 // blocks they can see), with the two products on mma.sync m16n8k16: the 16 pairs are the M rows of both.
@@ -238,7 +261,8 @@ latent_attn_kernel(const float* __restrict__ q_abs, const CT* __restrict__ cache
 //   softmax fp32, one warp per two rows, lane = key (as in the FMA kernel): running maximum and sum, P rounded to bf16
 //   output  O [16 x kv_rank] += P [16 x 32] C [32 x kv_rank]: warp w owns the 8-column tiles w, w + 8, ... (fp32 accumulators
 //           in registers for the whole walk), C read straight from the staged rows with ldmatrix.trans
-// Cache blocks arrive by cp.async, double-buffered: block i + 1 lands while block i is being used.  Q is scaled and rounded
+// Cache blocks arrive by cp.async, double-buffered: block i + 1 lands while block i is being used, the first while Q is read (four
+// 16-byte loads in flight a thread: 32 sequences of 64 to 88 keys, 16 heads, row 576: 17.7 -> 13.1 us).  Q is scaled and rounded
 // to bf16 once.  A query's arithmetic still depends only on its own position and its sequence's block grid.
 __device__ __forceinline__ void lat_cp_async_16(void* smem, const void* gmem) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
@@ -289,19 +313,6 @@ latent_attn_mma_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __r
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int pos0 = sq.kv_len - sq.q_len + tile.q0;
   const int row0 = sq.q_start + tile.q0;
-  // zero once what no copy fills, then fill Q
-  {  // all of Q (unused pair rows, k padding); of the two K buffers only the columns behind D (the copies fill the rest)
-    uint32_t* z = reinterpret_cast<uint32_t*>(smem_raw);
-    for (int i = tid; i < LATENT_PAIRS * LDQ / 2; i += LAT_THREADS) z[i] = 0u;
-    const int pad = LDQ - D;
-    for (int i = tid; i < 2 * KV_BLOCK * pad; i += LAT_THREADS) Ks[(size_t)(i / pad) * LDQ + D + i % pad] = __float2bfloat16_rn(0.f);
-  }
-  __syncthreads();
-  for (int e = tid; e < npairs * D; e += LAT_THREADS) {
-    const int p = e / D, d = e - p * D;
-    const int tq = p / nh, h = h0 + p - tq * nh;
-    Qs[(size_t)p * LDQ + d] = __float2bfloat16_rn(q_abs[((size_t)(row0 + tq) * g.heads + h) * D + d] * g.scale);
-  }
   const int pos_last = pos0 + tile.nq - 1;
   const int kmin = g.window > 0 ? max(0, pos0 - g.window + 1) : 0;
   int blk0 = kmin / KV_BLOCK, blk1 = pos_last / KV_BLOCK;
@@ -323,16 +334,41 @@ latent_attn_mma_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __r
     }
   }
   const int32_t* bt = block_table + (size_t)sq.block_row * bt_stride;
-  const int chunks_per_row = D / 8;
+  const uint32_t per_row = (uint32_t)D / 8, magic = ((1u << 20) + per_row - 1) / per_row;   // c / per_row for c < 32 per_row <= 2^15
   auto load_block = [&](int blk, int st) {
     const bf* src = cache + (size_t)bt[blk] * KV_BLOCK * D;
     bf* dst = Ks + (size_t)st * KV_BLOCK * LDQ;
-    for (int c = tid; c < KV_BLOCK * chunks_per_row; c += LAT_THREADS) {
-      const int r = c / chunks_per_row, cc = c - r * chunks_per_row;
-      lat_cp_async_16(dst + (size_t)r * LDQ + cc * 8, src + (size_t)r * D + cc * 8);
-    }
+#pragma unroll 4
+    for (uint32_t c = tid; c < KV_BLOCK * per_row; c += LAT_THREADS)
+      lat_cp_async_16(dst + c * 8 + ((c * magic) >> 20) * (uint32_t)(LDQ - D), src + c * 8);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
+  load_block(blk0, 0);   // (on its way while Q is read)
+  {  // Q, scaled and rounded to bf16 once; zeros where no copy comes (unused pair rows, k padding)
+    const int pad = LDQ - D, d4 = D / 4;
+    for (int i = npairs * LDQ / 2 + tid; i < LATENT_PAIRS * LDQ / 2; i += LAT_THREADS) reinterpret_cast<uint32_t*>(Qs)[i] = 0u;
+    for (int i = tid; i < npairs * pad; i += LAT_THREADS) Qs[(size_t)(i / pad) * LDQ + D + i % pad] = __float2bfloat16_rn(0.f);
+    for (int i = tid; i < 2 * KV_BLOCK * pad; i += LAT_THREADS) Ks[(size_t)(i / pad) * LDQ + D + i % pad] = __float2bfloat16_rn(0.f);
+    auto put = [&](int e, const float4& v) {
+      const int p = e / d4, d = (e - p * d4) * 4;
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x * g.scale, v.y * g.scale), hi = __floats2bfloat162_rn(v.z * g.scale, v.w * g.scale);
+      *reinterpret_cast<uint2*>(Qs + (size_t)p * LDQ + d) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    };
+    auto at = [&](int e) {
+      const int p = e / d4, d = (e - p * d4) * 4, tq = p / nh, h = h0 + p - tq * nh;
+      return *reinterpret_cast<const float4*>(q_abs + ((size_t)(row0 + tq) * g.heads + h) * D + d);
+    };
+    const int n = npairs * d4;
+    int e = tid;
+    for (; e + 3 * LAT_THREADS < n; e += 4 * LAT_THREADS) {   // (four loads in flight)
+      const float4 v0 = at(e), v1 = at(e + LAT_THREADS), v2 = at(e + 2 * LAT_THREADS), v3 = at(e + 3 * LAT_THREADS);
+      put(e, v0);
+      put(e + LAT_THREADS, v1);
+      put(e + 2 * LAT_THREADS, v2);
+      put(e + 3 * LAT_THREADS, v3);
+    }
+    for (; e < n; e += LAT_THREADS) put(e, at(e));
+  }
   // softmax rows of this warp (two pairs), as in the FMA kernel
   int prow[2], posq[2];
   bool on[2];
@@ -352,7 +388,6 @@ latent_attn_mma_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __r
   const int ks_lo = half == 0 ? 0 : KS / 2, ks_hi = half == 0 ? KS / 2 : KS;
   const int gq = lane >> 2, t2 = (lane & 3) * 2;
 
-  load_block(blk0, 0);
   for (int blk = blk0; blk <= blk1; ++blk) {
     const int st = (blk - blk0) & 1;
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -682,6 +717,225 @@ cudaError_t launch_attn_wide(const float* q_abs, const void* cache, const AttnSe
                   q_abs, reinterpret_cast<const __nv_bfloat16*>(cache), seqs, tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g);
 }
 
+// ---- fp32 prompts: two or four tiles of one sequence per CTA ---------------------------------------------------------------
+// The FMA kernel above reads three numbers from shared memory for two multiply-adds, and with two tokens a tile (eight heads) a prompt's
+// neighbours stream the same cache rows again.  Here a CTA takes RT tiles, 16 RT (token, head) rows, against each staged 32-row block:
+//   scores  thread (ty, tx): rows ty + 16 i, keys tx and tx + 16, four dims to a load, the next four on their way;
+//   softmax four lanes per row with eight keys each;
+//   output  warp w: 2 RT rows, a lane four columns of each 128: a row's weight is one broadcast, two columns one packed fma.
+// Every sum runs in the order of the FMA kernel, so a query has the same bits whichever of the two its step takes.  Blocks arrive by
+// cp.async, the next one under the work on this one where two fit.  Bound by latencies at one CTA of eight warps per SM; prompts of 19, 107
+// and 263 tokens, 8 heads, rank 256: 157 -> 73 us a launch (81 with half-warps instead of neighbouring lanes on one key row).
+template <int RT, int CPL>  // CPL * 32 >= kv_rank
+__global__ void __launch_bounds__(LAT_THREADS, 1)
+latent_attn_rows_kernel(const float* __restrict__ q_abs, const float* __restrict__ cache, const AttnSeq* __restrict__ seqs, const LatentTile* __restrict__ tiles,
+                        int tile_tokens, const int32_t* __restrict__ block_table, int bt_stride, void* __restrict__ o_lat, int o_dtype, LatentGeom g, int stages) {
+  constexpr int ROWS = RT * LATENT_PAIRS, RPW = ROWS / LAT_WARPS, LDS_ = 36, LDP = ROWS + 4;
+  extern __shared__ __align__(16) float smem_f[];
+  const int D = g.row(), R = g.kv_rank, LD = lat_ld32(D);
+  float* Qs = smem_f;                                   // [ROWS][LD]
+  float* Ks = Qs + (size_t)ROWS * LD;                   // [stages][32][LD]
+  float* Sp = Ks + (size_t)stages * KV_BLOCK * LD;      // [ROWS][36]
+  float* Pt = Sp + ROWS * LDS_;                         // [32][ROWS + 4]
+  float* corr_s = Pt + KV_BLOCK * LDP;                  // [ROWS]
+  float* inv_s = corr_s + ROWS;                         // [ROWS]
+  griddep_launch();
+  griddep_wait();
+  const LatentTile tile = tiles[blockIdx.x];
+  const AttnSeq sq = seqs[tile.seq];
+  const int pos0 = sq.kv_len - sq.q_len + tile.q0, row0 = sq.q_start + tile.q0;
+  const int group = RT * tile_tokens, at = pos0 % group;   // the first of a group's tiles does the work (latent_attn_wide_kernel)
+  if (tile.q0 != 0 && at >= tile_tokens) return;
+  const int h0 = blockIdx.y * LATENT_PAIRS, nh = min(g.heads - h0, LATENT_PAIRS);
+  const int nq = min((group - at + tile_tokens - 1) / tile_tokens * tile_tokens, sq.q_len - tile.q0), rows = nq * nh;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, d4 = D / 4;
+  for (int e = tid; e < ROWS * d4; e += LAT_THREADS) {
+    const int p = e / d4, d = (e - p * d4) * 4, tq = p / nh, h = h0 + p - tq * nh;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (p < rows) v = *reinterpret_cast<const float4*>(q_abs + ((size_t)(row0 + tq) * g.heads + h) * D + d);
+    *reinterpret_cast<float4*>(Qs + (size_t)p * LD + d) = make_float4(v.x * g.scale, v.y * g.scale, v.z * g.scale, v.w * g.scale);
+  }
+  const int pos_last = pos0 + nq - 1, kmin = g.window > 0 ? max(0, pos0 - g.window + 1) : 0;
+  const int blk0 = kmin / KV_BLOCK, blk1 = pos_last / KV_BLOCK;
+  const int32_t* bt = block_table + (size_t)sq.block_row * bt_stride;
+  auto load_block = [&](int blk, int st) {
+    const float* src = cache + (size_t)bt[blk] * KV_BLOCK * D;
+    float* dst = Ks + (size_t)st * KV_BLOCK * LD;
+    for (int c = tid; c < KV_BLOCK * d4; c += LAT_THREADS) {
+      const int r = c / d4;
+      lat_cp_async_16(dst + (size_t)r * LD + (c - r * d4) * 4, src + (size_t)c * 4);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  const int ty = warp * 2 + (lane & 1), tx = lane >> 1;   // (neighbouring lanes share a key row: two passes over the banks instead of four)
+  const int sr = tid >> 2, sk = tid & 3, sposq = sr < rows ? pos0 + sr / nh : -1;
+  float m_run = -FLT_MAX, l_run = 0.f;
+  unsigned long long acc[RPW][CPL / 2];
+#pragma unroll
+  for (int r = 0; r < RPW; ++r)
+#pragma unroll
+    for (int c = 0; c < CPL / 2; ++c) acc[r][c] = 0;   // packed zeros
+
+  load_block(blk0, 0);
+  for (int blk = blk0; blk <= blk1; ++blk) {
+    const int st = stages > 1 ? (blk - blk0) & 1 : 0;
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();   // block `blk` has landed for everyone; everyone is done with the other buffer, P, S and corr
+    if (stages > 1 && blk < blk1) load_block(blk + 1, st ^ 1);
+    const float* Kb = Ks + (size_t)st * KV_BLOCK * LD;
+    {  // ---- scores
+      float c[RT][2];
+#pragma unroll
+      for (int i = 0; i < RT; ++i) c[i][0] = c[i][1] = 0.f;
+      const float *qp = Qs + (size_t)ty * LD, *kp = Kb + (size_t)tx * LD;
+      float4 x[2][RT], k[2][2];
+      auto take = [&](int b, int d) {
+#pragma unroll
+        for (int i = 0; i < RT; ++i) x[b][i] = *reinterpret_cast<const float4*>(qp + (size_t)(16 * i) * LD + d);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) k[b][j] = *reinterpret_cast<const float4*>(kp + (size_t)(16 * j) * LD + d);
+      };
+      auto use = [&](int b) {
+#pragma unroll
+        for (int i = 0; i < RT; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) c[i][j] = fmaf(x[b][i].x, k[b][j].x, c[i][j]);
+#pragma unroll
+        for (int i = 0; i < RT; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) c[i][j] = fmaf(x[b][i].y, k[b][j].y, c[i][j]);
+#pragma unroll
+        for (int i = 0; i < RT; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) c[i][j] = fmaf(x[b][i].z, k[b][j].z, c[i][j]);
+#pragma unroll
+        for (int i = 0; i < RT; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) c[i][j] = fmaf(x[b][i].w, k[b][j].w, c[i][j]);
+      };
+      take(0, 0);
+      int d = 0;
+#pragma unroll 2
+      for (; d + 8 <= D; d += 8) {
+        take(1, d + 4);
+        use(0);
+        if (d + 8 < D) take(0, d + 8);
+        use(1);
+      }
+      if (d < D) use(0);
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) Sp[(ty + 16 * i) * LDS_ + tx + 16 * j] = c[i][j];
+    }
+    __syncthreads();
+    if (sr < ROWS) {  // ---- softmax: keys sk, sk + 4, ... of row sr; sums in the order of a warp's sixteen-, eight-, ... lane exchanges over 32 keys
+      float x[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = Sp[sr * LDS_ + sk + 4 * e];
+      const int last = sposq - (blk * KV_BLOCK + sk), first = g.window > 0 ? last - g.window + 1 : 0;   // visible: first <= 4 e <= last
+      float m_new = -FLT_MAX;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) m_new = fmaxf(m_new, 4 * e <= last && 4 * e >= first ? x[e] : -FLT_MAX);
+      m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 1));
+      m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 2));
+      m_new = fmaxf(m_run, m_new);
+      // nothing visible so far (m_new still the sentinel): all weights 0, state unchanged
+      const float corr = m_new == -FLT_MAX ? 1.f : expf(m_run - m_new);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] = 4 * e <= last && 4 * e >= first ? expf(x[e] - m_new) : 0.f;
+      float sum = ((x[0] + x[4]) + (x[2] + x[6])) + ((x[1] + x[5]) + (x[3] + x[7]));
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      l_run = l_run * corr + sum;
+      m_run = m_new;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) Pt[(sk + 4 * e) * LDP + sr] = x[e];
+      if (sk == 0) corr_s[sr] = corr;
+    }
+    __syncthreads();
+    {  // ---- output: rescale, then O += P C; in a block with hidden keys a weight of zero is left out (its row may hold anything)
+      const bool whole = (blk + 1) * KV_BLOCK - 1 <= pos0 && (g.window <= 0 || pos_last - blk * KV_BLOCK < g.window);
+      const float* pt = Pt + warp * RPW;
+#pragma unroll
+      for (int r = 0; r < RPW; ++r) {
+        const float f = corr_s[warp * RPW + r];
+        const unsigned long long f2 = pack2f(f, f);
+#pragma unroll
+        for (int c = 0; c < CPL / 2; ++c) acc[r][c] = mul2f(acc[r][c], f2);
+      }
+#pragma unroll 2
+      for (int j = 0; j < KV_BLOCK; ++j) {
+        float p[RPW];
+#pragma unroll
+        for (int r = 0; r < RPW; r += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(pt + j * LDP + r);
+          p[r] = v.x; p[r + 1] = v.y; p[r + 2] = v.z; p[r + 3] = v.w;
+        }
+        ulonglong2 cv[CPL / 4];
+#pragma unroll
+        for (int c = 0; c < CPL / 4; ++c)
+          cv[c] = (lane + 32 * c) * 4 < R ? *reinterpret_cast<const ulonglong2*>(Kb + (size_t)j * LD + (lane + 32 * c) * 4) : make_ulonglong2(0, 0);
+#pragma unroll
+        for (int r = 0; r < RPW; ++r) {
+          if (!whole && p[r] == 0.f) continue;   // warp-uniform
+          const unsigned long long p2 = pack2f(p[r], p[r]);
+#pragma unroll
+          for (int c = 0; c < CPL / 4; ++c) {
+            acc[r][2 * c] = fma2f(p2, cv[c].x, acc[r][2 * c]);
+            acc[r][2 * c + 1] = fma2f(p2, cv[c].y, acc[r][2 * c + 1]);
+          }
+        }
+      }
+    }
+    if (stages == 1 && blk < blk1) {
+      __syncthreads();
+      load_block(blk + 1, 0);
+    }
+  }
+  if (sk == 0 && sr < rows) inv_s[sr] = 1.f / (l_run + (g.sink != nullptr ? expf(g.sink[h0 + sr % nh] - m_run) : 0.f));
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < RPW; ++r) {
+    const int p = warp * RPW + r;
+    if (p >= rows) break;
+    const int tq = p / nh, h = h0 + p - tq * nh;
+    const size_t o = ((size_t)(row0 + tq) * g.heads + h) * R;
+    const float inv = inv_s[p];
+#pragma unroll
+    for (int c = 0; c < CPL / 4; ++c) {
+      const int n = (lane + 32 * c) * 4;
+      if (n >= R) continue;
+      float v[4];
+      unpack2f(acc[r][2 * c], v[0], v[1]);
+      unpack2f(acc[r][2 * c + 1], v[2], v[3]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] *= inv;
+      if (o_dtype == DT_F32) {
+        *reinterpret_cast<float4*>(reinterpret_cast<float*>(o_lat) + o + n) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) st_any(o_lat, o_dtype, o + n + e, v[e]);
+      }
+    }
+  }
+}
+
+template <int RT>
+cudaError_t launch_attn_rows(const float* q_abs, const float* cache, const AttnSeq* seqs, const LatentTile* tiles, int n_tiles, int tile_tokens,
+                             const int32_t* block_table, int bt_stride, void* o_lat, int o_dtype, const LatentGeom& g, cudaStream_t stream) {
+  const int stages = lat_rows_smem(g.row(), RT, 2) <= LAT_ROWS_SMEM ? 2 : 1;
+  auto launch = [&](auto kernel) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LAT_ROWS_SMEM);
+    if (e != cudaSuccess) return e;
+    return launch_k(kernel, dim3(n_tiles, (g.heads + LATENT_PAIRS - 1) / LATENT_PAIRS), dim3(LAT_THREADS), lat_rows_smem(g.row(), RT, stages), stream, q_abs,
+                    cache, seqs, tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g, stages);
+  };
+  if (g.kv_rank <= 128) return launch(latent_attn_rows_kernel<RT, 4>);
+  if (g.kv_rank <= 256) return launch(latent_attn_rows_kernel<RT, 8>);
+  return launch(latent_attn_rows_kernel<RT, 16>);
+}
+
 // o_lat[pair] = sum_z e^(m_z - M) acc_z / sum_z e^(m_z - M) l_z over the splits in ascending order, M = max_z m_z.
 // One CTA per (tile, head group, pair); the split weights are worked out once in shared memory.
 constexpr int LATENT_MAX_SPLITS = 64;
@@ -754,13 +1008,13 @@ cudaError_t launch_attn_mma(const float* q_abs, const void* cache, const AttnSeq
                   (const float*)part, n_splits, seqs, tiles, o_lat, o_dtype, g);
 }
 
-bool latent_mma_eligible(const void* cache, int dtype, const LatentGeom& g) {
+bool latent_mma_eligible(const float* q_abs, const void* cache, int dtype, const LatentGeom& g) {
   static int on = -1;
   if (on < 0) {
     const char* e = getenv("TGIS_LATENT_ATTN_MMA");
     on = (e && e[0] == '0') ? 0 : 1;
   }
-  return on && dtype == DT_BF16 && g.row() % 8 == 0 && g.kv_rank % 8 == 0 && g.kv_rank <= 512 &&
+  return on && dtype == DT_BF16 && (reinterpret_cast<uintptr_t>(q_abs) & 15) == 0 && g.row() % 8 == 0 && g.kv_rank % 8 == 0 && g.kv_rank <= 512 &&
          (reinterpret_cast<uintptr_t>(cache) & 15) == 0 && lat_mma_smem(g.row()) <= 200 * 1024;
 }
 
@@ -820,7 +1074,7 @@ cudaError_t latent_attn_launch(const float* q_abs, const void* cache, int dtype,
                                size_t split_ws_floats, int max_kv_len, int num_sms, int* n_launched, int n_seqs, int tile_tokens) {
   if (n_launched) *n_launched = n_tiles > 0 ? 1 : 0;
   if (n_tiles <= 0) return cudaSuccess;
-  if (latent_mma_eligible(cache, dtype, g)) {
+  if (latent_mma_eligible(q_abs, cache, dtype, g)) {
     // Steps with too few tiles to fill the GPU (decode-shaped): every tile's key range is cut into fixed splits that run as
     // CTAs of their own.  The split count is a function of the longest sequence rounded up to whole splits (and of the
     // window), so a captured launch stays valid for every step of its CUDA-graph key.
@@ -842,7 +1096,7 @@ cudaError_t latent_attn_launch(const float* q_abs, const void* cache, int dtype,
     if (n_launched && n_splits > 1) *n_launched = 2;  // + the merge kernel
     // prompts (four tiles of a sequence and more on average): the wide kernel.  Below that its CTAs would hold one M tile each.
     if (n_splits == 1 && n_seqs > 0 && tile_tokens > 0 && tile_tokens <= latent_tile_tokens(g.heads) && n_tiles >= 4 * n_seqs &&
-        lat_wide_smem(g.row()) <= 227 * 1024 && (reinterpret_cast<uintptr_t>(q_abs) & 15) == 0 && (reinterpret_cast<uintptr_t>(o_lat) & 15) == 0) {
+        lat_wide_smem(g.row()) <= 227 * 1024 && (reinterpret_cast<uintptr_t>(o_lat) & 15) == 0) {
       if (g.kv_rank <= 128) return launch_attn_wide<2>(q_abs, cache, seqs, tiles, n_tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g, stream);
       if (g.kv_rank <= 256) return launch_attn_wide<4>(q_abs, cache, seqs, tiles, n_tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g, stream);
       return launch_attn_wide<8>(q_abs, cache, seqs, tiles, n_tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g, stream);
@@ -850,6 +1104,15 @@ cudaError_t latent_attn_launch(const float* q_abs, const void* cache, int dtype,
     if (g.kv_rank <= 128) return launch_attn_mma<2>(q_abs, cache, seqs, tiles, n_tiles, block_table, bt_stride, o_lat, o_dtype, g, stream, split_ws, n_splits);
     if (g.kv_rank <= 256) return launch_attn_mma<4>(q_abs, cache, seqs, tiles, n_tiles, block_table, bt_stride, o_lat, o_dtype, g, stream, split_ws, n_splits);
     return launch_attn_mma<8>(q_abs, cache, seqs, tiles, n_tiles, block_table, bt_stride, o_lat, o_dtype, g, stream, split_ws, n_splits);
+  }
+  // fp32 prompts: two tiles of a sequence and more on average; four to a CTA where two would leave none idle
+  if (dtype == DT_F32 && n_seqs > 0 && tile_tokens > 0 && tile_tokens <= latent_tile_tokens(g.heads) && n_tiles >= 2 * n_seqs && g.row() % 4 == 0 &&
+      g.kv_rank % 4 == 0 && g.kv_rank <= 512 && lat_rows_smem(g.row(), 2, 1) <= LAT_ROWS_SMEM && (reinterpret_cast<uintptr_t>(cache) & 15) == 0 &&
+      (reinterpret_cast<uintptr_t>(q_abs) & 15) == 0 && (reinterpret_cast<uintptr_t>(o_lat) & 15) == 0) {
+    const int hg = (g.heads + LATENT_PAIRS - 1) / LATENT_PAIRS;
+    if (n_tiles / 4 * hg >= num_sms && lat_rows_smem(g.row(), 4, 1) <= LAT_ROWS_SMEM)
+      return launch_attn_rows<4>(q_abs, (const float*)cache, seqs, tiles, n_tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g, stream);
+    return launch_attn_rows<2>(q_abs, (const float*)cache, seqs, tiles, n_tiles, tile_tokens, block_table, bt_stride, o_lat, o_dtype, g, stream);
   }
   if (dtype == DT_BF16)
     return launch_attn_ct<__nv_bfloat16>(q_abs, cache, seqs, tiles, n_tiles, block_table, bt_stride, o_lat, o_dtype, g, stream);
