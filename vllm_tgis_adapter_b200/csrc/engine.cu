@@ -410,6 +410,7 @@ struct tgis_engine {
   CUtensorMap xm_xn[N_BT], xm_attn[N_BT], xm_act[N_BT], xm_last[N_BT], xm_resid[N_BT];
   DevBuf<float> gemm_ws, part_o, part_ml, samp_scratch;
   DevBuf<int> gemm_counters, attn_arrive;
+  DevBuf<float> skinny_ssq;   // [2][8][hidden / 8] sums of squares of eight columns (gemm_skinny_add_launch)
   DevBuf<float> norm_ssq;  // [2][GEMM_NORM_MAX_T][hidden / 128] partial sums of h^2 (fused residual RMSNorm)
   DevBuf<uint32_t> seen_bitmap;
   // guided decoding: allowed-token bits of the step, one row per sequence slot (same geometry as seen_bitmap); the
@@ -733,6 +734,7 @@ struct tgis_engine {
     attn_arrive.alloc((size_t)S_max * std::max(nkv, 1));
     attn_arrive.zero();
     norm_ssq.alloc((size_t)2 * GEMM_NORM_MAX_T * (c.hidden / 128 + 1));
+    skinny_ssq.alloc((size_t)2 * 8 * (c.hidden / 8));
     const int G = c.n_q_heads / std::max(c.n_kv_heads, 1);
     part_o.alloc((size_t)S_max * nkv * max_splits_cap * G * HEAD_DIM);
     part_ml.alloc((size_t)S_max * nkv * max_splits_cap * G * 2);
@@ -3319,6 +3321,10 @@ struct tgis_engine {
     // on chip): o-proj -> [post-attention norm] -> gate_up and down-proj -> [next layer's input norm] -> qkv
     const bool norm_fused = !pnx_on && !lora && fuse_norm && tp == 1 && !cfg.debug_gemm_ref && T <= GEMM_NORM_MAX_T && H % 128 == 0 && H / 128 <= GEMM_NORM_MAX_PARTS &&
                             gemm_cluster_split(T, H, q_dim, num_sms) > 0 && gemm_cluster_split(T, H, F, num_sms) > 0;
+    // ... and between the register products of a small model's steps of a few tokens
+    const bool skinny_norm = !pnx_on && !opt && !lora && !norm_fused && tp == 1 && !cfg.debug_gemm_ref && !profiling && gemm_skinny_norm_takes(T, H, q_dim, qkv_dim, F);
+    float* ssq_o = skinny_ssq.p;                                       // left by the o and by the down projection
+    float* ssq_d = skinny_ssq.p + (size_t)8 * (H / 8);
     const int n_parts = H / 128;
     float* ssq_attn = norm_ssq.p;                                      // written by o-proj, read by gate_up
     float* ssq_mlp = norm_ssq.p + (size_t)GEMM_NORM_MAX_T * n_parts;   // written by down-proj, read by the next qkv
@@ -3334,7 +3340,8 @@ struct tgis_engine {
         if (li == 0) {
           CK(rmsnorm_launch(resid.p, l.ln1, xn.p, T, H, c.rms_eps, stream));
           ++n_launches;
-        } else if (qkv_norm_in) {
+        } else if (skinny_norm || qkv_norm_in) {
+          // (skinny_norm: the stream and the sums of its squares are there, the qkv product normalises)
           // the previous layer's down-proj left h in resid and sum(h^2) in ssq_mlp; the qkv GEMM normalises on the fly
         } else if (ar_fused) {
           fused_ar_norm(1, l.ln1, T);  // previous layer's down-proj partials
@@ -3354,8 +3361,13 @@ struct tgis_engine {
           g.mod[2] = LoraModule{ll.A_v, ll.B_v, H, kvd, LR, q_dim + kvd, 2 * LR};
           lora_shrink(g, xn.p, H);
         }
-        gemm(qkv_norm_in ? xm_resid : xm_xn, l.m_qkv, xn.p, l.wqkv, qkv.p, T, qkv_dim, H, 0, &l.m_o, T, H, q_dim, 0,
-             rope_fused ? &rp : nullptr, qkv_norm_in ? &cons_qkv : nullptr);
+        if (skinny_norm && li > 0) {
+          CK(gemm_skinny_norm_launch(resid.p, ssq_d, l.ln1, c.rms_eps, l.wqkv, qkv.p, qkv_dim, T, qkv_dim, H, 0, rope_fused ? &rp : nullptr, stream));
+          ++n_launches;
+        } else {
+          gemm(qkv_norm_in ? xm_resid : xm_xn, l.m_qkv, xn.p, l.wqkv, qkv.p, T, qkv_dim, H, 0, &l.m_o, T, H, q_dim, 0,
+               rope_fused ? &rp : nullptr, qkv_norm_in ? &cons_qkv : nullptr);
+        }
         if (lora) lora_expand(g, qkv.p, qkv_dim);
       }
       bf16* kc = k_cache.p + (size_t)li * kv_layer_elems;
@@ -3378,6 +3390,18 @@ struct tgis_engine {
         ++n_launches;
       }
       if (lora) lora_shrink(lora_one(lora_layers[li].A_o, lora_layers[li].B_o, q_dim, H, LR), attn_out.p, q_dim);
+      if (skinny_norm) {   // o projection, norm, gate and up projection in two launches
+        CK(gemm_skinny_add_launch(attn_out.p, l.wo, resid.p, ssq_o, T, H, q_dim, stream));
+        CK(gemm_skinny_norm_launch(resid.p, ssq_o, l.ln2, c.rms_eps, l.wgu, act.p, F, T, 2 * F, H, 2, nullptr, stream));
+        n_launches += 2;
+        if (li + 1 < c.n_layers) {
+          CK(gemm_skinny_add_launch(act.p, l.wd, resid.p, ssq_d, T, H, F, stream));
+          ++n_launches;
+        } else {
+          gemm(xm_act, l.m_d, act.p, l.wd, tmp.p, T, H, F, 0, R > 0 ? &m_lm : nullptr, R, Vl, H);
+        }
+        continue;
+      }
       gemm(xm_attn, l.m_o, attn_out.p, l.wo, ar_fused ? ar_buf(0) : tmp.p, T, H, q_dim, 0, &l.m_gu, T, 2 * F, H, 0, nullptr,
            norm_fused ? &prod_attn : nullptr);
       if (lora) lora_expand(lora_one(lora_layers[li].A_o, lora_layers[li].B_o, q_dim, H, LR), tmp.p, H);

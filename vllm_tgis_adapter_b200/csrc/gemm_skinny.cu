@@ -33,6 +33,20 @@ struct SkinnyBatch : SkinnyArgs {
   int scale_ld;
 };
 
+// Y goes into the residual stream, resid[t] = bf16(bf16(Y[t]) + resid[t]), and every eight columns of it leave the sum of their squares:
+// the number with which a thread of rmsnorm_kernel enters its reduction.
+struct SkinnyAdd : SkinnyArgs {
+  __nv_bfloat16* resid;
+  float* ssq;                    // [T][N / 8]
+};
+// X is the residual stream; what is multiplied is its RMS norm, which every CTA makes from those sums in the order of rmsnorm_kernel: the
+// same bits as with a launch of its own.
+struct SkinnyNorm : SkinnyArgs {
+  const float* ssq;              // [T][K / 8]
+  const __nv_bfloat16* w_norm;
+  float eps;
+};
+
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -50,7 +64,8 @@ __device__ __forceinline__ float skinny_glu(int mode, float g, float u) {
 // ROPE (MT = 2): the CTA's two tiles are the dims [16 q, 16 q + 16) of one head and their rotary partners, 64 dims on.
 template <int MT, int NT, int WARPS, bool ROPE, class Args>
 __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_kernel(const Args a) {
-  constexpr bool BATCH = std::is_same<Args, SkinnyBatch>::value;
+  constexpr bool BATCH = std::is_same<Args, SkinnyBatch>::value, ADD = std::is_same<Args, SkinnyAdd>::value, NORM = std::is_same<Args, SkinnyNorm>::value;
+  static_assert(!(ADD || NORM) || (NT == 1 && WARPS >= 8), "a warp per token makes its norm");
   constexpr int R = 16 * MT, TT = 8 * NT, LD = R + 1;
   extern __shared__ __align__(16) float part[];   // [WARPS][TT][LD]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -96,13 +111,60 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_k
         for (int s = 0; s < 2; ++s) wv[m][h][s] = ldg_stream(wr[m][h] + c * 64 + s * 32);
   };
   if (warp < chunks) load_w(warp);   // (weights are static)
+  uint4 nw[2], x0[2];                // NORM: the norm's weights of a chunk, the first chunk of X
+  float rs = 0.f;                    // ... and 1 / rms of the lane's token
+  if constexpr (NORM) {
+#pragma unroll
+    for (int s = 0; s < 2; ++s) nw[s] = warp < chunks ? *reinterpret_cast<const uint4*>(a.w_norm + warp * 64 + s * 32 + t * 8) : make_uint4(0, 0, 0, 0);
+  }
   griddep_wait();
+  if constexpr (NORM) {
+    __shared__ float rs_s[8];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) x0[s] = warp < chunks ? *reinterpret_cast<const uint4*>(xr[0] + warp * 64 + s * 32) : make_uint4(0, 0, 0, 0);
+    if (warp < a.T) {
+      const int np = a.K / 8;
+      float v[8], tot = 0.f;   // 256 threads of eight columns: eight warps' sums, then theirs
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = q * 32 + lane < np ? a.ssq[(size_t)warp * np + q * 32 + lane] : 0.f;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) tot = lane == q ? v[q] : tot;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+      if (lane == 0) rs_s[warp] = rsqrtf(tot / (float)a.K + a.eps);
+    }
+    __syncthreads();
+    rs = rs_s[min(g, a.T - 1)];
+  }
   for (int c = warp; c < chunks; c += WARPS) {
     uint4 xv[NT][2], wc[MT][2][2];
 #pragma unroll
     for (int n = 0; n < NT; ++n)
 #pragma unroll
-      for (int s = 0; s < 2; ++s) xv[n][s] = *reinterpret_cast<const uint4*>(xr[n] + c * 64 + s * 32);
+      for (int s = 0; s < 2; ++s) {
+        if constexpr (NORM) {
+          if (c != warp) {
+            x0[s] = *reinterpret_cast<const uint4*>(xr[n] + c * 64 + s * 32);
+            nw[s] = *reinterpret_cast<const uint4*>(a.w_norm + c * 64 + s * 32 + t * 8);
+          }
+          const uint32_t xs[4] = {x0[s].x, x0[s].y, x0[s].z, x0[s].w}, ws[4] = {nw[s].x, nw[s].y, nw[s].z, nw[s].w};
+          uint32_t o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float lo = bf16_round(__uint_as_float(xs[e] << 16) * rs) * __uint_as_float(ws[e] << 16);
+            const float hi = bf16_round(__uint_as_float(xs[e] & 0xffff0000u) * rs) * __uint_as_float(ws[e] & 0xffff0000u);
+            const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+            o[e] = *reinterpret_cast<const uint32_t*>(&p);
+          }
+          xv[n][s] = make_uint4(o[0], o[1], o[2], o[3]);
+        } else {
+          xv[n][s] = *reinterpret_cast<const uint4*>(xr[n] + c * 64 + s * 32);
+        }
+      }
 #pragma unroll
     for (int m = 0; m < MT; ++m)
 #pragma unroll
@@ -136,7 +198,26 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 16 ? 1 : 2) gemm_skinny_k
     return v;
   };
   __nv_bfloat16* __restrict__ Y = reinterpret_cast<__nv_bfloat16*>(a.Y);
-  if constexpr (ROPE) {
+  if constexpr (ADD) {
+    for (int i = threadIdx.x; i < ((a.T * R + 31) & ~31); i += WARPS * 32) {   // (whole warps: eight lanes meet)
+      const int tok = i / R, j = i % R;
+      const bool in = tok < a.T && n0 + j < a.N;
+      __nv_bfloat16* r = a.resid + (size_t)tok * a.N + n0 + j;
+      float z = 0.f;
+      if (in) {
+        const __nv_bfloat16 v = __float2bfloat16_rn(bf16_round(sum(tok, j)) + __bfloat162float(*r));
+        *r = v;
+        z = __bfloat162float(v);
+      }
+      float ss = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float f = __shfl_sync(0xffffffffu, z, (lane & ~7) + e);
+        ss = fmaf(f, f, ss);
+      }
+      if (in && (j & 7) == 0) a.ssq[(size_t)tok * (a.N / 8) + (n0 + j) / 8] = ss;
+    }
+  } else if constexpr (ROPE) {
     // rotary embedding and the scatter into the paged cache (arithmetic and rounding points of rope_kvwrite_kernel)
     const int head = n0 / HEAD_DIM, d0 = n0 % HEAD_DIM;
     for (int i = threadIdx.x; i < a.T * 16; i += WARPS * 32) {
@@ -239,6 +320,32 @@ cudaError_t gemm_skinny_launch(const void* X, const void* W, void* Y, int ldy, i
   }
   if (!sixteen) return T <= 8 ? launch<2, 1, 8, false>(a, stream) : launch_nt<1, 8, false>(a, stream);
   return N > SKINNY_ONE_WAVE ? launch_nt<2, 16, false>(a, stream) : launch_nt<1, 16, false>(a, stream);
+}
+
+// Norms between the products of a small model's decode steps, for up to eight tokens: the product in front adds to the residual stream and
+// leaves sums of squares, the one behind normalises its rows as it loads them.  In a chain a launch of its own costs 0.45 us more (12
+// layers 768 wide, one request, 17 + 16 tokens: 4.34 -> 4.17 ms).  Every CTA reading the whole row and norming it over again had been slower
+// than that launch (6.9 us against 4.0 + 2.0): it had a row to wait for and to sum; here it has three numbers a lane.
+bool gemm_skinny_norm_takes(int T, int hidden, int q_dim, int qkv_dim, int ffn) {
+  return T >= 1 && T <= 8 && hidden % 8 == 0 && hidden <= 2048 &&   // (2048: one vector a thread of rmsnorm_kernel)
+         gemm_skinny_takes(T, qkv_dim, hidden) && gemm_skinny_takes(T, hidden, q_dim) && gemm_skinny_takes(T, 2 * ffn, hidden) && gemm_skinny_takes(T, hidden, ffn);
+}
+cudaError_t gemm_skinny_add_launch(const void* X, const void* W, __nv_bfloat16* resid, float* ssq, int T, int N, int K, cudaStream_t stream) {
+  if (T < 1 || T > 8 || N % 8 != 0 || N > SKINNY_ONE_WAVE || !gemm_skinny_takes(T, N, K)) return cudaErrorInvalidValue;
+  const SkinnyAdd a{{(const __nv_bfloat16*)X, (const __nv_bfloat16*)W, nullptr, N, T, N, K, 0, {}}, resid, ssq};
+  return launch<1, 1, 16, false>(a, stream);
+}
+cudaError_t gemm_skinny_norm_launch(const void* h, const float* ssq, const __nv_bfloat16* w_norm, float eps, const void* W, void* Y, int ldy, int T, int N, int K,
+                                    int out_mode, const GemmRope* rope, cudaStream_t stream) {
+  if (T < 1 || T > 8 || K > 2048 || !gemm_skinny_takes(T, N, K)) return cudaErrorInvalidValue;
+  SkinnyNorm a{{(const __nv_bfloat16*)h, (const __nv_bfloat16*)W, Y, ldy, T, N, K, out_mode, {}}, ssq, w_norm, eps};
+  const bool sixteen = N <= 2 * SKINNY_ONE_WAVE;   // (as above)
+  if (rope != nullptr) {
+    a.rope = *rope;
+    return sixteen ? launch<2, 1, 16, true>(a, stream) : launch<2, 1, 8, true>(a, stream);
+  }
+  if (!sixteen) return launch<2, 1, 8, false>(a, stream);
+  return N > SKINNY_ONE_WAVE ? launch<2, 1, 16, false>(a, stream) : launch<1, 1, 16, false>(a, stream);
 }
 
 // One product per head (the up-projections that latent attention folds into queries and outputs), up to 32 tokens: grid (16 weight

@@ -145,6 +145,12 @@ int gemm_pair_fault(int nth);
 bool gemm_skinny_takes(int T, int N, int K);
 cudaError_t gemm_skinny_launch(const void* X, const void* W, void* Y, int ldy, int T, int N, int K, int out_mode, const GemmRope* rope,
                                cudaStream_t stream);
+// Norms inside the products of a decode step of up to eight tokens (all pointers on 16 bytes): resid += X W^T and sums of squares
+// [T][N / 8]; Y = rmsnorm(h) W^T from such sums.  The bits are those of gemm_skinny_launch and add_rmsnorm_launch.
+bool gemm_skinny_norm_takes(int T, int hidden, int q_dim, int qkv_dim, int ffn);
+cudaError_t gemm_skinny_add_launch(const void* X, const void* W, __nv_bfloat16* resid, float* ssq, int T, int N, int K, cudaStream_t stream);
+cudaError_t gemm_skinny_norm_launch(const void* h, const float* ssq, const __nv_bfloat16* w_norm, float eps, const void* W, void* Y, int ldy, int T, int N, int K,
+                                    int out_mode, const GemmRope* rope, cudaStream_t stream);
 
 // ---- gemm_ref.cu (debug cross-check only; never on the product path) ---------------------------------------------
 cudaError_t gemm_bf16_ref_launch(const __nv_bfloat16* X, int ldx, const __nv_bfloat16* W, void* Y, int ldy, int T,

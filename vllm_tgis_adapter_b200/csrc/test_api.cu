@@ -217,6 +217,29 @@ int tgis_k_gemm_rope(const void* x_dev, const void* w_dev, void* y_dev, int32_t 
   return product_end();
 }
 
+// resid += a w1^T, norm, y2 = norm(resid) w2^T by the register products of a few tokens: with the norm inside them (fused) or as a launch
+// of its own; 1: not products that it goes with
+int tgis_k_skinny_norm_chain(const void* a, const void* w1, void* resid, const void* w_norm, const void* w2, void* y2, int32_t T, int32_t K1, int32_t H,
+                             int32_t N2, float eps, int32_t out_mode2, int32_t fused) {
+  if (!gemm_skinny_norm_takes(T, H, K1, N2, 64)) return 1;
+  const int ldy = out_mode2 == 2 || out_mode2 == 3 ? N2 / 2 : N2;
+  Tmp<bf16> y1, xn;
+  Tmp<float> ssq;
+  KCK(y1.alloc((size_t)T * H));
+  KCK(xn.alloc((size_t)T * H));
+  KCK(ssq.alloc((size_t)T * (H / 8)));
+  if (fused) {
+    KCK(gemm_skinny_add_launch(a, w1, (bf16*)resid, ssq.p, T, H, K1, 0));
+    KCK(gemm_skinny_norm_launch(resid, ssq.p, (const bf16*)w_norm, eps, w2, y2, ldy, T, N2, H, out_mode2, nullptr, 0));
+  } else {
+    KCK(gemm_skinny_launch(a, w1, y1.p, H, T, H, K1, 0, nullptr, 0));
+    KCK(add_rmsnorm_launch(y1.p, (bf16*)resid, (const bf16*)w_norm, xn.p, T, H, eps, 0));
+    KCK(gemm_skinny_launch(xn.p, w2, y2, ldy, T, N2, H, out_mode2, nullptr, 0));
+  }
+  KCK(cudaDeviceSynchronize());
+  return 0;
+}
+
 // Layer-stack slice  a -> [GEMM W1] -> (+ residual, RMSNorm w_norm) -> [GEMM W2 (out_mode2: 0 bf16, 2 fused SwiGLU)] -> y2
 // run either as three launches (fused = 0: gemm, add_rmsnorm_launch, gemm) or as two with the add + norm folded into the
 // two GEMMs (fused = 1, GemmNorm).  residual [T, H] is updated in place either way.  Returns 1 when the launch plan cannot
