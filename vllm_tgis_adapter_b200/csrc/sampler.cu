@@ -9,16 +9,23 @@
 // Contract order per row: raw log-softmax -> typical-p -> ExpDecay(EOS) -> min_tokens(EOS)
 // -> repetition penalty -> greedy argmax | temperature -> top-k -> top-p -> sample -> logprob / rank / top-n (raw).
 //
-// Shape of the problem: a [rows, V=128256] scan with integer-ish selection work; a sampling row needs ~10 passes of
-// 50-100 instructions per element, which is ISSUE bound on one SM (1 ms per row).  So a row is owned by a thread-block
-// CLUSTER of 8 CTAs x 1024 threads on 8 SMs: each CTA scans one eighth of the vocabulary, block results are exchanged
-// through distributed shared memory and combined in rank order (deterministic).  The fp32 row (512 KiB) is read from
-// HBM once and stays in the 126 MB L2 for the selection passes (radix-select thresholds instead of the reference's
-// full sorts).  Every sweep takes eight entries per thread and 16-byte load; a row's sweeps: the first (max, sum, greedy argmax),
-// entropy and four radix rounds behind typical-p, processed maximum, race, and one for rank and top-n together.
-// Measured, 128256 bf16 logits, microseconds, scalar sweeps with one sweep per top-n entry -> here: greedy with top-5 36 -> 22 (32
-// rows), 97 -> 38 (96 rows); typical-p with penalties 88 -> 62, 350 -> 160 (flat rows 679 -> 287); top-k and top-p 101 -> 86, 442 -> 246.
+// Shape of the problem: a [rows, V=128256] scan with integer-ish selection work; a sampling row needs several passes of
+// 50-100 instructions per element, which is ISSUE bound on one SM.  So a row is owned by a thread-block CLUSTER of up to 8 CTAs x
+// 1024 threads: each scans its part of the vocabulary, block results are exchanged through distributed shared memory and combined
+// in a fixed order (deterministic).  The row is read from HBM once and stays in shared memory or the L2 for the selection passes
+// (radix-select thresholds instead of the reference's full sorts).  Every sweep takes eight entries per thread and 16-byte load.
+//   first sweep   32 entries a thread at a time: their maximum, then exponentials that do not wait for one another (an online
+//                 maximum per entry was a chain of a branch and an exponential each: 9100 of a greedy row's 27000 cycles); behind
+//                 typical-p the entropy's sum too
+//   reductions    maximum, sums and best entry in one; an exchange is one 16-byte read per lane and shuffles
+//   typical-p     three radix rounds and a fourth over the few entries that share sixteen bits; the race over what is left
+//   rank, top-n   one sweep and one exchange, the slices' lists ordered by eight threads a candidate
+// Measured, 128256 bf16 logits with top-5, microseconds, with the online maximum, an exchange for each part and clusters by SM count ->
+// here: greedy 19.7 -> 17.3 (1 row), 39 -> 17 (16), 22 -> 18 (32), 38 -> 29 (96), 73 -> 55 (150); typical-p 45 -> 38 (1), 88 -> 48 (16),
+// 91 -> 74 (64), 157 -> 124 (96), 309 -> 240 (150); flat rows 63 -> 58, 285 -> 263; top-k with top-p 63 -> 59 (1), 240 -> 214 (96).
 #include <cooperative_groups.h>
+
+#include <algorithm>
 
 #include "kernels.h"
 #include "launch.cuh"
@@ -30,7 +37,7 @@ namespace tgis {
 
 TGIS_STL_DEFINE(sampler)
 
-constexpr int SAMP_MAX_CL = 8;  // CTAs (SMs) per row: 1, 2, 4 or 8, chosen per launch (sampler_launch)
+constexpr int SAMP_MAX_CL = 8;  // CTAs (SMs) per row: 1, 2, 4 or 8, chosen per launch (sampler_cluster_size)
 constexpr int SAMP_THREADS = 1024;
 constexpr int SAMP_WARPS = SAMP_THREADS / 32;
 constexpr int SAMP_LIST = SAMP_THREADS;
@@ -143,36 +150,16 @@ __device__ __forceinline__ void process8(const RowCtx<LT>& c, int i0, float (&v)
   }
 }
 
-// ---------------------------------------------------------------- block reductions (1024 threads, result in every thread)
+// ---------------------------------------------------------------- block reductions (result in every thread)
+// maximum m, sum of e^(x - m) and, for the entropy, sum of (x - m) e^(x - m)
 struct MaxSum {
-  float m, s;
+  float m, s, w;
 };
-__device__ __forceinline__ MaxSum ms_combine(MaxSum a, MaxSum b) {
-  if (a.m == -INFINITY) return b;
-  if (b.m == -INFINITY) return a;
-  const float m = fmaxf(a.m, b.m);
-  return {m, a.s * __expf(a.m - m) + b.s * __expf(b.m - m)};
-}
-__device__ MaxSum block_maxsum(MaxSum v, float* red /*[2*SAMP_WARPS]*/) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    MaxSum t{__shfl_xor_sync(0xffffffffu, v.m, o), __shfl_xor_sync(0xffffffffu, v.s, o)};
-    v = ms_combine(v, t);
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) {
-    red[2 * w] = v.m;
-    red[2 * w + 1] = v.s;
-  }
-  __syncthreads();
-  MaxSum r{red[2 * l], red[2 * l + 1]};
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    MaxSum t{__shfl_xor_sync(0xffffffffu, r.m, o), __shfl_xor_sync(0xffffffffu, r.s, o)};
-    r = ms_combine(r, t);
-  }
-  return r;
+// ... as they are against a larger maximum
+__device__ __forceinline__ MaxSum ms_against(MaxSum t, float m) {
+  if (t.m == -INFINITY) return {m, 0.f, 0.f};
+  const float d = t.m - m, f = expf(d);
+  return {m, t.s * f, f * (t.w + d * t.s)};
 }
 // argmax with lowest-index tie break (torch.argmax semantics relied on by greedy parity)
 struct ValIdx {
@@ -203,6 +190,38 @@ __device__ ValIdx block_argmax(ValIdx v, float* redf, int* redi) {
   }
   __syncthreads();
   return warp_argmax(ValIdx{redf[l], redi[l]});
+}
+// these together with the best entry: every sum is brought to its warp's and then to the block's maximum once
+struct MaxSumBest {
+  MaxSum ms;
+  ValIdx best;
+};
+__device__ __forceinline__ MaxSumBest warp_maxsum_best(MaxSumBest t) {
+  float m = t.ms.m;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  t.ms = ms_against(t.ms, m);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    t.ms.s += __shfl_xor_sync(0xffffffffu, t.ms.s, o);
+    t.ms.w += __shfl_xor_sync(0xffffffffu, t.ms.w, o);
+    const ValIdx b{__shfl_xor_sync(0xffffffffu, t.best.v, o), __shfl_xor_sync(0xffffffffu, t.best.i, o)};
+    t.best = vi_better(t.best, b);
+  }
+  return t;
+}
+struct RedBest {
+  float m, s, w, v;
+  int i;
+};
+__device__ __forceinline__ MaxSumBest block_maxsum_best(MaxSumBest t, RedBest* red /*[SAMP_WARPS]*/) {
+  t = warp_maxsum_best(t);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) red[w] = RedBest{t.ms.m, t.ms.s, t.ms.w, t.best.v, t.best.i};
+  __syncthreads();
+  static_assert(SAMP_WARPS == 32, "a lane per warp");
+  const RedBest r = red[l];
+  return warp_maxsum_best(MaxSumBest{{r.m, r.s, r.w}, {r.v, r.i}});
 }
 __device__ float block_sumf(float v, float* red) {
 #pragma unroll
@@ -249,40 +268,38 @@ __device__ __forceinline__ T dsmem_read(const Cl& c, T* local, int rank) {
 struct Xch4 {
   float a, b, c, d;
 };
-// publish this CTA's 4 words (already block-reduced: every thread holds them) and return a functor-friendly snapshot
-// of all ranks' words through `get(r)`
+// publish this CTA's words (already block-reduced: every thread holds them); lane r of every warp then holds those of rank r
 struct XchView {
-  const Cl* cl;
-  float* slot;
+  float4 mine;
   __device__ Xch4 get(int r) const {
-    return Xch4{dsmem_read(*cl, slot, r), dsmem_read(*cl, slot + 1, r), dsmem_read(*cl, slot + 2, r),
-                dsmem_read(*cl, slot + 3, r)};
+    return Xch4{__shfl_sync(0xffffffffu, mine.x, r), __shfl_sync(0xffffffffu, mine.y, r), __shfl_sync(0xffffffffu, mine.z, r),
+                __shfl_sync(0xffffffffu, mine.w, r)};
   }
 };
-__device__ XchView cl_publish(Cl& c, float (*xch)[4], Xch4 v) {
-  float* slot = xch[c.xe & 1];
+__device__ XchView cl_publish(Cl& c, float4* xch, Xch4 v) {
+  float4* slot = xch + (c.xe & 1);
   ++c.xe;
-  if (threadIdx.x == 0) {
-    slot[0] = v.a;
-    slot[1] = v.b;
-    slot[2] = v.c;
-    slot[3] = v.d;
-  }
+  if (threadIdx.x == 0) *slot = make_float4(v.a, v.b, v.c, v.d);
   c.sync();
-  return XchView{&c, slot};
+  const int lane = threadIdx.x & 31;
+  return XchView{dsmem_read(c, slot, lane < c.ncl ? lane : 0)};
 }
-__device__ MaxSum cluster_maxsum(Cl& c, MaxSum v, float* red, float (*xch)[4]) {
-  v = block_maxsum(v, red);
-  const XchView w = cl_publish(c, xch, Xch4{v.m, v.s, 0.f, 0.f});
-  Xch4 t = w.get(0);
-  MaxSum acc{t.a, t.b};
-  for (int r = 1; r < c.ncl; ++r) {
-    t = w.get(r);
-    acc = ms_combine(acc, MaxSum{t.a, t.b});
-  }
-  return acc;
+__device__ float cluster_max(Cl& c, float v, float* red, float4* xch) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  __syncthreads();
+  if (l == 0) red[w] = v;
+  __syncthreads();
+  float m = red[l];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  m = cl_publish(c, xch, Xch4{m, 0.f, 0.f, 0.f}).mine.x;   // (lanes behind the last rank repeat rank 0)
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  return m;
 }
-__device__ ValIdx cluster_argmax(Cl& c, ValIdx v, float* redf, int* redi, float (*xch)[4]) {
+__device__ ValIdx cluster_argmax(Cl& c, ValIdx v, float* redf, int* redi, float4* xch) {
   v = block_argmax(v, redf, redi);
   const XchView w = cl_publish(c, xch, Xch4{v.v, __int_as_float(v.i), 0.f, 0.f});
   Xch4 t = w.get(0);
@@ -293,14 +310,14 @@ __device__ ValIdx cluster_argmax(Cl& c, ValIdx v, float* redf, int* redi, float 
   }
   return acc;
 }
-__device__ float cluster_sumf(Cl& c, float v, float* red, float (*xch)[4]) {
+__device__ float cluster_sumf(Cl& c, float v, float* red, float4* xch) {
   v = block_sumf(v, red);
   const XchView w = cl_publish(c, xch, Xch4{v, 0.f, 0.f, 0.f});
   float acc = w.get(0).a;
   for (int r = 1; r < c.ncl; ++r) acc += w.get(r).a;
   return acc;
 }
-__device__ int cluster_sumi(Cl& c, int v, int* red, float (*xch)[4]) {
+__device__ int cluster_sumi(Cl& c, int v, int* red, float4* xch) {
   v = block_sumi(v, red);
   const XchView w = cl_publish(c, xch, Xch4{__int_as_float(v), 0.f, 0.f, 0.f});
   int acc = 0;
@@ -419,7 +436,7 @@ __device__ __forceinline__ void hist_add8(uint32_t* h, const uint32_t (&digit)[8
 }
 // a round's histogram: all copies to zero / their sum in the first
 __device__ __forceinline__ void hist_clear(uint32_t* h) {
-  if (threadIdx.x < 256 * HIST_COPIES) h[threadIdx.x] = 0u;
+  for (int i = threadIdx.x; i < 256 * HIST_COPIES; i += SAMP_THREADS) h[i] = 0u;
   __syncthreads();
 }
 __device__ __forceinline__ void hist_fold(uint32_t* h) {
@@ -440,7 +457,7 @@ __device__ __forceinline__ void hist_fold(uint32_t* h) {
 // 4 rounds of 8 bits; every CTA histograms its slice, the cluster sums them, every CTA runs the same scan.
 template <class LoadF, class KeyF, class WF>
 __device__ uint32_t select_weighted_asc(Cl& c, int lo, int hi, LoadF load, KeyF keyf, WF wf, float target, bool strict,
-                                        uint32_t (*hist)[256 * HIST_COPIES], uint32_t* hsum, uint32_t* bcast) {
+                                        uint32_t (*hist)[256 * HIST_COPIES], uint32_t* hsum, uint32_t* bcast, float* few, int* n_few) {
   const uint32_t T = __float2uint_rn(fminf(fmaxf(target, 0.f), 2.f) * SAMP_FIX);
   uint32_t prefix = 0, below = 0;
   for (int round = 0; round < 4; ++round) {
@@ -448,22 +465,38 @@ __device__ uint32_t select_weighted_asc(Cl& c, int lo, int hi, LoadF load, KeyF 
     uint32_t* h = hist[c.he & 1];
     ++c.he;
     hist_clear(h);
-    for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
-      const int i0 = base + threadIdx.x * 8;
-      uint32_t digit[8], w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (i0 < hi) {
-        float v[8];
-        load(i0, v);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          // after the first round only ~1/256 of the entries still carry the selected prefix: test the (cheap) key first
-          // and evaluate the weight (an expf) for those only
-          const uint32_t k = keyf(v[e]);
-          digit[e] = (k >> shift) & 255;
-          if (round == 0 || (k >> (shift + 8)) == (prefix >> (shift + 8))) w[e] = __float2uint_rn(wf(v[e]) * SAMP_FIX);
-        }
+    if (round == 2 && threadIdx.x == 0) *n_few = 0;
+    if (round == 2) __syncthreads();
+    if (round == 3 && *n_few <= SAMP_LIST) {   // the entries that shared sixteen bits were listed in the round before
+      for (int i = threadIdx.x; i < *n_few; i += SAMP_THREADS) {
+        const uint32_t k = keyf(few[i]);
+        if ((k >> 8) == (prefix >> 8)) atomicAdd(&h[k & 255], __float2uint_rn(wf(few[i]) * SAMP_FIX));
       }
-      hist_add8(h, digit, w);
+    } else {
+      for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
+        const int i0 = base + threadIdx.x * 8;
+        uint32_t digit[8], w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (i0 < hi) {
+          const bool listing = round == 2 && *n_few <= SAMP_LIST;
+          float v[8];
+          load(i0, v);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            // after the first round only ~1/256 of the entries still carry the selected prefix: test the (cheap) key first
+            // and evaluate the weight (an expf) for those only
+            const uint32_t k = keyf(v[e]);
+            digit[e] = (k >> shift) & 255;
+            if (round == 0 || (k >> (shift + 8)) == (prefix >> (shift + 8))) {
+              w[e] = __float2uint_rn(wf(v[e]) * SAMP_FIX);
+              if (listing) {
+                const int at = atomicAdd(n_few, 1);
+                if (at < SAMP_LIST) few[at] = v[e];
+              }
+            }
+          }
+        }
+        hist_add8(h, digit, w);
+      }
     }
     hist_fold(h);
     radix_round_pick(c, h, hsum, bcast, below, T, strict, /*descending=*/false);
@@ -538,17 +571,16 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
   __shared__ uint32_t hist[2][256 * HIST_COPIES];
   __shared__ uint32_t hsum[256];
   __shared__ uint32_t bcast[4];
-  __shared__ float xch[2][4];
+  __shared__ float4 xch[2];
+  __shared__ RedBest redb[SAMP_WARPS];
+  __shared__ float wmax[SAMP_WARPS];    // of the slice's raw entries, by warp
   __shared__ float cand_v[MAX_TOPN];
   __shared__ int cand_i[MAX_TOPN];
-  __shared__ float list_v[SAMP_LIST];   // thread maxima, then the entries that can be among the slice's top-n
+  __shared__ float list_v[SAMP_LIST];   // in turn: a weighted selection's last candidates, what the race is run over, what can be among the top-n, the slices' best
   __shared__ int list_i[SAMP_LIST];
   __shared__ int list_n;
   STL_ENTER(6);
   griddep_launch();
-  griddep_wait();
-  STL_WAITED();
-
   Cl cl;
   cl.ncl = ncl;
   cl.rank = ncl > 1 ? (int)cg::this_cluster().block_rank() : 0;
@@ -556,7 +588,7 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
   const int r = blockIdx.x / ncl;
   const int crank = cl.rank;
   RowCtx<LT> c;
-  c.p = rows[r];
+  c.p = rows[r];   // (written by the host before the step)
   c.V = V;
   {
     const int per = ((V + ncl - 1) / ncl + 7) / 8 * 8;
@@ -582,23 +614,39 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
   float* y = cache_y ? reinterpret_cast<float*>(dyn_smem + (cache_x ? (size_t)per_cta * sizeof(LT) : 0)) - lo
                      : scratch + (size_t)r * V;
 
+  griddep_wait();
+  STL_WAITED();
+
   // ---- pass 1: raw max / sum-exp (+ greedy argmax of the processed logits in the same sweep); the slice is staged in
   // shared memory on the way when it fits
-  MaxSum ms{-INFINITY, 0.f};
+  MaxSum ms{-INFINITY, 0.f, 0.f};
   ValIdx best{-INFINITY, -1};
   const bool do_typ = (c.p.flags & SAMPLE_TYPICAL) != 0 && !forced;
   const bool greedy_fast = greedy && !do_typ;  // argmax fused into the first sweep
+  // a batch of entries at once: their maximum, then exponentials that do not wait for one another
+  auto batch_max = [&](float m) {
+    if (m > ms.m) ms = ms_against(ms, m);
+  };
   auto consume8 = [&](float (&xs)[8], int i0) {
+    float s0 = 0.f, s1 = 0.f;
+    if (ms.m == -INFINITY) {   // (nothing allowed so far)
+    } else if (do_typ) {
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float x = xs[e];
-      if (x > ms.m) {
-        ms.s = ms.s * __expf(ms.m - x) + 1.f;
-        ms.m = x;
-      } else if (x != -INFINITY) {
-        ms.s += __expf(x - ms.m);
+      for (int e = 0; e < 8; ++e) {
+        const float d = xs[e] - ms.m, p = expf(d);
+        s0 += p;
+        s1 += d == -INFINITY ? 0.f : d * p;
       }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; e += 2) {
+        s0 += __expf(xs[e] - ms.m);
+        s1 += __expf(xs[e + 1] - ms.m);
+      }
+      s0 += s1;
     }
+    ms.s += s0;
+    if (do_typ) ms.w += s1;
     if (greedy_fast) {
       process8(c, i0, xs);
 #pragma unroll
@@ -614,6 +662,7 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
       const int iu = i0 + u * SAMP_THREADS * 8;
       if (iu < hi) load_x8(c.x, iu, xv[u]);
     }
+    float m = -INFINITY;
 #pragma unroll
     for (int u = 0; u < P1_UNROLL; ++u) {
       const int iu = i0 + u * SAMP_THREADS * 8;
@@ -625,50 +674,42 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
             if (!((bits >> e) & 1u)) xv[u][e] = -INFINITY;
         }
         if (cache_x) store_x8(xs + (iu - lo), xv[u]);
-        consume8(xv[u], iu);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) m = fmaxf(m, xv[u][e]);
       }
+    }
+    batch_max(m);
+#pragma unroll
+    for (int u = 0; u < P1_UNROLL; ++u) {
+      const int iu = i0 + u * SAMP_THREADS * 8;
+      if (iu < hi) consume8(xv[u], iu);
     }
   }
   if (cache_x) c.xc = xs;  // visible to every thread after the barriers of the reductions below
-  const float thread_max = ms.m;
+  const int n_topn = min(c.p.n_topn, MAX_TOPN);
+  if (n_topn > 0) {
+    float m = ms.m;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = m;   // (read behind the barriers of the reductions)
+  }
   int token;
-  if (greedy_fast) {
-    // one exchange for both reductions: {max, sum-exp, best value, best index}
-    ms = block_maxsum(ms, redf);
-    best = block_argmax(best, redf, redi);
-    const XchView w = cl_publish(cl, xch, Xch4{ms.m, ms.s, best.v, __int_as_float(best.i)});
-    Xch4 t = w.get(0);
-    MaxSum am{t.a, t.b};
-    ValIdx ab{t.c, __float_as_int(t.d)};
-    for (int q = 1; q < ncl; ++q) {
-      t = w.get(q);
-      am = ms_combine(am, MaxSum{t.a, t.b});
-      ab = vi_better(ab, ValIdx{t.c, __float_as_int(t.d)});
-    }
-    ms = am;
-    token = ab.i;
-  } else {
-    ms = cluster_maxsum(cl, ms, redf, xch);
-    token = -1;
+  {
+    // one exchange for all of it: {max, sum-exp, best value, best index}, or {max, sum-exp, the entropy's sum}
+    const MaxSumBest t = block_maxsum_best(MaxSumBest{ms, best}, redb);
+    const XchView w = cl_publish(cl, xch, Xch4{t.ms.m, t.ms.s, greedy_fast ? t.best.v : t.ms.w, __int_as_float(t.best.i)});
+    const bool in = (int)(threadIdx.x & 31) < ncl;
+    const MaxSumBest all = warp_maxsum_best(MaxSumBest{{in ? w.mine.x : -INFINITY, in ? w.mine.y : 0.f, in && !greedy_fast ? w.mine.z : 0.f},
+                                                       {in && greedy_fast ? w.mine.z : -INFINITY, in && greedy_fast ? __float_as_int(w.mine.w) : -1}});
+    ms = all.ms;
+    token = all.best.i;
   }
   c.raw_max = ms.m;
   c.raw_logz = logf(ms.s);
 
   // ---- typical-p threshold (R8): entropy, then weighted select over s = |-lp - H| ascending
   if (do_typ) {
-    float part = 0.f;
-    for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
-      float x[8];
-      load_slice8(c, i0, x);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float lp = (x[e] - c.raw_max) - c.raw_logz;
-        const float p = expf(lp);
-        const float term = lp * p;
-        if (term == term) part += term;  // nansum
-      }
-    }
-    c.ent = -cluster_sumf(cl, part, redf, xch);
+    c.ent = c.raw_logz - ms.w / ms.s;   // -sum p log p with log p = (x - max) - log z
     const float rm = c.raw_max, lz = c.raw_logz, ent = c.ent;
     const RowCtx<LT>& cr = c;
     auto load = [&cr](int i0, float (&v)[8]) { load_slice8(cr, i0, v); };
@@ -677,7 +718,7 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
       return __float_as_uint(fabsf((-lp) - ent));
     };
     auto wf = [=](float x) { return expf((x - rm) - lz); };
-    const uint32_t k = select_weighted_asc(cl, lo, hi, load, keyf, wf, c.p.typical_p, false, hist, hsum, bcast);
+    const uint32_t k = select_weighted_asc(cl, lo, hi, load, keyf, wf, c.p.typical_p, false, hist, hsum, bcast, list_v, &list_n);
     c.typ_thr = __uint_as_float(k);
     c.typical = true;
   }
@@ -710,17 +751,25 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
         if (v[e] != -INFINITY) v[e] = __fdiv_rn(v[e], temp);   // (-inf behind typical-p: the quotient is -inf too)
     };
     auto load_y = [=](int i0, float (&v)[8]) { load_x8(y, i0, v); };
+    if (threadIdx.x == 0) list_n = 0;
+    __syncthreads();
     for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
       float v[8];
       scaled8(i0, v);
       if (keep_y) store_x8(y + i0, v);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) mx = fmaxf(mx, v[e]);
+      for (int e = 0; e < 8; ++e) {
+        mx = fmaxf(mx, v[e]);
+        if (!keep_y && v[e] != -INFINITY && list_n <= SAMP_LIST) {   // what typical-p left: mostly a few
+          const int at = atomicAdd(&list_n, 1);
+          if (at < SAMP_LIST) {
+            list_v[at] = v[e];
+            list_i[at] = i0 + e;
+          }
+        }
+      }
     }
-    {
-      MaxSum t = cluster_maxsum(cl, MaxSum{mx, 0.f}, redf, xch);
-      mx = t.m;
-    }
+    mx = cluster_max(cl, mx, redf, xch);
     // ---- top-k (S6): keep y >= k-th largest value
     float lo_thr = -INFINITY;
     if (use_topk) {
@@ -741,24 +790,28 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
       const float lt = lo_thr;
       auto keyf = [](float v) { return f2key(v); };
       auto wf = [=](float v) { return (v >= lt) ? expf(v - mx) / z : 0.f; };
-      const uint32_t k = select_weighted_asc(cl, lo, hi, load_y, keyf, wf, 1.0f - c.p.top_p, true, hist, hsum, bcast);
+      const uint32_t k = select_weighted_asc(cl, lo, hi, load_y, keyf, wf, 1.0f - c.p.top_p, true, hist, hsum, bcast, list_v, &list_n);
       lo_thr = fmaxf(lo_thr, key2f(k));
     }
     // ---- exponential race == Gumbel max over the kept set
     const uint2 key = make_uint2(c.p.seed_lo, c.p.seed_hi);
     ValIdx bs{-INFINITY, -1};
-    for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
-      float v[8];
-      if (keep_y) load_y(i0, v);
-      else scaled8(i0, v);
+    auto race = [&](float v, int i) {
+      const uint4 rnd = philox4x32(make_uint4((uint32_t)i, c.p.step, 0u, 0u), key);
+      const float u = ((float)(rnd.x >> 8) + 0.5f) * (1.0f / 16777216.0f);
+      const float score = (v - mx) - logf(-logf(u));
+      if (bs.i < 0 || score > bs.v) bs = {score, i};
+    };
+    if (!keep_y && list_n <= SAMP_LIST) {
+      if ((int)threadIdx.x < list_n) race(list_v[threadIdx.x], list_i[threadIdx.x]);
+    } else {
+      for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
+        float v[8];
+        if (keep_y) load_y(i0, v);
+        else scaled8(i0, v);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        if (v[e] >= lo_thr && v[e] != -INFINITY) {
-          const uint4 rnd = philox4x32(make_uint4((uint32_t)(i0 + e), c.p.step, 0u, 0u), key);
-          const float u = ((float)(rnd.x >> 8) + 0.5f) * (1.0f / 16777216.0f);
-          const float score = (v[e] - mx) - logf(-logf(u));
-          if (bs.i < 0 || score > bs.v) bs = {score, i0 + e};
-        }
+        for (int e = 0; e < 8; ++e)
+          if (v[e] >= lo_thr && v[e] != -INFINITY) race(v[e], i0 + e);
       }
     }
     bs = cluster_argmax(cl, bs, redf, redi, xch);
@@ -776,49 +829,35 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
 
   // ---- logprob / rank / top-n on the RAW log-softmax (S1, S8)
   // The row's top-n is contained in the union of the slices' top-n.  A slice's n-th largest entry is no smaller than the n-th
-  // largest of its threads' maxima (each a different entry, known from the first sweep), so the sweep that counts the token's
+  // largest of its warps' maxima (each a different entry, known from the first sweep), so the sweep that counts the token's
   // rank also lists the entries from that bound on, a few more than n.
   float tok_lp = 0.f;
-  int rank = 0;
+  int rank = 0, cnt = 0;
   SampleOut* o = outs + r;
-  const int n_topn = min(c.p.n_topn, MAX_TOPN);
   float bound = INFINITY;
   if (n_topn > 0) {
-    __syncthreads();
-    list_v[threadIdx.x] = thread_max;
-    if (threadIdx.x == 0) list_n = 0;
-    __syncthreads();
-    if (threadIdx.x < 32) {   // the n-th largest of the 1024 maxima, taken out one by one
-      float mine = -INFINITY;
-      int at = 0;
-      auto rescan = [&]() {
-        mine = -INFINITY;
-        for (int j = 0; j < SAMP_THREADS / 32; ++j) {
-          const float v = list_v[j * 32 + threadIdx.x];
-          if (v > mine) { mine = v; at = j; }
-        }
-      };
-      rescan();
-      float m = -INFINITY;
-      for (int n = 0; n < n_topn; ++n) {
-        m = mine;
+    if (threadIdx.x < 32) {
+      const int l = threadIdx.x;
+      const float v = l < SAMP_WARPS ? wmax[l] : -INFINITY;
+      int before = 0;
 #pragma unroll
-        for (int o2 = 16; o2 > 0; o2 >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o2));
-        const uint32_t who = __ballot_sync(0xffffffffu, mine == m);
-        if ((int)threadIdx.x == __ffs(who) - 1) {
-          list_v[at * 32 + threadIdx.x] = -INFINITY;
-          rescan();
-        }
+      for (int j = 0; j < SAMP_WARPS; ++j) {
+        const float t = __shfl_sync(0xffffffffu, v, j);
+        before += (t > v || (t == v && j < l)) ? 1 : 0;
       }
-      if (threadIdx.x == 0) bcast[0] = __float_as_uint(m);
+      if (l == 0) {
+        list_n = 0;
+        bcast[0] = __float_as_uint(-INFINITY);   // (maxima that are no numbers: the sweep per entry below)
+      }
+      __syncwarp();
+      if (before == n_topn - 1 && l < SAMP_WARPS) bcast[0] = __float_as_uint(v);
     }
     __syncthreads();
     bound = __uint_as_float(bcast[0]);
   }
-  const bool listed = n_topn > 0 && bound > -INFINITY;   // (-inf: fewer than n entries are allowed in this slice)
+  const bool listed = n_topn > 0 && bound > -INFINITY;   // (-inf: fewer than n warps have an entry that is allowed)
   if (want_lp || listed) {
     if (want_lp) tok_lp = (load_x_any(c, token) - c.raw_max) - c.raw_logz;
-    int cnt = 0;
     for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
       float x[8];
       load_slice8(c, i0, x);
@@ -835,11 +874,9 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
         }
       }
     }
-    if (want_lp) rank = cluster_sumi(cl, cnt, redi, xch);
+    cnt = block_sumi(cnt, redi);
   }
-  if (n_topn > 0) {
-    // every CTA extracts its own n best (value desc, index asc), ONE cluster barrier publishes the lists, and warp 0 of the
-    // cluster's rank-0 CTA merges the <= 8 x 12 candidates in registers.
+  if (n_topn > 0) {   // this CTA's own n best (value desc, index asc)
     __syncthreads();
     const int found = listed ? list_n : SAMP_LIST + 1;
     if (found <= SAMP_LIST) {   // (at least n: the maxima that made the bound are among them)
@@ -853,7 +890,7 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
           cand_i[before] = i;
         }
       }
-    } else {   // masked to a few tokens, or more ties than the list holds: one sweep per entry
+    } else {   // masked to a few tokens, a short slice, or more ties than the list holds: one sweep per entry
       float prev_v = INFINITY;
       int prev_i = -1;
       for (int n = 0; n < n_topn; ++n) {
@@ -872,28 +909,34 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
         }
       }
     }
-    cl.sync();
-    if (crank == 0 && threadIdx.x < 32) {
-      constexpr int PER_LANE = (SAMP_MAX_CL * MAX_TOPN + 31) / 32;  // 3
-      ValIdx mine[PER_LANE];
-#pragma unroll
-      for (int j = 0; j < PER_LANE; ++j) {
-        const int e = (int)threadIdx.x + 32 * j;
-        const int q = e / MAX_TOPN, n = e % MAX_TOPN;
-        mine[j] = ValIdx{-INFINITY, -1};
-        if (q < ncl && n < n_topn) mine[j] = ValIdx{dsmem_read(cl, cand_v + n, q), dsmem_read(cl, cand_i + n, q)};
+  }
+  if (want_lp || n_topn > 0) {   // ONE exchange for the counts and the lists; the cluster's rank-0 CTA orders the <= 8 x 12 candidates
+    const XchView w = cl_publish(cl, xch, Xch4{__int_as_float(cnt), 0.f, 0.f, 0.f});
+    if (want_lp)
+      for (int q = 0; q < ncl; ++q) rank += __float_as_int(w.get(q).a);
+    const int total = ncl * n_topn;
+    if (crank == 0 && n_topn > 0) {
+      const int e = threadIdx.x;
+      if (e < total) {
+        list_v[e] = dsmem_read(cl, cand_v + e % n_topn, e / n_topn);
+        list_i[e] = dsmem_read(cl, cand_i + e % n_topn, e / n_topn);
       }
-      for (int n = 0; n < n_topn; ++n) {
-        ValIdx b{-INFINITY, -1};
+      if (e < n_topn) o->topn_ids[e] = -1;   // (only numbers that do not compare leave a place empty)
+      __syncthreads();
+      if (e < 8 * 32 * ((total + 31) / 32)) {   // eight threads to a candidate (whole warps)
+        const int at = min(e >> 3, total - 1), i = list_i[at];
+        const float v = list_v[at];
+        int before = 0;
+        for (int j = e & 7; j < total; j += 8) {   // (an index below zero: the slice had no more)
+          const float u = list_v[j];
+          const int k = list_i[j];
+          before += k < 0 ? (i < 0 && j < at) : (i < 0 || u > v || (u == v && k < i));
+        }
 #pragma unroll
-        for (int j = 0; j < PER_LANE; ++j) b = vi_better(b, mine[j]);
-        b = warp_argmax(b);
-#pragma unroll
-        for (int j = 0; j < PER_LANE; ++j)
-          if (mine[j].i == b.i) mine[j].i = -1;  // consumed (indices are unique across slices)
-        if (threadIdx.x == 0) {
-          o->topn_ids[n] = b.i;
-          o->topn_lps[n] = (b.v - c.raw_max) - c.raw_logz;
+        for (int k = 1; k < 8; k <<= 1) before += __shfl_xor_sync(0xffffffffu, before, k);
+        if ((e & 7) == 0 && (e >> 3) < total && before < n_topn) {
+          o->topn_ids[before] = i;
+          o->topn_lps[before] = (v - c.raw_max) - c.raw_logz;
         }
       }
     }
@@ -910,21 +953,20 @@ tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRo
   STL_EXIT();
 }
 
-// Cluster size of a launch: just enough CTAs per row to cover the GPU once.  The choice is a function of the launch shape
-// only, so a captured CUDA graph replays the same launch; any_complex still selects the shared-memory staging of the
-// processed row.
-int sampler_cluster_size(int n_rows, int any_complex, int num_sms) {
+// Cluster size of a launch: the most CTAs per row that run in one wave, a function of the launch's shape only, so that a captured
+// CUDA graph replays the same launch.  Clusters do not fill a GPU whose groups of SMs are no multiple of them: of 148 SMs, 15
+// clusters of eight and 33 of four are there at a time (16 rows took two waves of eight: 39 us greedy, 88 typical-p; as fours 17 and
+// 48; 34 rows in fours 33 and 94, in pairs 22 and 73).  Greedy rows, which have two sweeps and as many exchanges, take four, where eight
+// only cost a longer exchange (one row of 128256 17.3 us against 18.0, of 50272 14.4 against 16.6), up to the vocabulary where the
+// sweeps outweigh that.
+int sampler_cluster_size(int n_rows, int any_complex, int vocab, int num_sms) {
   if (const char* e = getenv("TGIS_SAMPLER_CLUSTER")) {
     const int v = atoi(e);
     if (v == 1 || v == 2 || v == 4 || v == 8) return v;
   }
-  // one wave of clusters over the GPU: the largest power of two with n_rows * ncl <= #SMs.  Measured for sampling rows too
-  // (64 rows with typical-p and penalties 403 us with 8 CTAs per row = 4 waves of resident clusters, 256 us
-  // with 2; 32 rows 241 vs 137 us with 4), so the rule does not depend on the row type any more.
-  (void)any_complex;
-  int ncl = 8;
-  while (ncl > 1 && n_rows * ncl > num_sms) ncl >>= 1;
-  return ncl;
+  if (n_rows * 8 <= num_sms - 28 && (any_complex || vocab > 160 * 1024)) return 8;
+  if (n_rows * 4 <= num_sms - 16) return 4;
+  return n_rows * 2 <= num_sms ? 2 : 1;
 }
 
 template <class LT, bool MASKED>
@@ -968,7 +1010,7 @@ cudaError_t sampler_launch(const void* logits, int logits_bf16, int ld, int voca
                            cudaStream_t stream, int any_complex, int num_sms, const uint32_t* allow_bitmap) {
   if (n_rows <= 0) return cudaSuccess;
   if (vocab % 8 != 0 || ld % 8 != 0) return cudaErrorInvalidValue;
-  const int ncl = sampler_cluster_size(n_rows, any_complex, num_sms);
+  const int ncl = sampler_cluster_size(n_rows, any_complex, vocab, num_sms);
   if (logits_bf16)
     return sampler_launch_t(static_cast<const __nv_bfloat16*>(logits), ld, vocab, rows, n_rows,
                             const_cast<uint32_t*>(seen_bitmap), bitmap_words, scratch, out, ncl, any_complex, stream,
