@@ -560,10 +560,9 @@ __device__ __forceinline__ uint4 philox4x32(uint4 ctr, uint2 key) {
 // guided rows -- every benchmark configuration -- run exactly the code they ran before the mask existed).
 template <class LT, bool MASKED>
 __global__ void __launch_bounds__(SAMP_THREADS, 1)
-tgis_sampler_kernel(const LT* __restrict__ logits, int ld, int V, const SampleRow* __restrict__ rows,
-                    uint32_t* __restrict__ seen_bitmap, int bitmap_words, float* __restrict__ scratch,
-                    SampleOut* __restrict__ outs, int ncl, int cache_x, int cache_y,
-                    const uint32_t* __restrict__ allow_bitmap) {
+tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict__ rows, uint32_t* seen_bitmap,
+                    int bitmap_words, float* scratch, SampleOut* __restrict__ outs, int ncl, int cache_x, int cache_y,
+                    const uint32_t* allow_bitmap) {
   // dynamic shared memory: [slice of the raw logits (cache_x)] [slice of the processed logits, fp32 (cache_y)]
   extern __shared__ __align__(16) uint8_t dyn_smem[];
   __shared__ float redf[2 * SAMP_WARPS];
