@@ -3214,7 +3214,7 @@ struct tgis_engine {
   // prefetched into L2 by this launch's producer warp (gemm_tcgen05.cu)
   void gemm(const CUtensorMap* xmaps, const CUtensorMap& wm, const bf16* X, const bf16* W, void* Y, int T, int N, int K,
             int out_f32 = 0, const CUtensorMap* next_wm = nullptr, int nT = 0, int nN = 0, int nK = 0, int ldy = 0,
-            const GemmRope* rope = nullptr, const GemmNorm* norm = nullptr) {
+            const GemmRope* rope = nullptr, const GemmNorm* norm = nullptr, bool late = false) {
     if (ldy == 0) ldy = N;
     cudaEvent_t pe0 = nullptr, pe1 = nullptr;
     if (profiling && (!prof_decode_only || step_is_decode)) {
@@ -3236,7 +3236,7 @@ struct tgis_engine {
       GemmNext nx{};
       if (next_wm && l2_prefetch_kb > 0) nx = gemm_next_desc(nT, nN, nK, num_sms, l2_prefetch_kb);
       CK(gemm_bf16_launch(wm, xmaps[bt_index(T, N, num_sms)], Y, ldy, T, N, K, gemm_ws.p, gemm_counters.p, num_sms, stream, out_f32,
-                          nx.kb_prefetch > 0 ? next_wm : nullptr, nx.kb_prefetch > 0 ? &nx : nullptr, rope, norm, X, W));
+                          nx.kb_prefetch > 0 ? next_wm : nullptr, nx.kb_prefetch > 0 ? &nx : nullptr, rope, norm, X, W, late));
     }
     if (pe1) CK(cudaEventRecord(pe1, stream));
     ++n_launches;
@@ -3299,10 +3299,13 @@ struct tgis_engine {
     const bool lora = (samp_complex & 4) != 0 && max_loras > 0;
     const int32_t* d_toklora = ds<int32_t>(off_toklora);
     const int LR = lora_R, kvd = nkv * HEAD_DIM;
-    auto lora_shrink = [&](const LoraGroup& g, const bf16* x, int ldx) {   // (before the projection it corrects)
-      CK(lora_shrink_launch(x, ldx, d_toklora, g, lora_v.p, T, stream));
+    // A projection and the shrink over the same x: side by side where the projection's kernel can let the shrink start under it, else
+    // the shrink ahead (lora.cu)
+    auto lora_shrink = [&](const LoraGroup& g, const bf16* x, int ldx, bool beside) {
+      CK(lora_shrink_launch(x, ldx, d_toklora, g, lora_v.p, T, stream, beside));
       ++n_launches;
     };
+    auto lora_late = [&](int N, int K) { return lora && !cfg.debug_gemm_ref && gemm_route(T, N, K, num_sms, true) != GEMM_REGISTERS; };
     auto lora_expand = [&](const LoraGroup& g, bf16* y, int ldy, bf16* act_out = nullptr) {
       CK(lora_expand_launch(lora_v.p, d_toklora, g, y, ldy, T, stream, act_out));
       ++n_launches;
@@ -3359,15 +3362,17 @@ struct tgis_engine {
           g.mod[0] = LoraModule{ll.A_q, ll.B_q, H, q_dim, LR, 0, 0};
           g.mod[1] = LoraModule{ll.A_k, ll.B_k, H, kvd, LR, q_dim, LR};
           g.mod[2] = LoraModule{ll.A_v, ll.B_v, H, kvd, LR, q_dim + kvd, 2 * LR};
-          lora_shrink(g, xn.p, H);
         }
+        const bool late = lora_late(qkv_dim, H);
+        if (lora && !late) lora_shrink(g, xn.p, H, false);
         if (skinny_norm && li > 0) {
           CK(gemm_skinny_norm_launch(resid.p, ssq_d, l.ln1, c.rms_eps, l.wqkv, qkv.p, qkv_dim, T, qkv_dim, H, 0, rope_fused ? &rp : nullptr, stream));
           ++n_launches;
         } else {
           gemm(qkv_norm_in ? xm_resid : xm_xn, l.m_qkv, xn.p, l.wqkv, qkv.p, T, qkv_dim, H, 0, &l.m_o, T, H, q_dim, 0,
-               rope_fused ? &rp : nullptr, qkv_norm_in ? &cons_qkv : nullptr);
+               rope_fused ? &rp : nullptr, qkv_norm_in ? &cons_qkv : nullptr, late);
         }
+        if (late) lora_shrink(g, xn.p, H, true);
         if (lora) lora_expand(g, qkv.p, qkv_dim);
       }
       bf16* kc = k_cache.p + (size_t)li * kv_layer_elems;
@@ -3389,7 +3394,8 @@ struct tgis_engine {
                                d_bt, bt_stride, attn_out.p, q_dim, T, nq, nkv, scale, num_sms, stream));
         ++n_launches;
       }
-      if (lora) lora_shrink(lora_one(lora_layers[li].A_o, lora_layers[li].B_o, q_dim, H, LR), attn_out.p, q_dim);
+      const bool late_o = lora_late(H, q_dim), late_gu = lora_late(2 * F, H), late_d = lora_late(H, F);
+      if (lora && !late_o) lora_shrink(lora_one(lora_layers[li].A_o, lora_layers[li].B_o, q_dim, H, LR), attn_out.p, q_dim, false);
       if (skinny_norm) {   // o projection, norm, gate and up projection in two launches
         CK(gemm_skinny_add_launch(attn_out.p, l.wo, resid.p, ssq_o, T, H, q_dim, stream));
         CK(gemm_skinny_norm_launch(resid.p, ssq_o, l.ln2, c.rms_eps, l.wgu, act.p, F, T, 2 * F, H, 2, nullptr, stream));
@@ -3403,7 +3409,8 @@ struct tgis_engine {
         continue;
       }
       gemm(xm_attn, l.m_o, attn_out.p, l.wo, ar_fused ? ar_buf(0) : tmp.p, T, H, q_dim, 0, &l.m_gu, T, 2 * F, H, 0, nullptr,
-           norm_fused ? &prod_attn : nullptr);
+           norm_fused ? &prod_attn : nullptr, late_o);
+      if (late_o) lora_shrink(lora_one(lora_layers[li].A_o, lora_layers[li].B_o, q_dim, H, LR), attn_out.p, q_dim, true);
       if (lora) lora_expand(lora_one(lora_layers[li].A_o, lora_layers[li].B_o, q_dim, H, LR), tmp.p, H);
       if (norm_fused) {
       } else if (ar_fused) {
@@ -3417,18 +3424,20 @@ struct tgis_engine {
       if (lora) {
         // raw interleaved gate_up -> + adapter deltas (gate and up as one module of capacity 2R) -> SwiGLU
         const LoraGroup g = lora_one(lora_layers[li].A_gu, lora_layers[li].B_gu, H, 2 * F, 2 * LR);
-        lora_shrink(g, xn.p, H);
-        gemm(xm_xn, l.m_gu, xn.p, l.wgu, gu_buf.p, T, 2 * F, H, /*out_mode=*/0, &l.m_d, T, H, F, /*ldy=*/2 * F);
+        if (!late_gu) lora_shrink(g, xn.p, H, false);
+        gemm(xm_xn, l.m_gu, xn.p, l.wgu, gu_buf.p, T, 2 * F, H, /*out_mode=*/0, &l.m_d, T, H, F, /*ldy=*/2 * F, nullptr, nullptr, late_gu);
+        if (late_gu) lora_shrink(g, xn.p, H, true);
         lora_expand(g, gu_buf.p, 2 * F, act.p);
       } else
       gemm(norm_fused ? xm_resid : xm_xn, l.m_gu, xn.p, l.wgu, act.p, T, 2 * F, H, /*out_mode=*/2, &l.m_d, T, H, F,
            /*ldy=*/F, nullptr, norm_fused ? &cons_gu : nullptr);
       bf16* down_out = ar_fused ? ar_buf(1) : tmp.p;
-      if (lora) lora_shrink(lora_one(lora_layers[li].A_d, lora_layers[li].B_d, F, H, LR), act.p, F);
+      if (lora && !late_d) lora_shrink(lora_one(lora_layers[li].A_d, lora_layers[li].B_d, F, H, LR), act.p, F, false);
       if (li + 1 < c.n_layers)
         gemm(xm_act, l.m_d, act.p, l.wd, down_out, T, H, F, 0, &layers[li + 1].m_qkv, T, qkv_dim, H, 0, nullptr,
-             norm_fused ? &prod_mlp : nullptr);
-      else gemm(xm_act, l.m_d, act.p, l.wd, down_out, T, H, F, 0, R > 0 ? &m_lm : nullptr, R, Vl, H);
+             norm_fused ? &prod_mlp : nullptr, late_d);
+      else gemm(xm_act, l.m_d, act.p, l.wd, down_out, T, H, F, 0, R > 0 ? &m_lm : nullptr, R, Vl, H, 0, nullptr, nullptr, late_d);
+      if (late_d) lora_shrink(lora_one(lora_layers[li].A_d, lora_layers[li].B_d, F, H, LR), act.p, F, true);
       if (lora) lora_expand(lora_one(lora_layers[li].A_d, lora_layers[li].B_d, F, H, LR), down_out, H);
       if (!ar_fused) all_reduce_tmp(T);
     }

@@ -58,6 +58,7 @@ struct PairArgs {
   int batch, x_cs;          // dense: problems side by side (0 or 1: one); columns of X between them (W: N rows, Y: y_bs elements)
   long long y_bs;
   int scale_ld;             // PAIR_ROWSCALE: scale of token t and problem z: row_scale[t * scale_ld + z]
+  int late;                 // dense: the next kernel starts once X is final
 };
 
 // ---------------------------------------------------------------- cta_group::2 forms
@@ -292,7 +293,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   cluster_sync_all();   // the peer's barriers exist
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_smem;
-  griddep_launch();
+  if (!a.late) griddep_launch();
   if (GROUPED) {   // the segment offsets come from a kernel of this step
     griddep_wait();
     if (warp == 0) {   // exclusive prefix sum of the segments' tile counts
@@ -349,6 +350,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
         const int pre = have ? min(KB, PAIR_STAGES) : 0;
         for (int kb = 0; kb < pre; ++kb) load_w(kb, kb);
         griddep_wait();
+        if (a.late) griddep_launch_after();
         for (int kb = 0; kb < pre; ++kb) load_x(kb, kb);
         issued = pre;
         stage = pre % PAIR_STAGES;
@@ -526,7 +528,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
   cluster_sync_all();   // the peer's barriers exist
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_smem;
-  griddep_launch();
+  if (!a.late) griddep_launch();
 
   if (warp == 0) {
     // ===================== TMA producer (both CTAs) =====================
@@ -551,6 +553,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant
       const int pre = pair < ra.tiles ? min(KS, ra.stages) : 0;
       for (int ks = 0; ks < pre; ++ks) load_w(ks, ks, (pair * 2 + rank) * ra.R);
       griddep_wait();
+      if (a.late) griddep_launch_after();
       for (int ks = 0; ks < pre; ++ks) load_x(ks, ks);
       stage = pre % ra.stages;
       phase = pre == ra.stages ? 1 : 0;
@@ -719,13 +722,13 @@ int gemm_pair_plan(int T, int N, int pairs) {
 }
 
 cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int y_f32, int mode, int T, int N, int K,
-                             int num_sms, cudaStream_t stream) {
+                             int num_sms, cudaStream_t stream, bool late) {
   if (T <= 0 || N <= 0 || K <= 0 || (y_f32 && mode != PAIR_PLAIN)) return cudaErrorInvalidValue;
   const int pairs = num_sms / 2;
   if (pairs < 1) return cudaErrorInvalidValue;
   PairArgs a{};
   a.Y = Y; a.ldy = ldy; a.T = T; a.N = N; a.K = K;
-  a.y_f32 = y_f32; a.mode = mode;
+  a.y_f32 = y_f32; a.mode = mode; a.late = late;
   a.n_tiles = (N + 255) / 256;
   a.x_tiles = gemm_pair_plan(T, N, pairs);
   const int tiles = a.n_tiles * a.x_tiles;
@@ -788,13 +791,13 @@ bool gemm_rows_takes(int T, int N, int K, int num_sms) {
   return T <= 128 ? R >= 40 || (T > 64 && N >= 8 * pairs) : N > 256 * pairs;
 }
 cudaError_t gemm_rows_launch(const void* X, const void* W, void* Y, int ldy, int y_f32, int mode, int T, int N, int K, int num_sms,
-                             cudaStream_t stream) {
+                             cudaStream_t stream, bool late) {
   if (!gemm_rows_takes(T, N, K, num_sms) || (y_f32 && mode != PAIR_PLAIN)) return cudaErrorInvalidValue;
   const int pairs = num_sms / 2;
   RowsArgs ra{};
   PairArgs& a = ra.p;
   a.Y = Y; a.ldy = ldy; a.T = T; a.N = N; a.K = K;
-  a.y_f32 = y_f32; a.mode = mode;
+  a.y_f32 = y_f32; a.mode = mode; a.late = late;
   ra.R = rows_share(N, pairs);
   ra.n = (T + PAIR_UNIT - 1) / PAIR_UNIT * PAIR_UNIT;
   ra.tiles = (N + 2 * ra.R - 1) / (2 * ra.R);

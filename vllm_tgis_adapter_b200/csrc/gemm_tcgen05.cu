@@ -259,6 +259,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
   // t = r (mod s) belong to rank r), ONE cluster barrier, then each owner sums its own shared memory in rank order -- no
   // remote read latency and no exit barrier (pull variant: park locally, barrier, read peers, barrier)
   const bool cl_push = (stream_weights & 4) != 0;
+  const bool late = (stream_weights & 8) != 0;   // (GemmLate: dependents start once the operands are final)
   stream_weights &= 1;
   const long long total = sched.sk_total;  // stream-K region (== everything for decode-shaped launches)
 
@@ -290,7 +291,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
   // running before the first remote store (arrive now, wait right before pushing: free by then)
   if (cl_push) asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   const uint32_t tmem_base = *tmem_base_smem;
-  griddep_launch();  // PDL: the next kernel may start its prologue now
+  if (!late) griddep_launch();  // PDL: the next kernel may start its prologue now
   if (threadIdx.x == 0) TL(1);  // setup done (barriers, TMEM)
   int cl_tile = -1, cl_tvalid = 0;  // cluster mode: the split tile this CTA contributed to (epilogue warps)
 
@@ -423,6 +424,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
       }
       TL(2);           // weight prefetch issued
       griddep_wait();  // activations (and everything the epilogue will touch) are now final
+      if (late) griddep_launch_after();
       TL(3);           // dependency wait returned
       if (threadIdx.x == 0) STL_WAITED();
       int stage = 0;
@@ -1134,7 +1136,7 @@ int gemm_cluster_split(int T, int N, int K, int num_sms) {
 template <int BT, int NW>
 static cudaError_t launch_bt(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int T, int N, int K,
                              float* ws, int* counters, int num_sms, int out_f32, cudaStream_t stream,
-                             const CUtensorMap& next_wmap, const GemmNext& nxt, const GemmRope& rope, const GemmNorm& norm) {
+                             const CUtensorMap& next_wmap, const GemmNext& nxt, const GemmRope& rope, const GemmNorm& norm, bool late) {
   using Cfg = GemmCfg<BT, NW>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -1164,6 +1166,7 @@ static cudaError_t launch_bt(const CUtensorMap& wmap, const CUtensorMap& xmap, v
   }
   const bool push = push_env && split > 0 && BT <= 32 && NW == 1 && norm.h == nullptr;
   if (push) stream_weights |= 4;
+  if (late) stream_weights |= 8;
   // the fused RoPE epilogue lives in the two split-tile reductions (cluster and global fix-up): every tile must be split
   if (rope.positions != nullptr && (gemm_even_split(T, N, K, num_sms) < 2 || out_f32 != 0 ||
                                     N != (rope.n_q + 2 * rope.n_kv) * HEAD_DIM))
@@ -1207,18 +1210,19 @@ bool gemm_fuses_rope(int T, int N, int K, int num_sms, bool named) {
 cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int T, int N, int K,
                              float* ws, int* counters, int num_sms, cudaStream_t stream, int out_f32,
                              const CUtensorMap* next_wmap, const GemmNext* next, const GemmRope* rope, const GemmNorm* norm,
-                             const void* X, const void* W) {
+                             const void* X, const void* W, bool late) {
   const bool named = X != nullptr && W != nullptr && norm == nullptr && ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) == 0;
   const GemmRoute route = gemm_route(T, N, K, num_sms, named);
   if (rope != nullptr && (out_f32 != 0 || N != (rope->n_q + 2 * rope->n_kv) * HEAD_DIM || !gemm_fuses_rope(T, N, K, num_sms, named)))
     return cudaErrorInvalidValue;
+  if (late && (route == GEMM_REGISTERS || norm != nullptr)) return cudaErrorInvalidValue;
   if (route == GEMM_REGISTERS) return gemm_skinny_launch(X, W, Y, ldy, T, N, K, out_f32, rope, stream);
   if (route != GEMM_CUT) {
     if (norm != nullptr || out_f32 < 0 || out_f32 > 4) return cudaErrorInvalidValue;
-    if (route == GEMM_SHARES) return gemm_rows_launch(X, W, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream);
+    if (route == GEMM_SHARES) return gemm_rows_launch(X, W, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream, late);
     CUtensorMap xm;
     if (route == GEMM_SMALL_PAIRS && make_tmap_bf16_2d(&xm, X, T, K, K, GEMM_X_BOX_MANY, 64) != 0) return cudaErrorInvalidValue;
-    return gemm_pair_launch(wmap, route == GEMM_SMALL_PAIRS ? xm : xmap, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream);
+    return gemm_pair_launch(wmap, route == GEMM_SMALL_PAIRS ? xm : xmap, Y, ldy, out_f32 == 1, pair_mode(out_f32), T, N, K, num_sms, stream, late);
   }
   GemmRope rp{};
   if (rope) rp = *rope;
@@ -1229,8 +1233,8 @@ cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
   const CUtensorMap& nm = (next && next_wmap) ? *next_wmap : wmap;
   const int nw = gemm_nw(T);
 #define TGIS_GEMM_CASE(B)                                                                                              \
-  return nw == 2 ? launch_bt<B, 2>(wmap, xmap, Y, ldy, T, N, K, ws, counters, num_sms, out_f32, stream, nm, nx, rp, nr) \
-                 : launch_bt<B, 1>(wmap, xmap, Y, ldy, T, N, K, ws, counters, num_sms, out_f32, stream, nm, nx, rp, nr)
+  return nw == 2 ? launch_bt<B, 2>(wmap, xmap, Y, ldy, T, N, K, ws, counters, num_sms, out_f32, stream, nm, nx, rp, nr, late) \
+                 : launch_bt<B, 1>(wmap, xmap, Y, ldy, T, N, K, ws, counters, num_sms, out_f32, stream, nm, nx, rp, nr, late)
   switch (gemm_pick_bt(T)) {
     case 16: TGIS_GEMM_CASE(16);
     case 32: TGIS_GEMM_CASE(32);

@@ -112,7 +112,8 @@ cudaError_t gemm_bf16_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, v
                              float* ws, int* counters, int num_sms, cudaStream_t stream, int out_f32 = 0,
                              const CUtensorMap* next_wmap = nullptr, const GemmNext* next = nullptr,
                              const GemmRope* rope = nullptr, const GemmNorm* norm = nullptr, const void* X = nullptr,
-                             const void* W = nullptr);  // X, W: the operands behind the maps ([T, K], [N, K]), if contiguous
+                             const void* W = nullptr,  // X, W: the operands behind the maps ([T, K], [N, K]), if contiguous
+                             bool late = false);  // the next kernel of the stream starts once X is final (not GEMM_REGISTERS): lora_shrink_launch
 
 // ---- gemm_pair.cu: the same product on CTA pairs (tcgen05 cta_group::2), thousands of tokens or expert segments ----------
 constexpr int PAIR_PLAIN = 0;        // Y[row, n] = acc
@@ -125,11 +126,11 @@ constexpr int PAIR_TANH = 6;
 constexpr int PAIR_ROWSCALE = 7;     // times a scale per row (and problem)
 // wmap: boxes of 128 rows x 64; xmap: boxes of GEMM_X_BOX_MANY rows x 64; Y fp32 (y_f32) or bf16
 cudaError_t gemm_pair_launch(const CUtensorMap& wmap, const CUtensorMap& xmap, void* Y, int ldy, int y_f32, int mode, int T, int N,
-                             int K, int num_sms, cudaStream_t stream);
+                             int K, int num_sms, cudaStream_t stream, bool late = false);
 // the same for up to 256 tokens in equal shares of weight rows; X [T, K], W [N, K] contiguous
 bool gemm_rows_takes(int T, int N, int K, int num_sms);
 cudaError_t gemm_rows_launch(const void* X, const void* W, void* Y, int ldy, int y_f32, int mode, int T, int N, int K, int num_sms,
-                             cudaStream_t stream);
+                             cudaStream_t stream, bool late = false);
 // CTA pairs with 129 to 256 tokens where no share of rows is large enough and k is short
 inline bool gemm_small_pairs(int T, int K) { return T > 128 && T <= 256 && K <= 4096; }
 int gemm_pair_plan(int T, int N, int pairs);   // token tiles of the dense launch
@@ -214,7 +215,7 @@ struct LoraGroup {
   int v_ld;                // floats per token in the shrink buffer (a multiple of four)
 };
 cudaError_t lora_shrink_launch(const __nv_bfloat16* x, int ldx, const int32_t* tok_slot, const LoraGroup& g, float* v, int T,
-                               cudaStream_t stream);
+                               cudaStream_t stream, bool beside = false);
 // act != nullptr (one module over interleaved gate / up columns): act[t, j] = bf16(silu(gate)) * up of the sum instead of y
 cudaError_t lora_expand_launch(const float* v, const int32_t* tok_slot, const LoraGroup& g, __nv_bfloat16* y, int ldy, int T,
                                cudaStream_t stream, __nv_bfloat16* act = nullptr);

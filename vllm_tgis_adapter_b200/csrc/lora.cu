@@ -19,8 +19,12 @@
 //   expand : CTA = (tile of 16 tokens, 512 output columns), warp = 64 columns: B rows as fragments of mma.sync straight from global
 //            memory, all requested in one round, each lane 8 neighbouring columns of 2 tokens.  24 tokens, four adapters of rank 16, 8B
 //            widths, microseconds a launch against multiply-adds from shared memory (8 tokens x 1024 columns): 6.3 -> 4.0, with SwiGLU 19.8 -> 10.4.
-// Both are launches of a few microseconds of dependent loads.  The engine runs shrink BEFORE the base projection, which it
-// does not depend on: the projection's first weights are on their way while it runs.
+// Both are launches of a few microseconds of dependent loads.  Shrink and the base projection read the same x and need nothing of
+// each other, so shrink runs beside the projection: launched behind it, started when every block of the projection is past its own wait
+// for x (griddep_launch_after; the products on tensor cores have that form), and, having done its work, it waits for the
+// projection, which is what lets the expand wait for one kernel only.  Ahead of the projection it was 4 to 10 us of a chain in which
+// the weights stood still (24 tokens, four adapters of rank 16, 8B widths, one layer, PDL: 144 us with shrink ahead and B asked for
+// behind the expand's wait, 126 so; without adapters 102).  Where the projection runs on register products, shrink stays ahead.
 // Adapter storage (engine.cu): per layer and module  A [slots][Rm][K] and B [slots][N][Rm] bf16, zero padded to the module's
 // rank capacity Rm, so no kernel needs the adapter's true rank.  gate_proj / up_proj are stored as ONE module of capacity
 // 2R over the interleaved gate_up projection (row 2j = gate_j, row 2j+1 = up_j: block-sparse B), see engine.cu.
@@ -108,10 +112,11 @@ __device__ __forceinline__ F8 cvt8(const uint4& r) {
 // A launch is a chain of latencies: rows of A are asked for under the kernel before and a round ahead, 32 sums meet in 31 exchanges
 // instead of 160, the modules' table is read from the parameters instead of a copy in local memory (24 requests with adapters, average
 // launch, microseconds: 8.1 -> 7.3, the expands 4.8 -> 4.0 and 11.3 -> 10.4 by the last of these).
+// beside: see above; x is complete when the kernel starts, so only what comes behind waits
 constexpr int LORA_RPC = 4;
 __global__ void __launch_bounds__(256)
-lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* __restrict__ tok_slot, const __grid_constant__ LoraGroup g,
-                   float* __restrict__ v, int T) {
+lora_shrink_kernel(const __nv_bfloat16* x, int ldx, const int32_t* __restrict__ tok_slot, const __grid_constant__ LoraGroup g,
+                   float* __restrict__ v, int T, int beside) {
   __shared__ float part[8][LORA_RPC][LORA_ST];
   griddep_launch();
   int m = 0, r0 = (int)blockIdx.y * LORA_RPC;  // blockIdx.y enumerates (module, group of LORA_RPC rank rows)
@@ -130,7 +135,7 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* 
   for (int p = blockIdx.z;; p += gridDim.z, first = false) {
     const int slot = tile.distinct(p, 1);   // (slots and adapters are written ahead of the step: x alone is waited for)
     if (slot < 0) {
-      if (first) griddep_wait();
+      if (first || beside) griddep_wait();   // (beside a product: the kernel behind this one waits for both by waiting for this one)
       return;
     }
     static_assert(LORA_RPC * LORA_ST == 32, "one sum per lane");
@@ -142,11 +147,11 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* 
       for (int q = 0; q < LORA_RPC; ++q) ar[q] = kv < nvec ? a0[(size_t)q * nvec + kv] : make_uint4(0u, 0u, 0u, 0u);
     };
     load_a(warp * 32 + lane);
-    if (first) griddep_wait();
+    if (first && !beside) griddep_wait();
     for (int kv = warp * 32 + lane; kv < nvec; kv += 256) {
       uint4 xr[LORA_ST];
 #pragma unroll
-      for (int j = 0; j < LORA_ST; ++j) xr[j] = tile.s[j] == slot ? xq[(size_t)(t0 + j) * ldq + kv] : make_uint4(0u, 0u, 0u, 0u);
+      for (int j = 0; j < LORA_ST; ++j) xr[j] = tile.s[j] == slot ? __ldcg(xq + (size_t)(t0 + j) * ldq + kv) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
       for (int j = 0; j < LORA_ST; ++j) {
         const F8 xf = cvt8(xr[j]);
@@ -185,10 +190,11 @@ lora_shrink_kernel(const __nv_bfloat16* __restrict__ x, int ldx, const int32_t* 
 constexpr int LORA_ECOLS = 512;   // columns per CTA of the expand: 8 warps x 64
 // ACT: the columns are interleaved (gate_j, up_j) pairs; act[t, j] = bf16(silu(gate)) * up of the corrected projection is
 // written (for tokens without an adapter too) and y is only read: the projection's own kernel after it drops out.
+// (v and y, and x of the shrink, are not __restrict__: a load through such a pointer may be moved ahead of a wait that stands in a branch)
 template <bool ACT>
 __global__ void __launch_bounds__(256, 2)
-lora_expand_kernel(const float* __restrict__ v, const int32_t* __restrict__ tok_slot, const __grid_constant__ LoraGroup gr,
-                   __nv_bfloat16* __restrict__ y, int ldy, __nv_bfloat16* __restrict__ act, int T) {
+lora_expand_kernel(const float* v, const int32_t* __restrict__ tok_slot, const __grid_constant__ LoraGroup gr,
+                   __nv_bfloat16* y, int ldy, __nv_bfloat16* __restrict__ act, int T) {
   __shared__ __align__(16) __nv_bfloat16 vs[LORA_TT][LORA_MAX_RM + 8];   // the tile's rank vectors
   griddep_launch();
   const int t0 = (int)blockIdx.y * LORA_TT;
@@ -199,10 +205,35 @@ lora_expand_kernel(const float* __restrict__ v, const int32_t* __restrict__ tok_
   const int n0 = (int)blockIdx.x * LORA_ECOLS + warp * 64;
   const int kc = (md.Rm + 15) / 16;   // chunks of 16 rank indices
   const int slot_of[2] = {tile.of(g), tile.of(g + 8)};
-  griddep_wait();
+  bool first = true;
   for (int p = blockIdx.z / gr.n_mods;; p += gridDim.z / gr.n_mods) {
     const int slot = tile.distinct(p, ACT ? 0 : 1);
-    if (slot < 0) return;
+    if (slot < 0) {
+      if (first) griddep_wait();
+      return;
+    }
+    // the adapter's rows are static: asked for under the kernel before
+    const __nv_bfloat16* brow[2][4];
+    uint2 nxt[2][4];
+    auto load = [&](int c) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          nxt[h][j] = c * 16 + t * 4 < md.Rm ? *reinterpret_cast<const uint2*>(brow[h][j] + c * 16 + t * 4) : make_uint2(0u, 0u);
+    };
+    if (slot > 0) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int n = min(n0 + 32 * h + 8 * (g >> 1) + 2 * j + (g & 1), md.N - 1);
+          brow[h][j] = md.B + ((size_t)(slot - 1) * md.N + n) * md.Rm;
+        }
+      load(0);
+    }
+    if (first) griddep_wait();
+    first = false;
     // columns n0 + 32 h + 8 t .. + 7 of tokens g and g + 8 are this lane's; of the products' column blocks j = 0 .. 3 (8 wide) lane
     // group t holds the neighbours 2 j, 2 j + 1, so block j is made of the columns 8 (c / 2) + 2 j + c % 2, c = 0 .. 7
     uint4 yv[2][2];
@@ -220,23 +251,6 @@ lora_expand_kernel(const float* __restrict__ v, const int32_t* __restrict__ tok_
       }
     float acc[2][4][4] = {};
     if (slot > 0) {
-      const __nv_bfloat16* brow[2][4];
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int n = min(n0 + 32 * h + 8 * (g >> 1) + 2 * j + (g & 1), md.N - 1);
-          brow[h][j] = md.B + ((size_t)(slot - 1) * md.N + n) * md.Rm;
-        }
-      uint2 nxt[2][4];
-      auto load = [&](int c) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            nxt[h][j] = c * 16 + t * 4 < md.Rm ? *reinterpret_cast<const uint2*>(brow[h][j] + c * 16 + t * 4) : make_uint2(0u, 0u);
-      };
-      load(0);
       // the fp32 shrink sums enter the second product as bf16 (lora_expand_op.py casts the buffer to the weight dtype)
       const int row4 = kc * 4;
       for (int i = threadIdx.x; i < LORA_TT * row4; i += 256) {
@@ -244,7 +258,7 @@ lora_expand_kernel(const float* __restrict__ v, const int32_t* __restrict__ tok_
         float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
         if (t0 + tok < T && r < md.Rm && tok_slot[t0 + tok] == slot) {
           const float* from = v + (size_t)(t0 + tok) * gr.v_ld + md.v_off + r;
-          f = *reinterpret_cast<const float4*>(from);
+          f = __ldcg(reinterpret_cast<const float4*>(from));
         }
         const __nv_bfloat162 lo = __floats2bfloat162_rn(f.x, f.y), hi = __floats2bfloat162_rn(f.z, f.w);
         *reinterpret_cast<uint2*>(&vs[tok][r]) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
@@ -318,13 +332,13 @@ static bool lora_group_ok(const LoraGroup& g) {
 }
 
 cudaError_t lora_shrink_launch(const __nv_bfloat16* x, int ldx, const int32_t* tok_slot, const LoraGroup& g, float* v, int T,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, bool beside) {
   if (T <= 0) return cudaSuccess;
   if (!lora_group_ok(g) || ldx % 8 != 0) return cudaErrorInvalidValue;
   int groups = 0;
   for (int m = 0; m < g.n_mods; ++m) groups += g.mod[m].Rm / LORA_RPC;
   return launch_k(lora_shrink_kernel, dim3((T + LORA_ST - 1) / LORA_ST, groups, lora_passes_apart(T)), dim3(256), 0, stream, x, ldx, tok_slot,
-                  g, v, T);
+                  g, v, T, beside ? 1 : 0);
 }
 
 cudaError_t lora_expand_launch(const float* v, const int32_t* tok_slot, const LoraGroup& g, __nv_bfloat16* y, int ldy, int T,

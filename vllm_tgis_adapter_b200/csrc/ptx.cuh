@@ -284,6 +284,11 @@ __device__ __forceinline__ void silu_mul_bf16_n(const float (&g)[N], const float
 }
 
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+// behind griddep_wait by every thread block's one calling thread: a kernel that starts now may read what the kernels before this one
+// wrote (they are complete, their writes performed), though not what this one writes, without a wait of its own
+__device__ __forceinline__ void griddep_launch_after() {
+  asm volatile("fence.acq_rel.gpu;\n griddepcontrol.launch_dependents;\n" ::: "memory");
+}
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
 // ---------------------------------------------------------------- in-situ step timeline (debug builds only)
