@@ -1,6 +1,6 @@
-"""The sampler's selections (csrc/sampler.cu) at the edges of what they list: typical-p and top-p over rows where the entries of
-one sixteen-bit key are none, a few, or more than the list holds (all equal, two values, a fine ramp), rows masked to a few tokens,
-at cluster sizes one to eight.  With one seed the kept set is known in fp64 but for entries at the threshold itself, and the race
+"""The sampler's selections (csrc/sampler.cu) at the edges of what they list: typical-p, top-k and top-p over rows where the entries of
+one step of the first sweep are none, a few, or more than the list holds (all equal, two values, a fine ramp), rows masked to a few
+tokens, at cluster sizes one to eight.  With one seed the kept set is known in fp64 but for entries at the threshold itself, and the race
 over it has one winner."""
 import numpy as np
 import pytest
@@ -23,11 +23,7 @@ def kept_typical(x, p, slack):
     return key <= at(p - slack) - slack, key > at(p + slack) + slack
 
 
-@pytest.mark.parametrize("cluster", ["1", "2", "4", "8"])
-@pytest.mark.parametrize("V,dtype", [(1024, torch.float32), (50272, torch.float32), (128256, torch.bfloat16)])
-def test_typical_rows_keep_what_sorting_keeps(V, dtype, cluster, monkeypatch):
-    monkeypatch.setenv("TGIS_SAMPLER_CLUSTER", cluster)
-    rows = 12
+def rows_of_all_kinds(rows, V):
     gen = torch.Generator().manual_seed(V)
     logits = torch.randn(rows, V, generator=gen)
     for i in range(rows):
@@ -37,12 +33,20 @@ def test_typical_rows_keep_what_sorting_keeps(V, dtype, cluster, monkeypatch):
         elif kind == 2:
             logits[i] = (logits[i] > 0).float() * 2.0            # two
         elif kind == 3:
-            logits[i] = torch.linspace(0.0, 1e-3, V)             # more entries to sixteen bits than the list holds
+            logits[i] = torch.linspace(0.0, 1e-3, V)             # more entries to a step than the list holds
         elif kind == 4:
             logits[i, 7 * i] += 18.0                             # one entry is all there is
         elif kind == 5:
             logits[i, 3:] = -float("inf")
-    logits = logits.to(dtype)
+    return logits
+
+
+@pytest.mark.parametrize("cluster", ["1", "2", "4", "8"])
+@pytest.mark.parametrize("V,dtype", [(1024, torch.float32), (50272, torch.float32), (128256, torch.bfloat16)])
+def test_typical_rows_keep_what_sorting_keeps(V, dtype, cluster, monkeypatch):
+    monkeypatch.setenv("TGIS_SAMPLER_CLUSTER", cluster)
+    rows = 12
+    logits = rows_of_all_kinds(rows, V).to(dtype)
     r = np.zeros(rows, dtype=U.SAMPLE_ROW_DTYPE)
     r["temperature"], r["top_p"], r["rep_penalty"], r["eos_id"], r["seq_slot"] = 1.0, 1.0, 1.0, -1, -1
     r["logits_row"], r["typical_p"], r["flags"] = np.arange(rows), 0.6, U.SAMPLE_TYPICAL | U.SAMPLE_LOGPROBS
@@ -59,6 +63,42 @@ def test_typical_rows_keep_what_sorting_keeps(V, dtype, cluster, monkeypatch):
         if int((~never).sum()) == 1:
             assert all(t[i] == int(torch.nonzero(~never)) for t in seen)
         elif int(sure.sum()) > 100:
+            assert len({int(t[i]) for t in seen}) > 1
+
+
+@pytest.mark.parametrize("cluster", ["1", "2", "4", "8"])
+@pytest.mark.parametrize("V,dtype", [(1024, torch.float32), (50272, torch.float32), (128256, torch.bfloat16)])
+def test_top_k_and_top_p_keep_what_sorting_keeps(V, dtype, cluster, monkeypatch):
+    """At temperature one the k-th largest logit is exact; the mass below top-p's threshold is known to 1e-5 (steps of 2^-30 an entry,
+    expf to 2 ulp).  Rows with fewer than k entries left keep them all."""
+    monkeypatch.setenv("TGIS_SAMPLER_CLUSTER", cluster)
+    rows, k, p = 18, 50, 0.7
+    logits = rows_of_all_kinds(rows, V).to(dtype)
+    r = np.zeros(rows, dtype=U.SAMPLE_ROW_DTYPE)
+    r["temperature"], r["rep_penalty"], r["eos_id"], r["seq_slot"] = 1.0, 1.0, -1, -1
+    r["logits_row"] = np.arange(rows)
+    r["top_k"] = [k if i // 6 != 1 else 0 for i in range(rows)]
+    r["top_p"] = [p if i // 6 != 0 else 1.0 for i in range(rows)]
+    seen = []
+    for seed in range(8):
+        r["seed_lo"] = 100 + seed
+        seen.append(U.run_sampler(logits.cuda(), r)["token"].copy())
+    for i in range(rows):
+        x = logits[i].double()
+        left = x > -float("inf")
+        if r["top_k"][i]:
+            left &= x >= torch.sort(x, descending=True).values[k - 1]
+        never = ~left
+        if r["top_p"][i] < 1:
+            pr = torch.softmax(torch.where(left, x, torch.full_like(x, -float("inf"))), -1)
+            order = torch.argsort(x)
+            cum = pr[order].cumsum(0)
+            thr = x[order[min(int((cum <= 1 - p - 1e-5).sum()), V - 1)]]     # entries below it are out whatever rounds how
+            never |= x < thr
+        assert not any(bool(never[t[i]]) for t in seen), i
+        if int((~never).sum()) == 1:
+            assert all(t[i] == int(torch.nonzero(~never)) for t in seen)
+        elif float(torch.softmax(torch.where(never, torch.full_like(x, -float("inf")), x), -1).max()) < 0.1:   # (not eight times the same)
             assert len({int(t[i]) for t in seen}) > 1
 
 

@@ -18,11 +18,15 @@
 //                 maximum per entry was a chain of a branch and an exponential each: 9100 of a greedy row's 27000 cycles); behind
 //                 typical-p the entropy's sum too
 //   reductions    maximum, sums and best entry in one; an exchange is one 16-byte read per lane and shuffles
-//   typical-p     three radix rounds and a fourth over the few entries that share sixteen bits; the race over what is left
+//   selections    (typical-p, top-k, top-p) one sweep over steps of a 32nd of an octave, one that lists the selected step's entries, radix
+//                 rounds over the list
+//   race          behind typical-p over the list of what is left; in flat rows over kept processed logits, two logarithms only
+//                 for entries that 1 - u cannot rule out (186 instructions an entry -> 100; it was 38 % of a flat row)
 //   rank, top-n   one sweep and one exchange, the slices' lists ordered by eight threads a candidate
-// Measured, 128256 bf16 logits with top-5, microseconds, with the online maximum, an exchange for each part and clusters by SM count ->
-// here: greedy 19.7 -> 17.3 (1 row), 39 -> 17 (16), 22 -> 18 (32), 38 -> 29 (96), 73 -> 55 (150); typical-p 45 -> 38 (1), 88 -> 48 (16),
-// 91 -> 74 (64), 157 -> 124 (96), 309 -> 240 (150); flat rows 63 -> 58, 285 -> 263; top-k with top-p 63 -> 59 (1), 240 -> 214 (96).
+// Measured, 128256 bf16 logits with top-5, microseconds, with the online maximum, an exchange for each part, clusters by SM count and four
+// radix rounds over leading bits -> here: greedy 19.7 -> 17 (1 row), 39 -> 17 (16), 22 -> 18 (32), 38 -> 28 (96), 73 -> 54 (150); typical-p
+// 45 -> 36 (1), 88 -> 42 (16), 91 -> 59 (64), 157 -> 91 (96), 309 -> 177 (150); flat rows 63 -> 48 (1), 285 -> 173 (96); top-k with
+// top-p 63 -> 52 (1), 240 -> 129 (96).  (Only rows of equal logits, which no list holds, gain nothing: 438 -> 519, 80 of them with top-k.)
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -41,6 +45,8 @@ constexpr int SAMP_MAX_CL = 8;  // CTAs (SMs) per row: 1, 2, 4 or 8, chosen per 
 constexpr int SAMP_THREADS = 1024;
 constexpr int SAMP_WARPS = SAMP_THREADS / 32;
 constexpr int SAMP_LIST = SAMP_THREADS;
+constexpr int SAMP_FEW = 3 * SAMP_THREADS;
+constexpr float SAMP_FLAT = 7.f;  // nats: as spread as over 1100 entries, more than a list holds
 constexpr float SAMP_FIX = 1073741824.0f;  // 2^30: probabilities are accumulated as fixed-point integers (see below)
 
 // LT = logits element type: __nv_bfloat16 on the product path (vLLM's lm_head emits model-dtype logits and the sampler
@@ -339,10 +345,11 @@ __device__ __forceinline__ float key2f(uint32_t k) {
 //   ascending (weighted select): first bin b with  below + sum_{<= b} >= target  (strict: > target); none: last nonempty
 //   descending (k-th largest)  : first bin b from the top with  above + sum_{>= b} >= target
 // Returns (bin, weight strictly before the bin in scan order) to every thread through bcast[0..1].
+template <int BINS>
 __device__ void radix_round_pick(const Cl& c, uint32_t* hist, uint32_t* hsum, uint32_t* bcast, uint32_t before,
                                  uint32_t target, bool strict, bool descending) {
   c.sync();  // every CTA's histogram of this round is complete
-  if (threadIdx.x < 256) {
+  if (threadIdx.x < BINS) {
     uint32_t t = 0;
     for (int r = 0; r < c.ncl; ++r) t += dsmem_read(c, hist + threadIdx.x, r);
     hsum[threadIdx.x] = t;
@@ -350,10 +357,11 @@ __device__ void radix_round_pick(const Cl& c, uint32_t* hist, uint32_t* hsum, ui
   __syncthreads();
   if (threadIdx.x < 32) {
     const int l = threadIdx.x;
-    uint32_t h[8], tot = 0;
+    constexpr int PER = BINS / 32;
+    uint32_t h[PER], tot = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int b = descending ? 255 - (8 * l + j) : 8 * l + j;
+    for (int j = 0; j < PER; ++j) {
+      const int b = descending ? BINS - 1 - (PER * l + j) : PER * l + j;
       h[j] = hsum[b];
       tot += h[j];
     }
@@ -368,11 +376,11 @@ __device__ void radix_round_pick(const Cl& c, uint32_t* hist, uint32_t* hsum, ui
     uint32_t sel_before = 0;
     int last_nonempty = -1;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < PER; ++j) {
       const uint32_t nc = cum + h[j];
-      if (h[j] > 0) last_nonempty = 8 * l + j;
+      if (h[j] > 0) last_nonempty = PER * l + j;
       if (sel < 0 && h[j] > 0 && (strict ? (nc > target) : (nc >= target))) {
-        sel = 8 * l + j;
+        sel = PER * l + j;
         sel_before = cum;
       }
       cum = nc;
@@ -389,18 +397,18 @@ __device__ void radix_round_pick(const Cl& c, uint32_t* hist, uint32_t* hsum, ui
       int ln = last_nonempty;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) ln = max(ln, __shfl_xor_sync(0xffffffffu, ln, o));
-      out_sel = ln < 0 ? 255 : ln;
+      out_sel = ln < 0 ? BINS - 1 : ln;
       // weight before that bin: lanes below contribute their totals, the owning lane its bins before it
       uint32_t part = 0;
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (8 * l + j < out_sel) part += h[j];
+      for (int j = 0; j < PER; ++j)
+        if (PER * l + j < out_sel) part += h[j];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
       out_before = before + part;
     }
     if (l == 0) {
-      bcast[0] = (uint32_t)(descending ? 255 - out_sel : out_sel);  // back to a digit value
+      bcast[0] = (uint32_t)(descending ? BINS - 1 - out_sel : out_sel);  // back to a digit value
       bcast[1] = out_before;
     }
   }
@@ -409,8 +417,9 @@ __device__ void radix_round_pick(const Cl& c, uint32_t* hist, uint32_t* hsum, ui
 
 // Adds eight (digit, weight) pairs of every lane to the histogram (weight 0: does not count).  Where the whole warp's 256
 // entries share a digit (the leading digits of most rows) one redux and one atomic do; else every entry is a shared-memory
-// atomic of its own, on HIST_COPIES copies of the histogram so that lanes of equal digits meet less often.
-constexpr int HIST_COPIES = 4;
+// atomic of its own, on several copies of the histogram so that lanes of equal digits meet less often.
+constexpr int HIST_WORDS = 1024;   // copies of the histogram, as many as fit
+template <int BINS>
 __device__ __forceinline__ void hist_add8(uint32_t* h, const uint32_t (&digit)[8], const uint32_t (&w)[8]) {
   uint32_t d = 0xffffffffu, sum = 0;
   bool same = true;
@@ -429,115 +438,115 @@ __device__ __forceinline__ void hist_add8(uint32_t* h, const uint32_t (&digit)[8
     if ((threadIdx.x & 31) == 0) atomicAdd(&h[d0], all);
     return;
   }
-  uint32_t* mine = h + (threadIdx.x & (HIST_COPIES - 1)) * 256;
+  uint32_t* mine = h + (threadIdx.x & (HIST_WORDS / BINS - 1)) * BINS;
 #pragma unroll
   for (int e = 0; e < 8; ++e)
     if (w[e] > 0) atomicAdd(&mine[digit[e]], w[e]);
 }
 // a round's histogram: all copies to zero / their sum in the first
 __device__ __forceinline__ void hist_clear(uint32_t* h) {
-  for (int i = threadIdx.x; i < 256 * HIST_COPIES; i += SAMP_THREADS) h[i] = 0u;
+  for (int i = threadIdx.x; i < HIST_WORDS; i += SAMP_THREADS) h[i] = 0u;
   __syncthreads();
 }
+template <int BINS>
 __device__ __forceinline__ void hist_fold(uint32_t* h) {
   __syncthreads();
-  if (threadIdx.x < 256) {
+  if (threadIdx.x < BINS) {
     uint32_t t = h[threadIdx.x];
 #pragma unroll
-    for (int k = 1; k < HIST_COPIES; ++k) t += h[k * 256 + threadIdx.x];
+    for (int k = 1; k < HIST_WORDS / BINS; ++k) t += h[k * BINS + threadIdx.x];
     h[threadIdx.x] = t;
   }
 }
 
-// Smallest key K (ascending) such that  sum_{key_i <= K} w_i  >= target  (strict: > target); if never reached, the
-// largest present key.  load(i0, v) -> eight values, keyf(v) -> uint32 key, wf(v) -> probability-like weight in [0, 1] (sums
-// to ~1 over the row).  Weights are accumulated as 2^-30 fixed-point integers: integer addition is associative, so the
-// histograms -- and with them the selected threshold and every seeded draw -- are bit-reproducible whatever the order in
-// which warps and CTAs arrive (float atomics were not).
-// 4 rounds of 8 bits; every CTA histograms its slice, the cluster sums them, every CTA runs the same scan.
-template <class LoadF, class KeyF, class WF>
-__device__ uint32_t select_weighted_asc(Cl& c, int lo, int hi, LoadF load, KeyF keyf, WF wf, float target, bool strict,
-                                        uint32_t (*hist)[256 * HIST_COPIES], uint32_t* hsum, uint32_t* bcast, float* few, int* n_few) {
-  const uint32_t T = __float2uint_rn(fminf(fmaxf(target, 0.f), 2.f) * SAMP_FIX);
-  uint32_t prefix = 0, below = 0;
+// The first sweep of a selection sorts by this instead of by leading bits: of a distance >= 0, steps of a 32nd of an octave from 2^-10
+// to 2^6 (what lies outside joins the first or the last).  Leading bits of a float are its exponent: two steps of an octave hold nine
+// tenths of a flat row, which then was swept three times, with an exponential and an atomic for most entries each time.
+constexpr int CODES = 512;
+__device__ __forceinline__ uint32_t distance_code(float t) {
+  const int c = (int)(__float_as_uint(t) >> 18) - ((127 - 10) << 5);
+  return (uint32_t)min(max(c, 0), CODES - 1);
+}
+
+// Smallest key K (ascending) such that  sum_{key_i <= K} w_i  >= target  (strict: > target), or with `descending` the largest with
+// sum_{key_i >= K}; if never reached, the last present key.  load(i0, v) -> eight values, code(v) < CODES, not falling with the
+// key, keyf(v) -> uint32 key, wq(v) -> integer weight: integer addition is associative, so the
+// result is the same on every cluster size.  Every CTA histograms its slice, the cluster sums the histograms, every CTA runs the same
+// scan: codes first; then a sweep that lists the entries of the selected code, and four rounds of 8 bits over the list, or, where
+// that has no room, over the slice.
+template <class LoadF, class CodeF, class KeyF, class WQ>
+__device__ uint32_t select_key(Cl& c, int lo, int hi, LoadF load, CodeF code, KeyF keyf, WQ wq, uint32_t T, bool strict, bool descending,
+                               uint32_t (*hist)[HIST_WORDS], uint32_t* hsum, uint32_t* bcast, float* few, int* n_few) {
+  uint32_t* h = hist[c.he & 1];
+  ++c.he;
+  hist_clear(h);
+  for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
+    const int i0 = base + threadIdx.x * 8;
+    uint32_t digit[8], w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (i0 < hi) {
+      float v[8];
+      load(i0, v);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        digit[e] = code(v[e]);
+        w[e] = wq(v[e]);
+      }
+    }
+    hist_add8<CODES>(h, digit, w);
+  }
+  hist_fold<CODES>(h);
+  if (threadIdx.x == 0) *n_few = 0;
+  radix_round_pick<CODES>(c, h, hsum, bcast, 0u, T, strict, descending);
+  const uint32_t sel = bcast[0];
+  uint32_t prefix = 0, before = bcast[1];
+  for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
+    if (*n_few > SAMP_FEW) break;
+    float v[8];
+    load(i0, v);
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (code(v[e]) == sel) {
+        const int at = atomicAdd(n_few, 1);
+        if (at < SAMP_FEW) few[at] = v[e];
+      }
+  }
   for (int round = 0; round < 4; ++round) {
     const int shift = 24 - 8 * round;
-    uint32_t* h = hist[c.he & 1];
+    auto counts = [&](uint32_t k) { return round == 0 || (k >> (shift + 8)) == (prefix >> (shift + 8)); };
+    h = hist[c.he & 1];
     ++c.he;
     hist_clear(h);
-    if (round == 2 && threadIdx.x == 0) *n_few = 0;
-    if (round == 2) __syncthreads();
-    if (round == 3 && *n_few <= SAMP_LIST) {   // the entries that shared sixteen bits were listed in the round before
-      for (int i = threadIdx.x; i < *n_few; i += SAMP_THREADS) {
+    const int n = *n_few;
+    if (n <= SAMP_FEW) {
+      for (int i = threadIdx.x; i < n; i += SAMP_THREADS) {
         const uint32_t k = keyf(few[i]);
-        if ((k >> 8) == (prefix >> 8)) atomicAdd(&h[k & 255], __float2uint_rn(wf(few[i]) * SAMP_FIX));
+        if (counts(k)) atomicAdd(&h[(threadIdx.x & 3) * 256 + ((k >> shift) & 255)], wq(few[i]));
       }
     } else {
       for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
         const int i0 = base + threadIdx.x * 8;
         uint32_t digit[8], w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         if (i0 < hi) {
-          const bool listing = round == 2 && *n_few <= SAMP_LIST;
           float v[8];
           load(i0, v);
 #pragma unroll
           for (int e = 0; e < 8; ++e) {
-            // after the first round only ~1/256 of the entries still carry the selected prefix: test the (cheap) key first
-            // and evaluate the weight (an expf) for those only
             const uint32_t k = keyf(v[e]);
             digit[e] = (k >> shift) & 255;
-            if (round == 0 || (k >> (shift + 8)) == (prefix >> (shift + 8))) {
-              w[e] = __float2uint_rn(wf(v[e]) * SAMP_FIX);
-              if (listing) {
-                const int at = atomicAdd(n_few, 1);
-                if (at < SAMP_LIST) few[at] = v[e];
-              }
-            }
+            if (code(v[e]) == sel && counts(k)) w[e] = wq(v[e]);
           }
         }
-        hist_add8(h, digit, w);
+        hist_add8<256>(h, digit, w);
       }
     }
-    hist_fold(h);
-    radix_round_pick(c, h, hsum, bcast, below, T, strict, /*descending=*/false);
+    hist_fold<256>(h);
+    radix_round_pick<256>(c, h, hsum, bcast, before, T, strict, descending);
     prefix |= bcast[0] << shift;
-    below = bcast[1];
+    before = bcast[1];
   }
   return prefix;
 }
-
-// k-th largest key (k >= 1) by count
-template <class LoadF, class KeyF>
-__device__ uint32_t select_kth_largest(Cl& c, int lo, int hi, LoadF load, KeyF keyf, int k, uint32_t (*hist)[256 * HIST_COPIES], uint32_t* hsum,
-                                       uint32_t* bcast) {
-  uint32_t prefix = 0, above = 0;
-  for (int round = 0; round < 4; ++round) {
-    const int shift = 24 - 8 * round;
-    uint32_t* h = hist[c.he & 1];
-    ++c.he;
-    hist_clear(h);
-    for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
-      const int i0 = base + threadIdx.x * 8;
-      uint32_t digit[8], w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (i0 < hi) {
-        float v[8];
-        load(i0, v);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const uint32_t key = keyf(v[e]);
-          digit[e] = (key >> shift) & 255;
-          w[e] = round == 0 || (key >> (shift + 8)) == (prefix >> (shift + 8)) ? 1u : 0u;
-        }
-      }
-      hist_add8(h, digit, w);
-    }
-    hist_fold(h);
-    radix_round_pick(c, h, hsum, bcast, above, (uint32_t)k, false, /*descending=*/true);
-    prefix |= bcast[0] << shift;
-    above = bcast[1];
-  }
-  return prefix;
-}
+__device__ __forceinline__ uint32_t mass_target(float target) { return __float2uint_rn(fminf(fmaxf(target, 0.f), 2.f) * SAMP_FIX); }
 
 // ---------------------------------------------------------------- Philox4x32-10
 __device__ __forceinline__ uint4 philox4x32(uint4 ctr, uint2 key) {
@@ -567,16 +576,19 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
   extern __shared__ __align__(16) uint8_t dyn_smem[];
   __shared__ float redf[2 * SAMP_WARPS];
   __shared__ int redi[SAMP_WARPS];
-  __shared__ uint32_t hist[2][256 * HIST_COPIES];
-  __shared__ uint32_t hsum[256];
+  __shared__ uint32_t hist[2][HIST_WORDS];
+  __shared__ uint32_t hsum[CODES];
   __shared__ uint32_t bcast[4];
   __shared__ float4 xch[2];
   __shared__ RedBest redb[SAMP_WARPS];
   __shared__ float wmax[SAMP_WARPS];    // of the slice's raw entries, by warp
   __shared__ float cand_v[MAX_TOPN];
   __shared__ int cand_i[MAX_TOPN];
-  __shared__ float list_v[SAMP_LIST];   // in turn: a weighted selection's last candidates, what the race is run over, what can be among the top-n, the slices' best
-  __shared__ int list_i[SAMP_LIST];
+  // in turn: the entries of a selection's code, what the race is run over, what can be among the top-n, the slices' best
+  __shared__ uint32_t list_words[SAMP_FEW];
+  float* few = reinterpret_cast<float*>(list_words);
+  float* list_v = few;
+  int* list_i = reinterpret_cast<int*>(list_words + SAMP_LIST);
   __shared__ int list_n;
   STL_ENTER(6);
   griddep_launch();
@@ -716,8 +728,9 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
       const float lp = (x - rm) - lz;
       return __float_as_uint(fabsf((-lp) - ent));
     };
-    auto wf = [=](float x) { return expf((x - rm) - lz); };
-    const uint32_t k = select_weighted_asc(cl, lo, hi, load, keyf, wf, c.p.typical_p, false, hist, hsum, bcast, list_v, &list_n);
+    auto code = [=](float x) { return distance_code(fabsf((-((x - rm) - lz)) - ent)); };
+    auto wq = [=](float x) { return __float2uint_rn(expf((x - rm) - lz) * SAMP_FIX); };
+    const uint32_t k = select_key(cl, lo, hi, load, code, keyf, wq, mass_target(c.p.typical_p), false, false, hist, hsum, bcast, few, &list_n);
     c.typ_thr = __uint_as_float(k);
     c.typical = true;
   }
@@ -741,7 +754,8 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
     // entries are left, made again
     float mx = -INFINITY;
     const float temp = c.p.temperature;
-    const bool use_topk = c.p.top_k > 0 && c.p.top_k < V, use_topp = c.p.top_p < 1.0f, keep_y = use_topk || use_topp || !c.typical;
+    const bool use_topk = c.p.top_k > 0 && c.p.top_k < V, use_topp = c.p.top_p < 1.0f, 
+               keep_y = use_topk || use_topp || !c.typical || c.ent > SAMP_FLAT;
     auto scaled8 = [&](int i0, float (&v)[8]) {
       load_slice8(c, i0, v);
       process8(c, i0, v);
@@ -771,9 +785,14 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
     mx = cluster_max(cl, mx, redf, xch);
     // ---- top-k (S6): keep y >= k-th largest value
     float lo_thr = -INFINITY;
-    if (use_topk) {
-      auto keyf = [](float v) { return f2key(v); };
-      lo_thr = key2f(select_kth_largest(cl, lo, hi, load_y, keyf, c.p.top_k, hist, hsum, bcast));
+    auto keyf = [](float v) { return f2key(v); };
+    auto code = [=](float v) {   // of the distance below the maximum (no number: the maximum is infinite, or v is none)
+      const float t = mx - v;
+      return t == t ? CODES - 1 - distance_code(t) : CODES - 1;
+    };
+    if (use_topk) {   // (with fewer than k entries left it is the smallest of them)
+      auto wq = [](float v) { return v != -INFINITY ? 1u : 0u; };
+      lo_thr = key2f(select_key(cl, lo, hi, load_y, code, keyf, wq, (uint32_t)c.p.top_k, false, true, hist, hsum, bcast, few, &list_n));
     }
     // ---- top-p (S6): drop the low-probability tail whose cumulative mass <= 1 - p
     if (use_topp) {
@@ -787,9 +806,8 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
       }
       const float z = cluster_sumf(cl, part, redf, xch);
       const float lt = lo_thr;
-      auto keyf = [](float v) { return f2key(v); };
-      auto wf = [=](float v) { return (v >= lt) ? expf(v - mx) / z : 0.f; };
-      const uint32_t k = select_weighted_asc(cl, lo, hi, load_y, keyf, wf, 1.0f - c.p.top_p, true, hist, hsum, bcast, list_v, &list_n);
+      auto wq = [=](float v) { return v >= lt ? __float2uint_rn(expf(v - mx) / z * SAMP_FIX) : 0u; };
+      const uint32_t k = select_key(cl, lo, hi, load_y, code, keyf, wq, mass_target(1.0f - c.p.top_p), true, false, hist, hsum, bcast, few, &list_n);
       lo_thr = fmaxf(lo_thr, key2f(k));
     }
     // ---- exponential race == Gumbel max over the kept set
@@ -798,6 +816,9 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
     auto race = [&](float v, int i) {
       const uint4 rnd = philox4x32(make_uint4((uint32_t)i, c.p.step, 0u, 0u), key);
       const float u = ((float)(rnd.x >> 8) + 0.5f) * (1.0f / 16777216.0f);
+      // to be ahead, -log u has to be below e^(v - mx - best), and it is at least 1 - u: most entries need no logarithm (the
+      // margin is a thousand times the rounding of what is compared)
+      if (1.f - u > fmaf(__expf((v - mx) - bs.v), 1.001f, 1e-6f)) return;
       const float score = (v - mx) - logf(-logf(u));
       if (bs.i < 0 || score > bs.v) bs = {score, i};
     };
