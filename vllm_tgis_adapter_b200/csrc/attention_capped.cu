@@ -204,6 +204,13 @@ capattn_kernel(const CT* __restrict__ q, const CT* __restrict__ k_cache, const C
 // through ldmatrix.trans).  Scale, soft cap, mask and the running softmax are fp32 on the accumulator fragments; the
 // weights are rounded to bf16 once and the SAME rounded numbers are summed for the normaliser.  Rows padded by 16 bytes keep
 // every fragment load free of bank conflicts.  A row's arithmetic does not depend on the other rows of its tile.
+//
+// What bounds it is issue: 62 million warp instructions for 2048 tokens in 7 prompts and 16 heads, of which a tile's products, tanh and
+// exponentials are less than a third; the rest was division by sizes known only at run time, in the copies.  With 128-wide heads known
+// when it is compiled, two k-steps to a load of key fragments, no comparison of positions in blocks that every query sees, and the
+// tiles with the most keys first: 138 -> 75 us a layer; 32 single tokens behind 64 to 88 keys 14.4 -> 11.0.  Single tokens (ONE) fill
+// the M rows with the query heads of a key/value head instead of 15 rows of nothing, a quarter of the CTAs and of the copies: 11.0 ->
+// 8.0.  No faster: 32 queries a CTA (166 registers; 94 us), a warp per head of the group (186 registers; 89 us).
 constexpr int MMA_KS = 8, MMA_NT = 8;
 __device__ __forceinline__ void ca_ldsm_x4(uint32_t (&r)[4], const void* smem) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
@@ -224,6 +231,29 @@ __device__ __forceinline__ void ca_cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(a), "l"(gmem) : "memory");
 }
 
+// c += Q K^T of 16 queries and the 8 keys whose rows start at `row` (lane & 7), dims in ascending order; DIM > 0: known, a multiple of 32
+template <int DIM>
+__device__ __forceinline__ void score_tile(float (&c)[4], const uint32_t (&qa)[MMA_KS][4], const __nv_bfloat16* row, int lane, int nks) {
+  if constexpr (DIM > 0) {
+#pragma unroll
+    for (int ks = 0; ks < DIM / 16; ks += 2) {
+      uint32_t kb[4];
+      ca_ldsm_x4(kb, row + ks * 16 + (lane >> 3) * 8);
+      mma_16816(c, qa[ks], kb[0], kb[1]);
+      mma_16816(c, qa[ks + 1], kb[2], kb[3]);
+    }
+  } else {
+#pragma unroll
+    for (int ks = 0; ks < MMA_KS; ++ks)
+      if (ks < nks) {
+        uint32_t kb[2];
+        ca_ldsm_x2(kb, row + ks * 16 + ((lane >> 3) & 1) * 8);
+        mma_16816(c, qa[ks], kb[0], kb[1]);
+      }
+  }
+}
+
+template <int DIM, int VDIM, bool ONE>
 __global__ void __launch_bounds__(CA_THREADS)
 capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k_cache,
                    const __nv_bfloat16* __restrict__ v_cache, const AttnSeq* __restrict__ seqs,
@@ -231,7 +261,7 @@ capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
                    const float* __restrict__ gate, int gate_ld, __nv_bfloat16* __restrict__ out, CapAttnGeom g) {
   using bf = __nv_bfloat16;
   extern __shared__ __align__(16) uint8_t cam_smem[];
-  const int d = g.dim, dv = g.vdim, LDK = d + 8, LDV = dv + 8, LDP = KV_BLOCK + 8;
+  const int d = DIM > 0 ? DIM : g.dim, dv = DIM > 0 ? VDIM : g.vdim, LDK = d + 8, LDV = dv + 8, LDP = KV_BLOCK + 8;
   bf* Qs = reinterpret_cast<bf*>(cam_smem);            // [16][LDK]
   bf* Ks2 = Qs + CA_QT * LDK;                          // [2][32][LDK]   two blocks: one in use, the next one landing
   bf* Vs2 = Ks2 + 2 * KV_BLOCK * LDK;                  // [2][32][LDV]
@@ -239,16 +269,17 @@ capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   float* smax = reinterpret_cast<float*>(Ps + CA_QT * LDP);   // [4][16]; reused for the final row sums
   griddep_launch();
   griddep_wait();
-  const LatentTile tl = tiles[blockIdx.x];
+  const int per_tile = ONE ? g.kv_heads : g.heads;
+  const LatentTile tl = tiles[(gridDim.x - 1 - blockIdx.x) / per_tile];   // (a sequence's later tiles, which have more keys, first)
   const AttnSeq sq = seqs[tl.seq];
-  const int h = blockIdx.y, kvh = h / (g.heads / g.kv_heads);
+  const int gs = g.heads / g.kv_heads, hx = blockIdx.x % per_tile, h = ONE ? hx * gs : hx, kvh = ONE ? hx : h / gs;   // ONE: row r is head h + r
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t2 = (lane & 3) * 2;
-  const int row0 = sq.q_start + tl.q0, pos0 = sq.kv_len - sq.q_len + tl.q0, nq = tl.nq;
+  const int row0 = sq.q_start + tl.q0, pos0 = sq.kv_len - sq.q_len + tl.q0, nq = ONE ? gs : tl.nq, last = ONE ? 1 : nq;
   const int dch = d / 8, vch = dv / 8;   // 16-byte chunks per row
   for (int i = tid; i < CA_QT * dch; i += CA_THREADS) {
     const int qi = i / dch, ch = i % dch;
     uint4 v = make_uint4(0, 0, 0, 0);
-    if (qi < nq) v = *reinterpret_cast<const uint4*>(q + ((size_t)(row0 + qi) * g.heads + h) * d + ch * 8);
+    if (qi < nq) v = *reinterpret_cast<const uint4*>(q + (ONE ? (size_t)row0 * g.heads + h + qi : (size_t)(row0 + qi) * g.heads + h) * d + ch * 8);
     *reinterpret_cast<uint4*>(Qs + qi * LDK + ch * 8) = v;
   }
   __syncthreads();
@@ -261,7 +292,7 @@ capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 #pragma unroll
   for (int j = 0; j < MMA_NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
   float m_run[2] = {-INFINITY, -INFINITY}, l_part[2] = {0.f, 0.f};   // rows gq and gq + 8
-  const int n_blocks = (pos0 + nq - 1) / KV_BLOCK + 1;
+  const int n_blocks = (pos0 + last - 1) / KV_BLOCK + 1;
   const int32_t* bt = block_table + (size_t)sq.block_row * bt_stride;
   const float inv_cap = g.softcap > 0.f ? 1.f / g.softcap : 0.f;
   // block b's K and V rows -> buffer b & 1, as 16-byte asynchronous copies (one commit group per block)
@@ -269,10 +300,12 @@ capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     const size_t blk = (size_t)bt[b];
     bf* Kd = Ks2 + (size_t)(b & 1) * KV_BLOCK * LDK;
     bf* Vd = Vs2 + (size_t)(b & 1) * KV_BLOCK * LDV;
+#pragma unroll 4
     for (int i = tid; i < KV_BLOCK * dch; i += CA_THREADS) {
       const int j = i / dch, ch = i % dch;
       ca_cp_async16(Kd + j * LDK + ch * 8, k_cache + ((blk * KV_BLOCK + j) * g.kv_heads + kvh) * d + ch * 8);
     }
+#pragma unroll 4
     for (int i = tid; i < KV_BLOCK * vch; i += CA_THREADS) {
       const int j = i / vch, ch = i % vch;
       ca_cp_async16(Vd + j * LDV + ch * 8, v_cache + ((blk * KV_BLOCK + j) * g.kv_heads + kvh) * dv + ch * 8);
@@ -293,18 +326,13 @@ capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     const bf* Vs = Vs2 + (size_t)(b & 1) * KV_BLOCK * LDV;
     // ---- scores of this warp's 8 keys
     float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int ks = 0; ks < MMA_KS; ++ks)
-      if (ks < nks) {
-        uint32_t kb[2];
-        ca_ldsm_x2(kb, Ks + (size_t)(warp * 8 + (lane & 7)) * LDK + ks * 16 + ((lane >> 3) & 1) * 8);
-        mma_16816(c, qa[ks], kb[0], kb[1]);
-      }
+    score_tile<DIM>(c, qa, Ks + (warp * 8 + (lane & 7)) * LDK, lane, nks);
+    const bool all = nq == CA_QT && (b + 1) * KV_BLOCK - 1 <= pos0;   // no key of the block is behind one of the tile's queries
     bool ok[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int qi = gq + (e >> 1) * 8, kpos = b * KV_BLOCK + warp * 8 + t2 + (e & 1);
-      ok[e] = qi < nq && kpos <= pos0 + qi;
+      ok[e] = all || (qi < nq && kpos <= pos0 + (ONE ? 0 : qi));
       float sc = c[e] * g.scale;
       if (g.softcap > 0.f) sc = g.softcap * tanhf(sc * inv_cap);
       c[e] = ok[e] ? sc : -INFINITY;
@@ -343,7 +371,7 @@ capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
 #pragma unroll
     for (int j = 0; j < MMA_NT; ++j) {
       const int n0 = (warp + 4 * j) * 8;
-      if (n0 < dv) {
+      if (DIM > 0 ? 32 * j < VDIM : n0 < dv) {   // (VDIM: a multiple of 32)
         acc[j][0] *= al[0]; acc[j][1] *= al[0]; acc[j][2] *= al[1]; acc[j][3] *= al[1];
         uint32_t vb[4];
         ca_ldsm_x4_trans(vb, Vs + (size_t)lane * LDV + n0);
@@ -370,20 +398,21 @@ capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
     const int qi = gq + r * 8;
     if (qi >= nq) continue;
     const float inv_l = 1.f / (smax[qi] + smax[CA_QT + qi] + smax[2 * CA_QT + qi] + smax[3 * CA_QT + qi]);
-    const size_t row = (size_t)(row0 + qi);
+    const size_t row = ONE ? (size_t)row0 : (size_t)(row0 + qi);
+    const int hr = ONE ? h + qi : h;
 #pragma unroll
     for (int j = 0; j < MMA_NT; ++j) {
       const int n = (warp + 4 * j) * 8 + t2;
-      if (n < dv) {
+      if (DIM > 0 ? 32 * j < VDIM : n < dv) {
         float o0 = acc[j][2 * r] * inv_l, o1 = acc[j][2 * r + 1] * inv_l;
         if (gate != nullptr) {
-          const float* gr = gate + row * gate_ld + (size_t)h * dv + n;
+          const float* gr = gate + row * gate_ld + (size_t)hr * dv + n;
           o0 *= 1.f / (1.f + expf(-gr[0]));
           o1 *= 1.f / (1.f + expf(-gr[1]));
         }
         __nv_bfloat162 pk;
         pk.x = __float2bfloat16_rn(o0); pk.y = __float2bfloat16_rn(o1);
-        *reinterpret_cast<__nv_bfloat162*>(out + (row * g.heads + h) * dv + n) = pk;
+        *reinterpret_cast<__nv_bfloat162*>(out + (row * g.heads + hr) * dv + n) = pk;
       }
     }
   }
@@ -598,7 +627,7 @@ cudaError_t capattn_prep_launch(const float* y, int ldy, int q_off, int k_off, i
 cudaError_t capattn_launch(const void* q, const void* k_cache, const void* v_cache, int dtype, const AttnSeq* seqs,
                            const LatentTile* tiles, int n_tiles, const int32_t* block_table, int bt_stride,
                            const float* gate, int gate_ld, void* out, int out_dtype, const CapAttnGeom& g,
-                           cudaStream_t stream) {
+                           cudaStream_t stream, bool single) {
   if (n_tiles <= 0) return cudaSuccess;
   if (g.heads < 1 || g.kv_heads < 1 || g.heads % g.kv_heads != 0 || g.heads > 65535 || g.dim < 1 || g.vdim < 1 ||
       g.vdim > CAPATTN_MAX_VDIM || capattn_smem(g) > 200 * 1024 || out_dtype != dtype)
@@ -614,13 +643,13 @@ cudaError_t capattn_launch(const void* q, const void* k_cache, const void* v_cac
   if (dtype == DT_BF16 && capattn_mma_eligible(g, q, k_cache, v_cache, out)) {
     const size_t smem = ((size_t)(CA_QT + 2 * KV_BLOCK) * (g.dim + 8) + (size_t)2 * KV_BLOCK * (g.vdim + 8) + CA_QT * (KV_BLOCK + 8)) * sizeof(bf) +
                         4 * CA_QT * sizeof(float);   // <= 58 KB
-    static bool attr_set = false;
-    if (!attr_set) {
-      const cudaError_t e = cudaFuncSetAttribute(capattn_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    const bool known = g.dim == 128 && g.vdim == 128, one = single && known && g.heads / g.kv_heads <= CA_QT;
+    const auto kernel = !known ? capattn_mma_kernel<0, 0, false> : one ? capattn_mma_kernel<128, 128, true> : capattn_mma_kernel<128, 128, false>;
+    if (smem > 48 * 1024) {
+      static const cudaError_t e = cudaFuncSetAttribute(capattn_mma_kernel<0, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);   // (the others: 42 KB)
       if (e != cudaSuccess) return e;
-      attr_set = true;
     }
-    return launch_k(capattn_mma_kernel, dim3(n_tiles, g.heads), dim3(CA_THREADS), smem, stream, reinterpret_cast<const bf*>(q),
+    return launch_k(kernel, dim3((unsigned)n_tiles * (one ? g.kv_heads : g.heads)), dim3(CA_THREADS), smem, stream, reinterpret_cast<const bf*>(q),
                     reinterpret_cast<const bf*>(k_cache), reinterpret_cast<const bf*>(v_cache), seqs, tiles, block_table, bt_stride,
                     gate, gate_ld, reinterpret_cast<bf*>(out), g);
   }

@@ -2474,7 +2474,7 @@ struct tgis_engine {
       CK(capattn_prep_launch(pnx_y1, ld, l.c_q, l.c_k, l.c_v, l.ca, l.qk_norm, l.qk_norm + s.dim, eps, d_pos, d_slot, pnx_q,
                              l.k_cache, l.v_cache, A, T, stream));
       CK(capattn_launch(pnx_q, l.k_cache, l.v_cache, A, d_seqs, ds<LatentTile>(off_ltiles), step_n_ltiles, ds<int32_t>(off_bt),
-                        bt_stride, pnx_y1 + l.c_g, ld, pnx_oA, A, l.ca, stream));
+                        bt_stride, pnx_y1 + l.c_g, ld, pnx_oA, A, l.ca, stream, T == S));
       pnx_gemm(pnx_oA, A, H * s.vdim, l.w_o, pnx_o, DT_F32, W, T, W, H * s.vdim);
       OuterScan os{};
       os.single = T == S;

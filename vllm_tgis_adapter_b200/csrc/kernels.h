@@ -533,7 +533,7 @@ cudaError_t capattn_prep_launch(const float* y, int ldy, int q_off, int k_off, i
 cudaError_t capattn_launch(const void* q, const void* k_cache, const void* v_cache, int dtype, const AttnSeq* seqs,
                            const LatentTile* tiles, int n_tiles, const int32_t* block_table, int bt_stride,
                            const float* gate, int gate_ld, void* out, int out_dtype, const CapAttnGeom& g,
-                           cudaStream_t stream);
+                           cudaStream_t stream, bool single);   // single: one token a sequence, a tile each
 
 // ---- attention_sigmoid.cu: grouped-query attention with rotary positions, a window, and sigmoid weights -------------------
 // weight(i, j) = sigmoid(scale * q_h(i) . k_g(j) + head_bias[h]) for 0 <= i - j < window (window <= 0: every earlier position),

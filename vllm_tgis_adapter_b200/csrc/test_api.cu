@@ -788,7 +788,7 @@ int tgis_k_capattn(const void* q, const void* k_cache, const void* v_cache, int3
   KCK(d_tiles.upload(tiles.data(), tiles.size()));
   KCK(d_bt.upload(block_table_host, (size_t)bt_rows * bt_stride));
   KCK(capattn_launch(q, k_cache, v_cache, dt, d_seqs.p, d_tiles.p, (int)tiles.size(), d_bt.p, bt_stride, gate, gate_ld, out, dt,
-                     to_cap(g), 0));
+                     to_cap(g), 0, std::all_of(seqs.begin(), seqs.end(), [](const AttnSeq& s) { return s.q_len == 1; })));
   KCK(cudaDeviceSynchronize());
   return 0;
 }
