@@ -163,11 +163,6 @@ int tgis_k_latent_q_rope(const void* q, int32_t q_dt, const tgis_k_latent_geom* 
 int tgis_k_latent_attn(const float* q_abs, const void* cache, int32_t dt, const int32_t* seqs_host, int32_t n_seqs,
                        const int32_t* block_table_host, int32_t bt_rows, int32_t bt_stride, void* o_lat, int32_t o_dt,
                        const tgis_k_latent_geom* g);
-// The same attention in head space (attention_heads.cu): q bf16 [T][heads][192] (its rotary part is turned in place), kv bf16 [keys][heads][128] |
-// [heads][128] made from the gathered rows by w_ukv [heads * 256, kv_rank] (nullptr: given); -3: not a geometry it takes, -4: a wait ran out
-int tgis_k_latent_heads(void* q, const void* cache, const void* w_ukv, const int32_t* positions, const float* cos_sin, const float* gate, const float* sink,
-                        const int32_t* seqs_host, int32_t n_seqs, const int32_t* block_table_host, int32_t bt_rows, int32_t bt_stride, void* kv, void* out,
-                        const tgis_k_latent_geom* g);
 int tgis_k_moe_route(const float* logits, int32_t ld, const float* bias, int32_t E, int32_t top, int32_t* ids, float* w,
                      float* side_gate, int32_t T);
 /* scores softmax(logits) over E outputs, the `top` largest of score + bias among the `keep` best of `groups` equal groups; w: the chosen

@@ -272,7 +272,6 @@ struct tgis_engine {
     LatentGeom g{};
     void *w_down = nullptr, *w_uq = nullptr, *w_ukT = nullptr, *w_uv = nullptr, *w_o = nullptr;   // operand type
     float *norm1 = nullptr, *norm1b = nullptr, *norm2 = nullptr, *norm2b = nullptr, *qnorm = nullptr, *kvnorm = nullptr;
-    void* w_ukv = nullptr;           // attention_heads.cu: the heads' key rows [heads * dim, kv_rank], w_uv under them (nullptr: w_uv by itself)
     const float* cos_sin = nullptr;  // [max_model_len][rot_dims]
     void* cache = nullptr;           // [num_blocks][KV_BLOCK][kv_rank + rot_dim], operand type
     void *w_router = nullptr, *w_gu_e = nullptr, *w_d_e = nullptr, *w_gu_s = nullptr, *w_d_s = nullptr;
@@ -380,15 +379,6 @@ struct tgis_engine {
   float* pnx_attn_ws = nullptr;                      // split partials of decode-shaped attention launches
   size_t pnx_attn_ws_floats = 0;
   size_t off_ltiles = 0;
-  // prompts of latent layers that attend in head space (attention_heads.cu): gathered keys, and what the step's launches read
-  bool heads_any = false, heads_no_window = false;
-  int heads_window = 0, heads_cap = 0;               // the widest window of such layers; keys of one pass
-  void *lat_rows = nullptr, *lat_rot = nullptr, *lat_kv = nullptr;
-  size_t off_lspans = 0, off_lunits = 0;
-  struct HeadsPass { int span0, n_spans, n_blocks, unit0, n_units, n_keys; };
-  std::vector<HeadsPass> step_heads;
-  std::vector<LatentTile> heads_tiles;
-  int step_rest_T = 0, step_rest_tiles = 0, step_rest_seqs = 0;   // of the sequences that do not: leading tokens, tiles, number
   int logit_rows_cap = 0;                            // rows of the logits buffer (>= max_num_seqs)
   int logits_ld = 0;                                 // its row length: the vocabulary rounded up to the sampler's 8-column
                                                      // vectors; the padding columns hold -inf for good
@@ -770,8 +760,6 @@ struct tgis_engine {
     off_epoch = place(4 * sizeof(uint32_t));  // tensor parallelism: exchange epochs before this step ([0], [1]: per
                                                // parity) and the logits-gather epoch ([2])
     off_ltiles = place(sizeof(LatentTile) * (size_t)(T_max + S_max));  // attention query tiles of the layer-list architectures
-    off_lspans = place(sizeof(LatentSpan) * (size_t)S_max);
-    off_lunits = place(sizeof(LatentUnit) * (size_t)(T_max / 256 + S_max));
     off_ltiles16 = place(sizeof(LatentTile) * (size_t)(T_max / POOLATTN_TILE + S_max + 1));
     off_bt = place(4 * (size_t)S_max * bt_stride);
     // decode work items follow the USED part of the block table (items_off(S)); room for the worst case
@@ -1265,22 +1253,6 @@ struct tgis_engine {
     pnx_allocs.push_back(q);
     return reinterpret_cast<T*>(q);
   }
-  // w_uv, and where the layer's prompts can attend in head space the keys' rows in front of it
-  void latent_up_weights(PnxLayer& l, size_t& m_kv, size_t& m_rank) {
-    const tgis_layer_spec& s = l.sp;
-    const size_t uk = (size_t)s.heads * s.dim * s.kv_rank, uv = (size_t)s.heads * s.vdim * s.kv_rank;
-    if (!pnx_tc || cfg.debug_gemm_ref || !latent_heads_takes(l.g, pnx_dt)) {
-      l.w_uv = pnx_alloc_dt(uv);
-      return;
-    }
-    l.w_ukv = pnx_alloc_dt(uk + uv);
-    l.w_uv = reinterpret_cast<bf16*>(l.w_ukv) + uk;
-    heads_any = true;
-    heads_no_window |= s.window <= 0;
-    heads_window = std::max(heads_window, s.window);
-    m_kv = std::max(m_kv, (size_t)s.heads * (s.dim + s.vdim));
-    m_rank = std::max<size_t>(m_rank, s.kv_rank);
-  }
   void* pnx_alloc_dt(size_t count, bool zero = false) {
     return pnx_alloc<uint8_t>(count * dt_size(pnx_dt), zero);
   }
@@ -1362,7 +1334,7 @@ struct tgis_engine {
       pnx_expected_tensors += 2;  // final.norm.b, final.norm.alpha
     }
     size_t m_f1 = 1, m_f2 = 1, m_f3 = 1, m_mix = 1;
-    size_t m_down = 1, m_qr = 1, m_q = 1, m_qabs = 1, m_olat = 1, m_latkv = 1, m_latrank = 1, m_ov = 1, m_heads = 1, m_E = 1, m_top = 1, m_ff = 1, m_ffs = 1;
+    size_t m_down = 1, m_qr = 1, m_q = 1, m_qabs = 1, m_olat = 1, m_ov = 1, m_heads = 1, m_E = 1, m_top = 1, m_ff = 1, m_ffs = 1;
     size_t cache_row_bytes = 0;
     pnx_tile_tokens = LATENT_PAIRS;
     pnx_layers.resize(pnx_layer_specs.size());
@@ -1428,7 +1400,7 @@ struct tgis_engine {
           l.w_down = pnx_alloc_dt((size_t)l.n_down() * W);
           l.w_uq = pnx_alloc_dt((size_t)s.heads * hd * s.q_rank);
           l.w_ukT = pnx_alloc_dt((size_t)s.heads * s.kv_rank * s.dim);
-          latent_up_weights(l, m_latkv, m_latrank);
+          l.w_uv = pnx_alloc_dt((size_t)s.heads * s.vdim * s.kv_rank);
           l.w_o = pnx_alloc_dt(W * s.heads * s.vdim);
           l.qnorm = pnx_alloc<float>(s.q_rank);
           l.kvnorm = pnx_alloc<float>(s.kv_rank);
@@ -1768,7 +1740,7 @@ struct tgis_engine {
       l.w_down = pnx_alloc_dt((size_t)l.n_down() * W);
       l.w_uq = pnx_alloc_dt((size_t)s.heads * hd * s.q_rank);
       l.w_ukT = pnx_alloc_dt((size_t)s.heads * s.kv_rank * s.dim);
-      latent_up_weights(l, m_latkv, m_latrank);
+      l.w_uv = pnx_alloc_dt((size_t)s.heads * s.vdim * s.kv_rank);
       l.w_o = pnx_alloc_dt(W * s.heads * s.vdim);
       l.norm1 = pnx_alloc<float>(W);
       l.norm1b = pnx_alloc<float>(W);
@@ -1860,13 +1832,6 @@ struct tgis_engine {
     pnx_q = pnx_alloc_dt(T * m_q, true);
     pnx_qabs = pnx_alloc<float>(T * m_qabs);
     pnx_olat = pnx_alloc_dt(T * m_olat, true);
-    if (heads_any) {
-      // a portion's keys: the longest context or a step's tokens, whichever is more, up to 16384 (150 MB with 16 heads)
-      heads_cap = std::min(std::max(T_max, cfg.max_model_len), 16384);
-      lat_rows = pnx_alloc_dt((size_t)heads_cap * m_latrank, true);
-      lat_rot = pnx_alloc_dt((size_t)heads_cap * LATENT_HEAD_ROT, true);
-      lat_kv = pnx_alloc_dt((size_t)heads_cap * m_latkv, true);
-    }
     pnx_oA = pnx_alloc_dt(T * m_ov, true);
     pnx_o = pnx_alloc<float>(T * W);
     pnx_rl = pnx_alloc<float>(T * m_E);
@@ -1995,16 +1960,13 @@ struct tgis_engine {
       return 0;
     };
     // [heads * dim, kv_rank] -> per head the transpose [kv_rank, dim]: the matrix that folds a key up-projection into the query
-    // [heads * dim, kv_rank] -> per head the transpose [kv_rank, dim]: the matrix that folds W_uk into the query (and as it is, for prompts)
-    auto place_uk = [&](PnxLayer& l) -> int {
-      const tgis_layer_spec& s = l.sp;
-      if (n != (int64_t)s.heads * s.dim * s.kv_rank) return bad_shape();
-      for (int h = 0; h < s.heads; ++h) {
-        const cudaError_t e = weight_place_launch(tmp_src + (size_t)h * s.dim * s.kv_rank, s.dim, s.kv_rank,
-                                                  at(l.w_ukT, (size_t)h * s.kv_rank * s.dim), pnx_dt, 1, s.dim, 0);
+    auto place_ukT = [&](void* dst, int heads, int dim, int kv_rank) -> int {
+      if (n != (int64_t)heads * dim * kv_rank) return bad_shape();
+      for (int h = 0; h < heads; ++h) {
+        const cudaError_t e = weight_place_launch(tmp_src + (size_t)h * dim * kv_rank, dim, kv_rank,
+                                                  at(dst, (size_t)h * kv_rank * dim), pnx_dt, 1, dim, 0);
         if (e != cudaSuccess) return fail("weight placement failed for " + name);
       }
-      if (l.w_ukv != nullptr) return mat(l.w_ukv, (int64_t)s.heads * s.dim, s.kv_rank);
       if (cudaDeviceSynchronize() != cudaSuccess) return fail("weight placement failed for " + name);
       pnx_loaded.insert(name);
       return 0;
@@ -2081,7 +2043,7 @@ struct tgis_engine {
         if (sub == "mix.dq.norm") return vec(l.qnorm, s.q_rank);
         if (sub == "mix.dkv.norm") return vec(l.kvnorm, s.kv_rank);
         if (sub == "mix.uq") return mat(l.w_uq, s.heads * hd, s.q_rank);
-        if (sub == "mix.uk") return place_uk(l);
+        if (sub == "mix.uk") return place_ukT(l.w_ukT, s.heads, s.dim, s.kv_rank);
         if (sub == "mix.uv") return mat(l.w_uv, (int64_t)s.heads * s.vdim, s.kv_rank);
         if (sub == "mix.sink" && l.sink != nullptr) return vec(l.sink, s.heads);
         if (sub == "mix.o") return mat(l.w_o, W, (int64_t)s.heads * s.vdim);
@@ -2346,7 +2308,18 @@ struct tgis_engine {
     if (sub == "mix.dq.norm") return vec(l.qnorm, s.q_rank);
     if (sub == "mix.dkv.norm") return vec(l.kvnorm, s.kv_rank);
     if (sub == "mix.uq") return mat(l.w_uq, s.heads * hd, s.q_rank);
-    if (sub == "mix.uk") return place_uk(l);
+    if (sub == "mix.uk") {
+      // [heads * dim, kv_rank] -> per head the transpose [kv_rank, dim]: the matrix that folds W_uk into the query
+      if (n != (int64_t)s.heads * s.dim * s.kv_rank) return bad_shape();
+      for (int h = 0; h < s.heads; ++h) {
+        const cudaError_t e = weight_place_launch(tmp_src + (size_t)h * s.dim * s.kv_rank, s.dim, s.kv_rank,
+                                                  at(l.w_ukT, (size_t)h * s.kv_rank * s.dim), pnx_dt, 1, s.dim, 0);
+        if (e != cudaSuccess) return fail("weight placement failed for " + name);
+      }
+      if (cudaDeviceSynchronize() != cudaSuccess) return fail("weight placement failed for " + name);
+      pnx_loaded.insert(name);
+      return 0;
+    }
     if (sub == "mix.uv") return mat(l.w_uv, (int64_t)s.heads * s.vdim, s.kv_rank);
     if (sub == "mix.o") return mat(l.w_o, W, (int64_t)s.heads * s.vdim);
     if (s.mlp != TGIS_MLP_MOE) return fail("unknown layer weight " + name);
@@ -2386,7 +2359,6 @@ struct tgis_engine {
   size_t pnx_yE_bytes = 0;
   size_t pnx_rows_alloc = 0;  // rows of every activation buffer (>= 256: a TMA box never leaves the allocation)
   bool pnx_gemm_tc(const void* X, const void* Wt, void* Y, int ldy, int T, int N, int K, int out_mode) {
-    const int x_rows = X == lat_rows ? heads_cap : pnx_rows_alloc;   // of X's allocation
     auto wit = pnx_wmaps.find(Wt);
     if (wit == pnx_wmaps.end()) {
       CUtensorMap m;
@@ -2398,7 +2370,7 @@ struct tgis_engine {
     auto xit = pnx_xmaps.find(xkey);
     if (xit == pnx_xmaps.end()) {
       CUtensorMap m;
-      if (make_tmap_bf16_2d(&m, X, (uint64_t)x_rows, (uint64_t)K, (uint64_t)K, BT_VALUES[bi], 64) != 0) return false;
+      if (make_tmap_bf16_2d(&m, X, (uint64_t)pnx_rows_alloc, (uint64_t)K, (uint64_t)K, BT_VALUES[bi], 64) != 0) return false;
       xit = pnx_xmaps.emplace(xkey, m).first;
     }
     CK(gemm_bf16_launch(wit->second, xit->second, Y, ldy, T, N, K, on_side_stream ? gemm_ws2.p : gemm_ws.p,
@@ -2662,54 +2634,6 @@ struct tgis_engine {
     pnx_dump_resid(T);
   }
 
-  // Latent attention of a layer: pnx_q [T][heads][dim + rot_dim] -> pnx_oA [T][heads][vdim], times the heads' gates (nullptr: none).
-  // Single tokens and short portions in the folded form, the first step_rest_T tokens; other portions in head space, over rows of pnx_oA
-  // that the first have left undefined.
-  void latent_attend(PnxLayer& l, const float* gate, int T, int S) {
-    const tgis_layer_spec& s = l.sp;
-    const LatentGeom& g = l.g;
-    const int A = pnx_dt, H = s.heads, hd = s.dim + s.rot_dim, D = g.row();
-    const int32_t* d_pos = ds<int32_t>(off_pos);
-    const AttnSeq* d_seqs = ds<AttnSeq>(off_seqs);
-    const int32_t* d_bt = ds<int32_t>(off_bt);
-    const bool split = l.w_ukv != nullptr && !step_heads.empty();
-    const int Tf = split ? step_rest_T : T;
-    if (Tf > 0) {
-      CK(latent_q_rope_launch(pnx_q, A, g, d_pos, l.cos_sin, pnx_qabs, Tf, stream));
-      {  // q_abs_h = W_uk,h^T q_plain_h  (one problem per head)
-        GemmAny a{};
-        a.X = pnx_q; a.W = l.w_ukT; a.Y = pnx_qabs;
-        a.x_dtype = A; a.w_dtype = A; a.y_dtype = DT_F32;
-        a.T = Tf; a.N = s.kv_rank; a.K = s.dim; a.ldx = H * hd; a.ldw = s.dim; a.ldy = H * D;
-        a.batch = H; a.x_bs = hd; a.w_bs = (long long)s.kv_rank * s.dim; a.y_bs = D;
-        CK(gemm_any_launch(a, stream));
-      }
-      int attn_launches = 0;
-      CK(latent_attn_launch(pnx_qabs, l.cache, A, d_seqs, ds<LatentTile>(off_ltiles), split ? step_rest_tiles : step_n_ltiles, d_bt, bt_stride,
-                            pnx_olat, A, g, stream, pnx_attn_ws, pnx_attn_ws_floats, step_max_kv, num_sms, &attn_launches,
-                            split ? step_rest_seqs : S, pnx_tile_tokens));
-      {  // o_h = W_uv,h o_lat_h  (times the head's gate where the layer has one)
-        GemmAny a{};
-        a.X = pnx_olat; a.W = l.w_uv; a.Y = pnx_oA;
-        a.x_dtype = A; a.w_dtype = A; a.y_dtype = A;
-        a.T = Tf; a.N = s.vdim; a.K = s.kv_rank; a.ldx = H * s.kv_rank; a.ldw = s.kv_rank; a.ldy = H * s.vdim;
-        a.batch = H; a.x_bs = s.kv_rank; a.w_bs = (long long)s.vdim * s.kv_rank; a.y_bs = s.vdim;
-        if (gate != nullptr) { a.mode = GEMM_ANY_ROWSCALE; a.row_scale = gate; a.scale_ld = H; }
-        CK(gemm_any_launch(a, stream));
-      }
-      n_launches += 3 + attn_launches;
-    }
-    if (!split) return;
-    for (size_t i = 0; i < step_heads.size(); ++i) {
-      const HeadsPass& p = step_heads[i];
-      CK(latent_rows_launch(l.cache, ds<LatentSpan>(off_lspans) + p.span0, p.n_blocks, d_bt, bt_stride, lat_rows, lat_rot, pnx_q, g, d_pos, l.cos_sin,
-                            i == 0 ? T : 0, stream));
-      pnx_gemm(lat_rows, A, s.kv_rank, l.w_ukv, lat_kv, A, H * (s.dim + s.vdim), p.n_keys, H * (s.dim + s.vdim), s.kv_rank);
-      CK(latent_heads_launch(pnx_q, T, lat_kv, lat_rot, p.n_keys, ds<LatentUnit>(off_lunits) + p.unit0, p.n_units, gate, pnx_oA, g, num_sms, stream));
-      n_launches += 2;
-    }
-  }
-
   // One layer run of the parallel pair style (TGIS_STYLE_PARALLEL_PAIR).  On entry pnx_hA holds rms(x) * g1 and pnx_hB rms(x) * g2
   // (operand type; hB only when the layer has a feed-forward):
   //   x += mixer(hA) + ff(hB);   x += rms(P (gelu_tanh(G x) * e)) * w   (the per-layer token input; e: the layer's slice of the
@@ -2778,8 +2702,29 @@ struct tgis_engine {
       CK(latent_prep_launch(pnx_y1, l.n_down(), g, l.qnorm, l.kvnorm, eps, d_pos, d_slot, l.cos_sin, pnx_cq, l.cache, A,
                             l.out_gate ? pnx_gate : nullptr, T, stream));
       pnx_gemm(pnx_cq, A, s.q_rank, l.w_uq, pnx_q, A, H * hd, T, H * hd, s.q_rank);
-      ++n_launches;
-      latent_attend(l, l.out_gate ? pnx_gate : nullptr, T, S);
+      CK(latent_q_rope_launch(pnx_q, A, g, d_pos, l.cos_sin, pnx_qabs, T, stream));
+      {  // q_abs_h = W_uk,h^T q_plain_h  (one problem per head)
+        GemmAny a{};
+        a.X = pnx_q; a.W = l.w_ukT; a.Y = pnx_qabs;
+        a.x_dtype = A; a.w_dtype = A; a.y_dtype = DT_F32;
+        a.T = T; a.N = s.kv_rank; a.K = s.dim; a.ldx = H * hd; a.ldw = s.dim; a.ldy = H * D;
+        a.batch = H; a.x_bs = hd; a.w_bs = (long long)s.kv_rank * s.dim; a.y_bs = D;
+        CK(gemm_any_launch(a, stream));
+      }
+      int attn_launches = 0;
+      CK(latent_attn_launch(pnx_qabs, l.cache, A, d_seqs, ds<LatentTile>(off_ltiles), step_n_ltiles, d_bt, bt_stride, pnx_olat, A, g,
+                            stream, pnx_attn_ws, pnx_attn_ws_floats, step_max_kv, num_sms, &attn_launches, S, pnx_tile_tokens));
+      n_launches += attn_launches - 1;
+      {  // o_h = W_uv,h o_lat_h  (times the head's gate where the layer has one)
+        GemmAny a{};
+        a.X = pnx_olat; a.W = l.w_uv; a.Y = pnx_oA;
+        a.x_dtype = A; a.w_dtype = A; a.y_dtype = A;
+        a.T = T; a.N = s.vdim; a.K = s.kv_rank; a.ldx = H * s.kv_rank; a.ldw = s.kv_rank; a.ldy = H * s.vdim;
+        a.batch = H; a.x_bs = s.kv_rank; a.w_bs = (long long)s.vdim * s.kv_rank; a.y_bs = s.vdim;
+        if (l.out_gate) { a.mode = GEMM_ANY_ROWSCALE; a.row_scale = pnx_gate; a.scale_ld = H; }
+        CK(gemm_any_launch(a, stream));
+      }
+      n_launches += 5;
       pnx_gemm(pnx_oA, A, H * s.vdim, l.w_o, pnx_o, DT_F32, W, T, W, H * s.vdim);
     }
     if (forked) CK(cudaStreamWaitEvent(stream, ev_join, 0));
@@ -3159,8 +3104,29 @@ struct tgis_engine {
       CK(latent_prep_launch(pnx_y1, l.n_down(), g, l.qnorm, l.kvnorm, eps, d_pos, d_slot, l.cos_sin, pnx_cq, l.cache, A,
                             pnx_gate, T, stream));
       pnx_gemm(pnx_cq, A, s.q_rank, l.w_uq, pnx_q, A, H * hd, T, H * hd, s.q_rank);
-      ++n_launches;
-      latent_attend(l, pnx_gate, T, S);
+      CK(latent_q_rope_launch(pnx_q, A, g, d_pos, l.cos_sin, pnx_qabs, T, stream));
+      {  // q_abs_h = W_uk,h^T q_nope_h  (one problem per head)
+        GemmAny a{};
+        a.X = pnx_q; a.W = l.w_ukT; a.Y = pnx_qabs;
+        a.x_dtype = A; a.w_dtype = A; a.y_dtype = DT_F32;
+        a.T = T; a.N = s.kv_rank; a.K = s.dim; a.ldx = H * hd; a.ldw = s.dim; a.ldy = H * D;
+        a.batch = H; a.x_bs = hd; a.w_bs = (long long)s.kv_rank * s.dim; a.y_bs = D;
+        CK(gemm_any_launch(a, stream));
+      }
+      int attn_launches = 0;
+      CK(latent_attn_launch(pnx_qabs, l.cache, A, d_seqs, d_tiles, step_n_ltiles, d_bt, bt_stride, pnx_olat, A, g, stream,
+                            pnx_attn_ws, pnx_attn_ws_floats, step_max_kv, num_sms, &attn_launches, S, pnx_tile_tokens));
+      n_launches += attn_launches - 1;  // (one attention launch is part of the count below)
+      {  // o_h = gate_h * W_uv,h o_lat_h
+        GemmAny a{};
+        a.X = pnx_olat; a.W = l.w_uv; a.Y = pnx_oA;
+        a.x_dtype = A; a.w_dtype = A; a.y_dtype = A;
+        a.T = T; a.N = s.vdim; a.K = s.kv_rank; a.ldx = H * s.kv_rank; a.ldw = s.kv_rank; a.ldy = H * s.vdim;
+        a.batch = H; a.x_bs = s.kv_rank; a.w_bs = (long long)s.vdim * s.kv_rank; a.y_bs = s.vdim;
+        a.mode = GEMM_ANY_ROWSCALE; a.row_scale = pnx_gate; a.scale_ld = H;
+        CK(gemm_any_launch(a, stream));
+      }
+      n_launches += 5;
       pnx_gemm(pnx_oA, A, H * s.vdim, l.w_o, pnx_o, DT_F32, W, T, W, H * s.vdim);
       const bool moe = s.mlp == TGIS_MLP_MOE;
       {
@@ -3703,10 +3669,6 @@ struct tgis_engine {
     const int S = (int)batch.size();
     step_n_ltiles = 0;
     step_n_ltiles16 = 0;
-    step_heads.clear();
-    step_rest_T = step_rest_tiles = step_rest_seqs = 0;
-    int n_spans = 0, n_lunits = 0;
-    heads_tiles.clear();
     step_max_q = 0;
     step_n_lead1 = 0;
     step_max_kv = 0;
@@ -3735,27 +3697,8 @@ struct tgis_engine {
       }
       if (pnx_on) {  // latent-attention query tiles: prompts, portions and single tokens alike
         LatentTile* lt = hs<LatentTile>(off_ltiles);
-        // in head space: the keys that some token of the portion sees, from a multiple of 128 on (the tiles of that kernel)
-        const int first = heads_no_window ? 0 : std::max(0, r.n_computed - heads_window + 1) / 128 * 128, keys = kv_len - first;
-        const bool heads = heads_any && latent_heads_pays(q_len, keys) && keys <= heads_cap;
-        for (int q0 = 0; q0 < q_len; q0 += pnx_tile_tokens) {
-          const LatentTile t{s, q0, std::min(pnx_tile_tokens, q_len - q0), 0};
-          if (heads) heads_tiles.push_back(t);
-          else lt[step_n_ltiles++] = t;
-        }
-        if (heads) {
-          if (step_heads.empty() || step_heads.back().n_keys + keys > heads_cap) step_heads.push_back(HeadsPass{n_spans, 0, 0, n_lunits, 0, 0});
-          HeadsPass& p = step_heads.back();
-          hs<LatentSpan>(off_lspans)[n_spans++] = LatentSpan{s, first, keys, p.n_keys};
-          n_lunits += latent_units_build(hs<LatentUnit>(off_lunits) + n_lunits, seqs[s], first, p.n_keys);
-          ++p.n_spans;
-          p.n_blocks += (keys + KV_BLOCK - 1) / KV_BLOCK;
-          p.n_units = n_lunits - p.unit0;
-          p.n_keys += keys;
-        } else {
-          step_rest_T = T + q_len;
-          ++step_rest_seqs;
-        }
+        for (int q0 = 0; q0 < q_len; q0 += pnx_tile_tokens)
+          lt[step_n_ltiles++] = LatentTile{s, q0, std::min(pnx_tile_tokens, q_len - q0), 0};
         if (run_style()) {
           LatentTile* lt16 = hs<LatentTile>(off_ltiles16);
           for (int q0 = 0; q0 < q_len; q0 += POOLATTN_TILE)
@@ -3832,9 +3775,6 @@ struct tgis_engine {
       }
       T += q_len;
     }
-    step_rest_tiles = step_n_ltiles;   // (layers without the other form take all of them)
-    for (const LatentTile& t : heads_tiles) hs<LatentTile>(off_ltiles)[step_n_ltiles++] = t;
-    for (const HeadsPass& p : step_heads) latent_units_sort(hs<LatentUnit>(off_lunits) + p.unit0, p.n_units);
     // ---- ship metadata + run the layer stack (one CUDA graph launch for a pure-decode step when enabled)
     // decode work items: (sequence, DECODE_SPLIT-token split) entries; the copy covers the worst case for this
     // (S, max_splits) so that its size is a function of the CUDA-graph key

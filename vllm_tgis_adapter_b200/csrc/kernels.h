@@ -481,35 +481,7 @@ cudaError_t latent_attn_launch(const float* q_abs, const void* cache, int dtype,
                                const LatentTile* tiles, int n_tiles, const int32_t* block_table, int bt_stride,
                                void* o_lat, int o_dtype, const LatentGeom& g, cudaStream_t stream, float* split_ws = nullptr,
                                size_t split_ws_floats = 0, int max_kv_len = 0, int num_sms = 148, int* n_launched = nullptr,
-                               int n_seqs = 0, int tile_tokens = 0); // ---- attention_heads.cu: the same attention for prompts and portions, over keys and values made for every head -------------------------
-constexpr int LATENT_HEAD_DIM = 128, LATENT_HEAD_ROT = 64, LATENT_HEAD_VDIM = 128;
-struct LatentUnit {   // up to 256 query tokens of one sequence, read as one int4
-  int row0, rows;     // of the step's flat token batch
-  int pos0;           // position of the first one, counted from the first gathered key
-  int key0;           // row of that key among the gathered ones
-};
-struct LatentSpan {   // gathered keys of a sequence
-  int block_row;      // of the block table
-  int first, n;       // positions first (a multiple of KV_BLOCK) .. + n - 1
-  int row;            // of the first among the gathered keys
-};
-// Whether a portion of q_len tokens whose sequence has `keys` keys takes this form.  What it costs beside the folded one's is a product over
-// all keys, so short portions behind a long context stay with that.  Whole steps of 4 layers, microseconds, folded -> here, 8 heads on
-// rank 256: 16 tokens 331 -> 307, 4 x 16 642 -> 529; behind 1500 tokens 32 433 -> 461, 3 x 32 651 -> 724, 48 655 -> 598, 3 x 48 842 -> 763;
-// 16 heads on rank 512: 16 843 -> 798, 32 x 64 2448 -> 2096; behind 1500 tokens 20 933 -> 960, 32 1082 -> 1012, 3 x 64 2279 -> 1818.
-inline bool latent_heads_pays(int q_len, int keys) { return q_len >= 48 || (q_len >= 16 && keys <= 8 * q_len); }
-bool latent_heads_takes(const LatentGeom& g, int dtype);
-// units of a portion whose gathered keys begin with position `first` (a multiple of 128) at row key0; longest first
-int latent_units_build(LatentUnit* units, const AttnSeq& q, int first, int key0);
-void latent_units_sort(LatentUnit* units, int n);
-// cached rows -> rows bf16 [keys][kv_rank], rot [keys][64]; queries q bf16 [T][heads][192]: the rotary part turned in place
-cudaError_t latent_rows_launch(const void* cache, const LatentSpan* spans, int n_blocks, const int32_t* block_table, int bt_stride, void* rows, void* rot,
-                               void* q, const LatentGeom& g, const int32_t* positions, const float* cos_sin, int T, cudaStream_t stream);
-// kv: bf16 [keys][heads][128] | [heads][128], the product of `rows` with the key and the value up-projections, one under the other.
-// out bf16 [T][heads][128], times gate [T][heads] (nullptr: 1); rows of no unit are left alone.
-cudaError_t latent_heads_launch(const void* q, int T, const void* kv, const void* rot, int n_keys, const LatentUnit* units, int n_units, const float* gate,
-                                void* out, const LatentGeom& g, int num_sms, cudaStream_t stream);
- // sequences of the step, tokens of a full tile (0: unknown)
+                               int n_seqs = 0, int tile_tokens = 0);  // sequences of the step, tokens of a full tile (0: unknown)
 
 // ---- attention_capped.cu: grouped-query attention with normed queries / keys and a soft cap on the scores ------------
 // No rotation: positions enter through the causal mask and a query temperature.  Per head: q <- rmsnorm(q) * w_q *

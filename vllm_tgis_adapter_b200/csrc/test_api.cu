@@ -672,48 +672,6 @@ int tgis_k_latent_attn(const float* q_abs, const void* cache, int32_t dt, const 
   return 0;
 }
 
-int tgis_k_latent_heads(void* q, const void* cache, const void* w_ukv, const int32_t* positions, const float* cos_sin, const float* gate, const float* sink,
-                        const int32_t* seqs_host, int32_t n_seqs, const int32_t* block_table_host, int32_t bt_rows, int32_t bt_stride, void* kv, void* out,
-                        const tgis_k_latent_geom* g) {
-  LatentGeom geom = to_geom(g);
-  geom.sink = sink;
-  if (!latent_heads_takes(geom, DT_BF16)) return -3;
-  std::vector<LatentSpan> spans;
-  std::vector<LatentUnit> units(1 << 16);
-  int n_units = 0, n_keys = 0, n_blocks = 0, T = 0;
-  for (int i = 0; i < n_seqs; ++i) {
-    const AttnSeq q{seqs_host[4 * i], seqs_host[4 * i + 1], seqs_host[4 * i + 2], seqs_host[4 * i + 3]};
-    const int first = geom.window > 0 ? std::max(0, q.kv_len - q.q_len - geom.window + 1) / 128 * 128 : 0;
-    T = std::max(T, q.q_start + q.q_len);
-    spans.push_back(LatentSpan{q.block_row, first, q.kv_len - first, n_keys});
-    n_units += latent_units_build(units.data() + n_units, q, first, n_keys);
-    n_keys += q.kv_len - first;
-    n_blocks += (q.kv_len - first + KV_BLOCK - 1) / KV_BLOCK;
-  }
-  latent_units_sort(units.data(), n_units);
-  Tmp<LatentSpan> d_spans;
-  Tmp<LatentUnit> d_units;
-  Tmp<int32_t> d_bt;
-  Tmp<__nv_bfloat16> rows, rot;
-  KCK(d_spans.upload(spans.data(), spans.size()));
-  KCK(d_units.upload(units.data(), n_units));
-  KCK(d_bt.upload(block_table_host, (size_t)bt_rows * bt_stride));
-  KCK(rows.alloc((size_t)n_keys * geom.kv_rank));
-  KCK(rot.alloc((size_t)n_keys * LATENT_HEAD_ROT));
-  KCK(latent_rows_launch(cache, d_spans.p, n_blocks, d_bt.p, bt_stride, rows.p, rot.p, q, geom, positions, cos_sin, T, 0));
-  if (w_ukv != nullptr) {   // nullptr: kv is what the caller made of it
-    GemmAny a{};
-    a.X = rows.p; a.W = w_ukv; a.Y = kv;
-    a.x_dtype = a.w_dtype = a.y_dtype = DT_BF16;
-    a.T = n_keys; a.N = geom.heads * (LATENT_HEAD_DIM + LATENT_HEAD_VDIM); a.K = a.ldx = a.ldw = geom.kv_rank; a.ldy = a.N;
-    a.batch = 1;
-    KCK(gemm_any_launch(a, 0));
-  }
-  KCK(latent_heads_launch(q, T, kv, rot.p, n_keys, d_units.p, n_units, gate, out, geom, test_num_sms(), 0));
-  KCK(cudaDeviceSynchronize());
-  return gemm_pair_failed() ? -4 : 0;
-}
-
 int tgis_k_moe_route(const float* logits, int32_t ld, const float* bias, int32_t E, int32_t top, int32_t* ids, float* w,
                      float* side_gate, int32_t T) {
   KCK(moe_route_launch(logits, ld, bias, E, top, ids, w, side_gate, T, 0));
