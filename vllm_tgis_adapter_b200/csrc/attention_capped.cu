@@ -207,8 +207,8 @@ capattn_kernel(const CT* __restrict__ q, const CT* __restrict__ k_cache, const C
 //
 // What bounds it is issue: 62 million warp instructions for 2048 tokens in 7 prompts and 16 heads, of which a tile's products, tanh and
 // exponentials are less than a third; the rest was division by sizes known only at run time, in the copies.  With 128-wide heads known
-// when it is compiled, two k-steps to a load of key fragments, no comparison of positions in blocks that every query sees, and the
-// tiles with the most keys first: 138 -> 75 us a layer; 32 single tokens behind 64 to 88 keys 14.4 -> 11.0.  Single tokens (ONE) fill
+// when it is compiled, two k-steps to a load of key fragments, no comparison of positions in blocks that every query sees, and the heads
+// of a tile side by side (the caller lists long tiles first): 138 -> 75 us a layer; 32 single tokens behind 64 to 88 keys 14.4 -> 11.0.  Single tokens (ONE) fill
 // the M rows with the query heads of a key/value head instead of 15 rows of nothing, a quarter of the CTAs and of the copies: 11.0 ->
 // 8.0.  No faster: 32 queries a CTA (166 registers; 94 us), a warp per head of the group (186 registers; 89 us).
 constexpr int MMA_KS = 8, MMA_NT = 8;
@@ -270,7 +270,7 @@ capattn_mma_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __r
   griddep_launch();
   griddep_wait();
   const int per_tile = ONE ? g.kv_heads : g.heads;
-  const LatentTile tl = tiles[(gridDim.x - 1 - blockIdx.x) / per_tile];   // (a sequence's later tiles, which have more keys, first)
+  const LatentTile tl = tiles[blockIdx.x / per_tile];
   const AttnSeq sq = seqs[tl.seq];
   const int gs = g.heads / g.kv_heads, hx = blockIdx.x % per_tile, h = ONE ? hx * gs : hx, kvh = ONE ? hx : h / gs;   // ONE: row r is head h + r
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, t2 = (lane & 3) * 2;

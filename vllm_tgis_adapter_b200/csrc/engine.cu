@@ -3695,17 +3695,12 @@ struct tgis_engine {
           if (p + 1 < r.n_prompt) prompt_rows.push_back(PromptRow{T + j, r.tokens[p + 1], p + 1, &r});
         }
       }
-      if (pnx_on) {  // latent-attention query tiles: prompts, portions and single tokens alike
-        LatentTile* lt = hs<LatentTile>(off_ltiles);
-        for (int q0 = 0; q0 < q_len; q0 += pnx_tile_tokens)
-          lt[step_n_ltiles++] = LatentTile{s, q0, std::min(pnx_tile_tokens, q_len - q0), 0};
-        if (run_style()) {
-          LatentTile* lt16 = hs<LatentTile>(off_ltiles16);
-          for (int q0 = 0; q0 < q_len; q0 += POOLATTN_TILE)
-            lt16[step_n_ltiles16++] = LatentTile{s, q0, std::min(POOLATTN_TILE, q_len - q0), 0};
-          step_max_q = std::max(step_max_q, q_len);
-          if (q_len == 1 && step_n_lead1 == s) ++step_n_lead1;
-        }
+      if (pnx_on && run_style()) {
+        LatentTile* lt16 = hs<LatentTile>(off_ltiles16);
+        for (int q0 = 0; q0 < q_len; q0 += POOLATTN_TILE)
+          lt16[step_n_ltiles16++] = LatentTile{s, q0, std::min(POOLATTN_TILE, q_len - q0), 0};
+        step_max_q = std::max(step_max_q, q_len);
+        if (q_len == 1 && step_n_lead1 == s) ++step_n_lead1;
       }
       if (q_len == 1) {
         decids[n_dec++] = s;
@@ -3774,6 +3769,17 @@ struct tgis_engine {
         ++R;
       }
       T += q_len;
+    }
+    if (pnx_on) {
+      // query tiles, prompts, portions and single tokens alike: sequences with the most keys first and their last tiles ahead, so that no
+      // long walk over a cache starts when the others are done (seven prompts, the longest last: capped attention 88 -> 73 us)
+      LatentTile* lt = hs<LatentTile>(off_ltiles);
+      std::vector<int> order(S);
+      for (int s = 0; s < S; ++s) order[s] = s;
+      if (T > S) std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return seqs[a].kv_len > seqs[b].kv_len; });
+      for (int s : order)
+        for (int q0 = (seqs[s].q_len - 1) / pnx_tile_tokens * pnx_tile_tokens; q0 >= 0; q0 -= pnx_tile_tokens)
+          lt[step_n_ltiles++] = LatentTile{s, q0, std::min(pnx_tile_tokens, seqs[s].q_len - q0), 0};
     }
     // ---- ship metadata + run the layer stack (one CUDA graph launch for a pure-decode step when enabled)
     // decode work items: (sequence, DECODE_SPLIT-token split) entries; the copy covers the worst case for this
