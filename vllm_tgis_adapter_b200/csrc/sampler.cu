@@ -29,8 +29,6 @@
 // top-p 63 -> 52 (1), 240 -> 129 (96).  (Only rows of equal logits, which no list holds, gain nothing: 438 -> 519, 80 of them with top-k.)
 #include <cooperative_groups.h>
 
-#include <algorithm>
-
 #include "kernels.h"
 #include "launch.cuh"
 #include "ptx.cuh"
@@ -41,11 +39,10 @@ namespace tgis {
 
 TGIS_STL_DEFINE(sampler)
 
-constexpr int SAMP_MAX_CL = 8;  // CTAs (SMs) per row: 1, 2, 4 or 8, chosen per launch (sampler_cluster_size)
 constexpr int SAMP_THREADS = 1024;
 constexpr int SAMP_WARPS = SAMP_THREADS / 32;
-constexpr int SAMP_LIST = SAMP_THREADS;
-constexpr int SAMP_FEW = 3 * SAMP_THREADS;
+constexpr int SAMP_LIST = SAMP_THREADS;      // entries a race or a top-n list holds
+constexpr int SAMP_FEW = 3 * SAMP_THREADS;   // ... a selection's list
 constexpr float SAMP_FLAT = 7.f;  // nats: as spread as over 1100 entries, more than a list holds
 constexpr float SAMP_FIX = 1073741824.0f;  // 2^30: probabilities are accumulated as fixed-point integers (see below)
 
