@@ -137,7 +137,8 @@ def philox_uniform(n: int, seed: int, step: int) -> np.ndarray:
         c0, c1, c2, c3 = hi1 ^ c1 ^ k0, lo1, hi0 ^ c3 ^ k1, lo0
         k0 = np.uint32((int(k0) + 0x9E3779B9) & 0xFFFFFFFF)
         k1 = np.uint32((int(k1) + 0xBB67AE85) & 0xFFFFFFFF)
-    return ((c0 >> np.uint32(8)).astype(np.float32) + np.float32(0.5)) * np.float32(1.0 / 16777216.0)
+    u = ((c0 >> np.uint32(8)).astype(np.float32) + np.float32(0.5)) * np.float32(1.0 / 16777216.0)
+    return np.minimum(u, np.float32(1) - np.float32(2.0 ** -24))   # (24 ones and a half round to 2^24)
 
 
 # ---------------------------------------------------------------------------------------------- full row

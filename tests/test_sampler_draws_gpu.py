@@ -1,0 +1,44 @@
+"""The sampler's random draw at the end of its range, and rows with entries that are no numbers (csrc/sampler.cu, oracle/sampler_oracle.py).
+
+u = (24 bits + 1/2) / 2^24 has to stay below one: 2^24 - 1/2 is no fp32 number, and an entry with u = 1 would win whatever its probability.
+The places below are where the generator's 24 bits are all ones; the entry there is one that e^10 times likelier ones surround."""
+import numpy as np
+import pytest
+import torch
+
+import tgis_gpu_utils as U
+from oracle import sampler_oracle as so
+
+ALL_ONES = [(1024, 45, 174, 140), (1024, 148, 15, 222), (128256, 192, 0, 100010), (50272, 404, 0, 28925)]   # vocabulary, seed, step, index
+
+
+def unlikely(V, index):
+    logits = torch.zeros(V)
+    logits[index] = -10.0
+    return logits
+
+
+@pytest.mark.parametrize("V,seed,step,index", ALL_ONES)
+def test_the_oracles_u_is_below_one(V, seed, step, index):
+    u = so.philox_uniform(V, seed, step)
+    assert u.dtype == np.float32 and 0 < u.min() and u.max() < 1 and u[index] == np.float32(1) - np.float32(2.0 ** -24) == u.max()
+    case = so.SamplingCase(greedy=False, seed=seed, n_out=step)
+    assert so.sample_row(unlikely(V, index), case)["token"] != index
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cluster", ["1", "8"])
+@pytest.mark.parametrize("how", ["plain", "top_k", "typical"])   # (the race over all entries, over kept ones, over a list of what is left)
+@pytest.mark.parametrize("V,seed,step,index", ALL_ONES)
+def test_an_unlikely_entry_is_not_drawn_for_its_place(V, seed, step, index, how, cluster, monkeypatch):
+    monkeypatch.setenv("TGIS_SAMPLER_CLUSTER", cluster)
+    logits = unlikely(V, index)
+    r = np.zeros(1, dtype=U.SAMPLE_ROW_DTYPE)
+    r["temperature"], r["top_p"], r["rep_penalty"], r["eos_id"], r["seq_slot"], r["seed_lo"], r["step"] = 1.0, 1.0, 1.0, -1, -1, seed, step
+    if how == "top_k":
+        r["top_k"], logits[0] = V - 1, -20.0      # (all but entry 0, which is less likely still)
+    if how == "typical":
+        r["typical_p"], r["flags"] = 1.0, U.SAMPLE_TYPICAL   # (the whole mass: every entry that has some)
+    out = U.run_sampler(logits.unsqueeze(0).cuda(), r)
+    want = so.sample_row(logits, so.SamplingCase(greedy=False, seed=seed, n_out=step, top_k=int(r["top_k"][0])))["token"]
+    assert want != index and int(out["token"][0]) == want

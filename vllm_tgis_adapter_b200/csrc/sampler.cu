@@ -812,7 +812,9 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
     ValIdx bs{-INFINITY, -1};
     auto race = [&](float v, int i) {
       const uint4 rnd = philox4x32(make_uint4((uint32_t)i, c.p.step, 0u, 0u), key);
-      const float u = ((float)(rnd.x >> 8) + 0.5f) * (1.0f / 16777216.0f);
+      // (24 ones and a half round to 2^24: without the limit u is one there, its score infinite, and one draw of 130 over 128256 entries
+      // goes to such an entry whatever its probability)
+      const float u = fminf(((float)(rnd.x >> 8) + 0.5f) * (1.0f / 16777216.0f), 1.f - 1.0f / 16777216.0f);
       // to be ahead, -log u has to be below e^(v - mx - best), and it is at least 1 - u: most entries need no logarithm (the
       // margin is a thousand times the rounding of what is compared)
       if (1.f - u > fmaf(__expf((v - mx) - bs.v), 1.001f, 1e-6f)) return;
