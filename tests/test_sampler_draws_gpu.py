@@ -42,3 +42,20 @@ def test_an_unlikely_entry_is_not_drawn_for_its_place(V, seed, step, index, how,
     out = U.run_sampler(logits.unsqueeze(0).cuda(), r)
     want = so.sample_row(logits, so.SamplingCase(greedy=False, seed=seed, n_out=step, top_k=int(r["top_k"][0])))["token"]
     assert want != index and int(out["token"][0]) == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["plain", "typical"])
+@pytest.mark.parametrize("V", [8, 1024])
+def test_an_entry_that_is_no_number_is_not_drawn(V, how):
+    """It compares with nothing, so it is not among those at or above a threshold: by the sweep over all entries and by the list alike."""
+    rows = 64
+    logits, at = torch.zeros(rows, V), torch.arange(rows) % V
+    logits[torch.arange(rows), at] = float("nan")
+    r = np.zeros(rows, dtype=U.SAMPLE_ROW_DTYPE)
+    r["temperature"], r["top_p"], r["rep_penalty"], r["eos_id"], r["seq_slot"] = 1.0, 1.0, 1.0, -1, -1
+    r["logits_row"], r["seed_lo"] = np.arange(rows), 7 + np.arange(rows)
+    if how == "typical":
+        r["typical_p"], r["flags"] = 0.9, U.SAMPLE_TYPICAL
+    token = U.run_sampler(logits.cuda(), r)["token"]
+    assert ((token >= 0) & (token < V) & (token != at.numpy())).all()

@@ -770,7 +770,7 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         mx = fmaxf(mx, v[e]);
-        if (!keep_y && v[e] != -INFINITY && list_n <= SAMP_LIST) {   // what typical-p left: mostly a few
+        if (!keep_y && v[e] > -INFINITY && list_n <= SAMP_LIST) {   // what typical-p left: mostly a few (numbers, as in the sweep below)
           const int at = atomicAdd(&list_n, 1);
           if (at < SAMP_LIST) {
             list_v[at] = v[e];
