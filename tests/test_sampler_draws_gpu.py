@@ -59,3 +59,21 @@ def test_an_entry_that_is_no_number_is_not_drawn(V, how):
         r["typical_p"], r["flags"] = 0.9, U.SAMPLE_TYPICAL
     token = U.run_sampler(logits.cuda(), r)["token"]
     assert ((token >= 0) & (token < V) & (token != at.numpy())).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("top_p", [1.0, 0.9])
+@pytest.mark.parametrize("V,dtype", [(1024, torch.float32), (50272, torch.bfloat16), (50272, torch.float32)])
+def test_entries_that_are_no_numbers_are_not_among_the_k_largest(V, dtype, top_p):
+    """Every other entry a NaN, of either sign: what is drawn is one of the six largest numbers."""
+    gen = torch.Generator().manual_seed(V)
+    logits = torch.randn(16, V, generator=gen)
+    logits[:, ::2] = float("nan")
+    logits[8:, ::2] = -logits[8:, ::2]
+    logits = logits.to(dtype)
+    r = np.zeros(16, dtype=U.SAMPLE_ROW_DTYPE)
+    r["temperature"], r["top_p"], r["top_k"], r["rep_penalty"], r["eos_id"], r["seq_slot"] = 1.0, top_p, 6, 1.0, -1, -1
+    r["logits_row"], r["seed_lo"] = np.arange(16), 7 + np.arange(16)
+    token = torch.from_numpy(U.run_sampler(logits.cuda(), r)["token"].astype(np.int64))
+    numbers = torch.where(logits.isnan(), torch.full_like(logits, -100.0), logits).float()
+    assert (numbers[torch.arange(16), token] >= torch.topk(numbers, 6).values[:, -1]).all()

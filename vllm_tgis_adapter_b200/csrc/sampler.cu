@@ -788,7 +788,7 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
       return t == t ? CODES - 1 - distance_code(t) : CODES - 1;
     };
     if (use_topk) {   // (with fewer than k entries left it is the smallest of them)
-      auto wq = [](float v) { return v != -INFINITY ? 1u : 0u; };
+      auto wq = [](float v) { return v > -INFINITY ? 1u : 0u; };   // (numbers: a NaN's code and key are not in one order)
       lo_thr = key2f(select_key(cl, lo, hi, load_y, code, keyf, wq, (uint32_t)c.p.top_k, false, true, hist, hsum, bcast, few, &list_n));
     }
     // ---- top-p (S6): drop the low-probability tail whose cumulative mass <= 1 - p
