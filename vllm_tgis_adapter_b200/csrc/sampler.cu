@@ -18,16 +18,18 @@
 //                 maximum per entry was a chain of a branch and an exponential each: 9100 of a greedy row's 27000 cycles); behind
 //                 typical-p the entropy's sum too
 //   reductions    maximum, sums and best entry in one; an exchange is one 16-byte read per lane and shuffles
-//   selections    (typical-p, top-k, top-p) one sweep over steps of a 32nd of an octave, one that lists the selected step's entries, radix
-//                 rounds over the list
+//   selections    (typical-p, top-k, top-p) one sweep over steps of a 32nd of an octave, one that lists the selected step's entries, then
+//                 parts of a step and radix rounds over the list
 //   race          behind typical-p over the list of what is left; in flat rows over kept processed logits, two logarithms only
 //                 for entries that 1 - u cannot rule out (186 instructions an entry -> 100; it was 38 % of a flat row)
 //   rank, top-n   one sweep and one exchange, the slices' lists ordered by eight threads a candidate
 // Measured, 128256 bf16 logits with top-5, microseconds, with the online maximum, an exchange for each part, clusters by SM count and four
 // radix rounds over leading bits -> here: greedy 19.7 -> 17 (1 row), 39 -> 17 (16), 22 -> 18 (32), 38 -> 28 (96), 73 -> 54 (150); typical-p
 // 45 -> 36 (1), 88 -> 42 (16), 91 -> 59 (64), 157 -> 91 (96), 309 -> 177 (150); flat rows 63 -> 48 (1), 285 -> 173 (96); top-k with
-// top-p 63 -> 52 (1), 240 -> 129 (96).  (Only rows of equal logits, which no list holds, gain nothing: 438 -> 519, 80 of them with top-k.)
+// top-p 63 -> 52 (1), 240 -> 129 (96).
 #include <cooperative_groups.h>
+
+#include <type_traits>
 
 #include "kernels.h"
 #include "launch.cuh"
@@ -341,7 +343,7 @@ __device__ __forceinline__ float key2f(uint32_t k) {
 // cluster's histograms in rank order, then warp 0 scans the 256 bins in parallel (8 per lane + a shuffle prefix).
 //   ascending (weighted select): first bin b with  below + sum_{<= b} >= target  (strict: > target); none: last nonempty
 //   descending (k-th largest)  : first bin b from the top with  above + sum_{>= b} >= target
-// Returns (bin, weight strictly before the bin in scan order) to every thread through bcast[0..1].
+// Returns (bin, weight strictly before the bin in scan order, whether any bin has weight) to every thread through bcast[0..2].
 template <int BINS>
 __device__ void radix_round_pick(const Cl& c, uint32_t* hist, uint32_t* hsum, uint32_t* bcast, uint32_t before,
                                  uint32_t target, bool strict, bool descending) {
@@ -383,6 +385,7 @@ __device__ void radix_round_pick(const Cl& c, uint32_t* hist, uint32_t* hsum, ui
       cum = nc;
     }
     const uint32_t hit = __ballot_sync(0xffffffffu, sel >= 0);
+    const uint32_t nonempty = __ballot_sync(0xffffffffu, tot > 0);
     int out_sel;
     uint32_t out_before;
     if (hit) {
@@ -407,14 +410,15 @@ __device__ void radix_round_pick(const Cl& c, uint32_t* hist, uint32_t* hsum, ui
     if (l == 0) {
       bcast[0] = (uint32_t)(descending ? BINS - 1 - out_sel : out_sel);  // back to a digit value
       bcast[1] = out_before;
+      bcast[2] = nonempty;
     }
   }
   __syncthreads();
 }
 
 // Adds eight (digit, weight) pairs of every lane to the histogram (weight 0: does not count).  Where the whole warp's 256
-// entries share a digit (the leading digits of most rows) one redux and one atomic do; else every entry is a shared-memory
-// atomic of its own, on several copies of the histogram so that lanes of equal digits meet less often.
+// entries share a digit (the leading digits of most rows) one redux and one atomic do, where a lane's eight do one atomic; else every
+// entry is a shared-memory atomic of its own, on several copies of the histogram so that lanes of equal digits meet less often.
 constexpr int HIST_WORDS = 1024;   // copies of the histogram, as many as fit
 template <int BINS>
 __device__ __forceinline__ void hist_add8(uint32_t* h, const uint32_t (&digit)[8], const uint32_t (&w)[8]) {
@@ -436,6 +440,10 @@ __device__ __forceinline__ void hist_add8(uint32_t* h, const uint32_t (&digit)[8
     return;
   }
   uint32_t* mine = h + (threadIdx.x & (HIST_WORDS / BINS - 1)) * BINS;
+  if (same) {
+    if (sum > 0) atomicAdd(&mine[d], sum);
+    return;
+  }
 #pragma unroll
   for (int e = 0; e < 8; ++e)
     if (w[e] > 0) atomicAdd(&mine[digit[e]], w[e]);
@@ -460,81 +468,152 @@ __device__ __forceinline__ void hist_fold(uint32_t* h) {
 // to 2^6 (what lies outside joins the first or the last).  Leading bits of a float are its exponent: two steps of an octave hold nine
 // tenths of a flat row, which then was swept three times, with an exponential and an atomic for most entries each time.
 constexpr int CODES = 512;
+constexpr uint32_t CODE_FIRST = (127 - 10) << 5;   // leading 14 bits of the lowest step
 __device__ __forceinline__ uint32_t distance_code(float t) {
-  const int c = (int)(__float_as_uint(t) >> 18) - ((127 - 10) << 5);
+  const int c = (int)(__float_as_uint(t) >> 18) - (int)CODE_FIRST;
   return (uint32_t)min(max(c, 0), CODES - 1);
+}
+// ... and, within a step, by 512 of its parts: the next nine bits; equal parts of the lowest step, which begins at zero; steps of a 512th of
+// an octave in the last
+__device__ __forceinline__ uint32_t distance_part(float t) {
+  const uint32_t b = __float_as_uint(t), c = distance_code(t);
+  if (c == 0) return min((uint32_t)(t * 508400.f), (uint32_t)CODES - 1);   // (512 parts of 33 / 32 2^-10)
+  if (c == CODES - 1) return min((b >> 14) - ((CODE_FIRST + CODES - 1) << 4), (uint32_t)CODES - 1);
+  return (b >> 9) & (CODES - 1);
 }
 
 // Smallest key K (ascending) such that  sum_{key_i <= K} w_i  >= target  (strict: > target), or with `descending` the largest with
-// sum_{key_i >= K}; if never reached, the last present key.  load(i0, v) -> eight values, code(v) < CODES, not falling with the
-// key, keyf(v) -> uint32 key, wq(v) -> integer weight: integer addition is associative, so the
-// result is the same on every cluster size.  Every CTA histograms its slice, the cluster sums the histograms, every CTA runs the same
-// scan: codes first; then a sweep that lists the entries of the selected code, and four rounds of 8 bits over the list, or, where
-// that has no room, over the slice.
-template <class LoadF, class CodeF, class KeyF, class WQ>
-__device__ uint32_t select_key(Cl& c, int lo, int hi, LoadF load, CodeF code, KeyF keyf, WQ wq, uint32_t T, bool strict, bool descending,
-                               uint32_t (*hist)[HIST_WORDS], uint32_t* hsum, uint32_t* bcast, float* few, int* n_few) {
-  uint32_t* h = hist[c.he & 1];
-  ++c.he;
-  hist_clear(h);
-  for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
-    const int i0 = base + threadIdx.x * 8;
-    uint32_t digit[8], w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (i0 < hi) {
-      float v[8];
-      load(i0, v);
+// sum_{key_i >= K}; if never reached, the last present key.  load(i0, v) -> eight values; (code(v), part(v)), each < CODES, do not fall as
+// the key rises; keyf(v) -> uint32 key, wq(v) -> integer weight: integer addition is associative, so the result is the same on every
+// cluster size.  Every CTA histograms its slice, the cluster sums the histograms, every CTA runs the same scan: codes over the slice; a
+// sweep that lists the entries of the selected code; parts over the list, or, where that has no room, over the slice, and a sweep that
+// lists those of the selected part; then rounds of 8 bits over what is left, but for digits that all its keys share.
+// Flat rows on one CTA have 5000 entries to a code, more than the list holds, equal ones all of them.  80 rows of 128256 bf16, microseconds,
+// four rounds over leading bits of every key / four of the slice behind a list without room / parts: top-p of flat rows 267 / 307 / 249,
+// top-k of equal rows 287 / 332 / 267, top-k with top-p and typical-p of equal rows 551 / 669 / 457.  (What it costs where the list had room:
+// one row of 50272 behind typical-p 30.6 -> 32.6, 150 rows with top-p 246 -> 256; with all three 32 rows 77 -> 70, 96 rows 181 -> 180.)
+template <class LoadF, class CodeF, class PartF, class KeyF, class WQ>
+__device__ uint32_t select_key(Cl& c, int lo, int hi, LoadF load, CodeF code, PartF part, KeyF keyf, WQ wq, uint32_t T, bool strict, bool descending,
+                               uint32_t (*hist)[HIST_WORDS], uint32_t* hsum, uint32_t* bcast, float4* xch, float* few, int* n_few, uint32_t* key_bits) {
+  auto next_hist = [&]() {
+    uint32_t* h = hist[c.he & 1];
+    ++c.he;
+    hist_clear(h);
+    return h;
+  };
+  // put(v, digit, weight) of every entry of the slice (weight 0: does not count)
+  auto add_slice = [&](auto bins, uint32_t* h, auto put) {
+    for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
+      const int i0 = base + threadIdx.x * 8;
+      uint32_t digit[8], w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (i0 < hi) {
+        float v[8];
+        load(i0, v);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        digit[e] = code(v[e]);
-        w[e] = wq(v[e]);
+        for (int e = 0; e < 8; ++e) put(v[e], digit[e], w[e]);
       }
+      hist_add8<decltype(bins)::value>(h, digit, w);
     }
-    hist_add8<CODES>(h, digit, w);
-  }
+  };
+  auto list = [&](float v) {
+    const int at = atomicAdd(n_few, 1);
+    if (at < SAMP_FEW) few[at] = v;
+  };
+  constexpr std::integral_constant<int, CODES> codes{};
+  uint32_t* h = next_hist();
+  add_slice(codes, h, [&](float v, uint32_t& digit, uint32_t& w) {
+    digit = code(v);
+    w = wq(v);
+  });
   hist_fold<CODES>(h);
-  if (threadIdx.x == 0) *n_few = 0;
+  if (threadIdx.x == 0) {
+    *n_few = 0;
+    key_bits[0] = 0xffffffffu;
+    key_bits[1] = 0u;
+  }
   radix_round_pick<CODES>(c, h, hsum, bcast, 0u, T, strict, descending);
   const uint32_t sel = bcast[0];
-  uint32_t prefix = 0, before = bcast[1];
+  uint32_t before = bcast[1];
   for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
     if (*n_few > SAMP_FEW) break;
     float v[8];
     load(i0, v);
 #pragma unroll
     for (int e = 0; e < 8; ++e)
-      if (code(v[e]) == sel) {
-        const int at = atomicAdd(n_few, 1);
-        if (at < SAMP_FEW) few[at] = v[e];
-      }
+      if (code(v[e]) == sel) list(v[e]);
   }
+  h = next_hist();   // (behind its barrier the list is complete)
+  const int n_code = *n_few;
+  const bool code_listed = n_code <= SAMP_FEW;
+  if (code_listed) {
+    for (int i = threadIdx.x; i < n_code; i += SAMP_THREADS) atomicAdd(&h[(threadIdx.x & 1) * CODES + part(few[i])], wq(few[i]));
+  } else {
+    add_slice(codes, h, [&](float v, uint32_t& digit, uint32_t& w) {
+      if (code(v) != sel) return;
+      digit = part(v);
+      w = wq(v);
+    });
+  }
+  hist_fold<CODES>(h);
+  if (!code_listed && threadIdx.x == 0) *n_few = 0;   // (everyone has read it)
+  radix_round_pick<CODES>(c, h, hsum, bcast, before, T, strict, descending);
+  const uint32_t sub = bcast[0];
+  const bool some = bcast[2] != 0;
+  before = bcast[1];
+  uint32_t all = 0xffffffffu, any = 0u;   // key bits that every entry left has, and that any has
+  auto note = [&](float v) {
+    const uint32_t k = keyf(v);
+    all &= k;
+    any |= k;
+  };
+  if (code_listed) {
+    for (int i = threadIdx.x; i < n_code; i += SAMP_THREADS)
+      if (part(few[i]) == sub) note(few[i]);
+  } else {
+    for (int i0 = lo + threadIdx.x * 8; i0 < hi; i0 += SAMP_THREADS * 8) {
+      float v[8];
+      load(i0, v);
+      const bool room = *n_few <= SAMP_FEW;
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (code(v[e]) == sel && part(v[e]) == sub) {
+          note(v[e]);
+          if (room) list(v[e]);
+        }
+    }
+  }
+  all = __reduce_and_sync(0xffffffffu, all);
+  any = __reduce_or_sync(0xffffffffu, any);
+  if ((threadIdx.x & 31) == 0 && (all & ~any) == 0) {   // (of no entry: all bits and none)
+    atomicAnd(&key_bits[0], all);
+    atomicOr(&key_bits[1], any);
+  }
+  __syncthreads();
+  const XchView bits = cl_publish(c, xch, Xch4{__uint_as_float(key_bits[0]), __uint_as_float(key_bits[1]), 0.f, 0.f});
+  all = __reduce_and_sync(0xffffffffu, __float_as_uint(bits.mine.x));
+  any = __reduce_or_sync(0xffffffffu, __float_as_uint(bits.mine.y));
+  const uint32_t alike = some ? ~(all ^ any) : 0u;
+  const int n = *n_few;
+  uint32_t prefix = 0;
   for (int round = 0; round < 4; ++round) {
     const int shift = 24 - 8 * round;
+    if (((alike >> shift) & 255) == 255) {
+      prefix |= all & (255u << shift);
+      continue;
+    }
     auto counts = [&](uint32_t k) { return round == 0 || (k >> (shift + 8)) == (prefix >> (shift + 8)); };
-    h = hist[c.he & 1];
-    ++c.he;
-    hist_clear(h);
-    const int n = *n_few;
+    h = next_hist();
     if (n <= SAMP_FEW) {
       for (int i = threadIdx.x; i < n; i += SAMP_THREADS) {
         const uint32_t k = keyf(few[i]);
-        if (counts(k)) atomicAdd(&h[(threadIdx.x & 3) * 256 + ((k >> shift) & 255)], wq(few[i]));
+        if (part(few[i]) == sub && counts(k)) atomicAdd(&h[(threadIdx.x & 3) * 256 + ((k >> shift) & 255)], wq(few[i]));
       }
     } else {
-      for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
-        const int i0 = base + threadIdx.x * 8;
-        uint32_t digit[8], w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if (i0 < hi) {
-          float v[8];
-          load(i0, v);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const uint32_t k = keyf(v[e]);
-            digit[e] = (k >> shift) & 255;
-            if (code(v[e]) == sel && counts(k)) w[e] = wq(v[e]);
-          }
-        }
-        hist_add8<256>(h, digit, w);
-      }
+      add_slice(std::integral_constant<int, 256>{}, h, [&](float v, uint32_t& digit, uint32_t& w) {
+        const uint32_t k = keyf(v);
+        digit = (k >> shift) & 255;
+        if (code(v) == sel && part(v) == sub && counts(k)) w = wq(v);
+      });
     }
     hist_fold<256>(h);
     radix_round_pick<256>(c, h, hsum, bcast, before, T, strict, descending);
@@ -576,6 +655,7 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
   __shared__ uint32_t hist[2][HIST_WORDS];
   __shared__ uint32_t hsum[CODES];
   __shared__ uint32_t bcast[4];
+  __shared__ uint32_t key_bits[2];
   __shared__ float4 xch[2];
   __shared__ RedBest redb[SAMP_WARPS];
   __shared__ float wmax[SAMP_WARPS];    // of the slice's raw entries, by warp
@@ -726,8 +806,9 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
       return __float_as_uint(fabsf((-lp) - ent));
     };
     auto code = [=](float x) { return distance_code(fabsf((-((x - rm) - lz)) - ent)); };
+    auto fine = [=](float x) { return distance_part(fabsf((-((x - rm) - lz)) - ent)); };
     auto wq = [=](float x) { return __float2uint_rn(expf((x - rm) - lz) * SAMP_FIX); };
-    const uint32_t k = select_key(cl, lo, hi, load, code, keyf, wq, mass_target(c.p.typical_p), false, false, hist, hsum, bcast, few, &list_n);
+    const uint32_t k = select_key(cl, lo, hi, load, code, fine, keyf, wq, mass_target(c.p.typical_p), false, false, hist, hsum, bcast, xch, few, &list_n, key_bits);
     c.typ_thr = __uint_as_float(k);
     c.typical = true;
   }
@@ -787,9 +868,13 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
       const float t = mx - v;
       return t == t ? CODES - 1 - distance_code(t) : CODES - 1;
     };
+    auto fine = [=](float v) {
+      const float t = mx - v;
+      return t == t ? CODES - 1 - distance_part(t) : CODES - 1;
+    };
     if (use_topk) {   // (with fewer than k entries left it is the smallest of them)
       auto wq = [](float v) { return v > -INFINITY ? 1u : 0u; };   // (numbers: a NaN's code and key are not in one order)
-      lo_thr = key2f(select_key(cl, lo, hi, load_y, code, keyf, wq, (uint32_t)c.p.top_k, false, true, hist, hsum, bcast, few, &list_n));
+      lo_thr = key2f(select_key(cl, lo, hi, load_y, code, fine, keyf, wq, (uint32_t)c.p.top_k, false, true, hist, hsum, bcast, xch, few, &list_n, key_bits));
     }
     // ---- top-p (S6): drop the low-probability tail whose cumulative mass <= 1 - p
     if (use_topp) {
@@ -804,7 +889,7 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
       const float z = cluster_sumf(cl, part, redf, xch);
       const float lt = lo_thr;
       auto wq = [=](float v) { return v >= lt ? __float2uint_rn(expf(v - mx) / z * SAMP_FIX) : 0u; };
-      const uint32_t k = select_key(cl, lo, hi, load_y, code, keyf, wq, mass_target(1.0f - c.p.top_p), true, false, hist, hsum, bcast, few, &list_n);
+      const uint32_t k = select_key(cl, lo, hi, load_y, code, fine, keyf, wq, mass_target(1.0f - c.p.top_p), true, false, hist, hsum, bcast, xch, few, &list_n, key_bits);
       lo_thr = fmaxf(lo_thr, key2f(k));
     }
     // ---- exponential race == Gumbel max over the kept set
