@@ -63,3 +63,22 @@ def test_masses_among_keys_that_share_digits(how, many, cluster, monkeypatch):
         r["seed_lo"] = 50 * seed + np.arange(n)
         token = U.run_sampler(logits.cuda(), r)["token"]
         assert not any(bool(never[i][token[i]]) for i in range(n)), (seed, token)
+
+
+@pytest.mark.parametrize("cluster", ["1", "4", "8"])
+@pytest.mark.parametrize("V,dtype", [(1024, torch.float32), (50272, torch.float32), (128256, torch.bfloat16)])
+def test_topn_of_rows_in_order(V, dtype, cluster, monkeypatch):
+    """Rows whose largest entries stand side by side, so that few warps have them all: rising, falling, in saw teeth, with ties at the end."""
+    monkeypatch.setenv("TGIS_SAMPLER_CLUSTER", cluster)
+    up, rows = torch.linspace(-3, 3, V), []
+    for i in range(12):
+        rows.append([up, up.flip(0), torch.arange(V) % 2048 / 512.0, torch.arange(V) % 256 / 64.0, up.clamp(max=2.97), (up * 400).round() / 400][i % 6])
+    logits = torch.stack(rows).to(dtype)
+    r = np.zeros(12, dtype=U.SAMPLE_ROW_DTYPE)
+    r["temperature"], r["top_p"], r["rep_penalty"], r["eos_id"], r["seq_slot"], r["logits_row"] = 1.0, 1.0, 1.0, -1, -1, np.arange(12)
+    r["flags"], r["n_topn"] = U.SAMPLE_GREEDY | U.SAMPLE_LOGPROBS, 1 + np.arange(12)
+    out = U.run_sampler(logits.cuda(), r)
+    for i in range(12):
+        want = torch.sort(logits[i].double(), descending=True, stable=True).indices
+        assert out["topn_ids"][i][: i + 1].tolist() == want[: i + 1].tolist(), i
+        assert int(out["token"][i]) == int(want[0])
