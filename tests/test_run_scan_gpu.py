@@ -1,5 +1,6 @@
 """Scans over portions of several tokens: what a portion leaves and answers has the bits of its tokens one launch each (the kernels of
-single tokens), for lengths around the staged chunks, sequences of unequal length and columns that fill no whole piece."""
+single tokens), for lengths around the staged chunks, sequences of unequal length, columns that fill no whole piece, and rows that 16-byte
+loads reach and do not reach."""
 from __future__ import annotations
 
 import ctypes as C
@@ -33,12 +34,13 @@ def _runs(lengths, one_by_one):
 @pytest.mark.parametrize("lengths", [[1, 2, 15], [16, 17, 3, 33], [47, 64], [5] * 9])
 @pytest.mark.parametrize("d,dv,H", [(64, 64, 3), (128, 256, 2), (128, 40, 1), (256, 33, 1)])
 @pytest.mark.parametrize("mode", ["decay", "gated", "hgrn", "ssd", "lightning"])
-def test_memories(lib, mode, d, dv, H, lengths):
+@pytest.mark.parametrize("odd", [0, 1, 2])
+def test_memories(lib, mode, d, dv, H, lengths, odd):
     n, T, res = len(lengths), sum(lengths), []
     for one_by_one in (False, True):
         gen = torch.Generator(device="cuda").manual_seed(d + dv + T)
         rnd = lambda *s: torch.randn(*s, device="cuda", generator=gen)
-        x = rnd(T, 3 * H * d + H * dv + 2 * H)
+        x = rnd(T, -(-(3 * H * d + H * dv + 2 * H) // 4) * 4 + odd)
         ld, q, k, dec, v, gate = x.shape[1], x, x[:, H * d:], x[:, 2 * H * d:], x[:, 3 * H * d:], x[:, 3 * H * d + H * dv:]
         S, nrm, mx = rnd(n, H, d, dv), rnd(n, H, d).abs(), rnd(n, H)
         w0, u, b1, b2, last, heads = rnd(H * d), rnd(H * d).sigmoid(), rnd(H), rnd(H), torch.zeros(n, 24, device="cuda"), rnd(H).sigmoid()

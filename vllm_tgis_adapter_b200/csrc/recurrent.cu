@@ -476,7 +476,7 @@ selective_scan_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t
 // before the token loop, and its normaliser is kept a row per thread.
 // Bound by instruction issue and by the latency of a token's chain (one head's tokens are worked through one after the other, and a
 // prompt has only heads * vdim / 32 blocks).  Four rows to a shared-memory load and two to an fma.  This is the kernel of keys that leave
-// the last row group short, and of rows that 16-byte loads cannot reach; the others' prompts have outer_run_kernel.
+// the last row group short; the others' prompts have outer_run_kernel.
 __device__ __forceinline__ unsigned long long pack2(float x, float y) {
   unsigned long long d;
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
@@ -750,7 +750,8 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
 // Bound by instruction issue, of which the rows' packed multiply-adds are a third.  2048 tokens in 7 prompts (838 the longest), microseconds
 // without overlap, before -> here: gated, 8 heads of 128 x 256, 302 -> 136; decayed, 32 heads of 64 x 64, 234 -> 106; 32 prompts of 64 tokens 137 ->
 // 119 and 92 -> 90.  Slower: four columns a thread or 64 a piece (gated 184 to 194), chunks of eight tokens in a ring of four (154), one helping
-// group for all of it (174), vectors staged number by number (155).
+// group for all of it (174), vectors staged number by number (155).  Rows that 16-byte loads do not reach come in four loads each: gated 165
+// (311 in the kernel above while it knew full row groups, 481 since it tests every one), decayed 112 (222, 243), 256-row keys 229 (289, 587).
 template <int MODE>
 constexpr bool OS_OWN_DECAY = MODE == OUTER_SCAN_DECAY || MODE == OUTER_SCAN_HGRN || MODE == OUTER_SCAN_GLA;   // a decay per row
 template <int MODE>
@@ -771,7 +772,7 @@ __device__ __forceinline__ void bar_arrive_at(int i, int threads) {
   else asm volatile("bar.arrive %0, %1;\n" ::"n"(ID + 1), "r"(threads) : "memory");
 }
 
-template <int RPT, int MODE>
+template <int RPT, int MODE, bool VEC16>   // VEC16: q, k and decay rows begin on 16 bytes
 __global__ void __launch_bounds__(RUN_THREADS, RPT <= 16 ? 2 : 1)
 outer_run_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, int n_seqs, const int32_t* __restrict__ tok_slot) {
   constexpr int D = RPT * OS_GROUPS, NV = OS_VECS<MODE>, C = RUN_CHUNK, RING = RUN_RING, CT = 2, NG = RPT / 4, UNROLL = RPT <= 16 ? 2 : 1;
@@ -914,13 +915,16 @@ outer_run_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, int n_seqs, cons
     const bool v_in = c0 + lane < a.vdim;
     auto fetch = [&](int n) {
       const int nt = min(C, sq.q_len - n * C);
-      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      auto row = [&](const float* p, bool in) {
+        if (!in) return make_float4(0.f, 0.f, 0.f, 0.f);
+        return VEC16 ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+      };
 #pragma unroll
       for (int e = 0; e < EPT; ++e) {
         const bool in = tok + e * TSTEP < nt;
-        pq[e] = in ? *reinterpret_cast<const float4*>(q_at + (size_t)(e * TSTEP) * a.ldq) : zero;
-        if (MODE != OUTER_SCAN_HGRN) pk[e] = in ? *reinterpret_cast<const float4*>(k_at + (size_t)(e * TSTEP) * a.ldk) : zero;
-        if (OS_OWN_DECAY<MODE>) pd[e] = in ? *reinterpret_cast<const float4*>(d_at + (size_t)(e * TSTEP) * a.ldd) : zero;
+        pq[e] = row(q_at + (size_t)(e * TSTEP) * a.ldq, in);
+        if (MODE != OUTER_SCAN_HGRN) pk[e] = row(k_at + (size_t)(e * TSTEP) * a.ldk, in);
+        if (OS_OWN_DECAY<MODE>) pd[e] = row(d_at + (size_t)(e * TSTEP) * a.ldd, in);
       }
 #pragma unroll
       for (int e = 0; e < VPT; ++e) pv[e] = v_in && ht / OS_COLS + 4 * e < nt ? v_at[(size_t)(4 * e) * a.ldv] : 0.f;
@@ -1622,9 +1626,19 @@ cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_s
 
 template <int RPT, int MODE>
 static cudaError_t outer_run(const OuterScan& a, const AttnSeq* seqs, int n_seqs, int pieces, const int32_t* tok_slot, cudaStream_t stream) {
-  static const cudaError_t attr = cudaFuncSetAttribute(outer_run_kernel<RPT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RUN_SMEM<RPT, MODE>);
-  if (attr != cudaSuccess) return attr;
-  return launch_k(outer_run_kernel<RPT, MODE>, dim3(pieces), dim3(RUN_THREADS), RUN_SMEM<RPT, MODE>, stream, a, seqs, n_seqs, tok_slot);
+  auto al16 = [](const float* p, int ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; };   // (nullptr where the mode has none)
+  const bool vec16 = al16(a.q, a.ldq) && (MODE == OUTER_SCAN_HGRN || al16(a.k, a.ldk)) && (!OS_OWN_DECAY<MODE> || al16(a.decay_raw, a.ldd));
+  auto launch = [&](auto kernel, cudaError_t attr) {
+    if (attr != cudaSuccess) return attr;
+    return launch_k(kernel, dim3(pieces), dim3(RUN_THREADS), RUN_SMEM<RPT, MODE>, stream, a, seqs, n_seqs, tok_slot);
+  };
+  auto room = [](auto kernel) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RUN_SMEM<RPT, MODE>); };
+  if (vec16) {
+    static const cudaError_t attr = room(outer_run_kernel<RPT, MODE, true>);
+    return launch(outer_run_kernel<RPT, MODE, true>, attr);
+  }
+  static const cudaError_t attr = room(outer_run_kernel<RPT, MODE, false>);
+  return launch(outer_run_kernel<RPT, MODE, false>, attr);
 }
 template <int RPT, int MODE>
 static cudaError_t outer_scan_rows(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot, cudaStream_t stream) {
@@ -1635,9 +1649,7 @@ static cudaError_t outer_scan_rows(const OuterScan& a, const AttnSeq* seqs, int 
     }
   }
   const long long pieces = (long long)n_seqs * a.heads * ((a.vdim + OS_COLS - 1) / OS_COLS);
-  auto al16 = [](const float* p, int ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; };   // (nullptr where the mode has none)
-  if (a.dim == RPT * OS_GROUPS && pieces < (1ll << 31) && al16(a.q, a.ldq) && (MODE == OUTER_SCAN_HGRN || al16(a.k, a.ldk)) &&
-      (!OS_OWN_DECAY<MODE> || al16(a.decay_raw, a.ldd)))
+  if (a.dim == RPT * OS_GROUPS && pieces < (1ll << 31))
     return outer_run<RPT, MODE>(a, seqs, n_seqs, (int)pieces, tok_slot, stream);
   const dim3 grid(n_seqs, a.heads, (a.vdim + OS_COLS - 1) / OS_COLS);
   const size_t smem = ((size_t)OS_CHUNK * 3 * ((a.dim + 3) & ~3) + OS_CHUNK * OS_COLS) * sizeof(float);   // <= 50 KB (+ 17 KB static)
