@@ -97,3 +97,17 @@ def test_records_before_a_failure_stay_to_be_polled(max_tokens, monkeypatch):
     while more := eng.poll(0):
         got += more
     assert got == [_by_field(o) for step in lib.made[:20] for o in step]
+
+
+@pytest.mark.parametrize("max_tokens", [4, 400])
+def test_a_call_after_a_failure_takes_what_was_left_first(max_tokens, monkeypatch):
+    """In the order in which they were reported, whether or not a second thread made the records."""
+    lib = _Lib(30, 9, 3, fail_at=20)
+    monkeypatch.setattr(_lib, "last_error", lambda lib: "a step failed")
+    eng, sp = _engine(lib), make_sampling_params(max_tokens=max_tokens)
+    with pytest.raises(EngineError, match="a step failed"):
+        eng.generate_sync([[1], [2], [3]], sp)
+    flat = [_by_field(o) for step in lib.made[:20] for o in step]
+    lib.made, lib.fail_at = _Lib(12, 9, 3).made[5:], None
+    flat += [_by_field(o) for step in lib.made for o in step]
+    assert eng.generate_sync([[1], [2], [3]], sp) == [[o for o in flat if o.request_id == f"r{i}"] for i in range(3)]

@@ -391,11 +391,12 @@ class NativeEngine:
             params = [params] * len(prompts)
         for i, (p, sp) in enumerate(zip(prompts, params)):
             self.add_request(f"r{i}", p, sp)
+        new: list[StepOutput] = []
         if sum(sp.max_tokens for sp in params) < _COLLECT_FROM:
             self.run_until_idle()
-            outs = []
         else:
-            outs = self._run_and_collect()
+            new = self._run_and_collect()
+        outs, self._unread = self._unread + new, []   # (what a call that failed has left comes first)
         while more := self.poll(0):
             outs += more
         res: list[list[StepOutput]] = [[] for _ in prompts]
