@@ -59,6 +59,10 @@ int tgis_k_gemm_norm_chain(const void* a_dev, int32_t a_rows_alloc, const void* 
 /* The same between the register products of up to eight tokens (gemm_skinny.cu); fused = 0: the norm as a launch of its own. */
 int tgis_k_skinny_norm_chain(const void* a, const void* w1, void* resid, const void* w_norm, const void* w2, void* y2, int32_t T, int32_t K1, int32_t H,
                              int32_t N2, float eps, int32_t out_mode2, int32_t fused);
+/* ... in front of a qkv projection y2[T, (n_q + 2 n_kv) * 128] with rotary embedding and the scatter into the caches */
+int tgis_k_skinny_norm_rope(const void* a, const void* w1, void* resid, const void* w_norm, const void* w2, void* y2, int32_t T, int32_t K1, int32_t H,
+                            int32_t n_q, int32_t n_kv, float eps, const int32_t* positions_host, const int32_t* slot_mapping_host,
+                            const void* cos_sin_dev, void* k_cache_dev, void* v_cache_dev, int32_t fused);
 /* seqs_host: n_seqs x {q_start, q_len, kv_len, block_row}; block_table_host: [rows][bt_stride] */
 int tgis_k_attention(const void* qkv_dev, const void* k_cache_dev, const void* v_cache_dev, const int32_t* seqs_host,
                      int32_t n_seqs, const int32_t* block_table_host, int32_t bt_rows, int32_t bt_stride, void* out_dev,

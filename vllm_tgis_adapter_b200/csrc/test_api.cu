@@ -240,6 +240,35 @@ int tgis_k_skinny_norm_chain(const void* a, const void* w1, void* resid, const v
   return 0;
 }
 
+// The same in front of a qkv projection, y2 [T, (n_q + 2 n_kv) * 128], with rotary embedding and the scatter into the caches: inside the product
+// behind the norm (fused) or as launches of their own; 1: not products that it goes with
+int tgis_k_skinny_norm_rope(const void* a, const void* w1, void* resid, const void* w_norm, const void* w2, void* y2, int32_t T, int32_t K1, int32_t H,
+                            int32_t n_q, int32_t n_kv, float eps, const int32_t* positions_host, const int32_t* slot_mapping_host,
+                            const void* cos_sin_dev, void* k_cache_dev, void* v_cache_dev, int32_t fused) {
+  const int N = (n_q + 2 * n_kv) * HEAD_DIM;
+  if (!gemm_skinny_norm_takes(T, H, K1, N, 64)) return 1;
+  Tmp<bf16> y1, xn;
+  Tmp<float> ssq;
+  Tmp<int32_t> pos, sm;
+  KCK(y1.alloc((size_t)T * H));
+  KCK(xn.alloc((size_t)T * H));
+  KCK(ssq.alloc((size_t)T * (H / 8)));
+  KCK(pos.upload(positions_host, T));
+  KCK(sm.upload(slot_mapping_host, T));
+  const GemmRope rp{pos.p, sm.p, (const bf16*)cos_sin_dev, (bf16*)k_cache_dev, (bf16*)v_cache_dev, n_q, n_kv};
+  if (fused) {
+    KCK(gemm_skinny_add_launch(a, w1, (bf16*)resid, ssq.p, T, H, K1, 0));
+    KCK(gemm_skinny_norm_launch(resid, ssq.p, (const bf16*)w_norm, eps, w2, y2, N, T, N, H, 0, &rp, 0));
+  } else {
+    KCK(gemm_skinny_launch(a, w1, y1.p, H, T, H, K1, 0, nullptr, 0));
+    KCK(add_rmsnorm_launch(y1.p, (bf16*)resid, (const bf16*)w_norm, xn.p, T, H, eps, 0));
+    KCK(gemm_skinny_launch(xn.p, w2, y2, N, T, N, H, 0, nullptr, 0));
+    KCK(rope_kvwrite_launch((bf16*)y2, pos.p, sm.p, (const bf16*)cos_sin_dev, (bf16*)k_cache_dev, (bf16*)v_cache_dev, T, n_q, n_kv, 0));
+  }
+  KCK(cudaDeviceSynchronize());
+  return 0;
+}
+
 // Layer-stack slice  a -> [GEMM W1] -> (+ residual, RMSNorm w_norm) -> [GEMM W2 (out_mode2: 0 bf16, 2 fused SwiGLU)] -> y2
 // run either as three launches (fused = 0: gemm, add_rmsnorm_launch, gemm) or as two with the add + norm folded into the
 // two GEMMs (fused = 1, GemmNorm).  residual [T, H] is updated in place either way.  Returns 1 when the launch plan cannot

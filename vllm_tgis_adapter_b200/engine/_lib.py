@@ -150,7 +150,7 @@ ENGINE_SYMBOLS = [
     "tgis_engine_max_model_len", "tgis_engine_set_profiling", "tgis_nccl_unique_id", "tgis_engine_worker_run", "tgis_engine_shutdown", "tgis_engine_destroy", "tgis_engine_run_until_idle",
 ]
 KERNEL_SYMBOLS = [
-    "tgis_k_last_error", "tgis_k_pair_fault", "tgis_k_tp_wait", "tgis_k_gemm_timeline", "tgis_k_step_timeline_enable", "tgis_k_step_timeline_read", "tgis_k_gemm", "tgis_k_rmsnorm", "tgis_k_opt_layernorm", "tgis_k_opt_bias_act", "tgis_k_opt_embed", "tgis_k_silu_mul", "tgis_k_rope_kv", "tgis_k_gemm_rope", "tgis_k_gemm_norm_chain", "tgis_k_skinny_norm_chain", "tgis_k_attention",
+    "tgis_k_last_error", "tgis_k_pair_fault", "tgis_k_tp_wait", "tgis_k_gemm_timeline", "tgis_k_step_timeline_enable", "tgis_k_step_timeline_read", "tgis_k_gemm", "tgis_k_rmsnorm", "tgis_k_opt_layernorm", "tgis_k_opt_bias_act", "tgis_k_opt_embed", "tgis_k_silu_mul", "tgis_k_rope_kv", "tgis_k_gemm_rope", "tgis_k_gemm_norm_chain", "tgis_k_skinny_norm_chain", "tgis_k_skinny_norm_rope", "tgis_k_attention",
     "tgis_k_attention_bench", "tgis_k_decode_items", "tgis_k_gemm_plan", "tgis_k_gemm_route", "tgis_k_gemm_unit_rows",
     "tgis_k_sampler", "tgis_k_sampler_ex", "tgis_k_sampler_masked", "tgis_k_lora", "tgis_k_lora_bench", "tgis_k_lora_swiglu", "tgis_k_silu_mul_interleaved", "tgis_k_gemm_any", "tgis_k_gemm_any_room", "tgis_k_rmsnorm_f32", "tgis_k_resid_tail", "tgis_k_latent_prep", "tgis_k_latent_q_rope", "tgis_k_latent_attn", "tgis_k_moe_route", "tgis_k_moe_align", "tgis_k_moe_route_grouped", "tgis_k_dyt_tail", "tgis_k_lightning_scan", "tgis_k_retention_scan", "tgis_k_gla_scan", "tgis_k_moe_table_align", "tgis_k_resid_tail_plain", "tgis_k_capattn_prep", "tgis_k_capattn", "tgis_k_sigattn_prep", "tgis_k_sigattn", "tgis_k_poolattn_prep", "tgis_k_poolattn", "tgis_k_delta_scan", "tgis_k_ssd_scan", "tgis_k_token_shift", "tgis_k_short_conv", "tgis_k_selective_scan", "tgis_k_outer_scan", "tgis_k_head_norm_gate", "tgis_k_resid_tail_pair", "tgis_k_resid_tail_two", "tgis_k_sizeof_sample_row", "tgis_k_sizeof_sample_out", "tgis_k_kv_block",
 ]
@@ -209,6 +209,7 @@ def load_library() -> C.CDLL:
     lib.tgis_k_gemm.argtypes = [vp, vp, vp, i32, i32, i32, i32, i32, i32, C.POINTER(f32), i32]
     lib.tgis_k_rmsnorm.argtypes = [vp, vp, vp, vp, i32, i32, f32]
     lib.tgis_k_skinny_norm_chain.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, f32, i32, i32]
+    lib.tgis_k_skinny_norm_rope.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, f32, C.POINTER(i32), C.POINTER(i32), vp, vp, vp, i32]
     lib.tgis_k_gemm_norm_chain.argtypes = [vp, i32, vp, vp, vp, vp, vp, i32, i32, i32, i32, f32, i32, i32, i32,
                                            C.POINTER(f32)]
     lib.tgis_k_silu_mul.argtypes = [vp, vp, i32, i32]
