@@ -205,12 +205,12 @@ capattn_kernel(const CT* __restrict__ q, const CT* __restrict__ k_cache, const C
 // weights are rounded to bf16 once and the SAME rounded numbers are summed for the normaliser.  Rows padded by 16 bytes keep
 // every fragment load free of bank conflicts.  A row's arithmetic does not depend on the other rows of its tile.
 //
-// What bounds it is issue: 62 million warp instructions for 2048 tokens in 7 prompts and 16 heads, of which a tile's products, tanh and
-// exponentials are less than a third; the rest was division by sizes known only at run time, in the copies.  With 128-wide heads known
-// when it is compiled, two k-steps to a load of key fragments, no comparison of positions in blocks that every query sees, and the heads
-// of a tile side by side (the caller lists long tiles first): 138 -> 75 us a layer; 32 single tokens behind 64 to 88 keys 14.4 -> 11.0.  Single tokens (ONE) fill
-// the M rows with the query heads of a key/value head instead of 15 rows of nothing, a quarter of the CTAs and of the copies: 11.0 ->
-// 8.0.  No faster: 32 queries a CTA (166 registers; 94 us), a warp per head of the group (186 registers; 89 us).
+// What bounds it is issue: 65 million warp instructions for 2048 tokens in 7 prompts and 16 heads with sizes known only at run time, 37
+// with 128-wide heads known when it is compiled, two k-steps to a load of key fragments and no comparison of positions in blocks that
+// every query sees (profiles/work_ncu.csv).  With the heads of a tile side by side and long tiles first (the caller's list) 138 -> 70 us
+// a layer; 32 single tokens behind 64 to 88 keys 14.4 -> 11.0.  Single tokens (ONE) fill the M rows with the query heads of a key/value
+// head instead of 15 rows of nothing, a quarter of the CTAs and of the copies: 11.0 -> 8.0.  Other widths keep the general form in both
+// (not measured).  No faster: 32 queries a CTA (166 registers; 94 us), a warp per head of the group (186 registers; 89 us).
 constexpr int MMA_KS = 8, MMA_NT = 8;
 __device__ __forceinline__ void ca_ldsm_x4(uint32_t (&r)[4], const void* smem) {
   const uint32_t a = (uint32_t)__cvta_generic_to_shared(smem);
@@ -569,7 +569,8 @@ capattn_mma_group_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat1
 // TGIS_CAPATTN_GROUP=1 routes grouped-query shapes to capattn_mma_group_kernel (read at every launch).  Off by default: measured
 // at 16 query / 4 key-value heads of 128 it is slower than one head per CTA (2048-token prefill step 172 against 148 us, a decode
 // step of 32 sequences 0.87 against 0.76 ms per step for the whole model) -- a quarter of the CTAs, each warp walking its whole
-// 16 x 32 tile alone with 162 registers, costs more than the K / V traffic it saves while the rows come out of L2.
+// 16 x 32 tile alone with 162 registers, costs more than the K / V traffic it saves while the rows come out of L2.  (Both figures are
+// from before capattn_mma_kernel had its forms for 128-wide heads, which are further ahead.)
 bool capattn_group_on() {
   const char* e = getenv("TGIS_CAPATTN_GROUP");
   return e != nullptr && e[0] == '1';

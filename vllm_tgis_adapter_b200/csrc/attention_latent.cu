@@ -334,7 +334,9 @@ latent_attn_mma_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __r
     }
   }
   const int32_t* bt = block_table + (size_t)sq.block_row * bt_stride;
-  const uint32_t per_row = (uint32_t)D / 8, magic = ((1u << 20) + per_row - 1) / per_row;   // c / per_row for c < 32 per_row <= 2^15
+  // c / per_row by a product: exact for c < 32 per_row while per_row <= 188; rows of more than 154 pieces have no room in shared memory
+  // (latent_mma_eligible)
+  const uint32_t per_row = (uint32_t)D / 8, magic = ((1u << 20) + per_row - 1) / per_row;
   auto load_block = [&](int blk, int st) {
     const bf* src = cache + (size_t)bt[blk] * KV_BLOCK * D;
     bf* dst = Ks + (size_t)st * KV_BLOCK * LDQ;
@@ -556,7 +558,7 @@ latent_attn_wide_kernel(const float* __restrict__ q_abs, const __nv_bfloat16* __
   const int pos_last = pos0 + nq - 1, kmin = g.window > 0 ? max(0, pos0 - g.window + 1) : 0;
   const int blk0 = kmin / KV_BLOCK, blk1 = pos_last / KV_BLOCK;
   const int32_t* bt = block_table + (size_t)sq.block_row * bt_stride;
-  const uint32_t per_row = (uint32_t)D / 8, magic = ((1u << 20) + per_row - 1) / per_row;   // c / per_row for c < 32 per_row <= 2^15
+  const uint32_t per_row = (uint32_t)D / 8, magic = ((1u << 20) + per_row - 1) / per_row;   // c / per_row (latent_attn_mma_kernel)
   auto load_block = [&](int blk, int st) {
     const bf* src = cache + (size_t)bt[blk] * KV_BLOCK * D;
     bf* dst = Ks + (size_t)st * KV_BLOCK * LDQ;

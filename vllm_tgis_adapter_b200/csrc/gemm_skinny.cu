@@ -325,7 +325,7 @@ cudaError_t gemm_skinny_launch(const void* X, const void* W, void* Y, int ldy, i
 // Norms between the products of a small model's decode steps, for up to eight tokens: the product in front adds to the residual stream and
 // leaves sums of squares, the one behind normalises its rows as it loads them.  In a chain a launch of its own costs 0.45 us more (12
 // layers 768 wide, one request, 17 + 16 tokens: 4.34 -> 4.17 ms).  Every CTA reading the whole row and norming it over again had been slower
-// than that launch (6.9 us against 4.0 + 2.0): it had a row to wait for and to sum; here it has three numbers a lane.
+// than that launch (6.9 us against 4.0 + 2.0): it had a row to wait for and to sum; here it has hidden / 256 numbers a lane, three at 768, at most eight.
 bool gemm_skinny_norm_takes(int T, int hidden, int q_dim, int qkv_dim, int ffn) {
   return T >= 1 && T <= 8 && hidden % 8 == 0 && hidden <= 2048 &&   // (2048: one vector a thread of rmsnorm_kernel)
          gemm_skinny_takes(T, qkv_dim, hidden) && gemm_skinny_takes(T, hidden, q_dim) && gemm_skinny_takes(T, 2 * ffn, hidden) && gemm_skinny_takes(T, hidden, ffn);

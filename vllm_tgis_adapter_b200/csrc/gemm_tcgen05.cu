@@ -259,7 +259,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_
   // t = r (mod s) belong to rank r), ONE cluster barrier, then each owner sums its own shared memory in rank order -- no
   // remote read latency and no exit barrier (pull variant: park locally, barrier, read peers, barrier)
   const bool cl_push = (stream_weights & 4) != 0;
-  const bool late = (stream_weights & 8) != 0;   // (GemmLate: dependents start once the operands are final)
+  const bool late = (stream_weights & 8) != 0;   // (dependents start once the operands are final)
   stream_weights &= 1;
   const long long total = sched.sk_total;  // stream-K region (== everything for decode-shaped launches)
 

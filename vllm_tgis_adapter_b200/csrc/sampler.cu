@@ -15,18 +15,17 @@
 // in a fixed order (deterministic).  The row is read from HBM once and stays in shared memory or the L2 for the selection passes
 // (radix-select thresholds instead of the reference's full sorts).  Every sweep takes eight entries per thread and 16-byte load.
 //   first sweep   32 entries a thread at a time: their maximum, then exponentials that do not wait for one another (an online
-//                 maximum per entry was a chain of a branch and an exponential each: 9100 of a greedy row's 27000 cycles); behind
-//                 typical-p the entropy's sum too
+//                 maximum per entry was a chain of a branch and an exponential each); behind typical-p the entropy's sum too
 //   reductions    maximum, sums and best entry in one; an exchange is one 16-byte read per lane and shuffles
 //   selections    (typical-p, top-k, top-p) one sweep over steps of a 32nd of an octave, one that lists the selected step's entries, then
 //                 parts of a step and radix rounds over the list
 //   race          behind typical-p over the list of what is left; in flat rows over kept processed logits, two logarithms only
-//                 for entries that 1 - u cannot rule out (186 instructions an entry -> 100; it was 38 % of a flat row)
+//                 for entries that 1 - u cannot rule out
 //   rank, top-n   one sweep and one exchange, the slices' lists ordered by eight threads a candidate
 // Measured, 128256 bf16 logits with top-5, microseconds, with the online maximum, an exchange for each part, clusters by SM count and four
-// radix rounds over leading bits -> here: greedy 19.7 -> 17 (1 row), 39 -> 17 (16), 22 -> 18 (32), 38 -> 28 (96), 73 -> 54 (150); typical-p
-// 45 -> 36 (1), 88 -> 42 (16), 91 -> 59 (64), 157 -> 91 (96), 309 -> 177 (150); flat rows 63 -> 48 (1), 285 -> 173 (96); top-k with
-// top-p 63 -> 52 (1), 240 -> 129 (96).
+// radix rounds over leading bits -> here: greedy 19.7 -> 14 (1 row), 39 -> 15 (16), 22 -> 15 (32), 36 -> 29 (80), 73 -> 55 (150); typical-p
+// 44 -> 29 (1), 88 -> 38 (16), 61 -> 38 (32), 157 -> 91 (80), 312 -> 178 (150); flat rows 62 -> 41 (1), 286 -> 173 (80); top-k with top-p
+// 61 -> 42 (1), 238 -> 133 (80).  Warp instructions of 96 rows, millions (profiles/work_ncu.csv): greedy 19 -> 16, flat typical-p 152 -> 92.
 #include <cooperative_groups.h>
 
 #include <type_traits>
@@ -45,7 +44,7 @@ constexpr int SAMP_THREADS = 1024;
 constexpr int SAMP_WARPS = SAMP_THREADS / 32;
 constexpr int SAMP_LIST = SAMP_THREADS;      // entries a race or a top-n list holds
 constexpr int SAMP_FEW = 3 * SAMP_THREADS;   // ... a selection's list
-constexpr float SAMP_FLAT = 7.f;  // nats: as spread as over 1100 entries, more than a list holds
+constexpr float SAMP_FLAT = 7.f;  // nats: as spread as over 1100 entries, more than the list of a row's only CTA holds (of 2 to 8 CTAs: 2048 to 8192)
 constexpr float SAMP_FIX = 1073741824.0f;  // 2^30: probabilities are accumulated as fixed-point integers (see below)
 
 // LT = logits element type: __nv_bfloat16 on the product path (vLLM's lm_head emits model-dtype logits and the sampler
@@ -320,13 +319,6 @@ __device__ float cluster_sumf(Cl& c, float v, float* red, float4* xch) {
   const XchView w = cl_publish(c, xch, Xch4{v, 0.f, 0.f, 0.f});
   float acc = w.get(0).a;
   for (int r = 1; r < c.ncl; ++r) acc += w.get(r).a;
-  return acc;
-}
-__device__ int cluster_sumi(Cl& c, int v, int* red, float4* xch) {
-  v = block_sumi(v, red);
-  const XchView w = cl_publish(c, xch, Xch4{__int_as_float(v), 0.f, 0.f, 0.f});
-  int acc = 0;
-  for (int r = 0; r < c.ncl; ++r) acc += __float_as_int(w.get(r).a);
   return acc;
 }
 
@@ -650,7 +642,7 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
                     const uint32_t* allow_bitmap) {
   // dynamic shared memory: [slice of the raw logits (cache_x)] [slice of the processed logits, fp32 (cache_y)]
   extern __shared__ __align__(16) uint8_t dyn_smem[];
-  __shared__ float redf[2 * SAMP_WARPS];
+  __shared__ float redf[SAMP_WARPS];
   __shared__ int redi[SAMP_WARPS];
   __shared__ uint32_t hist[2][HIST_WORDS];
   __shared__ uint32_t hsum[CODES];
@@ -832,7 +824,7 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
     // entries are left, made again
     float mx = -INFINITY;
     const float temp = c.p.temperature;
-    const bool use_topk = c.p.top_k > 0 && c.p.top_k < V, use_topp = c.p.top_p < 1.0f, 
+    const bool use_topk = c.p.top_k > 0 && c.p.top_k < V, use_topp = c.p.top_p < 1.0f,
                keep_y = use_topk || use_topp || !c.typical || c.ent > SAMP_FLAT;
     auto scaled8 = [&](int i0, float (&v)[8]) {
       load_slice8(c, i0, v);
