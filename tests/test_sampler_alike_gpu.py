@@ -82,3 +82,28 @@ def test_topn_of_rows_in_order(V, dtype, cluster, monkeypatch):
         want = torch.sort(logits[i].double(), descending=True, stable=True).indices
         assert out["topn_ids"][i][: i + 1].tolist() == want[: i + 1].tolist(), i
         assert int(out["token"][i]) == int(want[0])
+
+
+@pytest.mark.parametrize("cluster", ["1", "4", "8"])
+@pytest.mark.parametrize("V", [8, 16, 24, 40, 256, 264, 1024, 1032, 4096])
+def test_topn_of_short_rows(V, cluster, monkeypatch):
+    """Slices shorter than the list, which few warps sweep: numbers, ties, rows of which all but a few or none are minus infinity."""
+    monkeypatch.setenv("TGIS_SAMPLER_CLUSTER", cluster)
+    gen, rows, n = torch.Generator().manual_seed(V), 24, min(V, 12)
+    logits = torch.randn(rows, V, generator=gen)
+    for i in range(rows):
+        if i % 4 == 1:
+            logits[i] = (logits[i] > 0.5).float()
+        elif i % 4 == 2:
+            logits[i, torch.randperm(V, generator=gen)[: V - 3]] = -float("inf")
+        elif i % 4 == 3:
+            logits[i] = logits[i].sort().values
+    r = np.zeros(rows, dtype=U.SAMPLE_ROW_DTYPE)
+    r["temperature"], r["top_p"], r["rep_penalty"], r["eos_id"], r["seq_slot"], r["logits_row"] = 1.0, 1.0, 1.0, -1, -1, np.arange(rows)
+    r["flags"], r["n_topn"] = U.SAMPLE_GREEDY | U.SAMPLE_LOGPROBS, 1 + np.arange(rows) % n
+    out = U.run_sampler(logits.cuda(), r)
+    for i in range(rows):
+        k = int(r["n_topn"][i])
+        want = torch.sort(logits[i].double(), descending=True, stable=True).indices[:k]
+        assert out["topn_ids"][i][:k].tolist() == want.tolist(), i
+        np.testing.assert_allclose(out["topn_lps"][i][:k], torch.log_softmax(logits[i].double(), -1)[want].numpy(), atol=2e-5)

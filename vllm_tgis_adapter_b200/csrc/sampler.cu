@@ -1027,7 +1027,7 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
         }
         b = block_argmax(b, redf, redi);
         prev_v = b.v;
-        prev_i = b.i;
+        prev_i = b.i < 0 ? 0x7fffffff : b.i;   // (the slice has no more: nothing comes behind that)
         if (threadIdx.x == 0) {
           cand_v[n] = b.v;
           cand_i[n] = b.i;
