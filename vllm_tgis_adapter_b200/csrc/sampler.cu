@@ -1082,10 +1082,11 @@ tgis_sampler_kernel(const LT* logits, int ld, int V, const SampleRow* __restrict
 
 // Cluster size of a launch: the most CTAs per row that run in one wave, a function of the launch's shape only, so that a captured
 // CUDA graph replays the same launch.  Clusters do not fill a GPU whose groups of SMs are no multiple of them: of 148 SMs, 15
-// clusters of eight and 33 of four are there at a time (16 rows took two waves of eight: 39 us greedy, 88 typical-p; as fours 17 and
-// 48; 34 rows in fours 33 and 94, in pairs 22 and 73).  Greedy rows, which have two sweeps and as many exchanges, take four, where eight
-// only cost a longer exchange (one row of 128256 17.3 us against 18.0, of 50272 14.4 against 16.6), up to the vocabulary where the
-// sweeps outweigh that.
+// clusters of eight and 33 of four are there at a time (16 rows in two waves of eight 24 us greedy, 57 typical-p, as fours 15 and 37; 34
+// rows in fours 28 and 73, in pairs 20 and 55).  Greedy rows, which have two sweeps and as many exchanges, take four where eight only cost a
+// longer exchange: one row of 8192 8.5 us against 10.3, fifteen of 32768 10.0 against 10.5.  The line lies where it was drawn before the
+// candidates' list had its closer bound; since then eight are ahead by themselves from 50272 on (one row 9.8 against 10.3, of 128256 11.3
+// against 13.2), which 16 steps of a 12-layer model with 50272 entries do not show (4137 us with eight, 4134 with four).
 int sampler_cluster_size(int n_rows, int any_complex, int vocab, int num_sms) {
   if (const char* e = getenv("TGIS_SAMPLER_CLUSTER")) {
     const int v = atoi(e);
