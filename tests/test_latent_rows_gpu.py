@@ -83,3 +83,23 @@ def test_hidden_rows_of_any_value_are_left_out():
     cache[2, 7:] = float("nan")   # positions 71 on
     dirty = run()
     assert torch.equal(dirty[:45], clean[:45]) and bool(dirty[45:].isnan().all())
+
+
+@pytest.mark.parametrize("n", [171, 1250])
+def test_a_key_of_no_weight_leaves_no_trace(n):
+    """A key whose scores are all minus infinity has a weight of zero and is left out, whatever its values are: alone and tile by tile."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    heads, kv_rank, cached, extra = 8, 128, 45, n + 10
+    geom, D, nb = _geom(heads, kv_rank, 8, 0), kv_rank + 8, -(-(45 + n) // 32)
+    cache, q = torch.randn(nb + 8, 32, D, generator=gen, device="cuda"), torch.randn(n + extra, heads, D, generator=gen, device="cuda")
+    q[..., 0] = -q[..., 0].abs() - 0.1
+    k = cache[:nb].reshape(-1, D).double()
+    cache[0, 17, 0] = cache[1, 3, 0] = float("inf")   # positions 17 and 35, every token's past
+    s = torch.einsum("qhd,kd->qhk", q[:n].double() * geom.scale, k)
+    hidden = torch.arange(nb * 32, device="cuda")[None, :] > torch.arange(cached, cached + n, device="cuda")[:, None]
+    hidden[:, [17, 35]] = True
+    want = torch.einsum("qhk,kd->qhd", torch.softmax(s.masked_fill(hidden[:, None], -float("inf")), -1), k[:, :kv_rank])
+    alone = _attend(q[:n].contiguous(), cache, [(0, n, cached + n, 0)], [list(range(nb))], geom)
+    assert ((alone.double() - want).abs() <= 2.0 ** -24 * (D * 30 + 400) * (want.abs() + 1)).all()
+    company = _attend(q, cache, [(0, n, cached + n, 0)] + [(n + i, 1, 3 + i % 10, 1 + i % 8) for i in range(extra)], [list(range(nb))] + [[nb + i] for i in range(8)], geom)
+    assert torch.equal(alone, company[:n])

@@ -832,6 +832,7 @@ latent_attn_rows_kernel(const float* __restrict__ q_abs, const float* __restrict
         for (int j = 0; j < 2; ++j) Sp[(ty + 16 * i) * LDS_ + tx + 16 * j] = c[i][j];
     }
     __syncthreads();
+    bool zero = false;
     if (sr < ROWS) {  // ---- softmax: keys sk, sk + 4, ... of row sr; sums in the order of a warp's sixteen-, eight-, ... lane exchanges over 32 keys
       float x[8];
 #pragma unroll
@@ -855,10 +856,12 @@ latent_attn_rows_kernel(const float* __restrict__ q_abs, const float* __restrict
 #pragma unroll
       for (int e = 0; e < 8; ++e) Pt[(sk + 4 * e) * LDP + sr] = x[e];
       if (sk == 0) corr_s[sr] = corr;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) zero |= x[e] == 0.f;
     }
-    __syncthreads();
-    {  // ---- output: rescale, then O += P C; in a block with hidden keys a weight of zero is left out (its row may hold anything)
-      const bool whole = (blk + 1) * KV_BLOCK - 1 <= pos0 && (g.window <= 0 || pos_last - blk * KV_BLOCK < g.window);
+    const bool whole = !__syncthreads_or(zero && sr < rows);
+    {  // ---- output: rescale, then O += P C; a weight of zero is left out (hidden keys, and keys of a score of minus infinity: their rows may
+       // hold anything), tested where the block has one
       const float* pt = Pt + warp * RPW;
 #pragma unroll
       for (int r = 0; r < RPW; ++r) {
