@@ -2449,7 +2449,7 @@ struct tgis_engine {
                         bt_stride, pnx_y1 + l.c_g, ld, pnx_oA, A, l.ca, stream, T == S));
       pnx_gemm(pnx_oA, A, H * s.vdim, l.w_o, pnx_o, DT_F32, W, T, W, H * s.vdim);
       OuterScan os{};
-      os.single = T == S;
+      os.single = T == S, os.longest = step_max_q, os.tokens = T;
       os.mode = OUTER_SCAN_GATED;
       os.q = pnx_y1 + l.c_mq; os.k = pnx_y1 + l.c_mk; os.v = pnx_y1 + l.c_mv; os.ldq = os.ldk = os.ldv = ld;
       os.q_scale = 1.f / std::sqrt((float)s.mm_dim);
@@ -2473,7 +2473,7 @@ struct tgis_engine {
       pnx_gemm(xc, A, I, l.w_x, flx_f2, DT_F32, R + 2 * N, T, R + 2 * N, I);
       pnx_gemm(flx_f2, DT_F32, R + 2 * N, l.w_dt, flx_f3, DT_F32, I, T, I, R);
       SelScan sc{};
-      sc.single = T == S;
+      sc.single = T == S, sc.longest = step_max_q, sc.tokens = T;
       sc.x = flx_f1; sc.xz = pnx_y1; sc.ld_xz = 2 * I; sc.proj = flx_f2; sc.ld_proj = R + 2 * N; sc.dt_rank = R;
       sc.dt_raw = flx_f3; sc.dt_b = l.dt_b; sc.A_log = l.A_log; sc.D = l.Dv; sc.S = l.st_S; sc.conv_state = l.st_conv;
       sc.out = flx_op2; sc.out_dtype = A; sc.inner = I; sc.state = N; sc.taps = s.conv;
@@ -2492,7 +2492,7 @@ struct tgis_engine {
       pnx_gemm(mix(4), A, W, l.w_w1, pnx_cq, A, R, T, R, W, GEMM_ANY_TANH);
       pnx_gemm(pnx_cq, A, R, l.w_w2, flx_f2, DT_F32, Ad, T, Ad, R);
       OuterScan os{};
-      os.single = T == S;
+      os.single = T == S, os.longest = step_max_q, os.tokens = T;
       os.mode = OUTER_SCAN_DECAY;
       os.q = pnx_y1; os.k = pnx_y1 + Ad; os.v = pnx_y1 + 2 * Ad; os.ldq = os.ldk = os.ldv = 4 * Ad;
       os.q_scale = 1.f;
@@ -2558,7 +2558,7 @@ struct tgis_engine {
       CK(short_conv_silu_launch(pnx_y1 + inner, ld, C, l.conv_w, l.conv_b, s.conv, d_pos, d_tokslot, l.st_conv, flx_f1, nullptr, A, T, stream));
       CK(conv_state_save_launch(pnx_y1 + inner, ld, C, s.conv, d_seqs, S, d_tokslot, l.st_conv, stream));
       OuterScan os{};
-      os.single = T == S;
+      os.single = T == S, os.longest = step_max_q, os.tokens = T;
       os.mode = OUTER_SCAN_SSD;
       os.v = flx_f1; os.k = flx_f1 + inner; os.q = flx_f1 + inner + GN; os.ldq = os.ldk = os.ldv = C;
       os.q_scale = 1.f;
@@ -2682,7 +2682,7 @@ struct tgis_engine {
       const int H = s.heads, hd = H * s.dim, hv = H * s.vdim, ld = l.in_cols;
       pnx_gemm(pnx_hA, A, W, l.w_in, pnx_y1, DT_F32, ld, T, ld, W);
       OuterScan os{};
-      os.single = T == S;
+      os.single = T == S, os.longest = step_max_q, os.tokens = T;
       os.mode = OUTER_SCAN_HGRN;
       os.q = pnx_y1 + l.c_q; os.k = nullptr; os.v = pnx_y1 + l.c_v; os.ldq = os.ldk = os.ldv = ld;
       os.q_scale = 1.f;
@@ -2781,7 +2781,7 @@ struct tgis_engine {
     auto lightning = [&](cudaStream_t st) {   // -> pnx_yS
       const int mH = s.mm_heads, mv = mH * s.mm_vdim;
       OuterScan os{};
-      os.single = T == S;
+      os.single = T == S, os.longest = step_max_q, os.tokens = T;
       os.mode = OUTER_SCAN_LIGHTNING;
       os.q = pnx_y1 + l.c_mq; os.k = pnx_y1 + l.c_mk; os.v = pnx_y1 + l.c_mv; os.ldq = os.ldk = os.ldv = ld;
       os.q_scale = 1.f;
@@ -2913,7 +2913,7 @@ struct tgis_engine {
         n_launches += 2;
       }
       OuterScan os{};
-      os.single = T == S;
+      os.single = T == S, os.longest = step_max_q, os.tokens = T;
       os.mode = OUTER_SCAN_GLA;
       os.q = pnx_y1 + l.c_q; os.k = pnx_y1 + l.c_k; os.v = pnx_y1 + l.c_v; os.ldq = os.ldk = os.ldv = ld;
       os.q_scale = 1.f / sqrtf((float)s.dim);
@@ -2936,7 +2936,7 @@ struct tgis_engine {
                       l.cos_sin2, d_pos, chunked ? flx_mix : nullptr, qkv, lead};
         CK(rotary_rows_launch(rr, T, st));
         OuterScan os{};
-        os.single = T == S;
+        os.single = T == S, os.longest = step_max_q, os.tokens = T;
         os.mode = OUTER_SCAN_RETENTION;
         os.q = pnx_y1 + l.c_mq; os.k = pnx_y1 + l.c_mk; os.v = pnx_y1 + l.c_mv; os.ldq = os.ldk = os.ldv = ld;
         os.q_scale = 1.f;
@@ -3677,6 +3677,7 @@ struct tgis_engine {
       const int q_len = batch[s].q_len;
       const int kv_len = r.n_computed + q_len;
       step_max_kv = std::max(step_max_kv, kv_len);
+      step_max_q = std::max(step_max_q, q_len);
       seqs[s] = AttnSeq{T, q_len, kv_len, s};
       memcpy(bt + (size_t)s * bt_stride, r.blocks.data(), sizeof(int32_t) * r.blocks.size());
       for (int j = 0; j < q_len; ++j) {
@@ -3699,7 +3700,6 @@ struct tgis_engine {
         LatentTile* lt16 = hs<LatentTile>(off_ltiles16);
         for (int q0 = 0; q0 < q_len; q0 += POOLATTN_TILE)
           lt16[step_n_ltiles16++] = LatentTile{s, q0, std::min(POOLATTN_TILE, q_len - q0), 0};
-        step_max_q = std::max(step_max_q, q_len);
         if (q_len == 1 && step_n_lead1 == s) ++step_n_lead1;
       }
       if (q_len == 1) {

@@ -604,6 +604,7 @@ struct SelScan {
   void* out; int out_dtype;
   int inner, state, taps;
   int single;            // every portion of the launch is one token
+  int longest, tokens;   // tokens of the longest portion (0: not said, taken for long) and of all
 };
 constexpr int SELSCAN_MAX_STATE = 128;
 cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot,
@@ -641,6 +642,7 @@ struct OuterScan {
   float inv_tau;                               // GLA
   int32_t* done;                               // GATED: [slots][heads], zero between launches
   int single;                                  // every portion of the launch is one token
+  int longest, tokens;                         // tokens of the longest portion (0: not said, taken for long) and of all
 };
 cudaError_t outer_scan_launch(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot,
                               cudaStream_t stream);

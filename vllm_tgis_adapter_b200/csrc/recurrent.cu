@@ -200,10 +200,12 @@ short_conv_run_kernel(const float* __restrict__ xz, int ld, int inner, const flo
   }
 }
 
-// The sequence of rank `rank` by length, longest first (ties in order), where the block has a thread for every one; else number `rank`.
-// (seqs is written by the host before the step.)
+// The sequence of rank `rank` by length, longest first (ties in order), of up to sixteen; of more, whose blocks fill the chip anyway, number
+// `rank` (a block's look at 64 lengths costs 2 us: 32 prompts of 32 tokens 77.7 -> 74.3 us without, 64 of 5 93.7 -> 84.4).  (seqs is
+// written by the host before the step.)
+constexpr int ORDERED_SEQS = 16;
 __device__ __forceinline__ int longest_first(const AttnSeq* __restrict__ seqs, int n_seqs, int rank, int* lens, int* pick) {
-  if (n_seqs <= 1 || n_seqs > (int)blockDim.x) return rank;
+  if (n_seqs <= 1 || n_seqs > ORDERED_SEQS) return rank;
   const int tid = threadIdx.x;
   if (tid < n_seqs) lens[tid] = seqs[tid].q_len;
   __syncthreads();
@@ -217,7 +219,7 @@ __device__ __forceinline__ int longest_first(const AttnSeq* __restrict__ seqs, i
 }
 
 // ------------------------------------------------------------------------------------------------ selective scan
-constexpr int SCAN_THREADS = 64, SCAN_CHUNK = 8, SCAN_REG_CHUNK = 16, SCAN_REG_STATE = 16, SCAN_LPC = 4, SCAN_RPL = SCAN_REG_STATE / SCAN_LPC;
+constexpr int SCAN_THREADS = 64, SCAN_CHUNK = 8, SCAN_REG_STATE = 16, SCAN_LPC = 4, SCAN_RPL = SCAN_REG_STATE / SCAN_LPC;
 // the convolution's tail: inputs of the last taps - 1 positions (entry e: position end - (taps - 1) + e)
 __device__ __forceinline__ void scan_save_conv(const SelScan& a, const AttnSeq& sq, int slot, int c) {
   const int K1 = a.taps - 1, first = sq.kv_len - sq.q_len;
@@ -233,20 +235,20 @@ __device__ __forceinline__ void scan_save_conv(const SelScan& a, const AttnSeq& 
 // Up to SCAN_REG_STATE states: grid (sequences * ceil(inner / 16)), SCAN_LPC lanes share a channel; lane `sub` keeps states
 // 4 sub .. + 3 and their decay rates in registers.  A channel's tokens follow one another, so what is bound is the number of
 // instructions a token takes, and where few channels are left their latency.  What the four lanes would all do is dealt out: of a chunk's
-// sixteen tokens a lane fetches four (step size, input, gate), takes their softplus, hands step size and input on by shuffle, and after the
-// chunk receives the four tokens' output sums (a transposing reduction: 12 shuffles for 16 tokens and 4 lanes) and gates and writes
+// CHUNK tokens a lane fetches a quarter (step size, input, gate), takes their softplus, hands step size and input on by shuffle, and after
+// the chunk receives its tokens' output sums (a transposing reduction: 12 shuffles for 16 tokens and 4 lanes) and gates and writes
 // them.  B and C rows go through two shared-memory buffers, read four states to a load; the next chunk's step sizes are worked out
 // beside this chunk's outputs, its loads a chunk before.  Whole chunks of ALL = SCAN_REG_STATE states have no branch in them, so that the
 // tokens' exponentials run beside one another and only the fma of a state waits for the token before; a sequence's last chunk tests
-// its tokens one by one.  Longest sequences first.  4096 channels of 16 states, microseconds without overlap: 2048 tokens in 7 prompts 306 -> 163, 32 prompts of
-// 64 tokens 142 -> 127; with chunks of 8 tokens 206 and 122, of 32 188 and 191.
-template <bool ALL>
+// its tokens one by one.  Longest sequences first.  4096 channels of 16 states, microseconds without overlap: 2048 tokens in 7 prompts 306 -> 163
+// (chunks of 32: 188); the length of a chunk stands at scan_chunk.
+template <bool ALL, int CHUNK>
 __global__ void __launch_bounds__(SCAN_THREADS)
 selective_scan_reg_kernel(SelScan a, const AttnSeq* __restrict__ seqs, int n_seqs, const int32_t* __restrict__ tok_slot) {
-  constexpr int CHUNK = SCAN_REG_CHUNK, TPL = CHUNK / SCAN_LPC, ROW = 2 * SCAN_REG_STATE, STAGE = CHUNK * ROW / SCAN_THREADS;
+  constexpr int TPL = CHUNK / SCAN_LPC, ROW = 2 * SCAN_REG_STATE, STAGE = CHUNK * ROW / SCAN_THREADS;
   static_assert(SCAN_LPC == 4 && SCAN_RPL == 4, "the reduction below deals a chunk's tokens to four lanes");
   __shared__ __align__(16) float BC[2][CHUNK * ROW];   // per token: B | C, zeros behind the last state
-  __shared__ int lens[SCAN_THREADS], pick;
+  __shared__ int lens[ORDERED_SEQS], pick;
   griddep_launch();
   constexpr int CH = SCAN_THREADS / SCAN_LPC;
   const int n_blk = (a.inner + CH - 1) / CH, N = ALL ? SCAN_REG_STATE : a.state, tid = threadIdx.x, lane = tid & 31, sub = tid % SCAN_LPC;
@@ -476,7 +478,7 @@ selective_scan_kernel(SelScan a, const AttnSeq* __restrict__ seqs, const int32_t
 // before the token loop, and its normaliser is kept a row per thread.
 // Bound by instruction issue and by the latency of a token's chain (one head's tokens are worked through one after the other, and a
 // prompt has only heads * vdim / 32 blocks).  Four rows to a shared-memory load and two to an fma.  This is the kernel of keys that leave
-// the last row group short; the others' prompts have outer_run_kernel.
+// the last row group short, and of steps whose portions are short; other prompts have outer_run_kernel.
 __device__ __forceinline__ unsigned long long pack2(float x, float y) {
   unsigned long long d;
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
@@ -498,11 +500,12 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long x, unsigne
   return d;
 }
 constexpr int OS_GROUPS = 8, OS_COLS = 32, OS_THREADS = OS_GROUPS * OS_COLS, OS_CHUNK = 16;
-template <int RPT, int MODE>
+// FULL: D == RPT * OS_GROUPS, every thread's rows are there (no branch in the token loop, so a token's loads go ahead of its sums).
+template <int RPT, int MODE, bool FULL>
 __global__ void __launch_bounds__(OS_THREADS)
 outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* __restrict__ tok_slot) {
   extern __shared__ __align__(16) float os_smem[];
-  const int D = a.dim, DP = (D + 3) & ~3;
+  const int D = FULL ? RPT * OS_GROUPS : a.dim, DP = (D + 3) & ~3;
   float* vec = os_smem;                                  // [OS_CHUNK][3][DP]: q | k | w (GATED: n q)
   float* vcol = vec + (size_t)OS_CHUNK * 3 * DP;         // [OS_CHUNK][OS_COLS]
   __shared__ float part[OS_CHUNK][OS_GROUPS][OS_COLS + 1];
@@ -670,7 +673,7 @@ outer_scan_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, const int32_t* 
 #pragma unroll
       for (int j = 0; j < NG; ++j) {
         const int i = 4 * (g + j * OS_GROUPS);
-        if (i + 4 <= D) {
+        if (FULL || i + 4 <= D) {
           const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(v3 + i), k4 = *reinterpret_cast<const ulonglong2*>(v3 + DP + i);
           ulonglong2 w4 = make_ulonglong2(wd2, wd2);
           if (OWN_DECAY) w4 = *reinterpret_cast<const ulonglong2*>(v3 + 2 * DP + i);
@@ -785,7 +788,7 @@ outer_run_kernel(OuterScan a, const AttnSeq* __restrict__ seqs, int n_seqs, cons
   float* part = vcol + RING * C * OS_COLS;       // [RING][C][OS_GROUPS][OS_COLS]
   float* vraw = part + RING * C * OS_GROUPS * OS_COLS;   // SSD: [RING][C][OS_COLS]
   __shared__ float gates[3][32][2], floor_m[3][32];  // as above, of three blocks of 32 tokens: one is made while chunks of the two before it are in the ring
-  __shared__ int lens[RUN_THREADS], pick, last_block;
+  __shared__ int lens[ORDERED_SEQS], pick, last_block;
   griddep_launch();
   const int tid = threadIdx.x, nz = (a.vdim + OS_COLS - 1) / OS_COLS, piece = blockIdx.x % (a.heads * nz);
   const int seq = longest_first(seqs, n_seqs, blockIdx.x / (a.heads * nz), lens, &pick);
@@ -1598,6 +1601,16 @@ cudaError_t short_conv_silu_launch(const float* xz, int ld, int inner, const flo
                   positions, tok_slot, conv_state, out_f32, out_op, out_dtype);
 }
 
+// Tokens of a chunk: sixteen for long portions, whose tokens' latency is what is bound; fewer where portions end inside their first chunks, or
+// where the blocks fill the chip several times over and eight tokens' registers let more of them in.  4096 channels of 16 states,
+// microseconds, chunks of 16 / 8 / 4: one portion of 1024 tokens 119 / 152 / -, 20 of 100 138 / 127 / 128, 32 of 16 44 / 36 / 36, 64 of 5 85 / 41 /
+// 37, 128 of 2 115 / 68 / 47, one of 200 beside 31 of 5 55 / 43 / 48; 256 channels, one of 128 beside 31 of 1 18 / 21 / 25.  (Before there were
+// chunks of 16 and branches out of the token loop: 282, 150, 43, 40, 61, 90; 36.)  Of fewer states chunks of eight are behind those of four.
+static int scan_chunk(const SelScan& a, int n_seqs, long long blocks) {
+  if (a.longest <= 0 || a.longest >= 256) return 16;
+  if (blocks <= 16 * 148) return a.longest >= 48 ? 16 : a.longest >= 7 ? 8 : 4;
+  return a.tokens >= 8 * n_seqs ? 8 : 4;
+}
 cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot,
                                   cudaStream_t stream) {
   if (n_seqs <= 0) return cudaSuccess;
@@ -1610,8 +1623,12 @@ cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_s
     constexpr int per_cta = SCAN_THREADS / SCAN_LPC;
     const long long blocks = (long long)n_seqs * ((a.inner + per_cta - 1) / per_cta);
     if (blocks >= (1ll << 31)) return cudaErrorInvalidValue;
-    return launch_k(a.state == SCAN_REG_STATE ? selective_scan_reg_kernel<true> : selective_scan_reg_kernel<false>, dim3((unsigned)blocks), dim3(SCAN_THREADS), 0,
-                    stream, a, seqs, n_seqs, tok_slot);
+    const bool all = a.state == SCAN_REG_STATE;
+    const int chunk = scan_chunk(a, n_seqs, blocks);
+    const auto kernel = chunk == 16 ? (all ? selective_scan_reg_kernel<true, 16> : selective_scan_reg_kernel<false, 16>)
+                      : chunk == 8 && all ? selective_scan_reg_kernel<true, 8>
+                      : all ? selective_scan_reg_kernel<true, 4> : selective_scan_reg_kernel<false, 4>;
+    return launch_k(kernel, dim3((unsigned)blocks), dim3(SCAN_THREADS), 0, stream, a, seqs, n_seqs, tok_slot);
   }
   const dim3 grid(n_seqs, (a.inner + SCAN_THREADS - 1) / SCAN_THREADS);
   const size_t smem = bc + (size_t)2 * a.state * SCAN_THREADS * sizeof(float);
@@ -1624,6 +1641,21 @@ cudaError_t selective_scan_launch(const SelScan& a, const AttnSeq* seqs, int n_s
   return launch_k(selective_scan_kernel, grid, dim3(SCAN_THREADS), smem, stream, a, seqs, tok_slot);
 }
 
+// Steps that run in outer_run_kernel.  It works a long portion through in half the time, but takes twice the time to begin and end one: of
+// few portions it is ahead from 16 or 17 tokens on (44 with keys of more than 128 rows and where the gate writes the key).  Where the pieces
+// fill the chip several times over it is from 28 on, and what many short portions lose outweighs the chain of one long one unless that is
+// twice as long as there are portions, or the portions are long on average.  Gated memory of 8 heads of 128 x 256, microseconds, outer_scan_kernel / here: 128
+// portions of 2 tokens 87 / 167, 32 of 16 43 / 51, of 32 75 / 74, of 64 143 / 124; one of 128 beside 31 of 1 60 / 48, of 64 beside 60 of 4
+// 62 / 82, of 100 beside 100 of 1 90 / 158.  One portion of 17 tokens 8.8 / 8.6, of 24 9.9 / 8.8, three of 3 5.7 / 7.6; 32 decayed heads of 64 x 64,
+// one portion of 17 5.4 / 4.7; keys that the gate writes, 8 heads of 128 x 128, one portion of 28 10.4 / 12.1.
+template <int RPT, int MODE>
+static bool outer_runs(const OuterScan& a, int n_seqs, long long pieces) {
+  constexpr bool slow = RPT > 16 || MODE == OUTER_SCAN_HGRN;
+  constexpr int chip = 3 * 148 * (RPT <= 16 ? 2 : 1);
+  if (a.longest <= 0) return true;
+  if (pieces <= chip) return a.longest >= (slow ? 44 : 16);
+  return a.longest >= (slow ? 44 : 28) && (a.longest >= 2 * n_seqs || a.tokens >= (RPT > 16 ? 80 : 40) * n_seqs);
+}
 template <int RPT, int MODE>
 static cudaError_t outer_run(const OuterScan& a, const AttnSeq* seqs, int n_seqs, int pieces, const int32_t* tok_slot, cudaStream_t stream) {
   auto al16 = [](const float* p, int ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; };   // (nullptr where the mode has none)
@@ -1649,15 +1681,16 @@ static cudaError_t outer_scan_rows(const OuterScan& a, const AttnSeq* seqs, int 
     }
   }
   const long long pieces = (long long)n_seqs * a.heads * ((a.vdim + OS_COLS - 1) / OS_COLS);
-  if (a.dim == RPT * OS_GROUPS && pieces < (1ll << 31))
+  if (a.dim == RPT * OS_GROUPS && pieces < (1ll << 31) && outer_runs<RPT, MODE>(a, n_seqs, pieces))
     return outer_run<RPT, MODE>(a, seqs, n_seqs, (int)pieces, tok_slot, stream);
   const dim3 grid(n_seqs, a.heads, (a.vdim + OS_COLS - 1) / OS_COLS);
   const size_t smem = ((size_t)OS_CHUNK * 3 * ((a.dim + 3) & ~3) + OS_CHUNK * OS_COLS) * sizeof(float);   // <= 50 KB (+ 17 KB static)
+  const auto kernel = a.dim == RPT * OS_GROUPS ? outer_scan_kernel<RPT, MODE, true> : outer_scan_kernel<RPT, MODE, false>;
   if (RPT > 16) {   // keys of more than 128 entries: the staged chunk passes the default 48 KB of shared memory
-    const cudaError_t e = cudaFuncSetAttribute(outer_scan_kernel<RPT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
     if (e != cudaSuccess) return e;
   }
-  return launch_k(outer_scan_kernel<RPT, MODE>, grid, dim3(OS_THREADS), smem, stream, a, seqs, tok_slot);
+  return launch_k(kernel, grid, dim3(OS_THREADS), smem, stream, a, seqs, tok_slot);
 }
 template <int MODE>
 static cudaError_t outer_scan_mode(const OuterScan& a, const AttnSeq* seqs, int n_seqs, const int32_t* tok_slot,

@@ -27,8 +27,11 @@ int kfail(const std::string& m) {
     if (_e != cudaSuccess) return kfail(std::string(#expr) + ": " + cudaGetErrorString(_e)); \
   } while (0)
 
-int all_single(const std::vector<AttnSeq>& seqs) {   // as the engine finds: every portion is one token
-  return std::all_of(seqs.begin(), seqs.end(), [](const AttnSeq& s) { return s.q_len == 1; });
+// as the engine finds: whether every portion is one token, the longest one, all tokens
+template <class Scan>
+void say_portions(Scan& a, const std::vector<AttnSeq>& seqs) {
+  a.single = 1;
+  for (const AttnSeq& s : seqs) a.longest = std::max(a.longest, s.q_len), a.tokens += s.q_len, a.single &= s.q_len == 1;
 }
 
 // end of a hook that may have launched products on CTA pairs
@@ -887,7 +890,7 @@ int tgis_k_ssd_scan(const float* q, const float* k, const float* v, int32_t ldq,
   a.mode = OUTER_SCAN_SSD; a.q = q; a.k = k; a.v = v; a.ldq = ldq; a.ldk = ldk; a.ldv = ldv; a.q_scale = 1.f;
   a.step_raw = step_raw; a.lds = lds; a.step_b = step_b; a.A_log = A_log; a.D = D;
   a.S = S; a.out = out; a.ldo = ldo; a.heads = heads; a.qk_heads = qk_heads; a.dim = dim; a.vdim = vdim;
-  a.single = all_single(seqs);
+  say_portions(a, seqs);
   KCK(outer_scan_launch(a, d_seqs.p, n_seqs, tok_slot, 0));
   KCK(cudaDeviceSynchronize());
   return 0;
@@ -920,7 +923,7 @@ int tgis_k_selective_scan(const float* x, const float* xz, int32_t ld_xz, const 
   a.x = x; a.xz = xz; a.ld_xz = ld_xz; a.proj = proj; a.ld_proj = ld_proj; a.dt_rank = dt_rank; a.dt_raw = dt_raw; a.dt_b = dt_b;
   a.A_log = A_log; a.D = D; a.S = S; a.conv_state = conv_state; a.out = out; a.out_dtype = out_dt; a.inner = inner;
   a.state = state; a.taps = taps;
-  a.single = all_single(seqs);
+  say_portions(a, seqs);
   KCK(selective_scan_launch(a, d_seqs.p, n_seqs, tok_slot, 0));
   KCK(cudaDeviceSynchronize());
   return 0;
@@ -954,7 +957,7 @@ int tgis_k_outer_scan(int32_t mode, const float* q, const float* k, const float*
     KCK(cudaMemset(done.p, 0, (size_t)heads * slots * sizeof(int32_t)));
     a.done = done.p;
   }
-  a.single = all_single(seqs);
+  say_portions(a, seqs);
   KCK(outer_scan_launch(a, d_seqs.p, n_seqs, tok_slot, 0));
   KCK(cudaDeviceSynchronize());
   return 0;
@@ -984,7 +987,7 @@ int tgis_k_lightning_scan(const float* q, const float* k, const float* v, int32_
     KCK(cudaDeviceSynchronize());
     return 0;
   }
-  a.single = all_single(seqs);
+  say_portions(a, seqs);
   KCK(outer_scan_launch(a, d_seqs.p, n_seqs, tok_slot, 0));
   KCK(cudaDeviceSynchronize());
   return 0;
@@ -1009,7 +1012,7 @@ int tgis_k_retention_scan(float* x, int32_t ld, int32_t q_off, int32_t k_off, in
     a.mode = OUTER_SCAN_RETENTION;
     a.q = x + q_off; a.k = x + k_off; a.v = x + v_off; a.ldq = a.ldk = a.ldv = ld; a.q_scale = 1.f;
     a.decay = decay; a.S = S; a.out = out; a.ldo = ldo; a.heads = heads; a.dim = dim; a.vdim = vdim;
-    a.single = all_single(seqs);
+    say_portions(a, seqs);
     KCK(outer_scan_launch(a, d_seqs.p, n_seqs, tok_slot, 0));
   }
   KCK(cudaDeviceSynchronize());
@@ -1048,7 +1051,7 @@ int tgis_k_gla_scan(const float* x, int32_t ld, int32_t q_off, int32_t k_off, in
   a.q = x + q_off; a.k = x + k_off; a.v = x + v_off; a.ldq = a.ldk = a.ldv = ld; a.q_scale = q_scale;
   a.decay_raw = z.p; a.ldd = hd; a.w0 = bias; a.inv_tau = inv_tau;
   a.S = S; a.out = out; a.ldo = ldo; a.heads = heads; a.dim = dim; a.vdim = vdim;
-  a.single = all_single(seqs);
+  say_portions(a, seqs);
   KCK(outer_scan_launch(a, d_seqs.p, n_seqs, tok_slot, 0));
   KCK(cudaDeviceSynchronize());
   return 0;
